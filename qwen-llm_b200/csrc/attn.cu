@@ -12,7 +12,7 @@ namespace dfl {
 
 // ---- front: reduce GEMM partials, per-head RMSNorm, partial NeoX RoPE, KV append ---------
 // grid (heads = n_q + 2 n_kv, n_rows), block = 128 threads (4 warps cooperate on one head).
-__global__ void __launch_bounds__(128) attn_front_kernel(AttnGeom g, int gated, const float* part, int splits,
+__global__ void __launch_bounds__(128) attn_front_kernel(AttnGeom g, int gated, const float* part, int splits, int part_rows,
                                                          int ld_part, const float* __restrict__ q_norm_w,
                                                          const float* __restrict__ k_norm_w, uint32_t start, void* k_cache,
                                                          void* v_cache, int kv_mode, float* q_rot,
@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(128) attn_front_kernel(AttnGeom g, int gated, 
     for (int d = threadIdx.x; d < hd; d += blockDim.x) {
         float v = 0.f, gt = 0.f;
         for (int s = 0; s < splits; ++s) {
-            const float* row = part + ((uint64_t)s * MAX_ROWS + tok) * ld_part;
+            const float* row = part + ((uint64_t)s * part_rows + tok) * ld_part;
             v += row[col0 + d];
             if (kind == 0 && gated) gt += row[col0 + hd + d];
         }
@@ -84,9 +84,9 @@ __global__ void __launch_bounds__(128) attn_front_kernel(AttnGeom g, int gated, 
 
 dfl_status launch_attn_front(cudaStream_t st, const AttnGeom& g, bool gated, const float* part, int splits, int ld_part,
                              const float* q_norm_w, const float* k_norm_w, uint32_t start, int n_rows, void* k_cache,
-                             void* v_cache, int kv_mode, float* q_rot, float* gate, const uint32_t* pos_override, long long cache_row0) {
+                             void* v_cache, int kv_mode, float* q_rot, float* gate, const uint32_t* pos_override, long long cache_row0, int part_rows) {
     dim3 grid((unsigned)(g.n_q + 2 * g.n_kv), (unsigned)n_rows);
-    launch_k(attn_front_kernel, dim3(grid), dim3(128), (g.hd + 4) * sizeof(float), st, g, gated ? 1 : 0, part, splits, ld_part, q_norm_w, k_norm_w, start,
+    launch_k(attn_front_kernel, dim3(grid), dim3(128), (g.hd + 4) * sizeof(float), st, g, gated ? 1 : 0, part, splits, part_rows, ld_part, q_norm_w, k_norm_w, start,
                                                                    k_cache, v_cache, kv_mode, q_rot, gate, pos_override, cache_row0);
     count_launch();
     DFL_CUDA(cudaGetLastError());

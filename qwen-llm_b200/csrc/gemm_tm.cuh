@@ -1,0 +1,437 @@
+// Many-row GEMM over the resident K-quant tiles (prompt passes: 17 rows and more); included by gemm_ts.cu only.
+//
+// Same weights, same arithmetic class as the few-row kernel: weights stay the integers q * sc (exact in f16), activations
+// are f16 hi + lo, products accumulate in f32 and the super-block scale d is applied in f32 after every 256 columns.
+// What changes is the ratio: one unpacked 128 x 256 weight tile is multiplied with 128 tokens instead of 16, so that the
+// tensor pipe, not the unpack, is what a CTA spends its time on.  Per 256-column block (1 CTA per SM):
+//   * MMA: 16 k-steps x {hi, lo} of M 128 N 128 K 16 (64 clocks each) = 2048 clocks, plus two for the K-quant min term;
+//     Q6_K: q * sc needs up to 13 bits, A1 = fl16(q * sc) and A2 = q * sc - A1 in {-1, 0, 1}; A1 x {hi, lo} + A2 x hi
+//     (A2 x lo is below 2^-24 of the product's range) = 3072 clocks;
+//   * unpack: 16 warps, about 1000 - 1300 clocks of issue, hidden under the MMAs;
+//   * activations: 128 KiB of hi / lo planes per block and CTA from L2, 60 bytes a clock, the other near-limit.
+// The min term -dmin * m_j * sum(x over sub-block j) rides in the same accumulator: its A operand is -(dmin / s) m_j as
+// an f16 hi + lo pair, s = the factor the accumulator is multiplied with afterwards (d, except where dmin / d would leave
+// the f16 range), its B operand the sub-block sums as f16 hi + lo.
+//
+// Warps: 0..15 unpack (two groups of eight; group g owns A buffer g: Q4_K / Q5_K half g of a block, Q6_K quarters g and
+// g + 2), 16..19 read the accumulator back (thread = weight row), 20 issues the MMAs, 21 streams weights, 22 activations.
+// Tensor memory: two 128-column block accumulators (one fills while the other is read back), the running sum over blocks
+// (128), two 64-column A buffers: all 512 columns.
+#pragma once
+
+namespace dfl {
+namespace ts {
+
+constexpr int TM_WARPS = 23, TM_THREADS = TM_WARPS * 32;
+constexpr int TM_MMA_WARP = 20, TM_W_WARP = 21, TM_B_WARP = 22;
+constexpr int TM_B_STAGES = 4;
+constexpr uint32_t TM2_D = 0, TM2_ACC = 256, TM2_A = 384;
+constexpr int TM_BAR_BYTES = 512;
+
+struct TmParams {
+    const uint8_t* w;
+    const uint8_t* acts;      // [token tile][column block] chunks of TM_CHUNK bytes
+    float* out;               // [splits][rows_pad][ld_out]
+    const float* sumsq;       // [n_sumsq][rows_pad]
+    int n_sumsq;
+    float norm_k, eps, out_scale;
+    int kblocks, splits, row_tiles, tok_tiles, n_rows, rows_pad;
+    uint32_t n_out, ld_out;
+    int* err;
+};
+
+template <int DT>
+struct TmFmt {
+    static constexpr bool MIN = DT != DFL_Q6_K;
+    static constexpr int W_STAGE = Fmt<DT>::STAGE;
+    static constexpr int W_STAGES = DT == DFL_Q6_K ? 2 : 3;
+    static constexpr int USES = MIN ? 1 : 2;      // how often a block uses each A buffer
+    static constexpr int OFF_W = TM_B_STAGES * TM_BSTAGE;
+    static constexpr int OFF_AM = OFF_W + W_STAGES * W_STAGE;          // [2] min-term A operand, 128 x 16
+    static constexpr int OFF_S = OFF_AM + (MIN ? 2 * 4096 : 0);        // [2] min-term B operand
+    static constexpr int OFF_SCL = OFF_S + (MIN ? 2 * TM_SUMS : 0);    // [4][128] block scales
+    static constexpr int OFF_BAR = OFF_SCL + 4 * TILE_R * 4;
+    static constexpr int SMEM = OFF_BAR + TM_BAR_BYTES;
+};
+
+// Scale of a row's accumulator for one block and the factor its min operand is divided by.  Normally s = d; where the
+// ratio dmin / d leaves the f16 range of the min operand, s grows by powers of two and the integer operand shrinks with it.
+struct TmScale {
+    float s, ratio, shrink;   // shrink: factor of the integer operand (1 unless rare)
+};
+__device__ __forceinline__ TmScale tm_scale(float d, float dmin) {
+    TmScale r{d, dmin / d, 1.f};
+    if (!(fabsf(r.ratio) <= 512.f)) {   // 512 * 63 < 65504; also d == 0
+        if (d == 0.f) { r.s = 1.f; r.shrink = 0.f; }
+        for (int i = 0; i < 48 && fabsf(dmin / r.s) > 512.f; ++i) { r.s *= 2.f; r.shrink *= 0.5f; }
+        r.ratio = dmin / r.s;
+    }
+    return r;
+}
+
+template <int DT>
+__global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p) {
+    using T = TmFmt<DT>;
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t* b_ring = smem;
+    uint8_t* w_ring = smem + T::OFF_W;
+    float* scl = reinterpret_cast<float*>(smem + T::OFF_SCL);
+    uint64_t* w_full = reinterpret_cast<uint64_t*>(smem + T::OFF_BAR);
+    uint64_t* w_empty = w_full + T::W_STAGES;
+    uint64_t* b_full = w_empty + T::W_STAGES;
+    uint64_t* b_empty = b_full + TM_B_STAGES;
+    uint64_t* s_full = b_empty + TM_B_STAGES;   // [2] sub-block sums of a block
+    uint64_t* s_empty = s_full + 2;
+    uint64_t* a_ready = s_empty + 2;            // [buffer] unpacked weights are in tensor memory
+    uint64_t* a_free = a_ready + 2;
+    uint64_t* d_ready = a_free + 2;             // [accumulator] every MMA of a block has completed
+    uint64_t* d_free = d_ready + 2;
+    __shared__ uint32_t tmem_slot;
+    __shared__ float tok_scale[TM_TOK];
+    __shared__ int abort_flag;
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int n_items = p.row_tiles * p.splits * p.tok_tiles;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < T::W_STAGES; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], UNPACK_WARPS); }
+        for (int i = 0; i < TM_B_STAGES; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&s_full[i], 1);
+            mbar_init(&s_empty[i], 1);
+            mbar_init(&a_ready[i], GROUP_WARPS);
+            mbar_init(&a_free[i], 1);
+            mbar_init(&d_ready[i], 1);
+            mbar_init(&d_free[i], DRAIN_WARPS);
+        }
+        abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == TM_MMA_WARP) tmem_alloc(&tmem_slot, 512);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+
+    // item -> (row tile, split, token tile): the token tiles of one weight tile are neighbours, so that its bytes come from
+    // HBM once and from L2 for the others
+    struct Item { int rt, tt, kb0, n_kb, sp; };
+    auto item_of = [&](int idx) {
+        Item it;
+        it.tt = idx % p.tok_tiles;
+        const int r = idx / p.tok_tiles;
+        it.sp = r % p.splits;
+        it.rt = r / p.splits;
+        it.kb0 = (int)((long long)it.sp * p.kblocks / p.splits);
+        it.n_kb = (int)((long long)(it.sp + 1) * p.kblocks / p.splits) - it.kb0;
+        return it;
+    };
+    bool ok = true;
+
+    if (warp == TM_W_WARP) {
+        // ------------------------------ weights ------------------------------
+        if (lane == 0) {
+            int s = 0;
+            uint32_t round = 0;
+            for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
+                const Item it = item_of(idx);
+                const uint8_t* src = p.w + ((uint64_t)it.rt * p.kblocks + it.kb0) * T::W_STAGE;
+                for (int k = 0; k < it.n_kb; ++k, src += T::W_STAGE) {
+                    if (round > 0 && !(ok = mbar_wait_bounded(&w_empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY))) break;
+                    mbar_arrive_expect_tx(&w_full[s], T::W_STAGE);
+                    bulk_g2s(w_ring + s * T::W_STAGE, src, T::W_STAGE, &w_full[s]);
+                    if (++s == T::W_STAGES) { s = 0; ++round; }
+                }
+            }
+        }
+    } else if (warp == TM_B_WARP) {
+        // ------------------------------ activations ------------------------------
+        if (lane == 0) {
+            pdl_wait();
+            int s = 0;
+            uint32_t round = 0, e = 0;
+            for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
+                const Item it = item_of(idx);
+                const uint8_t* src = p.acts + ((uint64_t)it.tt * p.kblocks + it.kb0) * TM_CHUNK;
+                for (int k = 0; k < it.n_kb && ok; ++k, src += TM_CHUNK, ++e) {
+                    if (T::MIN) {
+                        if (e >= 2) ok = mbar_wait_bounded(&s_empty[e & 1], ((e >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
+                        if (!ok) break;
+                        mbar_arrive_expect_tx(&s_full[e & 1], TM_SUMS);
+                        bulk_g2s(smem + T::OFF_S + (e & 1) * TM_SUMS, src + 4 * TM_BSTAGE, TM_SUMS, &s_full[e & 1]);
+                    }
+                    for (int q = 0; q < 4; ++q) {
+                        if (round > 0 && !(ok = mbar_wait_bounded(&b_empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY))) break;
+                        mbar_arrive_expect_tx(&b_full[s], TM_BSTAGE);
+                        bulk_g2s(b_ring + s * TM_BSTAGE, src + q * TM_BSTAGE, TM_BSTAGE, &b_full[s]);
+                        if (++s == TM_B_STAGES) { s = 0; ++round; }
+                    }
+                }
+            }
+        }
+    } else if (warp == TM_MMA_WARP) {
+        // ------------------------------ MMA issue ------------------------------
+        constexpr uint32_t IDESC = instr_desc(TM_TOK);
+        const uint64_t bd = smem_desc(smem_u32(b_ring), TM_TOK * 16, 128);
+        const uint32_t b_lo = (uint32_t)bd, b_hi = (uint32_t)(bd >> 32);
+        uint32_t e = 0, bs = 0, bround = 0;
+        auto wait = [&](uint64_t* bar, uint32_t parity) {
+            ok = mbar_wait_bounded(bar, parity, p.err, DEV_ERR_WAIT_FULL);
+            ok = __all_sync(0xffffffffu, ok);
+            return ok;
+        };
+        for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
+            const Item it = item_of(idx);
+            for (int k = 0; k < it.n_kb && ok; ++k, ++e) {
+                const uint32_t d = tmem + TM2_D + (e & 1) * 128;
+                if (e >= 2 && !wait(&d_free[e & 1], ((e >> 1) - 1) & 1)) break;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {   // 64 columns = one activation stage
+                    const int g = T::MIN ? q >> 1 : q & 1;
+                    const uint32_t a = tmem + TM2_A + 64 * g;
+                    if (!T::MIN || (q & 1) == 0) {
+                        if (!wait(&a_ready[g], (T::MIN ? e : 2 * e + (q >> 1)) & 1)) break;
+                    }
+                    if (!wait(&b_full[bs], bround & 1)) break;
+                    fence_after_sync();
+                    if (elect_one()) {
+                        const uint32_t b = b_lo + bs * (TM_BSTAGE / 16);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const uint32_t aj = a + (T::MIN ? 32 * (q & 1) : 0) + 8 * j;
+                            if (q == 0 && j == 0) mma_ts<false>(d, aj, b, b_hi, IDESC);
+                            else mma_ts<true>(d, aj, b + j * 256, b_hi, IDESC);
+                            mma_ts<true>(d, aj, b + (TM_BSTAGE / 32) + j * 256, b_hi, IDESC);
+                            if (!T::MIN) mma_ts<true>(d, aj + 32, b + j * 256, b_hi, IDESC);
+                        }
+                        mma_commit(&b_empty[bs]);
+                        if (!T::MIN) mma_commit(&a_free[g]);
+                    }
+                    __syncwarp();
+                    if (++bs == TM_B_STAGES) { bs = 0; ++bround; }
+                    if (T::MIN && q == 3) {
+                        if (!wait(&s_full[e & 1], (e >> 1) & 1)) break;
+                        if (elect_one()) {
+                            const uint64_t ad = smem_desc(smem_u32(smem + T::OFF_AM + (e & 1) * 4096), 2048, 128);
+                            const uint64_t sd = smem_desc(smem_u32(smem + T::OFF_S + (e & 1) * TM_SUMS), TM_TOK * 16, 128);
+                            mma_ss(d, ad, sd, IDESC, 1u);
+                            mma_ss(d, ad, sd + TM_SUMS / 32, IDESC, 1u);
+                            mma_commit(&s_empty[e & 1]);
+                        }
+                        __syncwarp();
+                    }
+                    if (T::MIN && (q & 1)) {
+                        if (elect_one()) mma_commit(&a_free[g]);
+                        __syncwarp();
+                    }
+                }
+                if (ok) {
+                    if (elect_one()) mma_commit(&d_ready[e & 1]);
+                    __syncwarp();
+                }
+            }
+        }
+    } else if (warp < UNPACK_WARPS) {
+        // ------------------------------ unpack ------------------------------
+        const int g = warp >> 3, q4 = warp & 3, kp2 = (warp >> 2) & 1;
+        const int row = 32 * q4 + lane;
+        const uint32_t a_buf = tmem + ((uint32_t)(32 * q4) << 16) + TM2_A + 64 * g;
+        uint32_t e = 0, use = 0;
+        int s = 0;
+        uint32_t round = 0;
+        for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
+            const int n_kb = item_of(idx).n_kb;
+            for (int k = 0; k < n_kb && ok; ++k, ++e) {
+                ok = mbar_wait_bounded(&w_full[s], round & 1, p.err, DEV_ERR_WAIT_FULL);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const uint8_t* st = w_ring + s * T::W_STAGE;
+#pragma unroll
+                for (int u = 0; u < T::USES; ++u, ++use) {
+                    uint32_t r[32], am[8];
+                    UnitScales us{0.f, 0.f};
+                    TmScale sc{0.f, 0.f, 1.f};
+                    if constexpr (T::MIN) {
+                        Fmt<DT>::unpack(st, g, row, kp2, r, am, us);
+                        sc = tm_scale(us.d, us.dmin);
+                        if (sc.shrink != 1.f) {
+                            const __half2 f2 = __float2half2_rn(sc.shrink);
+                            const uint32_t f = *reinterpret_cast<const uint32_t*>(&f2);
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) r[i] = h2mul(r[i], f);
+                        }
+                    } else {
+                        tm_unpack_q6k(st, g + 2 * u, row, kp2, r, us);
+                        sc.s = us.d;
+                    }
+                    if (u == T::USES - 1) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&w_empty[s]);   // every lane has its bytes in registers
+                    }
+                    if (use >= 1) {
+                        ok = mbar_wait_bounded(&a_free[g], (use - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        fence_after_sync();
+                    }
+                    if (T::MIN) {
+                        tmem_st32(a_buf + 32 * kp2, r);
+                        // the min operand of this thread's two sub-blocks, k = 2 kp and 2 kp + 1 (hi) and 8 further (lo)
+                        const float2 m = __half22float2(*reinterpret_cast<const __half2*>(&am[0]));
+                        const float f0 = -sc.ratio * m.x, f1 = -sc.ratio * m.y;
+                        const __half2 hi = __floats2half2_rn(f0, f1);
+                        const float2 back = __half22float2(hi);
+                        const __half2 lo = __floats2half2_rn(f0 - back.x, f1 - back.y);
+                        uint8_t* dst = smem + T::OFF_AM + (e & 1) * 4096 + (row >> 3) * 128 + (row & 7) * 16 + (2 * g + kp2) * 4;
+                        *reinterpret_cast<__half2*>(dst) = hi;
+                        *reinterpret_cast<__half2*>(dst + 2048) = lo;
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    } else {
+                        uint32_t a1[16], a2[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) { a1[i] = r[i]; a2[i] = r[16 + i]; }
+                        tmem_st16(a_buf + 16 * kp2, a1);
+                        tmem_st16(a_buf + 32 + 16 * kp2, a2);
+                    }
+                    if (g == 0 && u == 0 && kp2 == 0) scl[(e & 3) * TILE_R + row] = sc.s;
+                    wait_st();
+                    fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&a_ready[g]);
+                }
+                if (++s == T::W_STAGES) { s = 0; ++round; }
+            }
+        }
+    } else {
+        // ------------------------------ read-back ------------------------------
+        pdl_wait();
+        const int row = threadIdx.x - DRAIN_WARP0 * 32;   // weight row of the tile = tensor-memory lane
+        const uint32_t tm_l = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        uint32_t e = 0;
+        int scaled_tt = -1;
+        for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
+            const Item it = item_of(idx);
+            if (it.tt != scaled_tt) {   // per-token output scale of the token tile, thread = token
+                scaled_tt = it.tt;
+                named_sync(1, DRAIN_WARPS * 32);
+                float ss = 0.f;
+                if (p.sumsq)
+                    for (int q = 0; q < p.n_sumsq; ++q) ss += p.sumsq[(uint64_t)q * p.rows_pad + it.tt * TM_TOK + row];
+                tok_scale[row] = p.sumsq ? p.out_scale * (1.0f / sqrtf(ss / p.norm_k + p.eps)) : p.out_scale;
+                named_sync(1, DRAIN_WARPS * 32);
+            }
+            for (int k = 0; k < it.n_kb && ok; ++k, ++e) {
+                ok = mbar_wait_bounded(&d_ready[e & 1], (e >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                fence_after_sync();
+                const float s = scl[(e & 3) * TILE_R + row];
+                const uint32_t d = tm_l + TM2_D + (e & 1) * 128;
+                const bool last = k == it.n_kb - 1;
+                const uint32_t orow = (uint32_t)it.rt * TILE_R + row;
+#pragma unroll 1
+                for (int c = 0; c < 8; ++c) {   // 16 tokens
+                    float v[16], a[16];
+                    tmem_ld16(d + 16 * c, v);
+                    if (k > 0) tmem_ld16(tm_l + TM2_ACC + 16 * c, a);
+                    wait_ld();
+                    if (c == 7) {
+                        fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&d_free[e & 1]);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = k > 0 ? fmaf(s, v[j], a[j]) : s * v[j];
+                    if (!last) {
+                        uint32_t u[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(v[j]);
+                        tmem_st16(tm_l + TM2_ACC + 16 * c, u);
+                    } else if (orow < p.n_out) {
+                        const int tok0 = it.tt * TM_TOK + 16 * c;
+                        float* dst = p.out + ((uint64_t)it.sp * p.rows_pad + tok0) * p.ld_out + orow;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (tok0 + j < p.n_rows) dst[(uint64_t)j * p.ld_out] = v[j] * tok_scale[16 * c + j];
+                    }
+                    __syncwarp();
+                }
+                if (!last) wait_st();
+            }
+        }
+    }
+    if (!ok) abort_flag = 1;
+    fence_before_sync();
+    __syncthreads();
+    if (abort_flag && threadIdx.x == 0) {
+        // error word already set: a bounded chance for copies still in flight before the shared memory is released
+        auto settle = [](uint64_t* b) {
+            uint32_t spins = 0;
+            while (!mbar_try_wait(b, 0) && !mbar_try_wait(b, 1) && ++spins < (1u << 16)) __nanosleep(100);
+        };
+        for (int i = 0; i < T::W_STAGES; ++i) settle(&w_full[i]);
+        for (int i = 0; i < TM_B_STAGES; ++i) settle(&b_full[i]);
+        for (int i = 0; i < 2; ++i) settle(&s_full[i]);
+    }
+    __syncthreads();
+    if (warp == TM_MMA_WARP) {
+        fence_after_sync();
+        tmem_free(tmem, 512);
+    }
+}
+
+template <int DT>
+static dfl_status launch_tm(cudaStream_t st, const TmParams& p) {
+    static std::once_flag once[16];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaError_t e = cudaSuccess;
+    auto set = [&] { e = cudaFuncSetAttribute(gemm_tm_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TmFmt<DT>::SMEM); };
+    if (dev >= 0 && dev < 16) std::call_once(once[dev], set);
+    else set();
+    DFL_CUDA(e);
+    const int n_items = p.row_tiles * p.splits * p.tok_tiles;
+    DFL_CUDA(launch_k(gemm_tm_kernel<DT>, dim3((unsigned)(n_items < sm_count() ? n_items : sm_count())), dim3(TM_THREADS), (size_t)TmFmt<DT>::SMEM, st, p));
+    count_launch();
+    return DFL_OK;
+}
+
+}  // namespace ts
+
+// Split count of a many-row launch: waves of items times blocks per item (an item pays about a third of a block to start
+// and to end), plus the traffic of the partial slices (64 KiB per item written and read again, in units of a block's time).
+int gemm_tm_choose_splits(const int* row_tiles, int n_mats, int kblocks, int tok_tiles) {
+    int best = 1;
+    double best_cost = 1e30;
+    for (int s = 1; s <= 8 && s <= kblocks; ++s) {
+        double cost = 0.0;
+        for (int i = 0; i < n_mats; ++i) {
+            const int items = row_tiles[i] * tok_tiles * s;
+            const int rounds = (items + sm_count() - 1) / sm_count();
+            cost += rounds * ((double)((kblocks + s - 1) / s) + 0.35) + 0.02 * items;
+        }
+        if (cost < best_cost) { best_cost = cost; best = s; }
+    }
+    return best;
+}
+
+bool gemm_tm_supported(const QMatrix& m) {
+    return m.layout == LAYOUT_TS && (m.dtype == DFL_Q4_K || m.dtype == DFL_Q5_K || m.dtype == DFL_Q6_K);
+}
+
+dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_rows, int rows_pad,
+                          const float* sumsq, int n_sumsq, float norm_k, float eps, float out_scale, uint32_t ld_out, int* dev_err) {
+    if (!gemm_tm_supported(m)) return fail(DFL_ERR_UNSUPPORTED, "many-row gemm: weight dtype");
+    if (splits < 1 || splits > m.kblocks || n_rows < 1 || rows_pad % TM_TOK || n_rows > rows_pad) return fail(DFL_ERR_BAD_ARG, "many-row gemm: shape");
+    ts::TmParams p;
+    p.w = m.tiles; p.acts = acts; p.out = out; p.sumsq = sumsq; p.n_sumsq = n_sumsq; p.norm_k = norm_k; p.eps = eps; p.out_scale = out_scale;
+    p.kblocks = m.kblocks; p.splits = splits; p.row_tiles = m.row_tiles; p.tok_tiles = (n_rows + TM_TOK - 1) / TM_TOK;
+    p.n_rows = n_rows; p.rows_pad = rows_pad; p.n_out = (uint32_t)m.n_out; p.ld_out = ld_out ? ld_out : (uint32_t)m.n_out; p.err = dev_err;
+    switch (m.dtype) {
+        case DFL_Q4_K: return ts::launch_tm<DFL_Q4_K>(st, p);
+        case DFL_Q5_K: return ts::launch_tm<DFL_Q5_K>(st, p);
+        default: return ts::launch_tm<DFL_Q6_K>(st, p);
+    }
+}
+
+}  // namespace dfl

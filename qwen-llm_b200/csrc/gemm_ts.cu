@@ -344,3 +344,4 @@ struct Fmt<DFL_Q5_K> : FmtK45<DFL_Q5_K> {};
 #include "gemm_ts_q80.cuh"
 #include "gemm_tsb.cuh"
 #include "gemm_ts_kernel.cuh"
+#include "gemm_tm.cuh"

@@ -32,6 +32,15 @@ constexpr int TS_BMIN_OFF = TS_B_BYTES;
 constexpr int TS_BMIN_BYTES = 1536;  // [k-core 2][n-group 6][8][16 B]
 static_assert(ACTTS_CHUNK == TS_B_BYTES + TS_BMIN_BYTES, "activation chunk size");
 
+// Many-row kernel (gemm_tm.cuh), activation chunk per (128 tokens, 256 columns): four stages of 64 columns, each
+// [plane hi / lo][k-core 8][token 128][8 halfs] (K-major operand, k-cores 2048 bytes apart), columns in the order of
+// ts_act_kpos; then the 32-column sub-block sums as [plane hi / lo][k-core 2][token 128][8 halfs], both k-cores alike
+// (the A operand holds the hi part of the mins in its first eight columns and the lo part in the other eight).
+constexpr int TM_TOK = 128;
+constexpr int TM_BSTAGE = 2 * 64 * TM_TOK * 2;
+constexpr int TM_SUMS = 2 * 16 * TM_TOK * 2;
+constexpr int TM_CHUNK = 4 * TM_BSTAGE + TM_SUMS;
+
 constexpr int TSQ4_OFF_QS = 2048;
 constexpr int TSQ5_OFF_QH = 2048 + 16384;
 constexpr int TSQ6_OFF_D = 2048;
@@ -105,6 +114,11 @@ dfl_status launch_prep_acts_ts(cudaStream_t st, const float* x, int ld, int n_ro
                                int* dev_err);
 dfl_status launch_gemm_ts(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, const GemmEpilogue& ep,
                           int* dev_err, bool pdl, uint32_t ld_out);
+bool gemm_tm_supported(const QMatrix& m);
+int gemm_tm_choose_splits(const int* row_tiles, int n_mats, int kblocks, int tok_tiles);
+// out [splits][rows_pad][ld_out] (rows beyond n_rows are not written); rows_pad a multiple of 128
+dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_rows, int rows_pad,
+                          const float* sumsq, int n_sumsq, float norm_k, float eps, float out_scale, uint32_t ld_out, int* dev_err);
 int gemm_ts_choose_splits(const QMatrix& m);
 int gemm_ts_choose_splits_multi(const int* row_tiles, int n_mats, int kblocks);
 int gemm_ts_ctas_per_split(int row_tiles, int splits);

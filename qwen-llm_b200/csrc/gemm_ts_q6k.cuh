@@ -112,5 +112,33 @@ struct Fmt<DFL_Q6_K> {
     }
 };
 
+// For the many-row kernel: quarter h (64 columns) as A1 = fl16(q * sc) in r[0..15] and A2 = q * sc - A1 (in {-1, 0, 1}, the
+// one bit a product above 2048 does not fit) in r[16..31]; thread (row, kp2) owns block 2 h + kp2.
+__device__ __forceinline__ void tm_unpack_q6k(const uint8_t* st, int h, int row, int kp2, uint32_t (&r)[32], UnitScales& us) {
+    const int b = 2 * h + kp2;
+    const uint4* q = reinterpret_cast<const uint4*>(st + TSQ6_OFF_QS);
+    const uint4 qa = q[(b * 2 + 0) * 128 + row], qb = q[(b * 2 + 1) * 128 + row];
+    us.d = __half2float(__ushort_as_half(reinterpret_cast<const uint16_t*>(st + TSQ6_OFF_D)[row]));
+    us.dmin = 0.f;
+    const uint32_t sc2 = reinterpret_cast<const uint16_t*>(st)[row * 8 + b];
+    uint32_t s[2];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+        const __half2 e2 = __half2half2(__int2half_rn((int)(int8_t)((sc2 >> (8 * g)) & 0xffu)));
+        s[g] = *reinterpret_cast<const uint32_t*>(&e2);
+    }
+    const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+    for (int wi = 0; wi < 8; ++wi) {
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const uint32_t qq = h2sub(__byte_perm(w[wi], 0x64646464u, p ? 0x4342 : 0x4140), H2_1056);
+            const uint32_t a1 = h2mul(qq, s[wi >> 2]);
+            r[2 * wi + p] = a1;
+            r[16 + 2 * wi + p] = h2fma(qq, s[wi >> 2], a1 ^ 0x80008000u);
+        }
+    }
+}
+
 }  // namespace ts
 }  // namespace dfl

@@ -14,6 +14,7 @@ dfl_status draft_core(dfl_dsession* ds, int32_t carry, uint32_t noise_start, boo
 dfl_status draft_block_topk(dfl_dsession* ds, int32_t carry, uint32_t noise_start_pos, int32_t* out_tokens);
 dfl_status restore_partial_launch(const dfl_model* m, dfl_session* s, dfl_scratch* sc, uint32_t n_keep, uint32_t start_position);
 void dsession_set_after_enqueue(dfl_dsession* ds, void (*fn)(void*), void* arg);
+dfl_status dsession_append_dev(dfl_dsession* ds, const float* rows, cudaMemcpyKind kind, const uint32_t* positions, uint32_t count);
 }
 // accessors implemented next to the drafter session (drafter.cu)
 extern "C" {
@@ -55,18 +56,33 @@ dfl_status dfl_prefill(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
         if (ids[i] < 0 || (uint32_t)ids[i] >= m->arch.vocab_size) return fail(DFL_ERR_BAD_TOKEN, "prefill: token id out of range");
     const uint64_t KH = (uint64_t)sc->k_layers * m->arch.hidden_size;
     const uint32_t bs = sc->block_size;
-    for (uint64_t off = 0; off < n; off += bs) {
-        const uint32_t nb = (uint32_t)std::min<uint64_t>(bs, n - off);
-        const bool last = off + nb == n;
-        dfl_status st = verify_core(m, s, sc, layer_ids, n_layer_ids, ids + off, nb, start_position + (uint32_t)off, last && last_logits_host != nullptr);
+    const bool many = prompt_supported(m);
+    std::vector<uint32_t> positions;
+    for (uint64_t off = 0; off < n;) {
+        // More rows than a packed block: one many-row pass over up to PROMPT_ROWS of them.  A remainder that fits a packed block
+        // takes the packed path, which is then the cheaper one (a many-row pass pays for whole tiles of 128 rows).
+        const bool big = many && n - off > MAX_ROWS;
+        const uint32_t nb = (uint32_t)std::min<uint64_t>(big ? PROMPT_ROWS : bs, n - off);
+        const bool last = off + nb == n, head = last && last_logits_host != nullptr;
+        const uint32_t start = start_position + (uint32_t)off, last_rows = nb % bs ? nb % bs : bs;
+        dfl_status st = big ? prompt_core(m, s, sc, layer_ids, n_layer_ids, ids + off, nb, start, last_rows, head)
+                            : verify_core(m, s, sc, layer_ids, n_layer_ids, ids + off, nb, start, head);
         if (st != DFL_OK) { s->poisoned = true; return st; }
+        const float* capture = big ? prompt_capture(sc) : sc->capture;
         if (hidden_host && n_layer_ids)
-            cudaMemcpyAsync(hidden_host + off * KH, sc->capture, (size_t)nb * KH * 4, cudaMemcpyDeviceToHost, s->st);
-        if (last && last_logits_host)
-            cudaMemcpyAsync(last_logits_host, sc->logits + (uint64_t)(nb - 1) * m->arch.vocab_size, (size_t)m->arch.vocab_size * 4,
+            cudaMemcpyAsync(hidden_host + off * KH, capture, (size_t)nb * KH * 4, cudaMemcpyDeviceToHost, s->st);
+        if (head)
+            cudaMemcpyAsync(last_logits_host, sc->logits + (uint64_t)(big ? 0 : nb - 1) * m->arch.vocab_size, (size_t)m->arch.vocab_size * 4,
                             cudaMemcpyDeviceToHost, s->st);
         DFL_CHECK(session_drain(s));
-        if (feed_drafter) DFL_CHECK(dfl_dsession_append_from_scratch(feed_drafter, sc, 0, nb, start_position + (uint32_t)off));
+        if (feed_drafter) {
+            if (dsession_target(feed_drafter) != m) return fail(DFL_ERR_BAD_ARG, "append_from_scratch: scratch belongs to another model");
+            positions.resize(nb);
+            for (uint32_t i = 0; i < nb; ++i) positions[i] = start + i;
+            if (big) DFL_CHECK(dsession_append_dev(feed_drafter, capture, cudaMemcpyDeviceToDevice, positions.data(), nb));
+            else DFL_CHECK(dfl_dsession_append_from_scratch(feed_drafter, sc, 0, nb, start));
+        }
+        off += nb;
     }
     dfl_status st = check_dev_err(s->st, s->err);
     if (st != DFL_OK) s->poisoned = true;

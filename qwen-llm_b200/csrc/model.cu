@@ -175,6 +175,22 @@ static dfl_status completion_check(dfl_session* s) {
     return st;
 }
 
+// lm_head over the n normalised rows in sc->acts_h: logits, argmax and gap of every row.
+dfl_status head_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, uint32_t n, const GemmEpilogue& ep_norm) {
+    cudaStream_t st = s->st;
+    const uint64_t V = m->arch.vocab_size;
+    const MatGroup& lm = m->lm_head;
+    float* logits = sc->logits;
+    if (lm.splits == 1) {
+        DFL_CHECK(launch_group(st, lm, sc->acts_h, logits, ep_norm, s->err));
+        DFL_CHECK(launch_argmax_top2(st, logits, (int)n, V, V, sc->argmax, sc->gap, sc->am_scratch));
+    } else {
+        DFL_CHECK(launch_group(st, lm, sc->acts_h, sc->part, ep_norm, s->err));
+        DFL_CHECK(launch_reduce_argmax_top2(st, sc->part, lm.splits, (int)n, V, logits, V, sc->argmax, sc->gap, sc->am_scratch));
+    }
+    return DFL_OK;
+}
+
 dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids,
                        const int32_t* tokens, uint32_t n, uint32_t start, bool want_head) {
     const dfl_arch& a = m->arch;
@@ -395,18 +411,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             }
         }
     }
-    if (want_head) {
-        const uint64_t V = a.vocab_size;
-        const MatGroup& lm = m->lm_head;
-        float* logits = sc->logits;
-        if (lm.splits == 1) {
-            DFL_CHECK(launch_group(st, lm, sc->acts_h, logits, ep_norm, s->err));
-            DFL_CHECK(launch_argmax_top2(st, logits, (int)n, V, V, sc->argmax, sc->gap, sc->am_scratch));
-        } else {
-            DFL_CHECK(launch_group(st, lm, sc->acts_h, sc->part, ep_norm, s->err));
-            DFL_CHECK(launch_reduce_argmax_top2(st, sc->part, lm.splits, (int)n, V, logits, V, sc->argmax, sc->gap, sc->am_scratch));
-        }
-    }
+    if (want_head) DFL_CHECK(head_core(m, s, sc, n, ep_norm));
     DFL_CHECK(join_side());   // whatever the side streams still hold belongs to this pass
     DFL_CHECK(join_side2());
     s->kv_n_pos = start + n;
@@ -889,6 +894,7 @@ void dfl_scratch_destroy(dfl_scratch* sc) {
     if (sc->pinned_order) cudaFreeHost(sc->pinned_order);
     if (sc->order_dev) cudaFree(sc->order_dev);
     if (sc->sort_scratch) cudaFree(sc->sort_scratch);
+    prompt_ws_free(sc->prompt);
     delete sc;
 }
 

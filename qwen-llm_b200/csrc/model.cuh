@@ -72,6 +72,7 @@ struct LayerW {
 struct dfl_session;
 
 namespace dfl {
+struct PromptWs;
 // expert parallelism (ep_nccl.cpp)
 dfl_status ep_unique_id(uint8_t* id_out);
 dfl_status ep_comm_create(int rank, int world, const uint8_t* id_bytes, void** comm_out);
@@ -195,9 +196,20 @@ struct dfl_scratch {
     bool have_block = false;
     uint64_t part_floats = 0;
     std::vector<void*> allocs;
+    dfl::PromptWs* prompt = nullptr;   // buffers of the many-row prompt pass, made by the first prompt that needs them
 };
 
 namespace dfl {
+// many-row prompt pass (prompt.cu): whether the model's matrices have the kernels for it, the most rows of one pass, and one
+// pass of n rows at positions start ..; leaves the captured rows in the workspace (prompt_capture) and the scratch and the session
+// as a packed pass over the last `last_rows` rows would
+bool prompt_supported(const dfl_model* m);
+constexpr uint32_t PROMPT_ROWS = 512;
+dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids, const int32_t* tokens,
+                       uint32_t n, uint32_t start, uint32_t last_rows, bool want_head);
+const float* prompt_capture(const dfl_scratch* sc);
+void prompt_ws_free(PromptWs* w);
+dfl_status head_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, uint32_t n, const GemmEpilogue& ep_norm);
 // One packed forward of n <= 16 tokens at positions start..start+n-1 (the body shared by
 // dfl_packed_verify, dfl_single_token and dfl_prefill).  Leaves argmax/gap/logits/capture on the device.
 dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids,

@@ -236,7 +236,7 @@ __host__ __device__ inline uint32_t kv_tile_v_off(uint32_t key, int d) { return 
 dfl_status launch_attn_front(cudaStream_t st, const AttnGeom& g, bool gated, const float* part, int splits, int ld_part,
                              const float* q_norm_w, const float* k_norm_w, uint32_t start, int n_rows, void* k_cache,
                              void* v_cache, int kv_mode, float* q_rot, float* gate, const uint32_t* pos_override,
-                             long long cache_row0 = -1);
+                             long long cache_row0 = -1, int part_rows = MAX_ROWS);   // part_rows: rows of one partial slice
 // Causal attention of the n_rows query rows over cache positions [0, start + row]; partials per
 // 64-position chunk, then combine, sigmoid gate and activation packing for the o-projection.
 dfl_status launch_attn_verify(cudaStream_t st, const AttnGeom& g, const float* q_rot, const float* gate, const void* k_cache,
@@ -374,6 +374,45 @@ __device__ __forceinline__ void gdn_front_tile(const GdnFrontParams& p, int head
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         if (i0 + j < p.n_rows) *reinterpret_cast<float4*>(dst + (uint64_t)(i0 + j) * dst_ld) = make_float4(y[j][0], y[j][1], y[j][2], y[j][3]);
+}
+// One token of the recurrence for one state row shared by eight lanes: lane group member lg owns the sixteen columns
+// dk = 32 j + 4 lg + c (j, c < 4), so that the eight lanes of a row read 128 contiguous bytes of k and q per step.
+// The two row sums go through three shuffle levels each.
+__device__ __forceinline__ float gdn_token_step(float (&S)[16], const float* k_row, const float* q_row, float v, float gexp, float beta, int lg) {
+    float kk[16], qq[16];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 k4 = *reinterpret_cast<const float4*>(k_row + 32 * j + 4 * lg);
+        const float4 q4 = *reinterpret_cast<const float4*>(q_row + 32 * j + 4 * lg);
+        kk[4 * j] = k4.x; kk[4 * j + 1] = k4.y; kk[4 * j + 2] = k4.z; kk[4 * j + 3] = k4.w;
+        qq[4 * j] = q4.x; qq[4 * j + 1] = q4.y; qq[4 * j + 2] = q4.z; qq[4 * j + 3] = q4.w;
+    }
+    float p[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        p[j] = S[4 * j] * kk[4 * j];
+#pragma unroll
+        for (int c = 1; c < 4; ++c) p[j] = fmaf(S[4 * j + c], kk[4 * j + c], p[j]);
+    }
+    float sk = (p[0] + p[1]) + (p[2] + p[3]);
+#pragma unroll
+    for (int of = 4; of > 0; of >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, of);
+    const float coeff = beta * (v - gexp * sk);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int e = 4 * j + c;
+            S[e] = __fadd_rn(__fmul_rn(gexp, S[e]), __fmul_rn(coeff, kk[e]));
+        }
+        p[j] = S[4 * j] * qq[4 * j];
+#pragma unroll
+        for (int c = 1; c < 4; ++c) p[j] = fmaf(S[4 * j + c], qq[4 * j + c], p[j]);
+    }
+    float o = (p[0] + p[1]) + (p[2] + p[3]);
+#pragma unroll
+    for (int of = 4; of > 0; of >>= 1) o += __shfl_xor_sync(0xffffffffu, o, of);
+    return o;
 }
 #endif
 // conv1d + SiLU over the block, q/k L2 norm; keeps raw qkv rows for rollback; updates conv state in place.

@@ -1,0 +1,241 @@
+// Many-row pass of a prompt (reference: prefill_tokens_with_multi_hidden, crates/qwen-llm/src/metal_dflash.rs:10779): up to
+// PROMPT_ROWS tokens through every layer at once, each weight tile unpacked once per 128 tokens instead of once per 16.
+// The layer structure, the arithmetic class (integer weights, f16 hi + lo activations, f32 sums) and the session and scratch
+// state it leaves behind are those of the packed pass (model.cu: verify_core).
+#include <cstring>
+
+#include "prompt.cuh"
+
+namespace dfl {
+
+struct PromptWs {
+    uint32_t rows = 0;   // padded rows the buffers hold
+    float *x = nullptr, *xn = nullptr, *part = nullptr, *sumsq = nullptr, *q_rot = nullptr, *gate = nullptr, *o = nullptr;
+    float *q_n = nullptr, *k_n = nullptr, *v = nullptr, *ab = nullptr, *conv_new = nullptr, *capture = nullptr;
+    uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_v = nullptr;
+    int32_t* tokens = nullptr;
+    int32_t* pinned = nullptr;
+    std::vector<void*> allocs;
+};
+
+const float* prompt_capture(const dfl_scratch* sc) { return sc->prompt->capture; }
+
+void prompt_ws_free(PromptWs* w) {
+    if (!w) return;
+    for (void* p : w->allocs) cudaFree(p);
+    if (w->pinned) cudaFreeHost(w->pinned);
+    delete w;
+}
+
+static bool group_supported(const MatGroup& g) {
+    for (auto& m : g.mats)
+        if (!gemm_tm_supported(m)) return false;
+    return true;
+}
+
+bool prompt_supported(const dfl_model* m) {
+    if (m->act_layout != ACT_TS || m->arch.expert_count > 0 || m->ep_world > 1) return false;
+    // DFL_PROMPT_ROWS=0 keeps prompts on the packed path
+    static const bool enabled = [] { const char* e = getenv("DFL_PROMPT_ROWS"); return !(e && e[0] == '0'); }();
+    if (!enabled) return false;
+    for (auto& L : m->layers)
+        if (!(L.is_attn ? group_supported(L.qkv) && group_supported(L.wo) : group_supported(L.in_qkv_z) && group_supported(L.w_out)) ||
+            !group_supported(L.gate_up) || !group_supported(L.down))
+            return false;
+    return true;
+}
+
+static int tm_splits(const MatGroup& g, int tok_tiles) {
+    int tiles[8];
+    int n = 0;
+    for (auto& m : g.mats)
+        if (n < 8) tiles[n++] = m.row_tiles;
+    return gemm_tm_choose_splits(tiles, n, (int)(g.n_in / TILE_K), tok_tiles);
+}
+
+static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) {
+    if (sc->prompt && sc->prompt->rows >= rows) return DFL_OK;
+    prompt_ws_free(sc->prompt);
+    sc->prompt = nullptr;
+    auto* w = new PromptWs();
+    const dfl_arch& a = m->arch;
+    const GdnGeom gg = m->gdn_geom();
+    const uint64_t H = a.hidden_size, F = a.intermediate_size, R = rows;
+    const uint64_t q_dim = (uint64_t)a.n_q_heads * a.attn_head_dim, v_dim = (uint64_t)gg.n_v * 128, wide = std::max(q_dim, v_dim);
+    uint64_t part = 0;
+    for (int t = 1; t <= (int)(rows / TM_TOK); ++t)
+        for (auto& L : m->layers)
+            for (const MatGroup* g : {&L.qkv, &L.wo, &L.in_qkv_z, &L.w_out, &L.gate_up, &L.down})
+                if (!g->mats.empty()) part = std::max<uint64_t>(part, (uint64_t)tm_splits(*g, t) * t * TM_TOK * g->total_cols);
+    bool ok = true;
+    auto alloc = [&](auto** p, uint64_t bytes) {
+        void* q = nullptr;
+        ok = ok && cudaMalloc(&q, bytes ? bytes : 16) == cudaSuccess;
+        if (q) w->allocs.push_back(q);
+        *p = reinterpret_cast<std::remove_reference_t<decltype(**p)>*>(q);
+    };
+    const uint64_t tiles = rows / TM_TOK;
+    alloc(&w->x, R * H * 4);
+    alloc(&w->xn, R * H * 4);
+    alloc(&w->part, part * 4);
+    alloc(&w->sumsq, H / TILE_K * R * 4);
+    alloc(&w->q_rot, R * q_dim * 4);
+    alloc(&w->gate, R * q_dim * 4);
+    alloc(&w->o, R * wide * 4);
+    alloc(&w->q_n, R * gg.n_k * 128 * 4);
+    alloc(&w->k_n, R * gg.n_k * 128 * 4);
+    alloc(&w->v, R * v_dim * 4);
+    alloc(&w->ab, R * 2 * gg.n_v * 4);
+    alloc(&w->conv_new, 3ull * gg.conv_dim() * 4);
+    alloc(&w->capture, R * sc->k_layers * H * 4);
+    alloc(&w->acts_h, tiles * (H / TILE_K) * TM_CHUNK);
+    alloc(&w->acts_f, tiles * (F / TILE_K) * TM_CHUNK);
+    alloc(&w->acts_v, tiles * (wide / TILE_K) * TM_CHUNK);
+    alloc(&w->tokens, R * 4);
+    ok = ok && cudaMallocHost(&w->pinned, R * 4) == cudaSuccess;
+    if (!ok) {
+        std::string why = cudaGetErrorString(cudaGetLastError());
+        prompt_ws_free(w);
+        return fail(DFL_ERR_OOM, "prompt pass: allocation failed: " + why);
+    }
+    w->rows = rows;
+    sc->prompt = w;
+    return DFL_OK;
+}
+
+dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids, const int32_t* tokens,
+                       uint32_t n, uint32_t start, uint32_t last_rows, bool want_head) {
+    const dfl_arch& a = m->arch;
+    const int rows_pad = (int)((n + TM_TOK - 1) / TM_TOK * TM_TOK), tok_tiles = rows_pad / TM_TOK;
+    DFL_CHECK(ensure_ws(m, sc, (uint32_t)rows_pad));
+    PromptWs* w = sc->prompt;
+    cudaStream_t st = s->st;
+    const uint64_t H = a.hidden_size, F = a.intermediate_size, KH = sc->k_layers * H;
+    const AttnGeom ag = m->attn_geom();
+    const GdnGeom gg = m->gdn_geom();
+    const uint64_t q_dim = (uint64_t)ag.n_q * ag.hd;
+    const int n_sumsq = (int)(H / TILE_K);
+
+    memcpy(w->pinned, tokens, n * sizeof(int32_t));
+    DFL_CUDA(cudaMemcpyAsync(w->tokens, w->pinned, n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+    DFL_CHECK(launch_embed_rows(st, m->embd_dtype, m->embd_ggml, H, w->tokens, (int)n, w->x, (int)H));
+
+    auto glue_base = [&] {
+        TmGlue p;
+        p.n_rows = (int)n; p.rows_pad = rows_pad; p.err = s->err;
+        return p;
+    };
+    auto norm_glue = [&](int splits, const float* norm_w, bool want_xn, float* capture) -> dfl_status {
+        TmGlue p = glue_base();
+        if (splits) { p.part = w->part; p.splits = splits; p.ld_part = (int)H; }
+        p.x = w->x; p.ld_x = (int)H;
+        p.mul_w = norm_w;
+        p.acts = norm_w ? w->acts_h : nullptr;
+        if (want_xn) { p.xn = w->xn; p.ld_xn = (int)H; }
+        p.sumsq = norm_w ? w->sumsq : nullptr;
+        p.capture = capture; p.ld_capture = (int)KH;
+        return launch_tm_glue(st, p, H);
+    };
+    // one group of matrices over the same activations, side by side into w->part; returns the split count used
+    auto gemm = [&](const MatGroup& g, const uint8_t* acts, bool norm, float out_scale, int* splits) -> dfl_status {
+        *splits = tm_splits(g, tok_tiles);
+        for (size_t i = 0; i < g.mats.size(); ++i)
+            DFL_CHECK(launch_gemm_tm(st, g.mats[i], acts, w->part + g.col_off[i], *splits, (int)n, rows_pad, norm ? w->sumsq : nullptr,
+                                     norm ? n_sumsq : 0, (float)H, 1e-6f, out_scale, g.total_cols, s->err));
+        return DFL_OK;
+    };
+    DFL_CHECK(norm_glue(0, m->layers[0].attn_norm_w, !m->layers[0].is_attn, nullptr));
+
+    int gi = 0, ai = 0, splits = 1;
+    for (uint32_t il = 0; il < a.n_layer; ++il) {
+        const LayerW& L = m->layers[il];
+        const bool last = il + 1 == a.n_layer;
+        if (L.is_attn) {
+            DFL_CHECK(gemm(L.qkv, w->acts_h, true, 1.f, &splits));
+            DFL_CHECK(launch_attn_front(st, ag, true, w->part, splits, (int)L.qkv.total_cols, L.q_norm_w, L.k_norm_w, start, (int)n, s->k_cache[ai],
+                                        s->v_cache[ai], s->kv_mode, w->q_rot, w->gate, nullptr, -1, rows_pad));
+            for (uint32_t r = 0; r < n; r += MAX_ROWS)
+                DFL_CHECK(launch_attn_verify(st, ag, w->q_rot + r * q_dim, w->gate + r * q_dim, s->k_cache[ai], s->v_cache[ai], s->kv_mode, start + r,
+                                             (int)std::min<uint32_t>(MAX_ROWS, n - r), s->attn_partials, nullptr, m->act_layout, w->o + r * q_dim, s->err,
+                                             s->kv_capacity));
+            TmGlue p = glue_base();
+            p.mode = GLUE_COPY;
+            p.x = w->o; p.ld_x = (int)q_dim;
+            p.acts = w->acts_v;
+            DFL_CHECK(launch_tm_glue(st, p, q_dim));
+            DFL_CHECK(gemm(L.wo, w->acts_v, false, 1.f, &splits));
+            ++ai;
+        } else {
+            TmGdn p;
+            p.g = gg;
+            DFL_CHECK(gemm(L.in_qkv_z, w->acts_h, true, 1.f, &splits));
+            DFL_CHECK(launch_tm_small_matmul(st, L.w_ab, w->xn, (int)H, (int)n, rows_pad, H, 2 * gg.n_v, w->sumsq, n_sumsq, (float)H, 1e-6f, w->ab,
+                                             2 * gg.n_v));
+            const int cur = s->ssm_cur[gi];
+            p.part = w->part; p.splits = splits; p.ld_part = (int)L.in_qkv_z.total_cols; p.z_col = gg.conv_dim();
+            p.n_rows = (int)n; p.rows_pad = rows_pad; p.last_rows = (int)last_rows;
+            p.conv_w = L.conv_w; p.ab = w->ab; p.dt_bias = L.dt_bias; p.a_log = L.a_log; p.norm_w = L.ssm_norm_w;
+            p.conv_state = s->conv[gi]; p.conv_new = w->conv_new;
+            p.state_in = s->ssm[cur][gi]; p.state_out = s->ssm[cur ^ 1][gi];
+            p.q_n = w->q_n; p.k_n = w->k_n; p.v = w->v; p.o = w->o;
+            p.keep_raw = sc->qkv_raw[gi]; p.keep_pre = sc->conv_pre[gi]; p.keep_q = sc->q_n[gi]; p.keep_k = sc->k_n[gi]; p.keep_v = sc->v[gi];
+            p.keep_ab = sc->ab[gi];
+            p.acts = w->acts_v; p.err = s->err;
+            DFL_CHECK(launch_tm_gdn_front(st, p));
+            DFL_CHECK(launch_tm_gdn_scan(st, p));
+            DFL_CHECK(launch_tm_gdn_pack(st, p));
+            s->ssm_cur[gi] = cur ^ 1;
+            DFL_CHECK(gemm(L.w_out, w->acts_v, false, 1.f, &splits));
+            ++gi;
+        }
+        DFL_CHECK(norm_glue(splits, L.post_norm_w, false, nullptr));
+        DFL_CHECK(gemm(L.gate_up, w->acts_h, true, 1.f, &splits));
+        {
+            TmGlue p = glue_base();
+            p.mode = GLUE_SWIGLU;
+            p.part = w->part; p.splits = splits; p.ld_part = (int)L.gate_up.total_cols;
+            p.swiglu_f = (int)F;
+            p.pre_scale = 1.0f / 64.0f;   // as in the packed pass: keeps silu(g) * u inside the f16 operand range
+            p.acts = w->acts_f;
+            DFL_CHECK(launch_tm_glue(st, p, F));
+        }
+        DFL_CHECK(gemm(L.down, w->acts_f, false, 64.f, &splits));
+        float* cap = nullptr;
+        for (uint32_t k = 0; k < n_ids; ++k)
+            if (layer_ids[k] == il) { cap = w->capture + (uint64_t)k * H; break; }
+        DFL_CHECK(norm_glue(splits, last ? nullptr : m->layers[il + 1].attn_norm_w, !last && !m->layers[il + 1].is_attn, cap));
+        bool first = true;
+        for (uint32_t k = 0; k < n_ids && cap; ++k) {   // a layer listed twice: its other slots get a copy
+            if (layer_ids[k] != il) continue;
+            if (first) { first = false; continue; }
+            DFL_CUDA(cudaMemcpy2DAsync(w->capture + (uint64_t)k * H, KH * 4, cap, KH * 4, H * 4, n, cudaMemcpyDeviceToDevice, st));
+        }
+    }
+    if (want_head) {   // the last row alone, through the packed path's head
+        GlueParams p;
+        p.mode = GLUE_COPY;
+        p.x = w->x + (uint64_t)(n - 1) * H; p.ld_x = (int)H;
+        p.mul_w = m->out_norm_w;
+        p.acts = sc->acts_h; p.bf3 = m->act_layout;
+        p.sumsq = sc->sumsq;
+        p.n_rows = 1; p.err = s->err;
+        DFL_CHECK(launch_glue(st, p, H));
+        GemmEpilogue ep;
+        ep.sumsq = sc->sumsq;
+        ep.n_sumsq = (int)(H / GLUE_COLS);
+        ep.norm_k = (float)H;
+        ep.eps = 1e-6f;
+        DFL_CHECK(head_core(m, s, sc, 1, ep));
+    }
+    // the last block's captured rows where a packed pass would have left them
+    if (n_ids)
+        DFL_CUDA(cudaMemcpyAsync(sc->capture, w->capture + (uint64_t)(n - last_rows) * KH, (size_t)last_rows * KH * 4, cudaMemcpyDeviceToDevice, st));
+    s->kv_n_pos = start + n;
+    sc->last_n = last_rows;
+    sc->last_n_verify = last_rows;
+    sc->last_start = start + n - last_rows;
+    sc->have_block = true;
+    return DFL_OK;
+}
+
+}  // namespace dfl

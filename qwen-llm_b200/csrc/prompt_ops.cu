@@ -1,0 +1,413 @@
+// Element-wise, convolution and recurrence kernels of the many-row prompt pass (see prompt.cuh).
+#include "prompt.cuh"
+
+namespace dfl {
+
+// Eight consecutive columns k8 .. k8 + 7 (k8 % 8 == 0, inside one 256-column block) of token t of a 128-token tile -> the
+// hi / lo planes of the activation chunk: one 16-byte store each, eight tokens fill 128 contiguous bytes.
+__device__ __forceinline__ void pack_oct_tm(uint8_t* chunk, int t, int k8, const float (&v)[8], bool& overflow) {
+    uint16_t hi[8], lo[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        overflow |= (fabsf(v[e]) >= 65504.f) && (fabsf(v[e]) < INFINITY);
+        const __half h = __float2half_rn(v[e]);
+        hi[e] = __half_as_ushort(h);
+        lo[e] = __half_as_ushort(__float2half_rn(v[e] - __half2float(h)));
+    }
+    // k-positions of a quad: 0, 2, 1, 3 (ts_act_kpos)
+    auto quad = [](const uint16_t* h) { return make_uint2((uint32_t)h[0] | ((uint32_t)h[2] << 16), (uint32_t)h[1] | ((uint32_t)h[3] << 16)); };
+    uint8_t* dst = chunk + (k8 >> 6) * TM_BSTAGE + ((k8 >> 3) & 7) * (TM_TOK * 16) + t * 16;
+    const uint2 h0 = quad(hi), h1 = quad(hi + 4), l0 = quad(lo), l1 = quad(lo + 4);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(h0.x, h0.y, h1.x, h1.y);
+    *reinterpret_cast<uint4*>(dst + TM_BSTAGE / 2) = make_uint4(l0.x, l0.y, l1.x, l1.y);
+}
+// Sum of token t's activations over 32-column sub-block j -> hi / lo planes, both k-cores.
+__device__ __forceinline__ void pack_sum_tm(uint8_t* chunk, int t, int j, float sum, bool& overflow) {
+    overflow |= (fabsf(sum) >= 65504.f) && (fabsf(sum) < INFINITY);
+    const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
+    uint8_t* dst = chunk + 4 * TM_BSTAGE + t * 16 + j * 2;
+    *reinterpret_cast<__half*>(dst) = h;
+    *reinterpret_cast<__half*>(dst + TM_TOK * 16) = h;
+    *reinterpret_cast<__half*>(dst + TM_SUMS / 2) = l;
+    *reinterpret_cast<__half*>(dst + TM_SUMS / 2 + TM_TOK * 16) = l;
+}
+
+// Threads of the packing kernels: CTA = 8 tokens x one 256-column block; lane = (token lane & 7, core lane >> 3), a warp covers
+// the 32 columns of one sub-block, so reads are 128-byte runs of a token's row and stores 128-byte runs of a k-core.
+__global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
+    pdl_prologue();
+    __shared__ float ss_s[8][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tk = lane & 7, k8 = warp * 32 + (lane >> 3) * 8;
+    const int row = blockIdx.y * 8 + tk, col = blockIdx.x * 256 + k8;
+    const bool live = row < p.n_rows;
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = 0.f;
+    auto add8 = [](float (&a)[8], const float* src) {
+        const float4 x = __ldcg(reinterpret_cast<const float4*>(src)), y = __ldcg(reinterpret_cast<const float4*>(src) + 1);
+        a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+        a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
+    };
+    auto store8 = [](float* dst, const float (&a)[8]) {
+        reinterpret_cast<float4*>(dst)[0] = make_float4(a[0], a[1], a[2], a[3]);
+        reinterpret_cast<float4*>(dst)[1] = make_float4(a[4], a[5], a[6], a[7]);
+    };
+    if (live) {
+        const uint64_t stride = (uint64_t)p.rows_pad * p.ld_part;
+        const float* base = p.part ? p.part + (uint64_t)row * p.ld_part + col : nullptr;
+        if (p.mode == GLUE_SWIGLU) {
+            float g[8] = {}, u[8] = {};
+            for (int s = 0; s < p.splits; ++s) {
+                add8(g, base + s * stride);
+                add8(u, base + s * stride + p.swiglu_f);
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = silu_f(g[e]) * u[e];
+        } else {
+            if (base)
+                for (int s = 0; s < p.splits; ++s) add8(v, base + s * stride);
+            if (p.x) {
+                float xv[8] = {};
+                add8(xv, p.x + (uint64_t)row * p.ld_x + col);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = xv[e] + v[e];
+                if (base) store8(p.x + (uint64_t)row * p.ld_x + col, v);
+            }
+            if (p.gate) {
+                float gv[8] = {};
+                add8(gv, p.gate + (uint64_t)row * p.ld_x + col);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] *= sigmoid_f(gv[e]);
+            }
+        }
+        if (p.capture) store8(p.capture + (uint64_t)row * p.ld_capture + col, v);
+    }
+    if (p.sumsq) {
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 8);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+        if (lane < 8) ss_s[warp][lane] = ss;
+        __syncthreads();
+        if (threadIdx.x < 8) {
+            float t = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) t += ss_s[w][threadIdx.x];
+            p.sumsq[(uint64_t)blockIdx.x * p.rows_pad + blockIdx.y * 8 + threadIdx.x] = t;
+        }
+    }
+    if (p.mul_w) {
+        float w[8] = {};
+        add8(w, p.mul_w + col);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] *= w[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] *= p.pre_scale;
+    if (p.xn && live) store8(p.xn + (uint64_t)row * p.ld_xn + col, v);
+    if (p.acts) {
+        uint8_t* chunk = p.acts + ((uint64_t)(row / TM_TOK) * gridDim.x + blockIdx.x) * TM_CHUNK;
+        bool over = false;
+        pack_oct_tm(chunk, row % TM_TOK, k8, v, over);
+        float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        if (lane < 8) pack_sum_tm(chunk, row % TM_TOK, warp, sum, over);
+        if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
+    }
+}
+
+dfl_status launch_tm_glue(cudaStream_t st, const TmGlue& p, uint64_t k) {
+    if (k == 0 || k % TILE_K || p.rows_pad % TM_TOK) return fail(DFL_ERR_BAD_SHAPE, "tm_glue: shape");
+    launch_k(tm_glue_kernel, dim3((unsigned)(k / TILE_K), (unsigned)(p.rows_pad / 8)), dim3(256), 0, st, p);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+// ---- small f32 projections ----------------------------------------------------------------------
+// CTA = 16 rows x 16 outputs x the whole k: 256 threads split k (thread = 16 column lanes x 16 (row, output) sub-tiles of 4 x 4),
+// so that the few outputs of alpha / beta still give rows / 16 * n_out / 16 CTAs.  k-slices of a sub-tile are added in lane order.
+__global__ void __launch_bounds__(256) tm_small_matmul_kernel(const float* __restrict__ w, const float* xn, int ld_xn, int n_rows, int rows_pad,
+                                                              int k, int n_out, const float* sumsq, int n_sumsq, float norm_k, float eps,
+                                                              float* out, int ld_out) {
+    pdl_prologue();
+    const int r0 = blockIdx.x * 16 + (threadIdx.x >> 6) * 4, o0 = blockIdx.y * 16 + ((threadIdx.x >> 4) & 3) * 4, kl = threadIdx.x & 15;
+    float acc[4][4] = {};
+    const float* xp[4];
+    const float* wp[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        xp[i] = xn + (uint64_t)min(r0 + i, n_rows - 1) * ld_xn + kl * 4;
+        wp[i] = w + (uint64_t)min(o0 + i, n_out - 1) * k + kl * 4;
+    }
+    for (int c = 0; c < k; c += 64) {
+        if (c + kl * 4 >= k) break;
+        float4 xv[4], wv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            xv[i] = *reinterpret_cast<const float4*>(xp[i] + c);
+            wv[i] = *reinterpret_cast<const float4*>(wp[i] + c);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(wv[j].w, xv[i].w, fmaf(wv[j].z, xv[i].z, fmaf(wv[j].y, xv[i].y, fmaf(wv[j].x, xv[i].x, acc[i][j]))));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], o);
+    // lane kl of the sub-tile finishes (row kl >> 2, output kl & 3)
+    float v = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (kl == 4 * i + j) v = acc[i][j];
+    const int row = r0 + (kl >> 2), col = o0 + (kl & 3);
+    if (row < n_rows && col < n_out) {
+        float ss = 0.f;
+        for (int q = 0; q < n_sumsq; ++q) ss += sumsq[(uint64_t)q * rows_pad + row];
+        out[(uint64_t)row * ld_out + col] = v * (1.0f / sqrtf(ss / norm_k + eps));
+    }
+}
+
+dfl_status launch_tm_small_matmul(cudaStream_t st, const float* w, const float* xn, int ld_xn, int n_rows, int rows_pad, uint64_t k, int n_out,
+                                  const float* sumsq, int n_sumsq, float norm_k, float eps, float* out, int ld_out) {
+    if (k % 4) return fail(DFL_ERR_BAD_SHAPE, "tm_small_matmul: k must be a multiple of 4");
+    launch_k(tm_small_matmul_kernel, dim3((unsigned)((n_rows + 15) / 16), (unsigned)((n_out + 15) / 16)), dim3(256), 0, st, w, xn, ld_xn, n_rows,
+             rows_pad, (int)k, n_out, sumsq, n_sumsq, norm_k, eps, out, ld_out);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+// ---- gated delta net: conv + SiLU + L2 norms over all rows of the pass ---------------------------
+// grid (heads of 128 channels, rows / 16), four warps of four rows each, lane = four channels: gdn_front_tile with the three
+// preceding rows read from the pass's own projection output (or the conv state for the first rows).  The new conv state
+// goes to conv_new, because the first row block reads the old one; the scan moves it over.
+__global__ void __launch_bounds__(128) tm_gdn_front_kernel(const TmGdn p) {
+    pdl_prologue();
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.x;
+    const int conv_dim = p.g.conv_dim(), i0 = blockIdx.y * 16 + 4 * w, c = head * 128 + 4 * lane;
+    if (i0 >= p.n_rows) return;
+    float4 xv[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        const int row = i0 - 3 + k;
+        xv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < 0) xv[k] = *reinterpret_cast<const float4*>(p.conv_state + (row + 3) * conv_dim + c);
+        else if (row < p.n_rows) {
+            for (int s = 0; s < p.splits; ++s) {
+                const float4 a = __ldcg(reinterpret_cast<const float4*>(p.part + ((uint64_t)s * p.rows_pad + row) * p.ld_part + c));
+                xv[k].x += a.x; xv[k].y += a.y; xv[k].z += a.z; xv[k].w += a.w;
+            }
+        }
+    }
+    float4 tap[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) tap[e] = *reinterpret_cast<const float4*>(p.conv_w + (uint64_t)(c + e) * 4);
+    float y[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float in[4][4] = {{xv[j].x, xv[j + 1].x, xv[j + 2].x, xv[j + 3].x}, {xv[j].y, xv[j + 1].y, xv[j + 2].y, xv[j + 3].y},
+                                {xv[j].z, xv[j + 1].z, xv[j + 2].z, xv[j + 3].z}, {xv[j].w, xv[j + 1].w, xv[j + 2].w, xv[j + 3].w}};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float s = 0.f;
+            s += tap[e].x * in[e][0];
+            s += tap[e].y * in[e][1];
+            s += tap[e].z * in[e][2];
+            s += tap[e].w * in[e][3];
+            y[j][e] = silu_f(s);
+        }
+    }
+    const bool is_v = head >= 2 * p.g.n_k, is_q = head < p.g.n_k;
+    if (!is_v) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float sq = warp_sum((y[j][0] * y[j][0] + y[j][1] * y[j][1]) + (y[j][2] * y[j][2] + y[j][3] * y[j][3]));
+            const float inv = 1.0f / fmaxf(sqrtf(sq), 1e-6f);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[j][e] *= inv;
+        }
+    }
+    const int h = is_v ? head - 2 * p.g.n_k : is_q ? head : head - p.g.n_k;
+    const int ld = (is_v ? p.g.n_v : p.g.n_k) * 128;
+    float* dst = (is_v ? p.v : is_q ? p.q_n : p.k_n) + h * 128 + 4 * lane;
+    float* keep = (is_v ? p.keep_v : is_q ? p.keep_q : p.keep_k) + h * 128 + 4 * lane;
+    const int keep0 = p.n_rows - p.last_rows;   // first row of the last block
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int row = i0 + j;
+        if (row >= p.n_rows) break;
+        const float4 o = make_float4(y[j][0], y[j][1], y[j][2], y[j][3]);
+        *reinterpret_cast<float4*>(dst + (uint64_t)row * ld) = o;
+        if (p.last_rows && row >= keep0) {
+            *reinterpret_cast<float4*>(keep + (uint64_t)(row - keep0) * ld) = o;
+            *reinterpret_cast<float4*>(p.keep_raw + (uint64_t)(row - keep0) * conv_dim + c) = xv[j + 3];
+        }
+    }
+    // row r of the sequence {state rows -3 .. -1, rows 0 ..} is xv[r - i0 + 3]; every row has one owner (rows below 0: the first warp)
+    auto mine = [&](int r) { return (r >= i0 && r < i0 + 4) || (r < 0 && i0 == 0); };
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        const int r = i0 - 3 + k;
+        if (!mine(r)) continue;
+        const int tn = r - (p.n_rows - 3), tp = r - (keep0 - 3);   // index in the new state / in the state before the last block
+        if (tn >= 0 && tn < 3) *reinterpret_cast<float4*>(p.conv_new + tn * conv_dim + c) = xv[k];
+        if (p.last_rows && tp >= 0 && tp < 3) *reinterpret_cast<float4*>(p.keep_pre + tp * conv_dim + c) = xv[k];
+    }
+}
+
+dfl_status launch_tm_gdn_front(cudaStream_t st, const TmGdn& p) {
+    launch_k(tm_gdn_front_kernel, dim3((unsigned)(p.g.conv_dim() / 128), (unsigned)((p.n_rows + 15) / 16)), dim3(128), 0, st, p);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+// ---- gated delta net: the recurrence -------------------------------------------------------------
+// grid (n_v, 4 quarters of the value channels), 256 threads: a warp owns four state rows, eight lanes a row, sixteen key
+// channels a lane, as in gdn_scan_kernel.  The sequential chain per token is bound by latency (two fused multiply-add trees
+// and three shuffle levels), so the next 16 tokens' q, k and v rows travel with cp.async while the current 16 are scanned.
+constexpr int SCAN_BLK = 16;
+__global__ void __launch_bounds__(256) tm_gdn_scan_kernel(const TmGdn p) {
+    __shared__ __align__(16) float qs[2][SCAN_BLK][128], ks[2][SCAN_BLK][128], vs[2][SCAN_BLK][32];
+    __shared__ float gs[2][SCAN_BLK], bs[2][SCAN_BLK];
+    const GdnGeom& g = p.g;
+    const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rr = lane >> 3, lg = lane & 7, hk = h % g.n_k;
+    const int dv_cta = blockIdx.y * 32, dv = dv_cta + warp * 4 + rr;
+    const float dtb = p.dt_bias[h], alog = p.a_log[h];
+    pdl_prologue();
+    float S[16];
+    const uint64_t s_off = ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 s4 = __ldcg(reinterpret_cast<const float4*>(p.state_in + s_off + 32 * j));
+        S[4 * j] = s4.x; S[4 * j + 1] = s4.y; S[4 * j + 2] = s4.z; S[4 * j + 3] = s4.w;
+    }
+    auto cp16 = [](void* dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); };
+    auto fetch = [&](int blk) {
+        const int buf = blk & 1, r0 = blk * SCAN_BLK, n = min(SCAN_BLK, p.n_rows - r0);
+        for (int i = threadIdx.x; i < n * 32; i += 256) {
+            const int r = i >> 5, d = (i & 31) * 4;
+            cp16(&qs[buf][r][d], p.q_n + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
+            cp16(&ks[buf][r][d], p.k_n + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
+        }
+        for (int i = threadIdx.x; i < n * 8; i += 256) {
+            const int r = i >> 3, d = (i & 7) * 4;
+            cp16(&vs[buf][r][d], p.v + ((uint64_t)(r0 + r) * g.n_v + h) * 128 + dv_cta + d);
+        }
+        if ((int)threadIdx.x < n) {
+            const float* a = p.ab + (uint64_t)(r0 + threadIdx.x) * (2 * g.n_v) + h;
+            const float alpha = __ldcg(a), beta = __ldcg(a + g.n_v);
+            gs[buf][threadIdx.x] = expf(softplus_f(alpha + dtb) * alog);
+            bs[buf][threadIdx.x] = sigmoid_f(beta);
+            const int kr = r0 + (int)threadIdx.x - (p.n_rows - p.last_rows);
+            if (p.last_rows && kr >= 0 && blockIdx.y == 0) {
+                p.keep_ab[(uint64_t)kr * (2 * g.n_v) + h] = alpha;
+                p.keep_ab[(uint64_t)kr * (2 * g.n_v) + g.n_v + h] = beta;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto put = [&](float* dst) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(dst + s_off + 32 * j) = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+    };
+    // the conv state the front kernel could not write in place; one slice per CTA
+    {
+        const int n = 3 * g.conv_dim() / 4, per = (n + gridDim.x * gridDim.y - 1) / (gridDim.x * gridDim.y);
+        const int c0 = (blockIdx.y * gridDim.x + blockIdx.x) * per;
+        for (int i = c0 + threadIdx.x; i < min(n, c0 + per); i += 256)
+            reinterpret_cast<float4*>(p.conv_state)[i] = __ldcg(reinterpret_cast<const float4*>(p.conv_new) + i);
+    }
+    const int n_blk = (p.n_rows + SCAN_BLK - 1) / SCAN_BLK;
+    const int ckpt = p.last_rows ? p.n_rows - p.last_rows : -1;
+    fetch(0);
+    for (int b = 0; b < n_blk; ++b) {
+        if (b + 1 < n_blk) {
+            fetch(b + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const int buf = b & 1, r0 = b * SCAN_BLK, n = min(SCAN_BLK, p.n_rows - r0);
+        float* o_row = p.o + (uint64_t)r0 * g.n_v * 128 + h * 128 + dv;
+#pragma unroll 2
+        for (int i = 0; i < n; ++i) {
+            if (r0 + i == ckpt) put(p.state_in);
+            const float o = gdn_token_step(S, ks[buf][i], qs[buf][i], vs[buf][i][warp * 4 + rr], gs[buf][i], bs[buf][i], lg);
+            if (lg == 0) o_row[(uint64_t)i * g.n_v * 128] = o;
+        }
+        __syncthreads();   // the buffer is refilled by the next iteration's fetch
+    }
+    put(p.state_out);
+}
+
+dfl_status launch_tm_gdn_scan(cudaStream_t st, const TmGdn& p) {
+    launch_k(tm_gdn_scan_kernel, dim3((unsigned)p.g.n_v, 4), dim3(256), 0, st, p);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+// ---- gated delta net: y = rmsnorm(o; eps * 128) * w * silu(z), packed ------------------------------
+// CTA = 8 tokens x two heads (256 channels), threads as in tm_glue_kernel
+__global__ void __launch_bounds__(256) tm_gdn_pack_kernel(const TmGdn p) {
+    pdl_prologue();
+    __shared__ float ss_s[8][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tk = lane & 7, k8 = warp * 32 + (lane >> 3) * 8;
+    const int row = blockIdx.y * 8 + tk, col = blockIdx.x * 256 + k8;
+    const bool live = row < p.n_rows;
+    float v[8] = {}, z[8] = {};
+    auto add8 = [](float (&a)[8], const float* src) {
+        const float4 x = __ldcg(reinterpret_cast<const float4*>(src)), y = __ldcg(reinterpret_cast<const float4*>(src) + 1);
+        a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+        a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
+    };
+    if (live) {
+        add8(v, p.o + (uint64_t)row * p.g.n_v * 128 + col);
+        for (int s = 0; s < p.splits; ++s) add8(z, p.part + ((uint64_t)s * p.rows_pad + row) * p.ld_part + p.z_col + col);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 8);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+    if (lane < 8) ss_s[warp][lane] = ss;
+    __syncthreads();
+    const int w0 = warp & 4;   // the four warps of this head
+    const float tot = ((ss_s[w0][tk] + ss_s[w0 + 1][tk]) + ss_s[w0 + 2][tk]) + ss_s[w0 + 3][tk];
+    const float sc = 1.0f / sqrtf(tot / 128.f + 1e-6f * 128.f);
+    float nw[8] = {};
+    add8(nw, p.norm_w + (k8 & 127));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = live ? v[e] * sc * nw[e] * silu_f(z[e]) : 0.f;
+    uint8_t* chunk = p.acts + ((uint64_t)(row / TM_TOK) * gridDim.x + blockIdx.x) * TM_CHUNK;
+    bool over = false;
+    pack_oct_tm(chunk, row % TM_TOK, k8, v, over);
+    float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+    if (lane < 8) pack_sum_tm(chunk, row % TM_TOK, warp, sum, over);
+    if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
+}
+
+dfl_status launch_tm_gdn_pack(cudaStream_t st, const TmGdn& p) {
+    launch_k(tm_gdn_pack_kernel, dim3((unsigned)(p.g.n_v * 128 / 256), (unsigned)(p.rows_pad / 8)), dim3(256), 0, st, p);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+}  // namespace dfl

@@ -1,0 +1,83 @@
+"""The many-row prompt pass against packed 16-row blocks of the same tokens (which the oracle tests pin): logits, captured rows,
+K/V rows, recurrent and conv state, and the rollback of the prompt's last block, at the edges of its 128-token tiles, of its
+512-token passes and of the packed remainder."""
+import importlib
+
+import numpy as np
+import pytest
+
+import modelgen
+from dflb import pkg
+
+syn = importlib.import_module("qwen-llm_b200.synthetic")
+pytestmark = pytest.mark.gpu
+
+
+def _state(arch, sess, n):
+    n_attn = sum(modelgen.is_attn(arch, il) for il in range(arch.n_layer))
+    kv = [np.concatenate(sess.read_kv(ai, p)) for ai in range(n_attn) for p in (0, n // 2, n - 1)]
+    gdn = [np.concatenate(sess.read_gdn_state(gi)) for gi in range(arch.n_layer - n_attn)]
+    return kv + gdn
+
+
+def _check(arch, gm, n, start, layer_ids, kv_f16=True, capacity=None):
+    rng = np.random.default_rng(n + start)
+    capacity = capacity or start + n + 32
+    ids = rng.integers(0, arch.vocab_size, size=start + n)
+    a, b = pkg.Session(gm, capacity, kv_f16), pkg.Session(gm, capacity, kv_f16)
+    sa, sb = pkg.Scratch(gm, 16, len(layer_ids)), pkg.Scratch(gm, 16, len(layer_ids))
+    rows = []
+    for off in range(0, start + n, 16):
+        blk = ids[off:min(off + 16, start if off < start else start + n)]
+        am, gap, lg = pkg.packed_verify(gm, b, sb, layer_ids, blk, off, want_logits=True)
+        rows.append(sb.read_capture(blk.size))
+    rows = np.concatenate(rows)[start:]
+    if start:
+        pkg.prefill(gm, a, sa, layer_ids, ids[:start], 0)
+    logits, hidden = pkg.prefill(gm, a, sa, layer_ids, ids[start:], start, want_hidden=True)
+    tol = dict(rtol=2e-3, atol=2e-4)
+    np.testing.assert_allclose(logits, lg[-1], **tol)
+    np.testing.assert_allclose(hidden, rows, rtol=2e-3, atol=2e-3)
+    assert a.kv_n_pos == b.kv_n_pos == start + n
+    for x, y in zip(_state(arch, a, start + n), _state(arch, b, start + n)):
+        np.testing.assert_allclose(x, y, rtol=5e-3, atol=2e-3)
+    # the last block can be undone in part, and the sequence goes on from there
+    last = n % 16 or 16
+    at = start + n - last
+    np.testing.assert_allclose(sa.read_capture(last), rows[-last:], rtol=2e-3, atol=2e-3)
+    keep = max(1, last - 3)
+    for sess, scr in ((a, sa), (b, sb)):
+        pkg.restore_partial(gm, sess, scr, keep, at)
+    for x, y in zip(_state(arch, a, at + keep), _state(arch, b, at + keep)):
+        np.testing.assert_allclose(x, y, rtol=5e-3, atol=2e-3)
+    nxt = rng.integers(0, arch.vocab_size, size=5)
+    la = pkg.packed_verify(gm, a, sa, layer_ids, nxt, at + keep, want_logits=True)[2]
+    lb = pkg.packed_verify(gm, b, sb, layer_ids, nxt, at + keep, want_logits=True)[2]
+    np.testing.assert_allclose(la, lb, **tol)
+    for x in (a, b, sa, sb):
+        x.close()
+
+
+@pytest.fixture(scope="module")
+def tiny():
+    arch = modelgen.tiny_arch()
+    gm = pkg.Model(arch, modelgen.target_tensors(arch, seed=3))
+    yield arch, gm
+    gm.close()
+
+
+@pytest.mark.parametrize("n,start", [(17, 0), (32, 0), (127, 0), (128, 16), (129, 0), (512, 0), (513, 0), (529, 0), (700, 32)])
+def test_prompt_pass_equals_packed_blocks(tiny, n, start):
+    arch, gm = tiny
+    _check(arch, gm, n, start, [0, 3, 3])
+
+
+@pytest.mark.parametrize("n,kv_f16,capacity", [(77, True, None), (300, True, 16384), (300, False, None)])
+def test_prompt_pass_at_dense_widths(n, kv_f16, capacity):
+    arch = syn.arch_9b()
+    arch.n_layer = 4
+    ents = syn.target_entries(arch, seed=51, device=0)
+    gm = syn.build_model(arch, ents)
+    syn.free_entries(ents)
+    _check(arch, gm, n, 0, [0, 1, 2, 3], kv_f16, capacity)
+    gm.close()
