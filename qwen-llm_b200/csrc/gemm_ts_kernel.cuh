@@ -193,12 +193,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
             kb_e += kb_step;
             if (kb_e >= n_kb) kb_e -= n_kb;
             if (e < n_kb) {   // first row tile: the column block's activations may still be in flight
-                ok = mbar_wait_bounded(&acts_bar[e], 0, p.err, DEV_ERR_WAIT_FULL);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = mbar_wait_warp(&acts_bar[e], 0, p.err, DEV_ERR_WAIT_FULL);
             }
             if (ok && e >= 2) {   // the group's accumulators were last used by entry e - 2
-                ok = mbar_wait_bounded(&d_free[g], (((uint32_t)e >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = mbar_wait_warp(&d_free[g], (((uint32_t)e >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
             }
             // one descriptor per column block; a 16-column slice is 1024 bytes further = 64 in the address field (bits 0-13
             // of the low word, which cannot carry: shared-memory addresses stay below 256 KiB)
@@ -208,8 +206,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
             for (int h2 = 0; h2 < HALVES / 2; ++h2, ++uses) {
                 const int h = 2 * h2 + (int)c;   // this warp's half; the unrolled code below needs it as a constant: see the switch on c
                 if (ok) {
-                    ok = mbar_wait_bounded(&a_ready[2 * g + c], uses & 1, p.err, DEV_ERR_WAIT_FULL);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = mbar_wait_warp(&a_ready[2 * g + c], uses & 1, p.err, DEV_ERR_WAIT_FULL);
                 }
                 if (ok) {
                     fence_after_sync();
@@ -240,8 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
         uint32_t hc = 0;   // running half count of this group
         for (int e = g; e < n_it && ok; e += 2) {
             const int s = e % STAGES;
-            ok = mbar_wait_bounded(full_bar(full, e, s), full_parity(e), p.err, DEV_ERR_WAIT_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(full_bar(full, e, s), full_parity(e), p.err, DEV_ERR_WAIT_FULL);
             if (!ok) break;
             const uint8_t* st = ring + s * F::STAGE;
             uint32_t am_keep[HALVES];
@@ -253,8 +249,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
                 if (F::HAS_MIN && h < HALVES - 1) am_keep[h] = am[0];
                 const uint32_t hb = hc & 1;
                 if (ok && hc >= 2) {   // the half buffer was last read by the MMAs of the group's half hc - 2
-                    ok = mbar_wait_bounded(&a_free[2 * g + hb], ((hc >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = mbar_wait_warp(&a_free[2 * g + hb], ((hc >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
                     if (ok) fence_after_sync();
                 }
                 if (ok) {
@@ -311,8 +306,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
         int kb_e = 0, tile = 0;   // e % n_kb and e / n_kb, kept by addition
         for (int e = 0; e < n_it && ok; ++e) {
             const uint32_t a = (uint32_t)e & 1u;
-            ok = mbar_wait_bounded(&d_ready[a], ((uint32_t)e >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(&d_ready[a], ((uint32_t)e >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
             if (!ok) break;
             fence_after_sync();
             const float2 sc = scl[(e & 3) * TILE_R + row];   // published before the a_ready arrival the MMAs waited for

@@ -154,22 +154,19 @@ __global__ void __launch_bounds__(TSB_THREADS, 1) gemm_tsb_kernel(const ParamsB 
         // ------------------------------ MMA issuer ------------------------------
         if (n_it > 0) {
             constexpr uint32_t IDESC = instr_desc_bf16(48);
-            bool ok = mbar_wait_bounded(acts_bar, 0, p.err, DEV_ERR_WAIT_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            bool ok = mbar_wait_warp(acts_bar, 0, p.err, DEV_ERR_WAIT_FULL);
             const uint32_t acts_addr = smem_u32(acts_res), ring_addr = smem_u32(ring);
             int e = 0;
             for (int t = 0; t < n_my && ok; ++t) {
                 const int buf = t & 1;
                 if (t >= 2) {
-                    ok = mbar_wait_bounded(&d_empty[buf], ((t >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = mbar_wait_warp(&d_empty[buf], ((t >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
                     if (!ok) break;
                     fence_after_sync();
                 }
                 for (int h = 0; h < n_slots_tile && ok; ++h, ++e) {
                     const int s = e % TSB_STAGES;
-                    ok = mbar_wait_bounded(&full[s], (e / TSB_STAGES) & 1, p.err, DEV_ERR_WAIT_FULL);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = mbar_wait_warp(&full[s], (e / TSB_STAGES) & 1, p.err, DEV_ERR_WAIT_FULL);
                     if (!ok) break;
                     fence_after_sync();
                     if (elect_one()) {
@@ -204,8 +201,7 @@ __global__ void __launch_bounds__(TSB_THREADS, 1) gemm_tsb_kernel(const ParamsB 
         bool ok = true;
         for (int t = 0; t < n_my && ok; ++t) {
             const int buf = t & 1;
-            ok = mbar_wait_bounded(&d_full[buf], (t >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(&d_full[buf], (t >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
             if (!ok) break;
             fence_after_sync();
             float v0[16], v1[16], v2[16];
