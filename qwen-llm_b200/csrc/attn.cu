@@ -199,11 +199,12 @@ __global__ void __launch_bounds__(256) attn_chunk_kernel(AttnGeom g, const float
 template <int HD>
 __global__ void __launch_bounds__(32) attn_post_kernel(AttnGeom g, const float* partials, int pos_per_span, int recs_per_span,
                                                        const float* gate, uint32_t start, uint8_t* acts, int bf3,
-                                                       float* out_f32, int* err) {
+                                                       float* out_f32, int* err, int n_spans) {
     pdl_prologue();
     constexpr int PER = HD / 32;  // 4 or 8
     const int qh = blockIdx.x, row = blockIdx.y, lane = threadIdx.x;
-    const int group = g.n_q / g.n_kv, kvh = qh / group, qi = row * group + qh % group;
+    const int group = g.n_q / g.n_kv, kvh = qh / group, qi = (row % MAX_ROWS) * group + qh % group;
+    partials += (uint64_t)(row / MAX_ROWS) * n_spans * recs_per_span * g.n_kv * (MAX_ROWS * group) * (HD + 2);   // the row's 16-row block
     // records holding visible positions: one per 64-position chunk (scalar kernel), one per span of chunks (mma.sync
     // kernel) or two per span of tiles (tcgen05 kernel: one per half of the keys)
     const int n_chunks = ((int)((start + (uint32_t)row) / (uint32_t)pos_per_span) + 1) * recs_per_span;
@@ -350,8 +351,29 @@ dfl_status launch_attn_verify(cudaStream_t st, const AttnGeom& g, const float* q
         DFL_CHECK(launch_acts_clear(st, acts, (uint64_t)g.n_q * g.hd / TILE_K * (uint64_t)act_chunk_bytes(bf3)));
     }
     (void)n_chunks;
-    if (g.hd == 128) launch_k(attn_post_kernel<128>, dim3(dim3((unsigned)g.n_q, (unsigned)n_rows)), dim3(32), 0, st, g, partials, pos_per_span, recs_per_span, gate, start, acts, bf3, out_f32, err);
-    else launch_k(attn_post_kernel<256>, dim3(dim3((unsigned)g.n_q, (unsigned)n_rows)), dim3(32), 0, st, g, partials, pos_per_span, recs_per_span, gate, start, acts, bf3, out_f32, err);
+    if (g.hd == 128) launch_k(attn_post_kernel<128>, dim3(dim3((unsigned)g.n_q, (unsigned)n_rows)), dim3(32), 0, st, g, partials, pos_per_span, recs_per_span, gate, start, acts, bf3, out_f32, err, 0);
+    else launch_k(attn_post_kernel<256>, dim3(dim3((unsigned)g.n_q, (unsigned)n_rows)), dim3(32), 0, st, g, partials, pos_per_span, recs_per_span, gate, start, acts, bf3, out_f32, err, 0);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+bool attn_rows_supported(const AttnGeom& g, int kv_mode) {
+    return kv_mode == KV_F16_TILED || attn_tc_supported(g, kv_mode != KV_F32_ROWS);
+}
+uint64_t attn_rows_partials_floats(const AttnGeom& g, int n_rows) {
+    return (uint64_t)((n_rows + MAX_ROWS - 1) / MAX_ROWS) * 2 * g.n_q * MAX_ROWS * (g.hd + 2);
+}
+// Every 16-row block of a prompt pass in one launch.  A block's CTA walks all its positions (one span), so that there are
+// one or two records per query to merge and enough CTAs (row blocks x KV heads) for the chip.
+dfl_status launch_attn_rows(cudaStream_t st, const AttnGeom& g, const float* q_rot, const float* gate, const void* k_cache, const void* v_cache,
+                            int kv_mode, uint32_t start, int n_rows, float* partials, float* out_f32, int* err) {
+    constexpr int ALL = 1 << 24;   // chunks per span: more than any cache holds
+    const bool tiled = kv_mode == KV_F16_TILED;
+    DFL_CHECK(tiled ? launch_attn_t5(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ALL, err)
+                    : launch_attn_span_tc(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ALL));
+    launch_k(attn_post_kernel<128>, dim3((unsigned)g.n_q, (unsigned)n_rows), dim3(32), 0, st, g, partials, 1 << 30, tiled ? 2 : 1, gate, start,
+             nullptr, 0, out_f32, err, 1);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

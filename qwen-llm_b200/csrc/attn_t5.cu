@@ -74,6 +74,14 @@ __device__ __forceinline__ void split_pair_f(float a, float b, uint32_t& hi, uin
 __global__ void __launch_bounds__(T5_THREADS, 1)
 attn_t5_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __half* v_cache, uint32_t start, int n_rows, float* partials,
                int chunks_per_span, float rescale_above, int* err) {
+    // blockIdx.z: 16-row block of a prompt pass (one block in a verify pass); the later, longer ones start first
+    if (gridDim.z > 1) {
+        const uint32_t blk = gridDim.z - 1 - blockIdx.z;
+        start += blk * MAX_ROWS;
+        n_rows = min(n_rows - (int)blk * MAX_ROWS, MAX_ROWS);
+        q_rot += (uint64_t)blk * MAX_ROWS * g.n_q * T5_HD;
+        partials += (uint64_t)blk * gridDim.x * 2 * g.n_kv * T5_Q * (T5_HD + 2);
+    }
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* ring = smem;
     float* q_stage = reinterpret_cast<float*>(smem + T5_OFF_QSTAGE);   // [64][129] f32: the queries, loaded row by row
@@ -151,8 +159,7 @@ attn_t5_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __ha
         for (int i = 0; i < n_c && ok; ++i) {
             const int b = i & 1;
             if (__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&abort_flag) != 0)) { ok = false; break; }
-            ok = mbar_wait_spin(&s_ready[b], (uint32_t)(i >> 1) & 1u, err, DEV_ERR_WAIT_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(&s_ready[b], (uint32_t)(i >> 1) & 1u, err, DEV_ERR_WAIT_FULL);
             if (!ok) break;
             fence_after_sync();
             float s[64];
@@ -183,8 +190,7 @@ attn_t5_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __ha
                 const float alpha = need ? ex2f(m_ref - mc) : 1.0f;   // 0 when there was no maximum yet
                 if (i >= 1) {
                     // O must be at rest: the previous tile's O += P V has completed
-                    ok = mbar_wait_spin(&pv_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = mbar_wait_warp(&pv_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
                     if (!ok) break;
                     fence_after_sync();
 #pragma unroll
@@ -221,8 +227,7 @@ attn_t5_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __ha
             if (lane == 0) mbar_arrive(&p_ready[b]);
         }
         if (ok) {
-            ok = mbar_wait_spin(&pv_done[(n_c - 1) & 1], (uint32_t)((n_c - 1) >> 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(&pv_done[(n_c - 1) & 1], (uint32_t)((n_c - 1) >> 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
         }
         if (!ok) abort_flag = 1;
         fence_after_sync();
@@ -254,14 +259,12 @@ attn_t5_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __ha
         const uint32_t ring_addr = smem_u32(ring);
         // the query operand: p_ready[1] counts the four softmax warps once before its first use for a tile (tile 1 waits
         // for its phase 1)
-        bool ok = mbar_wait_spin(&p_ready[1], 0u, err, DEV_ERR_WAIT_FULL);
-        ok = __all_sync(0xffffffffu, ok);
+        bool ok = mbar_wait_warp(&p_ready[1], 0u, err, DEV_ERR_WAIT_FULL);
         auto issue_qk = [&](int i) {
             const int b = i & 1, slot = (2 * i) % T5_SLOTS;
-            ok = mbar_wait_spin(&full[slot], (uint32_t)((2 * i) / T5_SLOTS) & 1u, err, DEV_ERR_WAIT_FULL);
+            ok = mbar_wait_warp(&full[slot], (uint32_t)((2 * i) / T5_SLOTS) & 1u, err, DEV_ERR_WAIT_FULL);
             // the buffer's P was the operand of the tile two steps back
-            if (ok && i >= 2) ok = mbar_wait_spin(&pv_done[b], (uint32_t)((i >> 1) - 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
-            ok = __all_sync(0xffffffffu, ok);
+            if (ok && i >= 2) ok = mbar_wait_warp(&pv_done[b], (uint32_t)((i >> 1) - 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
             if (!ok) return;
             fence_after_sync();
             if (elect_one()) {
@@ -285,9 +288,8 @@ attn_t5_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __ha
             const int b = i & 1, slot = (2 * i + 1) % T5_SLOTS;
             // tile 1's P arrives in phase 1 of p_ready[1] (phase 0 announced the query operand)
             const uint32_t p_phase = b == 1 ? (uint32_t)((i >> 1) + 1) & 1u : (uint32_t)(i >> 1) & 1u;
-            ok = mbar_wait_spin(&p_ready[b], p_phase, err, DEV_ERR_WAIT_FULL);
-            if (ok) ok = mbar_wait_spin(&full[slot], (uint32_t)((2 * i + 1) / T5_SLOTS) & 1u, err, DEV_ERR_WAIT_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(&p_ready[b], p_phase, err, DEV_ERR_WAIT_FULL);
+            if (ok) ok = mbar_wait_warp(&full[slot], (uint32_t)((2 * i + 1) / T5_SLOTS) & 1u, err, DEV_ERR_WAIT_FULL);
             if (!ok) break;
             fence_after_sync();
             if (elect_one()) {
@@ -426,8 +428,7 @@ dattn_t5_kernel(AttnGeom g, const float* q_rot, const __half* ctx_tiles, const _
         for (int i = 0; i < n_c && ok; ++i) {
             const int b = i & 1, chunk = c_begin + i;
             if (__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&abort_flag) != 0)) { ok = false; break; }
-            ok = mbar_wait_spin(&s_ready[b], (uint32_t)(i >> 1) & 1u, err, DEV_ERR_WAIT_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(&s_ready[b], (uint32_t)(i >> 1) & 1u, err, DEV_ERR_WAIT_FULL);
             if (!ok) break;
             fence_after_sync();
             float s[64];
@@ -456,8 +457,7 @@ dattn_t5_kernel(AttnGeom g, const float* q_rot, const __half* ctx_tiles, const _
                 // phase completed long ago; the slot's next use cannot complete before this step's P is written)
                 if (causal) {
                     const int u0 = 4 * i;
-                    ok = mbar_wait_spin(&full[u0 % T5_SLOTS], (uint32_t)(u0 / T5_SLOTS) & 1u, err, DEV_ERR_WAIT_FULL);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = mbar_wait_warp(&full[u0 % T5_SLOTS], (uint32_t)(u0 / T5_SLOTS) & 1u, err, DEV_ERR_WAIT_FULL);
                     if (!ok) break;
                 }
                 const uint32_t* kp = kpos + 128 * b + k0;
@@ -476,8 +476,7 @@ dattn_t5_kernel(AttnGeom g, const float* q_rot, const __half* ctx_tiles, const _
             if (__any_sync(0xffffffffu, need)) {
                 const float alpha = need ? ex2f(m_ref - mc) : 1.0f;
                 if (i >= 1) {
-                    ok = mbar_wait_spin(&pv_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = mbar_wait_warp(&pv_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
                     if (!ok) break;
                     fence_after_sync();
 #pragma unroll
@@ -513,8 +512,7 @@ dattn_t5_kernel(AttnGeom g, const float* q_rot, const __half* ctx_tiles, const _
             if (lane == 0) mbar_arrive(&p_ready[b]);
         }
         if (ok) {
-            ok = mbar_wait_spin(&pv_done[(n_c - 1) & 1], (uint32_t)((n_c - 1) >> 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(&pv_done[(n_c - 1) & 1], (uint32_t)((n_c - 1) >> 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
         }
         if (!ok) abort_flag = 1;
         fence_after_sync();
@@ -540,15 +538,13 @@ dattn_t5_kernel(AttnGeom g, const float* q_rot, const __half* ctx_tiles, const _
     } else if (warp == 4) {
         constexpr uint32_t IDESC = instr_desc(128);
         const uint32_t ring_addr = smem_u32(ring);
-        bool ok = mbar_wait_spin(&p_ready[1], 0u, err, DEV_ERR_WAIT_FULL);
-        ok = __all_sync(0xffffffffu, ok);
+        bool ok = mbar_wait_warp(&p_ready[1], 0u, err, DEV_ERR_WAIT_FULL);
         // tile u of this CTA (four per step: K hi, K lo, V hi, V lo) lives in ring slot u % 6, use u / 6
-        auto wait_tile = [&](int u) { return mbar_wait_spin(&full[u % T5_SLOTS], (uint32_t)(u / T5_SLOTS) & 1u, err, DEV_ERR_WAIT_FULL); };
+        auto wait_tile = [&](int u) { return mbar_wait_warp(&full[u % T5_SLOTS], (uint32_t)(u / T5_SLOTS) & 1u, err, DEV_ERR_WAIT_FULL); };
         auto issue_qk = [&](int i) {
             const int b = i & 1, u = 4 * i;
             ok = wait_tile(u) && wait_tile(u + 1);
-            if (ok && i >= 2) ok = mbar_wait_spin(&pv_done[b], (uint32_t)((i >> 1) - 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
-            ok = __all_sync(0xffffffffu, ok);
+            if (ok && i >= 2) ok = mbar_wait_warp(&pv_done[b], (uint32_t)((i >> 1) - 1) & 1u, err, DEV_ERR_WAIT_EMPTY);
             if (!ok) return;
             fence_after_sync();
             if (elect_one()) {
@@ -574,9 +570,8 @@ dattn_t5_kernel(AttnGeom g, const float* q_rot, const __half* ctx_tiles, const _
             }
             const int b = i & 1, u = 4 * i + 2;
             const uint32_t p_phase = b == 1 ? (uint32_t)((i >> 1) + 1) & 1u : (uint32_t)(i >> 1) & 1u;
-            ok = mbar_wait_spin(&p_ready[b], p_phase, err, DEV_ERR_WAIT_FULL);
+            ok = mbar_wait_warp(&p_ready[b], p_phase, err, DEV_ERR_WAIT_FULL);
             if (ok) ok = wait_tile(u) && wait_tile(u + 1);
-            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             fence_after_sync();
             if (elect_one()) {
@@ -718,7 +713,7 @@ dfl_status launch_attn_t5(cudaStream_t st, const AttnGeom& g, const float* q_rot
         const float v = (float)atof(e);
         if (v >= 0.f && v <= 12.f) rescale_above = v;
     }
-    launch_k(attn_t5_kernel, dim3((unsigned)n_spans, (unsigned)g.n_kv), dim3(T5_THREADS), (size_t)T5_SMEM, st, g, q_rot,
+    launch_k(attn_t5_kernel, dim3((unsigned)n_spans, (unsigned)g.n_kv, (unsigned)((n_rows + MAX_ROWS - 1) / MAX_ROWS)), dim3(T5_THREADS), (size_t)T5_SMEM, st, g, q_rot,
               reinterpret_cast<const __half*>(k_cache), reinterpret_cast<const __half*>(v_cache), start, n_rows, partials, chunks_per_span, rescale_above, err);
     count_launch();
     DFL_CUDA(cudaGetLastError());

@@ -62,6 +62,14 @@ __device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, b
 
 __global__ void __launch_bounds__(128) attn_span_tc_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __half* v_cache,
                                                            uint32_t start, int n_rows, float* partials, int chunks_per_span) {
+    // blockIdx.z: 16-row block of a prompt pass (one block in a verify pass); the later, longer ones start first
+    if (gridDim.z > 1) {
+        const uint32_t blk = gridDim.z - 1 - blockIdx.z;
+        start += blk * MAX_ROWS;
+        n_rows = min(n_rows - (int)blk * MAX_ROWS, MAX_ROWS);
+        q_rot += (uint64_t)blk * MAX_ROWS * g.n_q * TC_HD;
+        partials += (uint64_t)blk * gridDim.x * g.n_kv * TC_Q * (TC_HD + 2);
+    }
     pdl_prologue();
     extern __shared__ __align__(16) uint8_t sm_raw[];
     __half* q_hi = reinterpret_cast<__half*>(sm_raw);           // [64][136]
@@ -514,7 +522,7 @@ dfl_status launch_attn_span_tc(cudaStream_t st, const AttnGeom& g, const float* 
     }
     const int n_chunks = (int)((start + (uint32_t)n_rows + ATTN_CHUNK - 1) / ATTN_CHUNK);
     const int n_spans = (n_chunks + chunks_per_span - 1) / chunks_per_span;
-    launch_k(attn_span_tc_kernel, dim3((unsigned)n_spans, (unsigned)g.n_kv), dim3(128), (size_t)TC_SMEM, st, g, q_rot,
+    launch_k(attn_span_tc_kernel, dim3((unsigned)n_spans, (unsigned)g.n_kv, (unsigned)((n_rows + MAX_ROWS - 1) / MAX_ROWS)), dim3(128), (size_t)TC_SMEM, st, g, q_rot,
               reinterpret_cast<const __half*>(k_cache), reinterpret_cast<const __half*>(v_cache), start, n_rows, partials, chunks_per_span);
     count_launch();
     DFL_CUDA(cudaGetLastError());

@@ -67,6 +67,46 @@ dfl_status launch_gdn_conv_restore(cudaStream_t st, const GdnGeom& g, const floa
     return DFL_OK;
 }
 
+// One token of the recurrence for one state row shared by eight lanes: lane group member lg owns the sixteen columns
+// dk = 32 j + 4 lg + c (j, c < 4), so that the eight lanes of a row read 128 contiguous bytes of k and q per step.
+// The two row sums go through three shuffle levels each.
+__device__ __forceinline__ float gdn_token_step(float (&S)[16], const float* k_row, const float* q_row, float v, float gexp, float beta, int lg) {
+    float kk[16], qq[16];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 k4 = *reinterpret_cast<const float4*>(k_row + 32 * j + 4 * lg);
+        const float4 q4 = *reinterpret_cast<const float4*>(q_row + 32 * j + 4 * lg);
+        kk[4 * j] = k4.x; kk[4 * j + 1] = k4.y; kk[4 * j + 2] = k4.z; kk[4 * j + 3] = k4.w;
+        qq[4 * j] = q4.x; qq[4 * j + 1] = q4.y; qq[4 * j + 2] = q4.z; qq[4 * j + 3] = q4.w;
+    }
+    float p[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        p[j] = S[4 * j] * kk[4 * j];
+#pragma unroll
+        for (int c = 1; c < 4; ++c) p[j] = fmaf(S[4 * j + c], kk[4 * j + c], p[j]);
+    }
+    float sk = (p[0] + p[1]) + (p[2] + p[3]);
+#pragma unroll
+    for (int of = 4; of > 0; of >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, of);
+    const float coeff = beta * (v - gexp * sk);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int e = 4 * j + c;
+            S[e] = __fadd_rn(__fmul_rn(gexp, S[e]), __fmul_rn(coeff, kk[e]));
+        }
+        p[j] = S[4 * j] * qq[4 * j];
+#pragma unroll
+        for (int c = 1; c < 4; ++c) p[j] = fmaf(S[4 * j + c], qq[4 * j + c], p[j]);
+    }
+    float o = (p[0] + p[1]) + (p[2] + p[3]);
+#pragma unroll
+    for (int of = 4; of > 0; of >>= 1) o += __shfl_xor_sync(0xffffffffu, o, of);
+    return o;
+}
+
 // ---- scan (+ gated RMSNorm and activation packing) ------------------------------------------
 // grid (n_v, 4) in clusters of four along y (the four quarters of a head's 128 value channels), block 256: a warp
 // owns 4 state rows (dv), eight lanes per row, sixteen columns (dk) per lane.  The state rows are fetched before the

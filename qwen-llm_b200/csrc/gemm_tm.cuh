@@ -14,7 +14,8 @@
 // the f16 range), its B operand the sub-block sums as f16 hi + lo.
 //
 // Warps: 0..15 unpack (two groups of eight; group g owns A buffer g: Q4_K / Q5_K half g of a block, Q6_K quarters g and
-// g + 2), 16..19 read the accumulator back (thread = weight row), 20 issues the MMAs, 21 streams weights, 22 activations.
+// g + 2), 16..23 read the accumulator back (thread = weight row and half of the
+// tokens), 24 issues the MMAs, 25 streams weights, 26 activations.
 // Tensor memory: two 128-column block accumulators (one fills while the other is read back), the running sum over blocks
 // (128), two 64-column A buffers: all 512 columns.
 #pragma once
@@ -22,8 +23,8 @@
 namespace dfl {
 namespace ts {
 
-constexpr int TM_WARPS = 23, TM_THREADS = TM_WARPS * 32;
-constexpr int TM_MMA_WARP = 20, TM_W_WARP = 21, TM_B_WARP = 22;
+constexpr int TM_WARPS = 27, TM_THREADS = TM_WARPS * 32;
+constexpr int TM_DRAIN_WARPS = 8, TM_MMA_WARP = 24, TM_W_WARP = 25, TM_B_WARP = 26;
 constexpr int TM_B_STAGES = 4;
 constexpr uint32_t TM2_D = 0, TM2_ACC = 256, TM2_A = 384;
 constexpr int TM_BAR_BYTES = 512;
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
             mbar_init(&a_ready[i], GROUP_WARPS);
             mbar_init(&a_free[i], 1);
             mbar_init(&d_ready[i], 1);
-            mbar_init(&d_free[i], DRAIN_WARPS);
+            mbar_init(&d_free[i], TM_DRAIN_WARPS);
         }
         abort_flag = 0;
         mbar_fence_init();
@@ -171,66 +172,61 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         }
     } else if (warp == TM_MMA_WARP) {
         // ------------------------------ MMA issue ------------------------------
+        // All tensor-memory addresses are literals (the CTA owns all 512 columns, so the allocation starts at 0) and a
+        // block's four activation stages are the ring's four slots, so that the issuing warp spends its slots on MMAs.
         constexpr uint32_t IDESC = instr_desc(TM_TOK);
-        const uint64_t bd = smem_desc(smem_u32(b_ring), TM_TOK * 16, 128);
-        const uint32_t b_lo = (uint32_t)bd, b_hi = (uint32_t)(bd >> 32);
-        uint32_t e = 0, bs = 0, bround = 0;
+        static_assert(TM_B_STAGES == 4, "stage q of every block is ring slot q");
+        const uint32_t b_addr = smem_u32(b_ring), am_addr = smem_u32(smem + T::OFF_AM), s_addr = smem_u32(smem + T::OFF_S);
+        uint32_t e = 0;
         auto wait = [&](uint64_t* bar, uint32_t parity) {
-            ok = mbar_wait_bounded(bar, parity, p.err, DEV_ERR_WAIT_FULL);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_one(bar, parity, p.err, DEV_ERR_WAIT_FULL);
             return ok;
         };
-        for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
-            const Item it = item_of(idx);
-            for (int k = 0; k < it.n_kb && ok; ++k, ++e) {
-                const uint32_t d = tmem + TM2_D + (e & 1) * 128;
-                if (e >= 2 && !wait(&d_free[e & 1], ((e >> 1) - 1) & 1)) break;
+        auto block = [&](auto odd) {   // one 256-column block into accumulator e & 1
+            constexpr uint32_t O = decltype(odd)::value, D = TM2_D + O * 128;
+            if (e >= 2 && !wait(&d_free[O], ((e >> 1) - 1) & 1)) return;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {   // 64 columns = one activation stage
-                    const int g = T::MIN ? q >> 1 : q & 1;
-                    const uint32_t a = tmem + TM2_A + 64 * g;
-                    if (!T::MIN || (q & 1) == 0) {
-                        if (!wait(&a_ready[g], (T::MIN ? e : 2 * e + (q >> 1)) & 1)) break;
-                    }
-                    if (!wait(&b_full[bs], bround & 1)) break;
-                    fence_after_sync();
-                    if (elect_one()) {
-                        const uint32_t b = b_lo + bs * (TM_BSTAGE / 16);
+            for (int q = 0; q < 4; ++q) {   // 64 columns = one activation stage
+                const int g = T::MIN ? q >> 1 : q & 1;
+                if ((!T::MIN || (q & 1) == 0) && !wait(&a_ready[g], (T::MIN ? e : 2 * e + (q >> 1)) & 1)) return;
+                if (!wait(&b_full[q], e & 1)) return;
+                if (T::MIN && q == 3 && !wait(&s_full[O], (e >> 1) & 1)) return;
+                fence_after_sync();
+                {
+                    const uint64_t bd = smem_desc(b_addr + q * TM_BSTAGE, TM_TOK * 16, 128);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const uint32_t aj = a + (T::MIN ? 32 * (q & 1) : 0) + 8 * j;
-                            if (q == 0 && j == 0) mma_ts<false>(d, aj, b, b_hi, IDESC);
-                            else mma_ts<true>(d, aj, b + j * 256, b_hi, IDESC);
-                            mma_ts<true>(d, aj, b + (TM_BSTAGE / 32) + j * 256, b_hi, IDESC);
-                            if (!T::MIN) mma_ts<true>(d, aj + 32, b + j * 256, b_hi, IDESC);
-                        }
-                        mma_commit(&b_empty[bs]);
-                        if (!T::MIN) mma_commit(&a_free[g]);
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t aj = TM2_A + 64 * g + (T::MIN ? 32 * (q & 1) : 0) + 8 * j;
+                        mma_ts_rt(D, aj, bd + j * 256, IDESC, (q | j) != 0);
+                        mma_ts_rt(D, aj, bd + j * 256 + TM_BSTAGE / 32, IDESC, 1u);
+                        if (!T::MIN) mma_ts_rt(D, aj + 32, bd + j * 256, IDESC, 1u);
                     }
-                    __syncwarp();
-                    if (++bs == TM_B_STAGES) { bs = 0; ++bround; }
+                    mma_commit(&b_empty[q]);
                     if (T::MIN && q == 3) {
-                        if (!wait(&s_full[e & 1], (e >> 1) & 1)) break;
-                        if (elect_one()) {
-                            const uint64_t ad = smem_desc(smem_u32(smem + T::OFF_AM + (e & 1) * 4096), 2048, 128);
-                            const uint64_t sd = smem_desc(smem_u32(smem + T::OFF_S + (e & 1) * TM_SUMS), TM_TOK * 16, 128);
-                            mma_ss(d, ad, sd, IDESC, 1u);
-                            mma_ss(d, ad, sd + TM_SUMS / 32, IDESC, 1u);
-                            mma_commit(&s_empty[e & 1]);
-                        }
-                        __syncwarp();
+                        const uint64_t ad = smem_desc(am_addr + O * 4096, 2048, 128), sd = smem_desc(s_addr + O * TM_SUMS, TM_TOK * 16, 128);
+                        mma_ss(D, ad, sd, IDESC, 1u);
+                        mma_ss(D, ad, sd + TM_SUMS / 32, IDESC, 1u);
+                        mma_commit(&s_empty[O]);
                     }
-                    if (T::MIN && (q & 1)) {
-                        if (elect_one()) mma_commit(&a_free[g]);
-                        __syncwarp();
-                    }
+                    if (!T::MIN || (q & 1)) mma_commit(&a_free[g]);
+                    if (q == 3) mma_commit(&d_ready[O]);
                 }
-                if (ok) {
-                    if (elect_one()) mma_commit(&d_ready[e & 1]);
-                    __syncwarp();
+            }
+        };
+        if (elect_one()) {   // one thread runs the whole loop: nothing to vote on between two MMAs
+            if (tmem != 0) {
+                atomicCAS(p.err, 0, DEV_ERR_WAIT_FULL);
+                ok = false;
+            }
+            for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
+                const int n_kb = item_of(idx).n_kb;
+                for (int k = 0; k < n_kb && ok; ++k, ++e) {
+                    if (e & 1) block(std::integral_constant<uint32_t, 1>{});
+                    else block(std::integral_constant<uint32_t, 0>{});
                 }
             }
         }
+        __syncwarp();
     } else if (warp < UNPACK_WARPS) {
         // ------------------------------ unpack ------------------------------
         const int g = warp >> 3, q4 = warp & 3, kp2 = (warp >> 2) & 1;
@@ -242,8 +238,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
             const int n_kb = item_of(idx).n_kb;
             for (int k = 0; k < n_kb && ok; ++k, ++e) {
-                ok = mbar_wait_bounded(&w_full[s], round & 1, p.err, DEV_ERR_WAIT_FULL);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = mbar_wait_warp(&w_full[s], round & 1, p.err, DEV_ERR_WAIT_FULL);
                 if (!ok) break;
                 const uint8_t* st = w_ring + s * T::W_STAGE;
 #pragma unroll
@@ -269,8 +264,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                         if (lane == 0) mbar_arrive(&w_empty[s]);   // every lane has its bytes in registers
                     }
                     if (use >= 1) {
-                        ok = mbar_wait_bounded(&a_free[g], (use - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
-                        ok = __all_sync(0xffffffffu, ok);
+                        ok = mbar_wait_warp(&a_free[g], (use - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
                         if (!ok) break;
                         fence_after_sync();
                     }
@@ -305,7 +299,8 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
     } else {
         // ------------------------------ read-back ------------------------------
         pdl_wait();
-        const int row = threadIdx.x - DRAIN_WARP0 * 32;   // weight row of the tile = tensor-memory lane
+        const int row = (threadIdx.x - DRAIN_WARP0 * 32) & 127;   // weight row of the tile = tensor-memory lane
+        const int half = (warp - DRAIN_WARP0) >> 2;                // tokens 64 half .. + 63
         const uint32_t tm_l = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
         uint32_t e = 0;
         int scaled_tt = -1;
@@ -313,16 +308,15 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
             const Item it = item_of(idx);
             if (it.tt != scaled_tt) {   // per-token output scale of the token tile, thread = token
                 scaled_tt = it.tt;
-                named_sync(1, DRAIN_WARPS * 32);
+                named_sync(1, TM_DRAIN_WARPS * 32);
                 float ss = 0.f;
-                if (p.sumsq)
+                if (p.sumsq && half == 0)
                     for (int q = 0; q < p.n_sumsq; ++q) ss += p.sumsq[(uint64_t)q * p.rows_pad + it.tt * TM_TOK + row];
-                tok_scale[row] = p.sumsq ? p.out_scale * (1.0f / sqrtf(ss / p.norm_k + p.eps)) : p.out_scale;
-                named_sync(1, DRAIN_WARPS * 32);
+                if (half == 0) tok_scale[row] = p.sumsq ? p.out_scale * (1.0f / sqrtf(ss / p.norm_k + p.eps)) : p.out_scale;
+                named_sync(1, TM_DRAIN_WARPS * 32);
             }
             for (int k = 0; k < it.n_kb && ok; ++k, ++e) {
-                ok = mbar_wait_bounded(&d_ready[e & 1], (e >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = mbar_wait_warp(&d_ready[e & 1], (e >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
                 if (!ok) break;
                 fence_after_sync();
                 const float s = scl[(e & 3) * TILE_R + row];
@@ -330,12 +324,12 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 const bool last = k == it.n_kb - 1;
                 const uint32_t orow = (uint32_t)it.rt * TILE_R + row;
 #pragma unroll 1
-                for (int c = 0; c < 8; ++c) {   // 16 tokens
+                for (int c = 4 * half; c < 4 * half + 4; ++c) {   // 16 tokens
                     float v[16], a[16];
                     tmem_ld16(d + 16 * c, v);
                     if (k > 0) tmem_ld16(tm_l + TM2_ACC + 16 * c, a);
                     wait_ld();
-                    if (c == 7) {
+                    if (c == 4 * half + 3) {
                         fence_before_sync();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&d_free[e & 1]);

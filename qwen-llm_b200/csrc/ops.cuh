@@ -242,6 +242,11 @@ dfl_status launch_attn_front(cudaStream_t st, const AttnGeom& g, bool gated, con
 dfl_status launch_attn_verify(cudaStream_t st, const AttnGeom& g, const float* q_rot, const float* gate, const void* k_cache,
                               const void* v_cache, int kv_mode, uint32_t start, int n_rows, float* partials, uint8_t* acts,
                               int act_layout, float* out_f32, int* err, uint32_t kv_capacity = 0);
+// the same for all rows of a prompt pass at once (fp16 caches of 128-wide heads in groups of four)
+bool attn_rows_supported(const AttnGeom& g, int kv_mode);
+uint64_t attn_rows_partials_floats(const AttnGeom& g, int n_rows);
+dfl_status launch_attn_rows(cudaStream_t st, const AttnGeom& g, const float* q_rot, const float* gate, const void* k_cache, const void* v_cache,
+                            int kv_mode, uint32_t start, int n_rows, float* partials, float* out_f32, int* err);
 // tcgen05 span kernel over a tiled fp16 cache (attn_t5.cu) and the conversions between that cache and position-major rows
 bool attn_t5_supported(const AttnGeom& g, bool kv_f16);
 int attn_t5_chunks_per_span(const AttnGeom& g, uint32_t kv_capacity);
@@ -374,45 +379,6 @@ __device__ __forceinline__ void gdn_front_tile(const GdnFrontParams& p, int head
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         if (i0 + j < p.n_rows) *reinterpret_cast<float4*>(dst + (uint64_t)(i0 + j) * dst_ld) = make_float4(y[j][0], y[j][1], y[j][2], y[j][3]);
-}
-// One token of the recurrence for one state row shared by eight lanes: lane group member lg owns the sixteen columns
-// dk = 32 j + 4 lg + c (j, c < 4), so that the eight lanes of a row read 128 contiguous bytes of k and q per step.
-// The two row sums go through three shuffle levels each.
-__device__ __forceinline__ float gdn_token_step(float (&S)[16], const float* k_row, const float* q_row, float v, float gexp, float beta, int lg) {
-    float kk[16], qq[16];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float4 k4 = *reinterpret_cast<const float4*>(k_row + 32 * j + 4 * lg);
-        const float4 q4 = *reinterpret_cast<const float4*>(q_row + 32 * j + 4 * lg);
-        kk[4 * j] = k4.x; kk[4 * j + 1] = k4.y; kk[4 * j + 2] = k4.z; kk[4 * j + 3] = k4.w;
-        qq[4 * j] = q4.x; qq[4 * j + 1] = q4.y; qq[4 * j + 2] = q4.z; qq[4 * j + 3] = q4.w;
-    }
-    float p[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        p[j] = S[4 * j] * kk[4 * j];
-#pragma unroll
-        for (int c = 1; c < 4; ++c) p[j] = fmaf(S[4 * j + c], kk[4 * j + c], p[j]);
-    }
-    float sk = (p[0] + p[1]) + (p[2] + p[3]);
-#pragma unroll
-    for (int of = 4; of > 0; of >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, of);
-    const float coeff = beta * (v - gexp * sk);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int e = 4 * j + c;
-            S[e] = __fadd_rn(__fmul_rn(gexp, S[e]), __fmul_rn(coeff, kk[e]));
-        }
-        p[j] = S[4 * j] * qq[4 * j];
-#pragma unroll
-        for (int c = 1; c < 4; ++c) p[j] = fmaf(S[4 * j + c], qq[4 * j + c], p[j]);
-    }
-    float o = (p[0] + p[1]) + (p[2] + p[3]);
-#pragma unroll
-    for (int of = 4; of > 0; of >>= 1) o += __shfl_xor_sync(0xffffffffu, o, of);
-    return o;
 }
 #endif
 // conv1d + SiLU over the block, q/k L2 norm; keeps raw qkv rows for rollback; updates conv state in place.

@@ -10,7 +10,7 @@ namespace dfl {
 
 struct PromptWs {
     uint32_t rows = 0;   // padded rows the buffers hold
-    float *x = nullptr, *xn = nullptr, *part = nullptr, *sumsq = nullptr, *q_rot = nullptr, *gate = nullptr, *o = nullptr;
+    float *x = nullptr, *xn = nullptr, *part = nullptr, *sumsq = nullptr, *q_rot = nullptr, *gate = nullptr, *o = nullptr, *attn_part = nullptr;
     float *q_n = nullptr, *k_n = nullptr, *v = nullptr, *ab = nullptr, *conv_new = nullptr, *capture = nullptr;
     uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_v = nullptr;
     int32_t* tokens = nullptr;
@@ -82,6 +82,7 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
     alloc(&w->q_rot, R * q_dim * 4);
     alloc(&w->gate, R * q_dim * 4);
     alloc(&w->o, R * wide * 4);
+    if (m->n_attn) alloc(&w->attn_part, attn_rows_partials_floats(m->attn_geom(), (int)rows) * 4);
     alloc(&w->q_n, R * gg.n_k * 128 * 4);
     alloc(&w->k_n, R * gg.n_k * 128 * 4);
     alloc(&w->v, R * v_dim * 4);
@@ -154,7 +155,9 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             DFL_CHECK(gemm(L.qkv, w->acts_h, true, 1.f, &splits));
             DFL_CHECK(launch_attn_front(st, ag, true, w->part, splits, (int)L.qkv.total_cols, L.q_norm_w, L.k_norm_w, start, (int)n, s->k_cache[ai],
                                         s->v_cache[ai], s->kv_mode, w->q_rot, w->gate, nullptr, -1, rows_pad));
-            for (uint32_t r = 0; r < n; r += MAX_ROWS)
+            if (attn_rows_supported(ag, s->kv_mode))
+                DFL_CHECK(launch_attn_rows(st, ag, w->q_rot, w->gate, s->k_cache[ai], s->v_cache[ai], s->kv_mode, start, (int)n, w->attn_part, w->o, s->err));
+            else for (uint32_t r = 0; r < n; r += MAX_ROWS)
                 DFL_CHECK(launch_attn_verify(st, ag, w->q_rot + r * q_dim, w->gate + r * q_dim, s->k_cache[ai], s->v_cache[ai], s->kv_mode, start + r,
                                              (int)std::min<uint32_t>(MAX_ROWS, n - r), s->attn_partials, nullptr, m->act_layout, w->o + r * q_dim, s->err,
                                              s->kv_capacity));

@@ -273,17 +273,29 @@ dfl_status launch_tm_gdn_front(cudaStream_t st, const TmGdn& p) {
 }
 
 // ---- gated delta net: the recurrence -------------------------------------------------------------
+// Sixteen tokens at a time.  With S0 the state before a block, u_i = S0 k_i, w_i = S0 q_i and D_ij = g_{j+1} .. g_i the decay
+// between two tokens of the block (G_i from its start), the token recurrence
+//     c_i = beta_i (v_i - g_i S_{i-1} k_i),  S_i = g_i S_{i-1} + c_i k_i^T,  o_i = S_i q_i
+// is, row by row of S (a row = one value channel),
+//     (I + L) c = b,  L_ij = beta_i D_ij (k_j . k_i) for j < i,  b_i = beta_i (v_i - G_i u_i),
+//     o_i = G_i w_i + sum_{j <= i} D_ij (k_j . q_i) c_j,   S = G_15 S0 + sum_j D_15,j c_j k_j^T,
+// all in f32 and without a division.  A token-by-token scan waits twice per token for a three-level shuffle sum (512 tokens:
+// 242 us a layer); here a block's 32 sums are in flight together and only the 16-step substitution is serial, in registers.
 // grid (n_v, 4 quarters of the value channels), 256 threads: a warp owns four state rows, eight lanes a row, sixteen key
-// channels a lane, as in gdn_scan_kernel.  The sequential chain per token is bound by latency (two fused multiply-add trees
-// and three shuffle levels), so the next 16 tokens' q, k and v rows travel with cp.async while the current 16 are scanned.
+// channels a lane.  The next block's rows travel with cp.async.
 constexpr int SCAN_BLK = 16;
-__global__ void __launch_bounds__(256) tm_gdn_scan_kernel(const TmGdn p) {
-    __shared__ __align__(16) float qs[2][SCAN_BLK][128], ks[2][SCAN_BLK][128], vs[2][SCAN_BLK][32];
-    __shared__ float gs[2][SCAN_BLK], bs[2][SCAN_BLK];
+struct ScanSmem {
+    float qs[2][SCAN_BLK][128], ks[2][SCAN_BLK][128], vs[2][SCAN_BLK][32];
+    float L[SCAN_BLK][SCAN_BLK + 4], M[SCAN_BLK][SCAN_BLK + 4];   // L[j][i] (column major: one step of the substitution reads a column), M[i][j]
+    float gs[2][SCAN_BLK], bs[2][SCAN_BLK], G[SCAN_BLK], D[SCAN_BLK];
+};
+__global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
+    extern __shared__ __align__(16) uint8_t scan_smem[];
+    ScanSmem& sm = *reinterpret_cast<ScanSmem*>(scan_smem);
     const GdnGeom& g = p.g;
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rr = lane >> 3, lg = lane & 7, hk = h % g.n_k;
-    const int dv_cta = blockIdx.y * 32, dv = dv_cta + warp * 4 + rr;
+    const int dv_cta = blockIdx.y * 32, dv_l = warp * 4 + rr, dv = dv_cta + dv_l;
     const float dtb = p.dt_bias[h], alog = p.a_log[h];
     pdl_prologue();
     float S[16];
@@ -294,29 +306,47 @@ __global__ void __launch_bounds__(256) tm_gdn_scan_kernel(const TmGdn p) {
         S[4 * j] = s4.x; S[4 * j + 1] = s4.y; S[4 * j + 2] = s4.z; S[4 * j + 3] = s4.w;
     }
     auto cp16 = [](void* dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); };
-    auto fetch = [&](int blk) {
-        const int buf = blk & 1, r0 = blk * SCAN_BLK, n = min(SCAN_BLK, p.n_rows - r0);
-        for (int i = threadIdx.x; i < n * 32; i += 256) {
+    // block boundaries: multiples of 16 from the start, and the first row of the part a rollback may undo
+    const int ckpt = p.last_rows ? p.n_rows - p.last_rows : 0;
+    auto next_of = [&](int r0) { return min(r0 < ckpt && r0 + SCAN_BLK > ckpt ? ckpt : r0 + SCAN_BLK, p.n_rows); };
+    auto fetch = [&](int r0, int buf) {   // rows beyond the block's are zeros: they add nothing and decay nothing
+        const int n = next_of(r0) - r0;
+        for (int i = threadIdx.x; i < SCAN_BLK * 32; i += 256) {
             const int r = i >> 5, d = (i & 31) * 4;
-            cp16(&qs[buf][r][d], p.q_n + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
-            cp16(&ks[buf][r][d], p.k_n + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
-        }
-        for (int i = threadIdx.x; i < n * 8; i += 256) {
-            const int r = i >> 3, d = (i & 7) * 4;
-            cp16(&vs[buf][r][d], p.v + ((uint64_t)(r0 + r) * g.n_v + h) * 128 + dv_cta + d);
-        }
-        if ((int)threadIdx.x < n) {
-            const float* a = p.ab + (uint64_t)(r0 + threadIdx.x) * (2 * g.n_v) + h;
-            const float alpha = __ldcg(a), beta = __ldcg(a + g.n_v);
-            gs[buf][threadIdx.x] = expf(softplus_f(alpha + dtb) * alog);
-            bs[buf][threadIdx.x] = sigmoid_f(beta);
-            const int kr = r0 + (int)threadIdx.x - (p.n_rows - p.last_rows);
-            if (p.last_rows && kr >= 0 && blockIdx.y == 0) {
-                p.keep_ab[(uint64_t)kr * (2 * g.n_v) + h] = alpha;
-                p.keep_ab[(uint64_t)kr * (2 * g.n_v) + g.n_v + h] = beta;
+            if (r < n) {
+                cp16(&sm.qs[buf][r][d], p.q_n + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
+                cp16(&sm.ks[buf][r][d], p.k_n + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
+            } else {
+                *reinterpret_cast<float4*>(&sm.qs[buf][r][d]) = make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(&sm.ks[buf][r][d]) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
+        if (threadIdx.x < SCAN_BLK * 8) {
+            const int r = threadIdx.x >> 3, d = (threadIdx.x & 7) * 4;
+            if (r < n) cp16(&sm.vs[buf][r][d], p.v + ((uint64_t)(r0 + r) * g.n_v + h) * 128 + dv_cta + d);
+            else *reinterpret_cast<float4*>(&sm.vs[buf][r][d]) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // gate inputs of a block: loaded a block ahead by 16 threads, turned into gates when the block starts
+    float ga = 0.f, gb = 0.f;
+    auto gate_load = [&](int r0) {
+        if (threadIdx.x < SCAN_BLK && r0 + (int)threadIdx.x < p.n_rows) {
+            const float* a = p.ab + (uint64_t)(r0 + threadIdx.x) * (2 * g.n_v) + h;
+            ga = __ldcg(a);
+            gb = __ldcg(a + g.n_v);
+        }
+    };
+    auto gate_store = [&](int r0, int buf) {
+        if (threadIdx.x >= SCAN_BLK) return;
+        const int n = next_of(r0) - r0, i = threadIdx.x;
+        sm.gs[buf][i] = i < n ? expf(softplus_f(ga + dtb) * alog) : 1.f;
+        sm.bs[buf][i] = i < n ? sigmoid_f(gb) : 0.f;
+        const int kr = r0 + i - ckpt;
+        if (p.last_rows && kr >= 0 && i < n && blockIdx.y == 0) {
+            p.keep_ab[(uint64_t)kr * (2 * g.n_v) + h] = ga;
+            p.keep_ab[(uint64_t)kr * (2 * g.n_v) + g.n_v + h] = gb;
+        }
     };
     auto put = [&](float* dst) {
 #pragma unroll
@@ -329,32 +359,132 @@ __global__ void __launch_bounds__(256) tm_gdn_scan_kernel(const TmGdn p) {
         for (int i = c0 + threadIdx.x; i < min(n, c0 + per); i += 256)
             reinterpret_cast<float4*>(p.conv_state)[i] = __ldcg(reinterpret_cast<const float4*>(p.conv_new) + i);
     }
-    const int n_blk = (p.n_rows + SCAN_BLK - 1) / SCAN_BLK;
-    const int ckpt = p.last_rows ? p.n_rows - p.last_rows : -1;
-    fetch(0);
-    for (int b = 0; b < n_blk; ++b) {
-        if (b + 1 < n_blk) {
-            fetch(b + 1);
+    fetch(0, 0);
+    gate_load(0);
+    int buf = 0;
+    for (int r0 = 0; r0 < p.n_rows; buf ^= 1) {
+        const int r1 = next_of(r0), n = r1 - r0;
+        gate_store(r0, buf);
+        if (r1 < p.n_rows) {
+            fetch(r1, buf ^ 1);
+            gate_load(r1);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        const int buf = b & 1, r0 = b * SCAN_BLK, n = min(SCAN_BLK, p.n_rows - r0);
-        float* o_row = p.o + (uint64_t)r0 * g.n_v * 128 + h * 128 + dv;
-#pragma unroll 2
-        for (int i = 0; i < n; ++i) {
-            if (r0 + i == ckpt) put(p.state_in);
-            const float o = gdn_token_step(S, ks[buf][i], qs[buf][i], vs[buf][i][warp * 4 + rr], gs[buf][i], bs[buf][i], lg);
-            if (lg == 0) o_row[(uint64_t)i * g.n_v * 128] = o;
+        // ---- the block's Gram matrices and decays: warp w takes rows i = 2 w, 2 w + 1; lane = (j = lane & 15, k or q by lane >> 4)
+        {
+            const int j = lane & 15;
+            const float(*src)[128] = lane < 16 ? sm.ks[buf] : sm.qs[buf];
+#pragma unroll
+            for (int ii = 0; ii < 2; ++ii) {
+                const int i = 2 * warp + ii;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                // columns rotated by lane so that the sixteen rows j fall on different banks
+#pragma unroll 8
+                for (int c = 0; c < 32; ++c) {
+                    const int d = ((c + j) & 31) * 4;
+                    const float4 a = *reinterpret_cast<const float4*>(&sm.ks[buf][j][d]);
+                    const float4 b = *reinterpret_cast<const float4*>(&src[i][d]);
+                    acc[0] = fmaf(a.x, b.x, acc[0]); acc[1] = fmaf(a.y, b.y, acc[1]);
+                    acc[2] = fmaf(a.z, b.z, acc[2]); acc[3] = fmaf(a.w, b.w, acc[3]);
+                }
+                const float dot = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+                float dec = 1.f;   // D_ij
+                for (int t = 1; t < SCAN_BLK; ++t) dec *= (t > j && t <= i) ? sm.gs[buf][t] : 1.f;
+                if (lane < 16) sm.L[j][i] = j < i ? sm.bs[buf][i] * dec * dot : 0.f;
+                else sm.M[i][j] = j <= i ? dec * dot : 0.f;
+                if (lane < 16 && i == SCAN_BLK - 1) sm.D[j] = dec;
+                if (lane == 0) {
+                    float gg = 1.f;
+                    for (int t = 0; t <= i; ++t) gg *= sm.gs[buf][t];
+                    sm.G[i] = gg;
+                }
+            }
         }
-        __syncthreads();   // the buffer is refilled by the next iteration's fetch
+        // ---- u = S0 k, w = S0 q for the row's sixteen tokens
+        float u[SCAN_BLK], w[SCAN_BLK];
+#pragma unroll
+        for (int i = 0; i < SCAN_BLK; ++i) {
+            float pk[4], pq[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 k4 = *reinterpret_cast<const float4*>(&sm.ks[buf][i][32 * j + 4 * lg]);
+                const float4 q4 = *reinterpret_cast<const float4*>(&sm.qs[buf][i][32 * j + 4 * lg]);
+                pk[j] = fmaf(S[4 * j + 3], k4.w, fmaf(S[4 * j + 2], k4.z, fmaf(S[4 * j + 1], k4.y, S[4 * j] * k4.x)));
+                pq[j] = fmaf(S[4 * j + 3], q4.w, fmaf(S[4 * j + 2], q4.z, fmaf(S[4 * j + 1], q4.y, S[4 * j] * q4.x)));
+            }
+            u[i] = (pk[0] + pk[1]) + (pk[2] + pk[3]);
+            w[i] = (pq[0] + pq[1]) + (pq[2] + pq[3]);
+        }
+#pragma unroll
+        for (int of = 4; of > 0; of >>= 1) {
+#pragma unroll
+            for (int i = 0; i < SCAN_BLK; ++i) u[i] += __shfl_xor_sync(0xffffffffu, u[i], of);
+        }
+        // w: lane lg keeps tokens 2 lg, 2 lg + 1 (halving: each step exchanges the half the partner keeps)
+#pragma unroll
+        for (int of = 4; of > 0; of >>= 1) {
+            const bool up = lg & of;
+#pragma unroll
+            for (int i = 0; i < 2 * of; ++i) {
+                const float give = up ? w[i] : w[i + 2 * of], keep = up ? w[i + 2 * of] : w[i];
+                w[i] = keep + __shfl_xor_sync(0xffffffffu, give, of);
+            }
+        }
+        __syncthreads();   // L, M, G, D
+        // ---- substitution: u becomes c
+#pragma unroll
+        for (int i = 0; i < SCAN_BLK; ++i) u[i] = sm.bs[buf][i] * (sm.vs[buf][i][dv_l] - sm.G[i] * u[i]);
+#pragma unroll
+        for (int j = 0; j < SCAN_BLK - 1; ++j) {
+#pragma unroll
+            for (int i4 = (j + 1) / 4; i4 < 4; ++i4) {
+                const float4 l = *reinterpret_cast<const float4*>(&sm.L[j][4 * i4]);   // zero for i <= j
+                if (4 * i4 > j) u[4 * i4] = fmaf(-l.x, u[j], u[4 * i4]);
+                if (4 * i4 + 1 > j) u[4 * i4 + 1] = fmaf(-l.y, u[j], u[4 * i4 + 1]);
+                if (4 * i4 + 2 > j) u[4 * i4 + 2] = fmaf(-l.z, u[j], u[4 * i4 + 2]);
+                if (4 * i4 + 3 > j) u[4 * i4 + 3] = fmaf(-l.w, u[j], u[4 * i4 + 3]);
+            }
+        }
+        // ---- outputs of tokens 2 lg, 2 lg + 1
+        float* o_row = p.o + (uint64_t)r0 * g.n_v * 128 + h * 128 + dv;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int i = 2 * lg + t;
+            float o0 = sm.G[i] * w[t], o1 = 0.f;
+#pragma unroll
+            for (int j4 = 0; j4 < 4; ++j4) {
+                const float4 m = *reinterpret_cast<const float4*>(&sm.M[i][4 * j4]);
+                o0 = fmaf(m.x, u[4 * j4], o0); o1 = fmaf(m.y, u[4 * j4 + 1], o1);
+                o0 = fmaf(m.z, u[4 * j4 + 2], o0); o1 = fmaf(m.w, u[4 * j4 + 3], o1);
+            }
+            if (i < n) o_row[(uint64_t)i * g.n_v * 128] = o0 + o1;
+        }
+        // ---- state
+        const float Gend = sm.G[SCAN_BLK - 1];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) S[e] *= Gend;
+#pragma unroll
+        for (int i = 0; i < SCAN_BLK; ++i) {
+            const float c = u[i] * sm.D[i];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 k4 = *reinterpret_cast<const float4*>(&sm.ks[buf][i][32 * j + 4 * lg]);
+                S[4 * j] = fmaf(c, k4.x, S[4 * j]); S[4 * j + 1] = fmaf(c, k4.y, S[4 * j + 1]);
+                S[4 * j + 2] = fmaf(c, k4.z, S[4 * j + 2]); S[4 * j + 3] = fmaf(c, k4.w, S[4 * j + 3]);
+            }
+        }
+        r0 = r1;
+        if (p.last_rows && r0 == ckpt) put(p.state_in);
+        __syncthreads();   // this block's buffers, L, M, G and D are free
     }
     put(p.state_out);
 }
 
 dfl_status launch_tm_gdn_scan(cudaStream_t st, const TmGdn& p) {
-    launch_k(tm_gdn_scan_kernel, dim3((unsigned)p.g.n_v, 4), dim3(256), 0, st, p);
+    launch_k(tm_gdn_scan_kernel, dim3((unsigned)p.g.n_v, 4), dim3(256), sizeof(ScanSmem), st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;
