@@ -426,9 +426,9 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
     bool ok = cudaStreamCreateWithFlags(&ds->st, cudaStreamNonBlocking) == cudaSuccess;
     auto alloc = [&](size_t bytes) -> void* {
         if (!ok) return nullptr;
-        void* q = nullptr;
-        ok = cudaMalloc(&q, bytes ? bytes : 16) == cudaSuccess;
-        if (ok) { cudaMemset(q, 0, bytes ? bytes : 16); ds->allocs.push_back(q); }
+        void* q = pool_alloc(bytes ? bytes : 16);
+        ok = q != nullptr;
+        if (ok) { cudaMemsetAsync(q, 0, bytes ? bytes : 16, ds->st); ds->allocs.push_back(q); }
         return q;
     };
     const AttnGeom g = d->geom((int)c.n_q_heads);
@@ -481,8 +481,8 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
         ds->acts_sel = (uint8_t*)alloc(acts_bytes(DFL_BF16, H));
     }
     ds->err = (int*)alloc(4);
-    ok = ok && cudaMallocHost(&ds->pinned_i, 2 * MAX_ROWS * 4) == cudaSuccess;
-    ok = ok && cudaMallocHost(&ds->pinned_sel, MAX_ROWS * 16 * 8 + (size_t)MAX_ROWS * c.selector_rank * 4) == cudaSuccess;
+    ok = ok && (ds->pinned_i = (int32_t*)pool_alloc_host(2 * MAX_ROWS * 4));
+    ok = ok && (ds->pinned_sel = (uint8_t*)pool_alloc_host(MAX_ROWS * 16 * 8 + (size_t)MAX_ROWS * c.selector_rank * 4));
     ok = ok && cudaEventCreate(&ds->ev0) == cudaSuccess && cudaEventCreate(&ds->ev1) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&ds->st_side, cudaStreamNonBlocking) == cudaSuccess;
     for (uint32_t il = 0; il < c.n_layer; ++il) ok = ok && cudaEventCreateWithFlags(&ds->ev_ctx[il], cudaEventDisableTiming) == cudaSuccess;
@@ -492,7 +492,7 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
         return fail(DFL_ERR_OOM, "dsession_create: allocation failed: " + why);
     }
     ds->pos_host.reserve(ctx_capacity);
-    cudaDeviceSynchronize();
+    cudaStreamSynchronize(ds->st);
     *out = ds;
     return DFL_OK;
 }
@@ -500,9 +500,11 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
 void dfl_dsession_destroy(dfl_dsession* ds) {
     if (!ds) return;
     cudaSetDevice(ds->d->target->device);
-    for (void* p : ds->allocs) cudaFree(p);
-    if (ds->pinned_i) cudaFreeHost(ds->pinned_i);
-    if (ds->pinned_sel) cudaFreeHost(ds->pinned_sel);
+    for (cudaStream_t st : {ds->st, ds->st_side})
+        if (st) cudaStreamSynchronize(st);
+    for (void* p : ds->allocs) pool_free(p);
+    pool_free(ds->pinned_i);
+    pool_free(ds->pinned_sel);
     if (ds->ev0) cudaEventDestroy(ds->ev0);
     if (ds->ev1) cudaEventDestroy(ds->ev1);
     for (auto& e : ds->ev_ctx)

@@ -661,6 +661,7 @@ void dfl_model_destroy(dfl_model* m) {
     ep_comm_destroy(m->ep_comm, m->ep_dead.load());
     if (m->embd_ggml) cudaFree(m->embd_ggml);
     if (m->out_norm_w) cudaFree(m->out_norm_w);
+    pool_trim(m->device);
     delete m;
 }
 
@@ -693,23 +694,23 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
     bool ok = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) == cudaSuccess;
     for (int i = 0; i < m->n_attn && ok; ++i) {
         void *k = nullptr, *v = nullptr;
-        ok = cudaMalloc(&k, kv_bytes) == cudaSuccess && cudaMalloc(&v, kv_bytes) == cudaSuccess;
+        ok = (k = pool_alloc(kv_bytes)) && (v = pool_alloc(kv_bytes));
         // whole tiles go through the tensor cores, positions not yet written included: they must hold finite values
-        if (ok && s->kv_mode == KV_F16_TILED) { cudaMemset(k, 0, kv_bytes); cudaMemset(v, 0, kv_bytes); }
+        if (ok && s->kv_mode == KV_F16_TILED) { cudaMemsetAsync(k, 0, kv_bytes, s->st); cudaMemsetAsync(v, 0, kv_bytes, s->st); }
         s->k_cache.push_back(k);
         s->v_cache.push_back(v);
     }
     for (int i = 0; i < m->n_gdn && ok; ++i) {
         float *c = nullptr, *s0 = nullptr, *s1 = nullptr;
-        ok = cudaMalloc(&c, conv_bytes) == cudaSuccess && cudaMalloc(&s0, ssm_bytes) == cudaSuccess && cudaMalloc(&s1, ssm_bytes) == cudaSuccess;
-        if (ok) { cudaMemset(c, 0, conv_bytes); cudaMemset(s0, 0, ssm_bytes); cudaMemset(s1, 0, ssm_bytes); }
+        ok = (c = (float*)pool_alloc(conv_bytes)) && (s0 = (float*)pool_alloc(ssm_bytes)) && (s1 = (float*)pool_alloc(ssm_bytes));
+        if (ok) { cudaMemsetAsync(c, 0, conv_bytes, s->st); cudaMemsetAsync(s0, 0, ssm_bytes, s->st); cudaMemsetAsync(s1, 0, ssm_bytes, s->st); }
         s->conv.push_back(c);
         s->ssm[0].push_back(s0);
         s->ssm[1].push_back(s1);
         s->ssm_cur.push_back(0);
     }
-    if (ok && m->n_attn) ok = cudaMalloc(&s->attn_partials, attn_partials_floats(m->attn_geom(), (uint32_t)cap_alloc) * 4) == cudaSuccess;   // two records per 128-position tile in tiled storage
-    ok = ok && cudaMalloc(&s->err, 4) == cudaSuccess;
+    if (ok && m->n_attn) ok = (s->attn_partials = (float*)pool_alloc(attn_partials_floats(m->attn_geom(), (uint32_t)cap_alloc) * 4)) != nullptr;   // two records per 128-position tile in tiled storage
+    ok = ok && (s->err = (int*)pool_alloc(4));
     ok = ok && cudaEventCreate(&s->ev0) == cudaSuccess && cudaEventCreate(&s->ev1) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&s->st_side, cudaStreamNonBlocking) == cudaSuccess &&
          cudaStreamCreateWithFlags(&s->st_side2, cudaStreamNonBlocking) == cudaSuccess;
@@ -722,8 +723,8 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
         dfl_session_destroy(s);
         return fail(DFL_ERR_OOM, "session_create: allocation failed: " + why);
     }
-    cudaMemset(s->err, 0, 4);
-    cudaDeviceSynchronize();
+    cudaMemsetAsync(s->err, 0, 4, s->st);
+    cudaStreamSynchronize(s->st);   // this session's memory only: other sessions' work goes on
     *out = s;
     return DFL_OK;
 }
@@ -731,13 +732,15 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
 void dfl_session_destroy(dfl_session* s) {
     if (!s) return;
     cudaSetDevice(s->m->device);
-    for (void* p : s->k_cache) cudaFree(p);
-    for (void* p : s->v_cache) cudaFree(p);
-    for (float* p : s->conv) cudaFree(p);
-    for (float* p : s->ssm[0]) cudaFree(p);
-    for (float* p : s->ssm[1]) cudaFree(p);
-    cudaFree(s->attn_partials);
-    cudaFree(s->err);
+    for (cudaStream_t st : {s->st, s->st_side, s->st_side2})   // nothing of this session is in flight when its blocks go back
+        if (st) cudaStreamSynchronize(st);
+    for (void* p : s->k_cache) pool_free(p);
+    for (void* p : s->v_cache) pool_free(p);
+    for (float* p : s->conv) pool_free(p);
+    for (float* p : s->ssm[0]) pool_free(p);
+    for (float* p : s->ssm[1]) pool_free(p);
+    pool_free(s->attn_partials);
+    pool_free(s->err);
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
@@ -831,8 +834,8 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
     bool ok = true;
     auto alloc = [&](auto** p, size_t bytes) {
         if (!ok) return;
-        void* q = nullptr;
-        ok = cudaMalloc(&q, bytes ? bytes : 16) == cudaSuccess;
+        void* q = pool_alloc(bytes ? bytes : 16);
+        ok = q != nullptr;
         if (ok) { cudaMemset(q, 0, bytes ? bytes : 16); sc->allocs.push_back(q); }
         *p = reinterpret_cast<std::remove_reference_t<decltype(**p)>*>(q);
     };
@@ -873,7 +876,7 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
     { uint8_t* am = nullptr; alloc(&am, MAX_ROWS * ARGMAX_PARTS * 16); sc->am_scratch = am; }
     alloc(&sc->capture, (size_t)MAX_ROWS * sc->k_layers * H * 4);
     alloc(&sc->tokens_dev, MAX_ROWS * 4);
-    ok = ok && cudaMallocHost(&sc->pinned_i, 2 * MAX_ROWS * 4) == cudaSuccess && cudaMallocHost(&sc->pinned_f, MAX_ROWS * 4) == cudaSuccess;
+    ok = ok && (sc->pinned_i = (int32_t*)pool_alloc_host(2 * MAX_ROWS * 4)) && (sc->pinned_f = (float*)pool_alloc_host(MAX_ROWS * 4));
     if (!ok) {
         std::string why = cudaGetErrorString(cudaGetLastError());
         dfl_scratch_destroy(sc);
@@ -887,9 +890,10 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
 void dfl_scratch_destroy(dfl_scratch* sc) {
     if (!sc) return;
     cudaSetDevice(sc->m->device);
-    for (void* p : sc->allocs) cudaFree(p);
-    if (sc->pinned_i) cudaFreeHost(sc->pinned_i);
-    if (sc->pinned_f) cudaFreeHost(sc->pinned_f);
+    cudaDeviceSynchronize();   // a scratch does not know the streams of the sessions that used it
+    for (void* p : sc->allocs) pool_free(p);
+    pool_free(sc->pinned_i);
+    pool_free(sc->pinned_f);
     if (sc->pinned_logits) cudaFreeHost(sc->pinned_logits);
     if (sc->pinned_order) cudaFreeHost(sc->pinned_order);
     if (sc->order_dev) cudaFree(sc->order_dev);

@@ -19,6 +19,13 @@ dfl_status qmatrix_create(int device, int dtype, uint64_t n_in, uint64_t n_out, 
                           cudaStream_t st, QMatrix* m, bool allow_ts = false, int kb_group = 0);
 void qmatrix_release(QMatrix* m);
 
+// device / pinned blocks that outlive one session (pool.cu): on the current device; nullptr when there is no memory.  A block
+// may only be given back when nothing in flight uses it any more.
+void* pool_alloc(size_t bytes);
+void* pool_alloc_host(size_t bytes);
+void pool_free(void* p);
+void pool_trim(int device);
+
 // Several matrices that consume the same activations and write side by side into one
 // partial buffer [splits][16][total_cols].
 struct MatGroup {

@@ -22,8 +22,8 @@ const float* prompt_capture(const dfl_scratch* sc) { return sc->prompt->capture;
 
 void prompt_ws_free(PromptWs* w) {
     if (!w) return;
-    for (void* p : w->allocs) cudaFree(p);
-    if (w->pinned) cudaFreeHost(w->pinned);
+    for (void* p : w->allocs) pool_free(p);
+    pool_free(w->pinned);
     delete w;
 }
 
@@ -55,6 +55,7 @@ static int tm_splits(const MatGroup& g, int tok_tiles) {
 
 static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) {
     if (sc->prompt && sc->prompt->rows >= rows) return DFL_OK;
+    if (sc->prompt) cudaDeviceSynchronize();
     prompt_ws_free(sc->prompt);
     sc->prompt = nullptr;
     auto* w = new PromptWs();
@@ -69,8 +70,8 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
                 if (!g->mats.empty()) part = std::max<uint64_t>(part, (uint64_t)tm_splits(*g, t) * t * TM_TOK * g->total_cols);
     bool ok = true;
     auto alloc = [&](auto** p, uint64_t bytes) {
-        void* q = nullptr;
-        ok = ok && cudaMalloc(&q, bytes ? bytes : 16) == cudaSuccess;
+        void* q = ok ? pool_alloc(bytes ? bytes : 16) : nullptr;
+        ok = q != nullptr;
         if (q) w->allocs.push_back(q);
         *p = reinterpret_cast<std::remove_reference_t<decltype(**p)>*>(q);
     };
@@ -93,7 +94,7 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
     alloc(&w->acts_f, tiles * (F / TILE_K) * TM_CHUNK);
     alloc(&w->acts_v, tiles * (wide / TILE_K) * TM_CHUNK);
     alloc(&w->tokens, R * 4);
-    ok = ok && cudaMallocHost(&w->pinned, R * 4) == cudaSuccess;
+    ok = ok && (w->pinned = (int32_t*)pool_alloc_host(R * 4));
     if (!ok) {
         std::string why = cudaGetErrorString(cudaGetLastError());
         prompt_ws_free(w);

@@ -27,7 +27,7 @@ struct TmGlue {
 };
 dfl_status launch_tm_glue(cudaStream_t st, const TmGlue& p, uint64_t k);
 
-// out [rows][ld_out] = rs[row] * xn[row] . w[j] in f32 (alpha / beta, router); k a multiple of 128
+// out [rows][ld_out] = rs[row] * xn[row] . w[j] in f32 (alpha / beta, router); k a multiple of 256
 dfl_status launch_tm_small_matmul(cudaStream_t st, const float* w, const float* xn, int ld_xn, int n_rows, int rows_pad, uint64_t k, int n_out,
                                   const float* sumsq, int n_sumsq, float norm_k, float eps, float* out, int ld_out);
 

@@ -1,7 +1,11 @@
 // Element-wise, convolution and recurrence kernels of the many-row prompt pass (see prompt.cuh).
+#include <cooperative_groups.h>
+
 #include "prompt.cuh"
 
 namespace dfl {
+
+namespace cg = cooperative_groups;
 
 // Eight consecutive columns k8 .. k8 + 7 (k8 % 8 == 0, inside one 256-column block) of token t of a 128-token tile -> the
 // hi / lo planes of the activation chunk: one 16-byte store each, eight tokens fill 128 contiguous bytes.
@@ -128,59 +132,70 @@ dfl_status launch_tm_glue(cudaStream_t st, const TmGlue& p, uint64_t k) {
 }
 
 // ---- small f32 projections ----------------------------------------------------------------------
-// CTA = 16 rows x 16 outputs x the whole k: 256 threads split k (thread = 16 column lanes x 16 (row, output) sub-tiles of 4 x 4),
-// so that the few outputs of alpha / beta still give rows / 16 * n_out / 16 CTAs.  k-slices of a sub-tile are added in lane order.
-__global__ void __launch_bounds__(256) tm_small_matmul_kernel(const float* __restrict__ w, const float* xn, int ld_xn, int n_rows, int rows_pad,
-                                                              int k, int n_out, const float* sumsq, int n_sumsq, float norm_k, float eps,
-                                                              float* out, int ld_out) {
+// Cluster of four CTAs = 32 rows x 32 outputs, a quarter of k each; 256 threads = sixteen 8 x 8 tiles (4 row groups x 4 output
+// groups) of sixteen k-lanes.  Straight from L1 without staging: an 8 x 8 tile reads 16 bytes per 64 multiply-adds, which
+// keeps the load unit and the multiply-add pipe about even.  Lanes, then the four quarters, are added in a fixed order.
+__global__ void __cluster_dims__(1, 1, 4) __launch_bounds__(256)
+tm_small_matmul_kernel(const float* __restrict__ w, const float* xn, int ld_xn, int n_rows, int rows_pad, int k, int n_out, const float* sumsq,
+                       int n_sumsq, float norm_k, float eps, float* out, int ld_out) {
+    __shared__ float part[32][33];
+    cg::cluster_group cluster = cg::this_cluster();
     pdl_prologue();
-    const int r0 = blockIdx.x * 16 + (threadIdx.x >> 6) * 4, o0 = blockIdx.y * 16 + ((threadIdx.x >> 4) & 3) * 4, kl = threadIdx.x & 15;
-    float acc[4][4] = {};
-    const float* xp[4];
-    const float* wp[4];
+    const int r0 = blockIdx.x * 32, o0 = blockIdx.y * 32, kq = k / 4, k0 = blockIdx.z * kq;
+    const int rg = (threadIdx.x >> 6) * 8, og = ((threadIdx.x >> 4) & 3) * 8, kl = threadIdx.x & 15;
+    float acc[64];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        xp[i] = xn + (uint64_t)min(r0 + i, n_rows - 1) * ld_xn + kl * 4;
-        wp[i] = w + (uint64_t)min(o0 + i, n_out - 1) * k + kl * 4;
+    for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+    uint32_t xo[8], wo[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        xo[i] = (uint32_t)min(r0 + rg + i, n_rows - 1) * ld_xn + k0 + kl * 4;
+        wo[i] = (uint32_t)min(o0 + og + i, n_out - 1) * k + k0 + kl * 4;
     }
-    for (int c = 0; c < k; c += 64) {
-        if (c + kl * 4 >= k) break;
-        float4 xv[4], wv[4];
+    for (int c = 0; c < kq; c += 64) {
+        float4 xv[8], wv[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            xv[i] = *reinterpret_cast<const float4*>(xp[i] + c);
-            wv[i] = *reinterpret_cast<const float4*>(wp[i] + c);
+        for (int i = 0; i < 8; ++i) {
+            xv[i] = *reinterpret_cast<const float4*>(xn + xo[i] + c);
+            wv[i] = *reinterpret_cast<const float4*>(w + wo[i] + c);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(wv[j].w, xv[i].w, fmaf(wv[j].z, xv[i].z, fmaf(wv[j].y, xv[i].y, fmaf(wv[j].x, xv[i].x, acc[i][j]))));
+            for (int j = 0; j < 8; ++j)
+                acc[8 * i + j] = fmaf(wv[j].w, xv[i].w, fmaf(wv[j].z, xv[i].z, fmaf(wv[j].y, xv[i].y, fmaf(wv[j].x, xv[i].x, acc[8 * i + j]))));
+    }
+    // lane kl keeps entries 4 kl .. 4 kl + 3 of the tile
+#pragma unroll
+    for (int n = 32; n >= 4; n >>= 1) {
+        const bool up = kl & (n / 4);
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float give = up ? acc[i] : acc[i + n], keep = up ? acc[i + n] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, n / 4);
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) part[rg + ((4 * kl + i) >> 3)][og + ((4 * kl + i) & 7)] = acc[i];
+    cluster.sync();
+    {
+        const int r = 8 * (int)cluster.block_rank() + (threadIdx.x >> 5), o = threadIdx.x & 31, row = r0 + r;
+        float v = 0.f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], o);
-    // lane kl of the sub-tile finishes (row kl >> 2, output kl & 3)
-    float v = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (kl == 4 * i + j) v = acc[i][j];
-    const int row = r0 + (kl >> 2), col = o0 + (kl & 3);
-    if (row < n_rows && col < n_out) {
-        float ss = 0.f;
-        for (int q = 0; q < n_sumsq; ++q) ss += sumsq[(uint64_t)q * rows_pad + row];
-        out[(uint64_t)row * ld_out + col] = v * (1.0f / sqrtf(ss / norm_k + eps));
+        for (unsigned q = 0; q < 4; ++q) v += *cluster.map_shared_rank(&part[r][o], q);
+        if (row < n_rows && o0 + o < n_out) {
+            float ss = 0.f;
+            for (int q = 0; q < n_sumsq; ++q) ss += sumsq[(uint64_t)q * rows_pad + row];
+            out[(uint64_t)row * ld_out + o0 + o] = v * (1.0f / sqrtf(ss / norm_k + eps));
+        }
     }
+    cluster.sync();   // nobody leaves while its part is being read
 }
 
 dfl_status launch_tm_small_matmul(cudaStream_t st, const float* w, const float* xn, int ld_xn, int n_rows, int rows_pad, uint64_t k, int n_out,
                                   const float* sumsq, int n_sumsq, float norm_k, float eps, float* out, int ld_out) {
-    if (k % 4) return fail(DFL_ERR_BAD_SHAPE, "tm_small_matmul: k must be a multiple of 4");
-    launch_k(tm_small_matmul_kernel, dim3((unsigned)((n_rows + 15) / 16), (unsigned)((n_out + 15) / 16)), dim3(256), 0, st, w, xn, ld_xn, n_rows,
+    if (k % 256) return fail(DFL_ERR_BAD_SHAPE, "tm_small_matmul: k must be a multiple of 256");
+    launch_k(tm_small_matmul_kernel, dim3((unsigned)((n_rows + 31) / 32), (unsigned)((n_out + 31) / 32), 4), dim3(256), 0, st, w, xn, ld_xn, n_rows,
              rows_pad, (int)k, n_out, sumsq, n_sumsq, norm_k, eps, out, ld_out);
     count_launch();
     DFL_CUDA(cudaGetLastError());
@@ -281,12 +296,16 @@ dfl_status launch_tm_gdn_front(cudaStream_t st, const TmGdn& p) {
 //     o_i = G_i w_i + sum_{j <= i} D_ij (k_j . q_i) c_j,   S = G_15 S0 + sum_j D_15,j c_j k_j^T,
 // all in f32 and without a division.  A token-by-token scan waits twice per token for a three-level shuffle sum (512 tokens:
 // 242 us a layer); here a block's 32 sums are in flight together and only the 16-step substitution is serial, in registers.
-// grid (n_v, 4 quarters of the value channels), 256 threads: a warp owns four state rows, eight lanes a row, sixteen key
-// channels a lane.  The next block's rows travel with cp.async.
+// grid (n_v, 4 quarters of the value channels), 256 threads: a warp owns four state rows and a lane four key channels of each,
+// so that one 16-byte load of a k or q row serves all four (with eight lanes a row the kernel was bound by shared-memory
+// bandwidth at the token scan's time).  The sums over the lanes halve the values they carry at every step; a lane keeps its
+// rows and tokens in an order rotated by its own number, so that what it passes on is always the upper half and no
+// select is needed.  Lane 8 r + l ends up with tokens 2 l, 2 l + 1 of row r.  The next block's rows travel with cp.async.
 constexpr int SCAN_BLK = 16;
 struct ScanSmem {
     float qs[2][SCAN_BLK][128], ks[2][SCAN_BLK][128], vs[2][SCAN_BLK][32];
     float L[SCAN_BLK][SCAN_BLK + 4], M[SCAN_BLK][SCAN_BLK + 4];   // L[j][i] (column major: one step of the substitution reads a column), M[i][j]
+    float C[32][SCAN_BLK + 4];   // c_j D_15,j of every state row
     float gs[2][SCAN_BLK], bs[2][SCAN_BLK], G[SCAN_BLK], D[SCAN_BLK];
 };
 __global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
@@ -295,15 +314,15 @@ __global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
     const GdnGeom& g = p.g;
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rr = lane >> 3, lg = lane & 7, hk = h % g.n_k;
-    const int dv_cta = blockIdx.y * 32, dv_l = warp * 4 + rr, dv = dv_cta + dv_l;
+    const int dv_cta = blockIdx.y * 32, dv_l = warp * 4 + rr, dv = dv_cta + dv_l;   // the row whose tokens this lane finishes
     const float dtb = p.dt_bias[h], alog = p.a_log[h];
     pdl_prologue();
-    float S[16];
-    const uint64_t s_off = ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
+    float S[4][4];   // S[r]: row r ^ rr of the warp's four, key channels 4 lane .. + 3
+    const uint64_t s_off = ((uint64_t)h * 128 + dv_cta + warp * 4) * 128 + 4 * lane;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float4 s4 = __ldcg(reinterpret_cast<const float4*>(p.state_in + s_off + 32 * j));
-        S[4 * j] = s4.x; S[4 * j + 1] = s4.y; S[4 * j + 2] = s4.z; S[4 * j + 3] = s4.w;
+    for (int r = 0; r < 4; ++r) {
+        const float4 s4 = __ldcg(reinterpret_cast<const float4*>(p.state_in + s_off + (r ^ rr) * 128));
+        S[r][0] = s4.x; S[r][1] = s4.y; S[r][2] = s4.z; S[r][3] = s4.w;
     }
     auto cp16 = [](void* dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); };
     // block boundaries: multiples of 16 from the start, and the first row of the part a rollback may undo
@@ -350,7 +369,23 @@ __global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
     };
     auto put = [&](float* dst) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(dst + s_off + 32 * j) = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+        for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + s_off + (r ^ rr) * 128) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
+    };
+    // dot products of the four rows with the block's sixteen rows of `src`, summed over the lanes: tokens 2 lg and 2 lg + 1 of row rr
+    auto dots = [&](const float (*src)[128], float& d0, float& d1) {
+        float v[64];   // [row slot][token slot]; token slot t is token t ^ 2 lg
+#pragma unroll
+        for (int t = 0; t < SCAN_BLK; ++t) {
+            const float4 x = *reinterpret_cast<const float4*>(&src[t ^ (2 * lg)][4 * lane]);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) v[16 * r + t] = fmaf(S[r][3], x.w, fmaf(S[r][2], x.z, fmaf(S[r][1], x.y, S[r][0] * x.x)));
+        }
+#pragma unroll
+        for (int n = 32; n >= 2; n >>= 1) {
+#pragma unroll
+            for (int i = 0; i < n; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i + n], n / 2);
+        }
+        d0 = v[0]; d1 = v[1];
     };
     // the conv state the front kernel could not write in place; one slice per CTA
     {
@@ -373,87 +408,89 @@ __global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        // ---- the block's Gram matrices and decays: warp w takes rows i = 2 w, 2 w + 1; lane = (j = lane & 15, k or q by lane >> 4)
+        // ---- the block's Gram matrices and decays: a thread computes a 4 x 4 tile of K K^T or Q K^T over sixteen of the 128 channels,
+        // eight lanes share a tile (the eight warps: 2 matrices x 16 tiles)
         {
-            const int j = lane & 15;
-            const float(*src)[128] = lane < 16 ? sm.ks[buf] : sm.qs[buf];
+            const int tile = threadIdx.x >> 3, i0 = ((tile >> 2) & 3) * 4, j0 = (tile & 3) * 4;
+            const bool is_m = tile >= 16;
+            if (j0 <= i0) {   // uniform over the tile's eight lanes
+                const float(*ri)[128] = is_m ? sm.qs[buf] : sm.ks[buf];
+                float acc[16];
 #pragma unroll
-            for (int ii = 0; ii < 2; ++ii) {
-                const int i = 2 * warp + ii;
-                float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                // columns rotated by lane so that the sixteen rows j fall on different banks
-#pragma unroll 8
-                for (int c = 0; c < 32; ++c) {
-                    const int d = ((c + j) & 31) * 4;
-                    const float4 a = *reinterpret_cast<const float4*>(&sm.ks[buf][j][d]);
-                    const float4 b = *reinterpret_cast<const float4*>(&src[i][d]);
-                    acc[0] = fmaf(a.x, b.x, acc[0]); acc[1] = fmaf(a.y, b.y, acc[1]);
-                    acc[2] = fmaf(a.z, b.z, acc[2]); acc[3] = fmaf(a.w, b.w, acc[3]);
+                for (int x = 0; x < 16; ++x) acc[x] = 0.f;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float4 a[4], b[4];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        a[x] = *reinterpret_cast<const float4*>(&ri[i0 + x][32 * c + 4 * lg]);
+                        b[x] = *reinterpret_cast<const float4*>(&sm.ks[buf][j0 + x][32 * c + 4 * lg]);
+                    }
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+#pragma unroll
+                        for (int y = 0; y < 4; ++y)
+                            acc[4 * x + y] = fmaf(a[x].w, b[y].w, fmaf(a[x].z, b[y].z, fmaf(a[x].y, b[y].y, fmaf(a[x].x, b[y].x, acc[4 * x + y]))));
                 }
-                const float dot = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-                float dec = 1.f;   // D_ij
-                for (int t = 1; t < SCAN_BLK; ++t) dec *= (t > j && t <= i) ? sm.gs[buf][t] : 1.f;
-                if (lane < 16) sm.L[j][i] = j < i ? sm.bs[buf][i] * dec * dot : 0.f;
-                else sm.M[i][j] = j <= i ? dec * dot : 0.f;
-                if (lane < 16 && i == SCAN_BLK - 1) sm.D[j] = dec;
-                if (lane == 0) {
-                    float gg = 1.f;
-                    for (int t = 0; t <= i; ++t) gg *= sm.gs[buf][t];
-                    sm.G[i] = gg;
+                const uint32_t mask = 0xffu << (lane & 24);
+#pragma unroll
+                for (int n = 8; n >= 2; n >>= 1) {   // lane lg keeps entries 2 lg, 2 lg + 1
+                    const bool up = lg & (n / 2);
+#pragma unroll
+                    for (int x = 0; x < n; ++x) {
+                        const float give = up ? acc[x] : acc[x + n], keep = up ? acc[x + n] : acc[x];
+                        acc[x] = keep + __shfl_xor_sync(mask, give, n / 2);
+                    }
                 }
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int e = 2 * lg + x, i = i0 + (e >> 2), j = j0 + (e & 3);
+                    float dec = 1.f;   // D_ij
+#pragma unroll
+                    for (int t = 1; t < SCAN_BLK; ++t) dec *= (t > j && t <= i) ? sm.gs[buf][t] : 1.f;
+                    if (is_m) sm.M[i][j] = j <= i ? dec * acc[x] : 0.f;
+                    else sm.L[j][i] = j < i ? sm.bs[buf][i] * dec * acc[x] : 0.f;
+                }
+            } else if (is_m) {   // above the diagonal
+                sm.M[i0 + (lg >> 1)][j0 + 2 * (lg & 1)] = 0.f;
+                sm.M[i0 + (lg >> 1)][j0 + 2 * (lg & 1) + 1] = 0.f;
+            }
+            if (threadIdx.x >= 256 - 32) {   // G_i and D_15,i
+                const int i = lane & 15;
+                float v = 1.f;
+#pragma unroll
+                for (int t = 0; t < SCAN_BLK; ++t) v *= (lane < 16 ? t <= i : t > i) ? sm.gs[buf][t] : 1.f;
+                (lane < 16 ? sm.G : sm.D)[i] = v;
             }
         }
-        // ---- u = S0 k, w = S0 q for the row's sixteen tokens
-        float u[SCAN_BLK], w[SCAN_BLK];
-#pragma unroll
-        for (int i = 0; i < SCAN_BLK; ++i) {
-            float pk[4], pq[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float4 k4 = *reinterpret_cast<const float4*>(&sm.ks[buf][i][32 * j + 4 * lg]);
-                const float4 q4 = *reinterpret_cast<const float4*>(&sm.qs[buf][i][32 * j + 4 * lg]);
-                pk[j] = fmaf(S[4 * j + 3], k4.w, fmaf(S[4 * j + 2], k4.z, fmaf(S[4 * j + 1], k4.y, S[4 * j] * k4.x)));
-                pq[j] = fmaf(S[4 * j + 3], q4.w, fmaf(S[4 * j + 2], q4.z, fmaf(S[4 * j + 1], q4.y, S[4 * j] * q4.x)));
-            }
-            u[i] = (pk[0] + pk[1]) + (pk[2] + pk[3]);
-            w[i] = (pq[0] + pq[1]) + (pq[2] + pq[3]);
-        }
-#pragma unroll
-        for (int of = 4; of > 0; of >>= 1) {
-#pragma unroll
-            for (int i = 0; i < SCAN_BLK; ++i) u[i] += __shfl_xor_sync(0xffffffffu, u[i], of);
-        }
-        // w: lane lg keeps tokens 2 lg, 2 lg + 1 (halving: each step exchanges the half the partner keeps)
-#pragma unroll
-        for (int of = 4; of > 0; of >>= 1) {
-            const bool up = lg & of;
-#pragma unroll
-            for (int i = 0; i < 2 * of; ++i) {
-                const float give = up ? w[i] : w[i + 2 * of], keep = up ? w[i + 2 * of] : w[i];
-                w[i] = keep + __shfl_xor_sync(0xffffffffu, give, of);
-            }
-        }
+        // ---- u = S0 k, w = S0 q
+        float u01[2], w01[2];
+        dots(sm.ks[buf], u01[0], u01[1]);
+        dots(sm.qs[buf], w01[0], w01[1]);
         __syncthreads();   // L, M, G, D
-        // ---- substitution: u becomes c
+        // ---- substitution, by all eight lanes of a row alike: u becomes c
+        float u[SCAN_BLK];
+#pragma unroll
+        for (int i = 0; i < SCAN_BLK; ++i) u[i] = __shfl_sync(0xffffffffu, u01[i & 1], 8 * rr + (i >> 1));
 #pragma unroll
         for (int i = 0; i < SCAN_BLK; ++i) u[i] = sm.bs[buf][i] * (sm.vs[buf][i][dv_l] - sm.G[i] * u[i]);
 #pragma unroll
         for (int j = 0; j < SCAN_BLK - 1; ++j) {
 #pragma unroll
             for (int i4 = (j + 1) / 4; i4 < 4; ++i4) {
-                const float4 l = *reinterpret_cast<const float4*>(&sm.L[j][4 * i4]);   // zero for i <= j
+                const float4 l = *reinterpret_cast<const float4*>(&sm.L[j][4 * i4]);
                 if (4 * i4 > j) u[4 * i4] = fmaf(-l.x, u[j], u[4 * i4]);
                 if (4 * i4 + 1 > j) u[4 * i4 + 1] = fmaf(-l.y, u[j], u[4 * i4 + 1]);
                 if (4 * i4 + 2 > j) u[4 * i4 + 2] = fmaf(-l.z, u[j], u[4 * i4 + 2]);
                 if (4 * i4 + 3 > j) u[4 * i4 + 3] = fmaf(-l.w, u[j], u[4 * i4 + 3]);
             }
         }
-        // ---- outputs of tokens 2 lg, 2 lg + 1
+        // ---- outputs of tokens 2 lg, 2 lg + 1; c for the state
         float* o_row = p.o + (uint64_t)r0 * g.n_v * 128 + h * 128 + dv;
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
             const int i = 2 * lg + t;
-            float o0 = sm.G[i] * w[t], o1 = 0.f;
+            float o0 = sm.G[i] * w01[t], o1 = 0.f;
 #pragma unroll
             for (int j4 = 0; j4 < 4; ++j4) {
                 const float4 m = *reinterpret_cast<const float4*>(&sm.M[i][4 * j4]);
@@ -462,18 +499,34 @@ __global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
             }
             if (i < n) o_row[(uint64_t)i * g.n_v * 128] = o0 + o1;
         }
+        if (lg == 0) {
+#pragma unroll
+            for (int j4 = 0; j4 < 4; ++j4) {
+                const float4 d = *reinterpret_cast<const float4*>(&sm.D[4 * j4]);
+                *reinterpret_cast<float4*>(&sm.C[dv_l][4 * j4]) = make_float4(u[4 * j4] * d.x, u[4 * j4 + 1] * d.y, u[4 * j4 + 2] * d.z, u[4 * j4 + 3] * d.w);
+            }
+        }
+        __syncwarp();
         // ---- state
         const float Gend = sm.G[SCAN_BLK - 1];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) S[e] *= Gend;
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int i = 0; i < SCAN_BLK; ++i) {
-            const float c = u[i] * sm.D[i];
+            for (int e = 0; e < 4; ++e) S[r][e] *= Gend;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float4 k4 = *reinterpret_cast<const float4*>(&sm.ks[buf][i][32 * j + 4 * lg]);
-                S[4 * j] = fmaf(c, k4.x, S[4 * j]); S[4 * j + 1] = fmaf(c, k4.y, S[4 * j + 1]);
-                S[4 * j + 2] = fmaf(c, k4.z, S[4 * j + 2]); S[4 * j + 3] = fmaf(c, k4.w, S[4 * j + 3]);
+        for (int i4 = 0; i4 < 4; ++i4) {
+            float4 k4[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) k4[t] = *reinterpret_cast<const float4*>(&sm.ks[buf][4 * i4 + t][4 * lane]);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float4 c4 = *reinterpret_cast<const float4*>(&sm.C[warp * 4 + (r ^ rr)][4 * i4]);
+                const float c[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    S[r][0] = fmaf(c[t], k4[t].x, S[r][0]); S[r][1] = fmaf(c[t], k4[t].y, S[r][1]);
+                    S[r][2] = fmaf(c[t], k4[t].z, S[r][2]); S[r][3] = fmaf(c[t], k4[t].w, S[r][3]);
+                }
             }
         }
         r0 = r1;
