@@ -2,7 +2,7 @@
 //
 // Same weights, same arithmetic class as the few-row kernel: weights stay the integers q * sc (exact in f16), activations
 // are f16 hi + lo, products accumulate in f32 and the super-block scale d is applied in f32 after every 256 columns.
-// What changes is the ratio: one unpacked 128 x 256 weight tile is multiplied with 128 tokens instead of 16, so that the
+// What changes is the ratio: one unpacked 128 x 256 weight tile is multiplied with up to 128 tokens instead of 16, so that the
 // tensor pipe, not the unpack, is what a CTA spends its time on.  Per 256-column block (1 CTA per SM):
 //   * MMA: 16 k-steps x {hi, lo} of M 128 N 128 K 16 (64 clocks each) = 2048 clocks, plus two for the K-quant min term;
 //     Q6_K: q * sc needs up to 13 bits, A1 = fl16(q * sc) and A2 = q * sc - A1 in {-1, 0, 1}; A1 x {hi, lo} + A2 x hi
@@ -36,7 +36,7 @@ struct TmParams {
     const float* sumsq;       // [n_sumsq][rows_pad]
     int n_sumsq;
     float norm_k, eps, out_scale;
-    int kblocks, splits, row_tiles, tok_tiles, n_rows, rows_pad;
+    int kblocks, splits, row_tiles, tok_tiles, tile_tok, n_rows, rows_pad;   // tile_tok: tokens per tile, a multiple of 16 up to 128
     uint32_t n_out, ld_out;
     int* err;
 };
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         // ------------------------------ MMA issue ------------------------------
         // All tensor-memory addresses are literals (the CTA owns all 512 columns, so the allocation starts at 0) and a
         // block's four activation stages are the ring's four slots, so that the issuing warp spends its slots on MMAs.
-        constexpr uint32_t IDESC = instr_desc(TM_TOK);
+        const uint32_t IDESC = instr_desc(p.tile_tok);
         static_assert(TM_B_STAGES == 4, "stage q of every block is ring slot q");
         const uint32_t b_addr = smem_u32(b_ring), am_addr = smem_u32(smem + T::OFF_AM), s_addr = smem_u32(smem + T::OFF_S);
         uint32_t e = 0;
@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         // ------------------------------ read-back ------------------------------
         pdl_wait();
         const int row = (threadIdx.x - DRAIN_WARP0 * 32) & 127;   // weight row of the tile = tensor-memory lane
-        const int half = (warp - DRAIN_WARP0) >> 2;                // tokens 64 half .. + 63
+        const int half = (warp - DRAIN_WARP0) >> 2, n_c = p.tile_tok / 16;   // the first or the second half of the tile's 16-token columns
+        const int c0 = half ? (n_c + 1) / 2 : 0, c1 = half ? n_c : (n_c + 1) / 2;
         const uint32_t tm_l = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
         uint32_t e = 0;
         int scaled_tt = -1;
@@ -310,8 +311,8 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 scaled_tt = it.tt;
                 named_sync(1, TM_DRAIN_WARPS * 32);
                 float ss = 0.f;
-                if (p.sumsq && half == 0)
-                    for (int q = 0; q < p.n_sumsq; ++q) ss += p.sumsq[(uint64_t)q * p.rows_pad + it.tt * TM_TOK + row];
+                if (p.sumsq && half == 0 && row < p.tile_tok)
+                    for (int q = 0; q < p.n_sumsq; ++q) ss += p.sumsq[(uint64_t)q * p.rows_pad + it.tt * p.tile_tok + row];
                 if (half == 0) tok_scale[row] = p.sumsq ? p.out_scale * (1.0f / sqrtf(ss / p.norm_k + p.eps)) : p.out_scale;
                 named_sync(1, TM_DRAIN_WARPS * 32);
             }
@@ -323,17 +324,19 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 const uint32_t d = tm_l + TM2_D + (e & 1) * 128;
                 const bool last = k == it.n_kb - 1;
                 const uint32_t orow = (uint32_t)it.rt * TILE_R + row;
+                auto release = [&] {
+                    fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&d_free[e & 1]);
+                };
+                if (c0 == c1) release();
 #pragma unroll 1
-                for (int c = 4 * half; c < 4 * half + 4; ++c) {   // 16 tokens
+                for (int c = c0; c < c1; ++c) {   // 16 tokens
                     float v[16], a[16];
                     tmem_ld16(d + 16 * c, v);
                     if (k > 0) tmem_ld16(tm_l + TM2_ACC + 16 * c, a);
                     wait_ld();
-                    if (c == 4 * half + 3) {
-                        fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&d_free[e & 1]);
-                    }
+                    if (c == c1 - 1) release();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = k > 0 ? fmaf(s, v[j], a[j]) : s * v[j];
                     if (!last) {
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                         for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(v[j]);
                         tmem_st16(tm_l + TM2_ACC + 16 * c, u);
                     } else if (orow < p.n_out) {
-                        const int tok0 = it.tt * TM_TOK + 16 * c;
+                        const int tok0 = it.tt * p.tile_tok + 16 * c;
                         float* dst = p.out + ((uint64_t)it.sp * p.rows_pad + tok0) * p.ld_out + orow;
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
@@ -392,6 +395,12 @@ static dfl_status launch_tm(cudaStream_t st, const TmParams& p) {
 
 }  // namespace ts
 
+// Tokens per tile of a pass: as few tiles as possible, of equal size (the time of a block follows the tile's tokens).
+int gemm_tm_tile_tok(int n_rows) {
+    const int tiles = (n_rows + TM_TOK - 1) / TM_TOK;
+    return ((n_rows + tiles - 1) / tiles + 15) / 16 * 16;
+}
+
 // Split count of a many-row launch: waves of items times blocks per item (an item pays about a third of a block to start
 // and to end), plus the traffic of the partial slices (64 KiB per item written and read again, in units of a block's time).
 int gemm_tm_choose_splits(const int* row_tiles, int n_mats, int kblocks, int tok_tiles) {
@@ -413,14 +422,15 @@ bool gemm_tm_supported(const QMatrix& m) {
     return m.layout == LAYOUT_TS && (m.dtype == DFL_Q4_K || m.dtype == DFL_Q5_K || m.dtype == DFL_Q6_K);
 }
 
-dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_rows, int rows_pad,
+dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_rows, int tile_tok,
                           const float* sumsq, int n_sumsq, float norm_k, float eps, float out_scale, uint32_t ld_out, int* dev_err) {
     if (!gemm_tm_supported(m)) return fail(DFL_ERR_UNSUPPORTED, "many-row gemm: weight dtype");
-    if (splits < 1 || splits > m.kblocks || n_rows < 1 || rows_pad % TM_TOK || n_rows > rows_pad) return fail(DFL_ERR_BAD_ARG, "many-row gemm: shape");
+    if (splits < 1 || splits > m.kblocks || n_rows < 1 || tile_tok < 16 || tile_tok > TM_TOK || tile_tok % 16)
+        return fail(DFL_ERR_BAD_ARG, "many-row gemm: shape");
     ts::TmParams p;
     p.w = m.tiles; p.acts = acts; p.out = out; p.sumsq = sumsq; p.n_sumsq = n_sumsq; p.norm_k = norm_k; p.eps = eps; p.out_scale = out_scale;
-    p.kblocks = m.kblocks; p.splits = splits; p.row_tiles = m.row_tiles; p.tok_tiles = (n_rows + TM_TOK - 1) / TM_TOK;
-    p.n_rows = n_rows; p.rows_pad = rows_pad; p.n_out = (uint32_t)m.n_out; p.ld_out = ld_out ? ld_out : (uint32_t)m.n_out; p.err = dev_err;
+    p.kblocks = m.kblocks; p.splits = splits; p.row_tiles = m.row_tiles; p.tile_tok = tile_tok; p.tok_tiles = (n_rows + tile_tok - 1) / tile_tok;
+    p.n_rows = n_rows; p.rows_pad = p.tok_tiles * tile_tok; p.n_out = (uint32_t)m.n_out; p.ld_out = ld_out ? ld_out : (uint32_t)m.n_out; p.err = dev_err;
     switch (m.dtype) {
         case DFL_Q4_K: return ts::launch_tm<DFL_Q4_K>(st, p);
         case DFL_Q5_K: return ts::launch_tm<DFL_Q5_K>(st, p);

@@ -116,8 +116,9 @@ dfl_status launch_gemm_ts(cudaStream_t st, const QMatrix& m, const uint8_t* acts
                           int* dev_err, bool pdl, uint32_t ld_out);
 bool gemm_tm_supported(const QMatrix& m);
 int gemm_tm_choose_splits(const int* row_tiles, int n_mats, int kblocks, int tok_tiles);
-// out [splits][rows_pad][ld_out] (rows beyond n_rows are not written); rows_pad a multiple of 128
-dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_rows, int rows_pad,
+// tile_tok tokens per tile (gemm_tm_tile_tok); out [splits][rows_pad][ld_out], rows_pad = tiles x tile_tok (rows beyond n_rows are not written)
+int gemm_tm_tile_tok(int n_rows);
+dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_rows, int tile_tok,
                           const float* sumsq, int n_sumsq, float norm_k, float eps, float out_scale, uint32_t ld_out, int* dev_err);
 int gemm_ts_choose_splits(const QMatrix& m);
 int gemm_ts_choose_splits_multi(const int* row_tiles, int n_mats, int kblocks);

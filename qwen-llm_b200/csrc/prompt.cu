@@ -15,14 +15,14 @@ struct PromptWs {
     uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_v = nullptr;
     int32_t* tokens = nullptr;
     int32_t* pinned = nullptr;
-    std::vector<void*> allocs;
+    uint8_t* base = nullptr;
 };
 
 const float* prompt_capture(const dfl_scratch* sc) { return sc->prompt->capture; }
 
 void prompt_ws_free(PromptWs* w) {
     if (!w) return;
-    for (void* p : w->allocs) pool_free(p);
+    pool_free(w->base);
     pool_free(w->pinned);
     delete w;
 }
@@ -68,34 +68,37 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
         for (auto& L : m->layers)
             for (const MatGroup* g : {&L.qkv, &L.wo, &L.in_qkv_z, &L.w_out, &L.gate_up, &L.down})
                 if (!g->mats.empty()) part = std::max<uint64_t>(part, (uint64_t)tm_splits(*g, t) * t * TM_TOK * g->total_cols);
-    bool ok = true;
+    // one block for all of it: sizes first, then the pointers
+    uint64_t total = 0;
     auto alloc = [&](auto** p, uint64_t bytes) {
-        void* q = ok ? pool_alloc(bytes ? bytes : 16) : nullptr;
-        ok = q != nullptr;
-        if (q) w->allocs.push_back(q);
-        *p = reinterpret_cast<std::remove_reference_t<decltype(**p)>*>(q);
+        if (w->base) *p = reinterpret_cast<std::remove_reference_t<decltype(**p)>*>(w->base + total);
+        total += (bytes + 255) / 256 * 256;
     };
-    const uint64_t tiles = rows / TM_TOK;
-    alloc(&w->x, R * H * 4);
-    alloc(&w->xn, R * H * 4);
-    alloc(&w->part, part * 4);
-    alloc(&w->sumsq, H / TILE_K * R * 4);
-    alloc(&w->q_rot, R * q_dim * 4);
-    alloc(&w->gate, R * q_dim * 4);
-    alloc(&w->o, R * wide * 4);
-    if (m->n_attn) alloc(&w->attn_part, attn_rows_partials_floats(m->attn_geom(), (int)rows) * 4);
-    alloc(&w->q_n, R * gg.n_k * 128 * 4);
-    alloc(&w->k_n, R * gg.n_k * 128 * 4);
-    alloc(&w->v, R * v_dim * 4);
-    alloc(&w->ab, R * 2 * gg.n_v * 4);
-    alloc(&w->conv_new, 3ull * gg.conv_dim() * 4);
-    alloc(&w->capture, R * sc->k_layers * H * 4);
-    alloc(&w->acts_h, tiles * (H / TILE_K) * TM_CHUNK);
-    alloc(&w->acts_f, tiles * (F / TILE_K) * TM_CHUNK);
-    alloc(&w->acts_v, tiles * (wide / TILE_K) * TM_CHUNK);
-    alloc(&w->tokens, R * 4);
-    ok = ok && (w->pinned = (int32_t*)pool_alloc_host(R * 4));
-    if (!ok) {
+    for (int pass = 0; pass < 2; ++pass) {
+        total = 0;
+        const uint64_t tiles = rows / TM_TOK;
+        alloc(&w->x, R * H * 4);
+        alloc(&w->xn, R * H * 4);
+        alloc(&w->part, part * 4);
+        alloc(&w->sumsq, H / TILE_K * R * 4);
+        alloc(&w->q_rot, R * q_dim * 4);
+        alloc(&w->gate, R * q_dim * 4);
+        alloc(&w->o, R * wide * 4);
+        if (m->n_attn) alloc(&w->attn_part, attn_rows_partials_floats(m->attn_geom(), (int)rows) * 4);
+        alloc(&w->q_n, R * gg.n_k * 128 * 4);
+        alloc(&w->k_n, R * gg.n_k * 128 * 4);
+        alloc(&w->v, R * v_dim * 4);
+        alloc(&w->ab, R * 2 * gg.n_v * 4);
+        alloc(&w->conv_new, 3ull * gg.conv_dim() * 4);
+        alloc(&w->capture, R * sc->k_layers * H * 4);
+        alloc(&w->acts_h, tiles * (H / TILE_K) * TM_CHUNK);
+        alloc(&w->acts_f, tiles * (F / TILE_K) * TM_CHUNK);
+        alloc(&w->acts_v, tiles * (wide / TILE_K) * TM_CHUNK);
+        alloc(&w->tokens, R * 4);
+        if (pass == 0 && !(w->base = (uint8_t*)pool_alloc(total))) break;
+    }
+    w->pinned = (int32_t*)pool_alloc_host(R * 4);
+    if (!w->base || !w->pinned) {
         std::string why = cudaGetErrorString(cudaGetLastError());
         prompt_ws_free(w);
         return fail(DFL_ERR_OOM, "prompt pass: allocation failed: " + why);
@@ -108,8 +111,8 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
 dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids, const int32_t* tokens,
                        uint32_t n, uint32_t start, uint32_t last_rows, bool want_head) {
     const dfl_arch& a = m->arch;
-    const int rows_pad = (int)((n + TM_TOK - 1) / TM_TOK * TM_TOK), tok_tiles = rows_pad / TM_TOK;
-    DFL_CHECK(ensure_ws(m, sc, (uint32_t)rows_pad));
+    const int tile_tok = gemm_tm_tile_tok((int)n), tok_tiles = (int)((n + tile_tok - 1) / tile_tok), rows_pad = tok_tiles * tile_tok;
+    DFL_CHECK(ensure_ws(m, sc, (uint32_t)(tok_tiles * TM_TOK)));
     PromptWs* w = sc->prompt;
     cudaStream_t st = s->st;
     const uint64_t H = a.hidden_size, F = a.intermediate_size, KH = sc->k_layers * H;
@@ -124,7 +127,7 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
 
     auto glue_base = [&] {
         TmGlue p;
-        p.n_rows = (int)n; p.rows_pad = rows_pad; p.err = s->err;
+        p.n_rows = (int)n; p.rows_pad = rows_pad; p.tile_tok = tile_tok; p.err = s->err;
         return p;
     };
     auto norm_glue = [&](int splits, const float* norm_w, bool want_xn, float* capture) -> dfl_status {
@@ -142,7 +145,7 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
     auto gemm = [&](const MatGroup& g, const uint8_t* acts, bool norm, float out_scale, int* splits) -> dfl_status {
         *splits = tm_splits(g, tok_tiles);
         for (size_t i = 0; i < g.mats.size(); ++i)
-            DFL_CHECK(launch_gemm_tm(st, g.mats[i], acts, w->part + g.col_off[i], *splits, (int)n, rows_pad, norm ? w->sumsq : nullptr,
+            DFL_CHECK(launch_gemm_tm(st, g.mats[i], acts, w->part + g.col_off[i], *splits, (int)n, tile_tok, norm ? w->sumsq : nullptr,
                                      norm ? n_sumsq : 0, (float)H, 1e-6f, out_scale, g.total_cols, s->err));
         return DFL_OK;
     };
@@ -177,7 +180,7 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
                                              2 * gg.n_v));
             const int cur = s->ssm_cur[gi];
             p.part = w->part; p.splits = splits; p.ld_part = (int)L.in_qkv_z.total_cols; p.z_col = gg.conv_dim();
-            p.n_rows = (int)n; p.rows_pad = rows_pad; p.last_rows = (int)last_rows;
+            p.n_rows = (int)n; p.rows_pad = rows_pad; p.tile_tok = tile_tok; p.last_rows = (int)last_rows;
             p.conv_w = L.conv_w; p.ab = w->ab; p.dt_bias = L.dt_bias; p.a_log = L.a_log; p.norm_w = L.ssm_norm_w;
             p.conv_state = s->conv[gi]; p.conv_new = w->conv_new;
             p.state_in = s->ssm[cur][gi]; p.state_out = s->ssm[cur ^ 1][gi];

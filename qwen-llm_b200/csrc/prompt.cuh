@@ -1,6 +1,6 @@
 // Kernels of the many-row (prompt) pass that sit between its GEMMs (prompt_ops.cu): the same steps as the 16-row kernels
 // of glue.cu / gdn.cu over up to a few hundred token rows, packing activations for gemm_tm.cuh.  Rows of a pass are padded to
-// whole tiles of 128 tokens; the packed rows beyond the pass's tokens are zeros.
+// whole tiles of tile_tok tokens; the packed rows beyond the pass's tokens are zeros.
 #pragma once
 #include "model.cuh"
 
@@ -22,7 +22,7 @@ struct TmGlue {
     int ld_capture = 0;
     int swiglu_f = 0;
     const float* gate = nullptr;    // GLUE_COPY: x * sigmoid(gate), gate [rows][ld_x]
-    int n_rows = 0, rows_pad = 0;
+    int n_rows = 0, rows_pad = 0, tile_tok = TM_TOK;   // rows_pad = token tiles x tile_tok
     int* err = nullptr;
 };
 dfl_status launch_tm_glue(cudaStream_t st, const TmGlue& p, uint64_t k);
@@ -35,7 +35,7 @@ struct TmGdn {
     GdnGeom g{};
     const float* part = nullptr;    // [splits][rows_pad][ld_part]: qkv columns first, z columns at z_col
     int splits = 0, ld_part = 0, z_col = 0;
-    int n_rows = 0, rows_pad = 0;
+    int n_rows = 0, rows_pad = 0, tile_tok = TM_TOK;   // rows_pad = token tiles x tile_tok
     int last_rows = 0;              // rows of the pass's last block (what a rollback after the pass can undo); 0: none kept
     const float *conv_w = nullptr, *ab = nullptr, *dt_bias = nullptr, *a_log = nullptr, *norm_w = nullptr;
     float *conv_state = nullptr, *conv_new = nullptr;

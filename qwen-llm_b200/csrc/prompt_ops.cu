@@ -1,6 +1,8 @@
 // Element-wise, convolution and recurrence kernels of the many-row prompt pass (see prompt.cuh).
 #include <cooperative_groups.h>
 
+#include <mutex>
+
 #include "prompt.cuh"
 
 namespace dfl {
@@ -112,19 +114,19 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
     for (int e = 0; e < 8; ++e) v[e] *= p.pre_scale;
     if (p.xn && live) store8(p.xn + (uint64_t)row * p.ld_xn + col, v);
     if (p.acts) {
-        uint8_t* chunk = p.acts + ((uint64_t)(row / TM_TOK) * gridDim.x + blockIdx.x) * TM_CHUNK;
+        uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * TM_CHUNK;
         bool over = false;
-        pack_oct_tm(chunk, row % TM_TOK, k8, v, over);
+        pack_oct_tm(chunk, row % p.tile_tok, k8, v, over);
         float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
         sum += __shfl_xor_sync(0xffffffffu, sum, 8);
         sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-        if (lane < 8) pack_sum_tm(chunk, row % TM_TOK, warp, sum, over);
+        if (lane < 8) pack_sum_tm(chunk, row % p.tile_tok, warp, sum, over);
         if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
     }
 }
 
 dfl_status launch_tm_glue(cudaStream_t st, const TmGlue& p, uint64_t k) {
-    if (k == 0 || k % TILE_K || p.rows_pad % TM_TOK) return fail(DFL_ERR_BAD_SHAPE, "tm_glue: shape");
+    if (k == 0 || k % TILE_K || p.rows_pad % p.tile_tok) return fail(DFL_ERR_BAD_SHAPE, "tm_glue: shape");
     launch_k(tm_glue_kernel, dim3((unsigned)(k / TILE_K), (unsigned)(p.rows_pad / 8)), dim3(256), 0, st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
@@ -133,11 +135,15 @@ dfl_status launch_tm_glue(cudaStream_t st, const TmGlue& p, uint64_t k) {
 
 // ---- small f32 projections ----------------------------------------------------------------------
 // Cluster of four CTAs = 32 rows x 32 outputs, a quarter of k each; 256 threads = sixteen 8 x 8 tiles (4 row groups x 4 output
-// groups) of sixteen k-lanes.  Straight from L1 without staging: an 8 x 8 tile reads 16 bytes per 64 multiply-adds, which
-// keeps the load unit and the multiply-add pipe about even.  Lanes, then the four quarters, are added in a fixed order.
+// groups) of sixteen k-lanes.  64 columns of the 32 + 32 rows travel with cp.async, three stages deep (read straight through L1
+// the rows, a multiple of 4 KiB apart, evict one another: 71 us at 77 rows x 64 outputs); an 8 x 8 tile then reads 16 bytes
+// per 64 multiply-adds, which keeps the load unit and the multiply-add pipe about even.  Lanes, then the four quarters, are
+// added in a fixed order.
+constexpr int SMM_PITCH = 68, SMM_STAGE = 64 * SMM_PITCH, SMM_STAGES = 3;
 __global__ void __cluster_dims__(1, 1, 4) __launch_bounds__(256)
 tm_small_matmul_kernel(const float* __restrict__ w, const float* xn, int ld_xn, int n_rows, int rows_pad, int k, int n_out, const float* sumsq,
                        int n_sumsq, float norm_k, float eps, float* out, int ld_out) {
+    extern __shared__ __align__(16) float smm[];   // [stage][32 x rows, 32 w rows][64 columns]
     __shared__ float part[32][33];
     cg::cluster_group cluster = cg::this_cluster();
     pdl_prologue();
@@ -146,24 +152,36 @@ tm_small_matmul_kernel(const float* __restrict__ w, const float* xn, int ld_xn, 
     float acc[64];
 #pragma unroll
     for (int i = 0; i < 64; ++i) acc[i] = 0.f;
-    uint32_t xo[8], wo[8];
+    const int n_steps = kq / 64;
+    auto fetch = [&](int step) {   // thread = (row of 64, a quarter of its 256 bytes)
+        if (step < n_steps) {
+            const int r = threadIdx.x >> 2, q = (threadIdx.x & 3) * 16;
+            const float* src = (r < 32 ? xn + (uint64_t)min(r0 + r, n_rows - 1) * ld_xn : w + (uint64_t)min(o0 + r - 32, n_out - 1) * k) + k0 + step * 64 + q;
+            float* dst = smm + (step % SMM_STAGES) * SMM_STAGE + r * SMM_PITCH + q;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        xo[i] = (uint32_t)min(r0 + rg + i, n_rows - 1) * ld_xn + k0 + kl * 4;
-        wo[i] = (uint32_t)min(o0 + og + i, n_out - 1) * k + k0 + kl * 4;
-    }
-    for (int c = 0; c < kq; c += 64) {
-        float4 xv[8], wv[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            xv[i] = *reinterpret_cast<const float4*>(xn + xo[i] + c);
-            wv[i] = *reinterpret_cast<const float4*>(w + wo[i] + c);
+            for (int i = 0; i < 4; ++i)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + 4 * i)), "l"(src + 4 * i) : "memory");
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    fetch(1);
+    for (int st = 0; st < n_steps; ++st) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();   // step st has landed for everyone; stage (st + 2) % 3 was consumed in step st - 1
+        fetch(st + 2);
+        const float* xs = smm + (st % SMM_STAGES) * SMM_STAGE + rg * SMM_PITCH + kl * 4;
+        const float* ws = smm + (st % SMM_STAGES) * SMM_STAGE + (32 + og) * SMM_PITCH + kl * 4;
+        float4 xv[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 8; ++i) xv[i] = *reinterpret_cast<const float4*>(xs + i * SMM_PITCH);
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                acc[8 * i + j] = fmaf(wv[j].w, xv[i].w, fmaf(wv[j].z, xv[i].z, fmaf(wv[j].y, xv[i].y, fmaf(wv[j].x, xv[i].x, acc[8 * i + j]))));
+        for (int j = 0; j < 8; ++j) {
+            const float4 wv = *reinterpret_cast<const float4*>(ws + j * SMM_PITCH);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                acc[8 * i + j] = fmaf(wv.w, xv[i].w, fmaf(wv.z, xv[i].z, fmaf(wv.y, xv[i].y, fmaf(wv.x, xv[i].x, acc[8 * i + j]))));
+        }
     }
     // lane kl keeps entries 4 kl .. 4 kl + 3 of the tile
 #pragma unroll
@@ -195,7 +213,14 @@ tm_small_matmul_kernel(const float* __restrict__ w, const float* xn, int ld_xn, 
 dfl_status launch_tm_small_matmul(cudaStream_t st, const float* w, const float* xn, int ld_xn, int n_rows, int rows_pad, uint64_t k, int n_out,
                                   const float* sumsq, int n_sumsq, float norm_k, float eps, float* out, int ld_out) {
     if (k % 256) return fail(DFL_ERR_BAD_SHAPE, "tm_small_matmul: k must be a multiple of 256");
-    launch_k(tm_small_matmul_kernel, dim3((unsigned)((n_rows + 31) / 32), (unsigned)((n_out + 31) / 32), 4), dim3(256), 0, st, w, xn, ld_xn, n_rows,
+    constexpr size_t SMEM = (size_t)SMM_STAGES * SMM_STAGE * sizeof(float);
+    static std::once_flag once[16];
+    int dev = 0;
+    DFL_CUDA(cudaGetDevice(&dev));
+    cudaError_t attr = cudaSuccess;
+    std::call_once(once[dev & 15], [&] { attr = cudaFuncSetAttribute(tm_small_matmul_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM); });
+    DFL_CUDA(attr);
+    launch_k(tm_small_matmul_kernel, dim3((unsigned)((n_rows + 31) / 32), (unsigned)((n_out + 31) / 32), 4), dim3(256), SMEM, st, w, xn, ld_xn, n_rows,
              rows_pad, (int)k, n_out, sumsq, n_sumsq, norm_k, eps, out, ld_out);
     count_launch();
     DFL_CUDA(cudaGetLastError());
@@ -576,13 +601,13 @@ __global__ void __launch_bounds__(256) tm_gdn_pack_kernel(const TmGdn p) {
     add8(nw, p.norm_w + (k8 & 127));
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = live ? v[e] * sc * nw[e] * silu_f(z[e]) : 0.f;
-    uint8_t* chunk = p.acts + ((uint64_t)(row / TM_TOK) * gridDim.x + blockIdx.x) * TM_CHUNK;
+    uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * TM_CHUNK;
     bool over = false;
-    pack_oct_tm(chunk, row % TM_TOK, k8, v, over);
+    pack_oct_tm(chunk, row % p.tile_tok, k8, v, over);
     float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
     sum += __shfl_xor_sync(0xffffffffu, sum, 8);
     sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-    if (lane < 8) pack_sum_tm(chunk, row % TM_TOK, warp, sum, over);
+    if (lane < 8) pack_sum_tm(chunk, row % p.tile_tok, warp, sum, over);
     if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
 }
 
