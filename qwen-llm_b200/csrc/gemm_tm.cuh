@@ -39,18 +39,21 @@ struct TmParams {
     int kblocks, splits, row_tiles, tok_tiles, tile_tok, n_rows, rows_pad;   // tile_tok: tokens per tile, a multiple of 16 up to 128
     uint32_t n_out, ld_out;
     int* err;
+    TmSegments g;             // g.seg != nullptr: segments of gathered rows instead of token tiles
 };
 
-template <int DT>
+template <int DT, int CAP>
 struct TmFmt {
     static constexpr bool MIN = DT != DFL_Q6_K;
     static constexpr int W_STAGE = Fmt<DT>::STAGE;
-    static constexpr int W_STAGES = DT == DFL_Q6_K ? 2 : 3;
+    static constexpr int BSTAGE = tm_bstage(CAP), SUMS = tm_sums(CAP);
+    // weight stages: what the activation ring leaves room for
+    static constexpr int W_STAGES = CAP == TM_TOK ? (DT == DFL_Q6_K ? 2 : 3) : (DT == DFL_Q6_K ? 4 : 6);
     static constexpr int USES = MIN ? 1 : 2;      // how often a block uses each A buffer
-    static constexpr int OFF_W = TM_B_STAGES * TM_BSTAGE;
+    static constexpr int OFF_W = TM_B_STAGES * BSTAGE;
     static constexpr int OFF_AM = OFF_W + W_STAGES * W_STAGE;          // [2] min-term A operand, 128 x 16
     static constexpr int OFF_S = OFF_AM + (MIN ? 2 * 4096 : 0);        // [2] min-term B operand
-    static constexpr int OFF_SCL = OFF_S + (MIN ? 2 * TM_SUMS : 0);    // [4][128] block scales
+    static constexpr int OFF_SCL = OFF_S + (MIN ? 2 * SUMS : 0);    // [4][128] block scales
     static constexpr int OFF_BAR = OFF_SCL + 4 * TILE_R * 4;
     static constexpr int SMEM = OFF_BAR + TM_BAR_BYTES;
 };
@@ -70,9 +73,11 @@ __device__ __forceinline__ TmScale tm_scale(float d, float dmin) {
     return r;
 }
 
-template <int DT>
+template <int DT, int CAP>
 __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p) {
-    using T = TmFmt<DT>;
+    using T = TmFmt<DT, CAP>;
+    constexpr bool SEG = CAP != TM_TOK;
+    static_assert(T::SMEM <= 227 * 1024 && (2 * T::W_STAGES + 2 * TM_B_STAGES + 12) * 8 <= TM_BAR_BYTES, "shared memory budget");
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* b_ring = smem;
     uint8_t* w_ring = smem + T::OFF_W;
@@ -92,7 +97,6 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
     __shared__ int abort_flag;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-    const int n_items = p.row_tiles * p.splits * p.tok_tiles;
     if (threadIdx.x == 0) {
         for (int i = 0; i < T::W_STAGES; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], UNPACK_WARPS); }
         for (int i = 0; i < TM_B_STAGES; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
@@ -115,16 +119,33 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
     pdl_launch_dependents();
 
     // item -> (row tile, split, token tile): the token tiles of one weight tile are neighbours, so that its bytes come from
-    // HBM once and from L2 for the others
-    struct Item { int rt, tt, kb0, n_kb, sp; };
+    // HBM once and from L2 for the others.  Segments: the row tiles of one segment are neighbours, they share its activations.
+    int n_items = p.row_tiles * p.splits * p.tok_tiles;
+    if (SEG) {   // the list comes from the kernel before
+        pdl_wait();
+        const int n = p.g.n_seg ? *p.g.n_seg + p.g.n_more : p.g.max_seg;
+        n_items = (n < p.g.max_seg ? n : p.g.max_seg) * p.g.n_tiles;
+    }
+    struct Item { int rt, tt, kb0, n_kb, sp, rows; };   // weight row tile, token tile or segment, column blocks of the matrix, split, live rows
     auto item_of = [&](int idx) {
         Item it;
+        if (SEG) {
+            it.tt = p.g.first + idx / p.g.n_tiles;
+            it.sp = idx % p.g.n_tiles;   // column tile of the output
+            const int2 s = p.g.seg[it.tt];
+            it.rt = s.x * p.g.tiles_per_block + it.sp + (it.sp >= p.g.half_tiles ? p.g.half_off - p.g.half_tiles : 0);
+            it.kb0 = s.x * p.g.kb_per_block;
+            it.n_kb = p.g.kblocks;
+            it.rows = s.y;
+            return it;
+        }
         it.tt = idx % p.tok_tiles;
         const int r = idx / p.tok_tiles;
         it.sp = r % p.splits;
         it.rt = r / p.splits;
         it.kb0 = (int)((long long)it.sp * p.kblocks / p.splits);
         it.n_kb = (int)((long long)(it.sp + 1) * p.kblocks / p.splits) - it.kb0;
+        it.rows = p.tile_tok;
         return it;
     };
     bool ok = true;
@@ -153,18 +174,18 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
             uint32_t round = 0, e = 0;
             for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
                 const Item it = item_of(idx);
-                const uint8_t* src = p.acts + ((uint64_t)it.tt * p.kblocks + it.kb0) * TM_CHUNK;
-                for (int k = 0; k < it.n_kb && ok; ++k, src += TM_CHUNK, ++e) {
+                const uint8_t* src = p.acts + (SEG ? (uint64_t)it.tt * it.n_kb : (uint64_t)it.tt * p.kblocks + it.kb0) * tm_chunk(CAP);
+                for (int k = 0; k < it.n_kb && ok; ++k, src += tm_chunk(CAP), ++e) {
                     if (T::MIN) {
                         if (e >= 2) ok = mbar_wait_bounded(&s_empty[e & 1], ((e >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
                         if (!ok) break;
-                        mbar_arrive_expect_tx(&s_full[e & 1], TM_SUMS);
-                        bulk_g2s(smem + T::OFF_S + (e & 1) * TM_SUMS, src + 4 * TM_BSTAGE, TM_SUMS, &s_full[e & 1]);
+                        mbar_arrive_expect_tx(&s_full[e & 1], T::SUMS);
+                        bulk_g2s(smem + T::OFF_S + (e & 1) * T::SUMS, src + 4 * T::BSTAGE, T::SUMS, &s_full[e & 1]);
                     }
                     for (int q = 0; q < 4; ++q) {
                         if (round > 0 && !(ok = mbar_wait_bounded(&b_empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY))) break;
-                        mbar_arrive_expect_tx(&b_full[s], TM_BSTAGE);
-                        bulk_g2s(b_ring + s * TM_BSTAGE, src + q * TM_BSTAGE, TM_BSTAGE, &b_full[s]);
+                        mbar_arrive_expect_tx(&b_full[s], T::BSTAGE);
+                        bulk_g2s(b_ring + s * T::BSTAGE, src + q * T::BSTAGE, T::BSTAGE, &b_full[s]);
                         if (++s == TM_B_STAGES) { s = 0; ++round; }
                     }
                 }
@@ -174,7 +195,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         // ------------------------------ MMA issue ------------------------------
         // All tensor-memory addresses are literals (the CTA owns all 512 columns, so the allocation starts at 0) and a
         // block's four activation stages are the ring's four slots, so that the issuing warp spends its slots on MMAs.
-        const uint32_t IDESC = instr_desc(p.tile_tok);
+        uint32_t IDESC = instr_desc(p.tile_tok);
         static_assert(TM_B_STAGES == 4, "stage q of every block is ring slot q");
         const uint32_t b_addr = smem_u32(b_ring), am_addr = smem_u32(smem + T::OFF_AM), s_addr = smem_u32(smem + T::OFF_S);
         uint32_t e = 0;
@@ -193,19 +214,19 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 if (T::MIN && q == 3 && !wait(&s_full[O], (e >> 1) & 1)) return;
                 fence_after_sync();
                 {
-                    const uint64_t bd = smem_desc(b_addr + q * TM_BSTAGE, TM_TOK * 16, 128);
+                    const uint64_t bd = smem_desc(b_addr + q * T::BSTAGE, CAP * 16, 128);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const uint32_t aj = TM2_A + 64 * g + (T::MIN ? 32 * (q & 1) : 0) + 8 * j;
-                        mma_ts_rt(D, aj, bd + j * 256, IDESC, (q | j) != 0);
-                        mma_ts_rt(D, aj, bd + j * 256 + TM_BSTAGE / 32, IDESC, 1u);
-                        if (!T::MIN) mma_ts_rt(D, aj + 32, bd + j * 256, IDESC, 1u);
+                        mma_ts_rt(D, aj, bd + j * (2 * CAP), IDESC, (q | j) != 0);
+                        mma_ts_rt(D, aj, bd + j * (2 * CAP) + T::BSTAGE / 32, IDESC, 1u);
+                        if (!T::MIN) mma_ts_rt(D, aj + 32, bd + j * (2 * CAP), IDESC, 1u);
                     }
                     mma_commit(&b_empty[q]);
                     if (T::MIN && q == 3) {
-                        const uint64_t ad = smem_desc(am_addr + O * 4096, 2048, 128), sd = smem_desc(s_addr + O * TM_SUMS, TM_TOK * 16, 128);
+                        const uint64_t ad = smem_desc(am_addr + O * 4096, 2048, 128), sd = smem_desc(s_addr + O * T::SUMS, CAP * 16, 128);
                         mma_ss(D, ad, sd, IDESC, 1u);
-                        mma_ss(D, ad, sd + TM_SUMS / 32, IDESC, 1u);
+                        mma_ss(D, ad, sd + T::SUMS / 32, IDESC, 1u);
                         mma_commit(&s_empty[O]);
                     }
                     if (!T::MIN || (q & 1)) mma_commit(&a_free[g]);
@@ -219,7 +240,9 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 ok = false;
             }
             for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
-                const int n_kb = item_of(idx).n_kb;
+                const Item it = item_of(idx);
+                const int n_kb = it.n_kb;
+                if (SEG) IDESC = instr_desc((it.rows + 15) & ~15);
                 for (int k = 0; k < n_kb && ok; ++k, ++e) {
                     if (e & 1) block(std::integral_constant<uint32_t, 1>{});
                     else block(std::integral_constant<uint32_t, 0>{});
@@ -300,20 +323,28 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         // ------------------------------ read-back ------------------------------
         pdl_wait();
         const int row = (threadIdx.x - DRAIN_WARP0 * 32) & 127;   // weight row of the tile = tensor-memory lane
-        const int half = (warp - DRAIN_WARP0) >> 2, n_c = p.tile_tok / 16;   // the first or the second half of the tile's 16-token columns
-        const int c0 = half ? (n_c + 1) / 2 : 0, c1 = half ? n_c : (n_c + 1) / 2;
+        const int half = (warp - DRAIN_WARP0) >> 2;   // takes the first or the second half of the tile's 16-token columns
         const uint32_t tm_l = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
         uint32_t e = 0;
         int scaled_tt = -1;
         for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
             const Item it = item_of(idx);
+            const int n_c = (it.rows + 15) / 16, c0 = half ? (n_c + 1) / 2 : 0, c1 = half ? n_c : (n_c + 1) / 2;
+            const int live = SEG ? it.rows : p.n_rows - it.tt * p.tile_tok;
             if (it.tt != scaled_tt) {   // per-token output scale of the token tile, thread = token
                 scaled_tt = it.tt;
                 named_sync(1, TM_DRAIN_WARPS * 32);
-                float ss = 0.f;
-                if (p.sumsq && half == 0 && row < p.tile_tok)
-                    for (int q = 0; q < p.n_sumsq; ++q) ss += p.sumsq[(uint64_t)q * p.rows_pad + it.tt * p.tile_tok + row];
-                if (half == 0) tok_scale[row] = p.sumsq ? p.out_scale * (1.0f / sqrtf(ss / p.norm_k + p.eps)) : p.out_scale;
+                if (half == 0 && row < it.rows) {
+                    float sc = p.out_scale;
+                    if (SEG) {
+                        if (p.g.row_scale) sc *= p.g.row_scale[it.tt * CAP + row];
+                    } else if (p.sumsq) {
+                        float ss = 0.f;
+                        for (int q = 0; q < p.n_sumsq; ++q) ss += p.sumsq[(uint64_t)q * p.rows_pad + it.tt * p.tile_tok + row];
+                        sc *= 1.0f / sqrtf(ss / p.norm_k + p.eps);
+                    }
+                    tok_scale[row] = sc;
+                }
                 named_sync(1, TM_DRAIN_WARPS * 32);
             }
             for (int k = 0; k < it.n_kb && ok; ++k, ++e) {
@@ -323,7 +354,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 const float s = scl[(e & 3) * TILE_R + row];
                 const uint32_t d = tm_l + TM2_D + (e & 1) * 128;
                 const bool last = k == it.n_kb - 1;
-                const uint32_t orow = (uint32_t)it.rt * TILE_R + row;
+                const uint32_t orow = (uint32_t)(SEG ? it.sp : it.rt) * TILE_R + row;
                 auto release = [&] {
                     fence_before_sync();
                     __syncwarp();
@@ -345,11 +376,11 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                         for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(v[j]);
                         tmem_st16(tm_l + TM2_ACC + 16 * c, u);
                     } else if (orow < p.n_out) {
-                        const int tok0 = it.tt * p.tile_tok + 16 * c;
-                        float* dst = p.out + ((uint64_t)it.sp * p.rows_pad + tok0) * p.ld_out + orow;
+                        const int tok0 = (SEG ? it.tt * CAP : it.sp * p.rows_pad + it.tt * p.tile_tok) + 16 * c;
+                        float* dst = p.out + (uint64_t)tok0 * p.ld_out + orow;
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
-                            if (tok0 + j < p.n_rows) dst[(uint64_t)j * p.ld_out] = v[j] * tok_scale[16 * c + j];
+                            if (16 * c + j < live) dst[(uint64_t)j * p.ld_out] = v[j] * tok_scale[16 * c + j];
                     }
                     __syncwarp();
                 }
@@ -377,18 +408,17 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
     }
 }
 
-template <int DT>
-static dfl_status launch_tm(cudaStream_t st, const TmParams& p) {
+template <int DT, int CAP>
+static dfl_status launch_tm(cudaStream_t st, const TmParams& p, int n_items) {
     static std::once_flag once[16];
     int dev = 0;
     cudaGetDevice(&dev);
     cudaError_t e = cudaSuccess;
-    auto set = [&] { e = cudaFuncSetAttribute(gemm_tm_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TmFmt<DT>::SMEM); };
+    auto set = [&] { e = cudaFuncSetAttribute(gemm_tm_kernel<DT, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, TmFmt<DT, CAP>::SMEM); };
     if (dev >= 0 && dev < 16) std::call_once(once[dev], set);
     else set();
     DFL_CUDA(e);
-    const int n_items = p.row_tiles * p.splits * p.tok_tiles;
-    DFL_CUDA(launch_k(gemm_tm_kernel<DT>, dim3((unsigned)(n_items < sm_count() ? n_items : sm_count())), dim3(TM_THREADS), (size_t)TmFmt<DT>::SMEM, st, p));
+    DFL_CUDA(launch_k(gemm_tm_kernel<DT, CAP>, dim3((unsigned)(n_items < sm_count() ? n_items : sm_count())), dim3(TM_THREADS), (size_t)TmFmt<DT, CAP>::SMEM, st, p));
     count_launch();
     return DFL_OK;
 }
@@ -431,10 +461,26 @@ dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts
     p.w = m.tiles; p.acts = acts; p.out = out; p.sumsq = sumsq; p.n_sumsq = n_sumsq; p.norm_k = norm_k; p.eps = eps; p.out_scale = out_scale;
     p.kblocks = m.kblocks; p.splits = splits; p.row_tiles = m.row_tiles; p.tile_tok = tile_tok; p.tok_tiles = (n_rows + tile_tok - 1) / tile_tok;
     p.n_rows = n_rows; p.rows_pad = p.tok_tiles * tile_tok; p.n_out = (uint32_t)m.n_out; p.ld_out = ld_out ? ld_out : (uint32_t)m.n_out; p.err = dev_err;
+    const int n_items = p.row_tiles * p.splits * p.tok_tiles;
     switch (m.dtype) {
-        case DFL_Q4_K: return ts::launch_tm<DFL_Q4_K>(st, p);
-        case DFL_Q5_K: return ts::launch_tm<DFL_Q5_K>(st, p);
-        default: return ts::launch_tm<DFL_Q6_K>(st, p);
+        case DFL_Q4_K: return ts::launch_tm<DFL_Q4_K, TM_TOK>(st, p, n_items);
+        case DFL_Q5_K: return ts::launch_tm<DFL_Q5_K, TM_TOK>(st, p, n_items);
+        default: return ts::launch_tm<DFL_Q6_K, TM_TOK>(st, p, n_items);
+    }
+}
+
+dfl_status launch_gemm_tm_seg(cudaStream_t st, const QMatrix& m, const TmSegments& g, const uint8_t* acts, float* out, float out_scale,
+                              uint32_t ld_out, int* dev_err) {
+    if (!gemm_tm_supported(m)) return fail(DFL_ERR_UNSUPPORTED, "segment gemm: weight dtype");
+    if (!g.seg || g.max_seg < 1 || g.n_tiles < 1 || g.kblocks < 1 || g.kblocks > m.kblocks) return fail(DFL_ERR_BAD_ARG, "segment gemm: shape");
+    ts::TmParams p{};
+    p.w = m.tiles; p.acts = acts; p.out = out; p.out_scale = out_scale; p.kblocks = m.kblocks;
+    p.n_out = (uint32_t)g.n_tiles * TILE_R; p.ld_out = ld_out; p.err = dev_err; p.g = g; p.tile_tok = TM_SEG;
+    const int n_items = g.max_seg * g.n_tiles;   // the most there can be
+    switch (m.dtype) {
+        case DFL_Q4_K: return ts::launch_tm<DFL_Q4_K, TM_SEG>(st, p, n_items);
+        case DFL_Q5_K: return ts::launch_tm<DFL_Q5_K, TM_SEG>(st, p, n_items);
+        default: return ts::launch_tm<DFL_Q6_K, TM_SEG>(st, p, n_items);
     }
 }
 

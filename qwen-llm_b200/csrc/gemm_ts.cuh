@@ -37,9 +37,12 @@ static_assert(ACTTS_CHUNK == TS_B_BYTES + TS_BMIN_BYTES, "activation chunk size"
 // ts_act_kpos; then the 32-column sub-block sums as [plane hi / lo][k-core 2][token 128][8 halfs], both k-cores alike
 // (the A operand holds the hi part of the mins in its first eight columns and the lo part in the other eight).
 constexpr int TM_TOK = 128;
-constexpr int TM_BSTAGE = 2 * 64 * TM_TOK * 2;
-constexpr int TM_SUMS = 2 * 16 * TM_TOK * 2;
-constexpr int TM_CHUNK = 4 * TM_BSTAGE + TM_SUMS;
+// the same with room for `cap` tokens (the routed experts' segments hold 32)
+constexpr int TM_SEG = 32;
+__host__ __device__ constexpr int tm_bstage(int cap) { return 2 * 64 * cap * 2; }
+__host__ __device__ constexpr int tm_sums(int cap) { return 2 * 16 * cap * 2; }
+__host__ __device__ constexpr int tm_chunk(int cap) { return 4 * tm_bstage(cap) + tm_sums(cap); }
+constexpr int TM_CHUNK = tm_chunk(TM_TOK);
 
 constexpr int TSQ4_OFF_QS = 2048;
 constexpr int TSQ5_OFF_QH = 2048 + 16384;
@@ -120,6 +123,21 @@ int gemm_tm_choose_splits(const int* row_tiles, int n_mats, int kblocks, int tok
 int gemm_tm_tile_tok(int n_rows);
 dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_rows, int tile_tok,
                           const float* sumsq, int n_sumsq, float norm_k, float eps, float out_scale, uint32_t ld_out, int* dev_err);
+// Routed experts: the same multiplication over segments of at most TM_SEG gathered rows.  Segment i (seg[i] = {block, rows}, the
+// count in *n_seg plus n_more; the launch takes that many, at most max_seg, from `first` on) multiplies its rows, chunks
+// acts + i * kblocks * tm_chunk(TM_SEG), with row tiles tile0 + block * tiles_per_block + j of the matrix and its column
+// blocks kb0 + block * kb_per_block .. + kblocks; tiles j >= half_tiles sit half_off tiles further (the up half of a gate | up
+// matrix).  Output row i * TM_SEG + r, column 128 j: out [.][ld_out], scaled by out_scale * row_scale[row] (row_scale optional).
+struct TmSegments {
+    const int2* seg = nullptr;
+    const int32_t* n_seg = nullptr;
+    int n_more = 0, first = 0, max_seg = 0;
+    int n_tiles = 0, half_tiles = 0, half_off = 0, tiles_per_block = 0;   // n_tiles: row tiles per segment
+    int kblocks = 0, kb_per_block = 0;
+    const float* row_scale = nullptr;
+};
+dfl_status launch_gemm_tm_seg(cudaStream_t st, const QMatrix& m, const TmSegments& g, const uint8_t* acts, float* out, float out_scale,
+                              uint32_t ld_out, int* dev_err);
 int gemm_ts_choose_splits(const QMatrix& m);
 int gemm_ts_choose_splits_multi(const int* row_tiles, int n_mats, int kblocks);
 int gemm_ts_ctas_per_split(int row_tiles, int splits);

@@ -94,7 +94,7 @@ dfl_status launch_moe_route(cudaStream_t st, const float* logits, int ld, int n_
                             float* shared_gate, int32_t* route_idx, int* err) {
     if (n_expert < 1 || n_expert > MOE_MAX_EXPERTS || n_used < 1 || n_used > 32 || n_used > n_expert)
         return fail(DFL_ERR_UNSUPPORTED, "moe_route: expert_count must be in [1, 1024] and expert_used_count in [1, 32]");
-    launch_k(moe_route_kernel, dim3(MAX_ROWS), dim3(32), 0, st, logits, ld, n_expert, n_used, n_rows, route_w, shared_gate, route_idx, err);
+    launch_k(moe_route_kernel, dim3((unsigned)(n_rows > MAX_ROWS ? n_rows : MAX_ROWS)), dim3(32), 0, st, logits, ld, n_expert, n_used, n_rows, route_w, shared_gate, route_idx, err);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

@@ -14,6 +14,11 @@ struct PromptWs {
     float *q_n = nullptr, *k_n = nullptr, *v = nullptr, *ab = nullptr, *conv_new = nullptr, *capture = nullptr;
     uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_v = nullptr;
     int32_t* tokens = nullptr;
+    // routed experts
+    float *route_logits = nullptr, *route_w = nullptr, *route_sg = nullptr, *row_scale = nullptr, *gu = nullptr, *down = nullptr;
+    int32_t *route_idx = nullptr, *n_seg = nullptr, *row_of = nullptr, *pos_of = nullptr;
+    int2* seg = nullptr;
+    uint8_t *acts_in = nullptr, *acts_mid = nullptr;
     int32_t* pinned = nullptr;
     uint8_t* base = nullptr;
 };
@@ -34,14 +39,20 @@ static bool group_supported(const MatGroup& g) {
 }
 
 bool prompt_supported(const dfl_model* m) {
-    if (m->act_layout != ACT_TS || m->arch.expert_count > 0 || m->ep_world > 1) return false;
+    const dfl_arch& a = m->arch;
+    if (m->act_layout != ACT_TS || m->ep_world > 1) return false;
     // DFL_PROMPT_ROWS=0 keeps prompts on the packed path
     static const bool enabled = [] { const char* e = getenv("DFL_PROMPT_ROWS"); return !(e && e[0] == '0'); }();
     if (!enabled) return false;
-    for (auto& L : m->layers)
-        if (!(L.is_attn ? group_supported(L.qkv) && group_supported(L.wo) : group_supported(L.in_qkv_z) && group_supported(L.w_out)) ||
-            !group_supported(L.gate_up) || !group_supported(L.down))
-            return false;
+    const bool moe = a.expert_count > 0;
+    if (moe && (a.expert_count > 1024 || a.expert_used_count > 16 || a.expert_shared_feed_forward_length != a.expert_feed_forward_length)) return false;
+    for (auto& L : m->layers) {
+        if (!(L.is_attn ? group_supported(L.qkv) && group_supported(L.wo) : group_supported(L.in_qkv_z) && group_supported(L.w_out))) return false;
+        if (moe) {
+            for (const MatGroup* g : {&L.moe_gate_up, &L.moe_down, &L.moe_down_sh})
+                if (g->mats.size() != 1 || !group_supported(*g)) return false;
+        } else if (!group_supported(L.gate_up) || !group_supported(L.down)) return false;
+    }
     return true;
 }
 
@@ -66,7 +77,7 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
     uint64_t part = 0;
     for (int t = 1; t <= (int)(rows / TM_TOK); ++t)
         for (auto& L : m->layers)
-            for (const MatGroup* g : {&L.qkv, &L.wo, &L.in_qkv_z, &L.w_out, &L.gate_up, &L.down})
+            for (const MatGroup* g : {&L.qkv, &L.wo, &L.in_qkv_z, &L.w_out, &L.gate_up, &L.down})   // empty where a layer has none
                 if (!g->mats.empty()) part = std::max<uint64_t>(part, (uint64_t)tm_splits(*g, t) * t * TM_TOK * g->total_cols);
     // one block for all of it: sizes first, then the pointers
     uint64_t total = 0;
@@ -95,6 +106,23 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
         alloc(&w->acts_f, tiles * (F / TILE_K) * TM_CHUNK);
         alloc(&w->acts_v, tiles * (wide / TILE_K) * TM_CHUNK);
         alloc(&w->tokens, R * 4);
+        if (a.expert_count > 0) {
+            const uint64_t E = a.expert_count, used = a.expert_used_count, Fe = a.expert_feed_forward_length;
+            const uint64_t segs = (uint64_t)tm_moe_max_segments((int)rows, (int)E, (int)used), P = segs * TM_SEG;
+            alloc(&w->route_logits, R * (E + 1) * 4);
+            alloc(&w->route_w, R * E * 4);
+            alloc(&w->route_sg, R * 4);
+            alloc(&w->route_idx, R * used * 4);
+            alloc(&w->seg, segs * 8);
+            alloc(&w->n_seg, 4);
+            alloc(&w->row_of, P * 4);
+            alloc(&w->pos_of, R * (used + 1) * 4);
+            alloc(&w->row_scale, P * 4);
+            alloc(&w->gu, P * 2 * Fe * 4);
+            alloc(&w->down, P * H * 4);
+            alloc(&w->acts_in, segs * (H / TILE_K) * tm_chunk(TM_SEG));
+            alloc(&w->acts_mid, segs * (Fe / TILE_K) * tm_chunk(TM_SEG));
+        }
         if (pass == 0 && !(w->base = (uint8_t*)pool_alloc(total))) break;
     }
     w->pinned = (int32_t*)pool_alloc_host(R * 4);
@@ -130,9 +158,13 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
         p.n_rows = (int)n; p.rows_pad = rows_pad; p.tile_tok = tile_tok; p.err = s->err;
         return p;
     };
+    const bool moe = a.expert_count > 0;
+    const int n_pos = (int)a.expert_used_count + 1;
+    // splits < 0: the routed experts' outputs
     auto norm_glue = [&](int splits, const float* norm_w, bool want_xn, float* capture) -> dfl_status {
         TmGlue p = glue_base();
-        if (splits) { p.part = w->part; p.splits = splits; p.ld_part = (int)H; }
+        if (splits > 0) { p.part = w->part; p.splits = splits; p.ld_part = (int)H; }
+        if (splits < 0) { p.part = w->down; p.ld_part = (int)H; p.pos_of = w->pos_of; p.n_pos = n_pos; }
         p.x = w->x; p.ld_x = (int)H;
         p.mul_w = norm_w;
         p.acts = norm_w ? w->acts_h : nullptr;
@@ -195,18 +227,50 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             DFL_CHECK(gemm(L.w_out, w->acts_v, false, 1.f, &splits));
             ++gi;
         }
-        DFL_CHECK(norm_glue(splits, L.post_norm_w, false, nullptr));
-        DFL_CHECK(gemm(L.gate_up, w->acts_h, true, 1.f, &splits));
-        {
-            TmGlue p = glue_base();
-            p.mode = GLUE_SWIGLU;
-            p.part = w->part; p.splits = splits; p.ld_part = (int)L.gate_up.total_cols;
-            p.swiglu_f = (int)F;
-            p.pre_scale = 1.0f / 64.0f;   // as in the packed pass: keeps silu(g) * u inside the f16 operand range
-            p.acts = w->acts_f;
-            DFL_CHECK(launch_tm_glue(st, p, F));
+        DFL_CHECK(norm_glue(splits, L.post_norm_w, moe, nullptr));
+        if (moe) {
+            // route every row, gather the rows by expert, gate | up and down over the segments (forward.rs:749-824)
+            const int E = (int)a.expert_count, used = (int)a.expert_used_count, Fe = (int)a.expert_feed_forward_length, T = Fe / TILE_R;
+            DFL_CHECK(launch_tm_small_matmul(st, L.router_w, w->xn, (int)H, (int)n, rows_pad, H, E + 1, w->sumsq, n_sumsq, (float)H, 1e-6f, w->route_logits,
+                                             E + 1));
+            DFL_CHECK(launch_moe_route(st, w->route_logits, E + 1, E, used, (int)n, w->route_w, w->route_sg, w->route_idx, s->err));
+            TmMoe q;
+            q.n_rows = (int)n; q.rows_pad = rows_pad; q.n_expert = E; q.n_used = used; q.f = Fe;
+            q.n_shared = ((int)n + TM_SEG - 1) / TM_SEG; q.max_seg = tm_moe_max_segments((int)n, E, used);
+            q.route_idx = w->route_idx; q.route_w = w->route_w; q.route_sg = w->route_sg;
+            q.seg = w->seg; q.n_seg = w->n_seg; q.row_of = w->row_of; q.pos_of = w->pos_of;
+            q.xn = w->xn; q.ld_xn = (int)H; q.sumsq = w->sumsq; q.n_sumsq = n_sumsq; q.norm_k = (float)H;
+            q.pre_scale = 1.0f / 64.0f;
+            q.row_scale = w->row_scale; q.gu = w->gu; q.acts_in = w->acts_in; q.acts_mid = w->acts_mid; q.err = s->err;
+            DFL_CHECK(launch_tm_moe_segments(st, q));
+            DFL_CHECK(launch_tm_moe_pack(st, q, 0, H));
+            TmSegments g;
+            g.seg = w->seg; g.n_seg = w->n_seg; g.n_more = q.n_shared; g.max_seg = q.max_seg;
+            g.n_tiles = 2 * T; g.half_tiles = T; g.half_off = (E + 1) * T; g.tiles_per_block = T;
+            g.kblocks = (int)(H / TILE_K); g.row_scale = w->row_scale;
+            DFL_CHECK(launch_gemm_tm_seg(st, L.moe_gate_up.mats[0], g, w->acts_in, w->gu, 1.f, (uint32_t)(2 * Fe), s->err));
+            DFL_CHECK(launch_tm_moe_pack(st, q, 1, (uint64_t)Fe));
+            TmSegments d;
+            d.seg = w->seg; d.n_seg = w->n_seg; d.first = q.n_shared; d.max_seg = q.max_seg - q.n_shared;
+            d.n_tiles = d.half_tiles = (int)(H / TILE_R);
+            d.kblocks = d.kb_per_block = Fe / TILE_K;
+            DFL_CHECK(launch_gemm_tm_seg(st, L.moe_down.mats[0], d, w->acts_mid, w->down, 64.f, (uint32_t)H, s->err));
+            d.n_seg = nullptr; d.first = 0; d.max_seg = q.n_shared; d.kb_per_block = 0;
+            DFL_CHECK(launch_gemm_tm_seg(st, L.moe_down_sh.mats[0], d, w->acts_mid, w->down, 64.f, (uint32_t)H, s->err));
+            splits = -1;
+        } else {
+            DFL_CHECK(gemm(L.gate_up, w->acts_h, true, 1.f, &splits));
+            {
+                TmGlue p = glue_base();
+                p.mode = GLUE_SWIGLU;
+                p.part = w->part; p.splits = splits; p.ld_part = (int)L.gate_up.total_cols;
+                p.swiglu_f = (int)F;
+                p.pre_scale = 1.0f / 64.0f;   // as in the packed pass: keeps silu(g) * u inside the f16 operand range
+                p.acts = w->acts_f;
+                DFL_CHECK(launch_tm_glue(st, p, F));
+            }
+            DFL_CHECK(gemm(L.down, w->acts_f, false, 64.f, &splits));
         }
-        DFL_CHECK(gemm(L.down, w->acts_f, false, 64.f, &splits));
         float* cap = nullptr;
         for (uint32_t k = 0; k < n_ids; ++k)
             if (layer_ids[k] == il) { cap = w->capture + (uint64_t)k * H; break; }
@@ -234,6 +298,9 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
         ep.eps = 1e-6f;
         DFL_CHECK(head_core(m, s, sc, 1, ep));
     }
+    if (moe)   // the last layer's choices for the last block's rows
+        DFL_CUDA(cudaMemcpyAsync(sc->route_idx, w->route_idx + (uint64_t)(n - last_rows) * a.expert_used_count, (size_t)last_rows * a.expert_used_count * 4,
+                                 cudaMemcpyDeviceToDevice, st));
     // the last block's captured rows where a packed pass would have left them
     if (n_ids)
         DFL_CUDA(cudaMemcpyAsync(sc->capture, w->capture + (uint64_t)(n - last_rows) * KH, (size_t)last_rows * KH * 4, cudaMemcpyDeviceToDevice, st));

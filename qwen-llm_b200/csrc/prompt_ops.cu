@@ -9,35 +9,6 @@ namespace dfl {
 
 namespace cg = cooperative_groups;
 
-// Eight consecutive columns k8 .. k8 + 7 (k8 % 8 == 0, inside one 256-column block) of token t of a 128-token tile -> the
-// hi / lo planes of the activation chunk: one 16-byte store each, eight tokens fill 128 contiguous bytes.
-__device__ __forceinline__ void pack_oct_tm(uint8_t* chunk, int t, int k8, const float (&v)[8], bool& overflow) {
-    uint16_t hi[8], lo[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        overflow |= (fabsf(v[e]) >= 65504.f) && (fabsf(v[e]) < INFINITY);
-        const __half h = __float2half_rn(v[e]);
-        hi[e] = __half_as_ushort(h);
-        lo[e] = __half_as_ushort(__float2half_rn(v[e] - __half2float(h)));
-    }
-    // k-positions of a quad: 0, 2, 1, 3 (ts_act_kpos)
-    auto quad = [](const uint16_t* h) { return make_uint2((uint32_t)h[0] | ((uint32_t)h[2] << 16), (uint32_t)h[1] | ((uint32_t)h[3] << 16)); };
-    uint8_t* dst = chunk + (k8 >> 6) * TM_BSTAGE + ((k8 >> 3) & 7) * (TM_TOK * 16) + t * 16;
-    const uint2 h0 = quad(hi), h1 = quad(hi + 4), l0 = quad(lo), l1 = quad(lo + 4);
-    *reinterpret_cast<uint4*>(dst) = make_uint4(h0.x, h0.y, h1.x, h1.y);
-    *reinterpret_cast<uint4*>(dst + TM_BSTAGE / 2) = make_uint4(l0.x, l0.y, l1.x, l1.y);
-}
-// Sum of token t's activations over 32-column sub-block j -> hi / lo planes, both k-cores.
-__device__ __forceinline__ void pack_sum_tm(uint8_t* chunk, int t, int j, float sum, bool& overflow) {
-    overflow |= (fabsf(sum) >= 65504.f) && (fabsf(sum) < INFINITY);
-    const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-    uint8_t* dst = chunk + 4 * TM_BSTAGE + t * 16 + j * 2;
-    *reinterpret_cast<__half*>(dst) = h;
-    *reinterpret_cast<__half*>(dst + TM_TOK * 16) = h;
-    *reinterpret_cast<__half*>(dst + TM_SUMS / 2) = l;
-    *reinterpret_cast<__half*>(dst + TM_SUMS / 2 + TM_TOK * 16) = l;
-}
-
 // Threads of the packing kernels: CTA = 8 tokens x one 256-column block; lane = (token lane & 7, core lane >> 3), a warp covers
 // the 32 columns of one sub-block, so reads are 128-byte runs of a token's row and stores 128-byte runs of a k-core.
 __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
@@ -71,20 +42,19 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[e] = silu_f(g[e]) * u[e];
         } else {
-            if (base)
+            if (p.pos_of) {   // the routed experts' outputs of this row: shared expert first, then its choices in order
+                for (int j = 0; j < p.n_pos; ++j) {
+                    const int pos = p.pos_of[row * p.n_pos + j];
+                    if (pos >= 0) add8(v, p.part + (uint64_t)pos * p.ld_part + col);
+                }
+            } else if (base)
                 for (int s = 0; s < p.splits; ++s) add8(v, base + s * stride);
             if (p.x) {
                 float xv[8] = {};
                 add8(xv, p.x + (uint64_t)row * p.ld_x + col);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = xv[e] + v[e];
-                if (base) store8(p.x + (uint64_t)row * p.ld_x + col, v);
-            }
-            if (p.gate) {
-                float gv[8] = {};
-                add8(gv, p.gate + (uint64_t)row * p.ld_x + col);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] *= sigmoid_f(gv[e]);
+                if (p.part) store8(p.x + (uint64_t)row * p.ld_x + col, v);
             }
         }
         if (p.capture) store8(p.capture + (uint64_t)row * p.ld_capture + col, v);
@@ -116,11 +86,11 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
     if (p.acts) {
         uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * TM_CHUNK;
         bool over = false;
-        pack_oct_tm(chunk, row % p.tile_tok, k8, v, over);
+        tm_pack_oct<TM_TOK>(chunk, row % p.tile_tok, k8, v, over);
         float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
         sum += __shfl_xor_sync(0xffffffffu, sum, 8);
         sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-        if (lane < 8) pack_sum_tm(chunk, row % p.tile_tok, warp, sum, over);
+        if (lane < 8) tm_pack_sum<TM_TOK>(chunk, row % p.tile_tok, warp, sum, over);
         if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
     }
 }
@@ -603,11 +573,11 @@ __global__ void __launch_bounds__(256) tm_gdn_pack_kernel(const TmGdn p) {
     for (int e = 0; e < 8; ++e) v[e] = live ? v[e] * sc * nw[e] * silu_f(z[e]) : 0.f;
     uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * TM_CHUNK;
     bool over = false;
-    pack_oct_tm(chunk, row % p.tile_tok, k8, v, over);
+    tm_pack_oct<TM_TOK>(chunk, row % p.tile_tok, k8, v, over);
     float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
     sum += __shfl_xor_sync(0xffffffffu, sum, 8);
     sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-    if (lane < 8) pack_sum_tm(chunk, row % p.tile_tok, warp, sum, over);
+    if (lane < 8) tm_pack_sum<TM_TOK>(chunk, row % p.tile_tok, warp, sum, over);
     if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
 }
 

@@ -81,3 +81,22 @@ def test_prompt_pass_at_dense_widths(n, kv_f16, capacity):
     syn.free_entries(ents)
     _check(arch, gm, n, 0, [0, 1, 2, 3], kv_f16, capacity)
     gm.close()
+
+
+@pytest.mark.parametrize("n,start", [(17, 0), (33, 16), (130, 0), (300, 0), (520, 0)])
+def test_prompt_pass_with_routed_experts(n, start):
+    arch = modelgen.tiny_arch(n_layer=4, expert_count=8, expert_used_count=3, expert_feed_forward_length=256, expert_shared_feed_forward_length=256,
+                              intermediate_size=0)
+    gm = pkg.Model(arch, modelgen.target_tensors(arch, seed=3))
+    _check(arch, gm, n, start, [0, 3])
+    gm.close()
+
+
+def test_prompt_pass_at_routed_widths():
+    arch = syn.arch_35b_a3b()
+    arch.n_layer = 4
+    ents = syn.target_entries(arch, seed=53, device=0)
+    gm = syn.build_model(arch, ents)
+    syn.free_entries(ents)
+    _check(arch, gm, 150, 0, [0, 3])
+    gm.close()
