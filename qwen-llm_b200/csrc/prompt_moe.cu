@@ -2,24 +2,29 @@
 // TM_SEG rows, so that every chosen expert's weights are streamed and unpacked once per segment whatever rows chose it (a
 // 16-row block streams two fifths of a layer's 256 experts for its own sixteen rows).
 // Padded row = segment * TM_SEG + position.  Segments 0 .. n_shared - 1 hold all rows in order for the shared expert.
+#include <mutex>
+
 #include "prompt.cuh"
 
 namespace dfl {
 
-// One CTA, thread e = expert e.  Pairs are ranked inside an expert in row order, so the layout does not depend on timing.
+// One CTA, thread e = expert e.  The rows that chose an expert are one bit each (a row chooses an expert at most once), so a
+// pair's rank inside its expert is a count of bits before its row: row order, whatever the timing, and no scan over the pairs.
 __global__ void __launch_bounds__(1024) tm_moe_segments_kernel(const TmMoe p) {
     pdl_prologue();
-    extern __shared__ int32_t idx_s[];   // [n_pairs padded to 4]
-    __shared__ int warp_sum[32];
-    const int n_pairs = p.n_rows * p.n_used, e = threadIdx.x, lane = e & 31, warp = e >> 5;
-    for (int i = e; i < (n_pairs + 3) / 4 * 4; i += 1024) idx_s[i] = i < n_pairs ? p.route_idx[i] : -1;
+    extern __shared__ uint32_t mask[];   // [expert][words]
+    __shared__ int warp_sum[32], first_s[1024];
+    const int words = (p.n_rows + 31) / 32, n_pairs = p.n_rows * p.n_used, e = threadIdx.x, lane = e & 31, warp = e >> 5;
+    for (int i = e; i < p.n_expert * words; i += 1024) mask[i] = 0u;
+    __syncthreads();
+    for (int i = e; i < n_pairs; i += 1024) {
+        const int x = p.route_idx[i], row = i / p.n_used;
+        if (x >= 0) atomicOr(&mask[x * words + (row >> 5)], 1u << (row & 31));
+    }
     __syncthreads();
     int cnt = 0;
     if (e < p.n_expert)
-        for (int i = 0; i < n_pairs; i += 4) {
-            const int4 v = *reinterpret_cast<const int4*>(idx_s + i);
-            cnt += (v.x == e) + (v.y == e) + (v.z == e) + (v.w == e);
-        }
+        for (int w = 0; w < words; ++w) cnt += __popc(mask[e * words + w]);
     const int n_seg = (cnt + TM_SEG - 1) / TM_SEG;
     int incl = n_seg;   // inclusive prefix sum over the experts
 #pragma unroll
@@ -32,24 +37,22 @@ __global__ void __launch_bounds__(1024) tm_moe_segments_kernel(const TmMoe p) {
     int before = 0;
     for (int w = 0; w < warp; ++w) before += warp_sum[w];
     const int first = p.n_shared + before + incl - n_seg;
+    first_s[e] = first;
     if (e == 1023) *p.n_seg = before + incl;   // expert segments
     for (int j = 0; j < n_seg; ++j) p.seg[first + j] = make_int2(e, min(TM_SEG, cnt - j * TM_SEG));
-    int at = first * TM_SEG;
-    if (cnt > 0)
-        for (int i = 0; i < n_pairs; i += 4) {
-            const int4 v = *reinterpret_cast<const int4*>(idx_s + i);
-            const int q[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int x = 0; x < 4; ++x)
-                if (q[x] == e) {
-                    const int row = (i + x) / p.n_used, j = (i + x) % p.n_used;
-                    p.row_of[at] = row;
-                    p.pos_of[row * (p.n_used + 1) + 1 + j] = at;
-                    ++at;
-                }
+    __syncthreads();
+    for (int i = e; i < n_pairs; i += 1024) {
+        const int x = p.route_idx[i], row = i / p.n_used, j = i % p.n_used;
+        int at = -1;   // a row that routes nowhere
+        if (x >= 0) {
+            const uint32_t* mx = mask + x * words;
+            int rank = __popc(mx[row >> 5] & ((1u << (row & 31)) - 1u));
+            for (int w = 0; w < (row >> 5); ++w) rank += __popc(mx[w]);
+            at = first_s[x] * TM_SEG + rank;
+            p.row_of[at] = row;
         }
-    for (int i = e; i < n_pairs; i += 1024)
-        if (idx_s[i] < 0) p.pos_of[i / p.n_used * (p.n_used + 1) + 1 + i % p.n_used] = -1;   // a row that routes nowhere
+        p.pos_of[row * (p.n_used + 1) + 1 + j] = at;
+    }
     for (int r = e; r < p.n_rows; r += 1024) {   // the shared expert's segments
         p.row_of[r] = r;
         p.pos_of[r * (p.n_used + 1)] = r;
@@ -109,8 +112,14 @@ int tm_moe_max_segments(int n_rows, int n_expert, int n_used) {
 
 dfl_status launch_tm_moe_segments(cudaStream_t st, const TmMoe& p) {
     if (p.n_expert > 1024) return fail(DFL_ERR_UNSUPPORTED, "tm_moe: expert count");
-    const size_t smem = (size_t)(p.n_rows * p.n_used + 3) / 4 * 16;
-    if (smem > 48 * 1024) return fail(DFL_ERR_UNSUPPORTED, "tm_moe: pairs");
+    const size_t smem = (size_t)p.n_expert * ((p.n_rows + 31) / 32) * 4;
+    if (smem > 64 * 1024) return fail(DFL_ERR_UNSUPPORTED, "tm_moe: experts x rows");
+    static std::once_flag once[16];
+    int dev = 0;
+    DFL_CUDA(cudaGetDevice(&dev));
+    cudaError_t attr = cudaSuccess;
+    std::call_once(once[dev & 15], [&] { attr = cudaFuncSetAttribute(tm_moe_segments_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024); });
+    DFL_CUDA(attr);
     launch_k(tm_moe_segments_kernel, dim3(1), dim3(1024), smem, st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
