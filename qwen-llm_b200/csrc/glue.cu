@@ -10,17 +10,22 @@
 
 namespace dfl {
 
-// grid = k / 64, block 256: thread = (token = tid / 16, four consecutive columns).  One float4 per
-// split per thread keeps every global load of the kernel independent (one latency round).
-__global__ void __launch_bounds__(256) glue_kernel(const GlueParams p) {
+// grid = (k / 64, 2), block 128: thread = (token = 8 y + tid / 16, four consecutive columns).  One float4 per split per
+// thread keeps every global load of the kernel independent (one latency round); the norm weight does not depend on the
+// kernel before and is fetched ahead of the dependency wait.  128 threads, because a GEMM CTA (800 threads of 72 registers)
+// leaves room for exactly such a CTA beside it: with 256 the following GEMM could not start on the 64 SMs that held a waiting
+// glue CTA, and its late CTAs set the end of every link of the chain (verify block 3160 -> see the table of measurements).
+__global__ void __launch_bounds__(128) glue_kernel(const GlueParams p) {
+    const int quad = threadIdx.x & 15;
+    const float4 w = p.mul_w ? *reinterpret_cast<const float4*>(p.mul_w + blockIdx.x * GLUE_COLS + quad * 4) : make_float4(1.f, 1.f, 1.f, 1.f);
     pdl_prologue();
     const int n_splits = p.splits_dev ? p.splits + *p.splits_dev : p.splits;
-    glue_quad(p, n_splits, blockIdx.x, threadIdx.x >> 4, threadIdx.x & 15);
+    glue_quad(p, n_splits, blockIdx.x, blockIdx.y * 8 + (threadIdx.x >> 4), quad, w);
 }
 
 dfl_status launch_glue(cudaStream_t st, const GlueParams& p, uint64_t k) {
     if (k == 0 || k % TILE_K) return fail(DFL_ERR_BAD_SHAPE, "glue: column count must be a positive multiple of 256");
-    launch_k(glue_kernel, dim3((unsigned)(k / GLUE_COLS)), dim3(256), 0, st, p);
+    launch_k(glue_kernel, dim3((unsigned)(k / GLUE_COLS), MAX_ROWS / 8), dim3(128), 0, st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

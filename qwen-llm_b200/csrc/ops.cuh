@@ -105,7 +105,7 @@ struct GlueParams {
 // The glue of one (token, four consecutive columns) item: columns 64 cb + 4 quad .. + 3 of token `tok`.  The 32 lanes of
 // the calling warp must be two tokens x the sixteen quads of one 64-column block (lane = 16 (tok & 1) + quad): the sum
 // of squares is reduced over a token's 16 lanes and the 32-column sub-block sums over 8 lanes.
-__device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int cb, int tok, int quad) {
+__device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int cb, int tok, int quad, const float4 w) {   // w: the quad's mul_w
     const int col0 = cb * GLUE_COLS + quad * 4;
     const bool live = tok < p.n_rows;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
@@ -162,7 +162,6 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
         if (quad == 0) p.sumsq[cb * MAX_ROWS + tok] = ss;
     }
     if (p.mul_w) {
-        const float4 w = *reinterpret_cast<const float4*>(p.mul_w + col0);
         v[0] *= w.x; v[1] *= w.y; v[2] *= w.z; v[3] *= w.w;
     }
     if (p.pre_scale != 1.f) {
