@@ -16,36 +16,6 @@ namespace dfl {
 
 namespace cg = cooperative_groups;
 
-// ---- front: conv1d(K=4) + SiLU over the block, q/k L2 norm -------------------------------
-// grid = conv_dim / 128 (one q, k or v head per CTA), block 128: warp = group of four rows, lane = four channels
-// (gdn_front_tile).  The conv state rows are read before the dependency wait: the previous pass wrote them and a
-// pass begins with a host-to-device copy, so no kernel of this pass is their author.
-__global__ void __launch_bounds__(128) gdn_front_kernel(const GdnFrontParams p) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.x;
-    float4 old[3] = {};
-    if (w == 0) gdn_front_old_state(p, head, lane, old);
-    pdl_prologue();
-    __syncthreads();   // the old state has been read before any warp writes the new one
-    gdn_front_tile(p, head, w, lane, old);
-}
-
-dfl_status launch_gdn_front_p(cudaStream_t st, const GdnFrontParams& p) {
-    if (p.g.hd != 128 || p.g.conv_k != 4) return fail(DFL_ERR_UNSUPPORTED, "gdn: head_dim must be 128 and conv kernel 4");
-    launch_k(gdn_front_kernel, dim3(p.g.conv_dim() / 128), dim3(128), 0, st, p);
-    count_launch();
-    DFL_CUDA(cudaGetLastError());
-    return DFL_OK;
-}
-
-dfl_status launch_gdn_front(cudaStream_t st, const GdnGeom& g, const float* part_qkv, int splits, int ld_part, int n_rows,
-                            const float* conv_w, float* conv_state, float* qkv_raw, float* q_n, float* k_n, float* v, float* conv_pre) {
-    GdnFrontParams p;
-    p.g = g;
-    p.part = part_qkv; p.splits = splits; p.ld_part = ld_part; p.n_rows = n_rows;
-    p.conv_w = conv_w; p.conv_state = conv_state; p.qkv_raw = qkv_raw; p.q_n = q_n; p.k_n = k_n; p.v_out = v; p.conv_pre = conv_pre;
-    return launch_gdn_front_p(st, p);
-}
-
 __global__ void gdn_conv_restore_kernel(int conv_dim, const float* conv_pre, const float* qkv_raw, int n_keep,
                                         float* conv_state) {
     pdl_prologue();
@@ -107,31 +77,19 @@ __device__ __forceinline__ float gdn_token_step(float (&S)[16], const float* k_r
     return o;
 }
 
-// ---- scan (+ gated RMSNorm and activation packing) ------------------------------------------
-// grid (n_v, 4) in clusters of four along y (the four quarters of a head's 128 value channels), block 256: a warp
-// owns 4 state rows (dv), eight lanes per row, sixteen columns (dk) per lane.  The state rows are fetched before the
-// dependency wait (the previous pass wrote them and a pass begins with a host-to-device copy, so no kernel of this
-// pass is their author); the block's q, k, v rows and gate scalars are staged in shared memory, so that the
-// sequential part touches no global memory; the z rows are requested before the token loop and used after it.
-// Per token (forward.rs:1054-1091): sk = S k (state before decay), coeff = beta (v - g sk), S = g S + coeff k, o = S q.
-// With `acts` the kernel also finishes the layer's mixer: y = rmsnorm(o; eps * 128) * w * silu(z) over the head's 128
-// channels (forward.rs:1093-1103).  Each CTA writes its quarter's share of every token's sum of squares into all four
-// CTAs of its cluster through distributed shared memory, one cluster barrier later each adds the four shares in rank
-// order, and packs its 32 columns of the out-projection's activations.  Without `acts` (the re-scan of a partial
-// accept) only the state is advanced.
-__global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(256)
-gdn_scan_kernel(GdnGeom g, const float* state_in, float* state_out, const float* q_n, const float* k_n, const float* v, const float* ab,
-                const float* __restrict__ dt_bias, const float* __restrict__ a_log, int n_rows, const float* part_z, int z_splits, int ld_part,
-                const float* __restrict__ norm_w, uint8_t* acts, int layout, int* err) {
+// ---- state alone (partial accept) -----------------------------------------------------------------
+// grid (n_v, 4 quarters of a head's 128 value channels), block 256: a warp owns 4 state rows (dv), eight lanes per row,
+// sixteen columns (dk) per lane; rows and gate inputs are staged in shared memory, so the serial part touches no global memory.
+__device__ __forceinline__ float gdn_gate(float alpha, float dt_bias, float a_log) { return expf(softplus_f(alpha + dt_bias) * a_log); }
+
+__global__ void __launch_bounds__(256) gdn_rescan_kernel(GdnGeom g, const float* state_in, float* state_out, const float* q_n, const float* k_n,
+                                                         const float* v, const float* ab, const float* __restrict__ dt_bias,
+                                                         const float* __restrict__ a_log, int n_rows) {
     __shared__ __align__(16) float qs[MAX_ROWS][128], ks[MAX_ROWS][128];
-    __shared__ float vs[MAX_ROWS][32], gs[MAX_ROWS], bs[MAX_ROWS], os[MAX_ROWS][32];
-    __shared__ float ss_all[4][MAX_ROWS];   // [cluster rank][token]: every quarter's share of the sum of squares
-    cg::cluster_group cluster = cg::this_cluster();
-    if (acts) cluster.barrier_arrive();   // matched by the wait before the first write into another CTA's shared memory
+    __shared__ float vs[MAX_ROWS][32], gs[MAX_ROWS], bs[MAX_ROWS];
+    pdl_prologue();
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rr = lane >> 3, lg = lane & 7;
-    const int hk = h % g.n_k;
-    const int dv_cta = blockIdx.y * 32, dv = dv_cta + warp * 4 + rr;
+    const int rr = lane >> 3, lg = lane & 7, hk = h % g.n_k, dv_cta = blockIdx.y * 32, dv = dv_cta + warp * 4 + rr;
     float S[16];
     const float* sin = state_in + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
 #pragma unroll
@@ -139,87 +97,279 @@ gdn_scan_kernel(GdnGeom g, const float* state_in, float* state_out, const float*
         const float4 s4 = __ldcg(reinterpret_cast<const float4*>(sin + 32 * j));
         S[4 * j] = s4.x; S[4 * j + 1] = s4.y; S[4 * j + 2] = s4.z; S[4 * j + 3] = s4.w;
     }
-    const float dtb = dt_bias[h], alog = a_log[h];
-    pdl_prologue();
     for (int idx = threadIdx.x; idx < n_rows * 32; idx += 256) {
         const int i = idx >> 5, d4 = (idx & 31) * 4;
         *reinterpret_cast<float4*>(&qs[i][d4]) = *reinterpret_cast<const float4*>(q_n + ((uint64_t)i * g.n_k + hk) * 128 + d4);
         *reinterpret_cast<float4*>(&ks[i][d4]) = *reinterpret_cast<const float4*>(k_n + ((uint64_t)i * g.n_k + hk) * 128 + d4);
-    }
-    for (int idx = threadIdx.x; idx < n_rows * 32; idx += 256) {
-        const int i = idx >> 5, d = idx & 31;
-        vs[i][d] = v[((uint64_t)i * g.n_v + h) * 128 + dv_cta + d];
+        vs[i][idx & 31] = v[((uint64_t)i * g.n_v + h) * 128 + dv_cta + (idx & 31)];
     }
     if (threadIdx.x < n_rows) {
-        // gate inputs: ab[i][0..n_v) = alpha projection, ab[i][n_v..2 n_v) = beta projection
-        const int i = threadIdx.x;
-        const float alpha = ab[(uint64_t)i * (2 * g.n_v) + h] + dtb;
-        gs[i] = expf(softplus_f(alpha) * alog);
-        bs[i] = sigmoid_f(ab[(uint64_t)i * (2 * g.n_v) + g.n_v + h]);
+        const float* a = ab + (uint64_t)threadIdx.x * (2 * g.n_v) + h;
+        gs[threadIdx.x] = gdn_gate(a[0], dt_bias[h], a_log[h]);
+        bs[threadIdx.x] = sigmoid_f(a[g.n_v]);
     }
-    // the finishing threads (token, four channels) fetch their z values now: the z projection's split-K partials
-    // summed in slice order; the loads complete under the token loop
+    __syncthreads();
+#pragma unroll 2
+    for (int i = 0; i < n_rows; ++i) gdn_token_step(S, ks[i], qs[i], vs[i][warp * 4 + rr], gs[i], bs[i], lg);
+    float* sout = state_out + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(sout + 32 * j) = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+}
+
+dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* state_in, float* state_out, const float* q_n, const float* k_n,
+                             const float* v, const float* ab, const float* dt_bias, const float* a_log, int n_rows) {
+    launch_k(gdn_rescan_kernel, dim3((unsigned)g.n_v, 4), dim3(256), 0, st, g, state_in, state_out, q_n, k_n, v, ab, dt_bias, a_log, n_rows);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+// ---- the whole mixer of a block -------------------------------------------------------------------
+// Convolution + SiLU, L2 norms of q and k, alpha / beta projections, delta-rule scan, gated RMSNorm and activation packing in one
+// kernel.  What bounds it is latency: as four kernels (two of them on side streams) the 16 rows took 28 us between the end of
+// the input projections and the start of the output projection, of which 1.8 us is the recurrence; every kernel boundary
+// and every cross-stream join is several us of waiting.
+// grid (n_v, 4) in clusters of four along y: CTA = one v head x a quarter (32) of its value channels, 256 threads.
+//   * convolution: warp = two rows, lane = four channels of the CTA's share: 32 q and 32 k channels of the head's k head and
+//     its own 32 v channels.  The q and k shares travel to the other three CTAs through distributed shared memory together
+//     with their sums of squares, so that each CTA holds the full 16 x 128 q and k rows and normalises them itself;
+//   * alpha / beta: each CTA takes a quarter of the k columns of the head's two weight rows; the 32 partial sums are exchanged
+//     in the same cluster barrier;
+//   * recurrence: a warp owns 4 state rows (dv), eight lanes per row, sixteen columns (dk) per lane; everything it reads is in
+//     shared memory.  State, filter taps, old conv rows and weights are fetched before the dependency wait (earlier passes
+//     wrote them, and a pass begins with a host-to-device copy), the z rows are requested before the token loop;
+//   * y = rmsnorm(o; eps * 128) * w * silu(z): every CTA writes its quarter's share of a token's sum of squares to all four,
+//     one cluster barrier, rank-ordered sum, then packs its 32 columns (one sub-block) of the output projection's activations.
+// A row's result does not depend on how many rows the block has.
+__global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(256) gdn_mix_kernel(const GdnMixParams p) {
+    __shared__ __align__(16) float qs[MAX_ROWS][128], ks[MAX_ROWS][128], vs[MAX_ROWS][32];
+    __shared__ float os[MAX_ROWS][32], gs[MAX_ROWS], bs[MAX_ROWS], red[8][33];
+    __shared__ float nrm[4][2][MAX_ROWS];   // [cluster rank][q, k][row]: sums of squares over the rank's 32 channels
+    __shared__ float abp[4][32];            // [cluster rank][2 row + (alpha, beta)]: sums over the rank's quarter of k
+    __shared__ float ss_all[4][MAX_ROWS];   // [cluster rank][token]: sums of squares of the outputs
+    __shared__ float rs[MAX_ROWS];
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_arrive();   // matched by the wait before the first write into another CTA's shared memory
+    const GdnGeom& g = p.g;
+    const int h = blockIdx.x, rank = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int hk = h % g.n_k, conv_dim = g.conv_dim(), dv_cta = rank * 32;
+    const bool owner = h < g.n_k;   // of several v heads on one k head, the one that writes the k head's rows
+    const int rr = lane >> 3, lg = lane & 7, dv = dv_cta + warp * 4 + rr;
+    // -- before the dependency wait --
+    float S[16];
+    const float* sin = p.state_in + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 s4 = __ldcg(reinterpret_cast<const float4*>(sin + 32 * j));
+        S[4 * j] = s4.x; S[4 * j + 1] = s4.y; S[4 * j + 2] = s4.z; S[4 * j + 3] = s4.w;
+    }
+    const int sec = lane >> 3;   // 0 q, 1 k, 2 v, 3 idle
+    const int c = (sec == 0 ? hk : sec == 1 ? g.n_k + hk : 2 * g.n_k + h) * 128 + dv_cta + 4 * lg;   // this lane's four channels
+    float4 tap[4], old[3];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) tap[e] = sec < 3 ? *reinterpret_cast<const float4*>(p.conv_w + (uint64_t)(c + e) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+        old[t] = sec < 3 && warp < 2 ? __ldcg(reinterpret_cast<const float4*>(p.conv_in + t * conv_dim + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int kq = p.k / 4, kc = 4 * threadIdx.x;   // the CTA's quarter of k; this thread's first four columns of it
+    const float *wa = p.w_ab + (uint64_t)h * p.k + rank * kq, *wb = p.w_ab + (uint64_t)(g.n_v + h) * p.k + rank * kq;
+    float4 wa4 = make_float4(0.f, 0.f, 0.f, 0.f), wb4 = wa4;
+    if (kc < kq) { wa4 = *reinterpret_cast<const float4*>(wa + kc); wb4 = *reinterpret_cast<const float4*>(wb + kc); }
+    const float dtb = p.dt_bias[h], alog = p.a_log[h];
+    pdl_prologue();
+    // -- convolution: rows 2 warp, 2 warp + 1; xv[k] = input at row 2 warp - 3 + k --
+    const int i0 = 2 * warp;
+    float4 xv[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) xv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (warp == 0) { xv[0] = old[0]; xv[1] = old[1]; xv[2] = old[2]; }
+    if (warp == 1) xv[0] = old[2];
+    if (sec < 3) {
+#pragma unroll 4
+        for (int s = 0; s < p.splits; ++s) {
+            const float* base = p.part + (uint64_t)s * MAX_ROWS * p.ld_part + c;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                const int row = i0 - 3 + k;
+                if (row >= 0 && row < p.n_rows) {
+                    const float4 a = __ldcg(reinterpret_cast<const float4*>(base + (uint64_t)row * p.ld_part));
+                    xv[k].x += a.x; xv[k].y += a.y; xv[k].z += a.z; xv[k].w += a.w;
+                }
+            }
+        }
+    }
+    // -- alpha / beta: v[2 row + which] over this thread's columns --
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    for (int kk = kc; kk < kq; kk += 1024) {
+        if (kk != kc) { wa4 = *reinterpret_cast<const float4*>(wa + kk); wb4 = *reinterpret_cast<const float4*>(wb + kk); }
+#pragma unroll
+        for (int i = 0; i < MAX_ROWS; ++i) {
+            if (i < p.n_rows) {
+                const float4 x = __ldcg(reinterpret_cast<const float4*>(p.xn + (uint64_t)i * p.k + rank * kq + kk));
+                v[2 * i] = fmaf(wa4.w, x.w, fmaf(wa4.z, x.z, fmaf(wa4.y, x.y, fmaf(wa4.x, x.x, v[2 * i]))));
+                v[2 * i + 1] = fmaf(wb4.w, x.w, fmaf(wb4.z, x.z, fmaf(wb4.y, x.y, fmaf(wb4.x, x.x, v[2 * i + 1]))));
+            }
+        }
+    }
+    {   // per-token scale of the normalised input, sixteen threads a token, fixed tree
+        const int tok = threadIdx.x >> 4, q0 = threadIdx.x & 15;
+        float ss = 0.f;
+        for (int i = q0; i < p.n_sumsq; i += 16) ss += p.sumsq[i * MAX_ROWS + tok];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (q0 == 0) rs[tok] = 1.0f / sqrtf(ss / p.norm_k + p.eps);
+    }
+    // -- convolution output, SiLU; q and k rows to every CTA of the cluster --
+    float y[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const float in[4][4] = {{xv[j].x, xv[j + 1].x, xv[j + 2].x, xv[j + 3].x}, {xv[j].y, xv[j + 1].y, xv[j + 2].y, xv[j + 3].y},
+                                {xv[j].z, xv[j + 1].z, xv[j + 2].z, xv[j + 3].z}, {xv[j].w, xv[j + 1].w, xv[j + 2].w, xv[j + 3].w}};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            // s = sum_k w[k] * window[k], k ascending (forward.rs:1000-1010)
+            float sacc = 0.f;
+            sacc += tap[e].x * in[e][0];
+            sacc += tap[e].y * in[e][1];
+            sacc += tap[e].z * in[e][2];
+            sacc += tap[e].w * in[e][3];
+            y[j][e] = i0 + j < p.n_rows ? silu_f(sacc) : 0.f;
+        }
+    }
+    cluster.barrier_wait();   // every CTA of the cluster has started: its shared memory may be written
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int row = i0 + j;
+        const float4 y4 = make_float4(y[j][0], y[j][1], y[j][2], y[j][3]);
+        float sq = (y4.x * y4.x + y4.y * y4.y) + (y4.z * y4.z + y4.w * y4.w);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if (sec < 2) {
+            float* dst = sec == 0 ? &qs[row][dv_cta + 4 * lg] : &ks[row][dv_cta + 4 * lg];
+#pragma unroll
+            for (unsigned r = 0; r < 4; ++r) {
+                *reinterpret_cast<float4*>(cluster.map_shared_rank(dst, r)) = y4;
+                if (lg == 0) *cluster.map_shared_rank(&nrm[rank][sec][row], r) = sq;
+            }
+        } else if (sec == 2) {
+            *reinterpret_cast<float4*>(&vs[row][4 * lg]) = y4;
+            if (row < p.n_rows) *reinterpret_cast<float4*>(p.v + ((uint64_t)row * g.n_v + h) * 128 + dv_cta + 4 * lg) = y4;
+        }
+        if (row < p.n_rows && (sec == 2 || (sec < 2 && owner))) *reinterpret_cast<float4*>(p.qkv_raw + (uint64_t)row * conv_dim + c) = xv[j + 3];
+    }
+    if (sec == 2 || (sec < 2 && owner)) {
+        // new conv state = rows n_rows .. n_rows + 2 of {three old rows, the block's rows}
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            const int r = p.n_rows + t - 3;   // row of the block, or below zero an old row
+            if (r < 0) {
+                if (warp == 0) *reinterpret_cast<float4*>(p.conv_out + t * conv_dim + c) = r == -2 ? old[1] : old[2];   // n_rows >= 1: never old[0]
+            } else if (r == i0 || r == i0 + 1) {
+                *reinterpret_cast<float4*>(p.conv_out + t * conv_dim + c) = r == i0 ? xv[3] : xv[4];
+            }
+        }
+    }
+    // -- alpha / beta sums: lanes (halving: lane l ends with value l), warps, then the cluster --
+#pragma unroll
+    for (int n = 16; n >= 1; n >>= 1) {
+        const bool up = lane & n;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, n);
+        }
+    }
+    red[warp][lane] = v[0];
+    __syncthreads();
+    if (warp == 0) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += red[w][lane];
+#pragma unroll
+        for (unsigned r = 0; r < 4; ++r) *cluster.map_shared_rank(&abp[rank][lane], r) = t;
+    }
+    cluster.sync();
+    // -- normalise q and k in place (64 quads a row); the owner keeps its share for a rollback --
+    for (int idx = threadIdx.x; idx < p.n_rows * 64; idx += 256) {
+        const int row = idx >> 6, sel = (idx >> 5) & 1, d4 = (idx & 31) * 4;
+        const float sq = ((nrm[0][sel][row] + nrm[1][sel][row]) + nrm[2][sel][row]) + nrm[3][sel][row];
+        const float inv = 1.0f / fmaxf(sqrtf(sq), 1e-6f);   // y / max(||y||, eps) (forward.rs:1269-1275)
+        float4* at = reinterpret_cast<float4*>(sel ? &ks[row][d4] : &qs[row][d4]);
+        float4 x = *at;
+        x.x *= inv; x.y *= inv; x.z *= inv; x.w *= inv;
+        *at = x;
+        if (owner && (d4 >> 5) == rank) *reinterpret_cast<float4*>((sel ? p.k_n : p.q_n) + ((uint64_t)row * g.n_k + hk) * 128 + d4) = x;
+    }
+    if (threadIdx.x < p.n_rows) {
+        const int i = threadIdx.x;
+        const float alpha = (((abp[0][2 * i] + abp[1][2 * i]) + abp[2][2 * i]) + abp[3][2 * i]) * rs[i];
+        const float beta = (((abp[0][2 * i + 1] + abp[1][2 * i + 1]) + abp[2][2 * i + 1]) + abp[3][2 * i + 1]) * rs[i];
+        gs[i] = gdn_gate(alpha, dtb, alog);
+        bs[i] = sigmoid_f(beta);
+        if (rank == 0) {
+            p.ab[(uint64_t)i * (2 * g.n_v) + h] = alpha;
+            p.ab[(uint64_t)i * (2 * g.n_v) + g.n_v + h] = beta;
+        }
+    }
+    // the finishing threads (token, four channels) fetch their z values now; the loads complete under the token loop
     const int ftok = threadIdx.x >> 3, fquad = threadIdx.x & 7;
     float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (acts && threadIdx.x < 128 && ftok < n_rows) {
-        const float* zp = part_z + (uint64_t)ftok * ld_part + h * 128 + dv_cta + fquad * 4;
+    if (threadIdx.x < 128 && ftok < p.n_rows) {
+        const float* zp = p.part + (uint64_t)ftok * p.ld_part + p.z_col + h * 128 + dv_cta + fquad * 4;
 #pragma unroll 4
-        for (int s = 0; s < z_splits; ++s) {
-            const float4 t = __ldcg(reinterpret_cast<const float4*>(zp + (uint64_t)s * MAX_ROWS * ld_part));
+        for (int s = 0; s < p.splits; ++s) {
+            const float4 t = __ldcg(reinterpret_cast<const float4*>(zp + (uint64_t)s * MAX_ROWS * p.ld_part));
             z4.x += t.x; z4.y += t.y; z4.z += t.z; z4.w += t.w;
         }
     }
     __syncthreads();
+    // -- per token (forward.rs:1054-1091): sk = S k (state before decay), coeff = beta (v - g sk), S = g S + coeff k, o = S q --
 #pragma unroll 2
-    for (int i = 0; i < n_rows; ++i) {
+    for (int i = 0; i < p.n_rows; ++i) {
         const float o = gdn_token_step(S, ks[i], qs[i], vs[i][warp * 4 + rr], gs[i], bs[i], lg);
         if (lg == 0) os[i][warp * 4 + rr] = o;
     }
-    float* sout = state_out + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
+    float* sout = p.state_out + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
 #pragma unroll
     for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(sout + 32 * j) = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
-    if (!acts) return;   // uniform over the grid: no CTA of any cluster reaches the cluster barriers below
     __syncthreads();
-    cluster.barrier_wait();   // every CTA of the cluster has started: its shared memory may be written
-    // this quarter's share of each token's sum of squares (two tokens per warp), written into all four CTAs
-    const unsigned my_rank = cluster.block_rank();
     for (int i = warp; i < MAX_ROWS; i += 8) {
-        const float x = i < n_rows ? os[i][lane] : 0.f;
+        const float x = i < p.n_rows ? os[i][lane] : 0.f;
         const float sq = warp_sum(x * x);
-        if (lane < 4) *cluster.map_shared_rank(&ss_all[my_rank][i], (unsigned)lane) = sq;
+        if (lane < 4) *cluster.map_shared_rank(&ss_all[rank][i], (unsigned)lane) = sq;
     }
     cluster.sync();   // all shares have arrived; nothing is written into another CTA after this point
     if (threadIdx.x < 128) {
-        const int tok = ftok, quad = fquad;
-        const int col0 = h * 128 + dv_cta + quad * 4;
-        float y[4] = {0.f, 0.f, 0.f, 0.f};
-        if (tok < n_rows) {
+        const int tok = ftok, quad = fquad, col0 = h * 128 + dv_cta + quad * 4;
+        float o[4] = {0.f, 0.f, 0.f, 0.f};
+        if (tok < p.n_rows) {
             const float tot = ((ss_all[0][tok] + ss_all[1][tok]) + ss_all[2][tok]) + ss_all[3][tok];   // rank order: the same sum in all four CTAs
             const float sc = 1.0f / sqrtf(tot / 128.f + 1e-6f * 128.f);   // eps = RMS_EPS * head_dim (forward.rs:1098)
-            const float4 nw = *reinterpret_cast<const float4*>(norm_w + dv_cta + quad * 4);
-            y[0] = os[tok][quad * 4 + 0] * sc * nw.x * silu_f(z4.x);
-            y[1] = os[tok][quad * 4 + 1] * sc * nw.y * silu_f(z4.y);
-            y[2] = os[tok][quad * 4 + 2] * sc * nw.z * silu_f(z4.z);
-            y[3] = os[tok][quad * 4 + 3] * sc * nw.w * silu_f(z4.w);
+            const float4 nw = *reinterpret_cast<const float4*>(p.norm_w + dv_cta + quad * 4);
+            o[0] = os[tok][quad * 4 + 0] * sc * nw.x * silu_f(z4.x);
+            o[1] = os[tok][quad * 4 + 1] * sc * nw.y * silu_f(z4.y);
+            o[2] = os[tok][quad * 4 + 2] * sc * nw.z * silu_f(z4.z);
+            o[3] = os[tok][quad * 4 + 3] * sc * nw.w * silu_f(z4.w);
         }
-        uint8_t* chunk = acts + (uint64_t)(col0 >> 8) * act_chunk_dev(layout);
+        uint8_t* chunk = p.acts + (uint64_t)(col0 >> 8) * act_chunk_dev(p.layout);
         bool over = false;
-        pack_quad_any(chunk, layout, tok, col0 & 255, y, over);
-        if (layout == ACT_F16 || layout == ACT_TS) {
-            float sum = y[0] + y[1] + y[2] + y[3];   // the CTA's 32 channels are one 32-column sub-block: eight neighbouring threads
+        pack_quad_any(chunk, p.layout, tok, col0 & 255, o, over);
+        if (p.layout == ACT_F16 || p.layout == ACT_TS) {
+            float sum = o[0] + o[1] + o[2] + o[3];   // the CTA's 32 channels are one 32-column sub-block: eight neighbouring threads
 #pragma unroll
             for (int of = 4; of > 0; of >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, of);
-            if (quad == 0) store_subsum(chunk, layout, tok, (col0 & 255) >> 5, sum, over);
+            if (quad == 0) store_subsum(chunk, p.layout, tok, (col0 & 255) >> 5, sum, over);
         }
-        if (over) atomicCAS(err, 0, DEV_ERR_OVERFLOW);
+        if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
     }
 }
 
-dfl_status launch_gdn_scan(cudaStream_t st, const GdnGeom& g, const float* state_in, float* state_out, const float* q_n,
-                           const float* k_n, const float* v, const float* ab, const float* dt_bias, const float* a_log, int n_rows,
-                           const float* part_z, int z_splits, int ld_part, const float* norm_w, uint8_t* acts, int act_layout, int* err) {
-    launch_k(gdn_scan_kernel, dim3(dim3((unsigned)g.n_v, 4)), dim3(256), 0, st, g, state_in, state_out, q_n, k_n, v, ab, dt_bias, a_log, n_rows,
-              part_z, z_splits, ld_part, norm_w, acts, act_layout, err);
+dfl_status launch_gdn_mix(cudaStream_t st, const GdnMixParams& p) {
+    if (p.g.hd != 128 || p.g.conv_k != 4) return fail(DFL_ERR_UNSUPPORTED, "gdn: head_dim must be 128 and conv kernel 4");
+    if (p.k % 16) return fail(DFL_ERR_BAD_SHAPE, "gdn: input width must be a multiple of 16");
+    launch_k(gdn_mix_kernel, dim3((unsigned)p.g.n_v, 4), dim3(256), 0, st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

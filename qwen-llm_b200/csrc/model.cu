@@ -197,24 +197,17 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
     cudaStream_t st = s->st;
     // DFL_SIDE_STREAM=0 keeps every launch of the pass on one stream
     static const bool side_enabled = [] { const char* e = getenv("DFL_SIDE_STREAM"); return !(e && e[0] == '0'); }();
-    cudaStream_t side = side_enabled ? s->st_side : st, side2 = side_enabled ? s->st_side2 : st;
-    auto fork_side = [&]() -> dfl_status {   // both side streams continue from here
+    cudaStream_t side = side_enabled ? s->st_side : st;
+    auto fork_side = [&]() -> dfl_status {   // the side stream continues from here
         if (side == st) return DFL_OK;
         DFL_CUDA(cudaEventRecord(s->ev_fork, st));
         DFL_CUDA(cudaStreamWaitEvent(side, s->ev_fork, 0));
-        DFL_CUDA(cudaStreamWaitEvent(side2, s->ev_fork, 0));
         return DFL_OK;
     };
-    auto join_side = [&]() -> dfl_status {   // the main stream waits for what the first side stream was given
+    auto join_side = [&]() -> dfl_status {   // the main stream waits for what the side stream was given
         if (side == st) return DFL_OK;
         DFL_CUDA(cudaEventRecord(s->ev_join, side));
         DFL_CUDA(cudaStreamWaitEvent(st, s->ev_join, 0));
-        return DFL_OK;
-    };
-    auto join_side2 = [&]() -> dfl_status {   // ... and for the second
-        if (side2 == st) return DFL_OK;
-        DFL_CUDA(cudaEventRecord(s->ev_join2, side2));
-        DFL_CUDA(cudaStreamWaitEvent(st, s->ev_join2, 0));
         return DFL_OK;
     };
     const uint64_t H = a.hidden_size, F = a.intermediate_size;
@@ -262,24 +255,19 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             out_proj = &L.wo;
             ++ai;
         } else {
-            const int cd = gg.conv_dim();
-            // qkv -> conv / norms on the main stream; the alpha / beta projection and the z projection (its own matrix
-            // when its format differs from qkv's) each on a side stream: all three read only the layer's normalised
-            // input and write disjoint outputs; the scan waits for alpha / beta, the gated norm for z
-            const MatGroup& G = L.in_qkv_z;
-            DFL_CHECK(fork_side());
-            DFL_CHECK(launch_gemm_fewrow(st, G.mats[0], sc->acts_h, sc->part + G.col_off[0], G.splits, ep_norm, s->err, pdl_enabled(), G.total_cols));
-            DFL_CHECK(launch_small_matmul(side, L.w_ab, sc->xn, (int)H, (int)n, H, 2 * gg.n_v, ep_norm, sc->ab[gi], 2 * gg.n_v));
-            for (size_t i = 1; i < G.mats.size(); ++i)
-                DFL_CHECK(launch_gemm_fewrow(side2, G.mats[i], sc->acts_h, sc->part + G.col_off[i], G.splits, ep_norm, s->err, pdl_enabled(), G.total_cols));
+            // one stream, one chain: qkv, z (its own matrix when its format differs), then the whole mixer
+            DFL_CHECK(launch_group(st, L.in_qkv_z, sc->acts_h, sc->part, ep_norm, s->err));
             const int cur = s->ssm_cur[gi];
-            DFL_CHECK(launch_gdn_front(st, gg, sc->part, L.in_qkv_z.splits, (int)L.in_qkv_z.total_cols, (int)n, L.conv_w, s->conv[gi],
-                                       sc->qkv_raw[gi], sc->q_n[gi], sc->k_n[gi], sc->v[gi], sc->conv_pre[gi]));
-            DFL_CHECK(join_side());    // alpha / beta
-            DFL_CHECK(join_side2());   // z
-            DFL_CHECK(launch_gdn_scan(st, gg, s->ssm[cur][gi], s->ssm[cur ^ 1][gi], sc->q_n[gi], sc->k_n[gi], sc->v[gi], sc->ab[gi],
-                                      L.dt_bias, L.a_log, (int)n, sc->part + cd, L.in_qkv_z.splits, (int)L.in_qkv_z.total_cols, L.ssm_norm_w,
-                                      sc->acts_v, m->act_layout, s->err));
+            GdnMixParams p;
+            p.g = gg;
+            p.part = sc->part; p.splits = L.in_qkv_z.splits; p.ld_part = (int)L.in_qkv_z.total_cols; p.z_col = gg.conv_dim(); p.n_rows = (int)n;
+            p.conv_w = L.conv_w; p.conv_in = s->conv[cur][gi]; p.conv_out = s->conv[cur ^ 1][gi];
+            p.state_in = s->ssm[cur][gi]; p.state_out = s->ssm[cur ^ 1][gi];
+            p.w_ab = L.w_ab; p.xn = sc->xn; p.sumsq = sc->sumsq; p.k = (int)H; p.n_sumsq = kb_h; p.norm_k = (float)H; p.eps = 1e-6f;
+            p.dt_bias = L.dt_bias; p.a_log = L.a_log; p.norm_w = L.ssm_norm_w;
+            p.qkv_raw = sc->qkv_raw[gi]; p.q_n = sc->q_n[gi]; p.k_n = sc->k_n[gi]; p.v = sc->v[gi]; p.ab = sc->ab[gi];
+            p.acts = sc->acts_v; p.layout = m->act_layout; p.err = s->err;
+            DFL_CHECK(launch_gdn_mix(st, p));
             s->ssm_cur[gi] = cur ^ 1;
             out_proj = &L.w_out;
             ++gi;
@@ -412,8 +400,6 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
         }
     }
     if (want_head) DFL_CHECK(head_core(m, s, sc, n, ep_norm));
-    DFL_CHECK(join_side());   // whatever the side streams still hold belongs to this pass
-    DFL_CHECK(join_side2());
     s->kv_n_pos = start + n;
     sc->last_n = n;
     sc->last_n_verify = n;
@@ -701,10 +687,11 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
         s->v_cache.push_back(v);
     }
     for (int i = 0; i < m->n_gdn && ok; ++i) {
-        float *c = nullptr, *s0 = nullptr, *s1 = nullptr;
-        ok = (c = (float*)pool_alloc(conv_bytes)) && (s0 = (float*)pool_alloc(ssm_bytes)) && (s1 = (float*)pool_alloc(ssm_bytes));
+        float *c = nullptr, *c1 = nullptr, *s0 = nullptr, *s1 = nullptr;
+        ok = (c = (float*)pool_alloc(conv_bytes)) && (c1 = (float*)pool_alloc(conv_bytes)) && (s0 = (float*)pool_alloc(ssm_bytes)) && (s1 = (float*)pool_alloc(ssm_bytes));
         if (ok) { cudaMemsetAsync(c, 0, conv_bytes, s->st); cudaMemsetAsync(s0, 0, ssm_bytes, s->st); cudaMemsetAsync(s1, 0, ssm_bytes, s->st); }
-        s->conv.push_back(c);
+        s->conv[0].push_back(c);
+        s->conv[1].push_back(c1);
         s->ssm[0].push_back(s0);
         s->ssm[1].push_back(s1);
         s->ssm_cur.push_back(0);
@@ -712,11 +699,9 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
     if (ok && m->n_attn) ok = (s->attn_partials = (float*)pool_alloc(attn_partials_floats(m->attn_geom(), (uint32_t)cap_alloc) * 4)) != nullptr;   // two records per 128-position tile in tiled storage
     ok = ok && (s->err = (int*)pool_alloc(4));
     ok = ok && cudaEventCreate(&s->ev0) == cudaSuccess && cudaEventCreate(&s->ev1) == cudaSuccess;
-    ok = ok && cudaStreamCreateWithFlags(&s->st_side, cudaStreamNonBlocking) == cudaSuccess &&
-         cudaStreamCreateWithFlags(&s->st_side2, cudaStreamNonBlocking) == cudaSuccess;
+    ok = ok && cudaStreamCreateWithFlags(&s->st_side, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming) == cudaSuccess &&
-         cudaEventCreateWithFlags(&s->ev_join2, cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&s->ev_watch, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         std::string why = cudaGetErrorString(cudaGetLastError());
@@ -732,11 +717,12 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
 void dfl_session_destroy(dfl_session* s) {
     if (!s) return;
     cudaSetDevice(s->m->device);
-    for (cudaStream_t st : {s->st, s->st_side, s->st_side2})   // nothing of this session is in flight when its blocks go back
+    for (cudaStream_t st : {s->st, s->st_side})   // nothing of this session is in flight when its blocks go back
         if (st) cudaStreamSynchronize(st);
     for (void* p : s->k_cache) pool_free(p);
     for (void* p : s->v_cache) pool_free(p);
-    for (float* p : s->conv) pool_free(p);
+    for (float* p : s->conv[0]) pool_free(p);
+    for (float* p : s->conv[1]) pool_free(p);
     for (float* p : s->ssm[0]) pool_free(p);
     for (float* p : s->ssm[1]) pool_free(p);
     pool_free(s->attn_partials);
@@ -745,10 +731,8 @@ void dfl_session_destroy(dfl_session* s) {
     if (s->ev1) cudaEventDestroy(s->ev1);
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
     if (s->ev_join) cudaEventDestroy(s->ev_join);
-    if (s->ev_join2) cudaEventDestroy(s->ev_join2);
     if (s->ev_watch) cudaEventDestroy(s->ev_watch);
     if (s->st_side) cudaStreamDestroy(s->st_side);
-    if (s->st_side2) cudaStreamDestroy(s->st_side2);
     if (s->st) cudaStreamDestroy(s->st);
     delete s;
 }
@@ -759,7 +743,7 @@ void dfl_session_fail_next_completion(dfl_session* s) { if (s) s->fail_next = tr
 
 dfl_status dfl_session_read_gdn_state(const dfl_session* s, uint32_t gdn_index, float* ssm_out, uint64_t n_ssm, float* conv_out, uint64_t n_conv) {
     if (!s) return fail(DFL_ERR_BAD_ARG, "read_gdn_state: null session");
-    if (gdn_index >= s->conv.size()) return fail(DFL_ERR_BAD_ARG, "read_gdn_state: layer index");
+    if (gdn_index >= s->conv[0].size()) return fail(DFL_ERR_BAD_ARG, "read_gdn_state: layer index");
     DFL_CHECK(use_device(s->m->device));
     const uint64_t want_ssm = (uint64_t)s->m->arch.gdn_n_v_heads * 128 * 128, want_conv = 3ull * s->m->gdn_geom().conv_dim();
     DFL_CUDA(cudaStreamSynchronize(s->st));
@@ -769,7 +753,7 @@ dfl_status dfl_session_read_gdn_state(const dfl_session* s, uint32_t gdn_index, 
     }
     if (conv_out) {
         if (n_conv != want_conv) return fail(DFL_ERR_BAD_SHAPE, "read_gdn_state: conv size");
-        DFL_CUDA(cudaMemcpy(conv_out, s->conv[gdn_index], want_conv * 4, cudaMemcpyDeviceToHost));
+        DFL_CUDA(cudaMemcpy(conv_out, s->conv[s->ssm_cur[gdn_index]][gdn_index], want_conv * 4, cudaMemcpyDeviceToHost));
     }
     return DFL_OK;
 }
@@ -861,14 +845,13 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
     alloc(&sc->q_rot, MAX_ROWS * q_dim * 4);
     alloc(&sc->gate, MAX_ROWS * q_dim * 4);
     for (int i = 0; i < m->n_gdn; ++i) {
-        float *a0, *a1, *a2, *a3, *a4, *a5;
+        float *a0, *a2, *a3, *a4, *a5;
         alloc(&a0, (size_t)MAX_ROWS * gg.conv_dim() * 4);
-        alloc(&a1, (size_t)3 * gg.conv_dim() * 4);
         alloc(&a2, (size_t)MAX_ROWS * gg.n_k * 128 * 4);
         alloc(&a3, (size_t)MAX_ROWS * gg.n_k * 128 * 4);
         alloc(&a4, (size_t)MAX_ROWS * gg.n_v * 128 * 4);
         alloc(&a5, (size_t)MAX_ROWS * 2 * gg.n_v * 4);
-        sc->qkv_raw.push_back(a0); sc->conv_pre.push_back(a1); sc->q_n.push_back(a2); sc->k_n.push_back(a3); sc->v.push_back(a4); sc->ab.push_back(a5);
+        sc->qkv_raw.push_back(a0); sc->q_n.push_back(a2); sc->k_n.push_back(a3); sc->v.push_back(a4); sc->ab.push_back(a5);
     }
     alloc(&sc->logits, MAX_ROWS * V * 4);
     alloc(&sc->gap, MAX_ROWS * 4);
@@ -1043,9 +1026,9 @@ dfl_status restore_partial_launch(const dfl_model* m, dfl_session* s, dfl_scratc
         const LayerW& L = m->layers[il];
         if (L.is_attn) continue;
         const int cur = s->ssm_cur[gi];  // advanced state; cur ^ 1 still holds the pre-block state
-        dfl_status st = launch_gdn_scan(s->st, gg, s->ssm[cur ^ 1][gi], s->ssm[cur][gi], sc->q_n[gi], sc->k_n[gi], sc->v[gi], sc->ab[gi],
-                                        L.dt_bias, L.a_log, (int)n_keep, nullptr, 0, 0, nullptr, nullptr, 0, s->err);
-        if (st == DFL_OK) st = launch_gdn_conv_restore(s->st, gg, sc->conv_pre[gi], sc->qkv_raw[gi], (int)n_keep, s->conv[gi]);
+        dfl_status st = launch_gdn_rescan(s->st, gg, s->ssm[cur ^ 1][gi], s->ssm[cur][gi], sc->q_n[gi], sc->k_n[gi], sc->v[gi], sc->ab[gi], L.dt_bias,
+                                          L.a_log, (int)n_keep);
+        if (st == DFL_OK) st = launch_gdn_conv_restore(s->st, gg, s->conv[cur ^ 1][gi], sc->qkv_raw[gi], (int)n_keep, s->conv[cur][gi]);
         if (st != DFL_OK) { s->poisoned = true; return st; }
         ++gi;
     }
@@ -1088,7 +1071,7 @@ dfl_status dfl_session_snapshot_identity(const dfl_model* m, const dfl_session* 
     const GdnGeom gg = m->gdn_geom();
     out->layout_version = DFL_SNAPSHOT_LAYOUT_VERSION;
     out->n_attn_layers = (uint32_t)s->k_cache.size();
-    out->n_gdn_layers = (uint32_t)s->conv.size();
+    out->n_gdn_layers = (uint32_t)s->conv[0].size();
     out->kv_dim_elements = m->arch.n_kv_heads * m->arch.attn_head_dim;
     out->kv_bytes_per_token = out->kv_dim_elements * (s->kv_f16 ? 2u : 4u);
     out->kv_storage_kind = s->kv_f16 ? 1u : 0u;
@@ -1140,9 +1123,9 @@ dfl_status dfl_session_snapshot(const dfl_model* m, dfl_session* s, dfl_dsession
             } else DFL_CUDA(cudaMemcpyAsync(p, src, per_layer, cudaMemcpyDeviceToHost, s->st));
         }
     if (rows_tmp) cudaFree(rows_tmp);
-    for (size_t gi = 0; gi < s->conv.size(); ++gi, p += (uint64_t)h.id.gdn_conv_elements_per_layer * 4)
-        DFL_CUDA(cudaMemcpyAsync(p, s->conv[gi], (uint64_t)h.id.gdn_conv_elements_per_layer * 4, cudaMemcpyDeviceToHost, s->st));
-    for (size_t gi = 0; gi < s->conv.size(); ++gi, p += (uint64_t)h.id.gdn_state_elements_per_layer * 4)
+    for (size_t gi = 0; gi < s->conv[0].size(); ++gi, p += (uint64_t)h.id.gdn_conv_elements_per_layer * 4)
+        DFL_CUDA(cudaMemcpyAsync(p, s->conv[s->ssm_cur[gi]][gi], (uint64_t)h.id.gdn_conv_elements_per_layer * 4, cudaMemcpyDeviceToHost, s->st));
+    for (size_t gi = 0; gi < s->conv[0].size(); ++gi, p += (uint64_t)h.id.gdn_state_elements_per_layer * 4)
         DFL_CUDA(cudaMemcpyAsync(p, s->ssm[s->ssm_cur[gi]][gi], (uint64_t)h.id.gdn_state_elements_per_layer * 4, cudaMemcpyDeviceToHost, s->st));
     DFL_CUDA(cudaStreamSynchronize(s->st));
     DFL_CHECK(completion_check(s));
@@ -1202,9 +1185,9 @@ dfl_status dfl_session_restore_snapshot(const dfl_model* m, dfl_session* s, dfl_
             } else DFL_CUDA(cudaMemcpyAsync(dst, p, per_layer, cudaMemcpyHostToDevice, s->st));
         }
     if (rows_tmp) cudaFree(rows_tmp);
-    for (size_t gi = 0; gi < s->conv.size(); ++gi, p += (uint64_t)id.gdn_conv_elements_per_layer * 4)
-        DFL_CUDA(cudaMemcpyAsync(s->conv[gi], p, (uint64_t)id.gdn_conv_elements_per_layer * 4, cudaMemcpyHostToDevice, s->st));
-    for (size_t gi = 0; gi < s->conv.size(); ++gi, p += (uint64_t)id.gdn_state_elements_per_layer * 4)
+    for (size_t gi = 0; gi < s->conv[0].size(); ++gi, p += (uint64_t)id.gdn_conv_elements_per_layer * 4)
+        DFL_CUDA(cudaMemcpyAsync(s->conv[s->ssm_cur[gi]][gi], p, (uint64_t)id.gdn_conv_elements_per_layer * 4, cudaMemcpyHostToDevice, s->st));
+    for (size_t gi = 0; gi < s->conv[0].size(); ++gi, p += (uint64_t)id.gdn_state_elements_per_layer * 4)
         DFL_CUDA(cudaMemcpyAsync(s->ssm[s->ssm_cur[gi]][gi], p, (uint64_t)id.gdn_state_elements_per_layer * 4, cudaMemcpyHostToDevice, s->st));
     DFL_CUDA(cudaStreamSynchronize(s->st));
     s->kv_n_pos = h.prefix_len;
@@ -1216,11 +1199,7 @@ dfl_status dfl_restore_pre_block(const dfl_model* m, dfl_session* s, dfl_scratch
     DFL_CHECK(session_guard(m, s, "restore_pre_block"));
     if (!sc || sc->m != m || !sc->have_block) return fail(DFL_ERR_BAD_ARG, "restore_pre_block: scratch holds no verify block");
     if (start_position != sc->last_start) return fail(DFL_ERR_KV_STATE, "restore_pre_block: start_position differs from the last verify");
-    const GdnGeom gg = m->gdn_geom();
-    for (size_t gi = 0; gi < s->conv.size(); ++gi) {
-        s->ssm_cur[gi] ^= 1;
-        DFL_CUDA(cudaMemcpyAsync(s->conv[gi], sc->conv_pre[gi], (size_t)3 * gg.conv_dim() * 4, cudaMemcpyDeviceToDevice, s->st));
-    }
+    for (int& cur : s->ssm_cur) cur ^= 1;   // the state and conv rows from before the block are in the other buffers
     s->kv_n_pos = start_position;
     sc->have_block = false;
     DFL_CUDA(cudaStreamSynchronize(s->st));

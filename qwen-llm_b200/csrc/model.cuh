@@ -159,17 +159,16 @@ struct dfl_session {
     bool poisoned = false;
     bool fail_next = false;
     std::vector<void*> k_cache, v_cache;  // per attention layer: [capacity][n_kv][hd] rows, or tiles of 128 positions per KV head (kv_mode)
-    std::vector<float*> conv;             // per GDN layer: [3][conv_dim]
+    std::vector<float*> conv[2];          // per GDN layer, double buffered like the recurrent state: [3][conv_dim]
     std::vector<float*> ssm[2];           // per GDN layer, double buffered: [n_v][128][128]
     std::vector<int> ssm_cur;
     float* attn_partials = nullptr;
     cudaStream_t st = nullptr;
     int* err = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // side stream for the branches of a layer that only depend on the layer's normalised input (the GDN z and
-    // alpha / beta projections, the expert router): they run beside the main projection instead of after it
-    cudaStream_t st_side = nullptr, st_side2 = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr, ev_watch = nullptr;
+    // side stream for the branches of a routed-expert layer that run beside the main projection instead of after it
+    cudaStream_t st_side = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_watch = nullptr;
 };
 
 struct dfl_scratch {
@@ -179,7 +178,7 @@ struct dfl_scratch {
     uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_v = nullptr;
     float *q_rot = nullptr, *gate = nullptr;
     // per GDN layer, kept for rollback
-    std::vector<float*> qkv_raw, conv_pre, q_n, k_n, v, ab;
+    std::vector<float*> qkv_raw, q_n, k_n, v, ab;
     float *logits = nullptr, *gap = nullptr;
     int32_t* argmax = nullptr;
     // routed experts: router logits [16][E + 1], dense route weights [16][E], shared-expert gates [16], chosen ids [16][k]

@@ -11,7 +11,7 @@ namespace dfl {
 struct PromptWs {
     uint32_t rows = 0;   // padded rows the buffers hold
     float *x = nullptr, *xn = nullptr, *part = nullptr, *sumsq = nullptr, *q_rot = nullptr, *gate = nullptr, *o = nullptr, *attn_part = nullptr;
-    float *q_n = nullptr, *k_n = nullptr, *v = nullptr, *ab = nullptr, *conv_new = nullptr, *capture = nullptr;
+    float *q_n = nullptr, *k_n = nullptr, *v = nullptr, *ab = nullptr, *conv_pre = nullptr, *capture = nullptr;
     uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_v = nullptr;
     int32_t* tokens = nullptr;
     // routed experts
@@ -100,7 +100,7 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
         alloc(&w->k_n, R * gg.n_k * 128 * 4);
         alloc(&w->v, R * v_dim * 4);
         alloc(&w->ab, R * 2 * gg.n_v * 4);
-        alloc(&w->conv_new, 3ull * gg.conv_dim() * 4);
+        alloc(&w->conv_pre, 3ull * gg.conv_dim() * 4);
         alloc(&w->capture, R * sc->k_layers * H * 4);
         alloc(&w->acts_h, tiles * (H / TILE_K) * TM_CHUNK);
         alloc(&w->acts_f, tiles * (F / TILE_K) * TM_CHUNK);
@@ -214,10 +214,10 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             p.part = w->part; p.splits = splits; p.ld_part = (int)L.in_qkv_z.total_cols; p.z_col = gg.conv_dim();
             p.n_rows = (int)n; p.rows_pad = rows_pad; p.tile_tok = tile_tok; p.last_rows = (int)last_rows;
             p.conv_w = L.conv_w; p.ab = w->ab; p.dt_bias = L.dt_bias; p.a_log = L.a_log; p.norm_w = L.ssm_norm_w;
-            p.conv_state = s->conv[gi]; p.conv_new = w->conv_new;
+            p.conv_in = s->conv[cur][gi]; p.conv_out = s->conv[cur ^ 1][gi];
             p.state_in = s->ssm[cur][gi]; p.state_out = s->ssm[cur ^ 1][gi];
             p.q_n = w->q_n; p.k_n = w->k_n; p.v = w->v; p.o = w->o;
-            p.keep_raw = sc->qkv_raw[gi]; p.keep_pre = sc->conv_pre[gi]; p.keep_q = sc->q_n[gi]; p.keep_k = sc->k_n[gi]; p.keep_v = sc->v[gi];
+            p.keep_raw = sc->qkv_raw[gi]; p.keep_pre = w->conv_pre; p.keep_q = sc->q_n[gi]; p.keep_k = sc->k_n[gi]; p.keep_v = sc->v[gi];
             p.keep_ab = sc->ab[gi];
             p.acts = w->acts_v; p.err = s->err;
             DFL_CHECK(launch_tm_gdn_front(st, p));

@@ -72,8 +72,8 @@ struct TmGdn {
     int n_rows = 0, rows_pad = 0, tile_tok = TM_TOK;   // rows_pad = token tiles x tile_tok
     int last_rows = 0;              // rows of the pass's last block (what a rollback after the pass can undo); 0: none kept
     const float *conv_w = nullptr, *ab = nullptr, *dt_bias = nullptr, *a_log = nullptr, *norm_w = nullptr;
-    float *conv_state = nullptr, *conv_new = nullptr;
-    float *state_in = nullptr, *state_out = nullptr;   // state_in is left holding the state before the last block
+    // conv rows and state: in -> out; the `in` buffers are left holding what precedes the last block (conv rows by way of keep_pre)
+    float *conv_in = nullptr, *conv_out = nullptr, *state_in = nullptr, *state_out = nullptr;
     float *q_n = nullptr, *k_n = nullptr, *v = nullptr, *o = nullptr;
     // the last block's rows for a rollback, as the 16-row pass leaves them in the scratch
     float *keep_raw = nullptr, *keep_pre = nullptr, *keep_q = nullptr, *keep_k = nullptr, *keep_v = nullptr, *keep_ab = nullptr;

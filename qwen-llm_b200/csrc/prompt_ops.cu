@@ -199,8 +199,7 @@ dfl_status launch_tm_small_matmul(cudaStream_t st, const float* w, const float* 
 
 // ---- gated delta net: conv + SiLU + L2 norms over all rows of the pass ---------------------------
 // grid (heads of 128 channels, rows / 16), four warps of four rows each, lane = four channels: gdn_front_tile with the three
-// preceding rows read from the pass's own projection output (or the conv state for the first rows).  The new conv state
-// goes to conv_new, because the first row block reads the old one; the scan moves it over.
+// preceding rows read from the pass's own projection output (or the conv rows of the session for the first rows).
 __global__ void __launch_bounds__(128) tm_gdn_front_kernel(const TmGdn p) {
     pdl_prologue();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.x;
@@ -211,7 +210,7 @@ __global__ void __launch_bounds__(128) tm_gdn_front_kernel(const TmGdn p) {
     for (int k = 0; k < 7; ++k) {
         const int row = i0 - 3 + k;
         xv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (row < 0) xv[k] = *reinterpret_cast<const float4*>(p.conv_state + (row + 3) * conv_dim + c);
+        if (row < 0) xv[k] = *reinterpret_cast<const float4*>(p.conv_in + (row + 3) * conv_dim + c);
         else if (row < p.n_rows) {
             for (int s = 0; s < p.splits; ++s) {
                 const float4 a = __ldcg(reinterpret_cast<const float4*>(p.part + ((uint64_t)s * p.rows_pad + row) * p.ld_part + c));
@@ -270,7 +269,7 @@ __global__ void __launch_bounds__(128) tm_gdn_front_kernel(const TmGdn p) {
         const int r = i0 - 3 + k;
         if (!mine(r)) continue;
         const int tn = r - (p.n_rows - 3), tp = r - (keep0 - 3);   // index in the new state / in the state before the last block
-        if (tn >= 0 && tn < 3) *reinterpret_cast<float4*>(p.conv_new + tn * conv_dim + c) = xv[k];
+        if (tn >= 0 && tn < 3) *reinterpret_cast<float4*>(p.conv_out + tn * conv_dim + c) = xv[k];
         if (p.last_rows && tp >= 0 && tp < 3) *reinterpret_cast<float4*>(p.keep_pre + tp * conv_dim + c) = xv[k];
     }
 }
@@ -382,12 +381,12 @@ __global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
         }
         d0 = v[0]; d1 = v[1];
     };
-    // the conv state the front kernel could not write in place; one slice per CTA
-    {
+    // the conv rows before the last block replace the pass's first ones, which the front kernel has read; one slice per CTA
+    if (p.last_rows) {
         const int n = 3 * g.conv_dim() / 4, per = (n + gridDim.x * gridDim.y - 1) / (gridDim.x * gridDim.y);
         const int c0 = (blockIdx.y * gridDim.x + blockIdx.x) * per;
         for (int i = c0 + threadIdx.x; i < min(n, c0 + per); i += 256)
-            reinterpret_cast<float4*>(p.conv_state)[i] = __ldcg(reinterpret_cast<const float4*>(p.conv_new) + i);
+            reinterpret_cast<float4*>(p.conv_in)[i] = __ldcg(reinterpret_cast<const float4*>(p.keep_pre) + i);
     }
     fetch(0, 0);
     gate_load(0);
