@@ -37,69 +37,76 @@ dfl_status launch_gdn_conv_restore(cudaStream_t st, const GdnGeom& g, const floa
     return DFL_OK;
 }
 
-// One token of the recurrence for one state row shared by eight lanes: lane group member lg owns the sixteen columns
-// dk = 32 j + 4 lg + c (j, c < 4), so that the eight lanes of a row read 128 contiguous bytes of k and q per step.
-// The two row sums go through three shuffle levels each.
-__device__ __forceinline__ float gdn_token_step(float (&S)[16], const float* k_row, const float* q_row, float v, float gexp, float beta, int lg) {
-    float kk[16], qq[16];
+// The recurrent state of four value channels (rows) in a warp: a lane owns four key channels (columns 4 lane .. + 3) of every
+// row, so that one 16-byte load of a k or q row serves all four (with eight lanes a row each warp read every k and q row
+// sixteen bytes at a time per row group, and the 16-token loop was bound by shared-memory bandwidth: 530 clocks a token).
+// Slot r of lane l holds row r ^ (l / 8): the first two steps of a sum over the lanes then always pass on the upper slots, and
+// lane group l / 8 ends with the sum of row l / 8.
+struct GdnRows {
+    float4 s[4];
+    __device__ __forceinline__ void load(const float* base, int rr) {   // base: row 0, this lane's columns
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float4 k4 = *reinterpret_cast<const float4*>(k_row + 32 * j + 4 * lg);
-        const float4 q4 = *reinterpret_cast<const float4*>(q_row + 32 * j + 4 * lg);
-        kk[4 * j] = k4.x; kk[4 * j + 1] = k4.y; kk[4 * j + 2] = k4.z; kk[4 * j + 3] = k4.w;
-        qq[4 * j] = q4.x; qq[4 * j + 1] = q4.y; qq[4 * j + 2] = q4.z; qq[4 * j + 3] = q4.w;
+        for (int r = 0; r < 4; ++r) s[r] = __ldcg(reinterpret_cast<const float4*>(base + (r ^ rr) * 128));
     }
-    float p[4];
+    __device__ __forceinline__ void store(float* base, int rr) const {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        p[j] = S[4 * j] * kk[4 * j];
-#pragma unroll
-        for (int c = 1; c < 4; ++c) p[j] = fmaf(S[4 * j + c], kk[4 * j + c], p[j]);
+        for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(base + (r ^ rr) * 128) = s[r];
     }
-    float sk = (p[0] + p[1]) + (p[2] + p[3]);
+    // Sums over the lanes of S k and S q: row l / 8 of S k in lanes with bit 2 clear, of S q in the others.  The two travel
+    // together: a token's output needs the state after its update, which is the state the next token's S k needs, so one
+    // pass over the lanes per token serves both and the output never waits in the chain.
+    __device__ __forceinline__ float dots(const float4 k, const float4 q, int lane) const {
+        float pk[4], pq[4];
 #pragma unroll
-    for (int of = 4; of > 0; of >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, of);
-    const float coeff = beta * (v - gexp * sk);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int e = 4 * j + c;
-            S[e] = __fadd_rn(__fmul_rn(gexp, S[e]), __fmul_rn(coeff, kk[e]));
+        for (int r = 0; r < 4; ++r) {
+            pk[r] = fmaf(s[r].w, k.w, fmaf(s[r].z, k.z, fmaf(s[r].y, k.y, s[r].x * k.x)));
+            pq[r] = fmaf(s[r].w, q.w, fmaf(s[r].z, q.z, fmaf(s[r].y, q.y, s[r].x * q.x)));
         }
-        p[j] = S[4 * j] * qq[4 * j];
 #pragma unroll
-        for (int c = 1; c < 4; ++c) p[j] = fmaf(S[4 * j + c], qq[4 * j + c], p[j]);
+        for (int r = 0; r < 2; ++r) {
+            pk[r] += __shfl_xor_sync(0xffffffffu, pk[r + 2], 16);
+            pq[r] += __shfl_xor_sync(0xffffffffu, pq[r + 2], 16);
+        }
+        pk[0] += __shfl_xor_sync(0xffffffffu, pk[1], 8);
+        pq[0] += __shfl_xor_sync(0xffffffffu, pq[1], 8);
+        const bool up = lane & 4;
+        float v = (up ? pq[0] : pk[0]) + __shfl_xor_sync(0xffffffffu, up ? pk[0] : pq[0], 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        return v;
     }
-    float o = (p[0] + p[1]) + (p[2] + p[3]);
+    // S = g S + c k^T with c = beta (v - g S k); sk and v: of row l / 8, meaningful in lanes with bit 2 clear
+    __device__ __forceinline__ void update(const float4 k, float sk, float v, float gexp, float beta, int rr) {
+        const float coeff = beta * (v - gexp * sk);
 #pragma unroll
-    for (int of = 4; of > 0; of >>= 1) o += __shfl_xor_sync(0xffffffffu, o, of);
-    return o;
-}
+        for (int r = 0; r < 4; ++r) {
+            const float c = __shfl_sync(0xffffffffu, coeff, (r ^ rr) * 8);
+            s[r].x = __fadd_rn(__fmul_rn(gexp, s[r].x), __fmul_rn(c, k.x));
+            s[r].y = __fadd_rn(__fmul_rn(gexp, s[r].y), __fmul_rn(c, k.y));
+            s[r].z = __fadd_rn(__fmul_rn(gexp, s[r].z), __fmul_rn(c, k.z));
+            s[r].w = __fadd_rn(__fmul_rn(gexp, s[r].w), __fmul_rn(c, k.w));
+        }
+    }
+};
 
 // ---- state alone (partial accept) -----------------------------------------------------------------
-// grid (n_v, 4 quarters of a head's 128 value channels), block 256: a warp owns 4 state rows (dv), eight lanes per row,
-// sixteen columns (dk) per lane; rows and gate inputs are staged in shared memory, so the serial part touches no global memory.
+// grid (n_v, 4 quarters of a head's 128 value channels), block 256: a warp owns 4 state rows (GdnRows); the block's rows and
+// gate inputs are staged in shared memory, so the serial part touches no global memory.
 __device__ __forceinline__ float gdn_gate(float alpha, float dt_bias, float a_log) { return expf(softplus_f(alpha + dt_bias) * a_log); }
 
-__global__ void __launch_bounds__(256) gdn_rescan_kernel(GdnGeom g, const float* state_in, float* state_out, const float* q_n, const float* k_n,
+__global__ void __launch_bounds__(256) gdn_rescan_kernel(GdnGeom g, const float* state_in, float* state_out, const float* k_n,
                                                          const float* v, const float* ab, const float* __restrict__ dt_bias,
                                                          const float* __restrict__ a_log, int n_rows) {
-    __shared__ __align__(16) float qs[MAX_ROWS][128], ks[MAX_ROWS][128];
+    __shared__ __align__(16) float ks[MAX_ROWS][128];
     __shared__ float vs[MAX_ROWS][32], gs[MAX_ROWS], bs[MAX_ROWS];
     pdl_prologue();
     const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rr = lane >> 3, lg = lane & 7, hk = h % g.n_k, dv_cta = blockIdx.y * 32, dv = dv_cta + warp * 4 + rr;
-    float S[16];
-    const float* sin = state_in + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float4 s4 = __ldcg(reinterpret_cast<const float4*>(sin + 32 * j));
-        S[4 * j] = s4.x; S[4 * j + 1] = s4.y; S[4 * j + 2] = s4.z; S[4 * j + 3] = s4.w;
-    }
+    const int rr = lane >> 3, hk = h % g.n_k, dv_cta = blockIdx.y * 32;
+    const uint64_t s_off = ((uint64_t)h * 128 + dv_cta + warp * 4) * 128 + 4 * lane;
+    GdnRows S;
+    S.load(state_in + s_off, rr);
     for (int idx = threadIdx.x; idx < n_rows * 32; idx += 256) {
         const int i = idx >> 5, d4 = (idx & 31) * 4;
-        *reinterpret_cast<float4*>(&qs[i][d4]) = *reinterpret_cast<const float4*>(q_n + ((uint64_t)i * g.n_k + hk) * 128 + d4);
         *reinterpret_cast<float4*>(&ks[i][d4]) = *reinterpret_cast<const float4*>(k_n + ((uint64_t)i * g.n_k + hk) * 128 + d4);
         vs[i][idx & 31] = v[((uint64_t)i * g.n_v + h) * 128 + dv_cta + (idx & 31)];
     }
@@ -109,60 +116,53 @@ __global__ void __launch_bounds__(256) gdn_rescan_kernel(GdnGeom g, const float*
         bs[threadIdx.x] = sigmoid_f(a[g.n_v]);
     }
     __syncthreads();
-#pragma unroll 2
-    for (int i = 0; i < n_rows; ++i) gdn_token_step(S, ks[i], qs[i], vs[i][warp * 4 + rr], gs[i], bs[i], lg);
-    float* sout = state_out + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(sout + 32 * j) = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+    for (int i = 0; i < n_rows; ++i) {
+        const float4 k = *reinterpret_cast<const float4*>(&ks[i][4 * lane]);
+        S.update(k, S.dots(k, k, lane), vs[i][warp * 4 + rr], gs[i], bs[i], rr);
+    }
+    S.store(state_out + s_off, rr);
 }
 
-dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* state_in, float* state_out, const float* q_n, const float* k_n,
+dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* state_in, float* state_out, const float* k_n,
                              const float* v, const float* ab, const float* dt_bias, const float* a_log, int n_rows) {
-    launch_k(gdn_rescan_kernel, dim3((unsigned)g.n_v, 4), dim3(256), 0, st, g, state_in, state_out, q_n, k_n, v, ab, dt_bias, a_log, n_rows);
+    launch_k(gdn_rescan_kernel, dim3((unsigned)g.n_v, 4), dim3(256), 0, st, g, state_in, state_out, k_n, v, ab, dt_bias, a_log, n_rows);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;
 }
 
 // ---- the whole mixer of a block -------------------------------------------------------------------
-// Convolution + SiLU, L2 norms of q and k, alpha / beta projections, delta-rule scan, gated RMSNorm and activation packing in one
+// Convolution + SiLU, L2 norms of q and k, delta-rule scan, gated RMSNorm and activation packing in one
 // kernel.  What bounds it is latency: as four kernels (two of them on side streams) the 16 rows took 28 us between the end of
-// the input projections and the start of the output projection, of which 1.8 us is the recurrence; every kernel boundary
+// the input projections (alpha / beta ride on CTAs behind the last of them) and the start of the output projection, of which 1.8 us is the recurrence; every kernel boundary
 // and every cross-stream join is several us of waiting.
 // grid (n_v, 4) in clusters of four along y: CTA = one v head x a quarter (32) of its value channels, 256 threads.
 //   * convolution: warp = two rows, lane = four channels of the CTA's share: 32 q and 32 k channels of the head's k head and
 //     its own 32 v channels.  The q and k shares travel to the other three CTAs through distributed shared memory together
 //     with their sums of squares, so that each CTA holds the full 16 x 128 q and k rows and normalises them itself;
-//   * alpha / beta: each CTA takes a quarter of the k columns of the head's two weight rows; the 32 partial sums are exchanged
-//     in the same cluster barrier;
-//   * recurrence: a warp owns 4 state rows (dv), eight lanes per row, sixteen columns (dk) per lane; everything it reads is in
-//     shared memory.  State, filter taps, old conv rows and weights are fetched before the dependency wait (earlier passes
+//   * recurrence: a warp owns 4 state rows (GdnRows); everything it reads is in shared memory.  State, filter taps and old conv
+//     rows are fetched before the dependency wait (earlier passes
 //     wrote them, and a pass begins with a host-to-device copy), the z rows are requested before the token loop;
 //   * y = rmsnorm(o; eps * 128) * w * silu(z): every CTA writes its quarter's share of a token's sum of squares to all four,
 //     one cluster barrier, rank-ordered sum, then packs its 32 columns (one sub-block) of the output projection's activations.
 // A row's result does not depend on how many rows the block has.
 __global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(256) gdn_mix_kernel(const GdnMixParams p) {
     __shared__ __align__(16) float qs[MAX_ROWS][128], ks[MAX_ROWS][128], vs[MAX_ROWS][32];
-    __shared__ float os[MAX_ROWS][32], gs[MAX_ROWS], bs[MAX_ROWS], red[8][33];
+    __shared__ float os[MAX_ROWS][32], gs[MAX_ROWS], bs[MAX_ROWS];
+    __shared__ float inv[2][MAX_ROWS];
     __shared__ float nrm[4][2][MAX_ROWS];   // [cluster rank][q, k][row]: sums of squares over the rank's 32 channels
-    __shared__ float abp[4][32];            // [cluster rank][2 row + (alpha, beta)]: sums over the rank's quarter of k
     __shared__ float ss_all[4][MAX_ROWS];   // [cluster rank][token]: sums of squares of the outputs
-    __shared__ float rs[MAX_ROWS];
     cg::cluster_group cluster = cg::this_cluster();
     cluster.barrier_arrive();   // matched by the wait before the first write into another CTA's shared memory
     const GdnGeom& g = p.g;
     const int h = blockIdx.x, rank = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int hk = h % g.n_k, conv_dim = g.conv_dim(), dv_cta = rank * 32;
     const bool owner = h < g.n_k;   // of several v heads on one k head, the one that writes the k head's rows
-    const int rr = lane >> 3, lg = lane & 7, dv = dv_cta + warp * 4 + rr;
+    const int rr = lane >> 3, lg = lane & 7;
+    const uint64_t s_off = ((uint64_t)h * 128 + dv_cta + warp * 4) * 128 + 4 * lane;
     // -- before the dependency wait --
-    float S[16];
-    const float* sin = p.state_in + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const float4 s4 = __ldcg(reinterpret_cast<const float4*>(sin + 32 * j));
-        S[4 * j] = s4.x; S[4 * j + 1] = s4.y; S[4 * j + 2] = s4.z; S[4 * j + 3] = s4.w;
-    }
+    GdnRows S;
+    S.load(p.state_in + s_off, rr);
     const int sec = lane >> 3;   // 0 q, 1 k, 2 v, 3 idle
     const int c = (sec == 0 ? hk : sec == 1 ? g.n_k + hk : 2 * g.n_k + h) * 128 + dv_cta + 4 * lg;   // this lane's four channels
     float4 tap[4], old[3];
@@ -171,10 +171,6 @@ __global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(256) gdn_mix_kernel(
 #pragma unroll
     for (int t = 0; t < 3; ++t)
         old[t] = sec < 3 && warp < 2 ? __ldcg(reinterpret_cast<const float4*>(p.conv_in + t * conv_dim + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int kq = p.k / 4, kc = 4 * threadIdx.x;   // the CTA's quarter of k; this thread's first four columns of it
-    const float *wa = p.w_ab + (uint64_t)h * p.k + rank * kq, *wb = p.w_ab + (uint64_t)(g.n_v + h) * p.k + rank * kq;
-    float4 wa4 = make_float4(0.f, 0.f, 0.f, 0.f), wb4 = wa4;
-    if (kc < kq) { wa4 = *reinterpret_cast<const float4*>(wa + kc); wb4 = *reinterpret_cast<const float4*>(wb + kc); }
     const float dtb = p.dt_bias[h], alog = p.a_log[h];
     pdl_prologue();
     // -- convolution: rows 2 warp, 2 warp + 1; xv[k] = input at row 2 warp - 3 + k --
@@ -198,28 +194,21 @@ __global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(256) gdn_mix_kernel(
             }
         }
     }
-    // -- alpha / beta: v[2 row + which] over this thread's columns --
-    float v[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = 0.f;
-    for (int kk = kc; kk < kq; kk += 1024) {
-        if (kk != kc) { wa4 = *reinterpret_cast<const float4*>(wa + kk); wb4 = *reinterpret_cast<const float4*>(wb + kk); }
-#pragma unroll
-        for (int i = 0; i < MAX_ROWS; ++i) {
-            if (i < p.n_rows) {
-                const float4 x = __ldcg(reinterpret_cast<const float4*>(p.xn + (uint64_t)i * p.k + rank * kq + kk));
-                v[2 * i] = fmaf(wa4.w, x.w, fmaf(wa4.z, x.z, fmaf(wa4.y, x.y, fmaf(wa4.x, x.x, v[2 * i]))));
-                v[2 * i + 1] = fmaf(wb4.w, x.w, fmaf(wb4.z, x.z, fmaf(wb4.y, x.y, fmaf(wb4.x, x.x, v[2 * i + 1]))));
-            }
-        }
+    float alpha = 0.f, beta = 0.f;
+    if (threadIdx.x < p.n_rows) {
+        alpha = __ldcg(p.ab + (uint64_t)threadIdx.x * (2 * g.n_v) + h);
+        beta = __ldcg(p.ab + (uint64_t)threadIdx.x * (2 * g.n_v) + g.n_v + h);
     }
-    {   // per-token scale of the normalised input, sixteen threads a token, fixed tree
-        const int tok = threadIdx.x >> 4, q0 = threadIdx.x & 15;
-        float ss = 0.f;
-        for (int i = q0; i < p.n_sumsq; i += 16) ss += p.sumsq[i * MAX_ROWS + tok];
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (q0 == 0) rs[tok] = 1.0f / sqrtf(ss / p.norm_k + p.eps);
+    // the finishing threads (token, four channels) fetch their z values now and use them after the token loop
+    const int ftok = threadIdx.x >> 3, fquad = threadIdx.x & 7;
+    float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (threadIdx.x < 128 && ftok < p.n_rows) {
+        const float* zp = p.part + (uint64_t)ftok * p.ld_part + p.z_col + h * 128 + dv_cta + fquad * 4;
+#pragma unroll 4
+        for (int s = 0; s < p.splits; ++s) {
+            const float4 t = __ldcg(reinterpret_cast<const float4*>(zp + (uint64_t)s * MAX_ROWS * p.ld_part));
+            z4.x += t.x; z4.y += t.y; z4.z += t.z; z4.w += t.w;
+        }
     }
     // -- convolution output, SiLU; q and k rows to every CTA of the cluster --
     float y[2][4];
@@ -271,69 +260,48 @@ __global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(256) gdn_mix_kernel(
             }
         }
     }
-    // -- alpha / beta sums: lanes (halving: lane l ends with value l), warps, then the cluster --
-#pragma unroll
-    for (int n = 16; n >= 1; n >>= 1) {
-        const bool up = lane & n;
-#pragma unroll
-        for (int i = 0; i < n; ++i) {
-            const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, n);
-        }
-    }
-    red[warp][lane] = v[0];
-    __syncthreads();
-    if (warp == 0) {
-        float t = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) t += red[w][lane];
-#pragma unroll
-        for (unsigned r = 0; r < 4; ++r) *cluster.map_shared_rank(&abp[rank][lane], r) = t;
-    }
     cluster.sync();
-    // -- normalise q and k in place (64 quads a row); the owner keeps its share for a rollback --
-    for (int idx = threadIdx.x; idx < p.n_rows * 64; idx += 256) {
-        const int row = idx >> 6, sel = (idx >> 5) & 1, d4 = (idx & 31) * 4;
-        const float sq = ((nrm[0][sel][row] + nrm[1][sel][row]) + nrm[2][sel][row]) + nrm[3][sel][row];
-        const float inv = 1.0f / fmaxf(sqrtf(sq), 1e-6f);   // y / max(||y||, eps) (forward.rs:1269-1275)
-        float4* at = reinterpret_cast<float4*>(sel ? &ks[row][d4] : &qs[row][d4]);
-        float4 x = *at;
-        x.x *= inv; x.y *= inv; x.z *= inv; x.w *= inv;
-        *at = x;
-        if (owner && (d4 >> 5) == rank) *reinterpret_cast<float4*>((sel ? p.k_n : p.q_n) + ((uint64_t)row * g.n_k + hk) * 128 + d4) = x;
+    if (threadIdx.x >= 64 && threadIdx.x < 96) {   // 1 / max(||y||, eps) of the q and k rows (forward.rs:1269-1275)
+        const int row = lane & 15, sel = lane >> 4;
+        inv[sel][row] = 1.0f / fmaxf(sqrtf(((nrm[0][sel][row] + nrm[1][sel][row]) + nrm[2][sel][row]) + nrm[3][sel][row]), 1e-6f);
     }
     if (threadIdx.x < p.n_rows) {
-        const int i = threadIdx.x;
-        const float alpha = (((abp[0][2 * i] + abp[1][2 * i]) + abp[2][2 * i]) + abp[3][2 * i]) * rs[i];
-        const float beta = (((abp[0][2 * i + 1] + abp[1][2 * i + 1]) + abp[2][2 * i + 1]) + abp[3][2 * i + 1]) * rs[i];
-        gs[i] = gdn_gate(alpha, dtb, alog);
-        bs[i] = sigmoid_f(beta);
-        if (rank == 0) {
-            p.ab[(uint64_t)i * (2 * g.n_v) + h] = alpha;
-            p.ab[(uint64_t)i * (2 * g.n_v) + g.n_v + h] = beta;
-        }
-    }
-    // the finishing threads (token, four channels) fetch their z values now; the loads complete under the token loop
-    const int ftok = threadIdx.x >> 3, fquad = threadIdx.x & 7;
-    float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (threadIdx.x < 128 && ftok < p.n_rows) {
-        const float* zp = p.part + (uint64_t)ftok * p.ld_part + p.z_col + h * 128 + dv_cta + fquad * 4;
-#pragma unroll 4
-        for (int s = 0; s < p.splits; ++s) {
-            const float4 t = __ldcg(reinterpret_cast<const float4*>(zp + (uint64_t)s * MAX_ROWS * p.ld_part));
-            z4.x += t.x; z4.y += t.y; z4.z += t.z; z4.w += t.w;
-        }
+        gs[threadIdx.x] = gdn_gate(alpha, dtb, alog);
+        bs[threadIdx.x] = sigmoid_f(beta);
     }
     __syncthreads();
     // -- per token (forward.rs:1054-1091): sk = S k (state before decay), coeff = beta (v - g sk), S = g S + coeff k, o = S q --
+    auto row4 = [&](const float(*rows)[128], int sel, int i) {
+        float4 x = *reinterpret_cast<const float4*>(&rows[i][4 * lane]);
+        const float f = inv[sel][i];
+        x.x *= f; x.y *= f; x.z *= f; x.w *= f;
+        return x;
+    };
+    float4 k4 = row4(ks, 1, 0), q4 = k4;   // q of the token before (none yet)
+    float vi = vs[0][warp * 4 + rr], gi = gs[0], bi = bs[0];
 #pragma unroll 2
-    for (int i = 0; i < p.n_rows; ++i) {
-        const float o = gdn_token_step(S, ks[i], qs[i], vs[i][warp * 4 + rr], gs[i], bs[i], lg);
-        if (lg == 0) os[i][warp * 4 + rr] = o;
+    for (int i = 0; i < p.n_rows; ++i) {   // the next token's operands are fetched while this one's sums travel
+        const int in = i + 1 < p.n_rows ? i + 1 : i;
+        const float4 qn = row4(qs, 0, i), kn = row4(ks, 1, in);
+        const float vn = vs[in][warp * 4 + rr], gn = gs[in], bn = bs[in];
+        const float sk = S.dots(k4, q4, lane);
+        if (i > 0 && lg == 4) os[i - 1][warp * 4 + rr] = sk;
+        S.update(k4, sk, vi, gi, bi, rr);
+        k4 = kn; q4 = qn; vi = vn; gi = gn; bi = bn;
     }
-    float* sout = p.state_out + ((uint64_t)h * 128 + dv) * 128 + 4 * lg;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(sout + 32 * j) = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+    {
+        const float o = S.dots(q4, q4, lane);
+        if (lg == 4) os[p.n_rows - 1][warp * 4 + rr] = o;
+    }
+    S.store(p.state_out + s_off, rr);
+    if (owner)   // the normalised rows of this CTA's share, for a rollback
+        for (int idx = threadIdx.x; idx < p.n_rows * 16; idx += 256) {
+            const int row = idx >> 4, sel = (idx >> 3) & 1, d = dv_cta + (idx & 7) * 4;
+            float4 x = *reinterpret_cast<const float4*>(sel ? &ks[row][d] : &qs[row][d]);
+            const float f = inv[sel][row];
+            x.x *= f; x.y *= f; x.z *= f; x.w *= f;
+            *reinterpret_cast<float4*>((sel ? p.k_n : p.q_n) + ((uint64_t)row * g.n_k + hk) * 128 + d) = x;
+        }
     __syncthreads();
     for (int i = warp; i < MAX_ROWS; i += 8) {
         const float x = i < p.n_rows ? os[i][lane] : 0.f;
@@ -368,7 +336,6 @@ __global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(256) gdn_mix_kernel(
 
 dfl_status launch_gdn_mix(cudaStream_t st, const GdnMixParams& p) {
     if (p.g.hd != 128 || p.g.conv_k != 4) return fail(DFL_ERR_UNSUPPORTED, "gdn: head_dim must be 128 and conv kernel 4");
-    if (p.k % 16) return fail(DFL_ERR_BAD_SHAPE, "gdn: input width must be a multiple of 16");
     launch_k(gdn_mix_kernel, dim3((unsigned)p.g.n_v, 4), dim3(256), 0, st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());

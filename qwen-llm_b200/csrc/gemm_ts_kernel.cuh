@@ -37,6 +37,10 @@ struct Params {
     const int32_t* n_tiles;
     const int32_t* kb_map;     // optional: column blocks to sum over, and how many (device memory)
     const int32_t* n_kb;
+    int main_grid;             // CTAs from here on run the side projection, four outputs each
+    const float *side_w, *side_x;
+    float* side_out;
+    int side_n, side_k, side_rows;
 };
 
 constexpr int SCL_BYTES = 4 * TILE_R * 8;   // four entries' {d, dmin} per row
@@ -49,6 +53,56 @@ constexpr int smem_bytes() {
 
 // named barrier among the draining warps only (every one of them reaches it unconditionally)
 __device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+// The side projection: this CTA's four outputs over all rows.  24 warps; the even ones take tokens 0 - 7, the odd ones 8 - 15,
+// a thread four columns of every 12 x 128.  Sums over lanes, then warps, in a fixed order.
+__device__ __forceinline__ void side_projection(const Params& p, float* smem) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, o0 = ((int)blockIdx.x - p.main_grid) * 4;
+    const int t0 = (warp & 1) * 8;
+    float v[32];   // [token - t0][output]
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    const float* w = p.side_w + (uint64_t)o0 * p.side_k;
+    if (warp < 24)
+        for (int k = (warp >> 1) * 128 + lane * 4; k < p.side_k; k += 12 * 128) {
+            float4 wv[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) wv[j] = *reinterpret_cast<const float4*>(w + (uint64_t)j * p.side_k + k);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (t0 + i >= p.side_rows) continue;
+                const float4 x = __ldcg(reinterpret_cast<const float4*>(p.side_x + (uint64_t)(t0 + i) * p.side_k + k));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[4 * i + j] = fmaf(wv[j].w, x.w, fmaf(wv[j].z, x.z, fmaf(wv[j].y, x.y, fmaf(wv[j].x, x.x, v[4 * i + j]))));
+            }
+        }
+#pragma unroll
+    for (int n = 16; n >= 1; n >>= 1) {   // lane l ends with value l
+        const bool up = lane & n;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, n);
+        }
+    }
+    if (warp < 24) smem[warp * 32 + lane] = v[0];
+    else {   // the spare warp: per-token scale, two lanes a token
+        const int tok = lane & 15;
+        float ss = 0.f;
+#pragma unroll 8
+        for (int q = lane >> 4; q < p.n_sumsq; q += 2) ss += __ldcg(p.sumsq + q * MAX_ROWS + tok);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+        if (lane < 16) smem[24 * 32 + tok] = 1.0f / sqrtf(ss / p.norm_k + p.eps);
+    }
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        const int tok = threadIdx.x >> 2, j = threadIdx.x & 3, par = tok >> 3, idx = 4 * (tok & 7) + j;
+        float t = 0.f;
+#pragma unroll
+        for (int w2 = 0; w2 < 12; ++w2) t += smem[(2 * w2 + par) * 32 + idx];
+        if (tok < p.side_rows && o0 + j < p.side_n) p.side_out[(uint64_t)tok * p.side_n + o0 + j] = t * smem[24 * 32 + tok];
+    }
+}
 
 // The eight MMAs of half h = 2 h2 + C of an entry into one accumulator (the first of them overwrites it when the half is
 // the accumulator's first of the entry).
@@ -102,6 +156,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
     __shared__ int abort_flag;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp-uniform by construction
+    if ((int)blockIdx.x >= p.main_grid) {
+        pdl_launch_dependents();
+        pdl_wait();
+        side_projection(p, reinterpret_cast<float*>(smem));
+        return;
+    }
     int row_tiles = p.row_tiles, kblocks = p.kblocks, splits = p.splits, cps = p.ctas_per_split;
     if (p.tile_map || p.kb_map) {   // the lists come from the preceding kernel: nothing may be fetched before it is complete
         pdl_wait();
@@ -472,6 +532,13 @@ dfl_status launch_gemm_ts(cudaStream_t st, const QMatrix& m, const uint8_t* acts
     p.n_kb = ep.n_kb;
     int grid = p.ctas_per_split * splits;
     if (ep.kb_map && ep.dynamic_splits && grid < sm_count()) grid = sm_count();   // room for the geometry chosen on the device
+    p.main_grid = grid;
+    p.side_w = ep.side_w; p.side_x = ep.side_x; p.side_out = ep.side_out;
+    p.side_n = ep.side_n; p.side_k = ep.side_k; p.side_rows = ep.side_rows;
+    if (ep.side_w) {
+        if (ep.side_n % 4 || ep.side_k % 4 || !ep.sumsq) return fail(DFL_ERR_BAD_SHAPE, "gemm: side projection shape");
+        grid += ep.side_n / 4;
+    }
     switch (m.dtype) {
         case DFL_Q4_K: return ts::launch_t<DFL_Q4_K>(st, p, grid, pdl);
         case DFL_Q5_K: return ts::launch_t<DFL_Q5_K>(st, p, grid, pdl);

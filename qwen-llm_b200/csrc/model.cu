@@ -255,15 +255,24 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             out_proj = &L.wo;
             ++ai;
         } else {
-            // one stream, one chain: qkv, z (its own matrix when its format differs), then the whole mixer
-            DFL_CHECK(launch_group(st, L.in_qkv_z, sc->acts_h, sc->part, ep_norm, s->err));
+            // one stream, one chain: qkv, z (its own matrix when its format differs) with alpha / beta behind it, the mixer
+            const MatGroup& G = L.in_qkv_z;
+            const bool ab_rides = m->act_layout == ACT_TS && gg.n_v % 2 == 0;
+            for (size_t i = 0; i < G.mats.size(); ++i) {
+                GemmEpilogue ep = ep_norm;
+                if (i + 1 == G.mats.size() && ab_rides) {
+                    ep.side_w = L.w_ab; ep.side_x = sc->xn; ep.side_out = sc->ab[gi];
+                    ep.side_n = 2 * gg.n_v; ep.side_k = (int)H; ep.side_rows = (int)n;
+                }
+                DFL_CHECK(launch_gemm_fewrow(st, G.mats[i], sc->acts_h, sc->part + G.col_off[i], G.splits, ep, s->err, pdl_enabled(), G.total_cols));
+            }
+            if (!ab_rides) DFL_CHECK(launch_small_matmul(st, L.w_ab, sc->xn, (int)H, (int)n, H, 2 * gg.n_v, ep_norm, sc->ab[gi], 2 * gg.n_v));
             const int cur = s->ssm_cur[gi];
             GdnMixParams p;
             p.g = gg;
             p.part = sc->part; p.splits = L.in_qkv_z.splits; p.ld_part = (int)L.in_qkv_z.total_cols; p.z_col = gg.conv_dim(); p.n_rows = (int)n;
             p.conv_w = L.conv_w; p.conv_in = s->conv[cur][gi]; p.conv_out = s->conv[cur ^ 1][gi];
             p.state_in = s->ssm[cur][gi]; p.state_out = s->ssm[cur ^ 1][gi];
-            p.w_ab = L.w_ab; p.xn = sc->xn; p.sumsq = sc->sumsq; p.k = (int)H; p.n_sumsq = kb_h; p.norm_k = (float)H; p.eps = 1e-6f;
             p.dt_bias = L.dt_bias; p.a_log = L.a_log; p.norm_w = L.ssm_norm_w;
             p.qkv_raw = sc->qkv_raw[gi]; p.q_n = sc->q_n[gi]; p.k_n = sc->k_n[gi]; p.v = sc->v[gi]; p.ab = sc->ab[gi];
             p.acts = sc->acts_v; p.layout = m->act_layout; p.err = s->err;
@@ -1026,7 +1035,7 @@ dfl_status restore_partial_launch(const dfl_model* m, dfl_session* s, dfl_scratc
         const LayerW& L = m->layers[il];
         if (L.is_attn) continue;
         const int cur = s->ssm_cur[gi];  // advanced state; cur ^ 1 still holds the pre-block state
-        dfl_status st = launch_gdn_rescan(s->st, gg, s->ssm[cur ^ 1][gi], s->ssm[cur][gi], sc->q_n[gi], sc->k_n[gi], sc->v[gi], sc->ab[gi], L.dt_bias,
+        dfl_status st = launch_gdn_rescan(s->st, gg, s->ssm[cur ^ 1][gi], s->ssm[cur][gi], sc->k_n[gi], sc->v[gi], sc->ab[gi], L.dt_bias,
                                           L.a_log, (int)n_keep);
         if (st == DFL_OK) st = launch_gdn_conv_restore(s->st, gg, s->conv[cur ^ 1][gi], sc->qkv_raw[gi], (int)n_keep, s->conv[cur][gi]);
         if (st != DFL_OK) { s->poisoned = true; return st; }

@@ -291,21 +291,18 @@ struct GdnMixParams {
     float* conv_out = nullptr;        // ... and after it (another buffer)
     const float* state_in = nullptr;
     float* state_out = nullptr;
-    // alpha / beta projections: [2 n_v][k] f32 over the layer's normalised input
-    const float *w_ab = nullptr, *xn = nullptr, *sumsq = nullptr;
-    int k = 0, n_sumsq = 0;
-    float norm_k = 1.f, eps = 0.f;
     const float *dt_bias = nullptr, *a_log = nullptr, *norm_w = nullptr;
+    const float* ab = nullptr;     // [16][2 n_v]: alpha projections, then beta projections
     // the block's rows, kept for a rollback
-    float *qkv_raw = nullptr, *q_n = nullptr, *k_n = nullptr, *v = nullptr, *ab = nullptr;
+    float *qkv_raw = nullptr, *q_n = nullptr, *k_n = nullptr, *v = nullptr;
     uint8_t* acts = nullptr;
     int layout = 0;
     int* err = nullptr;
 };
 dfl_status launch_gdn_mix(cudaStream_t st, const GdnMixParams& p);
 // Advances the recurrent state over the first n_rows kept rows of a block (the re-scan of a partial accept).
-dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* state_in, float* state_out, const float* q_n, const float* k_n,
-                             const float* v, const float* ab, const float* dt_bias, const float* a_log, int n_rows);
+dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* state_in, float* state_out, const float* k_n, const float* v,
+                             const float* ab, const float* dt_bias, const float* a_log, int n_rows);
 // conv state := last (conv_k-1) rows of {pre-block conv rows, raw qkv rows 0..n_keep-1}
 dfl_status launch_gdn_conv_restore(cudaStream_t st, const GdnGeom& g, const float* conv_pre, const float* qkv_raw, int n_keep,
                                    float* conv_state);

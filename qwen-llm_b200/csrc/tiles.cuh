@@ -206,6 +206,11 @@ struct GemmEpilogue {
     // n_kb[1] / n_kb[2] (when n_kb[1] > 0): split count and CTAs per split to use for this list length, their product
     // at most 148, the splits at most the launch's own; the caller sums that many partial slices
     bool dynamic_splits = false;
+    // A small f32 projection of the same rows that rides along (tensor-memory family only) on CTAs of its own behind the GEMM's:
+    // side_out[tok][j] = rs[tok] * sum_k side_x[tok][k] * side_w[j][k], j < side_n (a multiple of 4), rs from sumsq as above.
+    const float *side_w = nullptr, *side_x = nullptr;
+    float* side_out = nullptr;
+    int side_n = 0, side_k = 0, side_rows = 0;
 };
 int gemm_choose_splits(const QMatrix& m);
 int gemm_max_kblocks_per_cta(int dtype);  // column blocks one CTA can keep resident
