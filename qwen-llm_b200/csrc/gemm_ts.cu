@@ -50,8 +50,9 @@ __device__ __forceinline__ uint64_t src_block_index(uint64_t row, int kb, int kb
 
 template <int DT>
 __global__ void retile_ts_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, uint64_t n_out, int kblocks, int kb_group) {
-    constexpr int SRC_BLK = DT == DFL_Q4_K ? 144 : DT == DFL_Q5_K ? 176 : 210;
-    constexpr int STAGE = DT == DFL_Q4_K ? STAGE_Q4_K : DT == DFL_Q5_K ? STAGE_Q5_K : STAGE_Q6_K;
+    static_assert(DT == DFL_Q4_K || DT == DFL_Q5_K, "Q6_K and Q8_0 have packers of their own");
+    constexpr int SRC_BLK = DT == DFL_Q4_K ? 144 : 176;
+    constexpr int STAGE = DT == DFL_Q4_K ? STAGE_Q4_K_TS : STAGE_Q5_K_TS;
     const uint64_t tile_id = blockIdx.x;
     const int kb = (int)(tile_id % kblocks);
     const uint64_t rt = tile_id / kblocks;
@@ -62,11 +63,32 @@ __global__ void retile_ts_kernel(const uint8_t* __restrict__ src, uint8_t* __res
 #pragma unroll
         for (int b = 0; b < 16; ++b) out[b] = 0;
         const int off = idx * 16;
-        if (DT == DFL_Q4_K || DT == DFL_Q5_K) {
-            const int qs_src = DT == DFL_Q4_K ? 16 : 48;
+        const int qs_src = DT == DFL_Q4_K ? 16 : 48;
+        auto block_of = [&](int r) -> const uint8_t* {   // null beyond the matrix
+            const uint64_t row = rt * TILE_R + r;
+            return row < n_out ? src + src_block_index(row, kb, kblocks, n_out, kb_group) * (uint64_t)SRC_BLK : nullptr;
+        };
+        if (off < TSQ4_OFF_QS) {   // four rows' d, dmin or four rows' scale bytes
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const bool scales = off >= TSQ4_OFF_SC;
+                const int w = (off - (scales ? TSQ4_OFF_SC : 0)) / 4 + x, r = w & 127, kp = w >> 7;
+                const uint8_t* blk = block_of(r);
+                if (!blk) continue;
+                if (!scales) {
+                    for (int b = 0; b < 4; ++b) out[4 * x + b] = blk[b];
+                } else {
+                    for (int b = 0; b < 2; ++b) {
+                        uint32_t sc, m;
+                        k4_scale_min(blk + 4, 2 * kp + b, sc, m);
+                        out[4 * x + 2 * b] = (uint8_t)sc;
+                        out[4 * x + 2 * b + 1] = (uint8_t)m;
+                    }
+                }
+            }
+        } else {
             int r, src_off;
-            if (off < TSQ4_OFF_QS) { r = idx; src_off = 0; }                                  // header
-            else if (off < TSQ4_OFF_QS + 16384) {                                             // qs [kp][half][row]
+            if (off < TSQ4_OFF_QS + 16384) {                                                  // qs [kp][half][row]
                 const int i = idx - TSQ4_OFF_QS / 16;
                 r = i & 127;
                 src_off = qs_src + 32 * (i >> 8) + 16 * ((i >> 7) & 1);
@@ -75,23 +97,9 @@ __global__ void retile_ts_kernel(const uint8_t* __restrict__ src, uint8_t* __res
                 r = i & 127;
                 src_off = 16 + 16 * (i >> 7);
             }
-            const uint64_t row = rt * TILE_R + r;
-            if (row < n_out) {
-                const uint8_t* blk = src + src_block_index(row, kb, kblocks, n_out, kb_group) * (uint64_t)SRC_BLK + src_off;
+            if (const uint8_t* blk = block_of(r)) {
 #pragma unroll
-                for (int b = 0; b < 16; ++b) out[b] = blk[b];
-                if (off < TSQ4_OFF_QS) {
-                    // header: d, dmin, then the eight (scale, min) pairs as 12-bit fields, pair j at bit 12 j
-                    uint32_t f[3] = {0, 0, 0};
-                    for (int j = 0; j < 8; ++j) {
-                        uint32_t sc, m;
-                        k4_scale_min(blk + 4, j, sc, m);
-                        const uint64_t v = (uint64_t)(sc | (m << 6)) << ((12 * j) & 31);
-                        f[(12 * j) >> 5] |= (uint32_t)v;
-                        if (((12 * j) >> 5) < 2) f[((12 * j) >> 5) + 1] |= (uint32_t)(v >> 32);
-                    }
-                    for (int b = 0; b < 12; ++b) out[4 + b] = (uint8_t)(f[b >> 2] >> (8 * (b & 3)));
-                }
+                for (int b = 0; b < 16; ++b) out[b] = blk[src_off + b];
             }
         }
         *reinterpret_cast<uint4*>(stage + off) = *reinterpret_cast<const uint4*>(out);
@@ -133,13 +141,11 @@ __global__ void decode_tiles_ts_kernel(const uint8_t* __restrict__ tiles, int dt
     const uint8_t* stage = tiles + (rt * kblocks + kb) * (uint64_t)stage_bytes_of(dtype, LAYOUT_TS);
     float v = 0.f;
     if (dtype == DFL_Q4_K || dtype == DFL_Q5_K) {
-        const uint8_t* h = stage + r * 16;
+        const uint8_t* h = stage + r * 4;
         const float d = __half2float(__ushort_as_half((unsigned short)(h[0] | (h[1] << 8))));
         const float dmin = __half2float(__ushort_as_half((unsigned short)(h[2] | (h[3] << 8))));
-        const uint32_t* f = reinterpret_cast<const uint32_t*>(h + 4);
-        const int bit = 12 * (k >> 5);
-        const uint64_t two = (uint64_t)f[bit >> 5] | ((uint64_t)((bit >> 5) < 2 ? f[(bit >> 5) + 1] : 0u) << 32);
-        const uint32_t pair = (uint32_t)(two >> (bit & 31)) & 0xfffu, sc = pair & 63u, m = pair >> 6;
+        const uint8_t* pr = stage + TSQ4_OFF_SC + ((k >> 6) * 128 + r) * 4 + 2 * ((k >> 5) & 1);
+        const uint32_t sc = pr[0], m = pr[1];
         const int kp = k >> 6, hi = (k >> 5) & 1, l = k & 31;
         const uint8_t byte = stage[TSQ4_OFF_QS + ((kp * 2 + (l >> 4)) * 128 + r) * 16 + (l & 15)];
         uint32_t q = hi ? (byte >> 4) : (byte & 15);
@@ -266,9 +272,6 @@ constexpr uint32_t MAGIC = 0x64006400u;      // half2(1024, 1024): 1024 + small 
 constexpr uint32_t H2_NEG1024 = 0xe400e400u; // half2(-1024)
 constexpr uint32_t H2_16TH = 0x2c002c00u;    // half2(1/16)
 constexpr uint32_t H2_NEG64 = 0xd400d400u;   // half2(-64)
-// (a, b) small non-negative integers -> half2(a, b), exact
-__device__ __forceinline__ uint32_t int_pair_h2(uint32_t a, uint32_t b) { return h2sub((a | (b << 16)) | MAGIC, MAGIC); }
-
 struct UnitScales {
     float d, dmin;
 };
@@ -281,7 +284,7 @@ struct Fmt;
 // k-positions 2c, 2c + 1.
 template <int DT>
 struct FmtK45 {
-    static constexpr int STAGE = DT == DFL_Q4_K ? STAGE_Q4_K : STAGE_Q5_K;
+    static constexpr int STAGE = DT == DFL_Q4_K ? STAGE_Q4_K_TS : STAGE_Q5_K_TS;
     static constexpr int STAGES = KC == 4 ? (DT == DFL_Q4_K ? 7 : 6) : (DT == DFL_Q4_K ? 6 : 5);
     static constexpr int HALVES = 2;
     static constexpr bool HAS_MIN = true;
@@ -293,15 +296,14 @@ struct FmtK45 {
     __device__ static __forceinline__ void unpack(const uint8_t* st, int ps, int row, int kp2, uint32_t (&r)[32], uint32_t (&am)[8],
                                                   UnitScales& us) {
         const int kp = 2 * ps + kp2;
-        const uint4 h = reinterpret_cast<const uint4*>(st)[row];
+        const uint32_t dd = reinterpret_cast<const uint32_t*>(st)[row];
+        const uint32_t t = reinterpret_cast<const uint32_t*>(st + TSQ4_OFF_SC)[kp * 128 + row];   // sc0, m0, sc1, m1
         const uint4* qs = reinterpret_cast<const uint4*>(st + TSQ4_OFF_QS);
         const uint4 qa = qs[(kp * 2 + 0) * 128 + row], qb = qs[(kp * 2 + 1) * 128 + row];
-        us.d = __half2float(__ushort_as_half((unsigned short)(h.x & 0xffffu)));
-        us.dmin = __half2float(__ushort_as_half((unsigned short)(h.x >> 16)));
-        // (scale, min) pairs of sub-blocks 2kp and 2kp + 1: 24 bits at bit 24 kp of the 96-bit field h.y, h.z, h.w
-        const uint32_t t = (ps == 0 ? (kp2 ? __funnelshift_r(h.y, h.z, 24) : h.y) : (kp2 ? (h.w >> 8) : __funnelshift_r(h.z, h.w, 16)));
-        const uint32_t sc0 = t & 63u, m0 = (t >> 6) & 63u, sc1 = (t >> 12) & 63u, m1 = (t >> 18) & 63u;
-        const uint32_t s0 = int_pair_h2(sc0, sc0), s1 = int_pair_h2(sc1, sc1);
+        us.d = __half2float(__ushort_as_half((unsigned short)(dd & 0xffffu)));
+        us.dmin = __half2float(__ushort_as_half((unsigned short)(dd >> 16)));
+        // bytes under the exponent byte of 1024, minus 1024: half2(sc0, sc0), half2(sc1, sc1), half2(m0, m1)
+        const uint32_t s0 = h2sub(__byte_perm(t, 0x64646464u, 0x4040), MAGIC), s1 = h2sub(__byte_perm(t, 0x64646464u, 0x4242), MAGIC);
         const uint32_t cml = s0, cal = h2mul(s0, H2_NEG1024);                      // (1024 + q) * sc - 1024 sc
         const uint32_t cmh = h2mul(s1, H2_16TH), cah = h2mul(s1, H2_NEG64);        // (1024 + 16 q) * sc / 16 - 64 sc
         const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
@@ -328,7 +330,7 @@ struct FmtK45 {
             }
         }
         // column kp of the min-term A operand: the mins of this thread's two sub-blocks
-        am[0] = int_pair_h2(m0, m1);
+        am[0] = h2sub(__byte_perm(t, 0x64646464u, 0x4341), MAGIC);
     }
 };
 template <>

@@ -6,7 +6,9 @@
 // ggml byte counts except for Q6_K, ordered so that thread (row, kp) of the unpacking CTA - row = its
 // tensor-memory lane, kp = its quarter of the 256 columns - finds its bytes with conflict-free
 // 128-bit shared-memory loads:
-//   Q4_K: [128 x 16 B header {d, dmin, scales[12]}] [kp 4][half 2][row 128][16 B of qs]
+//   Q4_K: [row 128][f16 d, f16 dmin] [kp 4][row 128][scale, min, scale, min of sub-blocks 2 kp, 2 kp + 1, a byte each]
+//         [kp 4][half 2][row 128][16 B of qs]  (148 bytes a row instead of ggml's 144: byte scales come out with three byte
+//         permutes, ggml's twelve packed bytes cost some twenty shifts and masks per thread and block)
 //   Q5_K: as Q4_K, then [half 2][row 128][16 B of qh]
 //   Q6_K: [128 x 16 B scales i8] [128 x f16 d] [block 8][half 2][row 128][16 B of six-bit codes, one per byte]
 //         (35072 bytes per stage instead of ggml's 26880: see gemm_ts_q6k.cuh)
@@ -44,8 +46,9 @@ __host__ __device__ constexpr int tm_sums(int cap) { return 2 * 16 * cap * 2; }
 __host__ __device__ constexpr int tm_chunk(int cap) { return 4 * tm_bstage(cap) + tm_sums(cap); }
 constexpr int TM_CHUNK = tm_chunk(TM_TOK);
 
-constexpr int TSQ4_OFF_QS = 2048;
-constexpr int TSQ5_OFF_QH = 2048 + 16384;
+constexpr int TSQ4_OFF_SC = 512;
+constexpr int TSQ4_OFF_QS = 2560;
+constexpr int TSQ5_OFF_QH = TSQ4_OFF_QS + 16384;
 constexpr int TSQ6_OFF_D = 2048;
 constexpr int TSQ6_OFF_QS = 2304;
 

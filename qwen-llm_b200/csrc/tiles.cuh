@@ -89,8 +89,15 @@ __host__ __device__ inline bool dtype_uses_bf16_acts(int dtype) { return dtype =
 constexpr int LAYOUT_FRAG = 0, LAYOUT_TS = 1;
 // Q6_K row-lane tiles hold one code per byte: [128 x 16 i8 scales][128 x f16 d][128 rows x 256 bytes]
 constexpr int STAGE_Q6_K_TS = 2304 + TILE_R * 256;  // 35072
+// Q4_K / Q5_K row-lane tiles hold the eight (scale, min) pairs as bytes: 20 bytes of header per row instead of 16
+constexpr int STAGE_Q4_K_TS = STAGE_Q4_K + TILE_R * 4, STAGE_Q5_K_TS = STAGE_Q5_K + TILE_R * 4;
 __host__ __device__ inline int stage_bytes_of(int dtype, int layout) {
-    return (dtype == DFL_Q6_K && layout == LAYOUT_TS) ? STAGE_Q6_K_TS : stage_bytes_of(dtype);
+    if (layout == LAYOUT_TS) {
+        if (dtype == DFL_Q4_K) return STAGE_Q4_K_TS;
+        if (dtype == DFL_Q5_K) return STAGE_Q5_K_TS;
+        if (dtype == DFL_Q6_K) return STAGE_Q6_K_TS;
+    }
+    return stage_bytes_of(dtype);
 }
 constexpr int ACT_F16 = 0, ACT_BF3 = 1, ACT_TS = 2, ACT_TSB = 3;
 constexpr int ACTTS_CHUNK = 16384 + 1536;  // tensor-memory kernel: B operand + min-term operand per 256 columns
