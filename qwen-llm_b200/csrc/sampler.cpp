@@ -13,6 +13,10 @@
 #include <string>
 #include <vector>
 
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
+
 #include "../../include/dflash_b200.h"
 
 namespace dfl {
@@ -59,12 +63,10 @@ enum SErr { S_OK = 0, S_EMPTY, S_NAN, S_TOO_LARGE, S_NO_CANDIDATES, S_PROPOSAL_R
 inline uint32_t descending_bits(float f) {
     uint32_t b;
     std::memcpy(&b, &f, 4);
-    const uint32_t asc = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-    return ~asc;
+    return b ^ (~(uint32_t)((int32_t)b >> 31) & 0x7fffffffu);   // no branch on the sign: it is a coin toss
 }
 inline double key_logit(uint64_t key) {
-    const uint32_t asc = ~(uint32_t)(key >> 32);
-    const uint32_t bits = (asc & 0x80000000u) ? (asc & 0x7fffffffu) : ~asc;
+    const uint32_t d = (uint32_t)(key >> 32), bits = d ^ (~(uint32_t)((int32_t)d >> 31) & 0x7fffffffu);
     float f;
     std::memcpy(&f, &bits, 4);
     return (double)f;
@@ -145,6 +147,150 @@ SErr order_keys(const float* logits, uint64_t n, uint64_t top_k, Buffers& b, uin
         *count = top_k;
     }
     return S_OK;
+}
+
+// ---- bounds for the nucleus ------------------------------------------------------------------------------------
+// exp(x) for x <= 0 to about 1e-12: x = n ln 2 + r, Taylor polynomial of degree 10 in |r| <= ln 2 / 2.  It only ever decides which
+// tokens the exact computation has to look at, never a value that is returned.
+constexpr double kLn2 = 0.6931471805599453, kLog2e = 1.4426950408889634;
+constexpr int kDegree = 10;
+constexpr double kInvFact[kDegree + 1] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320, 1.0 / 362880, 1.0 / 3628800};
+inline double exp_bound(double x) {
+    if (!(x > -700.0)) return 0.0;
+    const double n = std::nearbyint(x * kLog2e), r = x - n * kLn2;
+    double p = kInvFact[kDegree];
+    for (int i = kDegree - 1; i >= 0; --i) p = p * r + kInvFact[i];
+    uint64_t b = (uint64_t)(int64_t)(n + 1023.0) << 52;
+    double scale;
+    std::memcpy(&scale, &b, 8);
+    return p * scale;
+}
+// weights exp(l inv_t - shift) of a row summed by steps of 1/16 below the maximum in log weight (the last step takes the rest);
+// two tables, so that neighbours of one step do not wait for each other
+constexpr int kSteps = 1024;
+constexpr double kPerUnit = 16.0;
+struct StepMass { double m[2][kSteps]; };
+inline void add_mass(StepMass& sm, int table, double x) {
+    const double below = -x * kPerUnit;
+    sm.m[table][below < (double)(kSteps - 1) ? (below > 0.0 ? (int)below : 0) : kSteps - 1] += exp_bound(x);
+}
+void step_mass_plain(const float* l, uint64_t n, double inv_t, double shift, StepMass& sm) {
+    for (uint64_t i = 0; i < n; ++i) add_mass(sm, (int)(i & 1), (double)l[i] * inv_t - shift);
+}
+// a row's largest logit; false if it holds a NaN
+bool max_of_plain(const float* l, uint64_t n, float* mx) {
+    float m = l[0];
+    bool nan = false;
+    for (uint64_t i = 0; i < n; ++i) { nan |= std::isnan(l[i]); m = l[i] > m ? l[i] : m; }
+    *mx = m;
+    return !nan;
+}
+// keys of the tokens with logits of at least thr, in token order (keys: n + 1 entries)
+uint64_t collect_plain(const float* l, uint64_t n, float thr, uint64_t* keys) {
+    uint64_t c = 0;
+    for (uint64_t i = 0; i < n; ++i) {
+        keys[c] = ((uint64_t)descending_bits(l[i]) << 32) | i;
+        c += l[i] >= thr;
+    }
+    return c;
+}
+#if defined(__x86_64__)
+#define DFL_AVX2 __attribute__((target("avx2,fma")))
+DFL_AVX2 void step_mass_avx2(const float* l, uint64_t n, double inv_t, double shift, StepMass& sm) {
+    const __m256d it = _mm256_set1_pd(inv_t), sh = _mm256_set1_pd(shift), l2e = _mm256_set1_pd(kLog2e), ln2 = _mm256_set1_pd(kLn2),
+                  floor_x = _mm256_set1_pd(-700.0), per_unit = _mm256_set1_pd(-kPerUnit);
+    const __m256d last_step = _mm256_set1_pd((double)(kSteps - 1)), zero = _mm256_setzero_pd();
+    alignas(32) double w[16];
+    alignas(16) int32_t step[16];
+    uint64_t i = 0;
+    for (; i + 16 <= n; i += 16) {
+        __m256d x[4], k[4], r[4], p[4];
+        for (int j = 0; j < 4; ++j) x[j] = _mm256_fmsub_pd(_mm256_cvtps_pd(_mm_loadu_ps(l + i + 4 * j)), it, sh);
+        for (int j = 0; j < 4; ++j) k[j] = _mm256_round_pd(_mm256_mul_pd(x[j], l2e), _MM_FROUND_TO_NEAREST_INT | _MM_FROUND_NO_EXC);
+        for (int j = 0; j < 4; ++j) r[j] = _mm256_fnmadd_pd(k[j], ln2, x[j]);
+        for (int j = 0; j < 4; ++j) p[j] = _mm256_set1_pd(kInvFact[kDegree]);
+        for (int d = kDegree - 1; d >= 0; --d)
+            for (int j = 0; j < 4; ++j) p[j] = _mm256_fmadd_pd(p[j], r[j], _mm256_set1_pd(kInvFact[d]));
+        for (int j = 0; j < 4; ++j) {
+            const __m256i e = _mm256_slli_epi64(_mm256_cvtepi32_epi64(_mm_add_epi32(_mm256_cvtpd_epi32(k[j]), _mm_set1_epi32(1023))), 52);
+            const __m256d v = _mm256_mul_pd(p[j], _mm256_castsi256_pd(e));
+            _mm256_store_pd(w + 4 * j, _mm256_and_pd(v, _mm256_cmp_pd(x[j], floor_x, _CMP_GT_OQ)));
+            _mm_store_si128((__m128i*)(step + 4 * j), _mm256_cvttpd_epi32(_mm256_max_pd(_mm256_min_pd(_mm256_mul_pd(x[j], per_unit), last_step), zero)));
+        }
+        for (int j = 0; j < 16; ++j) sm.m[j & 1][step[j]] += w[j];
+    }
+    for (; i < n; ++i) add_mass(sm, (int)(i & 1), (double)l[i] * inv_t - shift);
+}
+DFL_AVX2 bool max_of_avx2(const float* l, uint64_t n, float* mx) {
+    if (n < 16) return max_of_plain(l, n, mx);
+    __m256 m0 = _mm256_loadu_ps(l), m1 = _mm256_loadu_ps(l + 8), bad = _mm256_setzero_ps();
+    uint64_t i = 0;
+    for (; i + 16 <= n; i += 16) {
+        const __m256 a = _mm256_loadu_ps(l + i), b = _mm256_loadu_ps(l + i + 8);
+        bad = _mm256_or_ps(bad, _mm256_or_ps(_mm256_cmp_ps(a, a, _CMP_UNORD_Q), _mm256_cmp_ps(b, b, _CMP_UNORD_Q)));
+        m0 = _mm256_max_ps(m0, a);
+        m1 = _mm256_max_ps(m1, b);
+    }
+    float t[8];
+    _mm256_storeu_ps(t, _mm256_max_ps(m0, m1));
+    float m = t[0];
+    bool nan = _mm256_movemask_ps(bad) != 0;
+    for (int j = 1; j < 8; ++j) m = t[j] > m ? t[j] : m;
+    for (; i < n; ++i) { nan |= std::isnan(l[i]); m = l[i] > m ? l[i] : m; }
+    *mx = m;
+    return !nan;
+}
+DFL_AVX2 uint64_t collect_avx2(const float* l, uint64_t n, float thr, uint64_t* keys) {
+    const __m256 t = _mm256_set1_ps(thr);
+    uint64_t c = 0, i = 0;
+    for (; i + 8 <= n; i += 8) {
+        unsigned m = (unsigned)_mm256_movemask_ps(_mm256_cmp_ps(_mm256_loadu_ps(l + i), t, _CMP_GE_OQ));
+        if (!m) continue;
+        for (uint64_t j = i; j < i + 8; ++j, m >>= 1) {   // all eight written, the count moves past those that belong
+            keys[c] = ((uint64_t)descending_bits(l[j]) << 32) | j;
+            c += m & 1u;
+        }
+    }
+    for (; i < n; ++i)
+        if (l[i] >= thr) keys[c++] = ((uint64_t)descending_bits(l[i]) << 32) | i;
+    return c;
+}
+inline bool have_avx2() {
+    static const bool yes = __builtin_cpu_supports("avx2") && __builtin_cpu_supports("fma");
+    return yes;
+}
+inline void step_mass(const float* l, uint64_t n, double inv_t, double shift, StepMass& sm) {
+    have_avx2() ? step_mass_avx2(l, n, inv_t, shift, sm) : step_mass_plain(l, n, inv_t, shift, sm);
+}
+inline bool max_of(const float* l, uint64_t n, float* mx) { return have_avx2() ? max_of_avx2(l, n, mx) : max_of_plain(l, n, mx); }
+inline uint64_t collect(const float* l, uint64_t n, float thr, uint64_t* keys) { return have_avx2() ? collect_avx2(l, n, thr, keys) : collect_plain(l, n, thr, keys); }
+#else
+inline void step_mass(const float* l, uint64_t n, double inv_t, double shift, StepMass& sm) { step_mass_plain(l, n, inv_t, shift, sm); }
+inline bool max_of(const float* l, uint64_t n, float* mx) { return max_of_plain(l, n, mx); }
+inline uint64_t collect(const float* l, uint64_t n, float thr, uint64_t* keys) { return collect_plain(l, n, thr, keys); }
+#endif
+// keys in ascending order; they arrive in token order, so long lists take a stable radix over the logit half, 11 bits a pass, as
+// many passes as the spread of the logits has bits
+void sort_keys(std::vector<uint64_t>& keys, std::vector<uint64_t>& scratch, uint64_t n) {
+    if (n < 2048) { std::sort(keys.begin(), keys.begin() + (ptrdiff_t)n); return; }
+    uint32_t lo = 0xffffffffu, hi = 0;
+    for (uint64_t i = 0; i < n; ++i) { const uint32_t d = (uint32_t)(keys[i] >> 32); lo = std::min(lo, d); hi = std::max(hi, d); }
+    int bits = 0;
+    while (bits < 32 && ((hi - lo) >> bits) != 0) ++bits;
+    const int passes = (bits + 10) / 11;
+    const uint64_t base = (uint64_t)lo << 32;
+    uint32_t hist[3][2048];
+    std::memset(hist, 0, sizeof(uint32_t) * 2048 * passes);
+    for (uint64_t i = 0; i < n; ++i)
+        for (int p = 0; p < passes; ++p) ++hist[p][((keys[i] - base) >> (32 + 11 * p)) & 2047];
+    if (scratch.size() < keys.size()) scratch.resize(keys.size());   // the two change places: a short one would have to grow again
+    for (int p = 0; p < passes; ++p) {
+        uint32_t off = 0, *h = hist[p];
+        for (int i = 0; i < 2048; ++i) { const uint32_t c = h[i]; h[i] = off; off += c; }
+        const int shift = 32 + 11 * p;
+        for (uint64_t i = 0; i < n; ++i) scratch[h[((keys[i] - base) >> shift) & 2047]++] = keys[i];
+        keys.swap(scratch);
+    }
 }
 
 struct Dist {
@@ -240,7 +386,63 @@ struct dfl_sampler {
         if (take_prepared(logits, d, &e, nan_token)) return e;
         return distribution(logits, n, d, nan_token, buf);
     }
+    // The nucleus without ordering the row.  The general path orders all n tokens and takes exp of each, although what leaves it
+    // is the short sorted prefix whose weights reach top_p of the total; the total itself only enters one comparison.  So: the
+    // total to EPS and its split by steps of log weight in one vectorised pass, the tokens of the steps that hold the share, then
+    // ordering, exact weights and exact running sum over those alone.  Where the running sum comes within EPS of the target
+    // the general path decides: tokens, weights, total and draws are its own, bit for bit.  Below 1024 tokens the step tables
+    // cost more than ordering.  16 rows of 151 936, four accepted: 4.4 -> 1.2 ms; one row with 44 600 in its nucleus 4.3 -> 2.6 ms.
+    bool nucleus(const float* logits, uint64_t n, Dist& d, Buffers& buf) const {
+        if (cfg.top_k != 0 || cfg.min_p > 0.0f || !(cfg.top_p < 1.0f) || n < 1024 || n > 0x7fffffffull) return false;
+        float mx;
+        if (!max_of(logits, n, &mx) || !std::isfinite(mx)) return false;
+        const double t = (double)cfg.temperature, inv_t = 1.0 / t, max_logit = (double)mx / t;
+        StepMass sm{};
+        step_mass(logits, n, inv_t, (double)mx * inv_t, sm);
+        double total = 0.0;
+        for (int b = 0; b < kSteps; ++b) total += sm.m[0][b] + sm.m[1][b];
+        if (!std::isfinite(max_logit) || !std::isfinite(total) || total < 0.5) return false;
+        // what separates this sum from one taken in sorted order: the polynomial, n roundings, and those of l / t
+        const double EPS = 1e-11 + 4e-16 * (double)n + 1e-15 * (std::fabs(max_logit) + 700.0);
+        const double share = (double)cfg.top_p;
+        const double lo = total * (1.0 - EPS) * share, hi = total * (1.0 + EPS) * share;
+        double mass = 0.0;
+        int b = 0;
+        for (; b < kSteps - 1; ++b) {
+            mass += sm.m[0][b] + sm.m[1][b];
+            if (mass > hi) break;
+        }
+        if (b == kSteps - 1) return false;
+        // the smallest logit of steps 0..b, less what rounding can move it
+        const double l_low = t * (max_logit - (double)(b + 1) / kPerUnit);
+        const float thr = std::nextafterf((float)(l_low - 1e-6 * (std::fabs(l_low) + std::fabs((double)mx))), -std::numeric_limits<float>::infinity());
+        if (!std::isfinite(thr)) return false;
+        if (buf.keys.size() < n + 1) buf.keys.resize(n + 1);
+        const uint64_t len = collect(logits, n, thr, buf.keys.data());
+        if (len == 0) return false;
+        sort_keys(buf.keys, buf.scratch, len);
+        const uint64_t* keys = buf.keys.data();
+        d.weights.resize(len);
+        double cum = 0.0, *w = d.weights.data();
+        for (uint64_t first = 0; first < len; first += 1024) {
+            const uint64_t last = std::min<uint64_t>(len, first + 1024);
+            for (uint64_t i = first; i < last; ++i) w[i] = key_logit(keys[i]) / t - max_logit;
+            for (uint64_t i = first; i < last; ++i) w[i] = std::exp(w[i]);
+            for (uint64_t i = first; i < last; ++i) {
+                cum += w[i];
+                if (cum < lo) continue;
+                if (cum < hi) return false;   // too close to call with a bound on the total
+                d.weights.resize(i + 1);
+                d.tokens.resize(i + 1);
+                for (uint64_t j = 0; j <= i; ++j) d.tokens[j] = key_token(keys[j]);
+                d.total = cum;
+                return true;
+            }
+        }
+        return false;
+    }
     SErr distribution(const float* logits, uint64_t n, Dist& d, uint64_t* nan_token, Buffers& buf) const {
+        if (!order_for(logits, n) && nucleus(logits, n, d, buf)) return S_OK;
         uint64_t len = 0;
         bool order_used = false;
         SErr e = order_keys(logits, n, cfg.top_k, buf, &len, nan_token, order_for(logits, n), &order_used);
