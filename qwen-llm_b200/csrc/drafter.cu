@@ -667,6 +667,7 @@ dfl_status dsession_snapshot_validate(const dfl_dsession* ds, uint32_t cols, uin
 }
 dfl_status dsession_snapshot_read(dfl_dsession* ds, const uint8_t* src, uint32_t cols, uint64_t n_bytes) {
     const dfl_dflash_config& c = ds->d->cfg;
+    std::vector<Upload> list;
     const uint64_t kv_dim = (uint64_t)c.n_kv_heads * c.head_dim, rows = (uint64_t)cols * kv_dim * 4;
     DFL_CHECK(dsession_snapshot_validate(ds, cols, n_bytes));
     ds->ctx_len = ds->ready = ds->pending_base = 0;

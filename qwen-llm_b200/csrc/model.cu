@@ -1176,29 +1176,27 @@ dfl_status dfl_session_restore_snapshot(const dfl_model* m, dfl_session* s, dfl_
     }
     const uint8_t* p = (const uint8_t*)blob + sizeof(h);
     void* rows_tmp = nullptr;
-    if (s->kv_mode == KV_F16_TILED && per_layer) DFL_CUDA(cudaMalloc(&rows_tmp, per_layer));
+    if (s->kv_mode == KV_F16_TILED && per_layer && !(rows_tmp = pool_alloc(per_layer))) return fail(DFL_ERR_OOM, "restore_snapshot: row buffer");
+    std::vector<Upload> list;
     for (int which = 0; which < 2; ++which)
         for (size_t ai = 0; ai < s->k_cache.size(); ++ai, p += per_layer) {
             if (!per_layer) continue;
             void* dst = which ? s->v_cache[ai] : s->k_cache[ai];
-            if (rows_tmp) {
-                cudaError_t ce = cudaMemcpyAsync(rows_tmp, p, per_layer, cudaMemcpyHostToDevice, s->st);
-                dfl_status cs = ce == cudaSuccess ? launch_kv_rows_to_tiled(s->st, rows_tmp, which != 0, (int)m->arch.n_kv_heads, 0, h.prefix_len, dst) : DFL_OK;
-                if (ce == cudaSuccess) ce = cudaStreamSynchronize(s->st);
-                if (cs != DFL_OK || ce != cudaSuccess) {
-                    cudaFree(rows_tmp);
-                    s->poisoned = true;   // part of the state has been overwritten
-                    DFL_CHECK(cs);
-                    DFL_CUDA(ce);
-                }
-            } else DFL_CUDA(cudaMemcpyAsync(dst, p, per_layer, cudaMemcpyHostToDevice, s->st));
+            if (!rows_tmp) { list.push_back({dst, p, per_layer, nullptr}); continue; }
+            list.push_back({rows_tmp, p, per_layer, [=] { return launch_kv_rows_to_tiled(s->st, rows_tmp, which != 0, (int)m->arch.n_kv_heads, 0, h.prefix_len, dst); }});
         }
-    if (rows_tmp) cudaFree(rows_tmp);
-    for (size_t gi = 0; gi < s->conv[0].size(); ++gi, p += (uint64_t)id.gdn_conv_elements_per_layer * 4)
-        DFL_CUDA(cudaMemcpyAsync(s->conv[s->ssm_cur[gi]][gi], p, (uint64_t)id.gdn_conv_elements_per_layer * 4, cudaMemcpyHostToDevice, s->st));
-    for (size_t gi = 0; gi < s->conv[0].size(); ++gi, p += (uint64_t)id.gdn_state_elements_per_layer * 4)
-        DFL_CUDA(cudaMemcpyAsync(s->ssm[s->ssm_cur[gi]][gi], p, (uint64_t)id.gdn_state_elements_per_layer * 4, cudaMemcpyHostToDevice, s->st));
-    DFL_CUDA(cudaStreamSynchronize(s->st));
+    const uint64_t conv_bytes = (uint64_t)id.gdn_conv_elements_per_layer * 4, state_bytes = (uint64_t)id.gdn_state_elements_per_layer * 4;
+    for (size_t gi = 0; gi < s->conv[0].size(); ++gi, p += conv_bytes) list.push_back({s->conv[s->ssm_cur[gi]][gi], p, conv_bytes, nullptr});
+    for (size_t gi = 0; gi < s->conv[0].size(); ++gi, p += state_bytes) list.push_back({s->ssm[s->ssm_cur[gi]][gi], p, state_bytes, nullptr});
+    if (!list.empty()) {
+        const dfl_status up = upload_all(s->st, list);
+        if (up != DFL_OK) {
+            s->poisoned = true;   // part of the state has been overwritten
+            cudaStreamSynchronize(s->st);
+        }
+        pool_free(rows_tmp);
+        DFL_CHECK(up);
+    }
     s->kv_n_pos = h.prefix_len;
     if (ds) DFL_CHECK(dsession_snapshot_read(ds, p, h.drafter_cols, h.drafter_bytes));
     return completion_check(s);

@@ -7,6 +7,7 @@
 #include <functional>
 #include <map>
 #include <string>
+#include <functional>
 #include <vector>
 
 #include "ops.cuh"
@@ -25,6 +26,14 @@ void* pool_alloc(size_t bytes);
 void* pool_alloc_host(size_t bytes);
 void pool_free(void* p);
 void pool_trim(int device);
+// The uploads in order on `st`, each followed by what `after` queues behind it; returns when all of it is done.
+struct Upload {
+    void* dst;
+    const void* src;
+    size_t bytes;
+    std::function<dfl_status()> after;
+};
+dfl_status upload_all(cudaStream_t st, const std::vector<Upload>& list);
 
 // Several matrices that consume the same activations and write side by side into one
 // partial buffer [splits][16][total_cols].
