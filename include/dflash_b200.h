@@ -663,6 +663,12 @@ dfl_status dfl_synth_tensor(int32_t device, int32_t dtype, uint64_t n_in, uint64
 dfl_status dfl_device_free(int32_t device, void* dev_ptr);
 dfl_status dfl_device_to_host(int32_t device, const void* dev_ptr, void* host, uint64_t n_bytes);
 
+/* Pinned host memory for results (logits, captured rows): copies into it run at link speed.  Blocks come from
+ * a bounded pool; NULL when it is exhausted, the size is above 64 MiB or there is no device - use any other
+ * memory then.  dfl_host_free gives a block back once no call that writes it is running. */
+void* dfl_host_alloc(uint64_t n_bytes);
+void dfl_host_free(void* ptr);
+
 #ifdef __cplusplus
 }
 #endif

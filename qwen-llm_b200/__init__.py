@@ -109,6 +109,9 @@ def lib():
         if hasattr(L, "dfl_gguf_tensors"):
             L.dfl_gguf_tensors.restype = C.POINTER(Tensor)
             L.dfl_gguf_tensor_count.restype = C.c_uint64
+        if hasattr(L, "dfl_host_alloc"):
+            L.dfl_host_alloc.restype = C.c_void_p
+            L.dfl_host_free.argtypes = [C.c_void_p]
         if hasattr(L, "dfl_sampler_next_unit_f64"):
             L.dfl_sampler_next_unit_f64.restype = C.c_double
         _LIB = L
@@ -122,6 +125,26 @@ def check(status):
 
 def _ptr(a, t=C.c_void_p):
     return a.ctypes.data_as(t)
+
+
+class _ResultBlock:
+    """A block of the library's pinned host memory; goes back to its pool with the last array that views it."""
+
+    def __init__(self, ptr, shape):
+        self.ptr = ptr
+        self.__array_interface__ = {"shape": shape, "typestr": "<f4", "data": (ptr, False), "version": 3}
+
+    def __del__(self):
+        if _LIB is not None:    # None only while the interpreter goes away
+            _LIB.dfl_host_free(self.ptr)
+
+
+def _result_f32(shape):
+    """A float32 array for a call to fill completely: pinned when the pool has a block (copies from the device then run at
+    link speed), else ordinary memory.  Below 64 KB neither the copy nor the page faults are worth it."""
+    n = 4 * int(np.prod(shape))
+    ptr = lib().dfl_host_alloc(C.c_uint64(n)) if n >= 65536 else None
+    return np.asarray(_ResultBlock(ptr, shape)) if ptr else np.zeros(shape, dtype=np.float32)
 
 
 def set_host_wait(mode):
@@ -379,7 +402,7 @@ def packed_verify(model, session, scratch, layer_ids, tokens, start_position, wa
     ids = _u32(layer_ids)
     am = np.zeros(n, dtype=np.int32)
     gap = np.zeros(n, dtype=np.float32)
-    logits = np.zeros((n, model.arch.vocab_size), dtype=np.float32) if want_logits else None
+    logits = _result_f32((n, model.arch.vocab_size)) if want_logits else None
     if want_order:
         order = np.zeros((scratch.block_size, model.arch.vocab_size), dtype=np.uint32)
         check(lib().dfl_scratch_set_order_host(scratch.h, _ptr(order, C.POINTER(C.c_uint32))))
@@ -448,7 +471,7 @@ def restore_pre_block(model, session, scratch, start_position):
 
 def single_token(model, session, scratch, layer_ids, token, position, want_hidden=True):
     ids = _u32(layer_ids)
-    logits = np.zeros(model.arch.vocab_size, dtype=np.float32)
+    logits = _result_f32((model.arch.vocab_size,))
     hidden = np.zeros((ids.size, model.arch.hidden_size), dtype=np.float32) if (want_hidden and ids.size) else None
     check(lib().dfl_single_token(model.h, session.h, scratch.h, _ptr(ids) if ids.size else None, C.c_uint32(ids.size),
                                  C.c_int32(int(token)), C.c_uint32(position), _ptr(logits),
@@ -727,7 +750,7 @@ class DSession:
     def draft_block(self, carry, noise_start_pos, want_logits=False):
         n = self.drafter.cfg.block_size
         out = np.zeros(n, dtype=np.int32)
-        logits = np.zeros((n, self.drafter.target.arch.vocab_size), dtype=np.float32) if want_logits else None
+        logits = _result_f32((n, self.drafter.target.arch.vocab_size)) if want_logits else None
         check(lib().dfl_draft_block(self.h, C.c_int32(int(carry)), C.c_uint32(noise_start_pos), _ptr(out),
                                     _ptr(logits) if want_logits else None))
         return out, logits
@@ -741,8 +764,10 @@ class DSession:
 def prefill(model, session, scratch, layer_ids, ids, start_position=0, feed_drafter=None, want_hidden=False, want_logits=True):
     ids = np.ascontiguousarray(ids, dtype=np.int32)
     lids = _u32(layer_ids)
-    hidden = np.zeros((ids.size, scratch.k, model.arch.hidden_size), dtype=np.float32) if want_hidden else None
-    logits = np.zeros(model.arch.vocab_size, dtype=np.float32) if want_logits else None
+    hidden_shape = (ids.size, scratch.k, model.arch.hidden_size)
+    # with fewer capture layers than the scratch has slots, part of the rows stays zero
+    hidden = None if not want_hidden else _result_f32(hidden_shape) if lids.size == scratch.k else np.zeros(hidden_shape, dtype=np.float32)
+    logits = _result_f32((model.arch.vocab_size,)) if want_logits else None
     check(lib().dfl_prefill(model.h, session.h, scratch.h, _ptr(lids) if lids.size else None, C.c_uint32(lids.size), _ptr(ids),
                             C.c_uint64(ids.size), C.c_uint32(start_position), feed_drafter.h if feed_drafter is not None else None,
                             _ptr(hidden) if want_hidden else None, _ptr(logits) if want_logits else None))

@@ -925,7 +925,11 @@ dfl_status dfl_packed_verify(const dfl_model* m, dfl_session* s, dfl_scratch* sc
         // the rows' order for the host sampler, produced while the logits travel
         const uint64_t V = m->arch.vocab_size;   // the device buffers exist: dfl_scratch_set_order_host made them
         st = launch_sort_rows_desc(s->st, sc->logits, (int)n, V, V, sc->sort_scratch, sc->order_dev);
-        if (st != DFL_OK) { s->poisoned = true; return st; }
+        if (st != DFL_OK) {
+            cudaStreamSynchronize(s->st);   // the logits' copy writes the caller's memory
+            s->poisoned = true;
+            return st;
+        }
         cudaMemcpyAsync(sc->order_host, sc->order_dev, (size_t)n * V * 4, cudaMemcpyDeviceToHost, s->st);
     }
     DFL_CHECK(completion_check(s));

@@ -23,6 +23,8 @@ struct Pool {
     std::multimap<std::pair<int, size_t>, void*> idle;
     std::map<int, size_t> idle_bytes;
     std::unordered_map<void*, Block> live;
+    std::unordered_map<void*, size_t> lent;   // host blocks in callers' hands (dfl_host_alloc)
+    size_t lent_bytes = 0;
 
     static void release(int device, void* p) {
         if (device == HOST) { cudaFreeHost(p); return; }
@@ -44,6 +46,11 @@ struct Pool {
     void* take(int device, size_t bytes) {
         bytes = (bytes + 511) / 512 * 512;
         if (bytes == 0) bytes = 512;
+        if (device == HOST) {   // results of any row count: eight sizes an octave, so that requests find each other's blocks
+            size_t step = 512;
+            while (step * 16 <= bytes) step *= 2;
+            bytes = (bytes + step - 1) / step * step;
+        }
         {
             std::lock_guard<std::mutex> lock(mu);
             auto it = idle.find({device, bytes});
@@ -98,3 +105,36 @@ void pool_free(void* p) { pool().give(p); }
 void pool_trim(int device) { pool().trim(device); pool().trim(HOST); }
 
 }  // namespace dfl
+
+// ---- result buffers ----------------------------------------------------------------------------------------------
+// A block's logits are 10 MB: into fresh pageable memory they travel at 6 GB/s (a staging copy and a page fault every 4 KB), into a
+// pinned block at the link's 55.  The blocks in use by callers are bounded like the idle ones; beyond that dfl_host_alloc
+// gives nothing and the caller falls back to memory of its own.
+extern "C" void* dfl_host_alloc(uint64_t n_bytes) {
+    using namespace dfl;
+    static_assert(kPoolHostBytes >= (64u << 20), "one result must fit");
+    if (n_bytes > (64ull << 20)) return nullptr;
+    Pool& p = pool();
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        if (p.lent_bytes + n_bytes > kPoolHostBytes) return nullptr;
+        p.lent_bytes += n_bytes;
+    }
+    void* b = p.take(HOST, n_bytes);
+    std::lock_guard<std::mutex> lock(p.mu);
+    if (b) p.lent[b] = n_bytes;
+    else p.lent_bytes -= n_bytes;
+    return b;
+}
+extern "C" void dfl_host_free(void* p) {
+    using namespace dfl;
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lock(pool().mu);
+        auto it = pool().lent.find(p);
+        if (it == pool().lent.end()) return;
+        pool().lent_bytes -= it->second;
+        pool().lent.erase(it);
+    }
+    pool().give(p);
+}
