@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "gemm_ts.cuh"
+#include "model.cuh"
 
 namespace dfl {
 
@@ -95,24 +96,26 @@ extern "C" dfl_status dfl_set_host_wait(int32_t mode) {
 }
 
 // Reads the device error word; non-zero maps to a status.
-dfl_status check_dev_err(cudaStream_t st, int* dev_err) {
-    int h = 0;
-    DFL_CUDA(cudaMemcpyAsync(&h, dev_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    DFL_CUDA(cudaStreamSynchronize(st));
-    if (h == 0) return DFL_OK;
-    int zero = 0;
-    cudaMemcpyAsync(dev_err, &zero, sizeof(int), cudaMemcpyHostToDevice, st);
-    cudaStreamSynchronize(st);
-    switch (h) {
+dfl_status dev_err_status(int code) {
+    switch (code) {
+        case 0: return DFL_OK;
         case DEV_ERR_WAIT_FULL:
         case DEV_ERR_WAIT_EMPTY:
         case DEV_ERR_WAIT_DRAIN:
         case DEV_ERR_WAIT_PEER:
-        case DEV_ERR_WAIT_FLAG: return fail(DFL_ERR_TIMEOUT, "device-side bounded wait gave up (code " + std::to_string(h) + ")");
+        case DEV_ERR_WAIT_FLAG: return fail(DFL_ERR_TIMEOUT, "device-side bounded wait gave up (code " + std::to_string(code) + ")");
         case DEV_ERR_OVERFLOW: return fail(DFL_ERR_CUDA, "activation outside the f16 operand range");
         case DEV_ERR_NONFINITE: return fail(DFL_ERR_ROUTE_STATUS, "expert routing met a NaN / Inf router logit (route status NONFINITE)");
-        default: return fail(DFL_ERR_CUDA, "device error word " + std::to_string(h));
+        default: return fail(DFL_ERR_CUDA, "device error word " + std::to_string(code));
     }
+}
+// `err` is pinned host memory that kernels write themselves: after the wait it is simply read, where a copy of four bytes to
+// pageable memory cost every call some 10 us
+dfl_status check_dev_err(cudaStream_t st, int* err) {
+    DFL_CUDA(cudaStreamSynchronize(st));
+    const int code = *static_cast<volatile int*>(err);
+    if (code) *err = 0;
+    return dev_err_status(code);
 }
 
 dfl_status qmatrix_create(int device, int dtype, uint64_t n_in, uint64_t n_out, const void* data, uint64_t n_bytes,
@@ -194,14 +197,13 @@ struct dfl_c1 {
     const dfl_qmatrix* w1;
     const dfl_qmatrix* head;
     cudaStream_t st;
-    float *x, *part1, *h, *part2, *logits, *gap;
+    float *x, *part1, *part2, *logits;
     uint8_t *acts1, *acts2;
-    int32_t* argmax;
-    void* am_scratch;
-    int* err;
     int splits1, splits2;
     cudaEvent_t e0, e1;
-    float* pinned;  // staging for results
+    // pinned host memory that the kernels read and write themselves: the results and the error word (HostOut), then the block's rows
+    struct HostOut { int32_t argmax[MAX_ROWS]; float gap[MAX_ROWS]; int err; }* out;
+    float* x_host;
 };
 
 extern "C" {
@@ -273,14 +275,14 @@ dfl_status dfl_fewrow_matmul(const dfl_qmatrix* m, const float* x_host, int32_t 
     uint8_t* acts = nullptr;
     int* err = nullptr;
     dfl_status s = DFL_OK;
-    auto cleanup = [&]() { cudaFree(x); cudaFree(part); cudaFree(y); cudaFree(acts); cudaFree(err); };
+    auto cleanup = [&]() { cudaFree(x); cudaFree(part); cudaFree(y); cudaFree(acts); pool_free(err); };
     if (cudaMalloc(&x, (size_t)n_rows * q.n_in * 4) != cudaSuccess || cudaMalloc(&part, (size_t)splits * MAX_ROWS * q.n_out * 4) != cudaSuccess ||
         cudaMalloc(&y, (size_t)n_rows * q.n_out * 4) != cudaSuccess || cudaMalloc(&acts, acts_bytes_for(q)) != cudaSuccess ||
-        cudaMalloc(&err, 4) != cudaSuccess) {
+        !(err = (int*)pool_alloc_host(4))) {
         cleanup();
         return fail(DFL_ERR_OOM, "fewrow_matmul: cudaMalloc failed");
     }
-    cudaMemset(err, 0, 4);
+    *err = 0;
     cudaMemcpy(x, x_host, (size_t)n_rows * q.n_in * 4, cudaMemcpyHostToDevice);
     s = launch_prep_acts_for(0, q, x, (int)q.n_in, n_rows, 1.0f, acts, err);
     if (s == DFL_OK) s = launch_gemm_fewrow(0, q, acts, part, splits, GemmEpilogue{}, err, false);
@@ -301,15 +303,14 @@ dfl_status dfl_argmax_top2(int32_t device, const float* logits_host, int32_t n_r
     DFL_CHECK(use_device(device));
     float *l = nullptr, *g = nullptr;
     int32_t* a = nullptr;
-    void* sc = nullptr;
-    auto cleanup = [&]() { cudaFree(l); cudaFree(g); cudaFree(a); cudaFree(sc); };
+    auto cleanup = [&]() { cudaFree(l); cudaFree(g); cudaFree(a); };
     if (cudaMalloc(&l, (size_t)n_rows * vocab * 4) != cudaSuccess || cudaMalloc(&g, n_rows * 4) != cudaSuccess ||
-        cudaMalloc(&a, n_rows * 4) != cudaSuccess || cudaMalloc(&sc, (size_t)n_rows * ARGMAX_PARTS * 16) != cudaSuccess) {
+        cudaMalloc(&a, n_rows * 4) != cudaSuccess) {
         cleanup();
         return fail(DFL_ERR_OOM, "argmax_top2: cudaMalloc failed");
     }
     cudaMemcpy(l, logits_host, (size_t)n_rows * vocab * 4, cudaMemcpyHostToDevice);
-    dfl_status s = launch_argmax_top2(0, l, n_rows, vocab, vocab, a, g, sc);
+    dfl_status s = launch_argmax_top2(0, l, n_rows, vocab, vocab, a, g);
     if (s == DFL_OK) {
         cudaError_t e1 = cudaMemcpy(argmax_out, a, n_rows * 4, cudaMemcpyDeviceToHost);
         cudaError_t e2 = cudaMemcpy(gap_out, g, n_rows * 4, cudaMemcpyDeviceToHost);
@@ -335,22 +336,21 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
     bool ok = cudaStreamCreateWithFlags(&p->st, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaMalloc(&p->x, MAX_ROWS * k1 * 4) == cudaSuccess;
     ok = ok && cudaMalloc(&p->part1, (size_t)p->splits1 * MAX_ROWS * n1 * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->h, MAX_ROWS * n1 * 4) == cudaSuccess;
     ok = ok && cudaMalloc(&p->part2, (size_t)p->splits2 * MAX_ROWS * v * 4) == cudaSuccess;
     ok = ok && cudaMalloc(&p->logits, MAX_ROWS * v * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->gap, MAX_ROWS * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->argmax, MAX_ROWS * 4) == cudaSuccess;
     ok = ok && cudaMalloc(&p->acts1, acts_bytes_for(w1->m)) == cudaSuccess;
     ok = ok && cudaMalloc(&p->acts2, acts_bytes_for(head->m)) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->am_scratch, MAX_ROWS * ARGMAX_PARTS * 16) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->err, 4) == cudaSuccess;
     ok = ok && cudaEventCreate(&p->e0) == cudaSuccess && cudaEventCreate(&p->e1) == cudaSuccess;
-    ok = ok && cudaMallocHost(&p->pinned, MAX_ROWS * 8) == cudaSuccess;
+    ok = ok && cudaMallocHost(&p->out, sizeof(dfl_c1::HostOut)) == cudaSuccess;
+    ok = ok && cudaMallocHost(&p->x_host, MAX_ROWS * k1 * 4) == cudaSuccess;
     if (!ok) {
         dfl_c1_destroy(p);
         return fail(DFL_ERR_OOM, std::string("c1_create: allocation failed: ") + cudaGetErrorString(cudaGetLastError()));
     }
-    cudaMemsetAsync(p->err, 0, 4, p->st);
+    memset(p->out, 0, sizeof(*p->out));
+    // the parts of the packed rows that the glue kernel does not write stay zero
+    cudaMemsetAsync(p->acts1, 0, acts_bytes_for(w1->m), p->st);
+    cudaMemsetAsync(p->acts2, 0, acts_bytes_for(head->m), p->st);
     cudaStreamSynchronize(p->st);
     *out = p;
     return DFL_OK;
@@ -359,28 +359,35 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
 void dfl_c1_destroy(dfl_c1* p) {
     if (!p) return;
     cudaSetDevice(p->w1->m.device);
-    cudaFree(p->x); cudaFree(p->part1); cudaFree(p->h); cudaFree(p->part2); cudaFree(p->logits); cudaFree(p->gap);
-    cudaFree(p->argmax); cudaFree(p->acts1); cudaFree(p->acts2); cudaFree(p->am_scratch); cudaFree(p->err);
-    if (p->pinned) cudaFreeHost(p->pinned);
+    cudaFree(p->x); cudaFree(p->part1); cudaFree(p->part2); cudaFree(p->logits); cudaFree(p->acts1); cudaFree(p->acts2);
+    if (p->out) cudaFreeHost(p->out);
+    if (p->x_host) cudaFreeHost(p->x_host);
     if (p->e0) cudaEventDestroy(p->e0);
     if (p->e1) cudaEventDestroy(p->e1);
     if (p->st) cudaStreamDestroy(p->st);
     delete p;
 }
 
-static dfl_status c1_enqueue(dfl_c1* p, int n_rows) {
+// Five launches: pack the rows, GEMM, sum and pack, GEMM, rank.  `x` is device memory or the pinned rows, which the packing kernel
+// reads across the bus itself (256 KB: less than a copy engine's start-up away); argmax, gap and the error word land in pinned
+// memory, so that a step waits for its stream once and copies nothing.
+static dfl_status c1_enqueue(dfl_c1* p, const float* x, int n_rows) {
     const QMatrix& a = p->w1->m;
     const QMatrix& b = p->head->m;
-    DFL_CHECK(launch_prep_acts_for(p->st, a, p->x, (int)a.n_in, n_rows, 1.0f, p->acts1, p->err));
-    DFL_CHECK(launch_gemm_fewrow(p->st, a, p->acts1, p->part1, p->splits1, GemmEpilogue{}, p->err, false));
-    DFL_CHECK(launch_reduce_partials(p->st, p->part1, p->splits1, n_rows, a.n_out, p->h, (int)a.n_out));
-    DFL_CHECK(launch_prep_acts_for(p->st, b, p->h, (int)a.n_out, n_rows, 1.0f, p->acts2, p->err));
-    DFL_CHECK(launch_gemm_fewrow(p->st, b, p->acts2, p->part2, p->splits2, GemmEpilogue{}, p->err, false));
-    DFL_CHECK(launch_reduce_partials(p->st, p->part2, p->splits2, n_rows, b.n_out, p->logits, (int)b.n_out));
-    DFL_CHECK(launch_argmax_top2(p->st, p->logits, n_rows, b.n_out, b.n_out, p->argmax, p->gap, p->am_scratch));
-    return DFL_OK;
+    int* err = &p->out->err;
+    GlueParams in;
+    in.mode = GLUE_COPY; in.x = const_cast<float*>(x); in.ld_x = (int)a.n_in; in.acts = p->acts1; in.bf3 = act_layout_of(a);
+    in.n_rows = n_rows; in.err = err;
+    DFL_CHECK(launch_glue(p->st, in, a.n_in));
+    DFL_CHECK(launch_gemm_fewrow(p->st, a, p->acts1, p->part1, p->splits1, GemmEpilogue{}, err, true));
+    GlueParams mid;
+    mid.part = p->part1; mid.splits = p->splits1; mid.ld_part = (int)a.n_out; mid.acts = p->acts2; mid.bf3 = act_layout_of(b);
+    mid.n_rows = n_rows; mid.err = err;
+    DFL_CHECK(launch_glue(p->st, mid, a.n_out));
+    DFL_CHECK(launch_gemm_fewrow(p->st, b, p->acts2, p->splits2 == 1 ? p->logits : p->part2, p->splits2, GemmEpilogue{}, err, true));
+    if (p->splits2 == 1) return launch_argmax_top2(p->st, p->logits, n_rows, b.n_out, b.n_out, p->out->argmax, p->out->gap);
+    return launch_reduce_argmax_top2(p->st, p->part2, p->splits2, n_rows, b.n_out, p->logits, b.n_out, p->out->argmax, p->out->gap);
 }
-
 dfl_status dfl_c1_upload(dfl_c1* p, const float* x_host, int32_t n_rows) {
     if (!p || !x_host) return fail(DFL_ERR_BAD_ARG, "c1_upload: null argument");
     if (n_rows < 1 || n_rows > MAX_ROWS) return fail(DFL_ERR_BAD_SHAPE, "c1: n_rows must be in [1, 16]");
@@ -395,11 +402,11 @@ dfl_status dfl_c1_run_resident(dfl_c1* p, int32_t n_rows, int32_t iters, float* 
     if (n_rows < 1 || n_rows > MAX_ROWS || iters < 1) return fail(DFL_ERR_BAD_SHAPE, "c1_run_resident: arguments");
     DFL_CHECK(use_device(p->w1->m.device));
     DFL_CUDA(cudaEventRecord(p->e0, p->st));
-    for (int i = 0; i < iters; ++i) DFL_CHECK(c1_enqueue(p, n_rows));
+    for (int i = 0; i < iters; ++i) DFL_CHECK(c1_enqueue(p, p->x, n_rows));
     DFL_CUDA(cudaEventRecord(p->e1, p->st));
     DFL_CUDA(cudaEventSynchronize(p->e1));
     DFL_CUDA(cudaEventElapsedTime(ms_total, p->e0, p->e1));
-    return check_dev_err(p->st, p->err);
+    return check_dev_err(p->st, &p->out->err);
 }
 
 dfl_status dfl_c1_step(dfl_c1* p, const float* x_host, int32_t n_rows, const int32_t* draft_ids, int32_t* argmax_out,
@@ -407,15 +414,13 @@ dfl_status dfl_c1_step(dfl_c1* p, const float* x_host, int32_t n_rows, const int
     if (!p || !x_host || !argmax_out || !gap_out) return fail(DFL_ERR_BAD_ARG, "c1_step: null argument");
     if (n_rows < 1 || n_rows > MAX_ROWS) return fail(DFL_ERR_BAD_SHAPE, "c1: n_rows must be in [1, 16]");
     DFL_CHECK(use_device(p->w1->m.device));
-    DFL_CUDA(cudaMemcpyAsync(p->x, x_host, (size_t)n_rows * p->w1->m.n_in * 4, cudaMemcpyHostToDevice, p->st));
-    DFL_CHECK(c1_enqueue(p, n_rows));
-    DFL_CUDA(cudaMemcpyAsync(p->pinned, p->argmax, n_rows * 4, cudaMemcpyDeviceToHost, p->st));
-    DFL_CUDA(cudaMemcpyAsync(p->pinned + MAX_ROWS, p->gap, n_rows * 4, cudaMemcpyDeviceToHost, p->st));
+    memcpy(p->x_host, x_host, (size_t)n_rows * p->w1->m.n_in * 4);
+    DFL_CHECK(c1_enqueue(p, p->x_host, n_rows));
     if (logits_host)
         DFL_CUDA(cudaMemcpyAsync(logits_host, p->logits, (size_t)n_rows * p->head->m.n_out * 4, cudaMemcpyDeviceToHost, p->st));
-    DFL_CHECK(check_dev_err(p->st, p->err));  // synchronises the stream
-    memcpy(argmax_out, p->pinned, n_rows * 4);
-    memcpy(gap_out, p->pinned + MAX_ROWS, n_rows * 4);
+    DFL_CHECK(check_dev_err(p->st, &p->out->err));
+    memcpy(argmax_out, p->out->argmax, n_rows * 4);
+    memcpy(gap_out, p->out->gap, n_rows * 4);
     if (n_accepted && draft_ids) {
         // greedy prefix acceptance (crates/qwen-cli/src/qwen/dflash.rs:838-852)
         int n = 0;

@@ -14,7 +14,7 @@ dfl_status use_device(int device);
 namespace {
 
 constexpr int STATIC_MAX_ROWS = MAX_ROWS;       // 16 rows: one speculative block
-constexpr int STATIC_PARTS = ARGMAX_PARTS;      // 64 column ranges per row
+constexpr int STATIC_PARTS = 64;                // column ranges per row
 constexpr int STATIC_MAX_DEVICES = 64;
 
 struct Best2 {

@@ -276,8 +276,7 @@ struct dfl_dsession {
     float *x = nullptr, *part = nullptr, *sumsq = nullptr, *q_rot = nullptr, *k_noise = nullptr, *v_noise = nullptr, *attn_part = nullptr;
     uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_q = nullptr, *acts_fc = nullptr, *acts_lm = nullptr;
     float *logits = nullptr, *gap = nullptr;
-    int32_t *argmax = nullptr, *tokens_dev = nullptr;
-    void* am_scratch = nullptr;
+    int32_t* argmax = nullptr;      // pinned host memory, written by the kernel (err too)
     // top-16 per row and the selector's gate rows W_h h of the last pass
     int32_t* topk_ids = nullptr;
     float *topk_vals = nullptr, *sel_h = nullptr;
@@ -295,7 +294,6 @@ struct dfl_dsession {
     // queue the target's rollback behind the drafter's launches instead of in front of them
     void (*after_enqueue)(void*) = nullptr;
     void* after_enqueue_arg = nullptr;
-    int32_t* pinned_i = nullptr;
     cudaStream_t st = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int* err = nullptr;
@@ -470,9 +468,6 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
     ds->acts_lm = (uint8_t*)alloc(acts_bytes(DFL_BF16, H));
     ds->logits = (float*)alloc(MAX_ROWS * V * 4);
     ds->gap = (float*)alloc(MAX_ROWS * 4);
-    ds->argmax = (int32_t*)alloc(MAX_ROWS * 4);
-    ds->tokens_dev = (int32_t*)alloc(MAX_ROWS * 4);
-    ds->am_scratch = alloc(MAX_ROWS * ARGMAX_PARTS * 16);
     ds->topk_ids = (int32_t*)alloc(MAX_ROWS * 16 * 4);
     ds->topk_vals = (float*)alloc(MAX_ROWS * 16 * 4);
     ds->topk_scratch = alloc(topk16_scratch_bytes(MAX_ROWS));
@@ -480,8 +475,8 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
         ds->sel_h = (float*)alloc((size_t)MAX_ROWS * c.selector_rank * 4);
         ds->acts_sel = (uint8_t*)alloc(acts_bytes(DFL_BF16, H));
     }
-    ds->err = (int*)alloc(4);
-    ok = ok && (ds->pinned_i = (int32_t*)pool_alloc_host(2 * MAX_ROWS * 4));
+    ok = ok && (ds->err = (int*)pool_alloc_host(4)) && (ds->argmax = (int32_t*)pool_alloc_host(MAX_ROWS * 4));
+    if (ok) *ds->err = 0;
     ok = ok && (ds->pinned_sel = (uint8_t*)pool_alloc_host(MAX_ROWS * 16 * 8 + (size_t)MAX_ROWS * c.selector_rank * 4));
     ok = ok && cudaEventCreate(&ds->ev0) == cudaSuccess && cudaEventCreate(&ds->ev1) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&ds->st_side, cudaStreamNonBlocking) == cudaSuccess;
@@ -503,7 +498,8 @@ void dfl_dsession_destroy(dfl_dsession* ds) {
     for (cudaStream_t st : {ds->st, ds->st_side})
         if (st) cudaStreamSynchronize(st);
     for (void* p : ds->allocs) pool_free(p);
-    pool_free(ds->pinned_i);
+    pool_free(ds->err);
+    pool_free(ds->argmax);
     pool_free(ds->pinned_sel);
     if (ds->ev0) cudaEventDestroy(ds->ev0);
     if (ds->ev1) cudaEventDestroy(ds->ev1);
@@ -521,9 +517,7 @@ struct dfl_dsession_view {
     cudaStream_t st;
     cudaEvent_t ev0, ev1;
     int* err;
-    const int32_t* argmax_dev;
     const float* logits_dev;
-    int32_t* pinned_i;
     uint32_t block_size, n_target_layers;
     const uint32_t* target_layer_ids;
     const dfl_model* target;
@@ -531,7 +525,7 @@ struct dfl_dsession_view {
 };
 void dfl_dsession_view_get(dfl_dsession* ds, dfl_dsession_view* out) {
     out->st = ds->st; out->ev0 = ds->ev0; out->ev1 = ds->ev1; out->err = ds->err;
-    out->argmax_dev = ds->argmax; out->logits_dev = ds->logits; out->pinned_i = ds->pinned_i;
+    out->logits_dev = ds->logits;
     out->has_selector = ds->d->has_selector ? 1 : 0;
     out->block_size = ds->d->cfg.block_size; out->n_target_layers = ds->d->cfg.n_target_layers;
     out->target_layer_ids = ds->d->cfg.target_layer_ids; out->target = ds->d->target;
@@ -667,20 +661,21 @@ dfl_status dsession_snapshot_validate(const dfl_dsession* ds, uint32_t cols, uin
 }
 dfl_status dsession_snapshot_read(dfl_dsession* ds, const uint8_t* src, uint32_t cols, uint64_t n_bytes) {
     const dfl_dflash_config& c = ds->d->cfg;
-    std::vector<Upload> list;
     const uint64_t kv_dim = (uint64_t)c.n_kv_heads * c.head_dim, rows = (uint64_t)cols * kv_dim * 4;
     DFL_CHECK(dsession_snapshot_validate(ds, cols, n_bytes));
     ds->ctx_len = ds->ready = ds->pending_base = 0;
     ds->pos_host.assign(reinterpret_cast<const uint32_t*>(src), reinterpret_cast<const uint32_t*>(src) + cols);
     if (cols) DFL_CUDA(cudaMemcpyAsync(ds->pos_ctx_dev, ds->pos_host.data(), (size_t)cols * 4, cudaMemcpyHostToDevice, ds->st));
     src += (size_t)cols * 4;
+    std::vector<Upload> list;
     for (uint32_t il = 0; il < c.n_layer && cols; ++il) {
-        DFL_CUDA(cudaMemcpyAsync(ds->k_ctx[il], src, rows, cudaMemcpyHostToDevice, ds->st));
-        DFL_CUDA(cudaMemcpyAsync(ds->v_ctx[il], src + rows, rows, cudaMemcpyHostToDevice, ds->st));
-        if (ds->ctx_tiles[il]) DFL_CHECK(launch_dctx_tiles(ds->st, ds->k_ctx[il], ds->v_ctx[il], (int)c.n_kv_heads, 0, cols, 0, ds->ctx_tiles[il]));
+        list.push_back({ds->k_ctx[il], src, rows, nullptr});
+        list.push_back({ds->v_ctx[il], src + rows, rows, nullptr});
+        if (ds->ctx_tiles[il])
+            list.back().after = [=] { return launch_dctx_tiles(ds->st, ds->k_ctx[il], ds->v_ctx[il], (int)c.n_kv_heads, 0, cols, 0, ds->ctx_tiles[il]); };
         src += 2 * rows;
     }
-    DFL_CUDA(cudaStreamSynchronize(ds->st));
+    if (!list.empty()) DFL_CHECK(upload_all(ds->st, list));
     ds->ctx_len = ds->ready = ds->pending_base = cols;
     return DFL_OK;
 }
@@ -709,10 +704,10 @@ dfl_status draft_core(dfl_dsession* ds, int32_t carry, uint32_t noise_start, boo
     ep_norm.n_sumsq = (int)(H / GLUE_COLS);
     ep_norm.norm_k = (float)H;
     ep_norm.eps = c.rms_norm_eps;
-    ds->pinned_i[0] = carry;
-    for (int i = 1; i < n; ++i) ds->pinned_i[i] = c.mask_token_id;
-    DFL_CUDA(cudaMemcpyAsync(ds->tokens_dev, ds->pinned_i, n * 4, cudaMemcpyHostToDevice, st));
-    DFL_CHECK(launch_embed_rows(st, tgt->embd_dtype, tgt->embd_ggml, H, ds->tokens_dev, n, ds->x, (int)H));
+    int32_t block[MAX_ROWS];
+    block[0] = carry;
+    for (int i = 1; i < n; ++i) block[i] = c.mask_token_id;
+    DFL_CHECK(launch_embed_block(st, tgt->embd_dtype, tgt->embd_ggml, H, block, n, ds->x, (int)H));
     auto norm_glue = [&](const float* part, int splits, int ld_part, const float* w, uint8_t* acts, int layout) -> dfl_status {
         GlueParams p;
         p.mode = GLUE_RESID;
@@ -779,10 +774,10 @@ dfl_status draft_core(dfl_dsession* ds, int32_t carry, uint32_t noise_start, boo
     const MatGroup& lm = tgt->lm_head;
     if (lm.splits == 1) {
         DFL_CHECK(launch_group(st, lm, ds->acts_lm, ds->logits, ep_norm, ds->err));
-        DFL_CHECK(launch_argmax_top2(st, ds->logits, n, V, V, ds->argmax, ds->gap, ds->am_scratch));
+        DFL_CHECK(launch_argmax_top2(st, ds->logits, n, V, V, ds->argmax, ds->gap));
     } else {
         DFL_CHECK(launch_group(st, lm, ds->acts_lm, ds->part, ep_norm, ds->err));
-        DFL_CHECK(launch_reduce_argmax_top2(st, ds->part, lm.splits, n, V, ds->logits, V, ds->argmax, ds->gap, ds->am_scratch));
+        DFL_CHECK(launch_reduce_argmax_top2(st, ds->part, lm.splits, n, V, ds->logits, V, ds->argmax, ds->gap));
     }
     ds->have_topk = false;
     if (topk || d->has_selector) {
@@ -841,10 +836,9 @@ dfl_status draft_block_topk(dfl_dsession* ds, int32_t carry, uint32_t noise_star
     if (carry < 0 || (uint32_t)carry >= tgt->arch.vocab_size) return fail(DFL_ERR_BAD_TOKEN, "draft_block: carry token out of range");
     const uint32_t n = ds->d->cfg.block_size;
     DFL_CHECK(draft_core(ds, carry, noise_start_pos, true));
-    DFL_CUDA(cudaMemcpyAsync(ds->pinned_i + MAX_ROWS, ds->argmax, n * 4, cudaMemcpyDeviceToHost, ds->st));
     DFL_CHECK(check_dev_err(ds->st, ds->err));
     out_tokens[0] = carry;
-    for (uint32_t i = 1; i < n; ++i) out_tokens[i] = ds->pinned_i[MAX_ROWS + i];
+    for (uint32_t i = 1; i < n; ++i) out_tokens[i] = ds->argmax[i];
     return DFL_OK;
 }
 
@@ -878,7 +872,6 @@ dfl_status dfl_draft_block(dfl_dsession* ds, int32_t carry, uint32_t noise_start
     if (carry < 0 || (uint32_t)carry >= tgt->arch.vocab_size) return fail(DFL_ERR_BAD_TOKEN, "draft_block: carry token out of range");
     const uint32_t n = ds->d->cfg.block_size;
     DFL_CHECK(draft_core(ds, carry, noise_start_pos, false));
-    DFL_CUDA(cudaMemcpyAsync(ds->pinned_i + MAX_ROWS, ds->argmax, n * 4, cudaMemcpyDeviceToHost, ds->st));
     if (logits_host) DFL_CUDA(cudaMemcpyAsync(logits_host, ds->logits, (size_t)n * tgt->arch.vocab_size * 4, cudaMemcpyDeviceToHost, ds->st));
     if (ds->d->has_selector) {   // select_draft_path: the walk replaces the per-row argmax
         SelectorHost h;
@@ -890,7 +883,7 @@ dfl_status dfl_draft_block(dfl_dsession* ds, int32_t carry, uint32_t noise_start
     }
     DFL_CHECK(check_dev_err(ds->st, ds->err));
     out_tokens[0] = carry;
-    for (uint32_t i = 1; i < n; ++i) out_tokens[i] = ds->pinned_i[MAX_ROWS + i];
+    for (uint32_t i = 1; i < n; ++i) out_tokens[i] = ds->argmax[i];
     return DFL_OK;
 }
 

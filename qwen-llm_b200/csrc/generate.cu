@@ -22,9 +22,7 @@ struct dfl_dsession_view {
     cudaStream_t st;
     cudaEvent_t ev0, ev1;
     int* err;
-    const int32_t* argmax_dev;
     const float* logits_dev;
-    int32_t* pinned_i;
     uint32_t block_size, n_target_layers;
     const uint32_t* target_layer_ids;
     const dfl_model* target;

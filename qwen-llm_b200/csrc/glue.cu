@@ -32,21 +32,42 @@ dfl_status launch_glue(cudaStream_t st, const GlueParams& p, uint64_t k) {
 }
 
 // ---- embedding rows ---------------------------------------------------------------
-__global__ void embed_rows_kernel(int dtype, const uint8_t* __restrict__ ggml, uint64_t h, const int32_t* tokens,
-                                  float* x, int ld) {
-    pdl_prologue();
-    const int tok = blockIdx.y;
+__device__ __forceinline__ void embed_one(int dtype, const uint8_t* __restrict__ ggml, uint64_t h, int32_t token, float* row) {
     const uint64_t col = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= h) return;
     const uint64_t row_bytes = h / 256 * (uint64_t)ggml_bytes_per_256(dtype);
-    const uint8_t* seg = ggml + (uint64_t)tokens[tok] * row_bytes + (col >> 8) * (uint64_t)ggml_bytes_per_256(dtype);
-    x[(uint64_t)tok * ld + col] = ggml_decode_elem(dtype, seg, (int)(col & 255));
+    const uint8_t* seg = ggml + (uint64_t)token * row_bytes + (col >> 8) * (uint64_t)ggml_bytes_per_256(dtype);
+    row[col] = ggml_decode_elem(dtype, seg, (int)(col & 255));
+}
+__global__ void embed_rows_kernel(int dtype, const uint8_t* __restrict__ ggml, uint64_t h, const int32_t* tokens,
+                                  float* x, int ld) {
+    pdl_prologue();
+    embed_one(dtype, ggml, h, tokens[blockIdx.y], x + (uint64_t)blockIdx.y * ld);
+}
+// A block's tokens ride in the launch itself: the copy that used to carry 64 bytes to the device cost a pass 3 us and the overlap
+// of its first kernel with the end of the pass before.
+struct BlockTokens { int32_t id[MAX_ROWS]; };
+__global__ void embed_block_kernel(int dtype, const uint8_t* __restrict__ ggml, uint64_t h, const BlockTokens tokens, float* x, int ld) {
+    pdl_prologue();
+    embed_one(dtype, ggml, h, tokens.id[blockIdx.y], x + (uint64_t)blockIdx.y * ld);
 }
 
 dfl_status launch_embed_rows(cudaStream_t st, int dtype, const uint8_t* ggml, uint64_t h, const int32_t* tokens, int n_rows,
                              float* x, int ld) {
     if (h % 256 || ggml_bytes_per_256(dtype) == 0) return fail(DFL_ERR_UNSUPPORTED, "embed_rows: dtype or width");
     launch_k(embed_rows_kernel, dim3(dim3((unsigned)((h + 255) / 256), (unsigned)n_rows)), dim3(256), 0, st, dtype, ggml, h, tokens, x, ld);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+dfl_status launch_embed_block(cudaStream_t st, int dtype, const uint8_t* ggml, uint64_t h, const int32_t* tokens_host, int n_rows,
+                              float* x, int ld) {
+    if (h % 256 || ggml_bytes_per_256(dtype) == 0) return fail(DFL_ERR_UNSUPPORTED, "embed_block: dtype or width");
+    if (n_rows < 1 || n_rows > MAX_ROWS) return fail(DFL_ERR_BAD_SHAPE, "embed_block: 1 to 16 rows");
+    BlockTokens t{};
+    for (int i = 0; i < n_rows; ++i) t.id[i] = tokens_host[i];
+    launch_k(embed_block_kernel, dim3((unsigned)((h + 255) / 256), (unsigned)n_rows), dim3(256), 0, st, dtype, ggml, h, t, x, ld);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

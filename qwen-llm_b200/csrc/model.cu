@@ -183,10 +183,10 @@ dfl_status head_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, uint32
     float* logits = sc->logits;
     if (lm.splits == 1) {
         DFL_CHECK(launch_group(st, lm, sc->acts_h, logits, ep_norm, s->err));
-        DFL_CHECK(launch_argmax_top2(st, logits, (int)n, V, V, sc->argmax, sc->gap, sc->am_scratch));
+        DFL_CHECK(launch_argmax_top2(st, logits, (int)n, V, V, sc->argmax, sc->gap));
     } else {
         DFL_CHECK(launch_group(st, lm, sc->acts_h, sc->part, ep_norm, s->err));
-        DFL_CHECK(launch_reduce_argmax_top2(st, sc->part, lm.splits, (int)n, V, logits, V, sc->argmax, sc->gap, sc->am_scratch));
+        DFL_CHECK(launch_reduce_argmax_top2(st, sc->part, lm.splits, (int)n, V, logits, V, sc->argmax, sc->gap));
     }
     return DFL_OK;
 }
@@ -222,9 +222,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
     ep_norm.norm_k = (float)H;
     ep_norm.eps = 1e-6f;
 
-    memcpy(sc->pinned_i, tokens, n * sizeof(int32_t));
-    DFL_CUDA(cudaMemcpyAsync(sc->tokens_dev, sc->pinned_i, n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    DFL_CHECK(launch_embed_rows(st, m->embd_dtype, m->embd_ggml, H, sc->tokens_dev, (int)n, sc->x, (int)H));
+    DFL_CHECK(launch_embed_block(st, m->embd_dtype, m->embd_ggml, H, tokens, (int)n, sc->x, (int)H));
 
     auto norm_glue = [&](const float* part, int splits, int ld_part, const float* norm_w, bool want_xn, float* capture,
                          const int32_t* splits_dev = nullptr) -> dfl_status {
@@ -706,7 +704,7 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
         s->ssm_cur.push_back(0);
     }
     if (ok && m->n_attn) ok = (s->attn_partials = (float*)pool_alloc(attn_partials_floats(m->attn_geom(), (uint32_t)cap_alloc) * 4)) != nullptr;   // two records per 128-position tile in tiled storage
-    ok = ok && (s->err = (int*)pool_alloc(4));
+    ok = ok && (s->err = (int*)pool_alloc_host(4));
     ok = ok && cudaEventCreate(&s->ev0) == cudaSuccess && cudaEventCreate(&s->ev1) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&s->st_side, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
@@ -717,7 +715,7 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
         dfl_session_destroy(s);
         return fail(DFL_ERR_OOM, "session_create: allocation failed: " + why);
     }
-    cudaMemsetAsync(s->err, 0, 4, s->st);
+    *s->err = 0;
     cudaStreamSynchronize(s->st);   // this session's memory only: other sessions' work goes on
     *out = s;
     return DFL_OK;
@@ -863,12 +861,8 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
         sc->qkv_raw.push_back(a0); sc->q_n.push_back(a2); sc->k_n.push_back(a3); sc->v.push_back(a4); sc->ab.push_back(a5);
     }
     alloc(&sc->logits, MAX_ROWS * V * 4);
-    alloc(&sc->gap, MAX_ROWS * 4);
-    alloc(&sc->argmax, MAX_ROWS * 4);
-    { uint8_t* am = nullptr; alloc(&am, MAX_ROWS * ARGMAX_PARTS * 16); sc->am_scratch = am; }
     alloc(&sc->capture, (size_t)MAX_ROWS * sc->k_layers * H * 4);
-    alloc(&sc->tokens_dev, MAX_ROWS * 4);
-    ok = ok && (sc->pinned_i = (int32_t*)pool_alloc_host(2 * MAX_ROWS * 4)) && (sc->pinned_f = (float*)pool_alloc_host(MAX_ROWS * 4));
+    ok = ok && (sc->argmax = (int32_t*)pool_alloc_host(MAX_ROWS * 4)) && (sc->gap = (float*)pool_alloc_host(MAX_ROWS * 4));
     if (!ok) {
         std::string why = cudaGetErrorString(cudaGetLastError());
         dfl_scratch_destroy(sc);
@@ -884,8 +878,8 @@ void dfl_scratch_destroy(dfl_scratch* sc) {
     cudaSetDevice(sc->m->device);
     cudaDeviceSynchronize();   // a scratch does not know the streams of the sessions that used it
     for (void* p : sc->allocs) pool_free(p);
-    pool_free(sc->pinned_i);
-    pool_free(sc->pinned_f);
+    pool_free(sc->argmax);
+    pool_free(sc->gap);
     if (sc->pinned_logits) cudaFreeHost(sc->pinned_logits);
     if (sc->pinned_order) cudaFreeHost(sc->pinned_order);
     if (sc->order_dev) cudaFree(sc->order_dev);
@@ -918,8 +912,6 @@ dfl_status dfl_packed_verify(const dfl_model* m, dfl_session* s, dfl_scratch* sc
     if (!argmax_out) return fail(DFL_ERR_BAD_ARG, "packed_verify: argmax_out is null");
     dfl_status st = verify_core(m, s, sc, layer_ids, n_layer_ids, tokens, n, start_position, true);
     if (st != DFL_OK) { s->poisoned = true; return st; }
-    cudaMemcpyAsync(sc->pinned_i + MAX_ROWS, sc->argmax, n * 4, cudaMemcpyDeviceToHost, s->st);
-    cudaMemcpyAsync(sc->pinned_f, sc->gap, n * 4, cudaMemcpyDeviceToHost, s->st);
     if (logits_host) cudaMemcpyAsync(logits_host, sc->logits, (size_t)n * m->arch.vocab_size * 4, cudaMemcpyDeviceToHost, s->st);
     if (logits_host && sc->order_host) {
         // the rows' order for the host sampler, produced while the logits travel
@@ -933,8 +925,8 @@ dfl_status dfl_packed_verify(const dfl_model* m, dfl_session* s, dfl_scratch* sc
         cudaMemcpyAsync(sc->order_host, sc->order_dev, (size_t)n * V * 4, cudaMemcpyDeviceToHost, s->st);
     }
     DFL_CHECK(completion_check(s));
-    memcpy(argmax_out, sc->pinned_i + MAX_ROWS, n * 4);
-    if (gap_out) memcpy(gap_out, sc->pinned_f, n * 4);
+    memcpy(argmax_out, sc->argmax, n * 4);
+    if (gap_out) memcpy(gap_out, sc->gap, n * 4);
     return DFL_OK;
 }
 
@@ -1179,6 +1171,7 @@ dfl_status dfl_session_restore_snapshot(const dfl_model* m, dfl_session* s, dfl_
         DFL_CHECK(dsession_snapshot_validate(ds, h.drafter_cols, h.drafter_bytes));
     }
     const uint8_t* p = (const uint8_t*)blob + sizeof(h);
+    // one buffer of position-major rows serves every layer of a tiled cache: each upload waits on the stream for the layout kernel before
     void* rows_tmp = nullptr;
     if (s->kv_mode == KV_F16_TILED && per_layer && !(rows_tmp = pool_alloc(per_layer))) return fail(DFL_ERR_OOM, "restore_snapshot: row buffer");
     std::vector<Upload> list;

@@ -173,7 +173,7 @@ struct dfl_session {
     std::vector<int> ssm_cur;
     float* attn_partials = nullptr;
     cudaStream_t st = nullptr;
-    int* err = nullptr;
+    int* err = nullptr;           // error word of the session's kernels, in pinned host memory
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // side stream for the branches of a routed-expert layer that run beside the main projection instead of after it
     cudaStream_t st_side = nullptr;
@@ -188,17 +188,14 @@ struct dfl_scratch {
     float *q_rot = nullptr, *gate = nullptr;
     // per GDN layer, kept for rollback
     std::vector<float*> qkv_raw, q_n, k_n, v, ab;
-    float *logits = nullptr, *gap = nullptr;
-    int32_t* argmax = nullptr;
+    float* logits = nullptr;
+    int32_t* argmax = nullptr;    // argmax and gap of a block's rows: pinned host memory, written by the ranking kernel
+    float* gap = nullptr;
     // routed experts: router logits [16][E + 1], dense route weights [16][E], shared-expert gates [16], chosen ids [16][k]
     float *route_logits = nullptr, *route_w = nullptr, *route_sg = nullptr, *moe_out = nullptr;
     int32_t* route_idx = nullptr;
     int32_t *moe_tile_map = nullptr, *moe_n_tiles = nullptr, *moe_kb_map = nullptr;   // row tiles of the gate|up matrix the block's routing needs
-    void* am_scratch = nullptr;
     float* capture = nullptr;  // [16][k][H]
-    int32_t* tokens_dev = nullptr;
-    int32_t* pinned_i = nullptr;  // [16] tokens in, [16] argmax out
-    float* pinned_f = nullptr;    // [16] gaps
     float* pinned_logits = nullptr;  // [block][vocab], made on first use by the sampled outer loop
     // rows ordered on the device for the host sampler (sortrows.cu): destination on the host (null = off), device
     // order [block][vocab] and the sort's scratch (made on first use), and a pinned destination of the outer loop

@@ -207,6 +207,10 @@ dfl_status launch_moe_tiles(cudaStream_t st, const float* route_w, int n_rows, i
 dfl_status launch_embed_rows(cudaStream_t st, int dtype, const uint8_t* ggml, uint64_t h, const int32_t* tokens, int n_rows,
                              float* x, int ld);
 
+// the same for up to 16 rows whose tokens are in host memory
+dfl_status launch_embed_block(cudaStream_t st, int dtype, const uint8_t* ggml, uint64_t h, const int32_t* tokens_host, int n_rows,
+                              float* x, int ld);
+
 // out[tok][j] = rs[tok] * sum_k xn[tok][k] * w[j][k] for small f32 matrices (GDN alpha/beta, MoE router).
 dfl_status launch_small_matmul(cudaStream_t st, const float* w, const float* xn, int ld_xn, int n_rows, uint64_t k, int n_out,
                                const GemmEpilogue& ep, float* out, int ld_out);
