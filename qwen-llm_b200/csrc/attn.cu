@@ -358,8 +358,134 @@ dfl_status launch_attn_verify(cudaStream_t st, const AttnGeom& g, const float* q
     return DFL_OK;
 }
 
+// ---- every row of a prompt pass, CUDA cores --------------------------------------------------------
+// The widths and cache storages that neither tensor-core kernel takes (head dim 256, f32 cache).  grid (n_kv, row groups), block
+// 256: up to 32 queries of one KV head, four a warp with their running maximum, sum and accumulator in registers; the
+// CTA walks the 64-position chunks up to its last row, so a query leaves one record whatever the context.  The four queries share
+// every key and value word read from shared memory, which is what bounds the kernel (12 reads to 32 multiply-adds, against 3
+// to 2 with a query at a time).  300 rows, 2 KV heads of 8 queries, head dim 256: nineteen 16-row launches of 15 us -> 98 us in one.
+constexpr int ROWS_QUERIES = 32, ROWS_QW = ROWS_QUERIES / 8;
+template <typename KV, int HD>
+__global__ void __launch_bounds__(256) attn_rows_kernel(AttnGeom g, const float* q_rot, const KV* k_cache, const KV* v_cache,
+                                                        uint32_t start, int n_rows, float* partials, int rows_per_cta) {
+    pdl_prologue();
+    extern __shared__ float sm[];
+    constexpr int LD = HD + 1, EPV = 16 / (int)sizeof(KV), VPR = HD / EPV;
+    float* ks = sm;                                      // [64][LD]
+    float* vs = ks + ATTN_CHUNK * LD;                    // [64][LD]
+    float* qs = vs + ATTN_CHUNK * LD;                    // [32 queries][HD]
+    float* ps = qs + ROWS_QUERIES * HD;                  // [32 queries][64]
+    const int kvh = blockIdx.x, group = g.n_q / g.n_kv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * rows_per_cta;   // the rows that see most first
+    const int rows = min(rows_per_cta, n_rows - row0), n_query = rows * group;
+    const float scale = 1.0f / sqrtf((float)HD);
+    for (int i = threadIdx.x; i < n_query * HD; i += 256) {
+        const int qi = i / HD, d = i % HD;
+        qs[i] = q_rot[((uint64_t)(row0 + qi / group) * g.n_q + kvh * group + qi % group) * HD + d] * scale;
+    }
+    float m[ROWS_QW], l[ROWS_QW], acc[ROWS_QW][HD / 32];
+    int last[ROWS_QW];   // last visible position of the warp's query warp + 8 i, -1: none
+#pragma unroll
+    for (int i = 0; i < ROWS_QW; ++i) {
+        const int qi = warp + 8 * i;
+        last[i] = qi < n_query ? (int)start + row0 + qi / group : -1;
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < HD / 32; ++j) acc[i][j] = 0.f;
+    }
+    const int n_pos = (int)start + row0 + rows;
+    for (int p0 = 0; p0 < n_pos; p0 += ATTN_CHUNK) {
+        const int n_here = min(ATTN_CHUNK, n_pos - p0);
+        __syncthreads();
+#pragma unroll 4
+        for (int idx = threadIdx.x; idx < ATTN_CHUNK * VPR; idx += 256) {
+            const int kp = idx / VPR, vv = idx % VPR;
+            uint4 kr = make_uint4(0, 0, 0, 0), vr = make_uint4(0, 0, 0, 0);
+            if (kp < n_here) {
+                const uint64_t o = ((uint64_t)(p0 + kp) * g.n_kv + kvh) * HD + vv * EPV;
+                kr = *reinterpret_cast<const uint4*>(k_cache + o);
+                vr = *reinterpret_cast<const uint4*>(v_cache + o);
+            }
+            const KV* ke = reinterpret_cast<const KV*>(&kr);
+            const KV* ve = reinterpret_cast<const KV*>(&vr);
+#pragma unroll
+            for (int e = 0; e < EPV; ++e) {
+                ks[kp * LD + vv * EPV + e] = (float)ke[e];
+                vs[kp * LD + vv * EPV + e] = (float)ve[e];
+            }
+        }
+        __syncthreads();
+        float s[ROWS_QW][2];
+#pragma unroll
+        for (int i = 0; i < ROWS_QW; ++i) s[i][0] = s[i][1] = 0.f;
+        const float *k0 = ks + lane * LD, *k1 = ks + (lane + 32) * LD;
+#pragma unroll 4
+        for (int d = 0; d < HD; d += 4) {
+            float4 q[ROWS_QW];
+#pragma unroll
+            for (int i = 0; i < ROWS_QW; ++i) q[i] = *reinterpret_cast<const float4*>(qs + (warp + 8 * i) * HD + d);
+            const float a0 = k0[d], a1 = k0[d + 1], a2 = k0[d + 2], a3 = k0[d + 3], b0 = k1[d], b1 = k1[d + 1], b2 = k1[d + 2], b3 = k1[d + 3];
+#pragma unroll
+            for (int i = 0; i < ROWS_QW; ++i) {
+                s[i][0] = fmaf(q[i].w, a3, fmaf(q[i].z, a2, fmaf(q[i].y, a1, fmaf(q[i].x, a0, s[i][0]))));
+                s[i][1] = fmaf(q[i].w, b3, fmaf(q[i].z, b2, fmaf(q[i].y, b1, fmaf(q[i].x, b0, s[i][1]))));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < ROWS_QW; ++i) {
+            const bool ok0 = p0 + lane <= last[i], ok1 = p0 + lane + 32 <= last[i];
+            const float mn = fmaxf(m[i], warp_max(fmaxf(ok0 ? s[i][0] : -INFINITY, ok1 ? s[i][1] : -INFINITY)));
+            const float keep = mn > -INFINITY ? expf(m[i] - mn) : 1.f;
+            const float e0 = ok0 ? expf(s[i][0] - mn) : 0.f, e1 = ok1 ? expf(s[i][1] - mn) : 0.f;
+            l[i] = fmaf(l[i], keep, warp_sum(e0 + e1));
+            m[i] = mn;
+#pragma unroll
+            for (int j = 0; j < HD / 32; ++j) acc[i][j] *= keep;
+            ps[(warp + 8 * i) * ATTN_CHUNK + lane] = e0;
+            ps[(warp + 8 * i) * ATTN_CHUNK + lane + 32] = e1;
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (int kp = 0; kp < ATTN_CHUNK; kp += 4) {   // keys beyond the chunk's last carry weight 0 and value 0
+            float4 w[ROWS_QW];
+#pragma unroll
+            for (int i = 0; i < ROWS_QW; ++i) w[i] = *reinterpret_cast<const float4*>(ps + (warp + 8 * i) * ATTN_CHUNK + kp);
+#pragma unroll
+            for (int j = 0; j < HD / 32; ++j) {
+                const float* v = vs + kp * LD + lane + 32 * j;
+                const float v0 = v[0], v1 = v[LD], v2 = v[2 * LD], v3 = v[3 * LD];
+#pragma unroll
+                for (int i = 0; i < ROWS_QW; ++i) acc[i][j] = fmaf(w[i].w, v3, fmaf(w[i].z, v2, fmaf(w[i].y, v1, fmaf(w[i].x, v0, acc[i][j]))));
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS_QW; ++i) {
+        if (last[i] < 0) continue;
+        const int qi = warp + 8 * i, row = row0 + qi / group;
+        float* rec = partials + (((uint64_t)(row / MAX_ROWS) * g.n_kv + kvh) * (MAX_ROWS * group) + (row % MAX_ROWS) * group + qi % group) * (HD + 2);
+        if (lane == 0) { rec[0] = m[i]; rec[1] = l[i]; }
+#pragma unroll
+        for (int j = 0; j < HD / 32; ++j) rec[2 + lane + 32 * j] = acc[i][j];
+    }
+}
+template <typename KV, int HD>
+static dfl_status launch_rows(cudaStream_t st, const AttnGeom& g, const float* q_rot, const void* k_cache, const void* v_cache, uint32_t start, int n_rows,
+                              float* partials) {
+    const size_t smem = (size_t)(2 * ATTN_CHUNK * (HD + 1) + ROWS_QUERIES * (HD + ATTN_CHUNK)) * sizeof(float);
+    DFL_CUDA(cudaFuncSetAttribute(attn_rows_kernel<KV, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int rows_per_cta = ROWS_QUERIES / (g.n_q / g.n_kv);
+    launch_k(attn_rows_kernel<KV, HD>, dim3((unsigned)g.n_kv, (unsigned)((n_rows + rows_per_cta - 1) / rows_per_cta)), dim3(256), smem, st, g, q_rot,
+             reinterpret_cast<const KV*>(k_cache), reinterpret_cast<const KV*>(v_cache), start, n_rows, partials, rows_per_cta);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
+// more than 32 queries on a KV head: the 16-row path, block by block
 bool attn_rows_supported(const AttnGeom& g, int kv_mode) {
-    return kv_mode == KV_F16_TILED || attn_tc_supported(g, kv_mode != KV_F32_ROWS);
+    return kv_mode == KV_F16_TILED || attn_tc_supported(g, kv_mode != KV_F32_ROWS) || ((g.hd == 128 || g.hd == 256) && g.n_q / g.n_kv <= ROWS_QUERIES);
 }
 uint64_t attn_rows_partials_floats(const AttnGeom& g, int n_rows) {
     return (uint64_t)((n_rows + MAX_ROWS - 1) / MAX_ROWS) * 2 * g.n_q * MAX_ROWS * (g.hd + 2);
@@ -369,11 +495,17 @@ uint64_t attn_rows_partials_floats(const AttnGeom& g, int n_rows) {
 dfl_status launch_attn_rows(cudaStream_t st, const AttnGeom& g, const float* q_rot, const float* gate, const void* k_cache, const void* v_cache,
                             int kv_mode, uint32_t start, int n_rows, float* partials, float* out_f32, int* err) {
     constexpr int ALL = 1 << 24;   // chunks per span: more than any cache holds
-    const bool tiled = kv_mode == KV_F16_TILED;
-    DFL_CHECK(tiled ? launch_attn_t5(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ALL, err)
-                    : launch_attn_span_tc(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ALL));
-    launch_k(attn_post_kernel<128>, dim3((unsigned)g.n_q, (unsigned)n_rows), dim3(32), 0, st, g, partials, 1 << 30, tiled ? 2 : 1, gate, start,
-             nullptr, 0, out_f32, err, 1);
+    const bool tiled = kv_mode == KV_F16_TILED, kv_f16 = kv_mode != KV_F32_ROWS;
+    dfl_status s;
+    if (tiled) s = launch_attn_t5(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ALL, err);
+    else if (attn_tc_supported(g, kv_f16)) s = launch_attn_span_tc(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ALL);
+    else if (g.hd == 128) s = kv_f16 ? launch_rows<__half, 128>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials)
+                                     : launch_rows<float, 128>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials);
+    else s = kv_f16 ? launch_rows<__half, 256>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials)
+                    : launch_rows<float, 256>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials);
+    DFL_CHECK(s);
+    launch_k(g.hd == 128 ? attn_post_kernel<128> : attn_post_kernel<256>, dim3((unsigned)g.n_q, (unsigned)n_rows), dim3(32), 0, st, g, partials, 1 << 30,
+             tiled ? 2 : 1, gate, start, nullptr, 0, out_f32, err, 1);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;
