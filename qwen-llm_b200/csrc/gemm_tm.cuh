@@ -8,30 +8,35 @@
 //     Q6_K: q * sc needs up to 13 bits, A1 = fl16(q * sc) and A2 = q * sc - A1 in {-1, 0, 1}; A1 x {hi, lo} + A2 x hi
 //     (A2 x lo is below 2^-24 of the product's range) = 3072 clocks;
 //   * unpack: 16 warps, about 1000 - 1300 clocks of issue, hidden under the MMAs;
-//   * activations: 128 KiB of hi / lo planes per block and CTA from L2, 60 bytes a clock, the other near-limit.
+//   * activations: 1 KiB of hi / lo planes per token, block and CTA from L2.
+// With 128 tokens a block takes some 2330 clocks in the steady state and an item 2500 - 4000 more to end and to start (4096 ->
+// 24576 Q4_K over 512 rows: 156 us); with few, the latencies of the rings (1600 - 2000 clocks) are what is left.
 // The min term -dmin * m_j * sum(x over sub-block j) rides in the same accumulator: its A operand is -(dmin / s) m_j as
 // an f16 hi + lo pair, s = the factor the accumulator is multiplied with afterwards (d, except where dmin / d would leave
 // the f16 range), its B operand the sub-block sums as f16 hi + lo.
 //
 // Warps: 0..15 unpack (two groups of eight; group g owns A buffer g: Q4_K / Q5_K half g of a block, Q6_K quarters g and
 // g + 2), 16..23 read the accumulator back (thread = weight row and half of the
-// tokens), 24 issues the MMAs, 25 streams weights, 26 activations.
-// Tensor memory: two 128-column block accumulators (one fills while the other is read back), the running sum over blocks
-// (128), two 64-column A buffers: all 512 columns.
+// tokens), 24 and 25 issue the MMAs of even and odd blocks, 26 streams weights, 27 activations.  Two issuers, because one
+// spends 2400 - 3000 clocks on a block's MMAs, waits and commits whatever the tokens, more than the tensor pipe needs (161 us
+// for 4096 -> 24576 Q4_K over 512 rows with one, 41 us over 77).  Each has an accumulator and barriers of its own, so
+// that neither ever waits for a barrier phase whose predecessor it has not seen.
+// Tensor memory, for a capacity of C tokens: two C-column block accumulators (one fills while the other is read back), the running
+// sum over blocks (C columns), the A buffers of 64 columns.  At 128 tokens that leaves one A buffer a group, whose refill (store,
+// wait, two signals: 900 clocks) only the other group's MMAs cover; tiles of up to 80 tokens have two, so that what is
+// left of a block is mostly the unpack.
 #pragma once
 
 namespace dfl {
 namespace ts {
 
-constexpr int TM_WARPS = 27, TM_THREADS = TM_WARPS * 32;
-constexpr int TM_DRAIN_WARPS = 8, TM_MMA_WARP = 24, TM_W_WARP = 25, TM_B_WARP = 26;
-constexpr int TM_B_STAGES = 4;
-constexpr uint32_t TM2_D = 0, TM2_ACC = 256, TM2_A = 384;
+constexpr int TM_WARPS = 28, TM_THREADS = TM_WARPS * 32;
+constexpr int TM_DRAIN_WARPS = 8, TM_MMA_WARP = 24, TM_W_WARP = 26, TM_B_WARP = 27;   // two MMA warps
 constexpr int TM_BAR_BYTES = 512;
 
 struct TmParams {
     const uint8_t* w;
-    const uint8_t* acts;      // [token tile][column block] chunks of TM_CHUNK bytes
+    const uint8_t* acts;      // [token tile][column block] chunks of tm_chunk(tokens) bytes
     float* out;               // [splits][rows_pad][ld_out]
     const float* sumsq;       // [n_sumsq][rows_pad]
     int n_sumsq;
@@ -42,17 +47,28 @@ struct TmParams {
     TmSegments g;             // g.seg != nullptr: segments of gathered rows instead of token tiles
 };
 
+constexpr int TM_SMALL = 80;   // the most tokens that leave tensor memory for two A buffers a group: 3 * 80 + 4 * 64 <= 512 columns
+
 template <int DT, int CAP>
 struct TmFmt {
+    static constexpr int NA = CAP <= TM_SMALL ? 2 : 1;   // A buffers a group
+    static constexpr uint32_t ACC = 2 * CAP, A = 3 * CAP;
+    static_assert(3 * CAP + NA * 128 <= 512, "tensor memory");
+    // Activation stages (64 columns).  A slot is filled again 1400 - 1600 clocks after its MMAs (commit, producer, copy), so a ring of
+    // one block bounds a block at some 2000 clocks however few tokens there are: as many as fit.
+    static constexpr int NB = CAP == TM_TOK ? 4 : CAP == TM_SMALL ? 6 : 8;
+    static constexpr int N_AM = NA == 2 ? 4 : 3;
     static constexpr bool MIN = DT != DFL_Q6_K;
     static constexpr int W_STAGE = Fmt<DT>::STAGE;
     static constexpr int BSTAGE = tm_bstage(CAP), SUMS = tm_sums(CAP);
     // weight stages: what the activation ring leaves room for
-    static constexpr int W_STAGES = CAP == TM_TOK ? (DT == DFL_Q6_K ? 2 : 3) : (DT == DFL_Q6_K ? 4 : 6);
+    static constexpr int W_STAGES = CAP == TM_TOK ? (DT == DFL_Q6_K ? 2 : 3) : CAP == TM_SMALL ? (DT == DFL_Q4_K ? 4 : 3) : (DT == DFL_Q6_K ? 4 : 6);
     static constexpr int USES = MIN ? 1 : 2;      // how often a block uses each A buffer
-    static constexpr int OFF_W = TM_B_STAGES * BSTAGE;
-    static constexpr int OFF_AM = OFF_W + W_STAGES * W_STAGE;          // [2] min-term A operand, 128 x 16
-    static constexpr int OFF_S = OFF_AM + (MIN ? 2 * 4096 : 0);        // [2] min-term B operand
+    static constexpr int OFF_W = NB * BSTAGE;
+    // [N_AM] min-term A operand, 128 x 16.  The first group writes block e's after the first half of block e - NA has completed,
+    // which is behind the issuer's block before it, e - NA - 2, but says nothing of the last MMAs of block e - NA.
+    static constexpr int OFF_AM = OFF_W + W_STAGES * W_STAGE;
+    static constexpr int OFF_S = OFF_AM + (MIN ? N_AM * 4096 : 0);        // [2] min-term B operand
     static constexpr int OFF_SCL = OFF_S + (MIN ? 2 * SUMS : 0);    // [4][128] block scales
     static constexpr int OFF_BAR = OFF_SCL + 4 * TILE_R * 4;
     static constexpr int SMEM = OFF_BAR + TM_BAR_BYTES;
@@ -76,35 +92,36 @@ __device__ __forceinline__ TmScale tm_scale(float d, float dmin) {
 template <int DT, int CAP>
 __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p) {
     using T = TmFmt<DT, CAP>;
-    constexpr bool SEG = CAP != TM_TOK;
-    static_assert(T::SMEM <= 227 * 1024 && (2 * T::W_STAGES + 2 * TM_B_STAGES + 12) * 8 <= TM_BAR_BYTES, "shared memory budget");
+    constexpr bool SEG = CAP == TM_SEG;
+    static_assert(T::SMEM <= 227 * 1024 && (2 * T::W_STAGES + 3 * T::NB + 20) * 8 <= TM_BAR_BYTES, "shared memory budget");
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* b_ring = smem;
     uint8_t* w_ring = smem + T::OFF_W;
     float* scl = reinterpret_cast<float*>(smem + T::OFF_SCL);
     uint64_t* w_full = reinterpret_cast<uint64_t*>(smem + T::OFF_BAR);
     uint64_t* w_empty = w_full + T::W_STAGES;
-    uint64_t* b_full = w_empty + T::W_STAGES;
-    uint64_t* b_empty = b_full + TM_B_STAGES;
-    uint64_t* s_full = b_empty + TM_B_STAGES;   // [2] sub-block sums of a block
+    uint64_t* b_full = w_empty + T::W_STAGES;   // [block & 1][stage]
+    uint64_t* b_empty = b_full + 2 * T::NB;
+    uint64_t* s_full = b_empty + T::NB;   // [2] sub-block sums of a block
     uint64_t* s_empty = s_full + 2;
-    uint64_t* a_ready = s_empty + 2;            // [buffer] unpacked weights are in tensor memory
-    uint64_t* a_free = a_ready + 2;
-    uint64_t* d_ready = a_free + 2;             // [accumulator] every MMA of a block has completed
+    uint64_t* a_ready = s_empty + 2;            // [block & 1][use in the block][group] unpacked weights are in tensor memory
+    uint64_t* a_free = a_ready + 8;             // [A buffer of the group][group]
+    uint64_t* d_ready = a_free + 4;             // [accumulator] every MMA of a block has completed
     uint64_t* d_free = d_ready + 2;
     __shared__ uint32_t tmem_slot;
-    __shared__ float tok_scale[TM_TOK];
+    __shared__ __align__(16) float tok_scale[TM_TOK];
     __shared__ int abort_flag;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < T::W_STAGES; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], UNPACK_WARPS); }
-        for (int i = 0; i < TM_B_STAGES; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < T::NB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_full[T::NB + i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < 8; ++i) mbar_init(&a_ready[i], GROUP_WARPS);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&s_full[i], 1);
             mbar_init(&s_empty[i], 1);
-            mbar_init(&a_ready[i], GROUP_WARPS);
             mbar_init(&a_free[i], 1);
+            mbar_init(&a_free[2 + i], 1);
             mbar_init(&d_ready[i], 1);
             mbar_init(&d_free[i], TM_DRAIN_WARPS);
         }
@@ -148,6 +165,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         it.rows = p.tile_tok;
         return it;
     };
+    auto tok_of = [&](const Item& it) { return SEG ? tm_seg_tok(it.rows) : p.tile_tok; };   // tokens its activation chunks hold
     bool ok = true;
 
     if (warp == TM_W_WARP) {
@@ -159,7 +177,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 const Item it = item_of(idx);
                 const uint8_t* src = p.w + ((uint64_t)it.rt * p.kblocks + it.kb0) * T::W_STAGE;
                 for (int k = 0; k < it.n_kb; ++k, src += T::W_STAGE) {
-                    if (round > 0 && !(ok = mbar_wait_bounded(&w_empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY))) break;
+                    if (round > 0 && !(ok = mbar_wait_one(&w_empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY))) break;
                     mbar_arrive_expect_tx(&w_full[s], T::W_STAGE);
                     bulk_g2s(w_ring + s * T::W_STAGE, src, T::W_STAGE, &w_full[s]);
                     if (++s == T::W_STAGES) { s = 0; ++round; }
@@ -174,62 +192,67 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
             uint32_t round = 0, e = 0;
             for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
                 const Item it = item_of(idx);
-                const uint8_t* src = p.acts + (SEG ? (uint64_t)it.tt * it.n_kb : (uint64_t)it.tt * p.kblocks + it.kb0) * tm_chunk(CAP);
-                for (int k = 0; k < it.n_kb && ok; ++k, src += tm_chunk(CAP), ++e) {
+                const int tok = tok_of(it), spacing = tm_chunk(SEG ? CAP : tok), stage = tm_bstage(tok), sums = tm_sums(tok);
+                const uint8_t* src = p.acts + (SEG ? (uint64_t)it.tt * it.n_kb : (uint64_t)it.tt * p.kblocks + it.kb0) * spacing;
+                for (int k = 0; k < it.n_kb && ok; ++k, src += spacing, ++e) {
                     if (T::MIN) {
-                        if (e >= 2) ok = mbar_wait_bounded(&s_empty[e & 1], ((e >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
+                        if (e >= 2) ok = mbar_wait_one(&s_empty[e & 1], ((e >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
                         if (!ok) break;
-                        mbar_arrive_expect_tx(&s_full[e & 1], T::SUMS);
-                        bulk_g2s(smem + T::OFF_S + (e & 1) * T::SUMS, src + 4 * T::BSTAGE, T::SUMS, &s_full[e & 1]);
+                        mbar_arrive_expect_tx(&s_full[e & 1], sums);
+                        bulk_g2s(smem + T::OFF_S + (e & 1) * T::SUMS, src + 4 * stage, sums, &s_full[e & 1]);
                     }
                     for (int q = 0; q < 4; ++q) {
-                        if (round > 0 && !(ok = mbar_wait_bounded(&b_empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY))) break;
-                        mbar_arrive_expect_tx(&b_full[s], T::BSTAGE);
-                        bulk_g2s(b_ring + s * T::BSTAGE, src + q * T::BSTAGE, T::BSTAGE, &b_full[s]);
-                        if (++s == TM_B_STAGES) { s = 0; ++round; }
+                        if (round > 0 && !(ok = mbar_wait_one(&b_empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY))) break;
+                        uint64_t* fb = &b_full[(e & 1) * T::NB + s];
+                        mbar_arrive_expect_tx(fb, stage);
+                        bulk_g2s(b_ring + s * T::BSTAGE, src + q * stage, stage, fb);
+                        if (++s == T::NB) { s = 0; ++round; }
                     }
                 }
             }
         }
-    } else if (warp == TM_MMA_WARP) {
+    } else if (warp == TM_MMA_WARP || warp == TM_MMA_WARP + 1) {
         // ------------------------------ MMA issue ------------------------------
-        // All tensor-memory addresses are literals (the CTA owns all 512 columns, so the allocation starts at 0) and a
-        // block's four activation stages are the ring's four slots, so that the issuing warp spends its slots on MMAs.
-        uint32_t IDESC = instr_desc(p.tile_tok);
-        static_assert(TM_B_STAGES == 4, "stage q of every block is ring slot q");
+        // All tensor-memory addresses are literals (the CTA owns all 512 columns, so the allocation starts at 0), so that the
+        // issuing thread spends its slots on MMAs.
+        uint32_t IDESC = instr_desc(p.tile_tok), tok = p.tile_tok;
         const uint32_t b_addr = smem_u32(b_ring), am_addr = smem_u32(smem + T::OFF_AM), s_addr = smem_u32(smem + T::OFF_S);
-        uint32_t e = 0;
+        uint32_t e = 0, am = 0, sl = 0;   // am = e % N_AM, sl = 4 e % NB
+        uint32_t b_phase = 0;             // bit s: parity of this issuer's next use of slot s
         auto wait = [&](uint64_t* bar, uint32_t parity) {
             ok = mbar_wait_one(bar, parity, p.err, DEV_ERR_WAIT_FULL);
             return ok;
         };
         auto block = [&](auto odd) {   // one 256-column block into accumulator e & 1
-            constexpr uint32_t O = decltype(odd)::value, D = TM2_D + O * 128;
+            constexpr uint32_t O = decltype(odd)::value, D = O * CAP;
             if (e >= 2 && !wait(&d_free[O], ((e >> 1) - 1) & 1)) return;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {   // 64 columns = one activation stage
                 const int g = T::MIN ? q >> 1 : q & 1;
-                if ((!T::MIN || (q & 1) == 0) && !wait(&a_ready[g], (T::MIN ? e : 2 * e + (q >> 1)) & 1)) return;
-                if (!wait(&b_full[q], e & 1)) return;
+                const int ab = T::NA == 1 ? 0 : T::MIN ? (int)O : q >> 1;   // use number modulo the group's buffers
+                if ((!T::MIN || (q & 1) == 0) && !wait(&a_ready[4 * O + (T::MIN ? 0 : q & 2) + g], (e >> 1) & 1)) return;
+                const uint32_t slot = T::NB == 4 ? q : T::NB == 8 ? 4 * O + q : (sl + q >= (uint32_t)T::NB ? sl + q - T::NB : sl + q);
+                if (!wait(&b_full[O * T::NB + slot], (b_phase >> slot) & 1)) return;
+                b_phase ^= 1u << slot;
                 if (T::MIN && q == 3 && !wait(&s_full[O], (e >> 1) & 1)) return;
                 fence_after_sync();
                 {
-                    const uint64_t bd = smem_desc(b_addr + q * T::BSTAGE, CAP * 16, 128);
+                    const uint64_t bd = smem_desc(b_addr + slot * T::BSTAGE, tok * 16, 128);   // address field: 16-byte units
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const uint32_t aj = TM2_A + 64 * g + (T::MIN ? 32 * (q & 1) : 0) + 8 * j;
-                        mma_ts_rt(D, aj, bd + j * (2 * CAP), IDESC, (q | j) != 0);
-                        mma_ts_rt(D, aj, bd + j * (2 * CAP) + T::BSTAGE / 32, IDESC, 1u);
-                        if (!T::MIN) mma_ts_rt(D, aj + 32, bd + j * (2 * CAP), IDESC, 1u);
+                        const uint32_t aj = T::A + 128 * ab + 64 * g + (T::MIN ? 32 * (q & 1) : 0) + 8 * j;
+                        mma_ts_rt(D, aj, bd + j * (2 * tok), IDESC, (q | j) != 0);
+                        mma_ts_rt(D, aj, bd + j * (2 * tok) + 8 * tok, IDESC, 1u);
+                        if (!T::MIN) mma_ts_rt(D, aj + 32, bd + j * (2 * tok), IDESC, 1u);
                     }
-                    mma_commit(&b_empty[q]);
+                    mma_commit(&b_empty[slot]);
                     if (T::MIN && q == 3) {
-                        const uint64_t ad = smem_desc(am_addr + O * 4096, 2048, 128), sd = smem_desc(s_addr + O * T::SUMS, CAP * 16, 128);
+                        const uint64_t ad = smem_desc(am_addr + am * 4096, 2048, 128), sd = smem_desc(s_addr + O * T::SUMS, tok * 16, 128);
                         mma_ss(D, ad, sd, IDESC, 1u);
-                        mma_ss(D, ad, sd + T::SUMS / 32, IDESC, 1u);
+                        mma_ss(D, ad, sd + 2 * tok, IDESC, 1u);
                         mma_commit(&s_empty[O]);
                     }
-                    if (!T::MIN || (q & 1)) mma_commit(&a_free[g]);
+                    if (!T::MIN || (q & 1)) mma_commit(&a_free[2 * ab + g]);
                     if (q == 3) mma_commit(&d_ready[O]);
                 }
             }
@@ -242,8 +265,12 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
             for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
                 const Item it = item_of(idx);
                 const int n_kb = it.n_kb;
-                if (SEG) IDESC = instr_desc((it.rows + 15) & ~15);
-                for (int k = 0; k < n_kb && ok; ++k, ++e) {
+                if (SEG) {
+                    tok = tok_of(it);
+                    IDESC = instr_desc(tok);
+                }
+                for (int k = 0; k < n_kb && ok; ++k, ++e, am = am == T::N_AM - 1 ? 0 : am + 1, sl = (sl + 4) % T::NB) {
+                    if ((e & 1) != (uint32_t)(warp - TM_MMA_WARP)) continue;
                     if (e & 1) block(std::integral_constant<uint32_t, 1>{});
                     else block(std::integral_constant<uint32_t, 0>{});
                 }
@@ -254,13 +281,13 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         // ------------------------------ unpack ------------------------------
         const int g = warp >> 3, q4 = warp & 3, kp2 = (warp >> 2) & 1;
         const int row = 32 * q4 + lane;
-        const uint32_t a_buf = tmem + ((uint32_t)(32 * q4) << 16) + TM2_A + 64 * g;
-        uint32_t e = 0, use = 0;
+        const uint32_t a_buf = tmem + ((uint32_t)(32 * q4) << 16) + T::A + 64 * g;
+        uint32_t e = 0, use = 0, am_buf = 0;   // am_buf = e % N_AM
         int s = 0;
         uint32_t round = 0;
         for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
             const int n_kb = item_of(idx).n_kb;
-            for (int k = 0; k < n_kb && ok; ++k, ++e) {
+            for (int k = 0; k < n_kb && ok; ++k, ++e, am_buf = am_buf == T::N_AM - 1 ? 0 : am_buf + 1) {
                 ok = mbar_wait_warp(&w_full[s], round & 1, p.err, DEV_ERR_WAIT_FULL);
                 if (!ok) break;
                 const uint8_t* st = w_ring + s * T::W_STAGE;
@@ -286,20 +313,21 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&w_empty[s]);   // every lane has its bytes in registers
                     }
-                    if (use >= 1) {
-                        ok = mbar_wait_warp(&a_free[g], (use - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
+                    const uint32_t ab = T::NA == 1 ? 0 : use & 1, a_dst = a_buf + 128 * ab;
+                    if (use >= T::NA) {
+                        ok = mbar_wait_warp(&a_free[2 * ab + g], (T::NA == 1 ? use - 1 : (use >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
                         if (!ok) break;
                         fence_after_sync();
                     }
                     if (T::MIN) {
-                        tmem_st32(a_buf + 32 * kp2, r);
+                        tmem_st32(a_dst + 32 * kp2, r);
                         // the min operand of this thread's two sub-blocks, k = 2 kp and 2 kp + 1 (hi) and 8 further (lo)
                         const float2 m = __half22float2(*reinterpret_cast<const __half2*>(&am[0]));
                         const float f0 = -sc.ratio * m.x, f1 = -sc.ratio * m.y;
                         const __half2 hi = __floats2half2_rn(f0, f1);
                         const float2 back = __half22float2(hi);
                         const __half2 lo = __floats2half2_rn(f0 - back.x, f1 - back.y);
-                        uint8_t* dst = smem + T::OFF_AM + (e & 1) * 4096 + (row >> 3) * 128 + (row & 7) * 16 + (2 * g + kp2) * 4;
+                        uint8_t* dst = smem + T::OFF_AM + am_buf * 4096 + (row >> 3) * 128 + (row & 7) * 16 + (2 * g + kp2) * 4;
                         *reinterpret_cast<__half2*>(dst) = hi;
                         *reinterpret_cast<__half2*>(dst + 2048) = lo;
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -307,14 +335,14 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                         uint32_t a1[16], a2[16];
 #pragma unroll
                         for (int i = 0; i < 16; ++i) { a1[i] = r[i]; a2[i] = r[16 + i]; }
-                        tmem_st16(a_buf + 16 * kp2, a1);
-                        tmem_st16(a_buf + 32 + 16 * kp2, a2);
+                        tmem_st16(a_dst + 16 * kp2, a1);
+                        tmem_st16(a_dst + 32 + 16 * kp2, a2);
                     }
                     if (g == 0 && u == 0 && kp2 == 0) scl[(e & 3) * TILE_R + row] = sc.s;
                     wait_st();
                     fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&a_ready[g]);
+                    if (lane == 0) mbar_arrive(&a_ready[4 * (e & 1) + 2 * u + g]);
                 }
                 if (++s == T::W_STAGES) { s = 0; ++round; }
             }
@@ -352,7 +380,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 if (!ok) break;
                 fence_after_sync();
                 const float s = scl[(e & 3) * TILE_R + row];
-                const uint32_t d = tm_l + TM2_D + (e & 1) * 128;
+                const uint32_t d = tm_l + (e & 1) * CAP;
                 const bool last = k == it.n_kb - 1;
                 const uint32_t orow = (uint32_t)(SEG ? it.sp : it.rt) * TILE_R + row;
                 auto release = [&] {
@@ -365,26 +393,39 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 for (int c = c0; c < c1; ++c) {   // 16 tokens
                     float v[16], a[16];
                     tmem_ld16(d + 16 * c, v);
-                    if (k > 0) tmem_ld16(tm_l + TM2_ACC + 16 * c, a);
+                    if (k > 0) tmem_ld16(tm_l + T::ACC + 16 * c, a);
                     wait_ld();
                     if (c == c1 - 1) release();
+                    uint32_t u[16];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = k > 0 ? fmaf(s, v[j], a[j]) : s * v[j];
-                    if (!last) {
-                        uint32_t u[16];
+                    for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(k > 0 ? fmaf(s, v[j], a[j]) : s * v[j]);
+                    tmem_st16(tm_l + T::ACC + 16 * c, u);
+                }
+                wait_st();
+                if (!last) continue;
+                // the item's sums: in a loop of its own, so that the accumulators are back with the MMAs while the stores (6000 - 8000
+                // clocks when every CTA ends an item) drain
+#pragma unroll 1
+                for (int c = c0; c < c1; ++c) {
+                    // every scale before the first store: a load of shared memory behind a store to global memory waits for its turn in the
+                    // same queue, 70 - 110 clocks a token
+                    float v[16];
+                    tmem_ld16(tm_l + T::ACC + 16 * c, v);
+                    wait_ld();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(v[j]);
-                        tmem_st16(tm_l + TM2_ACC + 16 * c, u);
-                    } else if (orow < p.n_out) {
+                    for (int j = 0; j < 16; j += 4) {
+                        const float4 t = *reinterpret_cast<const float4*>(tok_scale + 16 * c + j);
+                        v[j] *= t.x; v[j + 1] *= t.y; v[j + 2] *= t.z; v[j + 3] *= t.w;
+                    }
+                    if (orow < p.n_out) {
                         const int tok0 = (SEG ? it.tt * CAP : it.sp * p.rows_pad + it.tt * p.tile_tok) + 16 * c;
                         float* dst = p.out + (uint64_t)tok0 * p.ld_out + orow;
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
-                            if (16 * c + j < live) dst[(uint64_t)j * p.ld_out] = v[j] * tok_scale[16 * c + j];
+                            if (16 * c + j < live) dst[(uint64_t)j * p.ld_out] = v[j];
                     }
                     __syncwarp();
                 }
-                if (!last) wait_st();
             }
         }
     }
@@ -398,7 +439,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
             while (!mbar_try_wait(b, 0) && !mbar_try_wait(b, 1) && ++spins < (1u << 16)) __nanosleep(100);
         };
         for (int i = 0; i < T::W_STAGES; ++i) settle(&w_full[i]);
-        for (int i = 0; i < TM_B_STAGES; ++i) settle(&b_full[i]);
+        for (int i = 0; i < 2 * T::NB; ++i) settle(&b_full[i]);
         for (int i = 0; i < 2; ++i) settle(&s_full[i]);
     }
     __syncthreads();
@@ -462,6 +503,10 @@ dfl_status launch_gemm_tm(cudaStream_t st, const QMatrix& m, const uint8_t* acts
     p.kblocks = m.kblocks; p.splits = splits; p.row_tiles = m.row_tiles; p.tile_tok = tile_tok; p.tok_tiles = (n_rows + tile_tok - 1) / tile_tok;
     p.n_rows = n_rows; p.rows_pad = p.tok_tiles * tile_tok; p.n_out = (uint32_t)m.n_out; p.ld_out = ld_out ? ld_out : (uint32_t)m.n_out; p.err = dev_err;
     const int n_items = p.row_tiles * p.splits * p.tok_tiles;
+    // Up to 80 tokens the deeper rings pay for Q4_K and Q5_K (4096 -> 24576 over 77 rows: 41.4 -> 38.7 us, 32 rows 36.4 -> 32.6);
+    // Q6_K, whose two passes per block keep the tensor pipe busier, was the same or slower (44.3 -> 45.8).
+    if (tile_tok <= ts::TM_SMALL && m.dtype == DFL_Q4_K) return ts::launch_tm<DFL_Q4_K, ts::TM_SMALL>(st, p, n_items);
+    if (tile_tok <= ts::TM_SMALL && m.dtype == DFL_Q5_K) return ts::launch_tm<DFL_Q5_K, ts::TM_SMALL>(st, p, n_items);
     switch (m.dtype) {
         case DFL_Q4_K: return ts::launch_tm<DFL_Q4_K, TM_TOK>(st, p, n_items);
         case DFL_Q5_K: return ts::launch_tm<DFL_Q5_K, TM_TOK>(st, p, n_items);

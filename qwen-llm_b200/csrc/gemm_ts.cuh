@@ -34,17 +34,17 @@ constexpr int TS_BMIN_OFF = TS_B_BYTES;
 constexpr int TS_BMIN_BYTES = 1536;  // [k-core 2][n-group 6][8][16 B]
 static_assert(ACTTS_CHUNK == TS_B_BYTES + TS_BMIN_BYTES, "activation chunk size");
 
-// Many-row kernel (gemm_tm.cuh), activation chunk per (128 tokens, 256 columns): four stages of 64 columns, each
-// [plane hi / lo][k-core 8][token 128][8 halfs] (K-major operand, k-cores 2048 bytes apart), columns in the order of
-// ts_act_kpos; then the 32-column sub-block sums as [plane hi / lo][k-core 2][token 128][8 halfs], both k-cores alike
+// Many-row kernel (gemm_tm.cuh), activation chunk per (tile of T tokens, 256 columns): four stages of 64 columns, each
+// [plane hi / lo][k-core 8][token T][8 halfs] (K-major operand, k-cores 16 T bytes apart), columns in the order of
+// ts_act_kpos; then the 32-column sub-block sums as [plane hi / lo][k-core 2][token T][8 halfs], both k-cores alike
 // (the A operand holds the hi part of the mins in its first eight columns and the lo part in the other eight).
-constexpr int TM_TOK = 128;
-// the same with room for `cap` tokens (the routed experts' segments hold 32)
-constexpr int TM_SEG = 32;
-__host__ __device__ constexpr int tm_bstage(int cap) { return 2 * 64 * cap * 2; }
-__host__ __device__ constexpr int tm_sums(int cap) { return 2 * 16 * cap * 2; }
-__host__ __device__ constexpr int tm_chunk(int cap) { return 4 * tm_bstage(cap) + tm_sums(cap); }
-constexpr int TM_CHUNK = tm_chunk(TM_TOK);
+// T is the pass's tile size, or a segment's rows rounded up to 16: what is fetched follows the tokens there are.
+constexpr int TM_TOK = 128;   // the most tokens a tile holds
+constexpr int TM_SEG = 32;    // the most rows a segment of the routed experts holds; its chunks are spaced for that many
+__host__ __device__ constexpr int tm_bstage(int tok) { return 2 * 64 * tok * 2; }
+__host__ __device__ constexpr int tm_sums(int tok) { return 2 * 16 * tok * 2; }
+__host__ __device__ constexpr int tm_chunk(int tok) { return 4 * tm_bstage(tok) + tm_sums(tok); }
+__host__ __device__ constexpr int tm_seg_tok(int rows) { return (rows + 15) & ~15; }
 
 constexpr int TSQ4_OFF_SC = 512;
 constexpr int TSQ4_OFF_QS = 2560;

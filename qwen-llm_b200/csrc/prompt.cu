@@ -102,9 +102,9 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
         alloc(&w->ab, R * 2 * gg.n_v * 4);
         alloc(&w->conv_pre, 3ull * gg.conv_dim() * 4);
         alloc(&w->capture, R * sc->k_layers * H * 4);
-        alloc(&w->acts_h, tiles * (H / TILE_K) * TM_CHUNK);
-        alloc(&w->acts_f, tiles * (F / TILE_K) * TM_CHUNK);
-        alloc(&w->acts_v, tiles * (wide / TILE_K) * TM_CHUNK);
+        alloc(&w->acts_h, tiles * (H / TILE_K) * tm_chunk(TM_TOK));
+        alloc(&w->acts_f, tiles * (F / TILE_K) * tm_chunk(TM_TOK));
+        alloc(&w->acts_v, tiles * (wide / TILE_K) * tm_chunk(TM_TOK));
         alloc(&w->tokens, R * 4);
         if (a.expert_count > 0) {
             const uint64_t E = a.expert_count, used = a.expert_used_count, Fe = a.expert_feed_forward_length;

@@ -7,10 +7,9 @@
 namespace dfl {
 
 #ifdef __CUDACC__
-// Eight consecutive columns k8 .. k8 + 7 (k8 % 8 == 0, inside one 256-column block) of token t of a tile of CAP tokens -> the
+// Eight consecutive columns k8 .. k8 + 7 (k8 % 8 == 0, inside one 256-column block) of token t of a tile of `tok` tokens -> the
 // hi / lo planes of the activation chunk: one 16-byte store each, eight tokens fill 128 contiguous bytes.
-template <int CAP>
-__device__ __forceinline__ void tm_pack_oct(uint8_t* chunk, int t, int k8, const float (&v)[8], bool& overflow) {
+__device__ __forceinline__ void tm_pack_oct(uint8_t* chunk, int tok, int t, int k8, const float (&v)[8], bool& overflow) {
     uint16_t hi[8], lo[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -21,21 +20,20 @@ __device__ __forceinline__ void tm_pack_oct(uint8_t* chunk, int t, int k8, const
     }
     // k-positions of a quad: 0, 2, 1, 3 (ts_act_kpos)
     auto quad = [](const uint16_t* h) { return make_uint2((uint32_t)h[0] | ((uint32_t)h[2] << 16), (uint32_t)h[1] | ((uint32_t)h[3] << 16)); };
-    uint8_t* dst = chunk + (k8 >> 6) * tm_bstage(CAP) + ((k8 >> 3) & 7) * (CAP * 16) + t * 16;
+    uint8_t* dst = chunk + (k8 >> 6) * tm_bstage(tok) + ((k8 >> 3) & 7) * (tok * 16) + t * 16;
     const uint2 h0 = quad(hi), h1 = quad(hi + 4), l0 = quad(lo), l1 = quad(lo + 4);
     *reinterpret_cast<uint4*>(dst) = make_uint4(h0.x, h0.y, h1.x, h1.y);
-    *reinterpret_cast<uint4*>(dst + tm_bstage(CAP) / 2) = make_uint4(l0.x, l0.y, l1.x, l1.y);
+    *reinterpret_cast<uint4*>(dst + tm_bstage(tok) / 2) = make_uint4(l0.x, l0.y, l1.x, l1.y);
 }
 // Sum of token t's activations over 32-column sub-block j -> hi / lo planes, both k-cores.
-template <int CAP>
-__device__ __forceinline__ void tm_pack_sum(uint8_t* chunk, int t, int j, float sum, bool& overflow) {
+__device__ __forceinline__ void tm_pack_sum(uint8_t* chunk, int tok, int t, int j, float sum, bool& overflow) {
     overflow |= (fabsf(sum) >= 65504.f) && (fabsf(sum) < INFINITY);
     const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
-    uint8_t* dst = chunk + 4 * tm_bstage(CAP) + t * 16 + j * 2;
+    uint8_t* dst = chunk + 4 * tm_bstage(tok) + t * 16 + j * 2;
     *reinterpret_cast<__half*>(dst) = h;
-    *reinterpret_cast<__half*>(dst + CAP * 16) = h;
-    *reinterpret_cast<__half*>(dst + tm_sums(CAP) / 2) = l;
-    *reinterpret_cast<__half*>(dst + tm_sums(CAP) / 2 + CAP * 16) = l;
+    *reinterpret_cast<__half*>(dst + tok * 16) = h;
+    *reinterpret_cast<__half*>(dst + tm_sums(tok) / 2) = l;
+    *reinterpret_cast<__half*>(dst + tm_sums(tok) / 2 + tok * 16) = l;
 }
 #endif
 

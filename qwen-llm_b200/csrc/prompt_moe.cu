@@ -96,11 +96,11 @@ __global__ void __launch_bounds__(256) tm_moe_pack_kernel(const TmMoe p) {
     }
     uint8_t* chunk = (MODE == 0 ? p.acts_in : p.acts_mid) + ((uint64_t)si * gridDim.x + blockIdx.x) * tm_chunk(TM_SEG);
     bool over = false;
-    tm_pack_oct<TM_SEG>(chunk, t, k8, v, over);
+    tm_pack_oct(chunk, tm_seg_tok(seg.y), t, k8, v, over);
     float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
     sum += __shfl_xor_sync(0xffffffffu, sum, 8);
     sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-    if (lane < 8) tm_pack_sum<TM_SEG>(chunk, t, warp, sum, over);
+    if (lane < 8) tm_pack_sum(chunk, tm_seg_tok(seg.y), t, warp, sum, over);
     if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
 }
 

@@ -84,13 +84,13 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
     for (int e = 0; e < 8; ++e) v[e] *= p.pre_scale;
     if (p.xn && live) store8(p.xn + (uint64_t)row * p.ld_xn + col, v);
     if (p.acts) {
-        uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * TM_CHUNK;
+        uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * tm_chunk(p.tile_tok);
         bool over = false;
-        tm_pack_oct<TM_TOK>(chunk, row % p.tile_tok, k8, v, over);
+        tm_pack_oct(chunk, p.tile_tok, row % p.tile_tok, k8, v, over);
         float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
         sum += __shfl_xor_sync(0xffffffffu, sum, 8);
         sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-        if (lane < 8) tm_pack_sum<TM_TOK>(chunk, row % p.tile_tok, warp, sum, over);
+        if (lane < 8) tm_pack_sum(chunk, p.tile_tok, row % p.tile_tok, warp, sum, over);
         if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
     }
 }
@@ -570,13 +570,13 @@ __global__ void __launch_bounds__(256) tm_gdn_pack_kernel(const TmGdn p) {
     add8(nw, p.norm_w + (k8 & 127));
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = live ? v[e] * sc * nw[e] * silu_f(z[e]) : 0.f;
-    uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * TM_CHUNK;
+    uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * tm_chunk(p.tile_tok);
     bool over = false;
-    tm_pack_oct<TM_TOK>(chunk, row % p.tile_tok, k8, v, over);
+    tm_pack_oct(chunk, p.tile_tok, row % p.tile_tok, k8, v, over);
     float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
     sum += __shfl_xor_sync(0xffffffffu, sum, 8);
     sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-    if (lane < 8) tm_pack_sum<TM_TOK>(chunk, row % p.tile_tok, warp, sum, over);
+    if (lane < 8) tm_pack_sum(chunk, p.tile_tok, row % p.tile_tok, warp, sum, over);
     if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
 }
 

@@ -100,3 +100,16 @@ def test_prompt_pass_at_routed_widths():
     syn.free_entries(ents)
     _check(arch, gm, 150, 0, [0, 3])
     gm.close()
+
+
+@pytest.mark.parametrize("n", [18, 32, 33, 80, 81, 97, 160, 161])
+def test_prompt_pass_at_tile_edges(n):
+    # around the token counts at which a tile's capacity, its ring and its buffers change; several blocks and items a CTA
+    arch = syn.arch_9b()
+    arch.n_layer = 4
+    arch.vocab_size = 8192
+    ents = syn.target_entries(arch, seed=57, device=0)
+    gm = syn.build_model(arch, ents)
+    syn.free_entries(ents)
+    _check(arch, gm, n, 0, [0, 3])
+    gm.close()
