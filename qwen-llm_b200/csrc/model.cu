@@ -13,7 +13,6 @@ dfl_status launch_group(cudaStream_t st, const MatGroup& g, const uint8_t* acts,
     return DFL_OK;
 }
 
-// A group of one K-quant matrix on the tensor-memory kernel can run the glue step that follows it inside the GEMM.
 static uint64_t tensor_elems(const dfl_tensor* t) {
     uint64_t n = 1;
     for (int i = 0; i < t->n_dims; ++i) n *= t->shape[i];
@@ -693,15 +692,19 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
         s->k_cache.push_back(k);
         s->v_cache.push_back(v);
     }
-    for (int i = 0; i < m->n_gdn && ok; ++i) {
-        float *c = nullptr, *c1 = nullptr, *s0 = nullptr, *s1 = nullptr;
-        ok = (c = (float*)pool_alloc(conv_bytes)) && (c1 = (float*)pool_alloc(conv_bytes)) && (s0 = (float*)pool_alloc(ssm_bytes)) && (s1 = (float*)pool_alloc(ssm_bytes));
-        if (ok) { cudaMemsetAsync(c, 0, conv_bytes, s->st); cudaMemsetAsync(s0, 0, ssm_bytes, s->st); cudaMemsetAsync(s1, 0, ssm_bytes, s->st); }
-        s->conv[0].push_back(c);
-        s->conv[1].push_back(c1);
-        s->ssm[0].push_back(s0);
-        s->ssm[1].push_back(s1);
-        s->ssm_cur.push_back(0);
+    // every layer's recurrent buffers in one block, those of the start first: one memset, where three a layer cost a request 0.2 ms.
+    // A pass writes the other halves before anything reads them.
+    if (ok && m->n_gdn) {
+        const size_t half = (ssm_bytes + conv_bytes) * m->n_gdn;
+        ok = (s->gdn_block = (uint8_t*)pool_alloc(2 * half)) != nullptr;
+        if (ok) cudaMemsetAsync(s->gdn_block, 0, half, s->st);
+        for (int i = 0; i < m->n_gdn && ok; ++i) {
+            for (int b = 0; b < 2; ++b) {
+                s->ssm[b].push_back((float*)(s->gdn_block + b * half + i * ssm_bytes));
+                s->conv[b].push_back((float*)(s->gdn_block + b * half + m->n_gdn * ssm_bytes + i * conv_bytes));
+            }
+            s->ssm_cur.push_back(0);
+        }
     }
     if (ok && m->n_attn) ok = (s->attn_partials = (float*)pool_alloc(attn_partials_floats(m->attn_geom(), (uint32_t)cap_alloc) * 4)) != nullptr;   // two records per 128-position tile in tiled storage
     ok = ok && (s->err = (int*)pool_alloc_host(4));
@@ -728,10 +731,7 @@ void dfl_session_destroy(dfl_session* s) {
         if (st) cudaStreamSynchronize(st);
     for (void* p : s->k_cache) pool_free(p);
     for (void* p : s->v_cache) pool_free(p);
-    for (float* p : s->conv[0]) pool_free(p);
-    for (float* p : s->conv[1]) pool_free(p);
-    for (float* p : s->ssm[0]) pool_free(p);
-    for (float* p : s->ssm[1]) pool_free(p);
+    pool_free(s->gdn_block);
     pool_free(s->attn_partials);
     pool_free(s->err);
     if (s->ev0) cudaEventDestroy(s->ev0);

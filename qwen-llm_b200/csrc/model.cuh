@@ -168,6 +168,7 @@ struct dfl_session {
     bool poisoned = false;
     bool fail_next = false;
     std::vector<void*> k_cache, v_cache;  // per attention layer: [capacity][n_kv][hd] rows, or tiles of 128 positions per KV head (kv_mode)
+    uint8_t* gdn_block = nullptr;   // backs conv and ssm
     std::vector<float*> conv[2];          // per GDN layer, double buffered like the recurrent state: [3][conv_dim]
     std::vector<float*> ssm[2];           // per GDN layer, double buffered: [n_v][128][128]
     std::vector<int> ssm_cur;
