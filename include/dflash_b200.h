@@ -397,7 +397,7 @@ dfl_status dfl_single_token(const dfl_model* m, dfl_session* s, dfl_scratch* sc,
                             const uint32_t* layer_ids, uint32_t n_layer_ids, int32_t token,
                             uint32_t position, float* logits_host, float* hidden_host);
 /* prefill_tokens_with_multi_hidden  metal_dflash.rs:10779-10787: feeds ids in
- * blocks of <=16 through the verify path; hidden_host (optional) [n][k][H] with
+ * passes of up to 512 rows (16 rows and fewer through the verify path); hidden_host (optional) [n][k][H] with
  * k = the scratch's capture slots (slots beyond n_layer_ids are not written);
  * last_logits_host (optional) [vocab].  With feed_drafter every captured row is
  * appended to that drafter session, so n_layer_ids must equal the scratch's
