@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(128) dattn_span_tc_kernel(AttnGeom g, const fl
                                                             const uint32_t* pos_ctx, int ctx_begin, int n_ctx, const float* k_noise,
                                                             const float* v_noise, uint32_t noise_start, int n_rows, int causal,
                                                             uint32_t window, float* partials, int chunks_per_span) {
-    pdl_prologue();
+    pdl_launch_dependents();
     extern __shared__ __align__(16) uint8_t sm_raw[];
     __half* q_hi = reinterpret_cast<__half*>(sm_raw);
     __half* q_lo = q_hi + TC_Q * TC_PITCH;
@@ -268,6 +268,14 @@ __global__ void __launch_bounds__(128) dattn_span_tc_kernel(AttnGeom g, const fl
     int c_end = (n_keys + ATTN_CHUNK - 1) / ATTN_CHUNK;
     if (c_end > c_begin + chunks_per_span) c_end = c_begin + chunks_per_span;
 
+    // The context columns were written by earlier passes (the block's newest ones may still be on their way: a prefetch is only a hint), so
+    // their way from DRAM to L2 need not wait for the kernel before.
+    for (int idx = threadIdx.x; idx < 2 * ATTN_CHUNK * 4; idx += 128) {   // 128-byte lines of the span's first chunk
+        const int kp = (idx >> 2) & (ATTN_CHUNK - 1), j = c_begin * ATTN_CHUNK + kp;
+        const float* row = (idx >= ATTN_CHUNK * 4 ? v_ctx : k_ctx) + ((uint64_t)(ctx_begin + j) * g.n_kv + kvh) * TC_HD + (idx & 3) * 32;
+        if (j < n_ctx) asm volatile("prefetch.global.L2 [%0];" ::"l"(row));
+    }
+    pdl_wait();
     const float scale = 1.4426950408889634f / sqrtf((float)TC_HD);
     for (int idx = threadIdx.x; idx < TC_Q * (TC_HD / 4); idx += 128) {
         const int pair = idx / (TC_HD / 4), d4 = (idx % (TC_HD / 4)) * 4;
@@ -293,14 +301,18 @@ __global__ void __launch_bounds__(128) dattn_span_tc_kernel(AttnGeom g, const fl
 
     float4 kk[8], vv[8];
     bool have_half = false;
-    const uint64_t row_stride = (uint64_t)g.n_kv * TC_HD;
+    // 32 keys of a chunk, eight K and eight V loads in flight per thread: context columns, then the block's own rows, then zeros
     auto load_half = [&](int chunk, int half) {
-        const uint64_t base = ((uint64_t)(ctx_begin + chunk * ATTN_CHUNK) * g.n_kv + kvh) * TC_HD;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int idx = threadIdx.x + 128 * (8 * half + i), kp = idx >> 5, d4 = (idx & 31) * 4;
-            kk[i] = *reinterpret_cast<const float4*>(k_ctx + base + kp * row_stride + d4);
-            vv[i] = *reinterpret_cast<const float4*>(v_ctx + base + kp * row_stride + d4);
+            const int idx = threadIdx.x + 128 * (8 * half + i), j = chunk * ATTN_CHUNK + (idx >> 5), d4 = (idx & 31) * 4;
+            const bool ctx = j < n_ctx;
+            const uint64_t off = ((uint64_t)(ctx ? ctx_begin + j : j - n_ctx) * g.n_kv + kvh) * TC_HD + d4;
+            kk[i] = vv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j < n_keys) {
+                kk[i] = *reinterpret_cast<const float4*>((ctx ? k_ctx : k_noise) + off);
+                vv[i] = *reinterpret_cast<const float4*>((ctx ? v_ctx : v_noise) + off);
+            }
         }
     };
     auto store_half = [&](int half) {
@@ -323,41 +335,12 @@ __global__ void __launch_bounds__(128) dattn_span_tc_kernel(AttnGeom g, const fl
         const int n_here = min(ATTN_CHUNK, n_keys - j0);
         __syncthreads();   // previous chunk fully consumed (and the query planes written)
         // K / V rows of the chunk: 64 x 512 B each, one float4 of K and of V per thread and step, split on the way in
-        if (j0 + ATTN_CHUNK <= n_ctx) {
-            // whole chunk inside the context: eight K and eight V loads in flight per thread before any of them is
-            // split; the first half was requested before the previous chunk's MMAs when that chunk took this path
-            if (!have_half) load_half(c, 0);
-            store_half(0);
-            load_half(c, 1);
-            store_half(1);
-        } else
-#pragma unroll 4
-        for (int i = 0; i < ATTN_CHUNK * 32 / 128; ++i) {
-            const int idx = threadIdx.x + 128 * i, kp = idx >> 5, d4 = (idx & 31) * 4;
-            float4 kk = make_float4(0.f, 0.f, 0.f, 0.f), vv = kk;
-            if (kp < n_here) {
-                const int j = j0 + kp;
-                if (j < n_ctx) {
-                    const uint64_t off = ((uint64_t)(ctx_begin + j) * g.n_kv + kvh) * TC_HD + d4;
-                    kk = *reinterpret_cast<const float4*>(k_ctx + off);
-                    vv = *reinterpret_cast<const float4*>(v_ctx + off);
-                } else {
-                    const uint64_t off = ((uint64_t)(j - n_ctx) * g.n_kv + kvh) * TC_HD + d4;
-                    kk = *reinterpret_cast<const float4*>(k_noise + off);
-                    vv = *reinterpret_cast<const float4*>(v_noise + off);
-                }
-            }
-            uint32_t h01, l01, h23, l23;
-            split_pair(kk.x, kk.y, h01, l01);
-            split_pair(kk.z, kk.w, h23, l23);
-            *reinterpret_cast<uint2*>(k_hi + kp * TC_PITCH + d4) = make_uint2(h01, h23);
-            *reinterpret_cast<uint2*>(k_lo + kp * TC_PITCH + d4) = make_uint2(l01, l23);
-            split_pair(vv.x, vv.y, h01, l01);
-            split_pair(vv.z, vv.w, h23, l23);
-            *reinterpret_cast<uint2*>(v_hi + kp * TC_PITCH + d4) = make_uint2(h01, h23);
-            *reinterpret_cast<uint2*>(v_lo + kp * TC_PITCH + d4) = make_uint2(l01, l23);
-        }
-        have_half = c + 1 < c_end && (c + 2) * ATTN_CHUNK <= n_ctx;
+        // before any of them is split; the first half was requested before the previous chunk's MMAs
+        if (!have_half) load_half(c, 0);
+        store_half(0);
+        load_half(c, 1);
+        store_half(1);
+        have_half = c + 1 < c_end;
         if (have_half) load_half(c + 1, 0);   // lands while this chunk's MMAs run
         if (threadIdx.x < ATTN_CHUNK) {
             const int j = j0 + (int)threadIdx.x;

@@ -862,18 +862,19 @@ __device__ __forceinline__ Top2 top2_block_reduce(Top2 a) {
 __device__ __forceinline__ float key_to_float(int32_t k) { return __int_as_float(k < 0 ? (k ^ 0x7fffffff) : k); }
 
 // One row per cluster of eight CTAs: grid (8, rows), 1024 threads.  Every thread ranks the columns of its CTA's range, eight
-// loads in flight; the CTAs' bests meet in the first one's shared memory, so the row needs neither a scratch array nor a second
+// loads (four columns of four slices with REDUCE) in flight; the CTAs' bests meet in the first one's shared memory, so the row needs neither a scratch array nor a second
 // launch (two kernels before: 4.7 + 3.2 us over 16 x 32 000, plus the boundary between them).  Eight CTAs a row put 128 on the
 // chip for a full block, and for one row still cover a 151 936-column range in 19 columns a thread, which is three round trips.
 // REDUCE: `src` holds split-K partial sums; each element is first reduced over the slices (slice order, as
 // reduce_partials_kernel does) and written to `logits`, so the head's logits are produced and ranked in one pass.
-constexpr int ARGMAX_CLUSTER = 8, ARGMAX_THREADS = 1024, ARGMAX_BATCH = 8;
+constexpr int ARGMAX_CLUSTER = 8, ARGMAX_THREADS = 1024;
 template <bool REDUCE>
 __global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(ARGMAX_THREADS)
 argmax_kernel(const float* src, uint64_t ld_src, int splits, uint64_t vocab, float* logits, uint64_t ld, int32_t* argmax, float* gap) {
     pdl_prologue();
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ Top2 best[ARGMAX_CLUSTER];
+    constexpr int ARGMAX_BATCH = REDUCE ? 4 : 8;
     const int row = blockIdx.y;
     const uint64_t per = (vocab + ARGMAX_CLUSTER - 1) / ARGMAX_CLUSTER;
     const uint64_t lo = blockIdx.x * per, hi = lo + per < vocab ? lo + per : vocab;
@@ -882,21 +883,23 @@ argmax_kernel(const float* src, uint64_t ld_src, int splits, uint64_t vocab, flo
     Top2 a{INT32_MIN, INT32_MAX, INT32_MIN, 0};
     for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += ARGMAX_BATCH * ARGMAX_THREADS) {
         float v[ARGMAX_BATCH];
+        if (!REDUCE) {
 #pragma unroll
-        for (int u = 0; u < ARGMAX_BATCH; ++u) {
-            const uint64_t i = i0 + u * ARGMAX_THREADS;
-            v[u] = i < hi ? (REDUCE ? 0.f + __ldcg(base + i) : __ldcg(base + i)) : 0.f;
-        }
-        if (REDUCE) {
-            for (int s = 1; s < splits; ++s) {
-                float t[ARGMAX_BATCH];
+            for (int u = 0; u < ARGMAX_BATCH; ++u) v[u] = i0 + u * ARGMAX_THREADS < hi ? __ldcg(base + i0 + u * ARGMAX_THREADS) : 0.f;
+        } else {
 #pragma unroll
-                for (int u = 0; u < ARGMAX_BATCH; ++u) {
-                    const uint64_t i = i0 + u * ARGMAX_THREADS;
-                    t[u] = i < hi ? __ldcg(base + (uint64_t)s * slice + i) : 0.f;
-                }
+            for (int u = 0; u < ARGMAX_BATCH; ++u) v[u] = 0.f;
+            for (int s0 = 0; s0 < splits; s0 += 4) {   // four slices of every column in flight, added in slice order
+                float t[4][ARGMAX_BATCH];
 #pragma unroll
-                for (int u = 0; u < ARGMAX_BATCH; ++u) v[u] += t[u];
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int u = 0; u < ARGMAX_BATCH; ++u)
+                        t[q][u] = s0 + q < splits && i0 + u * ARGMAX_THREADS < hi ? __ldcg(base + (uint64_t)(s0 + q) * slice + i0 + u * ARGMAX_THREADS) : 0.f;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int u = 0; u < ARGMAX_BATCH; ++u) v[u] += t[q][u];
             }
         }
 #pragma unroll
