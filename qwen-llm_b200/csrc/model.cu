@@ -326,6 +326,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             p.swiglu_f = inner;
             p.route_w = sc->route_w; p.route_sg = sc->route_sg; p.route_e = E; p.route_f = Fe;
             p.route_e0 = (int)m->ep_e0; p.route_n = En;
+            p.skip_unchosen = chosen_only && down_chosen;
             p.pre_scale = 1.0f / 64.0f;
             p.acts = sc->acts_f; p.bf3 = m->act_layout;
             p.n_rows = (int)n; p.err = s->err;
