@@ -8,6 +8,10 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <condition_variable>
+#include <deque>
+#include <mutex>
+#include <system_error>
 #include <thread>
 #include <limits>
 #include <string>
@@ -169,6 +173,7 @@ inline double exp_bound(double x) {
 // two tables, so that neighbours of one step do not wait for each other
 constexpr int kSteps = 1024;
 constexpr double kPerUnit = 16.0;
+constexpr double kNothing = -48.0;   // weights below e^-48 = 1.4e-21: 2^31 of them weigh 3e-12 of the largest, less than the bound on the sum
 struct StepMass { double m[2][kSteps]; };
 inline void add_mass(StepMass& sm, int table, double x) {
     const double below = -x * kPerUnit;
@@ -199,13 +204,15 @@ uint64_t collect_plain(const float* l, uint64_t n, float thr, uint64_t* keys) {
 DFL_AVX2 void step_mass_avx2(const float* l, uint64_t n, double inv_t, double shift, StepMass& sm) {
     const __m256d it = _mm256_set1_pd(inv_t), sh = _mm256_set1_pd(shift), l2e = _mm256_set1_pd(kLog2e), ln2 = _mm256_set1_pd(kLn2),
                   floor_x = _mm256_set1_pd(-700.0), per_unit = _mm256_set1_pd(-kPerUnit);
-    const __m256d last_step = _mm256_set1_pd((double)(kSteps - 1)), zero = _mm256_setzero_pd();
+    const __m256d last_step = _mm256_set1_pd((double)(kSteps - 1)), zero = _mm256_setzero_pd(), nothing = _mm256_set1_pd(kNothing);
     alignas(32) double w[16];
     alignas(16) int32_t step[16];
     uint64_t i = 0;
     for (; i + 16 <= n; i += 16) {
         __m256d x[4], k[4], r[4], p[4];
         for (int j = 0; j < 4; ++j) x[j] = _mm256_fmsub_pd(_mm256_cvtps_pd(_mm_loadu_ps(l + i + 4 * j)), it, sh);
+        const __m256d top = _mm256_max_pd(_mm256_max_pd(x[0], x[1]), _mm256_max_pd(x[2], x[3]));
+        if (_mm256_movemask_pd(_mm256_cmp_pd(top, nothing, _CMP_GT_OQ)) == 0) continue;
         for (int j = 0; j < 4; ++j) k[j] = _mm256_round_pd(_mm256_mul_pd(x[j], l2e), _MM_FROUND_TO_NEAREST_INT | _MM_FROUND_NO_EXC);
         for (int j = 0; j < 4; ++j) r[j] = _mm256_fnmadd_pd(k[j], ln2, x[j]);
         for (int j = 0; j < 4; ++j) p[j] = _mm256_set1_pd(kInvFact[kDegree]);
@@ -220,6 +227,55 @@ DFL_AVX2 void step_mass_avx2(const float* l, uint64_t n, double inv_t, double sh
         for (int j = 0; j < 16; ++j) sm.m[j & 1][step[j]] += w[j];
     }
     for (; i < n; ++i) add_mass(sm, (int)(i & 1), (double)l[i] * inv_t - shift);
+}
+#define DFL_AVX512 __attribute__((target("avx512f,avx512dq,avx2,fma")))
+DFL_AVX512 void step_mass_avx512(const float* l, uint64_t n, double inv_t, double shift, StepMass& sm) {
+    const __m512d it = _mm512_set1_pd(inv_t), sh = _mm512_set1_pd(shift), l2e = _mm512_set1_pd(kLog2e), ln2 = _mm512_set1_pd(kLn2),
+                  floor_x = _mm512_set1_pd(-700.0), per_unit = _mm512_set1_pd(-kPerUnit), nothing = _mm512_set1_pd(kNothing);
+    const __m512d last_step = _mm512_set1_pd((double)(kSteps - 1)), zero = _mm512_setzero_pd();
+    alignas(64) double w[32];
+    alignas(32) int32_t step[32];
+    uint64_t i = 0;
+    for (; i + 32 <= n; i += 32) {
+        __m512d x[4], k[4], r[4], p[4];
+        for (int j = 0; j < 4; ++j) x[j] = _mm512_fmsub_pd(_mm512_cvtps_pd(_mm256_loadu_ps(l + i + 8 * j)), it, sh);
+        const __m512d top = _mm512_max_pd(_mm512_max_pd(x[0], x[1]), _mm512_max_pd(x[2], x[3]));
+        if (_mm512_cmp_pd_mask(top, nothing, _CMP_GT_OQ) == 0) continue;
+        for (int j = 0; j < 4; ++j) k[j] = _mm512_roundscale_pd(_mm512_mul_pd(x[j], l2e), _MM_FROUND_TO_NEAREST_INT | _MM_FROUND_NO_EXC);
+        for (int j = 0; j < 4; ++j) r[j] = _mm512_fnmadd_pd(k[j], ln2, x[j]);
+        for (int j = 0; j < 4; ++j) p[j] = _mm512_set1_pd(kInvFact[kDegree]);
+        for (int d = kDegree - 1; d >= 0; --d)
+            for (int j = 0; j < 4; ++j) p[j] = _mm512_fmadd_pd(p[j], r[j], _mm512_set1_pd(kInvFact[d]));
+        for (int j = 0; j < 4; ++j) {
+            _mm512_store_pd(w + 8 * j, _mm512_maskz_scalef_pd(_mm512_cmp_pd_mask(x[j], floor_x, _CMP_GT_OQ), p[j], k[j]));
+            _mm256_store_si256((__m256i*)(step + 8 * j),
+                               _mm512_cvttpd_epi32(_mm512_max_pd(_mm512_min_pd(_mm512_mul_pd(x[j], per_unit), last_step), zero)));
+        }
+        for (int j = 0; j < 32; ++j) sm.m[j & 1][step[j]] += w[j];
+    }
+    for (; i < n; ++i) add_mass(sm, (int)(i & 1), (double)l[i] * inv_t - shift);
+}
+DFL_AVX512 uint64_t collect_avx512(const float* l, uint64_t n, float thr, uint64_t* keys) {
+    const __m512 t = _mm512_set1_ps(thr);
+    const __m512i magnitude = _mm512_set1_epi32(0x7fffffff), lanes = _mm512_set_epi64(7, 6, 5, 4, 3, 2, 1, 0);
+    uint64_t c = 0, i = 0;
+    for (; i + 16 <= n; i += 16) {
+        const __m512 v = _mm512_loadu_ps(l + i);
+        const unsigned m = _mm512_cmp_ps_mask(v, t, _CMP_GE_OQ);
+        if (!m) continue;
+        const __m512i b = _mm512_castps_si512(v), d = _mm512_xor_si512(b, _mm512_andnot_si512(_mm512_srai_epi32(b, 31), magnitude));
+        const __m512i at = _mm512_add_epi64(_mm512_set1_epi64((long long)i), lanes);
+        const __m512i k0 = _mm512_or_si512(_mm512_slli_epi64(_mm512_cvtepu32_epi64(_mm512_castsi512_si256(d)), 32), at);
+        const __m512i k1 = _mm512_or_si512(_mm512_slli_epi64(_mm512_cvtepu32_epi64(_mm512_extracti64x4_epi64(d, 1)), 32),
+                                           _mm512_add_epi64(at, _mm512_set1_epi64(8)));
+        _mm512_mask_compressstoreu_epi64(keys + c, (__mmask8)(m & 255u), k0);
+        c += (uint64_t)__builtin_popcount(m & 255u);
+        _mm512_mask_compressstoreu_epi64(keys + c, (__mmask8)(m >> 8), k1);
+        c += (uint64_t)__builtin_popcount(m >> 8);
+    }
+    for (; i < n; ++i)
+        if (l[i] >= thr) keys[c++] = ((uint64_t)descending_bits(l[i]) << 32) | i;
+    return c;
 }
 DFL_AVX2 bool max_of_avx2(const float* l, uint64_t n, float* mx) {
     if (n < 16) return max_of_plain(l, n, mx);
@@ -259,11 +315,17 @@ inline bool have_avx2() {
     static const bool yes = __builtin_cpu_supports("avx2") && __builtin_cpu_supports("fma");
     return yes;
 }
+inline bool have_avx512() {
+    static const bool yes = __builtin_cpu_supports("avx512f") && __builtin_cpu_supports("avx512dq");
+    return yes;
+}
 inline void step_mass(const float* l, uint64_t n, double inv_t, double shift, StepMass& sm) {
-    have_avx2() ? step_mass_avx2(l, n, inv_t, shift, sm) : step_mass_plain(l, n, inv_t, shift, sm);
+    have_avx512() ? step_mass_avx512(l, n, inv_t, shift, sm) : have_avx2() ? step_mass_avx2(l, n, inv_t, shift, sm) : step_mass_plain(l, n, inv_t, shift, sm);
 }
 inline bool max_of(const float* l, uint64_t n, float* mx) { return have_avx2() ? max_of_avx2(l, n, mx) : max_of_plain(l, n, mx); }
-inline uint64_t collect(const float* l, uint64_t n, float thr, uint64_t* keys) { return have_avx2() ? collect_avx2(l, n, thr, keys) : collect_plain(l, n, thr, keys); }
+inline uint64_t collect(const float* l, uint64_t n, float thr, uint64_t* keys) {
+    return have_avx512() ? collect_avx512(l, n, thr, keys) : have_avx2() ? collect_avx2(l, n, thr, keys) : collect_plain(l, n, thr, keys);
+}
 #else
 inline void step_mass(const float* l, uint64_t n, double inv_t, double shift, StepMass& sm) { step_mass_plain(l, n, inv_t, shift, sm); }
 inline bool max_of(const float* l, uint64_t n, float* mx) { return max_of_plain(l, n, mx); }
@@ -308,15 +370,18 @@ struct dfl_sampler {
     Xoshiro rng;
     uint64_t draws = 0;
     Buffers buf;
-    // Distributions of a block's rows built ahead of the sequential accept loop, one host thread per row: building a
-    // row's distribution draws nothing from the generator, so only the picks have to stay in row order.  Rows are
-    // built in waves as the loop reaches them (the first wave covers a typical accepted prefix), so a block rejected
-    // early does not pay for all of its rows.
+    // Distributions of a block's rows built ahead of the sequential accept loop: building a row's distribution draws nothing from
+    // the generator, so only the picks have to stay in row order.  The sampler's threads take rows in order up to a
+    // limit that moves with the loop (the first six cover a typical accepted prefix), so a block rejected early does
+    // not pay for all of its rows; a row that no thread has taken yet when the loop reaches it is built by the loop's own
+    // thread, so nothing waits for a thread to wake.  The threads are kept with the sampler: starting five of them a
+    // block cost 0.2 - 0.3 ms, as much as the rows themselves when each has a clear favourite.
     struct Prepared {
         const float* logits = nullptr;
         Dist dist;
         SErr err = S_OK;
         uint64_t nan_token = 0;
+        std::atomic<bool> done{false};
         Buffers buf;
     };
     // rows whose order was made elsewhere (dfl_sampler_set_row_order)
@@ -332,51 +397,111 @@ struct dfl_sampler {
         if (off % ord_vocab || off / ord_vocab >= ord_rows) return nullptr;
         return ord_base + off;
     }
-    std::vector<Prepared> prepared;
+    std::deque<Prepared> prepared;   // rows stay where they are when it grows
     const float* block_logits = nullptr;
     uint64_t block_vocab = 0;
-    uint32_t block_rows = 0, n_prepared = 0;
+    uint32_t block_rows = 0;
+    struct Threads {
+        std::vector<std::thread> th;
+        std::mutex mu;
+        std::condition_variable work, idle;
+        uint32_t next = 0, limit = 0, running = 0;   // rows [next, limit) may be taken; guarded by mu, like quit
+        bool quit = false;
+        std::atomic<bool> stop{false};   // the block has been decided: rows still being built are not wanted any more
+    } threads;
 
+    ~dfl_sampler() {
+        {
+            std::lock_guard<std::mutex> lock(threads.mu);
+            threads.quit = true;
+        }
+        threads.work.notify_all();
+        for (auto& t : threads.th) t.join();
+    }
+    void build_row(uint32_t r) {
+        Prepared& p = prepared[r];
+        p.err = distribution(p.logits, block_vocab, p.dist, &p.nan_token, p.buf, &threads.stop);
+        p.done.store(true, std::memory_order_release);
+    }
+    void thread_main() {
+        std::unique_lock<std::mutex> lock(threads.mu);
+        for (;;) {
+            threads.work.wait(lock, [&] { return threads.quit || threads.next < threads.limit; });
+            if (threads.quit) return;
+            const uint32_t r = threads.next++;
+            ++threads.running;
+            lock.unlock();
+            build_row(r);
+            lock.lock();
+            if (--threads.running == 0) threads.idle.notify_all();
+        }
+    }
+    // rows before `limit` may be built ahead
+    void allow_rows(uint32_t limit) {
+        limit = std::min(limit, block_rows);
+        const uint32_t wanted = std::min<uint32_t>(std::max(2u, worker_limit()) - 1, std::min(limit, 10u));
+        {
+            std::lock_guard<std::mutex> lock(threads.mu);
+            if (limit <= threads.limit) return;
+            threads.limit = limit;
+        }
+        try {
+            while (threads.th.size() < wanted) threads.th.emplace_back([this] { thread_main(); });
+        } catch (const std::system_error&) {}   // no more threads to be had: the loop builds what they do not
+        threads.work.notify_all();
+    }
     void prepare_rows(const float* logits, uint32_t n_rows, uint64_t vocab) {
         block_logits = nullptr;
-        n_prepared = block_rows = 0;
+        block_rows = 0;
         if (cfg.temperature == 0.0f || n_rows < 2 || vocab < 4096 || worker_limit() < 2) return;
         block_logits = logits;
         block_vocab = vocab;
         block_rows = n_rows;
-        if (prepared.size() < n_rows) prepared.resize(n_rows);
+        while (prepared.size() < n_rows) prepared.emplace_back();
+        for (uint32_t r = 0; r < n_rows; ++r) {
+            prepared[r].logits = logits + (uint64_t)r * vocab;
+            prepared[r].done.store(false, std::memory_order_relaxed);
+        }
+        {
+            std::lock_guard<std::mutex> lock(threads.mu);
+            threads.next = threads.limit = 0;
+            threads.stop.store(false, std::memory_order_relaxed);
+        }
+        allow_rows(6);
     }
-    void end_block() { block_logits = nullptr; n_prepared = block_rows = 0; }
+    // no thread reads the block's logits any more
+    void end_block() {
+        if (block_logits) {
+            threads.stop.store(true, std::memory_order_relaxed);
+            std::unique_lock<std::mutex> lock(threads.mu);
+            threads.limit = 0;
+            threads.idle.wait(lock, [&] { return threads.running == 0; });
+        }
+        block_logits = nullptr;
+        block_rows = 0;
+    }
     unsigned worker_limit() const { return workers ? workers : std::thread::hardware_concurrency(); }
-    void prepare_wave(uint32_t upto) {
-        const unsigned hw = std::max(2u, worker_limit());
-        const uint32_t first = n_prepared, last = std::min(block_rows, std::max(upto + 1, first + std::min<uint32_t>(hw, first == 0 ? 6 : 10)));
-        const uint32_t n_threads = std::min<uint32_t>(last - first, hw);
-        auto work = [&](uint32_t t) {
-            for (uint32_t r = first + t; r < last; r += n_threads) {
-                Prepared& p = prepared[r];
-                p.logits = block_logits + (uint64_t)r * block_vocab;
-                p.err = distribution(p.logits, block_vocab, p.dist, &p.nan_token, p.buf);
-            }
-        };
-        std::vector<std::thread> pool;
-        for (uint32_t t = 1; t < n_threads; ++t) pool.emplace_back(work, t);
-        work(0);
-        for (auto& t : pool) t.join();
-        n_prepared = last;
-    }
     // the prepared distribution of this row, if it belongs to the current block (moved out: a row is consumed once)
     bool take_prepared(const float* logits, Dist& d, SErr* e, uint64_t* nan_token) {
         if (!block_logits || logits < block_logits) return false;
         const uint64_t off = (uint64_t)(logits - block_logits);
         if (off % block_vocab || off / block_vocab >= block_rows) return false;
         const uint32_t r = (uint32_t)(off / block_vocab);
-        if (r >= n_prepared) prepare_wave(r);
-        if (prepared[r].logits != logits) return false;
-        *e = prepared[r].err;
-        *nan_token = prepared[r].nan_token;
-        std::swap(d, prepared[r].dist);
-        prepared[r].logits = nullptr;
+        Prepared& p = prepared[r];
+        if (p.logits != logits) return false;
+        bool taken;
+        {
+            std::lock_guard<std::mutex> lock(threads.mu);
+            taken = r < threads.next;
+            if (!taken) threads.next = r + 1;
+        }
+        if (r >= 4) allow_rows(r + 8);
+        if (!taken) build_row(r);
+        while (!p.done.load(std::memory_order_acquire)) std::this_thread::yield();
+        *e = p.err;
+        *nan_token = p.nan_token;
+        std::swap(d, p.dist);
+        p.logits = nullptr;
         return true;
     }
 
@@ -392,13 +517,18 @@ struct dfl_sampler {
     // ordering, exact weights and exact running sum over those alone.  Where the running sum comes within EPS of the target
     // the general path decides: tokens, weights, total and draws are its own, bit for bit.  Below 1024 tokens the step tables
     // cost more than ordering.  16 rows of 151 936, four accepted: 4.4 -> 1.2 ms; one row with 44 600 in its nucleus 4.3 -> 2.6 ms.
-    bool nucleus(const float* logits, uint64_t n, Dist& d, Buffers& buf) const {
+    // `stop` (optional): return at the next step with nothing of use.
+    bool nucleus(const float* logits, uint64_t n, Dist& d, Buffers& buf, const std::atomic<bool>* stop) const {
+        auto stopped = [&] { return stop && stop->load(std::memory_order_relaxed); };
         if (cfg.top_k != 0 || cfg.min_p > 0.0f || !(cfg.top_p < 1.0f) || n < 1024 || n > 0x7fffffffull) return false;
         float mx;
         if (!max_of(logits, n, &mx) || !std::isfinite(mx)) return false;
         const double t = (double)cfg.temperature, inv_t = 1.0 / t, max_logit = (double)mx / t;
         StepMass sm{};
-        step_mass(logits, n, inv_t, (double)mx * inv_t, sm);
+        for (uint64_t off = 0; off < n; off += 16384) {
+            if (stopped()) return true;
+            step_mass(logits + off, std::min<uint64_t>(16384, n - off), inv_t, (double)mx * inv_t, sm);
+        }
         double total = 0.0;
         for (int b = 0; b < kSteps; ++b) total += sm.m[0][b] + sm.m[1][b];
         if (!std::isfinite(max_logit) || !std::isfinite(total) || total < 0.5) return false;
@@ -420,11 +550,13 @@ struct dfl_sampler {
         if (buf.keys.size() < n + 1) buf.keys.resize(n + 1);
         const uint64_t len = collect(logits, n, thr, buf.keys.data());
         if (len == 0) return false;
+        if (stopped()) return true;
         sort_keys(buf.keys, buf.scratch, len);
         const uint64_t* keys = buf.keys.data();
         d.weights.resize(len);
         double cum = 0.0, *w = d.weights.data();
         for (uint64_t first = 0; first < len; first += 1024) {
+            if (stopped()) return true;
             const uint64_t last = std::min<uint64_t>(len, first + 1024);
             for (uint64_t i = first; i < last; ++i) w[i] = key_logit(keys[i]) / t - max_logit;
             for (uint64_t i = first; i < last; ++i) w[i] = std::exp(w[i]);
@@ -441,8 +573,8 @@ struct dfl_sampler {
         }
         return false;
     }
-    SErr distribution(const float* logits, uint64_t n, Dist& d, uint64_t* nan_token, Buffers& buf) const {
-        if (!order_for(logits, n) && nucleus(logits, n, d, buf)) return S_OK;
+    SErr distribution(const float* logits, uint64_t n, Dist& d, uint64_t* nan_token, Buffers& buf, const std::atomic<bool>* stop = nullptr) const {
+        if (!order_for(logits, n) && nucleus(logits, n, d, buf, stop)) return S_OK;
         uint64_t len = 0;
         bool order_used = false;
         SErr e = order_keys(logits, n, cfg.top_k, buf, &len, nan_token, order_for(logits, n), &order_used);
