@@ -341,8 +341,8 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
     ok = ok && cudaMalloc(&p->acts1, acts_bytes_for(w1->m)) == cudaSuccess;
     ok = ok && cudaMalloc(&p->acts2, acts_bytes_for(head->m)) == cudaSuccess;
     ok = ok && cudaEventCreate(&p->e0) == cudaSuccess && cudaEventCreate(&p->e1) == cudaSuccess;
-    ok = ok && cudaMallocHost(&p->out, sizeof(dfl_c1::HostOut)) == cudaSuccess;
-    ok = ok && cudaMallocHost(&p->x_host, MAX_ROWS * k1 * 4) == cudaSuccess;
+    ok = ok && (p->out = (dfl_c1::HostOut*)pool_alloc_host(sizeof(dfl_c1::HostOut)));
+    ok = ok && (p->x_host = (float*)pool_alloc_host(MAX_ROWS * k1 * 4));
     if (!ok) {
         dfl_c1_destroy(p);
         return fail(DFL_ERR_OOM, std::string("c1_create: allocation failed: ") + cudaGetErrorString(cudaGetLastError()));
@@ -360,8 +360,8 @@ void dfl_c1_destroy(dfl_c1* p) {
     if (!p) return;
     cudaSetDevice(p->w1->m.device);
     cudaFree(p->x); cudaFree(p->part1); cudaFree(p->part2); cudaFree(p->logits); cudaFree(p->acts1); cudaFree(p->acts2);
-    if (p->out) cudaFreeHost(p->out);
-    if (p->x_host) cudaFreeHost(p->x_host);
+    pool_free(p->out);
+    pool_free(p->x_host);
     if (p->e0) cudaEventDestroy(p->e0);
     if (p->e1) cudaEventDestroy(p->e1);
     if (p->st) cudaStreamDestroy(p->st);
@@ -369,8 +369,8 @@ void dfl_c1_destroy(dfl_c1* p) {
 }
 
 // Five launches: pack the rows, GEMM, sum and pack, GEMM, rank.  `x` is device memory or the pinned rows, which the packing kernel
-// reads across the bus itself (256 KB: less than a copy engine's start-up away); argmax, gap and the error word land in pinned
-// memory, so that a step waits for its stream once and copies nothing.
+// reads across the bus itself; argmax, gap and the error word land in pinned memory, so that a step waits for its stream
+// once and copies nothing.  (Packing the first half of the columns while the host still copies the second: no gain.)
 static dfl_status c1_enqueue(dfl_c1* p, const float* x, int n_rows) {
     const QMatrix& a = p->w1->m;
     const QMatrix& b = p->head->m;
@@ -388,6 +388,7 @@ static dfl_status c1_enqueue(dfl_c1* p, const float* x, int n_rows) {
     if (p->splits2 == 1) return launch_argmax_top2(p->st, p->logits, n_rows, b.n_out, b.n_out, p->out->argmax, p->out->gap);
     return launch_reduce_argmax_top2(p->st, p->part2, p->splits2, n_rows, b.n_out, p->logits, b.n_out, p->out->argmax, p->out->gap);
 }
+
 dfl_status dfl_c1_upload(dfl_c1* p, const float* x_host, int32_t n_rows) {
     if (!p || !x_host) return fail(DFL_ERR_BAD_ARG, "c1_upload: null argument");
     if (n_rows < 1 || n_rows > MAX_ROWS) return fail(DFL_ERR_BAD_SHAPE, "c1: n_rows must be in [1, 16]");
