@@ -404,6 +404,18 @@ void dfl_drafter_destroy(dfl_drafter* d) {
 
 uint64_t dfl_drafter_weight_bytes(const dfl_drafter* d) { return d ? d->weight_bytes : 0; }
 
+// the context projections' matrices are all bf16 on the tensor-memory kernel
+static bool grouped_projection(const dfl_drafter* d) {
+    auto ok = [](const MatGroup& g) {
+        for (auto& m : g.mats)
+            if (m.layout != LAYOUT_TS || m.dtype != DFL_BF16) return false;
+        return true;
+    };
+    bool all = ok(d->fc);
+    for (auto& L : d->layers) all = all && ok(L.kv);
+    return all;
+}
+
 dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_dsession** out) {
     if (!d || !out) return fail(DFL_ERR_BAD_ARG, "dsession_create: null argument");
     *out = nullptr;
@@ -469,13 +481,14 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
         ds->acts_h = (uint8_t*)alloc(acts_bytes(DFL_BF16, H));
         ds->acts_f = (uint8_t*)alloc(acts_bytes(DFL_BF16, F));
         ds->acts_q = (uint8_t*)alloc(acts_bytes(DFL_BF16, q_dim));
-        ds->acts_fc = (uint8_t*)alloc(acts_bytes(DFL_BF16, KH));
+        const uint64_t G = grouped_projection(d) ? TSB_GROUPS : 1;   // sixteen-row groups that are projected together
+        ds->acts_fc = (uint8_t*)alloc(G * acts_bytes(DFL_BF16, KH));
         {
             uint64_t part_c = (uint64_t)d->fc.splits * MAX_ROWS * d->fc.total_cols;
             for (auto& L : d->layers) part_c = std::max<uint64_t>(part_c, (uint64_t)L.kv.splits * MAX_ROWS * L.kv.total_cols);
-            ds->part_c = (float*)alloc(part_c * 4);
-            ds->sumsq_c = (float*)alloc((H / GLUE_COLS) * MAX_ROWS * 4);
-            ds->acts_hc = (uint8_t*)alloc(acts_bytes(DFL_BF16, H));
+            ds->part_c = (float*)alloc(G * part_c * 4);
+            ds->sumsq_c = (float*)alloc(G * (H / GLUE_COLS) * MAX_ROWS * 4);
+            ds->acts_hc = (uint8_t*)alloc(G * acts_bytes(DFL_BF16, H));
         }
         ds->acts_lm = (uint8_t*)alloc(acts_bytes(DFL_BF16, H));
         ds->logits = (float*)alloc(MAX_ROWS * V * 4);
@@ -571,7 +584,10 @@ dfl_status dsession_project_pending(dfl_dsession* ds, bool on_side) {
     ep_norm.eps = c.rms_norm_eps;
     const AttnGeom gkv = d->geom(0);
     while (ds->ready < ds->ctx_len) {
-        const uint32_t c0 = ds->ready, nb = std::min<uint32_t>(MAX_ROWS, ds->ctx_len - c0);
+        // more than sixteen columns: groups of sixteen share a pass over the weights (the same bits as one by one)
+        const bool many = ds->ctx_len - ds->ready > MAX_ROWS && grouped_projection(d);
+        const uint32_t c0 = ds->ready, nb = std::min<uint32_t>(many ? TSB_GROUPS * MAX_ROWS : MAX_ROWS, ds->ctx_len - c0);
+        const int n_groups = (int)((nb + MAX_ROWS - 1) / MAX_ROWS), part_rows = many ? TSB_GROUPS * MAX_ROWS : MAX_ROWS;
         const bool last_block = c0 + nb == ds->ctx_len;
         GlueParams p;
         p.mode = GLUE_COPY;
@@ -579,21 +595,27 @@ dfl_status dsession_project_pending(dfl_dsession* ds, bool on_side) {
         p.ld_x = (int)KH;
         p.acts = ds->acts_fc; p.bf3 = act_layout_of(d->fc.mats[0]);
         p.n_rows = (int)nb; p.err = ds->err;
-        DFL_CHECK(launch_glue(st, p, KH));
-        DFL_CHECK(launch_group(st, d->fc, ds->acts_fc, ds->part_c, GemmEpilogue{}, ds->err));
+        auto group = [&](const MatGroup& m, const uint8_t* acts, const GemmEpilogue& ep) -> dfl_status {
+            if (!many) return launch_group(st, m, acts, ds->part_c, ep, ds->err);
+            for (size_t i = 0; i < m.mats.size(); ++i)
+                DFL_CHECK(launch_gemm_tsb_groups(st, m.mats[i], acts, ds->part_c + m.col_off[i], m.splits, n_groups, ep, ds->err, (uint32_t)m.total_cols));
+            return DFL_OK;
+        };
+        DFL_CHECK(many ? launch_glue_groups(st, p, KH) : launch_glue(st, p, KH));
+        DFL_CHECK(group(d->fc, ds->acts_fc, GemmEpilogue{}));
         GlueParams q;
         q.mode = GLUE_RESID;
-        q.part = ds->part_c; q.splits = d->fc.splits; q.ld_part = (int)d->fc.total_cols;
+        q.part = ds->part_c; q.splits = d->fc.splits; q.ld_part = (int)d->fc.total_cols; q.part_rows = part_rows;
         q.mul_w = d->hidden_norm_w;
         q.sumsq = ds->sumsq_c;
         q.acts = ds->acts_hc; q.bf3 = act_layout_of(d->layers[0].kv.mats[0]);
         q.n_rows = (int)nb; q.err = ds->err;
-        DFL_CHECK(launch_glue(st, q, H));
+        DFL_CHECK(many ? launch_glue_groups(st, q, H) : launch_glue(st, q, H));
         for (uint32_t il = 0; il < c.n_layer; ++il) {
             const DLayerW& L = d->layers[il];
-            DFL_CHECK(launch_group(st, L.kv, ds->acts_hc, ds->part_c, ep_norm, ds->err));
+            DFL_CHECK(group(L.kv, ds->acts_hc, ep_norm));
             DFL_CHECK(launch_attn_front(st, gkv, false, ds->part_c, L.kv.splits, (int)L.kv.total_cols, nullptr, L.k_norm_w, 0, (int)nb, ds->k_ctx[il],
-                                        ds->v_ctx[il], KV_F32_ROWS, nullptr, nullptr, ds->pos_ctx_dev + c0, (long long)c0));
+                                        ds->v_ctx[il], KV_F32_ROWS, nullptr, nullptr, ds->pos_ctx_dev + c0, (long long)c0, part_rows));
             if (ds->ctx_tiles[il]) DFL_CHECK(launch_dctx_tiles(st, ds->k_ctx[il], ds->v_ctx[il], (int)c.n_kv_heads, c0, nb, c0, ds->ctx_tiles[il]));
             if (on_side && last_block) DFL_CUDA(cudaEventRecord(ds->ev_ctx[il], st));
         }

@@ -148,6 +148,9 @@ int gemm_ts_kc();
 int gemm_tsb_choose_splits_multi(const int* row_tiles, int n_mats, int kblocks);
 dfl_status launch_gemm_tsb(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, const GemmEpilogue& ep,
                            int* dev_err, bool pdl, uint32_t ld_out);
+constexpr int TSB_GROUPS = 4;   // sixteen-row groups of a grouped launch
+dfl_status launch_gemm_tsb_groups(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_groups,
+                                  const GemmEpilogue& ep, int* dev_err, uint32_t ld_out);
 dfl_status launch_prep_acts_tsb(cudaStream_t st, const float* x, int ld, int n_rows, uint64_t k, float pre_scale, uint8_t* acts);
 
 }  // namespace dfl

@@ -73,6 +73,7 @@ struct ParamsB {
     int kblocks, splits, row_tiles, ctas_per_split;
     uint32_t n_out, ld_out;
     int* err;
+    int n_groups = 1;   // gemm_tsb_groups_kernel: groups of sixteen rows
 };
 
 constexpr int tsb_smem_bytes() { return TSB_KC * ACTTSB_CHUNK + TSB_STAGES * TSB_SLOT + 256; }
@@ -241,6 +242,170 @@ __global__ void __launch_bounds__(TSB_THREADS, 1) gemm_tsb_kernel(const ParamsB 
     }
 }
 
+// ---- several groups of sixteen rows on one pass over the weights ----------------------------------------------------
+// A prompt's captured rows become drafter context hundreds at a time.  With sixteen rows a pass the weights are streamed once per
+// group (fc 20 480 -> 4096: 31 us for 16 rows, HBM bound); here a ring stage holds half a weight block and the matching
+// activations of up to four groups, each group with an accumulator of its own.  The MMAs of a group are those of
+// gemm_tsb_kernel in the same order over the same split ranges, so a row's result does not depend on which kernel computed it.
+// Activations travel through the ring (48 KiB a stage from L2) because four groups of a split's range do not fit beside it.
+constexpr int TSG_GROUPS = TSB_GROUPS, TSG_HALF = ACTTSB_CHUNK / 2, TSG_STAGE = TSB_SLOT + TSG_GROUPS * TSG_HALF, TSG_STAGES = 2;
+__host__ __device__ constexpr int tsg_smem_bytes() { return TSG_STAGES * TSG_STAGE + 256; }
+
+__global__ void __launch_bounds__(TSB_THREADS, 1) gemm_tsb_groups_kernel(const ParamsB p) {
+    static_assert(tsg_smem_bytes() <= 227 * 1024, "shared memory budget");
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + TSG_STAGES * TSG_STAGE);
+    uint64_t* empty = full + TSG_STAGES;
+    uint64_t* d_full = empty + TSG_STAGES;   // [2] a tile's accumulators are complete
+    uint64_t* d_empty = d_full + 2;          // [2] the epilogue has read them
+    __shared__ uint32_t tmem_slot;
+    __shared__ float tok_scale[TSG_GROUPS * MAX_ROWS];
+    __shared__ int abort_flag;
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int sp = blockIdx.x % p.splits, c = blockIdx.x / p.splits;
+    const int kb0 = (int)((long long)sp * p.kblocks / p.splits), kb1 = (int)((long long)(sp + 1) * p.kblocks / p.splits);
+    const int n_my = (p.row_tiles - c + p.ctas_per_split - 1) / p.ctas_per_split;
+    const int n_slots_tile = 2 * (kb1 - kb0), n_it = n_my * n_slots_tile;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < TSG_STAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&d_full[i], 1);
+            mbar_init(&d_empty[i], 4);
+        }
+        abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == 1) tmem_alloc(&tmem_slot, 512);   // [accumulator 2][group 4], 64 columns apart
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint64_t tile_stride = (uint64_t)p.kblocks * STAGE_B16, group_stride = (uint64_t)p.kblocks * ACTTSB_CHUNK;
+            auto weights = [&](int e, int pt, int pk) {
+                const int s = e % TSG_STAGES;
+                mbar_arrive_expect_tx(&full[s], TSB_SLOT + p.n_groups * TSG_HALF);
+                bulk_g2s(smem + s * TSG_STAGE, p.w + (uint64_t)(c + pt * p.ctas_per_split) * tile_stride + (uint64_t)kb0 * STAGE_B16 + (uint64_t)pk * TSB_SLOT,
+                         TSB_SLOT, &full[s]);
+            };
+            auto rows = [&](int e, int pk) {
+                const int s = e % TSG_STAGES;
+                const uint8_t* src = p.acts + (uint64_t)kb0 * ACTTSB_CHUNK + (uint64_t)pk * TSG_HALF;
+                for (int g = 0; g < p.n_groups; ++g) bulk_g2s(smem + s * TSG_STAGE + TSB_SLOT + g * TSG_HALF, src + g * group_stride, TSG_HALF, &full[s]);
+            };
+            // the weights do not depend on the previous kernel, the activations do
+            const int head = n_it < TSG_STAGES ? n_it : TSG_STAGES;
+            for (int e = 0; e < head; ++e) weights(e, e / n_slots_tile, e % n_slots_tile);
+            pdl_wait();
+            bool ok = true;
+            int pt = 0, pk = 0;
+            for (int e = 0; e < n_it && ok; ++e) {
+                if (e >= head) {
+                    ok = mbar_wait_one(&empty[e % TSG_STAGES], ((e / TSG_STAGES) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
+                    if (!ok) break;
+                    weights(e, pt, pk);
+                }
+                rows(e, pk);
+                if (++pk == n_slots_tile) { pk = 0; ++pt; }
+            }
+            if (!ok) abort_flag = 1;
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t IDESC = instr_desc_bf16(48);
+        bool ok = true;
+        const uint32_t ring_addr = smem_u32(smem);
+        int e = 0;
+        for (int t = 0; t < n_my && ok; ++t) {
+            const int buf = t & 1;
+            if (t >= 2) {
+                ok = mbar_wait_warp(&d_empty[buf], ((t >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
+                if (!ok) break;
+                fence_after_sync();
+            }
+            for (int h = 0; h < n_slots_tile && ok; ++h, ++e) {
+                const int s = e % TSG_STAGES;
+                ok = mbar_wait_warp(&full[s], (e / TSG_STAGES) & 1, p.err, DEV_ERR_WAIT_FULL);
+                if (!ok) break;
+                fence_after_sync();
+                if (elect_one()) {
+                    const uint32_t a_base = ring_addr + s * TSG_STAGE, b_base = a_base + TSB_SLOT;
+                    for (int g = 0; g < p.n_groups; ++g)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            mma_ss(tmem + 256 * buf + 64 * g, smem_desc(a_base + j * 4096, 2048, 128),
+                                   smem_desc(b_base + g * TSG_HALF + j * 1536, 768, 128), IDESC, (h | j) ? 1u : 0u);
+                    mma_commit(&empty[s]);
+                    if (h == n_slots_tile - 1) mma_commit(&d_full[buf]);
+                }
+                __syncwarp();
+            }
+        }
+        if (!ok) abort_flag = 1;
+    } else {
+        pdl_wait();
+        const int q4 = warp & 3, row = 32 * q4 + lane;
+        if (threadIdx.x - 64 < TSG_GROUPS * MAX_ROWS) {
+            const int r = threadIdx.x - 64, g = r / MAX_ROWS, tok = r % MAX_ROWS;
+            float ss = 0.f;
+            if (p.sumsq && g < p.n_groups)
+                for (int q = 0; q < p.n_sumsq; ++q) ss += p.sumsq[(g * p.n_sumsq + q) * MAX_ROWS + tok];
+            tok_scale[r] = p.sumsq ? p.out_scale * (1.0f / sqrtf(ss / p.norm_k + p.eps)) : p.out_scale;
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const uint32_t lane_base = tmem + ((uint32_t)(32 * q4) << 16);
+        bool ok = true;
+        for (int t = 0; t < n_my && ok; ++t) {
+            const int buf = t & 1;
+            ok = mbar_wait_warp(&d_full[buf], (t >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
+            if (!ok) break;
+            fence_after_sync();
+            const uint32_t orow = (uint32_t)(c + t * p.ctas_per_split) * TILE_R + row;
+            for (int g = 0; g < p.n_groups; ++g) {
+                float v0[16], v1[16], v2[16];
+                tmem_ld16(lane_base + 256 * buf + 64 * g, v0);
+                tmem_ld16(lane_base + 256 * buf + 64 * g + 16, v1);
+                tmem_ld16(lane_base + 256 * buf + 64 * g + 32, v2);
+                wait_ld();
+                if (g == p.n_groups - 1) {
+                    fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&d_empty[buf]);
+                }
+                auto col = [&](int i) { return i < 16 ? v0[i] : i < 32 ? v1[i - 16] : v2[i - 32]; };
+                if (orow < p.n_out) {
+                    float* dst = p.out + ((uint64_t)sp * TSG_GROUPS + g) * MAX_ROWS * p.ld_out + orow;
+#pragma unroll
+                    for (int tok = 0; tok < MAX_ROWS; ++tok)
+                        dst[(uint64_t)tok * p.ld_out] = ((col(3 * tok) + col(3 * tok + 1)) + col(3 * tok + 2)) * tok_scale[g * MAX_ROWS + tok];
+                }
+            }
+        }
+        if (!ok) abort_flag = 1;
+    }
+
+    fence_before_sync();
+    __syncthreads();
+    if (abort_flag && threadIdx.x == 0) {
+        for (int s = 0; s < TSG_STAGES; ++s) {
+            uint32_t spins = 0;
+            while (!mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1) && ++spins < (1u << 16)) __nanosleep(100);
+        }
+    }
+    __syncthreads();
+    if (warp == 1) {
+        fence_after_sync();
+        tmem_free(tmem, 512);
+    }
+}
+
 }  // namespace ts
 
 int gemm_tsb_choose_splits_multi(const int* row_tiles, int n_mats, int kblocks) {
@@ -305,6 +470,28 @@ dfl_status launch_gemm_tsb(cudaStream_t st, const QMatrix& m, const uint8_t* act
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     DFL_CUDA(cudaLaunchKernelEx(&cfg, ts::gemm_tsb_kernel, p));
+    count_launch();
+    return DFL_OK;
+}
+
+// n_groups (1 .. 4) groups of sixteen rows: acts [group][kblocks] chunks, sumsq [group][n_sumsq][16], out [splits][4 * 16][ld_out]
+dfl_status launch_gemm_tsb_groups(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, int n_groups,
+                                  const GemmEpilogue& ep, int* dev_err, uint32_t ld_out) {
+    if (m.layout != LAYOUT_TS || m.dtype != DFL_BF16) return fail(DFL_ERR_UNSUPPORTED, "grouped gemm: bf16 matrices only");
+    if (splits < 1 || splits > m.kblocks || n_groups < 1 || n_groups > ts::TSG_GROUPS) return fail(DFL_ERR_BAD_ARG, "grouped gemm: shape");
+    ts::ParamsB p;
+    p.w = m.tiles; p.acts = acts; p.out = out;
+    p.sumsq = ep.sumsq; p.n_sumsq = ep.n_sumsq; p.norm_k = ep.norm_k; p.eps = ep.eps; p.out_scale = ep.out_scale;
+    p.kblocks = m.kblocks; p.splits = splits; p.row_tiles = m.row_tiles; p.n_groups = n_groups;
+    int cps = sm_count() / splits;
+    if (cps < 1) cps = 1;
+    if (cps > m.row_tiles) cps = m.row_tiles;
+    p.ctas_per_split = cps;
+    p.n_out = (uint32_t)m.n_out;
+    p.ld_out = ld_out ? ld_out : (uint32_t)m.n_out;
+    p.err = dev_err;
+    DFL_CUDA(cudaFuncSetAttribute(ts::gemm_tsb_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ts::tsg_smem_bytes()));
+    DFL_CUDA(launch_k(ts::gemm_tsb_groups_kernel, dim3((unsigned)(cps * splits)), dim3(TSB_THREADS), (size_t)ts::tsg_smem_bytes(), st, p));
     count_launch();
     return DFL_OK;
 }

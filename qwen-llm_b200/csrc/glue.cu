@@ -38,6 +38,27 @@ dfl_status launch_glue(cudaStream_t st, const GlueParams& p, uint64_t k) {
     return DFL_OK;
 }
 
+__global__ void __launch_bounds__(128) glue_groups_kernel(GlueParams p) {
+    const int quad = threadIdx.x & 15, g = blockIdx.z;
+    const float4 w = p.mul_w ? *reinterpret_cast<const float4*>(p.mul_w + blockIdx.x * GLUE_COLS + quad * 4) : make_float4(1.f, 1.f, 1.f, 1.f);
+    pdl_prologue();
+    p.n_rows -= g * MAX_ROWS;
+    if (p.x) p.x += (uint64_t)g * MAX_ROWS * p.ld_x;
+    if (p.part) p.part += (uint64_t)g * MAX_ROWS * p.ld_part;
+    if (p.acts) p.acts += (uint64_t)g * (gridDim.x * GLUE_COLS / TILE_K) * act_chunk_dev(p.bf3);
+    if (p.sumsq) p.sumsq += (uint64_t)g * gridDim.x * MAX_ROWS;
+    glue_quad(p, p.splits, blockIdx.x, blockIdx.y * 8 + (threadIdx.x >> 4), quad, w);
+}
+
+dfl_status launch_glue_groups(cudaStream_t st, const GlueParams& p, uint64_t k) {
+    if (k == 0 || k % TILE_K || p.n_rows < 1) return fail(DFL_ERR_BAD_SHAPE, "glue groups: shape");
+    if (p.splits_dev || p.xn || p.capture || p.route_w) return fail(DFL_ERR_UNSUPPORTED, "glue groups: option");
+    launch_k(glue_groups_kernel, dim3((unsigned)(k / GLUE_COLS), MAX_ROWS / 8, (unsigned)((p.n_rows + MAX_ROWS - 1) / MAX_ROWS)), dim3(128), 0, st, p);
+    count_launch();
+    DFL_CUDA(cudaGetLastError());
+    return DFL_OK;
+}
+
 // ---- embedding rows ---------------------------------------------------------------
 __device__ __forceinline__ void embed_one(int dtype, const uint8_t* __restrict__ ggml, uint64_t h, int32_t token, float* row) {
     const uint64_t col = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -80,6 +80,7 @@ struct GlueParams {
     int splits = 0;
     const int32_t* splits_dev = nullptr;   // optional: *splits_dev more slices follow the first `splits` (a device-chosen count)
     int ld_part = 0;
+    int part_rows = MAX_ROWS;     // rows of one slice of part
     float* x = nullptr;           // [16][ld_x]
     int ld_x = 0;
     const float* mul_w = nullptr; // per-column multiplier (a folded RMSNorm weight)
@@ -119,7 +120,7 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
             if (w != 0.f) {
                 float g[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
                 const float* base = p.part + (uint64_t)tok * p.ld_part + col0;
-                const uint64_t stride = (uint64_t)MAX_ROWS * p.ld_part;
+                const uint64_t stride = (uint64_t)p.part_rows * p.ld_part;
 #pragma unroll 4
                 for (int s = 0; s < n_splits; ++s) {
                     const float4 a = __ldcg(reinterpret_cast<const float4*>(base + s * stride));
@@ -141,7 +142,7 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
                 // sum the split-K partials first (fixed order), then add to the residual
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
                 const float* base = p.part + (uint64_t)tok * p.ld_part + col0;
-                const uint64_t stride = (uint64_t)MAX_ROWS * p.ld_part;
+                const uint64_t stride = (uint64_t)p.part_rows * p.ld_part;
 #pragma unroll 4
                 for (int s = 0; s < n_splits; ++s) {
                     const float4 a = __ldcg(reinterpret_cast<const float4*>(base + s * stride));
@@ -186,6 +187,9 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
 #endif
 // k = number of columns (multiple of 256)
 dfl_status launch_glue(cudaStream_t st, const GlueParams& p, uint64_t k);
+// the same for p.n_rows > 16 rows in groups of sixteen: group g's x, part and acts start 16 g rows (acts: g * k / 256 chunks) further,
+// its sums of squares g * k / GLUE_COLS * 16
+dfl_status launch_glue_groups(cudaStream_t st, const GlueParams& p, uint64_t k);
 // Softmax + top-k routing of n_rows tokens over n_expert experts; logits[tok][n_expert] is the extra router row of
 // the shared expert's gate.  Writes route_w[16][n_expert] (zeros for experts not chosen), shared_gate[16],
 // route_idx[16][n_used].
