@@ -195,14 +195,17 @@ __global__ void __launch_bounds__(256) attn_chunk_kernel(AttnGeom g, const float
 }
 
 // ---- combine + sigmoid gate + activation packing ---------------------------------------------
-// grid (n_q, n_rows), block 32: one warp per (row, q head); lane owns hd/32 consecutive dims.
+// grid (n_q / 4, n_rows), block 128: one warp per (row, q head), four heads a CTA (one-warp CTAs, 16 384 of them for a prompt pass of
+// 512 rows, were bound by their launch: 21 us); lane owns hd/32 consecutive dims.
+constexpr int POST_HEADS = 4;
 template <int HD>
-__global__ void __launch_bounds__(32) attn_post_kernel(AttnGeom g, const float* partials, int pos_per_span, int recs_per_span,
+__global__ void __launch_bounds__(32 * POST_HEADS) attn_post_kernel(AttnGeom g, const float* partials, int pos_per_span, int recs_per_span,
                                                        const float* gate, uint32_t start, uint8_t* acts, int bf3,
                                                        float* out_f32, int* err, int n_spans) {
     pdl_prologue();
     constexpr int PER = HD / 32;  // 4 or 8
-    const int qh = blockIdx.x, row = blockIdx.y, lane = threadIdx.x;
+    const int qh = blockIdx.x * POST_HEADS + (threadIdx.x >> 5), row = blockIdx.y, lane = threadIdx.x & 31;
+    if (qh >= g.n_q) return;
     const int group = g.n_q / g.n_kv, kvh = qh / group, qi = (row % MAX_ROWS) * group + qh % group;
     partials += (uint64_t)(row / MAX_ROWS) * n_spans * recs_per_span * g.n_kv * (MAX_ROWS * group) * (HD + 2);   // the row's 16-row block
     // records holding visible positions: one per 64-position chunk (scalar kernel), one per span of chunks (mma.sync
@@ -351,8 +354,9 @@ dfl_status launch_attn_verify(cudaStream_t st, const AttnGeom& g, const float* q
         DFL_CHECK(launch_acts_clear(st, acts, (uint64_t)g.n_q * g.hd / TILE_K * (uint64_t)act_chunk_bytes(bf3)));
     }
     (void)n_chunks;
-    if (g.hd == 128) launch_k(attn_post_kernel<128>, dim3(dim3((unsigned)g.n_q, (unsigned)n_rows)), dim3(32), 0, st, g, partials, pos_per_span, recs_per_span, gate, start, acts, bf3, out_f32, err, 0);
-    else launch_k(attn_post_kernel<256>, dim3(dim3((unsigned)g.n_q, (unsigned)n_rows)), dim3(32), 0, st, g, partials, pos_per_span, recs_per_span, gate, start, acts, bf3, out_f32, err, 0);
+    const dim3 post_grid((unsigned)((g.n_q + POST_HEADS - 1) / POST_HEADS), (unsigned)n_rows);
+    if (g.hd == 128) launch_k(attn_post_kernel<128>, post_grid, dim3(32 * POST_HEADS), 0, st, g, partials, pos_per_span, recs_per_span, gate, start, acts, bf3, out_f32, err, 0);
+    else launch_k(attn_post_kernel<256>, post_grid, dim3(32 * POST_HEADS), 0, st, g, partials, pos_per_span, recs_per_span, gate, start, acts, bf3, out_f32, err, 0);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;
@@ -504,7 +508,7 @@ dfl_status launch_attn_rows(cudaStream_t st, const AttnGeom& g, const float* q_r
     else s = kv_f16 ? launch_rows<__half, 256>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials)
                     : launch_rows<float, 256>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials);
     DFL_CHECK(s);
-    launch_k(g.hd == 128 ? attn_post_kernel<128> : attn_post_kernel<256>, dim3((unsigned)g.n_q, (unsigned)n_rows), dim3(32), 0, st, g, partials, 1 << 30,
+    launch_k(g.hd == 128 ? attn_post_kernel<128> : attn_post_kernel<256>, dim3((unsigned)((g.n_q + POST_HEADS - 1) / POST_HEADS), (unsigned)n_rows), dim3(32 * POST_HEADS), 0, st, g, partials, 1 << 30,
              tiled ? 2 : 1, gate, start, nullptr, 0, out_f32, err, 1);
     count_launch();
     DFL_CUDA(cudaGetLastError());

@@ -11,7 +11,10 @@ namespace cg = cooperative_groups;
 
 // Threads of the packing kernels: CTA = 8 tokens x one 256-column block; lane = (token lane & 7, core lane >> 3), a warp covers
 // the 32 columns of one sub-block, so reads are 128-byte runs of a token's row and stores 128-byte runs of a k-core.
-__global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
+// The modes are compiled apart: in one body they took 72 registers, three CTAs an SM (512 rows: 14.6 -> 14.0 us a residual
+// step, 23.9 -> 19.6 a SwiGLU, cold).
+template <bool SWIGLU>
+__global__ void __launch_bounds__(256, SWIGLU ? 4 : 6) tm_glue_kernel(const TmGlue p) {
     pdl_prologue();
     __shared__ float ss_s[8][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -33,7 +36,7 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
     if (live) {
         const uint64_t stride = (uint64_t)p.rows_pad * p.ld_part;
         const float* base = p.part ? p.part + (uint64_t)row * p.ld_part + col : nullptr;
-        if (p.mode == GLUE_SWIGLU) {
+        if (SWIGLU) {
             float g[8] = {}, u[8] = {};
             for (int s = 0; s < p.splits; ++s) {
                 add8(g, base + s * stride);
@@ -57,9 +60,9 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
                 if (p.part) store8(p.x + (uint64_t)row * p.ld_x + col, v);
             }
         }
-        if (p.capture) store8(p.capture + (uint64_t)row * p.ld_capture + col, v);
+        if (!SWIGLU && p.capture) store8(p.capture + (uint64_t)row * p.ld_capture + col, v);
     }
-    if (p.sumsq) {
+    if (!SWIGLU && p.sumsq) {
         float ss = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
@@ -74,7 +77,7 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
             p.sumsq[(uint64_t)blockIdx.x * p.rows_pad + blockIdx.y * 8 + threadIdx.x] = t;
         }
     }
-    if (p.mul_w) {
+    if (!SWIGLU && p.mul_w) {
         float w[8] = {};
         add8(w, p.mul_w + col);
 #pragma unroll
@@ -82,7 +85,7 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= p.pre_scale;
-    if (p.xn && live) store8(p.xn + (uint64_t)row * p.ld_xn + col, v);
+    if (!SWIGLU && p.xn && live) store8(p.xn + (uint64_t)row * p.ld_xn + col, v);
     if (p.acts) {
         uint8_t* chunk = p.acts + ((uint64_t)(row / p.tile_tok) * gridDim.x + blockIdx.x) * tm_chunk(p.tile_tok);
         bool over = false;
@@ -97,7 +100,7 @@ __global__ void __launch_bounds__(256) tm_glue_kernel(const TmGlue p) {
 
 dfl_status launch_tm_glue(cudaStream_t st, const TmGlue& p, uint64_t k) {
     if (k == 0 || k % TILE_K || p.rows_pad % p.tile_tok) return fail(DFL_ERR_BAD_SHAPE, "tm_glue: shape");
-    launch_k(tm_glue_kernel, dim3((unsigned)(k / TILE_K), (unsigned)(p.rows_pad / 8)), dim3(256), 0, st, p);
+    launch_k(p.mode == GLUE_SWIGLU ? tm_glue_kernel<true> : tm_glue_kernel<false>, dim3((unsigned)(k / TILE_K), (unsigned)(p.rows_pad / 8)), dim3(256), 0, st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;
