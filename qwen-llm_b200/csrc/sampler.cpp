@@ -101,7 +101,8 @@ bool keys_from_order(const float* logits, uint64_t n, const uint32_t* order, uin
 
 // Orders candidate keys: whole row when top-k is off, else the top_k best.  Returns count or error.
 SErr order_keys(const float* logits, uint64_t n, uint64_t top_k, Buffers& b, uint64_t* count, uint64_t* nan_token,
-                const uint32_t* order = nullptr, bool* order_used = nullptr) {
+                const uint32_t* order = nullptr, bool* order_used = nullptr, const std::atomic<bool>* stop = nullptr) {
+    auto stopped = [&] { return stop && stop->load(std::memory_order_relaxed); };   // nobody wants the result any more: any will do
     if (n == 0) return S_EMPTY;
     if (n > 0x7fffffffull) return S_TOO_LARGE;
     const bool full = top_k == 0 || top_k >= n;
@@ -136,6 +137,7 @@ SErr order_keys(const float* logits, uint64_t n, uint64_t top_k, Buffers& b, uin
                 const int shift = 32 + 8 * digit;
                 uint32_t* h = hist[digit];
                 if (h[(b.keys[0] >> shift) & 255] == n) continue;   // every key has the same byte here
+                if (stopped()) break;
                 uint32_t off = 0;
                 for (int i = 0; i < 256; ++i) { const uint32_t c = h[i]; h[i] = off; off += c; }
                 const uint64_t* src = b.keys.data();
@@ -418,6 +420,7 @@ struct dfl_sampler {
         threads.work.notify_all();
         for (auto& t : threads.th) t.join();
     }
+    bool nucleus_path() const { return cfg.top_k == 0 && !(cfg.min_p > 0.0f) && cfg.top_p < 1.0f; }
     void build_row(uint32_t r) {
         Prepared& p = prepared[r];
         p.err = distribution(p.logits, block_vocab, p.dist, &p.nan_token, p.buf, &threads.stop);
@@ -495,7 +498,9 @@ struct dfl_sampler {
             taken = r < threads.next;
             if (!taken) threads.next = r + 1;
         }
-        if (r >= 4) allow_rows(r + 8);
+        // Where rows take the nucleus path they are cheap and stop quickly, so the limit keeps ahead of the loop; the ordered path's rows,
+        // milliseconds each, are only added when the loop has used up those it has.
+        if (nucleus_path() ? r >= 4 : r >= 6) allow_rows(nucleus_path() ? r + 8 : (r + 4) / 10 * 10 + 6);
         if (!taken) build_row(r);
         while (!p.done.load(std::memory_order_acquire)) std::this_thread::yield();
         *e = p.err;
@@ -520,7 +525,7 @@ struct dfl_sampler {
     // `stop` (optional): return at the next step with nothing of use.
     bool nucleus(const float* logits, uint64_t n, Dist& d, Buffers& buf, const std::atomic<bool>* stop) const {
         auto stopped = [&] { return stop && stop->load(std::memory_order_relaxed); };
-        if (cfg.top_k != 0 || cfg.min_p > 0.0f || !(cfg.top_p < 1.0f) || n < 1024 || n > 0x7fffffffull) return false;
+        if (!nucleus_path() || n < 1024 || n > 0x7fffffffull) return false;
         float mx;
         if (!max_of(logits, n, &mx) || !std::isfinite(mx)) return false;
         const double t = (double)cfg.temperature, inv_t = 1.0 / t, max_logit = (double)mx / t;
@@ -577,7 +582,7 @@ struct dfl_sampler {
         if (!order_for(logits, n) && nucleus(logits, n, d, buf, stop)) return S_OK;
         uint64_t len = 0;
         bool order_used = false;
-        SErr e = order_keys(logits, n, cfg.top_k, buf, &len, nan_token, order_for(logits, n), &order_used);
+        SErr e = order_keys(logits, n, cfg.top_k, buf, &len, nan_token, order_for(logits, n), &order_used, stop);
         if (order_used) ord_used.fetch_add(1, std::memory_order_relaxed);
         if (e != S_OK) return e;
         const uint64_t* keys = buf.keys.data();
@@ -608,9 +613,13 @@ struct dfl_sampler {
             bool finite = true;
             double* w = d.weights.data();
             for (uint64_t i = 0; i < len; ++i) w[i] = key_logit(keys[i]) / t - max_logit;   // vectorisable part first
-            for (uint64_t i = 0; i < len; ++i) {
-                w[i] = std::exp(w[i]);
-                finite &= std::isfinite(w[i]);
+            for (uint64_t first = 0; first < len; first += 8192) {
+                if (stop && stop->load(std::memory_order_relaxed)) return S_OK;
+                const uint64_t last = std::min<uint64_t>(len, first + 8192);
+                for (uint64_t i = first; i < last; ++i) {
+                    w[i] = std::exp(w[i]);
+                    finite &= std::isfinite(w[i]);
+                }
             }
             if (!finite) return S_NO_CANDIDATES;
         }
