@@ -341,8 +341,9 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
     ok = ok && cudaMalloc(&p->acts1, acts_bytes_for(w1->m)) == cudaSuccess;
     ok = ok && cudaMalloc(&p->acts2, acts_bytes_for(head->m)) == cudaSuccess;
     ok = ok && cudaEventCreate(&p->e0) == cudaSuccess && cudaEventCreate(&p->e1) == cudaSuccess;
-    ok = ok && (p->out = (dfl_c1::HostOut*)pool_alloc_host(sizeof(dfl_c1::HostOut)));
-    ok = ok && (p->x_host = (float*)pool_alloc_host(MAX_ROWS * k1 * 4));
+    static_assert(sizeof(dfl_c1::HostOut) <= 256, "the rows follow 256 bytes further");
+    ok = ok && (p->out = (dfl_c1::HostOut*)pool_alloc_host(256 + MAX_ROWS * k1 * 4));   // one block: pinning costs a millisecond each time
+    if (ok) p->x_host = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p->out) + 256);
     if (!ok) {
         dfl_c1_destroy(p);
         return fail(DFL_ERR_OOM, std::string("c1_create: allocation failed: ") + cudaGetErrorString(cudaGetLastError()));
@@ -361,7 +362,6 @@ void dfl_c1_destroy(dfl_c1* p) {
     cudaSetDevice(p->w1->m.device);
     cudaFree(p->x); cudaFree(p->part1); cudaFree(p->part2); cudaFree(p->logits); cudaFree(p->acts1); cudaFree(p->acts2);
     pool_free(p->out);
-    pool_free(p->x_host);
     if (p->e0) cudaEventDestroy(p->e0);
     if (p->e1) cudaEventDestroy(p->e1);
     if (p->st) cudaStreamDestroy(p->st);
