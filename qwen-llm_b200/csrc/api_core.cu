@@ -333,7 +333,7 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
     p->splits1 = gemm_choose_splits(w1->m);
     p->splits2 = gemm_choose_splits(head->m);
     const uint64_t k1 = w1->m.n_in, n1 = w1->m.n_out, v = head->m.n_out;
-    bool ok = cudaStreamCreateWithFlags(&p->st, cudaStreamNonBlocking) == cudaSuccess;
+    bool ok = (p->st = pool_stream()) != nullptr;
     ok = ok && cudaMalloc(&p->x, MAX_ROWS * k1 * 4) == cudaSuccess;
     ok = ok && cudaMalloc(&p->part1, (size_t)p->splits1 * MAX_ROWS * n1 * 4) == cudaSuccess;
     ok = ok && cudaMalloc(&p->part2, (size_t)p->splits2 * MAX_ROWS * v * 4) == cudaSuccess;
@@ -364,7 +364,7 @@ void dfl_c1_destroy(dfl_c1* p) {
     pool_free(p->out);
     if (p->e0) cudaEventDestroy(p->e0);
     if (p->e1) cudaEventDestroy(p->e1);
-    if (p->st) cudaStreamDestroy(p->st);
+    pool_stream_free(p->st);
     delete p;
 }
 

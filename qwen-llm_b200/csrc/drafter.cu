@@ -433,7 +433,7 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
     for (auto& L : d->layers) { upd(L.qkv); upd(L.kv); upd(L.wo); upd(L.gate_up); upd(L.down); }
     if (d->target->lm_head.splits > 1) upd(d->target->lm_head);
     if (d->has_selector) upd(d->sel_hidden);
-    bool ok = cudaStreamCreateWithFlags(&ds->st, cudaStreamNonBlocking) == cudaSuccess;
+    bool ok = (ds->st = pool_stream()) != nullptr;
     // All buffers in one zeroed block: sizes first, then the pointers (some thirty allocations and memsets cost a request 0.15 ms).
     uint8_t* base = nullptr;
     size_t used = 0;
@@ -505,7 +505,7 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
     if (ok) *ds->err = 0;
     ok = ok && (ds->pinned_sel = (uint8_t*)pool_alloc_host(MAX_ROWS * 16 * 8 + (size_t)MAX_ROWS * c.selector_rank * 4));
     ok = ok && cudaEventCreate(&ds->ev0) == cudaSuccess && cudaEventCreate(&ds->ev1) == cudaSuccess;
-    ok = ok && cudaStreamCreateWithFlags(&ds->st_side, cudaStreamNonBlocking) == cudaSuccess;
+    ok = ok && (ds->st_side = pool_stream());
     for (uint32_t il = 0; il < c.n_layer; ++il) ok = ok && cudaEventCreateWithFlags(&ds->ev_ctx[il], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         std::string why = cudaGetErrorString(cudaGetLastError());
@@ -531,8 +531,8 @@ void dfl_dsession_destroy(dfl_dsession* ds) {
     if (ds->ev1) cudaEventDestroy(ds->ev1);
     for (auto& e : ds->ev_ctx)
         if (e) cudaEventDestroy(e);
-    if (ds->st_side) cudaStreamDestroy(ds->st_side);
-    if (ds->st) cudaStreamDestroy(ds->st);
+    pool_stream_free(ds->st_side);
+    pool_stream_free(ds->st);
     delete ds;
 }
 

@@ -684,7 +684,7 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
     const size_t kv_bytes = kv_elems * (s->kv_f16 ? 2 : 4);
     const size_t conv_bytes = (size_t)3 * m->gdn_geom().conv_dim() * 4;
     const size_t ssm_bytes = (size_t)a.gdn_n_v_heads * 128 * 128 * 4;
-    bool ok = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) == cudaSuccess;
+    bool ok = (s->st = pool_stream()) != nullptr;
     for (int i = 0; i < m->n_attn && ok; ++i) {
         void *k = nullptr, *v = nullptr;
         ok = (k = pool_alloc(kv_bytes)) && (v = pool_alloc(kv_bytes));
@@ -710,7 +710,7 @@ dfl_status dfl_session_create(const dfl_model* m, uint32_t kv_capacity, int32_t 
     if (ok && m->n_attn) ok = (s->attn_partials = (float*)pool_alloc(attn_partials_floats(m->attn_geom(), (uint32_t)cap_alloc) * 4)) != nullptr;   // two records per 128-position tile in tiled storage
     ok = ok && (s->err = (int*)pool_alloc_host(4));
     ok = ok && cudaEventCreate(&s->ev0) == cudaSuccess && cudaEventCreate(&s->ev1) == cudaSuccess;
-    ok = ok && cudaStreamCreateWithFlags(&s->st_side, cudaStreamNonBlocking) == cudaSuccess;
+    ok = ok && (s->st_side = pool_stream());
     ok = ok && cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&s->ev_watch, cudaEventDisableTiming) == cudaSuccess;
@@ -740,8 +740,8 @@ void dfl_session_destroy(dfl_session* s) {
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
     if (s->ev_join) cudaEventDestroy(s->ev_join);
     if (s->ev_watch) cudaEventDestroy(s->ev_watch);
-    if (s->st_side) cudaStreamDestroy(s->st_side);
-    if (s->st) cudaStreamDestroy(s->st);
+    pool_stream_free(s->st_side);
+    pool_stream_free(s->st);
     delete s;
 }
 

@@ -26,6 +26,9 @@ void* pool_alloc(size_t bytes);
 void* pool_alloc_host(size_t bytes);
 void pool_free(void* p);
 void pool_trim(int device);
+// a non-blocking stream of the current device; given back (after its work) it waits for the next session
+cudaStream_t pool_stream();
+void pool_stream_free(cudaStream_t st);
 // The uploads in order on `st`, each followed by what `after` queues behind it; returns when all of it is done.
 struct Upload {
     void* dst;

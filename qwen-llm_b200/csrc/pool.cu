@@ -15,6 +15,7 @@ namespace dfl {
 
 namespace {
 constexpr size_t kPoolBytes = 8ull << 30, kPoolHostBytes = 256ull << 20;
+constexpr size_t kPoolStreams = 64;
 constexpr int HOST = -1;   // "device" of pinned host blocks
 
 struct Pool {
@@ -22,6 +23,7 @@ struct Pool {
     std::mutex mu;
     std::multimap<std::pair<int, size_t>, void*> idle;
     std::map<int, size_t> idle_bytes;
+    std::map<int, std::vector<cudaStream_t>> streams;
     std::unordered_map<void*, Block> live;
     std::unordered_map<void*, size_t> lent;   // host blocks in callers' hands (dfl_host_alloc)
     size_t lent_bytes = 0;
@@ -42,6 +44,8 @@ struct Pool {
             it = idle.erase(it);
         }
         idle_bytes[device] = 0;
+        for (cudaStream_t st : streams[device]) cudaStreamDestroy(st);
+        streams[device].clear();
     }
     void* take(int device, size_t bytes) {
         bytes = (bytes + 511) / 512 * 512;
@@ -102,6 +106,35 @@ void* pool_alloc(size_t bytes) {
 }
 void* pool_alloc_host(size_t bytes) { return pool().take(HOST, bytes); }
 void pool_free(void* p) { pool().give(p); }
+// Streams the same way: making and dropping the four of a request costs 0.25 ms.  At most kPoolStreams idle ones a device.
+cudaStream_t pool_stream() {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return nullptr;
+    {
+        std::lock_guard<std::mutex> lock(pool().mu);
+        auto& idle = pool().streams[device];
+        if (!idle.empty()) {
+            cudaStream_t st = idle.back();
+            idle.pop_back();
+            return st;
+        }
+    }
+    cudaStream_t st = nullptr;
+    return cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess ? st : nullptr;
+}
+void pool_stream_free(cudaStream_t st) {
+    if (!st) return;
+    int device = 0;
+    if (cudaStreamSynchronize(st) == cudaSuccess && cudaGetDevice(&device) == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(pool().mu);
+        auto& idle = pool().streams[device];
+        if (idle.size() < kPoolStreams) {
+            idle.push_back(st);
+            return;
+        }
+    }
+    cudaStreamDestroy(st);
+}
 void pool_trim(int device) { pool().trim(device); pool().trim(HOST); }
 
 }  // namespace dfl
