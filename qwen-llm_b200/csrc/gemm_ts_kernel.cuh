@@ -55,6 +55,24 @@ constexpr int smem_bytes() {
 // named barrier among the draining warps only (every one of them reaches it unconditionally)
 __device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
+// Whether the MMA warp of entry e (group e & 1, column block e % n_kb) waits for the block's activations: at its own first use of
+// the block.  With an even count a group meets the same blocks in every row tile; with an odd one its second tile brings the blocks that
+// only the other group has waited for (one block and two tiles: group 1's first entry).  The barrier has one phase, so a wait
+// that is not needed costs a test.
+__host__ __device__ constexpr bool waits_for_acts(int e, int n_kb) { return e < ((n_kb & 1) ? 2 * n_kb : n_kb); }
+constexpr bool every_first_use_waits() {
+    for (int n_kb = 1; n_kb <= KC; ++n_kb)
+        for (int g = 0; g < 2; ++g)
+            for (int kb = 0; kb < n_kb; ++kb)
+                for (int e = g; e < 4 * n_kb; e += 2)   // the group's entries in order, four row tiles
+                    if (e % n_kb == kb) {
+                        if (!waits_for_acts(e, n_kb)) return false;
+                        break;
+                    }
+    return true;
+}
+static_assert(every_first_use_waits(), "an MMA warp would read activations that may not have arrived");
+
 // The side projection: this CTA's four outputs over all rows.  24 warps; the even ones take tokens 0 - 7, the odd ones 8 - 15,
 // a thread four columns of every 12 x 128.  Sums over lanes, then warps, in a fixed order.
 __device__ __forceinline__ void side_projection(const Params& p, float* smem) {
@@ -233,11 +251,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
         const int kb_step = 2 % n_kb;
         for (int e = (int)g; e < n_it && ok; e += 2) {
             const uint32_t chunk = acts_addr + (uint32_t)kb_e * ACTTS_CHUNK;
+            if (waits_for_acts(e, n_kb)) ok = mbar_wait_warp(&acts_bar[kb_e], 0, p.err, DEV_ERR_WAIT_FULL);
             kb_e += kb_step;
             if (kb_e >= n_kb) kb_e -= n_kb;
-            if (e < n_kb) {   // first row tile: the column block's activations may still be in flight
-                ok = mbar_wait_warp(&acts_bar[e], 0, p.err, DEV_ERR_WAIT_FULL);
-            }
             if (ok && e >= 2) {   // the group's accumulator was last used by entry e - 2
                 ok = mbar_wait_warp(&d_free[g], (((uint32_t)e >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
             }

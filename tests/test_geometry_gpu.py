@@ -244,3 +244,29 @@ def test_a_repeated_verify_from_the_same_state_gives_the_same_bits(moe):
         assert got == first
         pkg.restore_pre_block(gm, sess, scr, pos)
     sess.close(); scr.close(); gm.close()
+
+
+def test_a_token_of_the_routed_model_gives_the_same_bits_and_the_block_s_logits():
+    """One token chooses eight experts: sixteen column blocks in ten splits, so that some CTAs of the down projection hold one
+    block and two row tiles and each of their MMA warps starts on the same activations."""
+    arch = _slice_arch(syn.arch_35b_a3b(), 4, 4)
+    arch.vocab_size = 8192
+    ents = syn.target_entries(arch, seed=47, device=0)
+    gm = syn.build_model(arch, ents)
+    syn.free_entries(ents)
+    sess, scr = pkg.Session(gm, 256, True), pkg.Scratch(gm, 16, 1)
+    rng = np.random.default_rng(6)
+    pkg.packed_verify(gm, sess, scr, [3], rng.integers(0, arch.vocab_size, size=16), 0)
+    toks = rng.integers(0, arch.vocab_size, size=16)
+    block = pkg.packed_verify(gm, sess, scr, [3], toks, 16, want_logits=True)[2]
+    pkg.restore_pre_block(gm, sess, scr, 16)
+    first = None
+    for _ in range(40):
+        logits, _ = pkg.single_token(gm, sess, scr, [3], int(toks[0]), 16)
+        if first is None:
+            first = logits.copy()
+            # the splits follow the number of chosen experts, so the block's sums are in another order
+            np.testing.assert_allclose(first, block[0], rtol=RTOL, atol=ATOL)
+        assert logits.tobytes() == first.tobytes()
+        pkg.restore_pre_block(gm, sess, scr, 16)
+    sess.close(); scr.close(); gm.close()
