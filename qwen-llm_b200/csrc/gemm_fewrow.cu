@@ -871,8 +871,9 @@ constexpr int ARGMAX_CLUSTER = 8, ARGMAX_THREADS = 1024;
 template <bool REDUCE>
 __global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(ARGMAX_THREADS)
 argmax_kernel(const float* src, uint64_t ld_src, int splits, uint64_t vocab, float* logits, uint64_t ld, int32_t* argmax, float* gap) {
-    pdl_prologue();
     cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_arrive();   // matched by the wait before the write into the first CTA's shared memory
+    pdl_prologue();
     __shared__ Top2 best[ARGMAX_CLUSTER];
     constexpr int ARGMAX_BATCH = REDUCE ? 4 : 8;
     const int row = blockIdx.y;
@@ -912,6 +913,7 @@ argmax_kernel(const float* src, uint64_t ld_src, int splits, uint64_t vocab, flo
         }
     }
     a = top2_block_reduce(a);
+    cluster.barrier_wait();   // the first CTA has started: its shared memory may be written (a CTA without columns is here at once)
     if (threadIdx.x == 0) *cluster.map_shared_rank(&best[blockIdx.x], 0) = a;
     cluster.sync();
     if (blockIdx.x != 0 || threadIdx.x != 0) return;

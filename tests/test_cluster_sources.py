@@ -1,0 +1,37 @@
+"""Shared memory of another CTA of a cluster may only be touched once that CTA is known to have started: every kernel that maps it
+passes a cluster barrier first.  A missing barrier shows on no GPU that starts a cluster's CTAs together, so the sources are read."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "qwen-llm_b200", "csrc")
+
+
+def kernels():
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__[^;{]*?\b(\w+_kernel)\s*\([^;{]*\)\s*\{", text):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[i], 0)
+                i += 1
+            body = text[m.end():i]
+            if "map_shared_rank" in body:
+                yield os.path.basename(path), m.group(1), body
+
+
+CASES = list(kernels())
+
+
+def test_the_kernels_are_found():
+    assert {"argmax_kernel", "gdn_mix_kernel", "tm_small_matmul_kernel"} <= {name for _, name, _ in CASES}
+
+
+@pytest.mark.parametrize("file,name,body", CASES, ids=[c[1] for c in CASES])
+def test_a_cluster_barrier_comes_before_remote_shared_memory(file, name, body):
+    before = body[:body.index("map_shared_rank")]
+    assert "cluster.sync()" in before or ("cluster.barrier_arrive()" in before and "cluster.barrier_wait()" in before), file
+    # and one behind the last use, so that no CTA leaves while its shared memory is used
+    assert "cluster.sync()" in body[body.rindex("map_shared_rank"):], file
