@@ -50,6 +50,12 @@ dfl_status dfl_prefill(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
         if (layer_ids[k] >= m->arch.n_layer) return fail(DFL_ERR_BAD_SHAPE, "prefill: capture layer id out of range");
     // the drafter consumes every slot of a captured row: a shorter id list would feed it slots no layer wrote
     if (feed_drafter && n_layer_ids != sc->k_layers) return fail(DFL_ERR_BAD_SHAPE, "prefill: feeding the drafter needs one capture layer per scratch slot");
+    if (feed_drafter) {   // before the first pass, whichever path it takes: the rows go to the drafter slot by slot
+        dfl_dsession_view dv;
+        dfl_dsession_view_get(feed_drafter, &dv);
+        if (dv.target != m) return fail(DFL_ERR_BAD_ARG, "prefill: the drafter session belongs to another model");
+        if (dv.n_target_layers != sc->k_layers) return fail(DFL_ERR_BAD_SHAPE, "prefill: scratch capture layer count differs from the drafter's");
+    }
     for (uint64_t i = 0; i < n; ++i)
         if (ids[i] < 0 || (uint32_t)ids[i] >= m->arch.vocab_size) return fail(DFL_ERR_BAD_TOKEN, "prefill: token id out of range");
     const uint64_t KH = (uint64_t)sc->k_layers * m->arch.hidden_size;
@@ -74,7 +80,6 @@ dfl_status dfl_prefill(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
                             cudaMemcpyDeviceToHost, s->st);
         DFL_CHECK(session_drain(s));
         if (feed_drafter) {
-            if (dsession_target(feed_drafter) != m) return fail(DFL_ERR_BAD_ARG, "append_from_scratch: scratch belongs to another model");
             positions.resize(nb);
             for (uint32_t i = 0; i < nb; ++i) positions[i] = start + i;
             if (big) DFL_CHECK(dsession_append_dev(feed_drafter, capture, cudaMemcpyDeviceToDevice, positions.data(), nb));

@@ -113,3 +113,32 @@ def test_prompt_pass_at_tile_edges(n):
     syn.free_entries(ents)
     _check(arch, gm, n, 0, [0, 3])
     gm.close()
+
+
+@pytest.mark.parametrize("slots", [1, 3])
+@pytest.mark.parametrize("n", [8, 40])
+def test_feeding_a_drafter_of_another_slot_count_is_refused_before_the_first_pass(tiny, n, slots):
+    arch, gm = tiny
+    cfg = modelgen.tiny_dflash_config(arch)   # two tap layers
+    gd = pkg.Drafter(gm, cfg, modelgen.drafter_tensors(arch, cfg, seed=4))
+    sess, scr, ds = pkg.Session(gm, 64), pkg.Scratch(gm, 16, slots), pkg.DSession(gd, 64)
+    with pytest.raises(pkg.DflError) as e:
+        pkg.prefill(gm, sess, scr, [0, 1, 3][:slots], np.arange(n), 0, feed_drafter=ds)
+    assert e.value.name == "BAD_SHAPE"
+    assert sess.kv_n_pos == 0 and ds.ctx_len == 0 and not sess.poisoned
+    for x in (sess, scr, ds, gd):
+        x.close()
+
+
+@pytest.mark.parametrize("n", [8, 40])
+def test_feeding_a_drafter_of_another_model_is_refused_before_the_first_pass(tiny, n):
+    arch, gm = tiny
+    other = pkg.Model(arch, modelgen.target_tensors(arch, seed=9))
+    cfg = modelgen.tiny_dflash_config(arch)
+    gd = pkg.Drafter(other, cfg, modelgen.drafter_tensors(arch, cfg, seed=4))
+    sess, scr, ds = pkg.Session(gm, 64), pkg.Scratch(gm, 16, 2), pkg.DSession(gd, 64)
+    with pytest.raises(pkg.DflError) as e:
+        pkg.prefill(gm, sess, scr, [1, 3], np.arange(n), 0, feed_drafter=ds)
+    assert e.value.name == "BAD_ARG" and sess.kv_n_pos == 0 and ds.ctx_len == 0
+    for x in (sess, scr, ds, gd, other):
+        x.close()
