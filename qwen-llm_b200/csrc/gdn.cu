@@ -141,8 +141,8 @@ dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* sta
 //     its own 32 v channels.  The q and k shares travel to the other three CTAs through distributed shared memory together
 //     with their sums of squares, so that each CTA holds the full 16 x 128 q and k rows and normalises them itself;
 //   * recurrence: a warp owns 4 state rows (GdnRows); everything it reads is in shared memory.  State, filter taps and old conv
-//     rows are fetched before the dependency wait (earlier passes
-//     wrote them, and a pass begins with a host-to-device copy), the z rows are requested before the token loop;
+//     rows are fetched before the dependency wait (earlier passes or a rollback wrote them, and a pass begins with a plain
+//     launch, launch_embed_block, which waits for all of that), the z rows are requested before the token loop;
 //   * y = rmsnorm(o; eps * 128) * w * silu(z): every CTA writes its quarter's share of a token's sum of squares to all four,
 //     one cluster barrier, rank-ordered sum, then packs its 32 columns (one sub-block) of the output projection's activations.
 // A row's result does not depend on how many rows the block has.

@@ -72,8 +72,7 @@ __global__ void embed_rows_kernel(int dtype, const uint8_t* __restrict__ ggml, u
     pdl_prologue();
     embed_one(dtype, ggml, h, tokens[blockIdx.y], x + (uint64_t)blockIdx.y * ld);
 }
-// A block's tokens ride in the launch itself: the copy that used to carry 64 bytes to the device cost a pass 3 us and the overlap
-// of its first kernel with the end of the pass before.
+// A block's tokens ride in the launch itself: the copy that used to carry 64 bytes to the device cost a pass 3 us.
 struct BlockTokens { int32_t id[MAX_ROWS]; };
 __global__ void embed_block_kernel(int dtype, const uint8_t* __restrict__ ggml, uint64_t h, const BlockTokens tokens, float* x, int ld) {
     pdl_prologue();
@@ -95,7 +94,11 @@ dfl_status launch_embed_block(cudaStream_t st, int dtype, const uint8_t* ggml, u
     if (n_rows < 1 || n_rows > MAX_ROWS) return fail(DFL_ERR_BAD_SHAPE, "embed_block: 1 to 16 rows");
     BlockTokens t{};
     for (int i = 0; i < n_rows; ++i) t.id[i] = tokens_host[i];
-    launch_k(embed_block_kernel, dim3((unsigned)((h + 255) / 256), (unsigned)n_rows), dim3(256), 0, st, dtype, ggml, h, t, x, ld);
+    // A plain launch: it starts a pass, and what follows in the pass may read before its own dependency wait what a pass or a rollback
+    // before it wrote (gdn_mix_kernel: recurrent state and conv rows).  Early launches reach back any number of
+    // kernels as long as all of them fit the chip, so the chain is cut here; nothing is lost, the host has waited for the
+    // pass before in every caller but the outer loop's rollback.
+    embed_block_kernel<<<dim3((unsigned)((h + 255) / 256), (unsigned)n_rows), 256, 0, st>>>(dtype, ggml, h, t, x, ld);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

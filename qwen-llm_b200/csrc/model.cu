@@ -1018,7 +1018,8 @@ dfl_status dfl_session_probe_wait_timeout(const dfl_model* m, dfl_session* s, ui
 
 namespace dfl {
 // The launches of dfl_restore_partial without the wait: the outer loop lets them run under the next draft (the drafter
-// never reads the target's recurrent state) and the next verify follows them in stream order.
+// never reads the target's recurrent state).  The next verify follows them in stream order: its first launch is a plain one, so
+// that its early reads of the recurrent state lie behind them (launch_embed_block).
 dfl_status restore_partial_launch(const dfl_model* m, dfl_session* s, dfl_scratch* sc, uint32_t n_keep, uint32_t start_position) {
     DFL_CHECK(session_guard(m, s, "restore_partial"));
     if (!sc || sc->m != m || !sc->have_block) return fail(DFL_ERR_BAD_ARG, "restore_partial: scratch holds no verify block");

@@ -123,6 +123,23 @@ def test_replayed_drafts_accept_fully_and_partially(world):
     assert stats2.restore_calls >= 1
 
 
+def test_rollbacks_of_a_model_with_one_recurrent_layer_keep_the_greedy_stream():
+    # the shortest way from a rollback's kernels to the next pass's mixer: two launches for one recurrent layer
+    arch = modelgen.tiny_arch(n_layer=2, full_attention_interval=2)
+    gm = pkg.Model(arch, modelgen.target_tensors(arch, seed=3))
+    cfg = modelgen.tiny_dflash_config(arch, ids=[0, 1])
+    gd = pkg.Drafter(gm, cfg, modelgen.drafter_tensors(arch, cfg, seed=4))
+    prompt = np.random.default_rng(11).integers(0, arch.vocab_size, size=17)
+    plain = plain_decode(gm, prompt, 150, pkg.Sampler(), gd.layer_ids())
+    bad = plain.copy()
+    bad[3::4] = (bad[3::4] + 1) % arch.vocab_size   # a strict prefix in every step
+    for runs_drafter in (False, True):
+        spec, stats = dflash_decode((arch, cfg, None, gm, None, gd), prompt, 120, pkg.Sampler(), replay_history=bad, replay_unchecked=True,
+                                    replay_runs_drafter=runs_drafter)
+        assert np.array_equal(spec, plain[:120]) and stats.restore_calls >= 25
+    gd.close(); gm.close()
+
+
 def test_sampled_one_hot_coupling_keeps_the_serial_stream(world):
     arch, cfg, om, gm, od, gd = world
     prompt = np.random.default_rng(12).integers(0, arch.vocab_size, size=23)

@@ -1,5 +1,8 @@
-"""Shared memory of another CTA of a cluster may only be touched once that CTA is known to have started: every kernel that maps it
-passes a cluster barrier first.  A missing barrier shows on no GPU that starts a cluster's CTAs together, so the sources are read."""
+"""Orderings that no run shows to be missing, read from the sources.
+
+Shared memory of another CTA of a cluster may only be touched once that CTA is known to have started: every kernel that maps it
+passes a cluster barrier first.  A kernel that reads before its dependency wait what an earlier pass wrote needs a plain
+launch, which waits for everything, at the start of its own pass."""
 import glob
 import os
 import re
@@ -35,3 +38,14 @@ def test_a_cluster_barrier_comes_before_remote_shared_memory(file, name, body):
     assert "cluster.sync()" in before or ("cluster.barrier_arrive()" in before and "cluster.barrier_wait()" in before), file
     # and one behind the last use, so that no CTA leaves while its shared memory is used
     assert "cluster.sync()" in body[body.rindex("map_shared_rank"):], file
+
+
+def test_a_pass_starts_with_a_plain_launch():
+    glue = open(os.path.join(CSRC, "glue.cu")).read()
+    body = re.search(r"dfl_status launch_embed_block\(.*?\n}", glue, re.S).group(0)
+    assert "embed_block_kernel<<<" in body and "launch_k(" not in body
+    for path, fn in (("model.cu", "verify_core"), ("drafter.cu", "draft_core")):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, path)).read())
+        core = text[re.search(r"dfl_status " + fn + r"\([^;{]*\{", text).end():]
+        queued = re.findall(r"DFL_CHECK\((launch_\w+)\(", core)   # on the pass's own stream, in order
+        assert queued[0] == "launch_embed_block", path
