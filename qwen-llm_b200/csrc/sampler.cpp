@@ -6,10 +6,12 @@
 // (`decide_dflash_accept_prefix` :76-183).  Acceptance runs on the host in the reference too.
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <condition_variable>
 #include <deque>
+#include <pthread.h>
 #include <mutex>
 #include <system_error>
 #include <thread>
@@ -61,7 +63,7 @@ struct Xoshiro {
     double next_unit() { return (double)(next_u64() >> 11) / 9007199254740992.0; }
 };
 
-enum SErr { S_OK = 0, S_EMPTY, S_NAN, S_TOO_LARGE, S_NO_CANDIDATES, S_PROPOSAL_RANGE, S_PROPOSAL_WEIGHT, S_MISSING_PROPOSAL };
+enum SErr { S_OK = 0, S_EMPTY, S_NAN, S_TOO_LARGE, S_NO_CANDIDATES, S_MEMORY, S_PROPOSAL_RANGE, S_PROPOSAL_WEIGHT, S_MISSING_PROPOSAL };
 
 // ascending u32 order == descending f32 total order
 inline uint32_t descending_bits(float f) {
@@ -357,6 +359,130 @@ void sort_keys(std::vector<uint64_t>& keys, std::vector<uint64_t>& scratch, uint
     }
 }
 
+// ---- threads that build rows ahead ------------------------------------------------------------------------------
+// One crew for all samplers of the process.  A sampler offers the rows of the block it is deciding; a free thread takes the next row of a
+// block that may have one more helper.  At most as many threads as the host runs at once, started when a block
+// finds none idle; one that has had nothing to do for two seconds ends.  (Threads of each sampler's own: 32 samplers held 224
+// idle threads on eight cores, and a limit set after the first block came too late.)
+class Crew {
+public:
+    struct Block {   // guarded by the crew's mutex, except `stop`
+        uint32_t next = 0, limit = 0;        // rows [next, limit) may be taken
+        uint32_t running = 0, helpers = 0;   // threads at work on it, and the most there may be
+        std::condition_variable idle;
+        std::atomic<bool> stop{false};       // the block has been decided: rows still being built are not wanted any more
+        void* owner = nullptr;
+        void (*build)(void* owner, uint32_t row) = nullptr;   // must not throw
+    };
+    static Crew& get() {
+        static std::once_flag once;
+        std::call_once(once, [] {
+            instance() = new Crew();
+            pthread_atfork(nullptr, nullptr, [] { instance() = new Crew(); });   // a child has none of its parent's threads
+        });
+        return *instance();
+    }
+    void begin(Block& b) {
+        std::lock_guard<std::mutex> lock(mu);
+        b.next = b.limit = b.running = 0;
+        b.stop.store(false, std::memory_order_relaxed);
+        blocks.push_back(&b);
+    }
+    // rows before `limit` may be built ahead
+    void allow(Block& b, uint32_t limit) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (limit <= b.limit) return;
+        b.limit = limit;
+        const uint32_t wanted = std::min(b.helpers > b.running ? b.helpers - b.running : 0, b.limit > b.next ? b.limit - b.next : 0);
+        const uint32_t most = std::max(2u, std::thread::hardware_concurrency());
+        try {
+            for (; n_idle < wanted && threads.size() - ended.size() < most; ++n_idle) {
+                ended.reserve(threads.size() + 1);
+                threads.emplace_back([this] { main(); });
+            }
+        } catch (...) {   // no more threads to be had: the caller builds what they do not
+        }
+        for (const std::thread::id id : ended) {
+            auto it = std::find_if(threads.begin(), threads.end(), [&](const std::thread& t) { return t.get_id() == id; });
+            it->join();
+            threads.erase(it);
+        }
+        ended.clear();
+        for (uint32_t i = 0; i < wanted; ++i) work.notify_one();
+    }
+    // whether nobody has taken the row; it is the caller's then
+    bool claim(Block& b, uint32_t row) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (row < b.next) return false;
+        b.next = row + 1;
+        return true;
+    }
+    // when it returns no thread works on the block, and none will
+    void end(Block& b) {
+        b.stop.store(true, std::memory_order_relaxed);
+        std::unique_lock<std::mutex> lock(mu);
+        b.limit = 0;
+        blocks.erase(std::remove(blocks.begin(), blocks.end(), &b), blocks.end());
+        b.idle.wait(lock, [&] { return b.running == 0; });
+    }
+    // before the code of the threads goes away (process exit, library unloaded)
+    static void shut_down() {
+        Crew* c = instance();
+        if (!c) return;
+        std::vector<std::thread> all;
+        {
+            std::lock_guard<std::mutex> lock(c->mu);
+            c->quit = true;
+            all.swap(c->threads);
+            c->ended.clear();
+        }
+        c->work.notify_all();
+        for (std::thread& t : all) t.join();
+    }
+
+private:
+    static Crew*& instance() { static Crew* c = nullptr; return c; }   // never destroyed
+    Block* pick() {
+        for (size_t i = 0; i < blocks.size(); ++i) {
+            Block* b = blocks[i];
+            if (b->next >= b->limit || b->running >= b->helpers) continue;
+            std::rotate(blocks.begin(), blocks.begin() + (ptrdiff_t)i + 1, blocks.end());   // blocks take turns
+            return b;
+        }
+        return nullptr;
+    }
+    void main() {   // counted as idle by whoever started it
+        std::unique_lock<std::mutex> lock(mu);
+        for (bool rested = false;;) {
+            Block* b = quit ? nullptr : pick();
+            if (!b) {
+                if (quit || rested) break;
+                rested = work.wait_for(lock, std::chrono::seconds(2)) == std::cv_status::timeout;
+                continue;
+            }
+            rested = false;
+            const uint32_t row = b->next++;
+            ++b->running;
+            --n_idle;
+            lock.unlock();
+            b->build(b->owner, row);
+            lock.lock();
+            ++n_idle;
+            if (--b->running == 0) b->idle.notify_all();
+        }
+        --n_idle;
+        if (!quit) ended.push_back(std::this_thread::get_id());   // joined by the next block that asks for threads; the space is reserved
+    }
+    std::mutex mu;
+    std::condition_variable work;
+    std::vector<Block*> blocks;
+    std::vector<std::thread> threads;
+    std::vector<std::thread::id> ended;
+    uint32_t n_idle = 0;
+    bool quit = false;
+};
+__attribute__((destructor)) void crew_shut_down() { Crew::shut_down(); }
+
 struct Dist {
     std::vector<int32_t> tokens;
     std::vector<double> weights;
@@ -373,10 +499,10 @@ struct dfl_sampler {
     uint64_t draws = 0;
     Buffers buf;
     // Distributions of a block's rows built ahead of the sequential accept loop: building a row's distribution draws nothing from
-    // the generator, so only the picks have to stay in row order.  The sampler's threads take rows in order up to a
+    // the generator, so only the picks have to stay in row order.  The crew takes rows in order up to a
     // limit that moves with the loop (the first six cover a typical accepted prefix), so a block rejected early does
     // not pay for all of its rows; a row that no thread has taken yet when the loop reaches it is built by the loop's own
-    // thread, so nothing waits for a thread to wake.  The threads are kept with the sampler: starting five of them a
+    // thread, so nothing waits for a thread to wake.  The threads outlive the block: starting five of them a
     // block cost 0.2 - 0.3 ms, as much as the rows themselves when each has a clear favourite.
     struct Prepared {
         const float* logits = nullptr;
@@ -403,83 +529,39 @@ struct dfl_sampler {
     const float* block_logits = nullptr;
     uint64_t block_vocab = 0;
     uint32_t block_rows = 0;
-    struct Threads {
-        std::vector<std::thread> th;
-        std::mutex mu;
-        std::condition_variable work, idle;
-        uint32_t next = 0, limit = 0, running = 0;   // rows [next, limit) may be taken; guarded by mu, like quit
-        bool quit = false;
-        std::atomic<bool> stop{false};   // the block has been decided: rows still being built are not wanted any more
-    } threads;
+    Crew::Block ahead;
 
-    ~dfl_sampler() {
-        {
-            std::lock_guard<std::mutex> lock(threads.mu);
-            threads.quit = true;
-        }
-        threads.work.notify_all();
-        for (auto& t : threads.th) t.join();
-    }
     bool nucleus_path() const { return cfg.top_k == 0 && !(cfg.min_p > 0.0f) && cfg.top_p < 1.0f; }
     void build_row(uint32_t r) {
         Prepared& p = prepared[r];
-        p.err = distribution(p.logits, block_vocab, p.dist, &p.nan_token, p.buf, &threads.stop);
-        p.done.store(true, std::memory_order_release);
-    }
-    void thread_main() {
-        std::unique_lock<std::mutex> lock(threads.mu);
-        for (;;) {
-            threads.work.wait(lock, [&] { return threads.quit || threads.next < threads.limit; });
-            if (threads.quit) return;
-            const uint32_t r = threads.next++;
-            ++threads.running;
-            lock.unlock();
-            build_row(r);
-            lock.lock();
-            if (--threads.running == 0) threads.idle.notify_all();
-        }
-    }
-    // rows before `limit` may be built ahead
-    void allow_rows(uint32_t limit) {
-        limit = std::min(limit, block_rows);
-        const uint32_t wanted = std::min<uint32_t>(std::max(2u, worker_limit()) - 1, std::min(limit, 10u));
-        {
-            std::lock_guard<std::mutex> lock(threads.mu);
-            if (limit <= threads.limit) return;
-            threads.limit = limit;
-        }
         try {
-            while (threads.th.size() < wanted) threads.th.emplace_back([this] { thread_main(); });
-        } catch (const std::system_error&) {}   // no more threads to be had: the loop builds what they do not
-        threads.work.notify_all();
+            p.err = distribution(p.logits, block_vocab, p.dist, &p.nan_token, p.buf, &ahead.stop);
+        } catch (...) {   // on a thread of the crew nobody could catch it
+            p.err = S_MEMORY;
+        }
+        p.done.store(true, std::memory_order_release);
     }
     void prepare_rows(const float* logits, uint32_t n_rows, uint64_t vocab) {
         block_logits = nullptr;
         block_rows = 0;
         if (cfg.temperature == 0.0f || n_rows < 2 || vocab < 4096 || worker_limit() < 2) return;
-        block_logits = logits;
-        block_vocab = vocab;
-        block_rows = n_rows;
         while (prepared.size() < n_rows) prepared.emplace_back();
         for (uint32_t r = 0; r < n_rows; ++r) {
             prepared[r].logits = logits + (uint64_t)r * vocab;
             prepared[r].done.store(false, std::memory_order_relaxed);
         }
-        {
-            std::lock_guard<std::mutex> lock(threads.mu);
-            threads.next = threads.limit = 0;
-            threads.stop.store(false, std::memory_order_relaxed);
-        }
-        allow_rows(6);
+        ahead.owner = this;
+        ahead.build = [](void* self, uint32_t r) { static_cast<dfl_sampler*>(self)->build_row(r); };
+        ahead.helpers = std::min(worker_limit() - 1, 10u);   // the loop's own thread is one of the workers
+        Crew::get().begin(ahead);
+        block_vocab = vocab;
+        block_rows = n_rows;
+        block_logits = logits;
+        Crew::get().allow(ahead, std::min(6u, n_rows));
     }
     // no thread reads the block's logits any more
     void end_block() {
-        if (block_logits) {
-            threads.stop.store(true, std::memory_order_relaxed);
-            std::unique_lock<std::mutex> lock(threads.mu);
-            threads.limit = 0;
-            threads.idle.wait(lock, [&] { return threads.running == 0; });
-        }
+        if (block_logits) Crew::get().end(ahead);
         block_logits = nullptr;
         block_rows = 0;
     }
@@ -492,16 +574,11 @@ struct dfl_sampler {
         const uint32_t r = (uint32_t)(off / block_vocab);
         Prepared& p = prepared[r];
         if (p.logits != logits) return false;
-        bool taken;
-        {
-            std::lock_guard<std::mutex> lock(threads.mu);
-            taken = r < threads.next;
-            if (!taken) threads.next = r + 1;
-        }
+        const bool mine = Crew::get().claim(ahead, r);
         // Where rows take the nucleus path they are cheap and stop quickly, so the limit keeps ahead of the loop; the ordered path's rows,
         // milliseconds each, are only added when the loop has used up those it has.
-        if (nucleus_path() ? r >= 4 : r >= 6) allow_rows(nucleus_path() ? r + 8 : (r + 4) / 10 * 10 + 6);
-        if (!taken) build_row(r);
+        if (nucleus_path() ? r >= 4 : r >= 6) Crew::get().allow(ahead, std::min(nucleus_path() ? r + 8 : (r + 4) / 10 * 10 + 6, block_rows));
+        if (mine) build_row(r);
         while (!p.done.load(std::memory_order_acquire)) std::this_thread::yield();
         *e = p.err;
         *nan_token = p.nan_token;
@@ -765,6 +842,7 @@ dfl_status sampling_fail(SErr e, uint64_t nan_token, int row) {
         case S_NAN: return fail(DFL_ERR_SAMPLING, where + "logit at token " + std::to_string(nan_token) + " is NaN");
         case S_TOO_LARGE: return fail(DFL_ERR_SAMPLING, where + "vocabulary size exceeds i32 token ids");
         case S_NO_CANDIDATES: return fail(DFL_ERR_SAMPLING, where + "sampling retained no finite-probability candidates");
+        case S_MEMORY: return fail(DFL_ERR_OOM, where + "no memory for the filtered distribution");
         case S_PROPOSAL_RANGE: return fail(DFL_ERR_SAMPLING, where + "proposal token is outside the target vocabulary");
         case S_PROPOSAL_WEIGHT: return fail(DFL_ERR_SAMPLING, where + "proposal weight must be finite and non-negative");
         case S_MISSING_PROPOSAL: return fail(DFL_ERR_SAMPLING, where + "sampled proposal token has no positive proposal weight");
