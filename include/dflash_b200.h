@@ -669,6 +669,12 @@ dfl_status dfl_device_to_host(int32_t device, const void* dev_ptr, void* host, u
 void* dfl_host_alloc(uint64_t n_bytes);
 void dfl_host_free(void* ptr);
 
+/* The rules of the pool that keeps blocks of closed sessions, over a source that only counts (no GPU): at most `limit` idle bytes, a source
+ * of `capacity` bytes, `host` nonzero for the size classes of pinned blocks.  ops[i] > 0 takes that many bytes (block number = takes so far),
+ * ops[i] < 0 gives block -ops[i] - 1 back, 0 trims.  trace [n_ops][3]: whether the take had memory, bytes the pool holds of its
+ * source, blocks fetched from it so far. */
+dfl_status dfl_pool_selftest(uint64_t limit, uint64_t capacity, int32_t host, const int64_t* ops, uint32_t n_ops, int64_t* trace);
+
 #ifdef __cplusplus
 }
 #endif

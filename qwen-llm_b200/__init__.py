@@ -151,6 +151,14 @@ def _result_f32(shape):
     return np.asarray(_ResultBlock(ptr, shape)) if ptr else np.zeros(shape, dtype=np.float32)
 
 
+def pool_selftest(ops, limit, capacity, host=False):
+    """The block pool's rules over a counting source (see dfl_pool_selftest): (had memory, bytes held, blocks fetched) after every op."""
+    ops = np.ascontiguousarray(ops, dtype=np.int64)
+    trace = np.zeros((ops.size, 3), dtype=np.int64)
+    check(lib().dfl_pool_selftest(C.c_uint64(limit), C.c_uint64(capacity), C.c_int32(1 if host else 0), _ptr(ops), C.c_uint32(ops.size), _ptr(trace)))
+    return trace
+
+
 def set_host_wait(mode):
     """'auto' | 'spin' | 'yield' | 'block': how host threads wait for the device (dfl_set_host_wait)."""
     check(lib().dfl_set_host_wait(C.c_int32({"auto": 0, "spin": 1, "yield": 2, "block": 3}[mode])))

@@ -130,7 +130,7 @@ dfl_status qmatrix_create(int device, int dtype, uint64_t n_in, uint64_t n_out, 
         if (n_bytes != n_in * n_out * 4) return fail(DFL_ERR_BAD_SHAPE, "qmatrix: f32 byte count mismatch");
         m->kblocks = 0;
         m->row_tiles = 0;
-        DFL_CUDA(cudaMalloc(&m->tiles, n_bytes));
+        DFL_CUDA(device_malloc(&m->tiles, n_bytes));
         DFL_CUDA(cudaMemcpyAsync(m->tiles, data, n_bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
         DFL_CUDA(cudaStreamSynchronize(st));
         return DFL_OK;
@@ -143,7 +143,7 @@ dfl_status qmatrix_create(int device, int dtype, uint64_t n_in, uint64_t n_out, 
     const uint8_t* src = static_cast<const uint8_t*>(data);
     uint8_t* tmp = nullptr;
     if (!on_device) {
-        DFL_CUDA(cudaMalloc(&tmp, n_bytes));
+        DFL_CUDA(device_malloc(&tmp, n_bytes));
         DFL_CUDA(cudaMemcpyAsync(tmp, data, n_bytes, cudaMemcpyHostToDevice, st));
         src = tmp;
     }
@@ -157,7 +157,7 @@ dfl_status qmatrix_create(int device, int dtype, uint64_t n_in, uint64_t n_out, 
         }
         if (!fits) m->layout = LAYOUT_FRAG;
     }
-    cudaError_t e = cudaMalloc(&m->tiles, m->bytes());   // the layout decides the resident size
+    cudaError_t e = device_malloc(&m->tiles, m->bytes());   // the layout decides the resident size
     if (e != cudaSuccess) {
         if (tmp) cudaFree(tmp);
         return fail(DFL_ERR_OOM, std::string("qmatrix: cudaMalloc: ") + cudaGetErrorString(e));
@@ -255,7 +255,7 @@ dfl_status dfl_qmatrix_dequant(const dfl_qmatrix* m, float* out_host, uint64_t n
         return DFL_OK;
     }
     float* d = nullptr;
-    DFL_CUDA(cudaMalloc(&d, n_floats * 4));
+    DFL_CUDA(device_malloc(&d, n_floats * 4));
     dfl_status s = m->m.layout == LAYOUT_TS ? decode_tiles_ts(0, m->m, d) : decode_tiles(0, m->m, d);
     cudaError_t e = cudaMemcpy(out_host, d, n_floats * 4, cudaMemcpyDeviceToHost);
     cudaFree(d);
@@ -276,8 +276,8 @@ dfl_status dfl_fewrow_matmul(const dfl_qmatrix* m, const float* x_host, int32_t 
     int* err = nullptr;
     dfl_status s = DFL_OK;
     auto cleanup = [&]() { cudaFree(x); cudaFree(part); cudaFree(y); cudaFree(acts); pool_free(err); };
-    if (cudaMalloc(&x, (size_t)n_rows * q.n_in * 4) != cudaSuccess || cudaMalloc(&part, (size_t)splits * MAX_ROWS * q.n_out * 4) != cudaSuccess ||
-        cudaMalloc(&y, (size_t)n_rows * q.n_out * 4) != cudaSuccess || cudaMalloc(&acts, acts_bytes_for(q)) != cudaSuccess ||
+    if (device_malloc(&x, (size_t)n_rows * q.n_in * 4) != cudaSuccess || device_malloc(&part, (size_t)splits * MAX_ROWS * q.n_out * 4) != cudaSuccess ||
+        device_malloc(&y, (size_t)n_rows * q.n_out * 4) != cudaSuccess || device_malloc(&acts, acts_bytes_for(q)) != cudaSuccess ||
         !(err = (int*)pool_alloc_host(4))) {
         cleanup();
         return fail(DFL_ERR_OOM, "fewrow_matmul: cudaMalloc failed");
@@ -304,8 +304,8 @@ dfl_status dfl_argmax_top2(int32_t device, const float* logits_host, int32_t n_r
     float *l = nullptr, *g = nullptr;
     int32_t* a = nullptr;
     auto cleanup = [&]() { cudaFree(l); cudaFree(g); cudaFree(a); };
-    if (cudaMalloc(&l, (size_t)n_rows * vocab * 4) != cudaSuccess || cudaMalloc(&g, n_rows * 4) != cudaSuccess ||
-        cudaMalloc(&a, n_rows * 4) != cudaSuccess) {
+    if (device_malloc(&l, (size_t)n_rows * vocab * 4) != cudaSuccess || device_malloc(&g, n_rows * 4) != cudaSuccess ||
+        device_malloc(&a, n_rows * 4) != cudaSuccess) {
         cleanup();
         return fail(DFL_ERR_OOM, "argmax_top2: cudaMalloc failed");
     }
@@ -334,12 +334,12 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
     p->splits2 = gemm_choose_splits(head->m);
     const uint64_t k1 = w1->m.n_in, n1 = w1->m.n_out, v = head->m.n_out;
     bool ok = (p->st = pool_stream()) != nullptr;
-    ok = ok && cudaMalloc(&p->x, MAX_ROWS * k1 * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->part1, (size_t)p->splits1 * MAX_ROWS * n1 * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->part2, (size_t)p->splits2 * MAX_ROWS * v * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->logits, MAX_ROWS * v * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->acts1, acts_bytes_for(w1->m)) == cudaSuccess;
-    ok = ok && cudaMalloc(&p->acts2, acts_bytes_for(head->m)) == cudaSuccess;
+    ok = ok && device_malloc(&p->x, MAX_ROWS * k1 * 4) == cudaSuccess;
+    ok = ok && device_malloc(&p->part1, (size_t)p->splits1 * MAX_ROWS * n1 * 4) == cudaSuccess;
+    ok = ok && device_malloc(&p->part2, (size_t)p->splits2 * MAX_ROWS * v * 4) == cudaSuccess;
+    ok = ok && device_malloc(&p->logits, MAX_ROWS * v * 4) == cudaSuccess;
+    ok = ok && device_malloc(&p->acts1, acts_bytes_for(w1->m)) == cudaSuccess;
+    ok = ok && device_malloc(&p->acts2, acts_bytes_for(head->m)) == cudaSuccess;
     ok = ok && cudaEventCreate(&p->e0) == cudaSuccess && cudaEventCreate(&p->e1) == cudaSuccess;
     static_assert(sizeof(dfl_c1::HostOut) <= 256, "the rows follow 256 bytes further");
     ok = ok && (p->out = (dfl_c1::HostOut*)pool_alloc_host(256 + MAX_ROWS * k1 * 4));   // one block: pinning costs a millisecond each time

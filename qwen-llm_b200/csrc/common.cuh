@@ -21,6 +21,14 @@ dfl_status fail(dfl_status st, const std::string& msg);
 extern std::atomic<uint64_t> g_launches;
 inline void count_launch(uint64_t n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
+// cudaMalloc / cudaMallocHost that give the idle blocks of the pool back (pool.cu) and try again when there is no memory
+cudaError_t device_malloc_bytes(void** p, size_t bytes);
+cudaError_t host_malloc_bytes(void** p, size_t bytes);
+template <typename T>
+inline cudaError_t device_malloc(T** p, size_t bytes) { return device_malloc_bytes(reinterpret_cast<void**>(p), bytes); }
+template <typename T>
+inline cudaError_t host_malloc(T** p, size_t bytes) { return host_malloc_bytes(reinterpret_cast<void**>(p), bytes); }
+
 #define DFL_CUDA(call)                                                                         \
     do {                                                                                       \
         cudaError_t _e = (call);                                                               \

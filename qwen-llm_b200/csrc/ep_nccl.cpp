@@ -134,7 +134,7 @@ dfl_status ep_p2p_exchange(void* comm, int rank, int world, void* local, cudaStr
     cudaIpcMemHandle_t mine;
     DFL_CUDA(cudaIpcGetMemHandle(&mine, local));
     uint8_t* dev_all = nullptr;
-    DFL_CUDA(cudaMalloc(&dev_all, (size_t)world * sizeof(mine)));
+    DFL_CUDA(device_malloc(&dev_all, (size_t)world * sizeof(mine)));
     std::vector<cudaIpcMemHandle_t> all((size_t)world);
     cudaError_t e = cudaMemcpyAsync(dev_all + (size_t)rank * sizeof(mine), &mine, sizeof(mine), cudaMemcpyHostToDevice, st);
     int rc = 0;
@@ -167,7 +167,7 @@ bool ep_barrier_bounded(void* comm, cudaStream_t st, uint32_t timeout_ms) {
     if (!g_nccl.CommAbort || !g_nccl.CommGetAsyncError) return false;
     float* one = nullptr;
     cudaEvent_t ev = nullptr;
-    if (cudaMalloc(&one, 4) != cudaSuccess) return false;
+    if (device_malloc(&one, 4) != cudaSuccess) return false;
     if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) { cudaFree(one); return false; }
     cudaMemsetAsync(one, 0, 4, st);
     bool ok = g_nccl.AllReduce(one, one, 1, 7, 0, comm, st) == 0 && cudaEventRecord(ev, st) == cudaSuccess;

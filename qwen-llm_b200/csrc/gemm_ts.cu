@@ -164,7 +164,7 @@ __global__ void decode_tiles_ts_kernel(const uint8_t* __restrict__ tiles, int dt
 // Whether every block scale of a Q8_0 matrix (ggml bytes on the device) leaves q * d inside the f16 range.
 dfl_status q80_scales_fit_ts(cudaStream_t st, const uint8_t* ggml_dev, uint64_t n_in, uint64_t n_out, bool* fits) {
     int* flag = nullptr;
-    DFL_CUDA(cudaMalloc(&flag, sizeof(int)));
+    DFL_CUDA(device_malloc(&flag, sizeof(int)));
     cudaMemsetAsync(flag, 0, sizeof(int), st);
     const uint64_t n_blocks = n_in / 32 * n_out;
     q80_scale_range_kernel<<<(unsigned)((n_blocks + 255) / 256), 256, 0, st>>>(ggml_dev, n_blocks, flag);

@@ -118,7 +118,7 @@ dfl_status dfl_generate(const dfl_model* m, dfl_session* s, dfl_scratch* sc, dfl
     }
     // the block's logits for the host sampler: pinned (the 16 x vocab copy runs at link speed) and kept with the scratch,
     // since pinning and unpinning 10 MB costs far more than a step
-    if (sampled && !sc->pinned_logits && cudaMallocHost(&sc->pinned_logits, (size_t)sc->block_size * V * 4) != cudaSuccess) {
+    if (sampled && !sc->pinned_logits && host_malloc(&sc->pinned_logits, (size_t)sc->block_size * V * 4) != cudaSuccess) {
         sc->pinned_logits = nullptr;
         if (proposal_sampler) dfl_sampler_destroy(proposal_sampler);
         return fail(DFL_ERR_OOM, "generate: pinned logits buffer");
@@ -127,7 +127,7 @@ dfl_status dfl_generate(const dfl_model* m, dfl_session* s, dfl_scratch* sc, dfl
     // rows ordered on the device: the order lands beside the logits and the sampler is told where (cleared on every exit)
     const bool device_order = sampled && params->device_row_order;
     if (device_order) {
-        if (!sc->pinned_order && cudaMallocHost(&sc->pinned_order, (size_t)sc->block_size * V * 4) != cudaSuccess) {
+        if (!sc->pinned_order && host_malloc(&sc->pinned_order, (size_t)sc->block_size * V * 4) != cudaSuccess) {
             sc->pinned_order = nullptr;
             if (proposal_sampler) dfl_sampler_destroy(proposal_sampler);
             return fail(DFL_ERR_OOM, "generate: pinned row-order buffer");

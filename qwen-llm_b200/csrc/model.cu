@@ -60,7 +60,7 @@ dfl_status build_group(int device, cudaStream_t st, const TensorMap& tm, const s
             DFL_CHECK(qmatrix_create(device, t0->dtype, n_in, rows, t0->data, t0->n_bytes, t0->on_device != 0, st, &qm, allow_ts, kb_group));
         } else {
             uint8_t* cat = nullptr;
-            DFL_CUDA(cudaMalloc(&cat, bytes));
+            DFL_CUDA(device_malloc(&cat, bytes));
             uint64_t off = 0;
             for (size_t k = i; k < j; ++k) {
                 const dfl_tensor* t = tm.find(names[k]);
@@ -115,13 +115,13 @@ dfl_status upload_f32(int device, cudaStream_t st, const TensorMap& tm, const st
         return fail(DFL_ERR_UNSUPPORTED, "tensor " + name + " must be f32, f16 or bf16");
     const uint64_t esz = t->dtype == DFL_F32 ? 4 : 2;
     if (t->n_bytes != n * esz) return fail(DFL_ERR_BAD_SHAPE, "tensor " + name + " byte count mismatch");
-    DFL_CUDA(cudaMalloc(out, n * 4));
+    DFL_CUDA(device_malloc(out, n * 4));
     if (t->dtype == DFL_F32) {
         DFL_CUDA(cudaMemcpyAsync(*out, t->data, n * 4, t->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
         DFL_CUDA(cudaStreamSynchronize(st));
     } else {
         uint8_t* tmp = nullptr;
-        DFL_CUDA(cudaMalloc(&tmp, t->n_bytes));
+        DFL_CUDA(device_malloc(&tmp, t->n_bytes));
         cudaMemcpyAsync(tmp, t->data, t->n_bytes, t->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st);
         decode_small_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(t->dtype, tmp, n, *out);
         count_launch();
@@ -483,7 +483,7 @@ static dfl_status model_create_impl(int32_t device, const dfl_arch* arch, const 
         if (!te) { s = fail(DFL_ERR_MISSING_TENSOR, "missing tensor token_embd.weight"); goto failed; }
         const uint64_t want = V * (H / 256) * (uint64_t)ggml_bytes_per_256(te->dtype);
         if (ggml_bytes_per_256(te->dtype) == 0 || te->n_bytes != want) { s = fail(DFL_ERR_BAD_SHAPE, "token_embd.weight: byte count"); goto failed; }
-        if (cudaMalloc(&m->embd_ggml, te->n_bytes) != cudaSuccess) { s = fail(DFL_ERR_OOM, "token_embd"); goto failed; }
+        if (device_malloc(&m->embd_ggml, te->n_bytes) != cudaSuccess) { s = fail(DFL_ERR_OOM, "token_embd"); goto failed; }
         cudaMemcpy(m->embd_ggml, te->data, te->n_bytes, te->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
         m->embd_dtype = te->dtype;
         const char* head_name = tm.find("output.weight") ? "output.weight" : "token_embd.weight";  // tied embeddings, loader.rs:445
@@ -516,7 +516,12 @@ static dfl_status model_create_impl(int32_t device, const dfl_arch* arch, const 
                 MC(upload_f32(device, st, tm, blk(il, "ssm_alpha.weight"), H * a.gdn_n_v_heads, &al));
                 s = upload_f32(device, st, tm, blk(il, "ssm_beta.weight"), H * a.gdn_n_v_heads, &be);
                 if (s != DFL_OK) { cudaFree(al); goto failed; }
-                cudaMalloc(&L.w_ab, 2 * H * a.gdn_n_v_heads * 4);
+                if (device_malloc(&L.w_ab, 2 * H * a.gdn_n_v_heads * 4) != cudaSuccess) {
+                    cudaFree(al);
+                    cudaFree(be);
+                    s = fail(DFL_ERR_OOM, "model_create: alpha / beta projection");
+                    goto failed;
+                }
                 cudaMemcpy(L.w_ab, al, H * a.gdn_n_v_heads * 4, cudaMemcpyDeviceToDevice);
                 cudaMemcpy(L.w_ab + H * a.gdn_n_v_heads, be, H * a.gdn_n_v_heads * 4, cudaMemcpyDeviceToDevice);
                 cudaFree(al);
@@ -561,7 +566,12 @@ static dfl_status model_create_impl(int32_t device, const dfl_arch* arch, const 
                 MC(upload_f32(device, st, tm, blk(il, "ffn_gate_inp.weight"), H * E, &rw));
                 s = upload_f32(device, st, tm, blk(il, "ffn_gate_inp_shexp.weight"), H, &sgw);
                 if (s != DFL_OK) { cudaFree(rw); goto failed; }
-                cudaMalloc(&L.router_w, (E + 1) * H * 4);
+                if (device_malloc(&L.router_w, (E + 1) * H * 4) != cudaSuccess) {
+                    cudaFree(rw);
+                    cudaFree(sgw);
+                    s = fail(DFL_ERR_OOM, "model_create: router");
+                    goto failed;
+                }
                 cudaMemcpy(L.router_w, rw, E * H * 4, cudaMemcpyDeviceToDevice);
                 cudaMemcpy(L.router_w + E * H, sgw, H * 4, cudaMemcpyDeviceToDevice);
                 cudaFree(rw);
@@ -588,7 +598,7 @@ static dfl_status model_create_impl(int32_t device, const dfl_arch* arch, const 
             const uint64_t recv_bytes = ep_recv_floats(ep_world, H) * 4;
             const uint64_t flag_bytes = 2ull * ep_world * ep_combine_ctas(H) * 4;
             void* local = nullptr;
-            if (cudaMalloc(&local, recv_bytes + flag_bytes) != cudaSuccess) { s = fail(DFL_ERR_OOM, "model_create: exchange buffer"); goto failed; }
+            if (device_malloc(&local, recv_bytes + flag_bytes) != cudaSuccess) { s = fail(DFL_ERR_OOM, "model_create: exchange buffer"); goto failed; }
             cudaMemset(local, 0, recv_bytes + flag_bytes);
             cudaDeviceSynchronize();
             void* peers[EP_MAX_WORLD] = {};
@@ -776,7 +786,7 @@ dfl_status dfl_session_read_kv(const dfl_session* s, uint32_t attn_index, uint32
     if (s->kv_mode == KV_F16_TILED) {
         std::vector<__half> hk(stride), hv(stride);
         __half* tmp = nullptr;
-        DFL_CUDA(cudaMalloc(&tmp, 2 * stride * 2));
+        DFL_CUDA(device_malloc(&tmp, 2 * stride * 2));
         dfl_status st = launch_kv_tiled_to_rows(s->st, s->k_cache[attn_index], false, (int)s->m->arch.n_kv_heads, pos, 1, tmp);
         if (st == DFL_OK) st = launch_kv_tiled_to_rows(s->st, s->v_cache[attn_index], true, (int)s->m->arch.n_kv_heads, pos, 1, tmp + stride);
         cudaError_t e = cudaStreamSynchronize(s->st);
@@ -938,12 +948,12 @@ dfl_status dfl_scratch_set_order_host(dfl_scratch* sc, uint32_t* order_host) {
     if (!sc->order_dev || !sc->sort_scratch) {   // device side of the ordering, made once per scratch and here, where failing is clean
         DFL_CHECK(use_device(sc->m->device));
         const uint64_t V = sc->m->arch.vocab_size;
-        if (!sc->order_dev && cudaMalloc(&sc->order_dev, (size_t)sc->block_size * V * 4) != cudaSuccess) {
+        if (!sc->order_dev && device_malloc(&sc->order_dev, (size_t)sc->block_size * V * 4) != cudaSuccess) {
             sc->order_dev = nullptr;
             cudaGetLastError();
             return fail(DFL_ERR_OOM, "set_order_host: device order buffer");
         }
-        if (!sc->sort_scratch && cudaMalloc(&sc->sort_scratch, sort_rows_scratch_bytes((int)sc->block_size, V)) != cudaSuccess) {
+        if (!sc->sort_scratch && device_malloc(&sc->sort_scratch, sort_rows_scratch_bytes((int)sc->block_size, V)) != cudaSuccess) {
             sc->sort_scratch = nullptr;
             cudaGetLastError();
             return fail(DFL_ERR_OOM, "set_order_host: sort scratch");
@@ -1113,7 +1123,7 @@ dfl_status dfl_session_snapshot(const dfl_model* m, dfl_session* s, dfl_dsession
     // packed to the prefix, as position-major rows whatever the session's storage: the unused tail of the cache is not
     // carried, and a snapshot restores into a session of either storage
     void* rows_tmp = nullptr;
-    if (s->kv_mode == KV_F16_TILED && per_layer) DFL_CUDA(cudaMalloc(&rows_tmp, per_layer));
+    if (s->kv_mode == KV_F16_TILED && per_layer) DFL_CUDA(device_malloc(&rows_tmp, per_layer));
     for (int which = 0; which < 2; ++which)
         for (size_t ai = 0; ai < s->k_cache.size(); ++ai, p += per_layer) {
             if (!per_layer) continue;

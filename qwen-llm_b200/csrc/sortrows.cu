@@ -183,8 +183,8 @@ extern "C" dfl_status dfl_sort_rows_desc(int32_t device, const float* logits_hos
     uint32_t* order = nullptr;
     void* sc = nullptr;
     auto cleanup = [&]() { cudaFree(x); cudaFree(order); cudaFree(sc); };
-    if (cudaMalloc(&x, (size_t)n_rows * vocab * 4) != cudaSuccess || cudaMalloc(&order, (size_t)n_rows * vocab * 4) != cudaSuccess ||
-        cudaMalloc(&sc, sort_rows_scratch_bytes(n_rows, vocab)) != cudaSuccess) {
+    if (device_malloc(&x, (size_t)n_rows * vocab * 4) != cudaSuccess || device_malloc(&order, (size_t)n_rows * vocab * 4) != cudaSuccess ||
+        device_malloc(&sc, sort_rows_scratch_bytes(n_rows, vocab)) != cudaSuccess) {
         cleanup();
         return fail(DFL_ERR_OOM, "sort_rows: cudaMalloc failed");
     }

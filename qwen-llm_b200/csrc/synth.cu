@@ -153,7 +153,7 @@ dfl_status dfl_synth_tensor(int32_t device, int32_t dtype, uint64_t n_in, uint64
         default: return fail(DFL_ERR_UNSUPPORTED, "synth_tensor: dtype");
     }
     uint8_t* p = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(DFL_ERR_OOM, "synth_tensor: cudaMalloc failed");
+    if (device_malloc(&p, bytes) != cudaSuccess) return fail(DFL_ERR_OOM, "synth_tensor: cudaMalloc failed");
     const unsigned tb = 128;
     switch (dtype) {
         case DFL_Q4_K: synth_k45_kernel<15><<<(unsigned)((blocks + tb - 1) / tb), tb>>>(p, blocks, seed, std_dev); break;

@@ -113,8 +113,8 @@ extern "C" dfl_status dfl_topk16(int32_t device, const float* x_host, int32_t n_
     int32_t* id = nullptr;
     void* sc = nullptr;
     auto cleanup = [&]() { cudaFree(x); cudaFree(v); cudaFree(id); cudaFree(sc); };
-    if (cudaMalloc(&x, (size_t)n_rows * n * 4) != cudaSuccess || cudaMalloc(&v, (size_t)n_rows * 64) != cudaSuccess ||
-        cudaMalloc(&id, (size_t)n_rows * 64) != cudaSuccess || cudaMalloc(&sc, topk16_scratch_bytes(n_rows)) != cudaSuccess) {
+    if (device_malloc(&x, (size_t)n_rows * n * 4) != cudaSuccess || device_malloc(&v, (size_t)n_rows * 64) != cudaSuccess ||
+        device_malloc(&id, (size_t)n_rows * 64) != cudaSuccess || device_malloc(&sc, topk16_scratch_bytes(n_rows)) != cudaSuccess) {
         cleanup();
         return fail(DFL_ERR_OOM, "topk16: cudaMalloc failed");
     }
