@@ -238,6 +238,12 @@ class C1Pipeline:
             lib().dfl_c1_destroy(self.h)
             self.h = C.c_void_p()
 
+    def __del__(self):
+        try:
+            self.close()
+        except Exception:
+            pass
+
     def step(self, x, draft_ids, want_logits=False):
         x = np.ascontiguousarray(x, dtype=np.float32).reshape(-1, self.w1.n_in)
         n = x.shape[0]

@@ -196,9 +196,11 @@ struct dfl_qmatrix {
 struct dfl_c1 {
     const dfl_qmatrix* w1;
     const dfl_qmatrix* head;
+    int device;   // kept here: a pipeline may be dropped after its matrices
     cudaStream_t st;
     float *x, *part1, *part2, *logits;
     uint8_t *acts1, *acts2;
+    uint8_t* block;   // backs x .. acts2
     int splits1, splits2;
     cudaEvent_t e0, e1;
     // pinned host memory that the kernels read and write themselves: the results and the error word (HostOut), then the block's rows
@@ -330,16 +332,28 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
     auto* p = new dfl_c1();
     p->w1 = w1;
     p->head = head;
+    p->device = w1->m.device;
     p->splits1 = gemm_choose_splits(w1->m);
     p->splits2 = gemm_choose_splits(head->m);
     const uint64_t k1 = w1->m.n_in, n1 = w1->m.n_out, v = head->m.n_out;
     bool ok = (p->st = pool_stream()) != nullptr;
-    ok = ok && device_malloc(&p->x, MAX_ROWS * k1 * 4) == cudaSuccess;
-    ok = ok && device_malloc(&p->part1, (size_t)p->splits1 * MAX_ROWS * n1 * 4) == cudaSuccess;
-    ok = ok && device_malloc(&p->part2, (size_t)p->splits2 * MAX_ROWS * v * 4) == cudaSuccess;
-    ok = ok && device_malloc(&p->logits, MAX_ROWS * v * 4) == cudaSuccess;
-    ok = ok && device_malloc(&p->acts1, acts_bytes_for(w1->m)) == cudaSuccess;
-    ok = ok && device_malloc(&p->acts2, acts_bytes_for(head->m)) == cudaSuccess;
+    // the block's buffers from the pool, one after another in one block: pipelines come and go with their requests
+    auto up = [](size_t bytes) { return (bytes + 511) / 512 * 512; };
+    const size_t sizes[] = {up(MAX_ROWS * k1 * 4), up((size_t)p->splits1 * MAX_ROWS * n1 * 4), up((size_t)p->splits2 * MAX_ROWS * v * 4), up(MAX_ROWS * v * 4),
+                            up(acts_bytes_for(w1->m)), up(acts_bytes_for(head->m))};
+    size_t total = 0;
+    for (size_t n : sizes) total += n;
+    ok = ok && (p->block = (uint8_t*)pool_alloc(total));
+    if (ok) {
+        uint8_t* at = p->block;
+        auto next = [&](int i) { uint8_t* q = at; at += sizes[i]; return q; };
+        p->x = (float*)next(0);
+        p->part1 = (float*)next(1);
+        p->part2 = (float*)next(2);
+        p->logits = (float*)next(3);
+        p->acts1 = next(4);
+        p->acts2 = next(5);
+    }
     ok = ok && cudaEventCreate(&p->e0) == cudaSuccess && cudaEventCreate(&p->e1) == cudaSuccess;
     static_assert(sizeof(dfl_c1::HostOut) <= 256, "the rows follow 256 bytes further");
     ok = ok && (p->out = (dfl_c1::HostOut*)pool_alloc_host(256 + MAX_ROWS * k1 * 4));   // one block: pinning costs a millisecond each time
@@ -359,8 +373,9 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
 
 void dfl_c1_destroy(dfl_c1* p) {
     if (!p) return;
-    cudaSetDevice(p->w1->m.device);
-    cudaFree(p->x); cudaFree(p->part1); cudaFree(p->part2); cudaFree(p->logits); cudaFree(p->acts1); cudaFree(p->acts2);
+    cudaSetDevice(p->device);
+    if (p->st) cudaStreamSynchronize(p->st);   // nothing of it is in flight when its blocks go back
+    pool_free(p->block);
     pool_free(p->out);
     if (p->e0) cudaEventDestroy(p->e0);
     if (p->e1) cudaEventDestroy(p->e1);

@@ -114,3 +114,26 @@ def test_results_beyond_the_pinned_bound_are_ordinary_arrays():
     assert pkg._result_f32((17 << 20,)).base is None                # above 64 MiB
     del kept
     assert pkg._result_f32((16, 151936)).base is not None           # given back with the arrays
+
+
+@pytest.mark.gpu
+def test_two_matrix_pipelines_that_are_dropped_give_everything_back():
+    import torch
+    ms = []
+    for n_in, n_out in ((1024, 1024), (1024, 32000)):
+        _, _, _, ptr, n_bytes = pkg.synth_tensor("w", pkg.Q4_K, n_in, n_out, 3 + n_out, 0.02)
+        ms.append(pkg.QMatrix(pkg.Q4_K, n_in, n_out, pkg.device_to_host(ptr, n_bytes)))
+        pkg.device_free(ptr)
+    x, draft = np.random.default_rng(0).standard_normal((16, 1024)).astype(np.float32), np.zeros(16, np.int32)
+    first, held = None, []
+    for _ in range(40):
+        am, gap, _, _ = pkg.C1Pipeline(*ms).step(x, draft)      # no close
+        first = first or (am.tobytes(), gap.tobytes())
+        assert (am.tobytes(), gap.tobytes()) == first
+        held.append(torch.cuda.mem_get_info(0)[0])
+    assert held[-1] == held[1]
+    last = pkg.C1Pipeline(*ms)
+    last.step(x, draft)
+    for m in ms:
+        m.close()
+    del last                                                    # after its matrices
