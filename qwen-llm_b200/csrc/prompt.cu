@@ -136,11 +136,17 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
     return DFL_OK;
 }
 
+static int token_tiles(uint32_t n) {
+    const int tile_tok = gemm_tm_tile_tok((int)n);
+    return ((int)n + tile_tok - 1) / tile_tok;
+}
+dfl_status prompt_reserve(const dfl_model* m, dfl_scratch* sc, uint32_t n) { return ensure_ws(m, sc, (uint32_t)(token_tiles(n) * TM_TOK)); }
+
 dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids, const int32_t* tokens,
                        uint32_t n, uint32_t start, uint32_t last_rows, bool want_head) {
     const dfl_arch& a = m->arch;
-    const int tile_tok = gemm_tm_tile_tok((int)n), tok_tiles = (int)((n + tile_tok - 1) / tile_tok), rows_pad = tok_tiles * tile_tok;
-    DFL_CHECK(ensure_ws(m, sc, (uint32_t)(tok_tiles * TM_TOK)));
+    const int tile_tok = gemm_tm_tile_tok((int)n), tok_tiles = token_tiles(n), rows_pad = tok_tiles * tile_tok;
+    DFL_CHECK(prompt_reserve(m, sc, n));
     PromptWs* w = sc->prompt;
     cudaStream_t st = s->st;
     const uint64_t H = a.hidden_size, F = a.intermediate_size, KH = sc->k_layers * H;

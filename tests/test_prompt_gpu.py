@@ -142,3 +142,40 @@ def test_feeding_a_drafter_of_another_model_is_refused_before_the_first_pass(tin
     assert e.value.name == "BAD_ARG" and sess.kv_n_pos == 0 and ds.ctx_len == 0
     for x in (sess, scr, ds, gd, other):
         x.close()
+
+
+def test_a_prompt_without_memory_for_its_workspace_takes_the_packed_path(tiny):
+    import torch
+    arch, gm = tiny
+    rng = np.random.default_rng(5)
+    ids, nxt = rng.integers(0, arch.vocab_size, 523), rng.integers(0, arch.vocab_size, 16)
+
+    def packed(sess, scr):
+        for off in range(0, ids.size, 16):
+            logits, _ = pkg.prefill(gm, sess, scr, [1, 3], ids[off:off + 16], off)
+        return logits
+
+    a, b = pkg.Session(gm, 640), pkg.Session(gm, 640)
+    sa, sb = pkg.Scratch(gm, 16, 2), pkg.Scratch(gm, 16, 2)
+    want = packed(b, sb).copy()          # also loads every kernel that the packed path needs
+    wnext = pkg.packed_verify(gm, b, sb, [1, 3], nxt, ids.size, want_logits=True)[2].copy()
+    held = [torch.empty(torch.cuda.mem_get_info(0)[0] - (1 << 30), dtype=torch.uint8, device="cuda:0")]
+    ptrs = []
+    try:
+        for kib in (1 << 18, 1 << 14, 1 << 11):          # 256, 16, 2 MiB until there is none left
+            try:
+                while True:
+                    ptrs.append(pkg.synth_tensor("w", pkg.F32, 256, kib, 7, 0.02)[3])
+            except pkg.DflError as e:
+                assert e.name == "OOM"
+        got, _ = pkg.prefill(gm, a, sa, [1, 3], ids, 0)
+        gnext = pkg.packed_verify(gm, a, sa, [1, 3], nxt, ids.size, want_logits=True)[2].copy()
+    finally:
+        for p in ptrs:
+            pkg.device_free(p)
+        del held
+        torch.cuda.empty_cache()
+    assert a.kv_n_pos == ids.size + 16 and not a.poisoned
+    assert got.tobytes() == want.tobytes() and gnext.tobytes() == wnext.tobytes()     # the packed path's own bits
+    for x in (a, b, sa, sb):
+        x.close()
