@@ -75,12 +75,14 @@ dfl_status dfl_prefill(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
                             : verify_core(m, s, sc, layer_ids, n_layer_ids, ids + off, nb, start, head);
         if (st != DFL_OK) { s->poisoned = true; return st; }
         const float* capture = big ? prompt_capture(sc) : sc->capture;
+        cudaError_t copied = cudaSuccess;
         if (hidden_host && n_layer_ids)
-            cudaMemcpyAsync(hidden_host + off * KH, capture, (size_t)nb * KH * 4, cudaMemcpyDeviceToHost, s->st);
+            copied = copy_captured(hidden_host + off * KH, capture, nb, n_layer_ids, sc->k_layers, m->arch.hidden_size, cudaMemcpyDeviceToHost, s->st);
         if (head)
             cudaMemcpyAsync(last_logits_host, sc->logits + (uint64_t)(big ? 0 : nb - 1) * m->arch.vocab_size, (size_t)m->arch.vocab_size * 4,
                             cudaMemcpyDeviceToHost, s->st);
         DFL_CHECK(session_drain(s));
+        DFL_CUDA(copied);
         if (feed_drafter) {
             positions.resize(nb);
             for (uint32_t i = 0; i < nb; ++i) positions[i] = start + i;

@@ -225,6 +225,9 @@ dfl_status prompt_reserve(const dfl_model* m, dfl_scratch* sc, uint32_t n);   //
 dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids, const int32_t* tokens,
                        uint32_t n, uint32_t start, uint32_t last_rows, bool want_head);
 const float* prompt_capture(const dfl_scratch* sc);
+// captured rows [rows][k_layers][hidden]: the first `slots` of every row
+cudaError_t copy_captured(float* dst, const float* src, uint32_t rows, uint32_t slots, uint32_t k_layers, uint64_t hidden, cudaMemcpyKind kind,
+                          cudaStream_t st);
 void prompt_ws_free(PromptWs* w);
 dfl_status head_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, uint32_t n, const GemmEpilogue& ep_norm);
 // One packed forward of n <= 16 tokens at positions start..start+n-1 (the body shared by

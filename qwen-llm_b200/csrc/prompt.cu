@@ -25,6 +25,14 @@ struct PromptWs {
 
 const float* prompt_capture(const dfl_scratch* sc) { return sc->prompt->capture; }
 
+// Only the slots that layers were named for: what the others hold in the workspace belongs to whoever had the block before.
+cudaError_t copy_captured(float* dst, const float* src, uint32_t rows, uint32_t slots, uint32_t k_layers, uint64_t hidden, cudaMemcpyKind kind,
+                          cudaStream_t st) {
+    const size_t pitch = (size_t)k_layers * hidden * 4;
+    if (slots == k_layers) return cudaMemcpyAsync(dst, src, rows * pitch, kind, st);
+    return cudaMemcpy2DAsync(dst, pitch, src, pitch, (size_t)slots * hidden * 4, rows, kind, st);
+}
+
 void prompt_ws_free(PromptWs* w) {
     if (!w) return;
     pool_free(w->base);
@@ -309,7 +317,7 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
                                  cudaMemcpyDeviceToDevice, st));
     // the last block's captured rows where a packed pass would have left them
     if (n_ids)
-        DFL_CUDA(cudaMemcpyAsync(sc->capture, w->capture + (uint64_t)(n - last_rows) * KH, (size_t)last_rows * KH * 4, cudaMemcpyDeviceToDevice, st));
+        DFL_CUDA(copy_captured(sc->capture, w->capture + (uint64_t)(n - last_rows) * KH, last_rows, n_ids, sc->k_layers, H, cudaMemcpyDeviceToDevice, st));
     s->kv_n_pos = start + n;
     sc->last_n = last_rows;
     sc->last_n_verify = last_rows;

@@ -179,3 +179,21 @@ def test_a_prompt_without_memory_for_its_workspace_takes_the_packed_path(tiny):
     assert got.tobytes() == want.tobytes() and gnext.tobytes() == wnext.tobytes()     # the packed path's own bits
     for x in (a, b, sa, sb):
         x.close()
+
+
+@pytest.mark.parametrize("n", [8, 40, 520])
+def test_capture_slots_without_a_layer_stay_untouched(tiny, n):
+    arch, gm = tiny
+    ids = np.random.default_rng(6).integers(0, arch.vocab_size, n)
+
+    def run(layer_ids):
+        sess, scr = pkg.Session(gm, 640), pkg.Scratch(gm, 16, 2)
+        rows = pkg.prefill(gm, sess, scr, layer_ids, ids, 0, want_hidden=True)[1].copy()
+        block = scr.read_capture(n % 16 or 16).copy()
+        sess.close(); scr.close()
+        return rows, block
+
+    both = run([1, 3])              # fills both slots; its memory goes to the next scratch
+    one = run([3])
+    assert np.array_equal(one[0][:, 0], both[0][:, 1]) and not one[0][:, 1].any()
+    assert np.array_equal(one[1][:, 0], both[1][:, 1]) and not one[1][:, 1].any()
