@@ -355,7 +355,8 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         const uint32_t tm_l = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
         uint32_t e = 0;
         int scaled_tt = -1;
-        for (int idx = blockIdx.x; idx < n_items && ok; idx += gridDim.x) {
+        // A warp that has given up a wait still walks the items: the named barriers below have no limit, so all eight warps must come.
+        for (int idx = blockIdx.x; idx < n_items; idx += gridDim.x) {
             const Item it = item_of(idx);
             const int n_c = (it.rows + 15) / 16, c0 = half ? (n_c + 1) / 2 : 0, c1 = half ? n_c : (n_c + 1) / 2;
             const int live = SEG ? it.rows : p.n_rows - it.tt * p.tile_tok;

@@ -2,7 +2,8 @@
 
 Shared memory of another CTA of a cluster may only be touched once that CTA is known to have started: every kernel that maps it
 passes a cluster barrier first.  A kernel that reads before its dependency wait what an earlier pass wrote needs a plain
-launch, which waits for everything, at the start of its own pass."""
+launch, which waits for everything, at the start of its own pass.  A named barrier has no limit, so no warp may skip it because one
+of its limited waits has run out."""
 import glob
 import os
 import re
@@ -49,3 +50,26 @@ def test_a_pass_starts_with_a_plain_launch():
         core = text[re.search(r"dfl_status " + fn + r"\([^;{]*\{", text).end():]
         queued = re.findall(r"DFL_CHECK\((launch_\w+)\(", core)   # on the pass's own stream, in order
         assert queued[0] == "launch_embed_block", path
+
+
+def _enclosing(text, at):
+    """Headers of the blocks around a position, innermost first."""
+    depth = 0
+    for i in range(at, -1, -1):
+        depth += {"}": 1, "{": -1}.get(text[i], 0)
+        if depth < 0:
+            depth = 0
+            start = max(text.rfind(c, 0, i) for c in "{}\n")
+            line = text.rfind("\n", 0, i) + 1
+            yield text[min(start + 1, line):i]
+
+
+def test_named_barriers_do_not_depend_on_a_limited_wait():
+    seen = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        text = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"named_sync\(1|bar\.sync 1,", text):
+            seen += 1
+            for header in _enclosing(text, m.start()):
+                assert not re.search(r"\bok\b", header), (os.path.basename(path), header.strip())
+    assert seen >= 8
