@@ -238,8 +238,8 @@ namespace ts {
 constexpr int GROUP_WARPS = 8;                          // unpacking warps per group; thread = (row = 32 * (warp % 4) + lane, kp2 = (warp / 4) % 2)
 constexpr int UNPACK_WARPS = 2 * GROUP_WARPS;           // two groups that take the entries alternately, so that their phases interleave
 constexpr int DRAIN_WARP0 = 16, DRAIN_WARPS = 4;        // thread = weight row; warp % 4 = its quarter of the tensor-memory lanes
-constexpr int MMA_WARP0 = 20, MMA_WARPS = 2;            // warp 20 + g issues the MMAs of group g
-constexpr int PRODUCER_WARP = 24;                       // on the scheduler of warp 20; 22 and 23 only help with a side projection
+constexpr int MMA_WARP0 = 20, MMA_WARPS = 4;            // warp 20 + 2 g + c issues the MMAs of group g's halves h with h % 2 == c
+constexpr int PRODUCER_WARP = 24;
 constexpr int THREADS = 25 * 32;                        // 800
 #ifndef DFL_TS_KC
 #define DFL_TS_KC 6
@@ -247,7 +247,7 @@ constexpr int THREADS = 25 * 32;                        // 800
 constexpr int KC = DFL_TS_KC;                           // column blocks whose activations stay resident
 
 // tensor-memory columns (32-bit each, 128 lanes), everything once per group: a 128-column A buffer (256 f16 per row)
-// written and consumed in two halves, a 32-column accumulator, the 8-column A operand of the
+// written and consumed in two halves, two 32-column accumulators (even / odd MMA steps), the 8-column A operand of the
 // min term and its 48-column accumulator
 constexpr uint32_t TM_A = 0, TM_A_STRIDE = 128, TM_D = 256, TM_D_STRIDE = 64, TM_AM = 384, TM_AM_STRIDE = 8, TM_DM = 400, TM_DM_STRIDE = 48,
                    TM_COLS = 512;

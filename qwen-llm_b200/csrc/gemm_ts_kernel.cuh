@@ -4,17 +4,18 @@
 // row tile.  Its work is the sequence of entries e = (tile, column block); the weight stage of
 // entry e travels through ring slot e % STAGES.  The sixteen unpacking warps form two groups of
 // eight that take the entries alternately (group = e & 1), each with its own A buffer,
-// accumulator and barriers, so that one group's arithmetic fills the time the other spends
+// accumulators and barriers, so that one group's arithmetic fills the time the other spends
 // storing to tensor memory and waiting.  A group unpacks an entry in HALVES steps of 64 A-buffer
 // columns (Q4_K / Q5_K: two halves of 128 weight columns; Q6_K: four of 64, each written as the
 // even / odd scale parts); the MMA warp issues eight MMAs per half as soon as it is stored.
 //
 //   producer thread     ring slot free?   -> bulk copy of the stage          -> full[slot]   (activations: a draining thread)
 //   unpacking group g   full[slot]        -> registers -> a_free[g][half]?   -> tcgen05.st -> a_ready[g][half], empty[slot]
-//   MMA warp g          a_ready[g][half], d_free[g]? -> 8 tcgen05.mma (+ min) -> commit: a_free[g][half], d_ready[g]
-//                       (one warp a group: with one per half, each half needed an accumulator of its own for the sum's order
-//                       not to depend on the warps' race, which cost the draining warps two more tensor-memory loads and
-//                       32 adds an entry; the GEMMs of a verify pass 1800 -> 1777 us together)
+//   MMA warp (g, c)     a_ready[g][c], d_free[g]?    -> 8 tcgen05.mma (+ min) -> commit: a_free[g][c], d_ready[g]
+//                       (c = half % 2: its MMAs accumulate into accumulator c of the group, so the order in which the
+//                       two warps of a group reach the tensor pipe does not change a bit of the result.  Two accumulators are also
+//                       what keeps the precision: each step of a tensor-core sum drops what lies below the sum's last place, and
+//                       one accumulator of twice the steps was 1.7 times further from the float64 result, for 1.3 % of the time)
 //   4 draining warps    d_ready[g]        -> tcgen05.ld -> d_free[g]         -> scale, add; tile end: global store
 //
 // The super-block scales d / dmin of an entry travel from the unpacking threads to the draining
@@ -123,6 +124,24 @@ __device__ __forceinline__ void side_projection(const Params& p, float* smem) {
     }
 }
 
+// The eight MMAs of half h = 2 h2 + C of an entry into one accumulator (the first of them overwrites it when the half is
+// the accumulator's first of the entry).
+template <class F, int C>
+__device__ __forceinline__ void issue_half(int h2, uint32_t d, uint32_t a_buf, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
+#pragma unroll
+    for (int hh = 0; hh < F::HALVES / 2; ++hh) {
+        if (hh != h2) continue;
+        constexpr int dummy = 0;
+        (void)dummy;
+        const int h = 2 * hh + C;
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj) {
+            if (hh == 0 && jj == 0) mma_ts<false>(d, a_buf + F::a_col(h, jj), b_lo + F::b_slice(h, jj) * 64u, b_hi, idesc);
+            else mma_ts<true>(d, a_buf + F::a_col(h, jj), b_lo + F::b_slice(h, jj) * 64u, b_hi, idesc);
+        }
+    }
+}
+
 template <int DT>
 __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
     using F = Fmt<DT>;
@@ -191,7 +210,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
             mbar_init(&a_free[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&d_ready[i], 1);
+            mbar_init(&d_ready[i], 2);
             mbar_init(&d_free[i], DRAIN_WARPS);
         }
 
@@ -239,14 +258,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
         }
     } else if (warp >= MMA_WARP0 && warp < MMA_WARP0 + MMA_WARPS) {
         // ------------------------------ MMA issuers ------------------------------
-        // Warp g issues group g's entries, half after half, into the group's accumulator.  The whole warp walks the loop so that
-        // addresses and descriptors stay warp-uniform; one elected lane issues.
+        // Warp (g, c) issues the halves h with h % 2 == c of group g's entries into accumulator c of that group.  The
+        // whole warp walks the loop so that addresses and descriptors stay warp-uniform; one elected lane issues.
         constexpr uint32_t IDESC_MAIN = instr_desc(32), IDESC_MIN = instr_desc(48);
-        const uint32_t g = (uint32_t)(warp - MMA_WARP0);
+        const uint32_t g = (uint32_t)(warp - MMA_WARP0) >> 1, c = (uint32_t)(warp - MMA_WARP0) & 1u;
         bool ok = true;
         const uint32_t acts_addr = smem_u32(acts_res);
-        const uint32_t a_buf = tmem + TM_A + g * TM_A_STRIDE, d_buf = tmem + TM_D + g * TM_D_STRIDE;
-        uint32_t hc = 0;   // running half count of the group
+        const uint32_t a_buf = tmem + TM_A + g * TM_A_STRIDE, d_buf = tmem + TM_D + g * TM_D_STRIDE + 32 * c;
+        uint32_t uses = 0;   // how often this warp's half buffer has been used
         int kb_e = (int)g % n_kb;   // e % n_kb, kept by addition
         const int kb_step = 2 % n_kb;
         for (int e = (int)g; e < n_it && ok; e += 2) {
@@ -262,22 +281,21 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
             const uint64_t bdesc = smem_desc(chunk, 512, 128), mdesc = smem_desc(chunk + TS_BMIN_OFF, 768, 128);
             const uint32_t b_lo = (uint32_t)bdesc, b_hi = (uint32_t)(bdesc >> 32);
 #pragma unroll
-            for (int h = 0; h < HALVES; ++h, ++hc) {
-                const uint32_t hb = hc & 1;
-                if (ok) ok = mbar_wait_warp(&a_ready[2 * g + hb], (hc >> 1) & 1, p.err, DEV_ERR_WAIT_FULL);
+            for (int h2 = 0; h2 < HALVES / 2; ++h2, ++uses) {
+                const int h = 2 * h2 + (int)c;   // this warp's half; the unrolled code below needs it as a constant: see the switch on c
+                if (ok) {
+                    ok = mbar_wait_warp(&a_ready[2 * g + c], uses & 1, p.err, DEV_ERR_WAIT_FULL);
+                }
                 if (ok) {
                     fence_after_sync();
                     if (elect_one()) {
-#pragma unroll
-                        for (int jj = 0; jj < 8; ++jj) {
-                            if (h == 0 && jj == 0) mma_ts<false>(d_buf, a_buf + F::a_col(h, jj), b_lo + F::b_slice(h, jj) * 64u, b_hi, IDESC_MAIN);
-                            else mma_ts<true>(d_buf, a_buf + F::a_col(h, jj), b_lo + F::b_slice(h, jj) * 64u, b_hi, IDESC_MAIN);
-                        }
+                        if (c == 0) issue_half<F, 0>(h2, d_buf, a_buf, b_lo, b_hi, IDESC_MAIN);
+                        else issue_half<F, 1>(h2, d_buf, a_buf, b_lo, b_hi, IDESC_MAIN);
                         if (F::HAS_MIN && h == HALVES - 1)   // every half has stored its column of the min operand by now
                             mma_ts<false>(tmem + TM_DM + g * TM_DM_STRIDE, tmem + TM_AM + g * TM_AM_STRIDE, (uint32_t)mdesc, (uint32_t)(mdesc >> 32),
                                           IDESC_MIN);
-                        mma_commit(&a_free[2 * g + hb]);
-                        if (h == HALVES - 1) mma_commit(&d_ready[g]);
+                        mma_commit(&a_free[2 * g + c]);
+                        if (h2 == HALVES / 2 - 1) mma_commit(&d_ready[g]);   // this warp's share of the entry; the barrier counts both warps
                     }
                     __syncwarp();
                 }
@@ -333,7 +351,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
             }
         }
         if (!ok) abort_flag = 1;
-    } else if (warp < DRAIN_WARP0 + DRAIN_WARPS) {
+    } else {
         // ------------------------------ draining warps ------------------------------
         pdl_wait();
         const int dtid = threadIdx.x - DRAIN_WARP0 * 32;   // 0..127 = weight row of the tile = tensor-memory lane
@@ -373,8 +391,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
             float t[MAX_ROWS], mn[MAX_ROWS];
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {   // tokens 8 hf .. 8 hf + 7
-                float v[16];
-                tmem_ld16(tm_l + TM_D + a * TM_D_STRIDE + 16 * hf, v);   // columns 2 tok + plane
+                float ve[16], vo[16];
+                tmem_ld16(tm_l + TM_D + a * TM_D_STRIDE + 16 * hf, ve);        // even MMA steps: columns 2 tok + plane
+                tmem_ld16(tm_l + TM_D + a * TM_D_STRIDE + 32 + 16 * hf, vo);   // odd MMA steps
                 if (F::HAS_MIN) {
                     float s0[8], s1[8], s2[8];   // 8 tokens x 3 planes, token j = flattened columns 3j .. 3j + 2
                     tmem_ld8(tm_l + TM_DM + a * TM_DM_STRIDE + 24 * hf, s0);
@@ -388,7 +407,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
                     wait_ld();
                 }
 #pragma unroll
-                for (int j = 0; j < 8; ++j) t[8 * hf + j] = v[2 * j] + v[2 * j + 1];
+                for (int j = 0; j < 8; ++j) t[8 * hf + j] = (ve[2 * j] + ve[2 * j + 1]) + (vo[2 * j] + vo[2 * j + 1]);
             }
             fence_before_sync();
             __syncwarp();

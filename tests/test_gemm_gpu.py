@@ -215,3 +215,20 @@ def test_config1_pipeline_matches_oracle_and_accepts_same_prefix():
     s = np.sort(want, axis=1)
     np.testing.assert_allclose(gap, s[:, -1] - s[:, -2], rtol=0, atol=1e-4)
     pipe.close(); w1.close(); w2.close()
+
+
+# A tensor-core accumulation drops what lies below the running sum's last place, so the error of a block of 256 columns grows with the
+# steps that one accumulator takes: some 2^-25 of the sum a step on average, more where the K-quants' products exceed the result by
+# the min term.  Eight steps in each of two accumulators: 3.5e-7 / 4.1e-7 (Q4_K, 16 and 4 blocks), 3.6e-7 / 4.6e-7 (Q5_K), 2.9e-7 (Q6_K),
+# 1.6e-7 (Q8_0) of the result; sixteen in one: 5.8e-7 / 6.4e-7, 7.0e-7 / 7.6e-7, 5.1e-7, 2.8e-7.  The bounds lie between.
+@pytest.mark.parametrize("dtype,bound", [(orc.Q4_K, 5.0e-7), (orc.Q5_K, 5.8e-7), (orc.Q6_K, 4.0e-7), (orc.Q8_0, 2.2e-7)])
+@pytest.mark.parametrize("n_in,n_out", [(4096, 2048), (1024, 4096)])
+def test_few_row_sums_against_float64(dtype, bound, n_in, n_out):
+    _, _, _, ptr, n_bytes = pkg.synth_tensor("w", dtype, n_in, n_out, 7, 0.02)
+    raw = pkg.device_to_host(ptr, n_bytes)
+    pkg.device_free(ptr)
+    m = pkg.QMatrix(dtype, n_in, n_out, raw)
+    x = np.random.default_rng(0).standard_normal((16, n_in)).astype(np.float32)
+    want = x.astype(np.float64) @ m.dequant().astype(np.float64).T
+    assert np.linalg.norm(m.matmul(x) - want) < bound * np.linalg.norm(want)
+    m.close()
