@@ -123,6 +123,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, i
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     return mbar_wait_warp_slow(bar, parity, err, code);
 }
+// The same for a warp that holds too many registers for a call.
+__device__ __forceinline__ bool mbar_wait_warp_inline(uint64_t* bar, uint32_t parity, int* err, int code) {
+    for (uint32_t it = 0; it < kWaitPolls; ++it)
+        if (__all_sync(0xffffffffu, it < 8 ? mbar_try_wait(bar, parity) : mbar_try_wait_for(bar, parity, kWaitSleepNs))) return true;
+    atomicCAS(err, 0, code);
+    return false;
+}
 // The same for a role that is one thread.
 static __device__ __noinline__ bool mbar_wait_one_slow(uint64_t* bar, uint32_t parity, int* err, int code) {
     for (int it = 0; it < 32; ++it)
