@@ -491,28 +491,47 @@ static dfl_status launch_rows(cudaStream_t st, const AttnGeom& g, const float* q
 bool attn_rows_supported(const AttnGeom& g, int kv_mode) {
     return kv_mode == KV_F16_TILED || attn_tc_supported(g, kv_mode != KV_F32_ROWS) || ((g.hd == 128 || g.hd == 256) && g.n_q / g.n_kv <= ROWS_QUERIES);
 }
-uint64_t attn_rows_partials_floats(const AttnGeom& g, int n_rows) {
-    return (uint64_t)((n_rows + MAX_ROWS - 1) / MAX_ROWS) * 2 * g.n_q * MAX_ROWS * (g.hd + 2);
+// Rows of a prompt pass that the tcgen05 kernel takes at a time: it leaves two records per query and span, as in the verify pass (one sum over a
+// long context would be hundreds of tensor-core steps long, each of which drops what lies below its last place: 12 000 positions,
+// the output short by 7e-6 of itself against 1.3e-6), 9.6 MB per 16 rows at 8 KV heads.
+constexpr int T5_ROWS = 128;
+uint64_t attn_rows_partials_floats(const AttnGeom& g, int n_rows, int kv_mode) {
+    const bool tiled = kv_mode == KV_F16_TILED;
+    const int rows = tiled && n_rows > T5_ROWS ? T5_ROWS : n_rows;
+    const uint64_t records = tiled ? 2ull * attn_t5_max_spans(g) : 1;
+    return (uint64_t)((rows + MAX_ROWS - 1) / MAX_ROWS) * records * g.n_q * MAX_ROWS * (g.hd + 2);
 }
-// Every 16-row block of a prompt pass in one launch.  A block's CTA walks all its positions (one span), so that there are
-// one or two records per query to merge and enough CTAs (row blocks x KV heads) for the chip.
 dfl_status launch_attn_rows(cudaStream_t st, const AttnGeom& g, const float* q_rot, const float* gate, const void* k_cache, const void* v_cache,
-                            int kv_mode, uint32_t start, int n_rows, float* partials, float* out_f32, int* err) {
-    constexpr int ALL = 1 << 24;   // chunks per span: more than any cache holds
+                            int kv_mode, uint32_t start, int n_rows, float* partials, float* out_f32, int* err, uint32_t kv_capacity) {
     const bool tiled = kv_mode == KV_F16_TILED, kv_f16 = kv_mode != KV_F32_ROWS;
+    auto post = [&](uint32_t first, int rows, int pos_per_span, int recs_per_span, int n_spans) -> dfl_status {
+        const uint64_t off = (uint64_t)(first - start) * g.n_q * g.hd;
+        launch_k(g.hd == 128 ? attn_post_kernel<128> : attn_post_kernel<256>, dim3((unsigned)((g.n_q + POST_HEADS - 1) / POST_HEADS), (unsigned)rows), dim3(32 * POST_HEADS),
+                 0, st, g, partials, pos_per_span, recs_per_span, gate ? gate + off : nullptr, first, nullptr, 0, out_f32 + off, err, n_spans);
+        count_launch();
+        DFL_CUDA(cudaGetLastError());
+        return DFL_OK;
+    };
+    if (tiled) {
+        const int cps = attn_t5_chunks_per_span(g, kv_capacity);
+        for (int r = 0; r < n_rows; r += T5_ROWS) {
+            const int rows = n_rows - r < T5_ROWS ? n_rows - r : T5_ROWS;
+            const uint32_t first = start + (uint32_t)r;
+            const int n_chunks = (int)((first + (uint32_t)rows + KV_TILE_KEYS - 1) / KV_TILE_KEYS), n_spans = (n_chunks + cps - 1) / cps;
+            DFL_CHECK(launch_attn_t5(st, g, q_rot + (uint64_t)r * g.n_q * g.hd, k_cache, v_cache, first, rows, partials, cps, err));
+            DFL_CHECK(post(first, rows, cps * KV_TILE_KEYS, 2, n_spans));
+        }
+        return DFL_OK;
+    }
+    // one record per query: a CTA walks all positions of its rows
     dfl_status s;
-    if (tiled) s = launch_attn_t5(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ALL, err);
-    else if (attn_tc_supported(g, kv_f16)) s = launch_attn_span_tc(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ALL);
+    if (attn_tc_supported(g, kv_f16)) s = launch_attn_span_tc(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ATTN_TC_FOLD);
     else if (g.hd == 128) s = kv_f16 ? launch_rows<__half, 128>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials)
                                      : launch_rows<float, 128>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials);
     else s = kv_f16 ? launch_rows<__half, 256>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials)
                     : launch_rows<float, 256>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials);
     DFL_CHECK(s);
-    launch_k(g.hd == 128 ? attn_post_kernel<128> : attn_post_kernel<256>, dim3((unsigned)((g.n_q + POST_HEADS - 1) / POST_HEADS), (unsigned)n_rows), dim3(32 * POST_HEADS), 0, st, g, partials, 1 << 30,
-             tiled ? 2 : 1, gate, start, nullptr, 0, out_f32, err, 1);
-    count_launch();
-    DFL_CUDA(cudaGetLastError());
-    return DFL_OK;
+    return post(start, n_rows, 1 << 30, 1, 1);
 }
 
 }  // namespace dfl

@@ -99,7 +99,8 @@ attn_t5_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __ha
     const int c_begin = span * chunks_per_span;
     int c_end = (int)((n_pos + KV_TILE_KEYS - 1) / KV_TILE_KEYS);
     if (c_end > c_begin + chunks_per_span) c_end = c_begin + chunks_per_span;
-    const int n_c = c_end - c_begin;   // >= 1 by the launch geometry
+    const int n_c = c_end - c_begin;
+    if (n_c <= 0) return;   // a span that only later rows of the launch reach; nothing has been set up yet
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < T5_SLOTS; ++i) {
@@ -695,6 +696,8 @@ int attn_t5_chunks_per_span(const AttnGeom& g, uint32_t kv_capacity) {
     if (b < 1) b = 1;
     return (int)b;
 }
+
+int attn_t5_max_spans(const AttnGeom& g) { return sm_count() / g.n_kv > 0 ? sm_count() / g.n_kv : 1; }
 
 dfl_status launch_attn_t5(cudaStream_t st, const AttnGeom& g, const float* q_rot, const void* k_cache, const void* v_cache, uint32_t start,
                           int n_rows, float* partials, int chunks_per_span, int* err) {

@@ -60,10 +60,15 @@ __device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, b
 }
 }  // namespace
 
+// FOLD (prompt passes: blockIdx.z = 16-row block, one span over all positions): every chunk is a span of its own whose record is merged
+// at once, in registers.  Carried on through the chunks, the output of a long prompt would be one sum of hundreds of
+// tensor-core steps, each of which drops what lies below its last place, and the weights would be rounded to f16 against a maximum that few
+// of them reach (3000 positions: 1.57e-4 from the float64 attention against 1.31e-4 chunk by chunk, the sum short by 3.8e-6 of itself
+// against 0.5e-6).
+template <bool FOLD>
 __global__ void __launch_bounds__(128) attn_span_tc_kernel(AttnGeom g, const float* q_rot, const __half* k_cache, const __half* v_cache,
                                                            uint32_t start, int n_rows, float* partials, int chunks_per_span) {
-    // blockIdx.z: 16-row block of a prompt pass (one block in a verify pass); the later, longer ones start first
-    if (gridDim.z > 1) {
+    if (FOLD) {   // the later, longer blocks start first
         const uint32_t blk = gridDim.z - 1 - blockIdx.z;
         start += blk * MAX_ROWS;
         n_rows = min(n_rows - (int)blk * MAX_ROWS, MAX_ROWS);
@@ -186,8 +191,9 @@ __global__ void __launch_bounds__(128) attn_span_tc_kernel(AttnGeom g, const flo
         mc1 = fmaxf(mc1, __shfl_xor_sync(0xffffffffu, mc1, 1));
         mc1 = fmaxf(mc1, __shfl_xor_sync(0xffffffffu, mc1, 2));
         const float mn0 = fmaxf(m0, mc0), mn1 = fmaxf(m1, mc1);
-        const float ms0 = mn0 > -INFINITY ? mn0 : 0.f, ms1 = mn1 > -INFINITY ? mn1 : 0.f;   // exp2(-inf - ms) = 0, never NaN
-        const float a0 = ex2(m0 - ms0), a1 = ex2(m1 - ms1);
+        // the maximum that the weights refer to: the chunk's own or the running one
+        const float mw0 = FOLD ? mc0 : mn0, mw1 = FOLD ? mc1 : mn1;
+        const float ms0 = mw0 > -INFINITY ? mw0 : 0.f, ms1 = mw1 > -INFINITY ? mw1 : 0.f;   // exp2(-inf - ms) = 0, never NaN
         float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt)
@@ -202,25 +208,47 @@ __global__ void __launch_bounds__(128) attn_span_tc_kernel(AttnGeom g, const flo
         sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
         sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1);
         sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
+        const float mg0 = mn0 > -INFINITY ? mn0 : 0.f, mg1 = mn1 > -INFINITY ? mn1 : 0.f;
+        const float a0 = ex2(m0 - mg0), a1 = ex2(m1 - mg1);                 // what the sums so far are scaled with
+        const float f0 = FOLD ? ex2(mc0 - mg0) : 1.f, f1 = FOLD ? ex2(mc1 - mg1) : 1.f;   // and the chunk's own
         m0 = mn0; m1 = mn1;
-        l0 = fmaf(l0, a0, sum0);
-        l1 = fmaf(l1, a1, sum1);
+        l0 = FOLD ? fmaf(sum0, f0, l0 * a0) : fmaf(l0, a0, sum0);
+        l1 = FOLD ? fmaf(sum1, f1, l1 * a1) : fmaf(l1, a1, sum1);
         // ---- O = O * alpha + P V ----
-#pragma unroll
-        for (int nt = 0; nt < 16; ++nt) { o[nt][0] *= a0; o[nt][1] *= a0; o[nt][2] *= a1; o[nt][3] *= a1; }
+        uint32_t h[ATTN_CHUNK / 16][4];   // A fragment of keys 16 kk .. 16 kk + 15 = score tiles 2 kk (k 0-7) and 2 kk + 1 (k 8-15)
 #pragma unroll
         for (int kk = 0; kk < ATTN_CHUNK / 16; ++kk) {
-            // A fragment of keys 16 kk .. 16 kk + 15 = score tiles 2 kk (k 0-7) and 2 kk + 1 (k 8-15)
-            const uint32_t h0 = pack_h2(s[2 * kk][0], s[2 * kk][1]), h1 = pack_h2(s[2 * kk][2], s[2 * kk][3]);
-            const uint32_t h2 = pack_h2(s[2 * kk + 1][0], s[2 * kk + 1][1]), h3 = pack_h2(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+            h[kk][0] = pack_h2(s[2 * kk][0], s[2 * kk][1]);
+            h[kk][1] = pack_h2(s[2 * kk][2], s[2 * kk][3]);
+            h[kk][2] = pack_h2(s[2 * kk + 1][0], s[2 * kk + 1][1]);
+            h[kk][3] = pack_h2(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+        }
+        // two 8-wide dim tiles per ldmatrix.x4; lanes 0-15: keys 16 kk + lane of dims 16 np .. + 7; lanes 16-31: the same keys of dims 16 np + 8 .. + 15
+        auto pv = [&](int kk, int np, float(&x)[4], float(&y)[4]) {
+            uint32_t b[4];
+            ldmatrix_x4_trans(b, vs + (16 * kk + (lane & 15)) * TC_PITCH + 16 * np + 8 * (lane >> 4));
+            mma16816(x, h[kk][0], h[kk][1], h[kk][2], h[kk][3], b[0], b[1]);
+            mma16816(y, h[kk][0], h[kk][1], h[kk][2], h[kk][3], b[2], b[3]);
+        };
+        if (FOLD) {
 #pragma unroll
-            for (int np = 0; np < 8; ++np) {   // two 8-wide dim tiles per ldmatrix.x4
-                // lanes 0-15: keys 16 kk + lane of dims 16 np .. + 7; lanes 16-31: the same keys of dims 16 np + 8 .. + 15
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, vs + (16 * kk + (lane & 15)) * TC_PITCH + 16 * np + 8 * (lane >> 4));
-                mma16816(o[2 * np], h0, h1, h2, h3, b[0], b[1]);
-                mma16816(o[2 * np + 1], h0, h1, h2, h3, b[2], b[3]);
+            for (int np = 0; np < 8; ++np) {
+                float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int kk = 0; kk < ATTN_CHUNK / 16; ++kk) pv(kk, np, x, y);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    o[2 * np][j] = fmaf(x[j], j < 2 ? f0 : f1, o[2 * np][j] * (j < 2 ? a0 : a1));
+                    o[2 * np + 1][j] = fmaf(y[j], j < 2 ? f0 : f1, o[2 * np + 1][j] * (j < 2 ? a0 : a1));
+                }
             }
+        } else {
+#pragma unroll
+            for (int nt = 0; nt < 16; ++nt) { o[nt][0] *= a0; o[nt][1] *= a0; o[nt][2] *= a1; o[nt][3] *= a1; }
+#pragma unroll
+            for (int kk = 0; kk < ATTN_CHUNK / 16; ++kk)
+#pragma unroll
+                for (int np = 0; np < 8; ++np) pv(kk, np, o[2 * np], o[2 * np + 1]);
         }
     }
     // ---- one record per (span, kv head, query): [m, l, O[128]], m back in the natural-log domain ----
@@ -498,15 +526,18 @@ int attn_tc_chunks_per_span(const AttnGeom& g, uint32_t kv_capacity) {
 
 dfl_status launch_attn_span_tc(cudaStream_t st, const AttnGeom& g, const float* q_rot, const void* k_cache, const void* v_cache,
                                uint32_t start, int n_rows, float* partials, int chunks_per_span) {
+    const bool fold = chunks_per_span == ATTN_TC_FOLD;
     static bool set = false;
     if (!set) {
-        DFL_CUDA(cudaFuncSetAttribute(attn_span_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
+        DFL_CUDA(cudaFuncSetAttribute(attn_span_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
+        DFL_CUDA(cudaFuncSetAttribute(attn_span_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
         set = true;
     }
     const int n_chunks = (int)((start + (uint32_t)n_rows + ATTN_CHUNK - 1) / ATTN_CHUNK);
     const int n_spans = (n_chunks + chunks_per_span - 1) / chunks_per_span;
-    launch_k(attn_span_tc_kernel, dim3((unsigned)n_spans, (unsigned)g.n_kv, (unsigned)((n_rows + MAX_ROWS - 1) / MAX_ROWS)), dim3(128), (size_t)TC_SMEM, st, g, q_rot,
-              reinterpret_cast<const __half*>(k_cache), reinterpret_cast<const __half*>(v_cache), start, n_rows, partials, chunks_per_span);
+    launch_k(fold ? attn_span_tc_kernel<true> : attn_span_tc_kernel<false>, dim3((unsigned)n_spans, (unsigned)g.n_kv, fold ? (unsigned)((n_rows + MAX_ROWS - 1) / MAX_ROWS) : 1u),
+             dim3(128), (size_t)TC_SMEM, st, g, q_rot, reinterpret_cast<const __half*>(k_cache), reinterpret_cast<const __half*>(v_cache), start, n_rows, partials,
+             chunks_per_span);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

@@ -66,7 +66,7 @@ dfl_status dfl_prefill(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
         // More rows than a packed block: one many-row pass over up to PROMPT_ROWS of them.  A remainder that fits a packed block
         // takes the packed path, which is then the cheaper one (a many-row pass pays for whole tiles of 128 rows).
         // So does every block when there is no memory for the pass's workspace: the packed path needs none.
-        if (many && n - off > MAX_ROWS && prompt_reserve(m, sc, (uint32_t)std::min<uint64_t>(PROMPT_ROWS, n - off)) != DFL_OK) many = false;
+        if (many && n - off > MAX_ROWS && prompt_reserve(m, s, sc, (uint32_t)std::min<uint64_t>(PROMPT_ROWS, n - off)) != DFL_OK) many = false;
         const bool big = many && n - off > MAX_ROWS;
         const uint32_t nb = (uint32_t)std::min<uint64_t>(big ? PROMPT_ROWS : bs, n - off);
         const bool last = off + nb == n, head = last && last_logits_host != nullptr;

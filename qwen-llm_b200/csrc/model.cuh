@@ -221,7 +221,7 @@ namespace dfl {
 // as a packed pass over the last `last_rows` rows would
 bool prompt_supported(const dfl_model* m);
 constexpr uint32_t PROMPT_ROWS = 512;
-dfl_status prompt_reserve(const dfl_model* m, dfl_scratch* sc, uint32_t n);   // the workspace of a pass of n rows, before anything is queued
+dfl_status prompt_reserve(const dfl_model* m, const dfl_session* s, dfl_scratch* sc, uint32_t n);   // the workspace of a pass of n rows, before anything is queued
 dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids, const int32_t* tokens,
                        uint32_t n, uint32_t start, uint32_t last_rows, bool want_head);
 const float* prompt_capture(const dfl_scratch* sc);

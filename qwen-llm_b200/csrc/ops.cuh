@@ -250,14 +250,16 @@ dfl_status launch_attn_front(cudaStream_t st, const AttnGeom& g, bool gated, con
 dfl_status launch_attn_verify(cudaStream_t st, const AttnGeom& g, const float* q_rot, const float* gate, const void* k_cache,
                               const void* v_cache, int kv_mode, uint32_t start, int n_rows, float* partials, uint8_t* acts,
                               int act_layout, float* out_f32, int* err, uint32_t kv_capacity = 0);
-// the same for all rows of a prompt pass at once (fp16 caches of 128-wide heads in groups of four)
+// The same for the rows of a prompt pass, [rows][n_q hd] f32 out (every cache storage; groups of up to 32 query heads per KV head).
+// `partials` holds attn_rows_partials_floats(g, n_rows, kv_mode).
 bool attn_rows_supported(const AttnGeom& g, int kv_mode);
-uint64_t attn_rows_partials_floats(const AttnGeom& g, int n_rows);
+uint64_t attn_rows_partials_floats(const AttnGeom& g, int n_rows, int kv_mode);
 dfl_status launch_attn_rows(cudaStream_t st, const AttnGeom& g, const float* q_rot, const float* gate, const void* k_cache, const void* v_cache,
-                            int kv_mode, uint32_t start, int n_rows, float* partials, float* out_f32, int* err);
+                            int kv_mode, uint32_t start, int n_rows, float* partials, float* out_f32, int* err, uint32_t kv_capacity);
 // tcgen05 span kernel over a tiled fp16 cache (attn_t5.cu) and the conversions between that cache and position-major rows
 bool attn_t5_supported(const AttnGeom& g, bool kv_f16);
 int attn_t5_chunks_per_span(const AttnGeom& g, uint32_t kv_capacity);
+int attn_t5_max_spans(const AttnGeom& g);   // over all capacities
 dfl_status launch_attn_t5(cudaStream_t st, const AttnGeom& g, const float* q_rot, const void* k_cache, const void* v_cache, uint32_t start,
                           int n_rows, float* partials, int chunks_per_span, int* err);
 // rows of logits ordered for the host sampler (sortrows.cu)
@@ -281,6 +283,7 @@ dfl_status launch_dattn_span_tc(cudaStream_t st, const AttnGeom& g, const float*
                                 const uint32_t* pos_ctx, int ctx_begin, int n_ctx, const float* k_noise, const float* v_noise,
                                 uint32_t noise_start, int n_rows, bool causal, uint32_t window, float* partials, uint32_t ctx_capacity,
                                 int* n_spans_out);
+constexpr int ATTN_TC_FOLD = 1 << 24;   // as chunks_per_span: all positions in one span, whose chunks are merged as they come (prompt passes)
 dfl_status launch_attn_span_tc(cudaStream_t st, const AttnGeom& g, const float* q_rot, const void* k_cache, const void* v_cache,
                                uint32_t start, int n_rows, float* partials, int chunks_per_span);
 uint64_t attn_partials_floats(const AttnGeom& g, uint32_t max_positions);

@@ -10,6 +10,7 @@ namespace dfl {
 
 struct PromptWs {
     uint32_t rows = 0;   // padded rows the buffers hold
+    bool tiled = false;  // attn_part for sessions with a tiled cache too
     float *x = nullptr, *xn = nullptr, *part = nullptr, *sumsq = nullptr, *q_rot = nullptr, *gate = nullptr, *o = nullptr, *attn_part = nullptr;
     float *q_n = nullptr, *k_n = nullptr, *v = nullptr, *ab = nullptr, *conv_pre = nullptr, *capture = nullptr;
     uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_v = nullptr;
@@ -72,8 +73,12 @@ static int tm_splits(const MatGroup& g, int tok_tiles) {
     return gemm_tm_choose_splits(tiles, n, (int)(g.n_in / TILE_K), tok_tiles);
 }
 
-static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) {
-    if (sc->prompt && sc->prompt->rows >= rows) return DFL_OK;
+static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows, bool tiled) {
+    if (sc->prompt && sc->prompt->rows >= rows && (sc->prompt->tiled || !tiled)) return DFL_OK;
+    if (sc->prompt) {   // what it held, it holds on to
+        rows = std::max(rows, sc->prompt->rows);
+        tiled |= sc->prompt->tiled;
+    }
     if (sc->prompt) cudaDeviceSynchronize();
     prompt_ws_free(sc->prompt);
     sc->prompt = nullptr;
@@ -103,7 +108,8 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
         alloc(&w->q_rot, R * q_dim * 4);
         alloc(&w->gate, R * q_dim * 4);
         alloc(&w->o, R * wide * 4);
-        if (m->n_attn) alloc(&w->attn_part, attn_rows_partials_floats(m->attn_geom(), (int)rows) * 4);
+        if (m->n_attn) alloc(&w->attn_part, std::max(attn_rows_partials_floats(m->attn_geom(), (int)rows, KV_F16_ROWS),
+                                                   tiled ? attn_rows_partials_floats(m->attn_geom(), (int)rows, KV_F16_TILED) : 0) * 4);
         alloc(&w->q_n, R * gg.n_k * 128 * 4);
         alloc(&w->k_n, R * gg.n_k * 128 * 4);
         alloc(&w->v, R * v_dim * 4);
@@ -140,6 +146,7 @@ static dfl_status ensure_ws(const dfl_model* m, dfl_scratch* sc, uint32_t rows) 
         return fail(DFL_ERR_OOM, "prompt pass: allocation failed: " + why);
     }
     w->rows = rows;
+    w->tiled = tiled;
     sc->prompt = w;
     return DFL_OK;
 }
@@ -148,13 +155,15 @@ static int token_tiles(uint32_t n) {
     const int tile_tok = gemm_tm_tile_tok((int)n);
     return ((int)n + tile_tok - 1) / tile_tok;
 }
-dfl_status prompt_reserve(const dfl_model* m, dfl_scratch* sc, uint32_t n) { return ensure_ws(m, sc, (uint32_t)(token_tiles(n) * TM_TOK)); }
+dfl_status prompt_reserve(const dfl_model* m, const dfl_session* s, dfl_scratch* sc, uint32_t n) {
+    return ensure_ws(m, sc, (uint32_t)(token_tiles(n) * TM_TOK), s->kv_mode == KV_F16_TILED);
+}
 
 dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, const uint32_t* layer_ids, uint32_t n_ids, const int32_t* tokens,
                        uint32_t n, uint32_t start, uint32_t last_rows, bool want_head) {
     const dfl_arch& a = m->arch;
     const int tile_tok = gemm_tm_tile_tok((int)n), tok_tiles = token_tiles(n), rows_pad = tok_tiles * tile_tok;
-    DFL_CHECK(prompt_reserve(m, sc, n));
+    DFL_CHECK(prompt_reserve(m, s, sc, n));
     PromptWs* w = sc->prompt;
     cudaStream_t st = s->st;
     const uint64_t H = a.hidden_size, F = a.intermediate_size, KH = sc->k_layers * H;
@@ -206,7 +215,8 @@ dfl_status prompt_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             DFL_CHECK(launch_attn_front(st, ag, true, w->part, splits, (int)L.qkv.total_cols, L.q_norm_w, L.k_norm_w, start, (int)n, s->k_cache[ai],
                                         s->v_cache[ai], s->kv_mode, w->q_rot, w->gate, nullptr, -1, rows_pad));
             if (attn_rows_supported(ag, s->kv_mode))
-                DFL_CHECK(launch_attn_rows(st, ag, w->q_rot, w->gate, s->k_cache[ai], s->v_cache[ai], s->kv_mode, start, (int)n, w->attn_part, w->o, s->err));
+                DFL_CHECK(launch_attn_rows(st, ag, w->q_rot, w->gate, s->k_cache[ai], s->v_cache[ai], s->kv_mode, start, (int)n, w->attn_part, w->o, s->err,
+                                           s->kv_capacity));
             else for (uint32_t r = 0; r < n; r += MAX_ROWS)
                 DFL_CHECK(launch_attn_verify(st, ag, w->q_rot + r * q_dim, w->gate + r * q_dim, s->k_cache[ai], s->v_cache[ai], s->kv_mode, start + r,
                                              (int)std::min<uint32_t>(MAX_ROWS, n - r), s->attn_partials, nullptr, m->act_layout, w->o + r * q_dim, s->err,

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 import modelgen
+import orc
 from dflb import pkg
 
 syn = importlib.import_module("qwen-llm_b200.synthetic")
@@ -227,5 +228,37 @@ def test_prompt_pass_is_as_close_as_the_packed_one(routed, n, bound):
     off["kv"] = rel(np.stack([np.concatenate(a.read_kv(0, p)) for p in range(n)]), np.stack([np.concatenate(b.read_kv(0, p)) for p in range(n)]))
     off["state"] = rel(np.stack([np.concatenate(a.read_gdn_state(g)) for g in range(3)]), np.stack([np.concatenate(b.read_gdn_state(g)) for g in range(3)]))
     assert max(off.values()) < bound, off
+    for x in (a, b, sa, sb, gm):
+        x.close()
+
+
+# The attention of a prompt pass keeps to the packed pass's spans (tiled cache) or merges chunk by chunk (row-major cache at the
+# capacities where a packed span is one chunk), so over the same keys and values the two differ by what their queries do, some 1e-6, and
+# by the f16 roundings (weights, the new rows' own keys and values) that this moves: 1.1e-5 to 1.5e-5 of the attention's output on average.
+# One sum over the whole context differed by 1.4e-4 to 2e-4: weights rounded against another maximum, and an output short by what
+# every further tensor-core step drops.
+@pytest.mark.parametrize("n,capacity", [(900, 4096), (3000, 4096), (1500, 16384), (3000, 16384)])
+def test_prompt_attention_is_the_packed_pass_s(n, capacity):
+    arch = syn.arch_9b()
+    arch.n_layer, arch.full_attention_interval, arch.vocab_size, arch.intermediate_size = 1, 1, 8192, 512
+    ents = syn.target_entries(arch, seed=71, device=0)
+    ents = [(nm, d, s, np.zeros(nb, np.uint8) if "ffn_down" in nm else data, nb) for nm, d, s, data, nb in ents]   # a layer of attention alone
+    embd = next(e for e in ents if e[0] == "token_embd.weight")
+    embd = orc.dequant(embd[1], pkg.device_to_host(embd[3], embd[4]), arch.hidden_size * arch.vocab_size).reshape(arch.vocab_size, -1)
+    gm = syn.build_model(arch, ents)
+    syn.free_entries([e for e in ents if isinstance(e[3], int)])
+    ids = np.random.default_rng(n).integers(0, arch.vocab_size, n + 32)
+    a, b = pkg.Session(gm, capacity, True), pkg.Session(gm, capacity, True)
+    sa, sb = pkg.Scratch(gm, 16, 1), pkg.Scratch(gm, 16, 1)
+    pkg.prefill(gm, a, sa, [0], ids[:n], 0)
+    pkg.session_restore_snapshot(gm, b, None, pkg.session_snapshot(gm, a, None))
+    got = pkg.prefill(gm, a, sa, [0], ids[n:], n, want_hidden=True)[1][:, 0]
+    rows = []
+    for off in (n, n + 16):
+        pkg.packed_verify(gm, b, sb, [0], ids[off:off + 16], off)
+        rows.append(sb.read_capture(16)[:, 0])
+    rows = np.concatenate(rows).astype(np.float64)
+    off = np.linalg.norm(got - rows, axis=1) / np.linalg.norm(rows - embd[ids[n:]], axis=1)
+    assert off.mean() < 4e-5 and off.max() < 1e-4, off
     for x in (a, b, sa, sb, gm):
         x.close()
