@@ -262,3 +262,16 @@ def test_prompt_attention_is_the_packed_pass_s(n, capacity):
     assert off.mean() < 4e-5 and off.max() < 1e-4, off
     for x in (a, b, sa, sb, gm):
         x.close()
+
+
+@pytest.mark.parametrize("n", [513, 540, 600])
+def test_prompt_of_several_passes_at_routed_widths(n):
+    # one pass of 512 rows (every expert chosen, segments of all sizes), then a packed remainder or a second pass
+    arch = syn.arch_35b_a3b()
+    arch.n_layer, arch.vocab_size = 2, 8192
+    arch.full_attention_interval = 2
+    ents = syn.target_entries(arch, seed=53, device=0)
+    gm = syn.build_model(arch, ents)
+    syn.free_entries(ents)
+    _check(arch, gm, n, 0, [0, 1])
+    gm.close()

@@ -1,12 +1,15 @@
 """Session snapshots: a session restored from a snapshot continues bitwise like the session it was taken from
 (the reference's guarantee for SessionSnapshot, metal_forward/session.rs:57-62), the drafter's context tail follows its
 capture-window rule (metal_dflash.rs:103-140), and mismatching snapshots are refused."""
+import importlib
+
 import numpy as np
 import pytest
 
 import modelgen
 from dflb import pkg
 
+syn = importlib.import_module("qwen-llm_b200.synthetic")
 pytestmark = pytest.mark.gpu
 
 
@@ -86,3 +89,60 @@ def test_restored_session_continues_bitwise(world, all_swa):
     assert fresh.kv_n_pos == 0
     gd3.close()
     gd.close()
+
+
+@pytest.fixture(scope="module")
+def wide():
+    arch = syn.arch_9b()
+    arch.n_layer, arch.vocab_size = 4, 8192
+    ents = syn.target_entries(arch, seed=61, device=0)
+    gm = syn.build_model(arch, ents)
+    syn.free_entries(ents)
+    cfg = syn.dflash_config_9b(arch)
+    cfg.n_layer, cfg.n_target_layers = 2, 2
+    cfg.layer_is_swa[0], cfg.layer_is_swa[1], cfg.swa_window = 1, 0, 256
+    cfg.target_layer_ids[0], cfg.target_layer_ids[1] = 1, 3
+    dents = syn.drafter_entries(arch, cfg, device=0)
+    gd = syn.build_drafter(gm, cfg, dents)
+    syn.free_entries(dents)
+    yield arch, gm, gd
+    gd.close(); gm.close()
+
+
+# Above 4 MiB a restore runs through the ring of pinned slots (1 MiB each, sixteen): rows of a chunk and more per layer, the tiled
+# layouts behind each upload, sections that end inside a chunk.  A drafter session of 16 384 columns keeps its tiled shadow too.
+@pytest.mark.parametrize("taken,restored", [(16384, 16384), (16384, 4096), (4096, 16384), (4096, 4096)])
+@pytest.mark.parametrize("n", [301, 1100])
+def test_a_long_snapshot_through_the_ring_continues_bitwise(wide, taken, restored, n):
+    arch, gm, gd = wide
+    ids = gd.layer_ids()
+    rng = np.random.default_rng(n)
+    prompt, block = rng.integers(0, arch.vocab_size, n), rng.integers(0, arch.vocab_size, 16)
+
+    def go_on(sess, scr, ds):
+        drafts, dl = ds.draft_block(5, n, want_logits=True)
+        logits = pkg.packed_verify(gm, sess, scr, ids, block, n, want_logits=True)[2]
+        kv = np.concatenate([np.concatenate(sess.read_kv(0, p)) for p in (0, 127, 128, n - 1)])
+        return [drafts.tobytes(), dl.tobytes(), logits.tobytes(), kv.tobytes()] + [np.concatenate(sess.read_gdn_state(g)).tobytes() for g in range(3)]
+
+    a, sa, da = pkg.Session(gm, taken), pkg.Scratch(gm, 16, len(ids)), pkg.DSession(gd, taken)
+    pkg.prefill(gm, a, sa, ids, prompt, 0, feed_drafter=da)
+    blob = pkg.session_snapshot(gm, a, da)
+    assert blob.nbytes > (8 << 20)
+    b, sb, db = pkg.Session(gm, restored), pkg.Scratch(gm, 16, len(ids)), pkg.DSession(gd, restored)
+    pkg.prefill(gm, b, sb, ids, prompt[::-1][:200], 0, feed_drafter=db)     # something else was there
+    for _ in range(2):                                                      # and the ring's memory is used again
+        pkg.session_restore_snapshot(gm, b, db, blob)
+    assert b.kv_n_pos == n and db.ctx_len == n
+    if taken == restored:
+        assert go_on(b, sb, db) == go_on(a, sa, da)
+    else:       # spans follow the capacity, so the comparison is with a session of the same one that holds the same rows
+        c, sc, dc = pkg.Session(gm, restored), pkg.Scratch(gm, 16, len(ids)), pkg.DSession(gd, restored)
+        pkg.session_restore_snapshot(gm, c, dc, pkg.session_snapshot(gm, b, db))
+        again = pkg.session_snapshot(gm, c, dc)
+        assert again.tobytes() == blob.tobytes()
+        assert go_on(c, sc, dc) == go_on(b, sb, db)
+        for x in (c, sc, dc):
+            x.close()
+    for x in (a, sa, da, b, sb, db):
+        x.close()
