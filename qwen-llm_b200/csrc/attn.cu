@@ -525,7 +525,8 @@ dfl_status launch_attn_rows(cudaStream_t st, const AttnGeom& g, const float* q_r
     }
     // one record per query: a CTA walks all positions of its rows
     dfl_status s;
-    if (attn_tc_supported(g, kv_f16)) s = launch_attn_span_tc(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ATTN_TC_FOLD);
+    const char* tc_env = getenv("DFL_ATTN_TC");   // 0: the CUDA-core kernels, as in the verify pass
+    if (attn_tc_supported(g, kv_f16) && !(tc_env && tc_env[0] == '0')) s = launch_attn_span_tc(st, g, q_rot, k_cache, v_cache, start, n_rows, partials, ATTN_TC_FOLD);
     else if (g.hd == 128) s = kv_f16 ? launch_rows<__half, 128>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials)
                                      : launch_rows<float, 128>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials);
     else s = kv_f16 ? launch_rows<__half, 256>(st, g, q_rot, k_cache, v_cache, start, n_rows, partials)

@@ -275,3 +275,19 @@ def test_prompt_of_several_passes_at_routed_widths(n):
     syn.free_entries(ents)
     _check(arch, gm, n, 0, [0, 1])
     gm.close()
+
+
+def test_the_scalar_attention_switch_holds_for_prompts(monkeypatch):
+    arch = modelgen.tiny_arch(n_q_heads=4)          # a group of four: the tensor-core kernel by default
+    gm = pkg.Model(arch, modelgen.target_tensors(arch, seed=3))
+    ids = np.random.default_rng(8).integers(0, arch.vocab_size, 100)
+    out = []
+    for value in (None, "0"):
+        if value is not None:
+            monkeypatch.setenv("DFL_ATTN_TC", value)
+        sess, scr = pkg.Session(gm, 128), pkg.Scratch(gm, 16, 1)
+        out.append(pkg.prefill(gm, sess, scr, [3], ids, 0, want_hidden=True)[1].copy())
+        sess.close(); scr.close()
+    assert out[0].tobytes() != out[1].tobytes()
+    np.testing.assert_allclose(out[0], out[1], rtol=2e-3, atol=2e-3)
+    gm.close()
