@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         const uint32_t b_addr = smem_u32(b_ring), am_addr = smem_u32(smem + T::OFF_AM), s_addr = smem_u32(smem + T::OFF_S);
         uint32_t e = 0, am = 0;   // am = e % N_AM
         uint32_t b_phase = 0;             // bit s: parity of this issuer's next use of slot s
-        uint32_t d_phase = 0, dn = 0;     // bit i: the same for its accumulators; dn = e * UNITS % ND
+        uint32_t d_phase = 0, dn = 0;     // bit i: the same for its accumulators; dn = 2 e % 3, for rings of three
         auto wait = [&](uint64_t* bar, uint32_t parity) {
             ok = mbar_wait_one(bar, parity, p.err, DEV_ERR_WAIT_FULL);
             return ok;

@@ -7,7 +7,6 @@
 #include <functional>
 #include <map>
 #include <string>
-#include <functional>
 #include <vector>
 
 #include "ops.cuh"

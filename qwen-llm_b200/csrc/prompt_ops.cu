@@ -201,8 +201,8 @@ dfl_status launch_tm_small_matmul(cudaStream_t st, const float* w, const float* 
 }
 
 // ---- gated delta net: conv + SiLU + L2 norms over all rows of the pass ---------------------------
-// grid (heads of 128 channels, rows / 16), four warps of four rows each, lane = four channels: gdn_front_tile with the three
-// preceding rows read from the pass's own projection output (or the conv rows of the session for the first rows).
+// grid (heads of 128 channels, rows / 16), four warps of four rows each, lane = four channels; the three rows before a warp's own come
+// from the pass's projection output again (or from the session's conv rows for the first ones).
 __global__ void __launch_bounds__(128) tm_gdn_front_kernel(const TmGdn p) {
     pdl_prologue();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.x;
