@@ -37,7 +37,8 @@ namespace dfl {
 namespace ts {
 
 constexpr int TM_WARPS = 28, TM_THREADS = TM_WARPS * 32;
-constexpr int TM_DRAIN_WARPS = 8, TM_MMA_WARP = 24, TM_W_WARP = 26, TM_B_WARP = 27;   // two MMA warps
+constexpr int TM_GROUP_WARPS = 8, TM_UNPACK_WARPS = 2 * TM_GROUP_WARPS;   // thread = (row = 32 * (warp % 4) + lane, kp2 = (warp / 4) % 2)
+constexpr int TM_DRAIN_WARP0 = 16, TM_DRAIN_WARPS = 8, TM_MMA_WARP = 24, TM_W_WARP = 26, TM_B_WARP = 27;   // two MMA warps
 constexpr int TM_BAR_BYTES = 512;
 // Registers a thread: what the launch gives, and the share of the unpacking and the read-back warps, which hold up to 64 running sums each.
 constexpr int TM_REGS = 72, TM_REGS_UNPACK = 56, TM_REGS_DRAIN = 104;
@@ -127,9 +128,9 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < T::W_STAGES; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], UNPACK_WARPS); }
+        for (int i = 0; i < T::W_STAGES; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], TM_UNPACK_WARPS); }
         for (int i = 0; i < T::NS; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_full[T::NS + i], 1); mbar_init(&b_empty[i], 1); }
-        for (int i = 0; i < 8; ++i) mbar_init(&a_ready[i], GROUP_WARPS);
+        for (int i = 0; i < 8; ++i) mbar_init(&a_ready[i], TM_GROUP_WARPS);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&s_full[i], 1);
             mbar_init(&s_empty[i], 1);
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
             }
         }
         __syncwarp();
-    } else if (warp < UNPACK_WARPS) {
+    } else if (warp < TM_UNPACK_WARPS) {
         // ------------------------------ unpack ------------------------------
         if constexpr (CAP != TM_SEG) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TM_REGS_UNPACK));
         const int g = warp >> 3, q4 = warp & 3, kp2 = (warp >> 2) & 1;
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                 const uint8_t* st = w_ring + s * T::W_STAGE;
 #pragma unroll
                 for (int u = 0; u < T::USES; ++u, ++use) {
-                    uint32_t r[32], am[8];
+                    uint32_t r[32], am = 0u;
                     UnitScales us{0.f, 0.f};
                     TmScale sc{0.f, 0.f, 1.f};
                     if constexpr (T::MIN) {
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
                     if (T::MIN) {
                         tmem_st32(a_dst + 32 * kp2, r);
                         // the min operand of this thread's two sub-blocks, k = 2 kp and 2 kp + 1 (hi) and 8 further (lo)
-                        const float2 m = __half22float2(*reinterpret_cast<const __half2*>(&am[0]));
+                        const float2 m = __half22float2(*reinterpret_cast<const __half2*>(&am));
                         const float f0 = -sc.ratio * m.x, f1 = -sc.ratio * m.y;
                         const __half2 hi = __floats2half2_rn(f0, f1);
                         const float2 back = __half22float2(hi);
@@ -400,8 +401,8 @@ __global__ void __launch_bounds__(TM_THREADS, 1) gemm_tm_kernel(const TmParams p
         // ------------------------------ read-back ------------------------------
         if constexpr (CAP != TM_SEG) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TM_REGS_DRAIN));
         pdl_wait();
-        const int row = (threadIdx.x - DRAIN_WARP0 * 32) & 127;   // weight row of the tile = tensor-memory lane
-        const int half = (warp - DRAIN_WARP0) >> 2;   // takes the first or the second half of the tile's 16-token columns
+        const int row = (threadIdx.x - TM_DRAIN_WARP0 * 32) & 127;   // weight row of the tile = tensor-memory lane
+        const int half = (warp - TM_DRAIN_WARP0) >> 2;   // takes the first or the second half of the tile's 16-token columns
         const uint32_t tm_l = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
         constexpr int NC = (CAP / 16 + 1) / 2;        // 16-token pieces that a thread holds at most
         float acc[NC][16];                            // their running sums over the column blocks

@@ -235,16 +235,7 @@ dfl_status launch_prep_acts_ts(cudaStream_t st, const float* x, int ld, int n_ro
 // ---------------------------------------------------------------------------------------------
 namespace ts {
 
-constexpr int GROUP_WARPS = 8;                          // unpacking warps per group; thread = (row = 32 * (warp % 4) + lane, kp2 = (warp / 4) % 2)
-constexpr int UNPACK_WARPS = 2 * GROUP_WARPS;           // two groups that take the entries alternately, so that their phases interleave
-constexpr int DRAIN_WARP0 = 16, DRAIN_WARPS = 4;        // thread = weight row; warp % 4 = its quarter of the tensor-memory lanes
-constexpr int MMA_WARP0 = 20, MMA_WARPS = 4;            // warp 20 + 2 g + c issues the MMAs of group g's halves h with h % 2 == c
-constexpr int PRODUCER_WARP = 24;
-constexpr int THREADS = 25 * 32;                        // 800
-#ifndef DFL_TS_KC
-#define DFL_TS_KC 6
-#endif
-constexpr int KC = DFL_TS_KC;                           // column blocks whose activations stay resident
+constexpr int KC_MAX = 6;                               // column blocks whose activations stay resident, at most
 
 // tensor-memory columns (32-bit each, 128 lanes), everything once per group: a 128-column A buffer (256 f16 per row)
 // written and consumed in two halves, two 32-column accumulators (even / odd MMA steps), the 8-column A operand of the
@@ -268,6 +259,12 @@ __device__ __forceinline__ uint32_t h2fma(uint32_t a, uint32_t b, uint32_t c) {
     asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
     return r;
 }
+// (a & mask) | bits in one instruction: written with operators, half of the unpack's selections came out as two
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xea;" : "=r"(r) : "r"(a), "r"(mask), "r"(bits));
+    return r;
+}
 constexpr uint32_t MAGIC = 0x64006400u;      // half2(1024, 1024): 1024 + small integer in the mantissa
 constexpr uint32_t H2_NEG1024 = 0xe400e400u; // half2(-1024)
 constexpr uint32_t H2_16TH = 0x2c002c00u;    // half2(1/16)
@@ -285,15 +282,14 @@ struct Fmt;
 template <int DT>
 struct FmtK45 {
     static constexpr int STAGE = DT == DFL_Q4_K ? STAGE_Q4_K_TS : STAGE_Q5_K_TS;
-    static constexpr int STAGES = KC == 4 ? (DT == DFL_Q4_K ? 7 : 6) : (DT == DFL_Q4_K ? 6 : 5);
+    __host__ __device__ static constexpr int stages(int) { return DT == DFL_Q4_K ? 6 : 5; }   // ring slots beside kc resident column blocks
     static constexpr int HALVES = 2;
     static constexpr bool HAS_MIN = true;
     // MMA step jj (0..7) of half h multiplies A-buffer columns a_col .. + 8 with 16-column slice b_slice of the block
     __device__ static __forceinline__ uint32_t a_col(int h, int jj) { return (uint32_t)(64 * h + 8 * jj); }
     __device__ static __forceinline__ uint32_t b_slice(int h, int jj) { return (uint32_t)(8 * h + jj); }
     __device__ static __forceinline__ void store(uint32_t buf, int h, int kp2, const uint32_t (&r)[32]) { tmem_st32(buf + 64 * h + 32 * kp2, r); }
-    __device__ static __forceinline__ int min_col(int h, int kp2) { return 2 * h + kp2; }
-    __device__ static __forceinline__ void unpack(const uint8_t* st, int ps, int row, int kp2, uint32_t (&r)[32], uint32_t (&am)[8],
+    __device__ static __forceinline__ void unpack(const uint8_t* st, int ps, int row, int kp2, uint32_t (&r)[32], uint32_t& am,
                                                   UnitScales& us) {
         const int kp = 2 * ps + kp2;
         const uint32_t dd = reinterpret_cast<const uint32_t*>(st)[row];
@@ -311,10 +307,10 @@ struct FmtK45 {
 #pragma unroll
             for (int wi = 0; wi < 8; ++wi) {
                 const uint32_t v = w[wi], v8 = v >> 8;
-                r[2 * wi] = h2fma((v & 0x000f000fu) | MAGIC, cml, cal);
-                r[2 * wi + 1] = h2fma((v8 & 0x000f000fu) | MAGIC, cml, cal);
-                r[16 + 2 * wi] = h2fma((v & 0x00f000f0u) | MAGIC, cmh, cah);
-                r[16 + 2 * wi + 1] = h2fma((v8 & 0x00f000f0u) | MAGIC, cmh, cah);
+                r[2 * wi] = h2fma(and_or(v, 0x000f000fu, MAGIC), cml, cal);
+                r[2 * wi + 1] = h2fma(and_or(v8, 0x000f000fu, MAGIC), cml, cal);
+                r[16 + 2 * wi] = h2fma(and_or(v, 0x00f000f0u, MAGIC), cmh, cah);
+                r[16 + 2 * wi + 1] = h2fma(and_or(v8, 0x00f000f0u, MAGIC), cmh, cah);
             }
         } else {
             const uint4* qh = reinterpret_cast<const uint4*>(st + TSQ5_OFF_QH);
@@ -323,14 +319,14 @@ struct FmtK45 {
 #pragma unroll
             for (int wi = 0; wi < 8; ++wi) {
                 const uint32_t v = w[wi], v8 = v >> 8, t = hw[wi] >> (2 * kp);
-                r[2 * wi] = h2fma((v & 0x000f000fu) | ((t << 4) & 0x00100010u) | MAGIC, cml, cal);
-                r[2 * wi + 1] = h2fma((v8 & 0x000f000fu) | ((t >> 4) & 0x00100010u) | MAGIC, cml, cal);
-                r[16 + 2 * wi] = h2fma((v & 0x00f000f0u) | ((t << 7) & 0x01000100u) | MAGIC, cmh, cah);
-                r[16 + 2 * wi + 1] = h2fma((v8 & 0x00f000f0u) | ((t >> 1) & 0x01000100u) | MAGIC, cmh, cah);
+                r[2 * wi] = h2fma(and_or(t << 4, 0x00100010u, and_or(v, 0x000f000fu, MAGIC)), cml, cal);
+                r[2 * wi + 1] = h2fma(and_or(t >> 4, 0x00100010u, and_or(v8, 0x000f000fu, MAGIC)), cml, cal);
+                r[16 + 2 * wi] = h2fma(and_or(t << 7, 0x01000100u, and_or(v, 0x00f000f0u, MAGIC)), cmh, cah);
+                r[16 + 2 * wi + 1] = h2fma(and_or(t >> 1, 0x01000100u, and_or(v8, 0x00f000f0u, MAGIC)), cmh, cah);
             }
         }
         // column kp of the min-term A operand: the mins of this thread's two sub-blocks
-        am[0] = h2sub(__byte_perm(t, 0x64646464u, 0x4341), MAGIC);
+        am = h2sub(__byte_perm(t, 0x64646464u, 0x4341), MAGIC);
     }
 };
 template <>

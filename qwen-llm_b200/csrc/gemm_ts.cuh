@@ -10,16 +10,16 @@
 //         [kp 4][half 2][row 128][16 B of qs]  (148 bytes a row instead of ggml's 144: byte scales come out with three byte
 //         permutes, ggml's twelve packed bytes cost some twenty shifts and masks per thread and block)
 //   Q5_K: as Q4_K, then [half 2][row 128][16 B of qh]
-//   Q6_K: [128 x 16 B scales i8] [128 x f16 d] [block 8][half 2][row 128][16 B of six-bit codes, one per byte]
+//   Q6_K: [128 x 16 B scales i8] [128 x f16 d] [block 8][half 2][row 128][16 B of q + 128]
 //         (35072 bytes per stage instead of ggml's 26880: see gemm_ts_q6k.cuh)
 //   Q8_0: [128 x 8 f16 d] [block 8][half 2][row 128][16 B of q + 128]
 //
 // Activation chunk per 256 columns (ACT_TS): the canonical K-major, no-swizzle operand layout of
 // tcgen05.mma: core matrices of 8 rows (n) x 16 bytes (8 halfs along k), the four n-groups of a
-// k-core contiguous (128 B apart), k-cores 512 B apart.  n = 2 * token + plane (plane 0 = f16
-// hi, 1 = lo, x = hi + lo).  Column k sits at k-position (k & ~3) + {0, 2, 1, 3}[k & 3], the order
+// k-core contiguous (128 B apart), k-cores 512 B apart.  n = 16 * plane + token (plane 0 = f16
+// hi, 1 = lo, x = hi + lo), so that a read-back thread finds neighbouring tokens of a plane side by side.  Column k sits at k-position (k & ~3) + {0, 2, 1, 3}[k & 3], the order
 // in which the nibble unpack emits its f16 pairs.  After the 16 KiB main operand comes a second,
-// small operand for the K-quant "min" term: S[sub-block j][n2 = 3 * token + plane], the sums of
+// small operand for the K-quant "min" term: S[sub-block j][n2 = 16 * plane + token], the sums of
 // the activations over each 32-column sub-block as an exact three-way f16 split, K padded from 8
 // to 16 with zeros (the second k-core is never written after the buffer was cleared).
 #pragma once
@@ -76,9 +76,9 @@ __device__ __forceinline__ void pack_quad_ts(uint8_t* chunk, int tok, int k, con
         lo[e] = __half_as_ushort(__float2half_rn(f - __half2float(h)));
     }
     // k-positions k + {0, 2, 1, 3}: stored order is v0, v2, v1, v3
-    *reinterpret_cast<uint2*>(chunk + ts_b_offset(2 * tok, k)) =
+    *reinterpret_cast<uint2*>(chunk + ts_b_offset(tok, k)) =
         make_uint2((uint32_t)hi[0] | ((uint32_t)hi[2] << 16), (uint32_t)hi[1] | ((uint32_t)hi[3] << 16));
-    *reinterpret_cast<uint2*>(chunk + ts_b_offset(2 * tok + 1, k)) =
+    *reinterpret_cast<uint2*>(chunk + ts_b_offset(MAX_ROWS + tok, k)) =
         make_uint2((uint32_t)lo[0] | ((uint32_t)lo[2] << 16), (uint32_t)lo[1] | ((uint32_t)lo[3] << 16));
 }
 __device__ __forceinline__ void pack_quad_tsb(uint8_t* chunk, int tok, int k, const float (&v)[4]) {
@@ -105,8 +105,8 @@ __device__ __forceinline__ void pack_subsum_ts(uint8_t* chunk, int tok, int j, f
 #pragma unroll
     for (int pl = 0; pl < 3; ++pl) {
         const __half h = __float2half_rn(f);
-        *reinterpret_cast<__half*>(chunk + ts_bmin_offset(3 * tok + pl, j)) = h;
-        *reinterpret_cast<__half*>(chunk + ts_bmin_offset(3 * tok + pl, j + 8)) = __ushort_as_half((unsigned short)0);  // K padding
+        *reinterpret_cast<__half*>(chunk + ts_bmin_offset(MAX_ROWS * pl + tok, j)) = h;
+        *reinterpret_cast<__half*>(chunk + ts_bmin_offset(MAX_ROWS * pl + tok, j + 8)) = __ushort_as_half((unsigned short)0);  // K padding
         f -= __half2float(h);
     }
 }

@@ -2,8 +2,8 @@
 //
 // CTA = one split (at most KC column blocks, activations resident) x every ctas_per_split-th
 // row tile.  Its work is the sequence of entries e = (tile, column block); the weight stage of
-// entry e travels through ring slot e % STAGES.  The sixteen unpacking warps form two groups of
-// eight that take the entries alternately (group = e & 1), each with its own A buffer,
+// entry e travels through ring slot e % STAGES.  The eight unpacking warps form two groups of
+// four that take the entries alternately (group = e & 1), each with its own A buffer,
 // accumulators and barriers, so that one group's arithmetic fills the time the other spends
 // storing to tensor memory and waiting.  A group unpacks an entry in HALVES steps of 64 A-buffer
 // columns (Q4_K / Q5_K: two halves of 128 weight columns; Q6_K: four of 64, each written as the
@@ -39,18 +39,24 @@ struct Params {
     const int32_t* n_tiles;
     const int32_t* kb_map;     // optional: column blocks to sum over, and how many (device memory)
     const int32_t* n_kb;
-    int main_grid;             // CTAs from here on run the side projection, four outputs each
-    const float *side_w, *side_x;
-    float* side_out;
-    int side_n, side_k, side_rows;
+    int trigger_late;          // let the next kernel start behind the dependency wait instead of at once
+    int wait_last;             // the kernels before were launched so: the inputs are complete, the dependency wait is for the kernels behind
 };
 
+constexpr int FR_GROUP_WARPS = 4;                           // unpacking warps per group; thread = weight row = 32 * (warp % 4) + lane
+constexpr int FR_UNPACK_WARPS = 2 * FR_GROUP_WARPS;         // two groups that take the entries alternately
+constexpr int DRAIN_WARP0 = 8, DRAIN_WARPS = 4;             // thread = weight row; warp % 4 = its quarter of the tensor-memory lanes
+constexpr int MMA_WARP0 = 12, MMA_WARPS = 4;                // warp 12 + 2 g + c issues the MMAs of group g's halves h with h % 2 == c
+constexpr int PRODUCER_WARP = 16;
+// 96 registers, the most that five warps on one scheduler leave.  With 88 a small CTA of the next kernel fits beside a GEMM CTA, but the GEMM lost
+// more (4096 x 24576 Q4_K 15.9 -> 16.4 us) than the early start gave; fifteen warps, two of which issue the MMAs, were 5 % slower.
+constexpr int THREADS = 17 * 32, REGS = 96;
 constexpr int SCL_BYTES = 4 * TILE_R * 8;   // four entries' {d, dmin} per row
 constexpr int BAR_BYTES = 512;              // up to 64 mbarriers
 
-template <int DT>
+template <int DT, int KC>
 constexpr int smem_bytes() {
-    return KC * ACTTS_CHUNK + Fmt<DT>::STAGES * Fmt<DT>::STAGE + SCL_BYTES + BAR_BYTES;
+    return KC * ACTTS_CHUNK + Fmt<DT>::stages(KC) * Fmt<DT>::STAGE + SCL_BYTES + BAR_BYTES;
 }
 
 // named barrier among the draining warps only (every one of them reaches it unconditionally)
@@ -62,7 +68,7 @@ __device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sy
 // that is not needed costs a test.
 __host__ __device__ constexpr bool waits_for_acts(int e, int n_kb) { return e < ((n_kb & 1) ? 2 * n_kb : n_kb); }
 constexpr bool every_first_use_waits() {
-    for (int n_kb = 1; n_kb <= KC; ++n_kb)
+    for (int n_kb = 1; n_kb <= KC_MAX; ++n_kb)
         for (int g = 0; g < 2; ++g)
             for (int kb = 0; kb < n_kb; ++kb)
                 for (int e = g; e < 4 * n_kb; e += 2)   // the group's entries in order, four row tiles
@@ -73,56 +79,6 @@ constexpr bool every_first_use_waits() {
     return true;
 }
 static_assert(every_first_use_waits(), "an MMA warp would read activations that may not have arrived");
-
-// The side projection: this CTA's four outputs over all rows.  24 warps; the even ones take tokens 0 - 7, the odd ones 8 - 15,
-// a thread four columns of every 12 x 128.  Sums over lanes, then warps, in a fixed order.
-__device__ __forceinline__ void side_projection(const Params& p, float* smem) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, o0 = ((int)blockIdx.x - p.main_grid) * 4;
-    const int t0 = (warp & 1) * 8;
-    float v[32];   // [token - t0][output]
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = 0.f;
-    const float* w = p.side_w + (uint64_t)o0 * p.side_k;
-    if (warp < 24)
-        for (int k = (warp >> 1) * 128 + lane * 4; k < p.side_k; k += 12 * 128) {
-            float4 wv[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) wv[j] = *reinterpret_cast<const float4*>(w + (uint64_t)j * p.side_k + k);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (t0 + i >= p.side_rows) continue;
-                const float4 x = __ldcg(reinterpret_cast<const float4*>(p.side_x + (uint64_t)(t0 + i) * p.side_k + k));
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v[4 * i + j] = fmaf(wv[j].w, x.w, fmaf(wv[j].z, x.z, fmaf(wv[j].y, x.y, fmaf(wv[j].x, x.x, v[4 * i + j]))));
-            }
-        }
-#pragma unroll
-    for (int n = 16; n >= 1; n >>= 1) {   // lane l ends with value l
-        const bool up = lane & n;
-#pragma unroll
-        for (int i = 0; i < n; ++i) {
-            const float give = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, n);
-        }
-    }
-    if (warp < 24) smem[warp * 32 + lane] = v[0];
-    else {   // the spare warp: per-token scale, two lanes a token
-        const int tok = lane & 15;
-        float ss = 0.f;
-#pragma unroll 8
-        for (int q = lane >> 4; q < p.n_sumsq; q += 2) ss += __ldcg(p.sumsq + q * MAX_ROWS + tok);
-        ss += __shfl_xor_sync(0xffffffffu, ss, 16);
-        if (lane < 16) smem[24 * 32 + tok] = 1.0f / sqrtf(ss / p.norm_k + p.eps);
-    }
-    __syncthreads();
-    if (threadIdx.x < 64) {
-        const int tok = threadIdx.x >> 2, j = threadIdx.x & 3, par = tok >> 3, idx = 4 * (tok & 7) + j;
-        float t = 0.f;
-#pragma unroll
-        for (int w2 = 0; w2 < 12; ++w2) t += smem[(2 * w2 + par) * 32 + idx];
-        if (tok < p.side_rows && o0 + j < p.side_n) p.side_out[(uint64_t)tok * p.side_n + o0 + j] = t * smem[24 * 32 + tok];
-    }
-}
 
 // The eight MMAs of half h = 2 h2 + C of an entry into one accumulator (the first of them overwrites it when the half is
 // the accumulator's first of the entry).
@@ -142,10 +98,10 @@ __device__ __forceinline__ void issue_half(int h2, uint32_t d, uint32_t a_buf, u
     }
 }
 
-template <int DT>
-__global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
+template <int DT, int KC>
+__global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
     using F = Fmt<DT>;
-    constexpr int STAGES = F::STAGES, HALVES = F::HALVES;
+    constexpr int STAGES = F::stages(KC), HALVES = F::HALVES;
     constexpr int OFF_RING = KC * ACTTS_CHUNK;
     constexpr int OFF_SCL = OFF_RING + STAGES * F::STAGE;
     constexpr int OFF_BAR = OFF_SCL + SCL_BYTES;
@@ -176,12 +132,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
     __shared__ int abort_flag;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp-uniform by construction
-    if ((int)blockIdx.x >= p.main_grid) {
-        pdl_launch_dependents();
-        pdl_wait();
-        side_projection(p, reinterpret_cast<float*>(smem));
-        return;
-    }
     int row_tiles = p.row_tiles, kblocks = p.kblocks, splits = p.splits, cps = p.ctas_per_split;
     if (p.tile_map || p.kb_map) {   // the lists come from the preceding kernel: nothing may be fetched before it is complete
         pdl_wait();
@@ -203,10 +153,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < FULL_SETS * STAGES; ++s) mbar_init(&full[s], 1);
-        for (int s = 0; s < STAGES; ++s) mbar_init(&empty[s], GROUP_WARPS);
+        for (int s = 0; s < STAGES; ++s) mbar_init(&empty[s], FR_GROUP_WARPS);
         for (int k = 0; k < KC; ++k) mbar_init(&acts_bar[k], 1);
         for (int i = 0; i < 4; ++i) {
-            mbar_init(&a_ready[i], GROUP_WARPS);
+            mbar_init(&a_ready[i], FR_GROUP_WARPS);
             mbar_init(&a_free[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -222,44 +172,56 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
-    pdl_launch_dependents();
+    if (!p.trigger_late) pdl_launch_dependents();
+    // The late form: every thread passes the dependency wait first, each role where it has nothing else to do (it does not matter how many of
+    // a CTA's threads the hardware counts, and a second call does nothing).
+    auto trigger = [&] {
+        if (!p.trigger_late) return;
+        pdl_wait();
+        pdl_launch_dependents();
+    };
 
     if (warp == PRODUCER_WARP) {
         // ------------------------------ bulk-copy producer ------------------------------
-        if (lane == 0) {
-            // weights do not depend on the previous kernel: the ring is filled without waiting for it.  The loop keeps
-            // running slot / round / source counters so that issuing a stage is a handful of instructions.
-            const uint64_t tile_stride = (uint64_t)p.kblocks * F::STAGE;
-            const bool mapped = p.tile_map != nullptr || p.kb_map != nullptr;
-            int pt = 0, pk = 0, s = 0;
-            uint32_t round = 0;
-            const uint8_t* src = p.w + (uint64_t)c * tile_stride + (uint64_t)kb0 * F::STAGE;   // tile c, first column block of the range
-            bool ok = true;
-            for (int e = 0; e < n_it; ++e) {
-                if (round > 0) ok = mbar_wait_bounded(&empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
-                if (!ok) break;
-                if (mapped) {
-                    const int slot = c + pt * cps;
-                    src = p.w + (uint64_t)(p.tile_map ? p.tile_map[slot] : slot) * tile_stride +
-                          (uint64_t)(p.kb_map ? p.kb_map[kb0 + pk] : kb0 + pk) * F::STAGE;
-                }
+        // Weights do not depend on the previous kernel: the ring is filled without waiting for it.  (Fetching 3 - 16 stages more into L2 meanwhile
+        // made the Q6_K launches 0.7 - 1.2 us shorter and the kernels before, whose loads it delayed, as much longer.)
+        // The whole warp walks the loop, one lane issues; slot / round / source are kept by addition.
+        const uint64_t tile_stride = (uint64_t)p.kblocks * F::STAGE;
+        const bool mapped = p.tile_map != nullptr || p.kb_map != nullptr;
+        int pt = 0, pk = 0, s = 0;
+        uint32_t round = 0;
+        const uint8_t* src = p.w + (uint64_t)c * tile_stride + (uint64_t)kb0 * F::STAGE;   // tile c, first column block of the range
+        const uint64_t next_tile = (uint64_t)cps * tile_stride - (uint64_t)n_kb * F::STAGE;   // from the range's end to its start in the CTA's next tile
+        bool ok = true;
+        for (int e = 0; e < n_it; ++e) {
+            if (round > 0) ok = mbar_wait_warp(&empty[s], (round - 1) & 1, p.err, DEV_ERR_WAIT_EMPTY);
+            if (!ok) break;
+            if (round == 1 && s == 0) trigger();
+            if (mapped) {
+                const int slot = c + pt * cps;
+                src = p.w + (uint64_t)(p.tile_map ? p.tile_map[slot] : slot) * tile_stride +
+                      (uint64_t)(p.kb_map ? p.kb_map[kb0 + pk] : kb0 + pk) * F::STAGE;
+            }
+            if (lane == 0) {
                 uint64_t* fb = full_bar(full, e, s);
                 mbar_arrive_expect_tx(fb, F::STAGE);
                 bulk_g2s(ring + s * F::STAGE, src, F::STAGE, fb);
-                src += F::STAGE;
-                if (++s == STAGES) { s = 0; ++round; }
-                if (++pk == n_kb) {   // next row tile of this CTA: cps tiles further, back to the first column block
-                    pk = 0;
-                    ++pt;
-                    src += (uint64_t)cps * tile_stride - (uint64_t)n_kb * F::STAGE;
-                }
             }
-            if (!ok) abort_flag = 1;
+            src += F::STAGE;
+            if (++pk == n_kb) {   // next row tile of this CTA: cps tiles further, back to the first column block
+                pk = 0;
+                ++pt;
+                src += next_tile;
+            }
+            if (++s == STAGES) { s = 0; ++round; }
         }
+        if (!ok) abort_flag = 1;
+        trigger();
     } else if (warp >= MMA_WARP0 && warp < MMA_WARP0 + MMA_WARPS) {
         // ------------------------------ MMA issuers ------------------------------
         // Warp (g, c) issues the halves h with h % 2 == c of group g's entries into accumulator c of that group.  The
         // whole warp walks the loop so that addresses and descriptors stay warp-uniform; one elected lane issues.
+        trigger();
         constexpr uint32_t IDESC_MAIN = instr_desc(32), IDESC_MIN = instr_desc(48);
         const uint32_t g = (uint32_t)(warp - MMA_WARP0) >> 1, c = (uint32_t)(warp - MMA_WARP0) & 1u;
         bool ok = true;
@@ -302,58 +264,76 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
             }
         }
         if (!ok) abort_flag = 1;
-    } else if (warp < UNPACK_WARPS) {
+    } else if (warp < FR_UNPACK_WARPS) {
         // ------------------------------ unpacking warps ------------------------------
         // They read weights only (shared memory filled by the producer), so they never wait for the previous kernel.
-        const int g = warp >> 3, q4 = warp & 3, kp2 = (warp >> 2) & 1;
+        // A half is announced when the first 64 columns of the next one are already unpacked: its stores have long landed by then,
+        // so that the wait for them costs nothing.
+        const int g = warp >> 2, q4 = warp & 3;
         const int row = 32 * q4 + lane;
         const uint32_t tm_l = tmem + ((uint32_t)(32 * q4) << 16);
         const uint32_t a_buf = tm_l + TM_A + g * TM_A_STRIDE, am_buf = tm_l + TM_AM + g * TM_AM_STRIDE;
         // K padding of the group's min-term operand (sub-block pairs 4..7): written once, never touched again
-        if (F::HAS_MIN && kp2 == 0) tmem_st4(am_buf + 4, 0u, 0u, 0u, 0u);
+        if (F::HAS_MIN) tmem_st4(am_buf + 4, 0u, 0u, 0u, 0u);
         bool ok = true;
-        uint32_t hc = 0;   // running half count of this group
-        for (int e = g; e < n_it && ok; e += 2) {
-            const int s = e % STAGES;
-            ok = mbar_wait_warp(full_bar(full, e, s), full_parity(e), p.err, DEV_ERR_WAIT_FULL);
-            if (!ok) break;
-            const uint8_t* st = ring + s * F::STAGE;
-            uint32_t am_keep[HALVES];
-#pragma unroll
-            for (int h = 0; h < HALVES; ++h, ++hc) {
-                uint32_t r[32], am[8];
-                UnitScales us{0.f, 0.f};
-                if (ok) F::unpack(st, h, row, kp2, r, am, us);
-                if (F::HAS_MIN && h < HALVES - 1) am_keep[h] = am[0];
-                const uint32_t hb = hc & 1;
-                if (ok && hc >= 2) {   // the half buffer was last read by the MMAs of the group's half hc - 2
-                    ok = mbar_wait_warp(&a_free[2 * g + hb], ((hc >> 1) - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
-                    if (ok) fence_after_sync();
-                }
-                if (ok) {
-                    F::store(a_buf, h, kp2, r);
-                    if (F::HAS_MIN && h == HALVES - 1) {
-                        // The min operand is read by the entry's last MMA, so it may only be replaced once the previous
-                        // entry's last half has completed - which this half's wait has just established.
-#pragma unroll
-                        for (int hh = 0; hh < HALVES - 1; ++hh) tmem_st1(am_buf + F::min_col(hh, kp2), am_keep[hh]);
-                        tmem_st1(am_buf + F::min_col(h, kp2), am[0]);
-                    }
-                    if (h == 0 && kp2 == 0) scl[(e & 3) * TILE_R + row] = make_float2(us.d, us.dmin);
-                    wait_st();
-                    fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive(&a_ready[2 * g + hb]);   // releases this warp's tensor-memory and side-buffer writes
-                        if (h == HALVES - 1) mbar_arrive(&empty[s]);
-                    }
-                }
+        int stored = -1;   // half buffer that has been written but not announced
+        auto announce = [&] {
+            if (stored < 0) return;
+            wait_st();
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&a_ready[2 * g + stored]);   // releases this warp's tensor-memory and side-buffer writes
+            stored = -1;
+        };
+        uint32_t uses = 0;   // how often each half buffer of the group has been used
+        int s = g;
+        for (int e = g; e < n_it; e += 2) {
+            uint64_t* fb = full_bar(full, e, s);
+            if (!__all_sync(0xffffffffu, mbar_try_wait(fb, full_parity(e)))) {
+                announce();
+                ok = mbar_wait_warp(fb, full_parity(e), p.err, DEV_ERR_WAIT_FULL);
+                if (!ok) break;
             }
+            const uint8_t* st = ring + s * F::STAGE;
+            uint32_t mins[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int h = 0; h < HALVES; ++h) {
+                constexpr int LAST = HALVES - 1;
+                const int hb = h & 1;
+                uint32_t r[32];
+                UnitScales us{0.f, 0.f};
+                F::unpack(st, h, row, 0, r, mins[(2 * h) & 3], us);
+                announce();
+                if (uses == 1) trigger();   // nothing can be stored before an MMA has run, which is behind the dependency wait
+                if (uses > 0) {   // the half buffer was last read by the MMAs of the group's half before the last
+                    ok = mbar_wait_warp_inline(&a_free[2 * g + hb], (uses - 1) & 1, p.err, DEV_ERR_WAIT_FULL);
+                    if (!ok) break;
+                    fence_after_sync();
+                }
+                F::store(a_buf, h, 0, r);
+                if (h == 0) scl[(e & 3) * TILE_R + row] = make_float2(us.d, us.dmin);
+                F::unpack(st, h, row, 1, r, mins[(2 * h + 1) & 3], us);
+                F::store(a_buf, h, 1, r);
+                if (h == LAST) {
+                    // The min operand is read by the entry's last MMA, so it may only be replaced once the previous
+                    // entry's last half has completed - which this half's wait has just established.
+                    if (F::HAS_MIN) tmem_st4(am_buf, mins[0], mins[1], mins[2], mins[3]);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty[s]);
+                }
+                stored = hb;
+                if (hb == 1) ++uses;
+            }
+            if (!ok) break;
+            s = s + 2 >= STAGES ? s + 2 - STAGES : s + 2;
         }
-        if (!ok) abort_flag = 1;
+        if (ok) announce();
+        else abort_flag = 1;
+        if (uses < 2) trigger();
     } else {
         // ------------------------------ draining warps ------------------------------
-        pdl_wait();
+        if (!p.wait_last) pdl_wait();
+        trigger();
         const int dtid = threadIdx.x - DRAIN_WARP0 * 32;   // 0..127 = weight row of the tile = tensor-memory lane
         if (dtid == 0 && n_it > 0) {
             // the activations (the previous kernel's output), in the order of their first use, one barrier each: the
@@ -377,9 +357,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
         named_sync(1, DRAIN_WARPS * 32);
         const int row = dtid;
         const uint32_t tm_l = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-        float acc[MAX_ROWS];
+        uint64_t acc[MAX_ROWS / 2];   // pairs of tokens
 #pragma unroll
-        for (int j = 0; j < MAX_ROWS; ++j) acc[j] = 0.f;
+        for (int j = 0; j < MAX_ROWS / 2; ++j) acc[j] = 0ull;
         bool ok = true;
         int kb_e = 0, tile = 0;   // e % n_kb and e / n_kb, kept by addition
         for (int e = 0; e < n_it && ok; ++e) {
@@ -388,34 +368,38 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
             if (!ok) break;
             fence_after_sync();
             const float2 sc = scl[(e & 3) * TILE_R + row];   // published before the a_ready arrival the MMAs waited for
-            float t[MAX_ROWS], mn[MAX_ROWS];
+            // columns 16 plane + token, one load of 32 at a time: two would not fit the registers
+            uint64_t t[MAX_ROWS / 2], mn[MAX_ROWS / 2];
+            {
+                float v[32];
+                tmem_ld32(tm_l + TM_D + a * TM_D_STRIDE, v);        // even MMA halves
+                wait_ld();
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {   // tokens 8 hf .. 8 hf + 7
-                float ve[16], vo[16];
-                tmem_ld16(tm_l + TM_D + a * TM_D_STRIDE + 16 * hf, ve);        // even MMA steps: columns 2 tok + plane
-                tmem_ld16(tm_l + TM_D + a * TM_D_STRIDE + 32 + 16 * hf, vo);   // odd MMA steps
-                if (F::HAS_MIN) {
-                    float s0[8], s1[8], s2[8];   // 8 tokens x 3 planes, token j = flattened columns 3j .. 3j + 2
-                    tmem_ld8(tm_l + TM_DM + a * TM_DM_STRIDE + 24 * hf, s0);
-                    tmem_ld8(tm_l + TM_DM + a * TM_DM_STRIDE + 24 * hf + 8, s1);
-                    tmem_ld8(tm_l + TM_DM + a * TM_DM_STRIDE + 24 * hf + 16, s2);
-                    wait_ld();
-                    auto col = [&](int i) { return i < 8 ? s0[i] : i < 16 ? s1[i - 8] : s2[i - 16]; };
+                for (int j = 0; j < MAX_ROWS / 2; ++j) t[j] = add2(pack2(v[2 * j], v[2 * j + 1]), pack2(v[16 + 2 * j], v[17 + 2 * j]));
+                tmem_ld32(tm_l + TM_D + a * TM_D_STRIDE + 32, v);   // odd MMA halves
+                wait_ld();
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) mn[8 * hf + j] = (col(3 * j) + col(3 * j + 1)) + col(3 * j + 2);
-                } else {
+                for (int j = 0; j < MAX_ROWS / 2; ++j) t[j] = add2(t[j], add2(pack2(v[2 * j], v[2 * j + 1]), pack2(v[16 + 2 * j], v[17 + 2 * j])));
+                if (F::HAS_MIN) {   // three planes of sixteen tokens
+                    tmem_ld32(tm_l + TM_DM + a * TM_DM_STRIDE, v);
                     wait_ld();
+#pragma unroll
+                    for (int j = 0; j < MAX_ROWS / 2; ++j) mn[j] = add2(pack2(v[2 * j], v[2 * j + 1]), pack2(v[16 + 2 * j], v[17 + 2 * j]));
+                    float v2[16];
+                    tmem_ld16(tm_l + TM_DM + a * TM_DM_STRIDE + 32, v2);
+                    wait_ld();
+#pragma unroll
+                    for (int j = 0; j < MAX_ROWS / 2; ++j) mn[j] = add2(mn[j], pack2(v2[2 * j], v2[2 * j + 1]));
                 }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) t[8 * hf + j] = (ve[2 * j] + ve[2 * j + 1]) + (vo[2 * j] + vo[2 * j + 1]);
             }
             fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&d_free[a]);   // the accumulator may be overwritten
+            const uint64_t d2 = pack2(sc.x, sc.x), m2 = pack2(-sc.y, -sc.y);
 #pragma unroll
-            for (int j = 0; j < MAX_ROWS; ++j) {
-                acc[j] = fmaf(sc.x, t[j], acc[j]);
-                if (F::HAS_MIN) acc[j] = fmaf(-sc.y, mn[j], acc[j]);
+            for (int j = 0; j < MAX_ROWS / 2; ++j) {
+                acc[j] = fma2(d2, t[j], acc[j]);
+                if (F::HAS_MIN) acc[j] = fma2(m2, mn[j], acc[j]);
             }
             if (++kb_e == n_kb) {   // the tile's last column block: write the partial result
                 kb_e = 0;
@@ -425,10 +409,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
                 if (orow < p.n_out) {
                     float* dst = p.out + (uint64_t)sp * MAX_ROWS * p.ld_out + orow;
 #pragma unroll
-                    for (int j = 0; j < MAX_ROWS; ++j) dst[(uint64_t)j * p.ld_out] = acc[j] * tok_scale[j];
+                    for (int j = 0; j < MAX_ROWS / 2; ++j) {
+                        float lo, hi;
+                        unpack2(acc[j], lo, hi);
+                        dst[(uint64_t)(2 * j) * p.ld_out] = lo * tok_scale[2 * j];
+                        dst[(uint64_t)(2 * j + 1) * p.ld_out] = hi * tok_scale[2 * j + 1];
+                    }
                 }
 #pragma unroll
-                for (int j = 0; j < MAX_ROWS; ++j) acc[j] = 0.f;
+                for (int j = 0; j < MAX_ROWS / 2; ++j) acc[j] = 0ull;
             }
         }
         if (!ok) abort_flag = 1;
@@ -453,9 +442,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_ts_kernel(const Params p) {
         fence_after_sync();
         tmem_free(tmem, TM_COLS);
     }
+    if (p.wait_last) pdl_wait();   // this kernel's completion says that those before are complete too
 }
 
-template <int DT>
+template <int DT, int KC>
 static dfl_status launch_t(cudaStream_t st, const Params& p, int grid, bool pdl) {
     static std::once_flag attr_once[16];
     int dev = 0;
@@ -463,23 +453,23 @@ static dfl_status launch_t(cudaStream_t st, const Params& p, int grid, bool pdl)
     if (dev >= 0 && dev < 16) {
         cudaError_t attr_err = cudaSuccess;
         std::call_once(attr_once[dev], [&] {
-            attr_err = cudaFuncSetAttribute(gemm_ts_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<DT>());
+            attr_err = cudaFuncSetAttribute(gemm_ts_kernel<DT, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<DT, KC>());
         });
         DFL_CUDA(attr_err);
     } else {
-        DFL_CUDA(cudaFuncSetAttribute(gemm_ts_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<DT>()));
+        DFL_CUDA(cudaFuncSetAttribute(gemm_ts_kernel<DT, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<DT, KC>()));
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem_bytes<DT>();
+    cfg.dynamicSmemBytes = smem_bytes<DT, KC>();
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    DFL_CUDA(cudaLaunchKernelEx(&cfg, gemm_ts_kernel<DT>, p));
+    DFL_CUDA(cudaLaunchKernelEx(&cfg, gemm_ts_kernel<DT, KC>, p));
     count_launch();
     return DFL_OK;
 }
@@ -500,12 +490,12 @@ int gemm_ts_choose_splits(const QMatrix& m) {
     return gemm_ts_choose_splits_multi(&tiles, 1, m.kblocks);
 }
 // CTAs per split of a launch over `row_tiles` row tiles (the least number of tiles a tile list must hold)
-int gemm_ts_kc() { return ts::KC; }   // column blocks a CTA keeps resident
+int gemm_ts_kc() { return ts::KC_MAX; }   // column blocks a CTA keeps resident
 int gemm_ts_ctas_per_split(int row_tiles, int splits) { return ts::ctas_per_split(row_tiles, splits); }
 // Several matrices that share their input and their partial buffer are launched one after the other
 // with one common split count: minimise the sum of their longest-CTA times.
 int gemm_ts_choose_splits_multi(const int* row_tiles, int n_mats, int kblocks) {
-    const int s_min = (kblocks + ts::KC - 1) / ts::KC;
+    const int s_min = (kblocks + ts::KC_MAX - 1) / ts::KC_MAX;
     int s_max = kblocks < 24 ? kblocks : 24;
     if (s_max < s_min) s_max = s_min;
     int best = s_min;
@@ -527,7 +517,7 @@ int gemm_ts_choose_splits_multi(const int* row_tiles, int n_mats, int kblocks) {
 dfl_status launch_gemm_ts(cudaStream_t st, const QMatrix& m, const uint8_t* acts, float* out, int splits, const GemmEpilogue& ep,
                           int* dev_err, bool pdl, uint32_t ld_out) {
     if (splits < 1 || splits > m.kblocks) return fail(DFL_ERR_BAD_ARG, "gemm: bad split count");
-    if ((m.kblocks + splits - 1) / splits > ts::KC) return fail(DFL_ERR_BAD_ARG, "gemm: too few splits for the resident activation window");
+    if ((m.kblocks + splits - 1) / splits > ts::KC_MAX) return fail(DFL_ERR_BAD_ARG, "gemm: too few splits for the resident activation window");
     ts::Params p;
     p.w = m.tiles;
     p.acts = acts;
@@ -548,20 +538,18 @@ dfl_status launch_gemm_ts(cudaStream_t st, const QMatrix& m, const uint8_t* acts
     p.n_tiles = ep.n_tiles;
     p.kb_map = ep.kb_map;
     p.n_kb = ep.n_kb;
+    p.trigger_late = ep.trigger_late;
+    p.wait_last = ep.behind_late;
+    if (ep.behind_late && (ep.trigger_late || ep.tile_map || ep.kb_map)) return fail(DFL_ERR_BAD_ARG, "gemm: dependency options");
     int grid = p.ctas_per_split * splits;
     if (ep.kb_map && ep.dynamic_splits && grid < sm_count()) grid = sm_count();   // room for the geometry chosen on the device
-    p.main_grid = grid;
-    p.side_w = ep.side_w; p.side_x = ep.side_x; p.side_out = ep.side_out;
-    p.side_n = ep.side_n; p.side_k = ep.side_k; p.side_rows = ep.side_rows;
-    if (ep.side_w) {
-        if (ep.side_n % 4 || ep.side_k % 4 || !ep.sumsq) return fail(DFL_ERR_BAD_SHAPE, "gemm: side projection shape");
-        grid += ep.side_n / 4;
-    }
+    // four resident column blocks leave room for a fourth ring slot of a 35 KB stage (4096 x 32768 Q6_K 32.0 -> 31.0 us)
+    const bool four = !ep.kb_map && (m.kblocks + splits - 1) / splits <= 4;
     switch (m.dtype) {
-        case DFL_Q4_K: return ts::launch_t<DFL_Q4_K>(st, p, grid, pdl);
-        case DFL_Q5_K: return ts::launch_t<DFL_Q5_K>(st, p, grid, pdl);
-        case DFL_Q6_K: return ts::launch_t<DFL_Q6_K>(st, p, grid, pdl);
-        case DFL_Q8_0: return ts::launch_t<DFL_Q8_0>(st, p, grid, pdl);
+        case DFL_Q4_K: return ts::launch_t<DFL_Q4_K, ts::KC_MAX>(st, p, grid, pdl);
+        case DFL_Q5_K: return ts::launch_t<DFL_Q5_K, ts::KC_MAX>(st, p, grid, pdl);
+        case DFL_Q6_K: return four ? ts::launch_t<DFL_Q6_K, 4>(st, p, grid, pdl) : ts::launch_t<DFL_Q6_K, ts::KC_MAX>(st, p, grid, pdl);
+        case DFL_Q8_0: return four ? ts::launch_t<DFL_Q8_0, 4>(st, p, grid, pdl) : ts::launch_t<DFL_Q8_0, ts::KC_MAX>(st, p, grid, pdl);
         default: return fail(DFL_ERR_UNSUPPORTED, "gemm: weight dtype has no tensor-memory kernel");
     }
 }

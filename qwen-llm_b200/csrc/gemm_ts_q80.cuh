@@ -64,12 +64,10 @@ __global__ void q80_scale_range_kernel(const uint8_t* __restrict__ src, uint64_t
 
 namespace ts {
 
-constexpr uint32_t H2_1152 = 0x64806480u;   // half2(1152) = 1024 + 128
-
 template <>
 struct Fmt<DFL_Q8_0> {
     static constexpr int STAGE = STAGE_Q8_0;
-    static constexpr int STAGES = KC == 4 ? 4 : 3;
+    __host__ __device__ static constexpr int stages(int kc) { return kc <= 4 ? 4 : 3; }   // ring slots beside kc resident column blocks
     static constexpr int HALVES = 4;   // half h: blocks 4 (h / 2) + 2 (h % 2) + kp2; written as A1 (64 columns) and A2 (64)
     static constexpr bool HAS_MIN = false;
     // steps 0..3 multiply A1, steps 4..7 A2, both with the half's four 16-column slices
@@ -83,9 +81,8 @@ struct Fmt<DFL_Q8_0> {
         tmem_st16(buf + 16 * kp, lo);
         tmem_st16(buf + 64 + 16 * kp, hi);
     }
-    __device__ static __forceinline__ int min_col(int, int) { return 0; }
     // r[0..15] = A1, r[16..31] = A2, column c = k' pair (2c, 2c + 1)
-    __device__ static __forceinline__ void unpack(const uint8_t* st, int h, int row, int kp2, uint32_t (&r)[32], uint32_t (&)[8],
+    __device__ static __forceinline__ void unpack(const uint8_t* st, int h, int row, int kp2, uint32_t (&r)[32], uint32_t&,
                                                   UnitScales& us) {
         const int b = 4 * (h >> 1) + 2 * (h & 1) + kp2;
         const uint4* q = reinterpret_cast<const uint4*>(st + TSQ8_OFF_QS);

@@ -252,18 +252,17 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             out_proj = &L.wo;
             ++ai;
         } else {
-            // one stream, one chain: qkv, z (its own matrix when its format differs) with alpha / beta behind it, the mixer
+            // one stream, one chain: qkv, z (its own matrix when its format differs), alpha / beta, the mixer.  z and alpha / beta do not depend on
+            // qkv: they start as its CTAs leave, and wait for it at their ends
             const MatGroup& G = L.in_qkv_z;
-            const bool ab_rides = m->act_layout == ACT_TS && gg.n_v % 2 == 0;
+            const bool late = G.mats[0].layout == LAYOUT_TS && G.mats[0].dtype != DFL_BF16;
             for (size_t i = 0; i < G.mats.size(); ++i) {
                 GemmEpilogue ep = ep_norm;
-                if (i + 1 == G.mats.size() && ab_rides) {
-                    ep.side_w = L.w_ab; ep.side_x = sc->xn; ep.side_out = sc->ab[gi];
-                    ep.side_n = 2 * gg.n_v; ep.side_k = (int)H; ep.side_rows = (int)n;
-                }
+                ep.trigger_late = i == 0 && late;
+                ep.behind_late = i > 0 && late;
                 DFL_CHECK(launch_gemm_fewrow(st, G.mats[i], sc->acts_h, sc->part + G.col_off[i], G.splits, ep, s->err, pdl_enabled(), G.total_cols));
             }
-            if (!ab_rides) DFL_CHECK(launch_small_matmul(st, L.w_ab, sc->xn, (int)H, (int)n, H, 2 * gg.n_v, ep_norm, sc->ab[gi], 2 * gg.n_v));
+            DFL_CHECK(launch_ab_proj(st, L.w_ab, sc->xn, (int)H, (int)n, H, 2 * gg.n_v, sc->ab_part, late));
             const int cur = s->ssm_cur[gi];
             GdnMixParams p;
             p.g = gg;
@@ -272,7 +271,9 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             p.state_in = s->ssm[cur][gi]; p.state_out = s->ssm[cur ^ 1][gi];
             p.dt_bias = L.dt_bias; p.a_log = L.a_log; p.norm_w = L.ssm_norm_w;
             p.qkv_raw = sc->qkv_raw[gi]; p.q_n = sc->q_n[gi]; p.k_n = sc->k_n[gi]; p.v = sc->v[gi]; p.ab = sc->ab[gi];
+            p.ab_part = sc->ab_part; p.sumsq = sc->sumsq; p.slices = ab_slices(H); p.n_sumsq = kb_h; p.norm_k = (float)H; p.eps = ep_norm.eps;
             p.acts = sc->acts_v; p.layout = m->act_layout; p.err = s->err;
+            p.prefetch = L.w_out.mats[0].tiles; p.prefetch_bytes = L.w_out.mats[0].bytes();
             DFL_CHECK(launch_gdn_mix(st, p));
             s->ssm_cur[gi] = cur ^ 1;
             out_proj = &L.w_out;
@@ -845,6 +846,7 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
     alloc(&sc->xn, MAX_ROWS * H * 4);
     alloc(&sc->part, part * 4);
     alloc(&sc->sumsq, (H / GLUE_COLS) * MAX_ROWS * 4);
+    alloc(&sc->ab_part, (uint64_t)ab_slices(H) * MAX_ROWS * 2 * gg.n_v * 4);
     const uint64_t chunk = (uint64_t)std::max(act_chunk_bytes(ACT_F16), act_chunk_bytes(ACT_TS));
     alloc(&sc->acts_h, H / TILE_K * chunk);
     const uint64_t f_inner = a.expert_count > 0 ? (uint64_t)m->ep_n * a.expert_feed_forward_length + m->ep_fs : F;

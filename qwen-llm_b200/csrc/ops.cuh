@@ -104,6 +104,19 @@ struct GlueParams {
     int* err = nullptr;
 };
 #ifdef __CUDACC__
+// Packs one item's values (columns col0 .. + 3) and, from eight neighbouring threads, its 32-column sub-block sum.
+__device__ __forceinline__ void glue_pack(const GlueParams& p, int col0, int tok, int quad, const float (&v)[4]) {
+    uint8_t* chunk = p.acts + (uint64_t)(col0 >> 8) * act_chunk_dev(p.bf3);
+    bool over = false;
+    pack_quad_any(chunk, p.bf3, tok, col0 & 255, v, over);
+    if ((p.bf3 == ACT_F16 || p.bf3 == ACT_TS)) {
+        float sum = v[0] + v[1] + v[2] + v[3];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((quad & 7) == 0) store_subsum(chunk, p.bf3, tok, (col0 & 255) >> 5, sum, over);
+    }
+    if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
+}
 // The glue of one (token, four consecutive columns) item: columns 64 cb + 4 quad .. + 3 of token `tok`.  The 32 lanes of
 // the calling warp must be two tokens x the sixteen quads of one 64-column block (lane = 16 (tok & 1) + quad): the sum
 // of squares is reduced over a token's 16 lanes and the 32-column sub-block sums over 8 lanes.
@@ -137,7 +150,7 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
             }
         } else {
             float4 xv = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (p.x) xv = *reinterpret_cast<const float4*>(p.x + (uint64_t)tok * p.ld_x + col0);
+            if (p.x) xv = __ldcg(reinterpret_cast<const float4*>(p.x + (uint64_t)tok * p.ld_x + col0));
             if (p.mode == GLUE_RESID && p.part) {
                 // sum the split-K partials first (fixed order), then add to the residual
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -171,18 +184,7 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
         for (int j = 0; j < 4; ++j) v[j] *= p.pre_scale;
     }
     if (p.xn && live) *reinterpret_cast<float4*>(p.xn + (uint64_t)tok * p.ld_xn + col0) = make_float4(v[0], v[1], v[2], v[3]);
-    if (p.acts) {
-        uint8_t* chunk = p.acts + (uint64_t)(col0 >> 8) * act_chunk_dev(p.bf3);
-        bool over = false;
-        pack_quad_any(chunk, p.bf3, tok, col0 & 255, v, over);
-        if ((p.bf3 == ACT_F16 || p.bf3 == ACT_TS)) {
-            float sum = v[0] + v[1] + v[2] + v[3];  // 32-column sub-block = eight neighbouring threads
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if ((quad & 7) == 0) store_subsum(chunk, p.bf3, tok, (col0 & 255) >> 5, sum, over);
-        }
-        if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
-    }
+    if (p.acts) glue_pack(p, col0, tok, quad, v);
 }
 #endif
 // k = number of columns (multiple of 256)
@@ -304,14 +306,27 @@ struct GdnMixParams {
     const float* state_in = nullptr;
     float* state_out = nullptr;
     const float *dt_bias = nullptr, *a_log = nullptr, *norm_w = nullptr;
-    const float* ab = nullptr;     // [16][2 n_v]: alpha projections, then beta projections
-    // the block's rows, kept for a rollback
-    float *qkv_raw = nullptr, *q_n = nullptr, *k_n = nullptr, *v = nullptr;
+    // alpha and beta projections in slices (launch_ab_proj; alpha first), to be summed and scaled by the rows' RMS norm:
+    // sumsq [n_sumsq][16] over norm_k columns
+    const float *ab_part = nullptr, *sumsq = nullptr;
+    int slices = 0, n_sumsq = 0;
+    float norm_k = 1.f, eps = 0.f;
+    // the block's rows, kept for a rollback; ab: the scaled projections [16][2 n_v]
+    float *qkv_raw = nullptr, *q_n = nullptr, *k_n = nullptr, *v = nullptr, *ab = nullptr;
     uint8_t* acts = nullptr;
     int layout = 0;
     int* err = nullptr;
+    // bytes that the next kernel streams (16-byte aligned), fetched into L2 meanwhile
+    const uint8_t* prefetch = nullptr;
+    uint64_t prefetch_bytes = 0;
 };
 dfl_status launch_gdn_mix(cudaStream_t st, const GdnMixParams& p);
+// ab_part[tok][o][slice] = sum over the slice's AB_COLS columns of xn[tok][c] * w[o][c], o < n_out.  behind_late_gemm: the kernel before is a GEMM
+// launched with ep.trigger_late, so that xn is complete when this one starts; it then runs beside that GEMM.
+constexpr int AB_COLS = 512;
+inline int ab_slices(uint64_t k) { return (int)((k + AB_COLS - 1) / AB_COLS); }
+dfl_status launch_ab_proj(cudaStream_t st, const float* w, const float* xn, int ld_xn, int n_rows, uint64_t k, int n_out, float* ab_part,
+                          bool behind_late_gemm);
 // Advances the recurrent state over the first n_rows kept rows of a block (the re-scan of a partial accept).
 dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* state_in, float* state_out, const float* k_n, const float* v,
                              const float* ab, const float* dt_bias, const float* a_log, int n_rows);

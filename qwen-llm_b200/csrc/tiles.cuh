@@ -87,7 +87,7 @@ __host__ __device__ inline bool dtype_uses_bf16_acts(int dtype) { return dtype =
 // row-lane tiles for the tensor-memory kernel (gemm_ts.cuh).  The packed activation format
 // follows the kernel that consumes it.
 constexpr int LAYOUT_FRAG = 0, LAYOUT_TS = 1;
-// Q6_K row-lane tiles hold one code per byte: [128 x 16 i8 scales][128 x f16 d][128 rows x 256 bytes]
+// Q6_K row-lane tiles hold one weight per byte: [128 x 16 i8 scales][128 x f16 d][128 rows x 256 bytes]
 constexpr int STAGE_Q6_K_TS = 2304 + TILE_R * 256;  // 35072
 // Q4_K / Q5_K row-lane tiles hold the eight (scale, min) pairs as bytes: 20 bytes of header per row instead of 16
 constexpr int STAGE_Q4_K_TS = STAGE_Q4_K + TILE_R * 4, STAGE_Q5_K_TS = STAGE_Q5_K + TILE_R * 4;
@@ -213,11 +213,12 @@ struct GemmEpilogue {
     // n_kb[1] / n_kb[2] (when n_kb[1] > 0): split count and CTAs per split to use for this list length, their product
     // at most 148, the splits at most the launch's own; the caller sums that many partial slices
     bool dynamic_splits = false;
-    // A small f32 projection of the same rows that rides along (tensor-memory family only) on CTAs of its own behind the GEMM's:
-    // side_out[tok][j] = rs[tok] * sum_k side_x[tok][k] * side_w[j][k], j < side_n (a multiple of 4), rs from sumsq as above.
-    const float *side_w = nullptr, *side_x = nullptr;
-    float* side_out = nullptr;
-    int side_n = 0, side_k = 0, side_rows = 0;
+    // The next kernel may start once this one's own dependencies are complete, not before (tensor-memory family only): it may then read
+    // what those wrote without a dependency wait.
+    bool trigger_late = false;
+    // Launched behind such a kernel, on inputs older than it (tensor-memory family only): starts without a dependency wait and waits at its end,
+    // for the kernels behind.
+    bool behind_late = false;
 };
 int gemm_choose_splits(const QMatrix& m);
 int gemm_max_kblocks_per_cta(int dtype);  // column blocks one CTA can keep resident
