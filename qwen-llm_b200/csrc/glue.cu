@@ -10,29 +10,55 @@
 
 namespace dfl {
 
+
 // grid = (k / 64, 2), block 128: thread = (token = 8 y + tid / 16, four consecutive columns).  One float4 per split per
 // thread keeps every global load of the kernel independent (one latency round); the norm weight does not depend on the
-// kernel before and is fetched ahead of the dependency wait.  128 threads, because a GEMM CTA (800 threads of 72 registers)
-// leaves room for exactly such a CTA beside it: with 256 the following GEMM could not start on the 64 SMs that held a waiting
-// glue CTA, and its late CTAs set the end of every link of the chain (verify block 3160 -> 3132 us).
-__global__ void __launch_bounds__(128) glue_kernel(const GlueParams p) {
+// kernel before and is fetched ahead of the dependency wait.  128 threads, so that two such CTAs fit beside a GEMM CTA (480 threads of 96
+// registers): the following GEMM cannot start on an SM before the glue CTAs that belong there have, and its late CTAs set the
+// end of every link of the chain (verify block 3160 -> 3132 us when 256 threads became 128).
+// What bounds the kernel is latency, and a good part of it was its own code: between two of its launches GEMMs stream 100 MB and more through
+// L2, so that every line of it came from far away behind the dependency wait.  The first warp therefore runs through it once
+// before, on a buffer that nobody reads (p.dry): a link of the chain 5.6 -> 5.1 us (residual), 5.6 -> 4.7 us (SwiGLU), a 9B-class verify block
+// of 97 links 2937 -> 2894 us under tracing.
+template <bool DRY>
+__global__ void __launch_bounds__(128, 7) glue_kernel(const GlueParams p) {
     const int quad = threadIdx.x & 15;
     const float4 w = p.mul_w ? *reinterpret_cast<const float4*>(p.mul_w + blockIdx.x * GLUE_COLS + quad * 4) : make_float4(1.f, 1.f, 1.f, 1.f);
-    pdl_prologue();
-    // columns of an expert that no row of the block chose, where the next GEMM reads chosen experts' columns only: nothing to do (at 16
-    // rows of 8 experts some 100 of 256 are chosen; packing zeros for the others wrote 5 MB a layer)
-    // (the first block stands in for a list of chosen experts that is empty: its zeros are read)
-    if (p.skip_unchosen && blockIdx.x >= TILE_K / GLUE_COLS && (int)blockIdx.x * GLUE_COLS < p.route_n * p.route_f) {
-        const int expert = p.route_e0 + (int)blockIdx.x * GLUE_COLS / p.route_f;
-        if (!__syncthreads_or(threadIdx.x < MAX_ROWS && p.route_w[threadIdx.x * p.route_e + expert] != 0.f)) return;
+    pdl_launch_dependents();
+#pragma unroll 1
+    for (int pass = DRY ? 0 : 1; pass < 2; ++pass) {
+        GlueParams q = p;
+        int cb = blockIdx.x, n_splits = 1;
+        if (pass == 0) {
+            if (threadIdx.x >= 32) continue;
+            float* f = reinterpret_cast<float*>(p.dry + GLUE_DRY_ACTS);
+            cb &= TILE_K / GLUE_COLS - 1;
+            q.acts = p.acts ? p.dry : nullptr;
+            q.part = p.part ? f : nullptr; q.ld_part = q.swiglu_f = 0;
+            q.x = p.x ? f : nullptr; q.ld_x = 0;
+            q.xn = p.xn ? f : nullptr; q.ld_xn = 0;
+            q.sumsq = p.sumsq ? f : nullptr;
+            q.capture = nullptr;
+            q.route_w = nullptr;
+        } else {
+            pdl_wait();
+            // columns of an expert that no row of the block chose, where the next GEMM reads chosen experts' columns only: nothing to do (at 16
+            // rows of 8 experts some 100 of 256 are chosen; packing zeros for the others wrote 5 MB a layer)
+            // (the first block stands in for a list of chosen experts that is empty: its zeros are read)
+            if (p.skip_unchosen && blockIdx.x >= TILE_K / GLUE_COLS && (int)blockIdx.x * GLUE_COLS < p.route_n * p.route_f) {
+                const int expert = p.route_e0 + (int)blockIdx.x * GLUE_COLS / p.route_f;
+                if (!__syncthreads_or(threadIdx.x < MAX_ROWS && p.route_w[threadIdx.x * p.route_e + expert] != 0.f)) return;
+            }
+            n_splits = p.splits_dev ? p.splits + *p.splits_dev : p.splits;
+        }
+        glue_quad<DRY ? 4 : 8>(q, n_splits, cb, blockIdx.y * 8 + (threadIdx.x >> 4), quad, w);
     }
-    const int n_splits = p.splits_dev ? p.splits + *p.splits_dev : p.splits;
-    glue_quad(p, n_splits, blockIdx.x, blockIdx.y * 8 + (threadIdx.x >> 4), quad, w);
 }
 
 dfl_status launch_glue(cudaStream_t st, const GlueParams& p, uint64_t k) {
     if (k == 0 || k % TILE_K) return fail(DFL_ERR_BAD_SHAPE, "glue: column count must be a positive multiple of 256");
-    launch_k(glue_kernel, dim3((unsigned)(k / GLUE_COLS), MAX_ROWS / 8), dim3(128), 0, st, p);
+    // the first pass only where (nearly) all CTAs wait beside the GEMM before: behind it, it would be time lost
+    launch_k(p.dry && 2 * k / GLUE_COLS <= 3 * (uint64_t)sm_count() ? glue_kernel<true> : glue_kernel<false>, dim3((unsigned)(k / GLUE_COLS), MAX_ROWS / 8), dim3(128), 0, st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

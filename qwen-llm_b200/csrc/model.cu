@@ -235,6 +235,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
         p.sumsq = sc->sumsq;
         p.capture = capture; p.ld_capture = (int)(sc->k_layers * H);
         p.n_rows = (int)n; p.err = s->err;
+        p.dry = splits_dev ? nullptr : sc->dry;   // behind the join with the side stream it would not start early
         return launch_glue(st, p, H);
     };
     DFL_CHECK(norm_glue(nullptr, 0, 0, m->layers[0].attn_norm_w, !m->layers[0].is_attn, nullptr));
@@ -331,6 +332,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             p.pre_scale = 1.0f / 64.0f;
             p.acts = sc->acts_f; p.bf3 = m->act_layout;
             p.n_rows = (int)n; p.err = s->err;
+            p.dry = sc->dry;
             DFL_CHECK(launch_glue(st, p, (uint64_t)inner));
             GemmEpilogue ep_down;
             ep_down.out_scale = 64.0f;
@@ -379,6 +381,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             p.pre_scale = 1.0f / 64.0f;  // keeps silu(g)*u inside the f16 operand range; undone in the GEMM epilogue
             p.acts = sc->acts_f; p.bf3 = m->act_layout;
             p.n_rows = (int)n; p.err = s->err;
+            p.dry = sc->dry;
             DFL_CHECK(launch_group(st, L.gate_up, sc->acts_h, sc->part, ep_norm, s->err));
             DFL_CHECK(launch_glue(st, p, F));
         }
@@ -846,6 +849,7 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
     alloc(&sc->xn, MAX_ROWS * H * 4);
     alloc(&sc->part, part * 4);
     alloc(&sc->sumsq, (H / GLUE_COLS) * MAX_ROWS * 4);
+    alloc(&sc->dry, GLUE_DRY_BYTES);
     alloc(&sc->ab_part, (uint64_t)ab_slices(H) * MAX_ROWS * 2 * gg.n_v * 4);
     const uint64_t chunk = (uint64_t)std::max(act_chunk_bytes(ACT_F16), act_chunk_bytes(ACT_TS));
     alloc(&sc->acts_h, H / TILE_K * chunk);

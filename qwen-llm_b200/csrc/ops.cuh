@@ -74,6 +74,7 @@ enum GlueMode : int {
     GLUE_COPY = 2     // v = x (read only)
 };
 
+constexpr int GLUE_DRY_ACTS = 32768, GLUE_DRY_BYTES = GLUE_DRY_ACTS + 4096;   // a chunk of activations, and rows of 256 floats
 struct GlueParams {
     int mode = GLUE_RESID;
     const float* part = nullptr;  // [splits][16][ld_part]
@@ -102,6 +103,8 @@ struct GlueParams {
     bool skip_unchosen = false;   // route_f must be a multiple of GLUE_COLS
     int n_rows = 0;
     int* err = nullptr;
+    // optional GLUE_DRY_BYTES of zeros that no result depends on: the kernel runs through its code once on them before its dependency wait
+    uint8_t* dry = nullptr;
 };
 #ifdef __CUDACC__
 // Packs one item's values (columns col0 .. + 3) and, from eight neighbouring threads, its 32-column sub-block sum.
@@ -120,6 +123,7 @@ __device__ __forceinline__ void glue_pack(const GlueParams& p, int col0, int tok
 // The glue of one (token, four consecutive columns) item: columns 64 cb + 4 quad .. + 3 of token `tok`.  The 32 lanes of
 // the calling warp must be two tokens x the sixteen quads of one 64-column block (lane = 16 (tok & 1) + quad): the sum
 // of squares is reduced over a token's 16 lanes and the 32-column sub-block sums over 8 lanes.
+template <int DEPTH = 4>   // residual mode: slices fetched at a time
 __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int cb, int tok, int quad, const float4 w) {   // w: the quad's mul_w
     const int col0 = cb * GLUE_COLS + quad * 4;
     const bool live = tok < p.n_rows;
@@ -156,7 +160,7 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
                 const float* base = p.part + (uint64_t)tok * p.ld_part + col0;
                 const uint64_t stride = (uint64_t)p.part_rows * p.ld_part;
-#pragma unroll 4
+#pragma unroll DEPTH
                 for (int s = 0; s < n_splits; ++s) {
                     const float4 a = __ldcg(reinterpret_cast<const float4*>(base + s * stride));
                     acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
