@@ -286,6 +286,7 @@ struct dfl_dsession {
     uint8_t* pinned_sel = nullptr;   // [16][16] ids | [16][16] vals | [16][rank] gate rows
     // projection of newly appended context columns: its own scratch, so that it can run on a side stream beside the
     // start of the draft pass (layer l's attention waits for ev_ctx[l])
+    uint8_t* dry = nullptr;   // GlueParams::dry
     float *part_c = nullptr, *sumsq_c = nullptr;
     uint8_t* acts_hc = nullptr;
     cudaStream_t st_side = nullptr;
@@ -474,6 +475,7 @@ dfl_status dfl_dsession_create(const dfl_drafter* d, uint32_t ctx_capacity, dfl_
         ds->x = (float*)alloc(MAX_ROWS * H * 4);
         ds->part = (float*)alloc(part * 4);
         ds->sumsq = (float*)alloc((H / GLUE_COLS) * MAX_ROWS * 4);
+        ds->dry = (uint8_t*)alloc(GLUE_DRY_BYTES);
         ds->q_rot = (float*)alloc(MAX_ROWS * q_dim * 4);
         ds->k_noise = (float*)alloc(MAX_ROWS * kv_dim * 4);
         ds->v_noise = (float*)alloc(MAX_ROWS * kv_dim * 4);
@@ -752,6 +754,7 @@ dfl_status draft_core(dfl_dsession* ds, int32_t carry, uint32_t noise_start, boo
         p.acts = acts; p.bf3 = layout;
         p.sumsq = ds->sumsq;
         p.n_rows = n; p.err = ds->err;
+        p.dry = ds->dry;
         return launch_glue(st, p, H);
     };
     auto bf = [](const MatGroup& g) { return act_layout_of(g.mats[0]); };
@@ -798,6 +801,7 @@ dfl_status draft_core(dfl_dsession* ds, int32_t carry, uint32_t noise_start, boo
         p.pre_scale = down_bf ? 1.0f : 1.0f / 64.0f;
         p.acts = ds->acts_f; p.bf3 = down_layout;
         p.n_rows = n; p.err = ds->err;
+        p.dry = ds->dry;
         DFL_CHECK(launch_glue(st, p, F));
         GemmEpilogue ep_down;
         ep_down.out_scale = down_bf ? 1.0f : 64.0f;

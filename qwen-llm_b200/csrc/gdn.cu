@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128, 7) ab_proj_kernel(const float* __restrict
     if (threadIdx.x < MAX_ROWS * AB_OUT) {
         const int tok = threadIdx.x / AB_OUT, o = o0 + threadIdx.x % AB_OUT;
         const float t = (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
-        if (tok < n_rows && o < n_out) ab_part[((uint64_t)tok * n_out + o) * gridDim.y + blockIdx.y] = t;
+        if (tok < n_rows && o < n_out) ab_part[((uint64_t)blockIdx.y * MAX_ROWS + tok) * n_out + o] = t;
     }
     if (!wait_first) pdl_wait();
 }
@@ -279,9 +279,9 @@ __global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(MIX_THREADS) gdn_mix
     float ab = 0.f;
     if (warp == 8) {
         if ((lane >> 1) < p.n_rows) {
-            const float* src = p.ab_part + ((uint64_t)(lane >> 1) * 2 * g.n_v + (lane & 1) * g.n_v + h) * p.slices;
+            const float* src = p.ab_part + (uint64_t)(lane >> 1) * 2 * g.n_v + (lane & 1) * g.n_v + h;
 #pragma unroll 8
-            for (int s = 0; s < p.slices; ++s) ab += __ldcg(src + s);
+            for (int s = 0; s < p.slices; ++s) ab += __ldcg(src + (uint64_t)s * MAX_ROWS * 2 * g.n_v);
         }
     } else {
         const int tok = threadIdx.x & 15, part = threadIdx.x >> 4;

@@ -132,25 +132,6 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
     __shared__ int abort_flag;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp-uniform by construction
-    int row_tiles = p.row_tiles, kblocks = p.kblocks, splits = p.splits, cps = p.ctas_per_split;
-    if (p.tile_map || p.kb_map) {   // the lists come from the preceding kernel: nothing may be fetched before it is complete
-        pdl_wait();
-        if (p.tile_map) row_tiles = *p.n_tiles;
-        if (p.kb_map) {
-            kblocks = p.n_kb[0];
-            if (p.n_kb[1] > 0) {   // the list's author also chose the split geometry for its length (the launch is the worst case)
-                splits = p.n_kb[1];
-                cps = p.n_kb[2];
-            }
-        }
-    }
-    if ((int)blockIdx.x >= splits * cps) return;   // nothing has been set up yet: a CTA beyond the geometry in use just leaves
-    const int sp = blockIdx.x % splits, c = blockIdx.x / splits;
-    const int kb0 = (int)((long long)sp * kblocks / splits), kb1 = (int)((long long)(sp + 1) * kblocks / splits);
-    const int n_kb = kb1 - kb0;
-    const int n_my = (row_tiles - c + cps - 1) / cps;   // row tiles c, c + cps, ... (of the list)
-    const int n_it = n_my * n_kb;            // entries
-
     if (threadIdx.x == 0) {
         for (int s = 0; s < FULL_SETS * STAGES; ++s) mbar_init(&full[s], 1);
         for (int s = 0; s < STAGES; ++s) mbar_init(&empty[s], FR_GROUP_WARPS);
@@ -173,6 +154,24 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
     if (!p.trigger_late) pdl_launch_dependents();
+    int row_tiles = p.row_tiles, kblocks = p.kblocks, splits = p.splits, cps = p.ctas_per_split;
+    if (p.tile_map || p.kb_map) {   // the lists come from the preceding kernel: nothing may be fetched before it is complete
+        if (!p.wait_last) pdl_wait();
+        if (p.tile_map) row_tiles = *p.n_tiles;
+        if (p.kb_map) {
+            kblocks = p.n_kb[0];
+            if (p.n_kb[1] > 0) {   // the list's author also chose the split geometry for its length (the launch is the worst case)
+                splits = p.n_kb[1];
+                cps = p.n_kb[2];
+            }
+        }
+    }
+    const int sp = blockIdx.x % splits, c = blockIdx.x / splits;
+    const int kb0 = (int)((long long)sp * kblocks / splits), kb1 = (int)((long long)(sp + 1) * kblocks / splits);
+    const int n_kb = kb1 - kb0;
+    const int n_my = (row_tiles - c + cps - 1) / cps;   // row tiles c, c + cps, ... (of the list)
+    const int n_it = (int)blockIdx.x < splits * cps ? n_my * n_kb : 0;   // entries; none for a CTA beyond the geometry in use
+
     // The late form: every thread passes the dependency wait first, each role where it has nothing else to do (it does not matter how many of
     // a CTA's threads the hardware counts, and a second call does nothing).
     auto trigger = [&] {
@@ -540,7 +539,7 @@ dfl_status launch_gemm_ts(cudaStream_t st, const QMatrix& m, const uint8_t* acts
     p.n_kb = ep.n_kb;
     p.trigger_late = ep.trigger_late;
     p.wait_last = ep.behind_late;
-    if (ep.behind_late && (ep.trigger_late || ep.tile_map || ep.kb_map)) return fail(DFL_ERR_BAD_ARG, "gemm: dependency options");
+    if (ep.behind_late && ep.trigger_late) return fail(DFL_ERR_BAD_ARG, "gemm: dependency options");
     int grid = p.ctas_per_split * splits;
     if (ep.kb_map && ep.dynamic_splits && grid < sm_count()) grid = sm_count();   // room for the geometry chosen on the device
     // four resident column blocks leave room for a fourth ring slot of a 35 KB stage (4096 x 32768 Q6_K 32.0 -> 31.0 us)

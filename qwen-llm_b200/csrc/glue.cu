@@ -55,8 +55,58 @@ __global__ void __launch_bounds__(128, 7) glue_kernel(const GlueParams p) {
     }
 }
 
+// The residual glue behind the routed experts, whose device-chosen split count can be 40 and more: grid (k / 64, 8); the four warps fetch a quarter
+// of the slices each (lane = token 2 y + lane / 16, four columns) and the first adds them in order, as one thread to all slices would: slices
+// that a row has no part in are zeros, so its sum does not depend on what the block's other rows chose.  With a thread to all slices the
+// kernel was ten rounds of loads on a third of the chip (32 x 2 CTAs): a link of the chain 12.0 -> 8.9 us, with the join it no longer waits for.
+constexpr int SLICES_STAGED = 64;
+__global__ void __launch_bounds__(128) glue_slices_kernel(const GlueParams p) {
+    __shared__ float4 red[SLICES_STAGED][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 15, tok = 2 * blockIdx.y + (lane >> 4), cb = blockIdx.x;
+    const int col0 = cb * GLUE_COLS + quad * 4;
+    const float4 w = p.mul_w ? *reinterpret_cast<const float4*>(p.mul_w + col0) : make_float4(1.f, 1.f, 1.f, 1.f);
+    pdl_prologue();
+    const int n_splits = p.splits + *p.splits_dev;
+    const bool live = tok < p.n_rows;
+    float4 xv = make_float4(0.f, 0.f, 0.f, 0.f), acc = xv;
+    if (live && warp == 0 && p.x) xv = __ldcg(reinterpret_cast<const float4*>(p.x + (uint64_t)tok * p.ld_x + col0));
+    const float* base = p.part + (uint64_t)tok * p.ld_part + col0;
+    const uint64_t stride = (uint64_t)p.part_rows * p.ld_part;
+    for (int s0 = 0; s0 < n_splits; s0 += SLICES_STAGED) {
+        const int n = min(SLICES_STAGED, n_splits - s0);
+        if (live) {
+#pragma unroll 8
+            for (int s = warp; s < n; s += 4) red[s][lane] = __ldcg(reinterpret_cast<const float4*>(base + (s0 + s) * stride));
+        }
+        __syncthreads();
+        if (live && warp == 0) {
+#pragma unroll 4
+            for (int s = 0; s < n; ++s) {
+                const float4 a = red[s][lane];
+                acc.x += a.x; acc.y += a.y; acc.z += a.z; acc.w += a.w;
+            }
+        }
+        __syncthreads();
+    }
+    if (warp > 0) return;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (live) {
+        v[0] = xv.x + acc.x; v[1] = xv.y + acc.y; v[2] = xv.z + acc.z; v[3] = xv.w + acc.w;
+        const float4 out = make_float4(v[0], v[1], v[2], v[3]);
+        if (p.x) *reinterpret_cast<float4*>(p.x + (uint64_t)tok * p.ld_x + col0) = out;
+        if (p.capture) *reinterpret_cast<float4*>(p.capture + (uint64_t)tok * p.ld_capture + col0) = out;
+    }
+    glue_finish(p, cb, tok, quad, w, v);
+}
+
 dfl_status launch_glue(cudaStream_t st, const GlueParams& p, uint64_t k) {
     if (k == 0 || k % TILE_K) return fail(DFL_ERR_BAD_SHAPE, "glue: column count must be a positive multiple of 256");
+    if (p.splits_dev && p.mode == GLUE_RESID && p.part) {
+        launch_k(glue_slices_kernel, dim3((unsigned)(k / GLUE_COLS), MAX_ROWS / 2), dim3(128), 0, st, p);
+        count_launch();
+        DFL_CUDA(cudaGetLastError());
+        return DFL_OK;
+    }
     // the first pass only where (nearly) all CTAs wait beside the GEMM before: behind it, it would be time lost
     launch_k(p.dry && 2 * k / GLUE_COLS <= 3 * (uint64_t)sm_count() ? glue_kernel<true> : glue_kernel<false>, dim3((unsigned)(k / GLUE_COLS), MAX_ROWS / 8), dim3(128), 0, st, p);
     count_launch();
@@ -133,7 +183,8 @@ dfl_status launch_embed_block(cudaStream_t st, int dtype, const uint8_t* ggml, u
 // ---- small f32 matrices --------------------------------------------------------------
 // A CTA of 512 threads per four output columns, a thread four columns of k at a time over all rows: the rows, which every CTA reads
 // from L2, are read a quarter as often as with one output per CTA (257 outputs over 2048 columns and 16 rows: 33 -> 8.5 MB,
-// 11.2 -> 7 us cold), and their loads are independent.  The first weights are on their way before the dependency wait.  Sums over
+// 11.2 -> 7 us cold), and their loads are independent.  The first weights are on their way before the dependency wait, and so is the code: where
+// one round of columns is all there is, the kernel runs through it once before, on whatever xn holds, and stores nothing.  Sums over
 // lanes, then warps, in a fixed order.
 constexpr int SMALL_OUT = 4;
 __global__ void __launch_bounds__(512) small_matmul_kernel(const float* __restrict__ w, const float* xn, int ld_xn,
@@ -150,55 +201,61 @@ __global__ void __launch_bounds__(512) small_matmul_kernel(const float* __restri
 #pragma unroll
         for (int j = 0; j < SMALL_OUT; ++j) wv[j] = *reinterpret_cast<const float4*>(wr[j] + c);
     }
-    pdl_prologue();
     __shared__ float scale_s[MAX_ROWS];
     __shared__ float red[16][MAX_ROWS * SMALL_OUT];
-    float acc[MAX_ROWS * SMALL_OUT];   // [row][output]
+    pdl_launch_dependents();
+#pragma unroll 1
+    for (int pass = k <= 512 * 4 ? 0 : 1; pass < 2; ++pass) {
+        if (pass) pdl_wait();
+        c = (uint64_t)threadIdx.x * 4;
+        float acc[MAX_ROWS * SMALL_OUT];   // [row][output]
 #pragma unroll
-    for (int i = 0; i < MAX_ROWS * SMALL_OUT; ++i) acc[i] = 0.f;
-    while (c < k) {
+        for (int i = 0; i < MAX_ROWS * SMALL_OUT; ++i) acc[i] = 0.f;
+        while (c < k) {
 #pragma unroll
-        for (int r = 0; r < MAX_ROWS; ++r) {
-            if (r < n_rows) {
-                const float4 xv = *reinterpret_cast<const float4*>(xn + (uint64_t)r * ld_xn + c);
+            for (int r = 0; r < MAX_ROWS; ++r) {
+                if (r < n_rows) {
+                    const float4 xv = __ldcg(reinterpret_cast<const float4*>(xn + (uint64_t)r * ld_xn + c));
 #pragma unroll
-                for (int j = 0; j < SMALL_OUT; ++j)
-                    acc[SMALL_OUT * r + j] = fmaf(wv[j].w, xv.w, fmaf(wv[j].z, xv.z, fmaf(wv[j].y, xv.y, fmaf(wv[j].x, xv.x, acc[SMALL_OUT * r + j]))));
+                    for (int j = 0; j < SMALL_OUT; ++j)
+                        acc[SMALL_OUT * r + j] = fmaf(wv[j].w, xv.w, fmaf(wv[j].z, xv.z, fmaf(wv[j].y, xv.y, fmaf(wv[j].x, xv.x, acc[SMALL_OUT * r + j]))));
+                }
+            }
+            c += 512 * 4;
+            if (c < k) {
+#pragma unroll
+                for (int j = 0; j < SMALL_OUT; ++j) wv[j] = *reinterpret_cast<const float4*>(wr[j] + c);
             }
         }
-        c += 512 * 4;
-        if (c < k) {
+        // per-token output scale (16 threads per token, fixed tree)
+        if (threadIdx.x < 256) {
+            const int tok = threadIdx.x >> 4, part = threadIdx.x & 15;
+            float ss = 0.f;
+            if (sumsq)
+                for (int i = part; i < n_sumsq; i += 16) ss += __ldcg(sumsq + i * MAX_ROWS + tok);
 #pragma unroll
-            for (int j = 0; j < SMALL_OUT; ++j) wv[j] = *reinterpret_cast<const float4*>(wr[j] + c);
+            for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (part == 0) scale_s[tok] = sumsq ? out_scale * (1.0f / sqrtf(ss / norm_k + eps)) : out_scale;
         }
-    }
-    // per-token output scale (16 threads per token, fixed tree)
-    if (threadIdx.x < 256) {
-        const int tok = threadIdx.x >> 4, part = threadIdx.x & 15;
-        float ss = 0.f;
-        if (sumsq)
-            for (int i = part; i < n_sumsq; i += 16) ss += sumsq[i * MAX_ROWS + tok];
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (part == 0) scale_s[tok] = sumsq ? out_scale * (1.0f / sqrtf(ss / norm_k + eps)) : out_scale;
-    }
+        for (int n = 32; n >= 2; n >>= 1) {   // lane l ends with values 2 l, 2 l + 1
+            const bool up = lane & (n >> 1);
 #pragma unroll
-    for (int n = 32; n >= 2; n >>= 1) {   // lane l ends with values 2 l, 2 l + 1
-        const bool up = lane & (n >> 1);
-#pragma unroll
-        for (int i = 0; i < n; ++i) {
-            const float give = up ? acc[i] : acc[i + n], keep = up ? acc[i + n] : acc[i];
-            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, n >> 1);
+            for (int i = 0; i < n; ++i) {
+                const float give = up ? acc[i] : acc[i + n], keep = up ? acc[i + n] : acc[i];
+                acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, n >> 1);
+            }
         }
-    }
-    *reinterpret_cast<float2*>(&red[warp][2 * lane]) = make_float2(acc[0], acc[1]);
-    __syncthreads();
-    if (threadIdx.x < MAX_ROWS * SMALL_OUT) {
-        const int r = threadIdx.x / SMALL_OUT, j = threadIdx.x % SMALL_OUT;
-        float s = 0.f;
+        *reinterpret_cast<float2*>(&red[warp][2 * lane]) = make_float2(acc[0], acc[1]);
+        __syncthreads();
+        if (threadIdx.x < MAX_ROWS * SMALL_OUT) {
+            const int r = threadIdx.x / SMALL_OUT, j = threadIdx.x % SMALL_OUT;
+            float s = 0.f;
 #pragma unroll
-        for (int wi = 0; wi < 16; ++wi) s += red[wi][threadIdx.x];
-        if (r < n_rows && o0 + j < n_out) out[(uint64_t)r * ld_out + o0 + j] = s * scale_s[r];
+            for (int wi = 0; wi < 16; ++wi) s += red[wi][threadIdx.x];
+            if (pass && r < n_rows && o0 + j < n_out) out[(uint64_t)r * ld_out + o0 + j] = s * scale_s[r];
+        }
+        __syncthreads();   // red and scale_s are free
     }
 }
 

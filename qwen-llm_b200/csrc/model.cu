@@ -235,7 +235,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
         p.sumsq = sc->sumsq;
         p.capture = capture; p.ld_capture = (int)(sc->k_layers * H);
         p.n_rows = (int)n; p.err = s->err;
-        p.dry = splits_dev ? nullptr : sc->dry;   // behind the join with the side stream it would not start early
+        p.dry = sc->dry;
         return launch_glue(st, p, H);
     };
     DFL_CHECK(norm_glue(nullptr, 0, 0, m->layers[0].attn_norm_w, !m->layers[0].is_attn, nullptr));
@@ -301,16 +301,12 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
                 const int min_tiles = gemm_ts_ctas_per_split(GU.mats[0].row_tiles, GU.splits);
                 const int down_tiles = down_chosen ? L.moe_down.mats[0].row_tiles : 1, down_max = down_chosen ? L.moe_down.splits : 0;
                 int32_t* kb_map = down_chosen ? sc->moe_kb_map : nullptr;
-                DFL_CHECK(launch_small_matmul(st, L.router_w, sc->xn, (int)H, (int)n, H, E + 1, ep_norm, sc->route_logits, E + 1));
-                if (moe_route_lists_fused(E)) {
-                    DFL_CHECK(launch_moe_route_lists(st, sc->route_logits, E + 1, E, (int)a.expert_used_count, (int)n, sc->route_w, sc->route_sg,
-                                                     sc->route_idx, (int)m->ep_e0, En, Fe / TILE_R, Fs / TILE_R, min_tiles, sc->moe_tile_map,
-                                                     sc->moe_n_tiles, Fe / TILE_K, 1, kb_map, sc->moe_n_tiles + 1, gemm_ts_kc(), down_tiles, down_max, s->err));
-                } else {
-                    DFL_CHECK(launch_moe_route(st, sc->route_logits, E + 1, E, (int)a.expert_used_count, (int)n, sc->route_w, sc->route_sg, sc->route_idx, s->err));
-                    DFL_CHECK(launch_moe_tiles(st, sc->route_w, (int)n, E, (int)m->ep_e0, En, Fe / TILE_R, Fs / TILE_R, min_tiles, sc->moe_tile_map,
-                                               sc->moe_n_tiles, Fe / TILE_K, 1, kb_map, sc->moe_n_tiles + 1, gemm_ts_kc(), down_tiles, down_max));
-                }
+                DFL_CHECK(launch_ab_proj(st, L.router_w, sc->xn, (int)H, (int)n, H, E + 1, sc->route_logits, false));
+                RouterLogits x;
+                x.part = sc->route_logits; x.slices = ab_slices(H); x.sumsq = sc->sumsq; x.n_sumsq = kb_h; x.norm_k = (float)H; x.eps = ep_norm.eps;
+                DFL_CHECK(launch_moe_route_lists(st, x, E, (int)a.expert_used_count, (int)n, sc->route_w, sc->route_sg, sc->route_idx, (int)m->ep_e0, En,
+                                                 Fe / TILE_R, Fs / TILE_R, min_tiles, sc->moe_tile_map, sc->moe_n_tiles, Fe / TILE_K, 1, kb_map,
+                                                 sc->moe_n_tiles + 1, gemm_ts_kc(), down_tiles, down_max, s->err));
                 GemmEpilogue ep_gu = ep_norm;
                 ep_gu.tile_map = sc->moe_tile_map;
                 ep_gu.n_tiles = sc->moe_n_tiles;
@@ -346,14 +342,16 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
                 ep_down_exps.dynamic_splits = true;
                 down_splits_dev = sc->moe_n_tiles + 2;
             }
-            // the shared expert's small down projection runs beside the routed experts' on the side stream
+            // The shared expert's small down projection and the routed experts' do not depend on each other: the second starts beside the first
+            // (without a dependency wait of its own) and waits for it at its end.  On a stream of its own the first cost 3.5 us of joining.
             if (Fs > 0) {
-                DFL_CHECK(fork_side());
-                DFL_CHECK(launch_group(side, L.moe_down_sh, sc->acts_f + (uint64_t)(En * Fe / TILE_K) * act_chunk_bytes(m->act_layout), sc->part,
+                const bool late = L.moe_down_sh.mats.size() == 1 && L.moe_down_sh.mats[0].layout == LAYOUT_TS && L.moe_down_sh.mats[0].dtype != DFL_BF16 &&
+                                  L.moe_down.mats.size() == 1 && L.moe_down.mats[0].layout == LAYOUT_TS && L.moe_down.mats[0].dtype != DFL_BF16;
+                ep_down.trigger_late = ep_down_exps.behind_late = late;
+                DFL_CHECK(launch_group(st, L.moe_down_sh, sc->acts_f + (uint64_t)(En * Fe / TILE_K) * act_chunk_bytes(m->act_layout), sc->part,
                                        ep_down, s->err));
             }
             DFL_CHECK(launch_group(st, L.moe_down, sc->acts_f, sc->part + (uint64_t)sh_splits * MAX_ROWS * H, ep_down_exps, s->err));
-            if (Fs > 0) DFL_CHECK(join_side());
             down_splits = sh_splits + (down_splits_dev ? 0 : L.moe_down.splits);
             if (m->ep_world > 1 && m->ep_p2p) {
                 // this rank's slices summed and pushed into every rank's receive buffer; the glue below adds the ranks'
@@ -856,7 +854,7 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
     const uint64_t f_inner = a.expert_count > 0 ? (uint64_t)m->ep_n * a.expert_feed_forward_length + m->ep_fs : F;
     alloc(&sc->acts_f, f_inner / TILE_K * chunk);
     if (a.expert_count > 0) {
-        alloc(&sc->route_logits, (size_t)MAX_ROWS * (a.expert_count + 1) * 4);
+        alloc(&sc->route_logits, (size_t)MAX_ROWS * (a.expert_count + 1) * ab_slices(H) * 4);
         alloc(&sc->route_w, (size_t)MAX_ROWS * a.expert_count * 4);
         alloc(&sc->route_sg, MAX_ROWS * 4);
         alloc(&sc->moe_out, MAX_ROWS * H * 4);

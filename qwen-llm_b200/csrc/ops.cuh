@@ -120,6 +120,26 @@ __device__ __forceinline__ void glue_pack(const GlueParams& p, int col0, int tok
     }
     if (over) atomicCAS(p.err, 0, DEV_ERR_OVERFLOW);
 }
+// What follows the sums: sums of squares, norm weight, scale, copy and packing of an item's values.
+__device__ __forceinline__ void glue_finish(const GlueParams& p, int cb, int tok, int quad, const float4 w, float (&v)[4]) {
+    const int col0 = cb * GLUE_COLS + quad * 4;
+    const bool live = tok < p.n_rows;
+    if (p.sumsq) {
+        float ss = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (quad == 0) p.sumsq[cb * MAX_ROWS + tok] = ss;
+    }
+    if (p.mul_w) {
+        v[0] *= w.x; v[1] *= w.y; v[2] *= w.z; v[3] *= w.w;
+    }
+    if (p.pre_scale != 1.f) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] *= p.pre_scale;
+    }
+    if (p.xn && live) *reinterpret_cast<float4*>(p.xn + (uint64_t)tok * p.ld_xn + col0) = make_float4(v[0], v[1], v[2], v[3]);
+    if (p.acts) glue_pack(p, col0, tok, quad, v);
+}
 // The glue of one (token, four consecutive columns) item: columns 64 cb + 4 quad .. + 3 of token `tok`.  The 32 lanes of
 // the calling warp must be two tokens x the sixteen quads of one 64-column block (lane = 16 (tok & 1) + quad): the sum
 // of squares is reduced over a token's 16 lanes and the 32-column sub-block sums over 8 lanes.
@@ -174,21 +194,7 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
         if (p.capture)
             *reinterpret_cast<float4*>(p.capture + (uint64_t)tok * p.ld_capture + col0) = make_float4(v[0], v[1], v[2], v[3]);
     }
-    if (p.sumsq) {
-        float ss = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (quad == 0) p.sumsq[cb * MAX_ROWS + tok] = ss;
-    }
-    if (p.mul_w) {
-        v[0] *= w.x; v[1] *= w.y; v[2] *= w.z; v[3] *= w.w;
-    }
-    if (p.pre_scale != 1.f) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] *= p.pre_scale;
-    }
-    if (p.xn && live) *reinterpret_cast<float4*>(p.xn + (uint64_t)tok * p.ld_xn + col0) = make_float4(v[0], v[1], v[2], v[3]);
-    if (p.acts) glue_pack(p, col0, tok, quad, v);
+    glue_finish(p, cb, tok, quad, w, v);
 }
 #endif
 // k = number of columns (multiple of 256)
@@ -202,16 +208,19 @@ dfl_status launch_glue_groups(cudaStream_t st, const GlueParams& p, uint64_t k);
 // A NaN / Inf logit in a row leaves that row unrouted and sets DEV_ERR_NONFINITE in *err (the reference's NONFINITE route status).
 dfl_status launch_moe_route(cudaStream_t st, const float* logits, int ld, int n_expert, int n_used, int n_rows, float* route_w,
                             float* shared_gate, int32_t* route_idx, int* err);
-// routing and the lists below in one launch (moe_route_lists_fused says whether the expert count allows it)
-bool moe_route_lists_fused(int n_expert);
-dfl_status launch_moe_route_lists(cudaStream_t st, const float* logits, int ld, int n_expert, int n_used, int n_rows, float* route_w,
+// A router's logits in slices (launch_ab_proj): part [slices][16][n_expert + 1], to be summed and scaled by the rows' RMS norm
+// (sumsq [n_sumsq][16] over norm_k columns)
+struct RouterLogits {
+    const float *part = nullptr, *sumsq = nullptr;
+    int slices = 0, n_sumsq = 0;
+    float norm_k = 1.f, eps = 0.f;
+};
+// Routing, and in the same launch the row tiles of the gate|up matrix (and column blocks of the down matrix) that belong to experts some row of the
+// block chose (plus the shared expert).
+dfl_status launch_moe_route_lists(cudaStream_t st, const RouterLogits& x, int n_expert, int n_used, int n_rows, float* route_w,
                                   float* shared_gate, int32_t* route_idx, int e0, int n_local, int tiles_per_expert, int shared_tiles,
                                   int min_tiles, int32_t* tile_map, int32_t* n_tiles, int kb_per_expert, int min_kb, int32_t* kb_map,
                                   int32_t* n_kb, int kc, int down_tiles, int max_splits, int* err);
-// row tiles of the gate|up matrix that belong to experts some row of the block chose (plus the shared expert)
-dfl_status launch_moe_tiles(cudaStream_t st, const float* route_w, int n_rows, int n_expert, int e0, int n_local, int tiles_per_expert,
-                            int shared_tiles, int min_tiles, int32_t* tile_map, int32_t* n_tiles, int kb_per_expert, int min_kb, int32_t* kb_map,
-                            int32_t* n_kb, int kc, int down_tiles, int max_splits);
 
 // x[tok][0..h) = decoded row tokens[tok] of a ggml matrix [vocab][h] (kernel_get_rows_*,
 // kernels/elementwise.metal:727-958).  tokens live on the device.
@@ -325,7 +334,7 @@ struct GdnMixParams {
     uint64_t prefetch_bytes = 0;
 };
 dfl_status launch_gdn_mix(cudaStream_t st, const GdnMixParams& p);
-// ab_part[tok][o][slice] = sum over the slice's AB_COLS columns of xn[tok][c] * w[o][c], o < n_out.  behind_late_gemm: the kernel before is a GEMM
+// ab_part[slice][16][o] = sum over the slice's AB_COLS columns of xn[tok][c] * w[o][c], o < n_out.  behind_late_gemm: the kernel before is a GEMM
 // launched with ep.trigger_late, so that xn is complete when this one starts; it then runs beside that GEMM.
 constexpr int AB_COLS = 512;
 inline int ab_slices(uint64_t k) { return (int)((k + AB_COLS - 1) / AB_COLS); }
