@@ -293,49 +293,49 @@ dfl_status launch_tm_gdn_front(cudaStream_t st, const TmGdn& p) {
 //     o_i = G_i w_i + sum_{j <= i} D_ij (k_j . q_i) c_j,   S = G_15 S0 + sum_j D_15,j c_j k_j^T,
 // all in f32 and without a division.  A token-by-token scan waits twice per token for a three-level shuffle sum (512 tokens:
 // 242 us a layer); here a block's 32 sums are in flight together and only the 16-step substitution is serial, in registers.
-// grid (n_v, 4 quarters of the value channels), 256 threads; state, k and q rows lie in shared memory, rows 132 floats apart so that eight
-// neighbouring ones start in different 16-byte bank groups.  Per block, a barrier behind each:
-//   A  dots: warp = 32 key channels x the k or the q rows, lane = four state rows x four tokens, sums in registers;
-//   B  the four channel ranges added, L and M from the Gram matrices and decays; the rows after next are requested;
-//   C  warp 0: substitution, lane = state row, 16 steps of one multiply-add; warps 4 - 7: the Gram matrices of the next block (they do not
-//      depend on the state); warp 1: its gates and decays;
-//   D  outputs (lane = state row) and the state.
-// No sum crosses lanes.  Before, a warp owned four rows and summed 64 + 64 values over its lanes per block (124 exchanges a warp) with the
-// Gram matrices in front: 148 us a layer for 512 tokens, now 135; what is left is
-// shared-memory bandwidth (4500 wavefronts a block of 16 tokens) and the substitution.
-constexpr int SCAN_BLK = 16, SCAN_GS = 132, SCAN_RS = 36, SCAN_BUFS = 3;
+// grid (n_v, 4 quarters of the value channels), 256 threads: a warp owns four state rows and a lane four key channels of each,
+// so that one 16-byte load of a k or q row serves all four (with eight lanes a row the kernel was bound by shared-memory
+// bandwidth at the token scan's time).  The sums over the lanes halve the values they carry at every step; a lane keeps its
+// rows and tokens in an order rotated by its own number, so that what it passes on is always the upper half and no
+// select is needed.  Lane 8 r + l ends up with tokens 2 l, 2 l + 1 of row r.  The next block's rows travel with cp.async.
+constexpr int SCAN_BLK = 16;
 struct ScanSmem {
-    float s[32][SCAN_GS];                  // state rows of the CTA
-    float kq[SCAN_BUFS][32][SCAN_GS];      // a block's k rows, then its q rows
-    float vs[SCAN_BUFS][SCAN_BLK][32];
-    float red[4][32 * SCAN_RS];            // [channel range][state row][k, q row]
-    float gram[4][SCAN_BLK * SCAN_RS];     // [channel range][k row][k, q row]
-    float a[32][33];                       // S0 k_i, S0 q_i: [vector][state row]
-    float L[SCAN_BLK][SCAN_BLK], M[SCAN_BLK][SCAN_BLK];   // [j][i]
-    float C[SCAN_BLK][32];                 // c_j of every state row
-    float gs[2][SCAN_BLK], bs[2][SCAN_BLK], G[2][SCAN_BLK], D[2][SCAN_BLK];
+    float qs[2][SCAN_BLK][128], ks[2][SCAN_BLK][128], vs[2][SCAN_BLK][32];
+    float L[SCAN_BLK][SCAN_BLK + 4], M[SCAN_BLK][SCAN_BLK + 4];   // L[j][i] (column major: one step of the substitution reads a column), M[i][j]
+    float C[32][SCAN_BLK + 4];   // c_j D_15,j of every state row
+    float gs[2][SCAN_BLK], bs[2][SCAN_BLK], G[SCAN_BLK], D[SCAN_BLK];
 };
 __global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
     extern __shared__ __align__(16) uint8_t scan_smem[];
     ScanSmem& sm = *reinterpret_cast<ScanSmem*>(scan_smem);
     const GdnGeom& g = p.g;
-    const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, hk = h % g.n_k, dv_cta = blockIdx.y * 32;
-    const int rg = lane >> 2, vg = lane & 3, c0 = (warp & 3) * 32;
+    const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rr = lane >> 3, lg = lane & 7, hk = h % g.n_k;
+    const int dv_cta = blockIdx.y * 32, dv_l = warp * 4 + rr, dv = dv_cta + dv_l;   // the row whose tokens this lane finishes
     const float dtb = p.dt_bias[h], alog = p.a_log[h];
     pdl_prologue();
-    const uint64_t s_off = ((uint64_t)h * 128 + dv_cta) * 128;
-    for (int i = threadIdx.x; i < 32 * 32; i += 256)
-        *reinterpret_cast<float4*>(&sm.s[i >> 5][4 * (i & 31)]) = __ldcg(reinterpret_cast<const float4*>(p.state_in + s_off) + i);
+    float S[4][4];   // S[r]: row r ^ rr of the warp's four, key channels 4 lane .. + 3
+    const uint64_t s_off = ((uint64_t)h * 128 + dv_cta + warp * 4) * 128 + 4 * lane;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const float4 s4 = __ldcg(reinterpret_cast<const float4*>(p.state_in + s_off + (r ^ rr) * 128));
+        S[r][0] = s4.x; S[r][1] = s4.y; S[r][2] = s4.z; S[r][3] = s4.w;
+    }
     auto cp16 = [](void* dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory"); };
     // block boundaries: multiples of 16 from the start, and the first row of the part a rollback may undo
     const int ckpt = p.last_rows ? p.n_rows - p.last_rows : 0;
     auto next_of = [&](int r0) { return min(r0 < ckpt && r0 + SCAN_BLK > ckpt ? ckpt : r0 + SCAN_BLK, p.n_rows); };
     auto fetch = [&](int r0, int buf) {   // rows beyond the block's are zeros: they add nothing and decay nothing
-        const int n = r0 < p.n_rows ? next_of(r0) - r0 : 0;
-        for (int i = threadIdx.x; i < 32 * 32; i += 256) {
-            const int v = i >> 5, r = v & 15, d = (i & 31) * 4;
-            if (r < n) cp16(&sm.kq[buf][v][d], (v < 16 ? p.k_n : p.q_n) + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
-            else *reinterpret_cast<float4*>(&sm.kq[buf][v][d]) = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int n = next_of(r0) - r0;
+        for (int i = threadIdx.x; i < SCAN_BLK * 32; i += 256) {
+            const int r = i >> 5, d = (i & 31) * 4;
+            if (r < n) {
+                cp16(&sm.qs[buf][r][d], p.q_n + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
+                cp16(&sm.ks[buf][r][d], p.k_n + ((uint64_t)(r0 + r) * g.n_k + hk) * 128 + d);
+            } else {
+                *reinterpret_cast<float4*>(&sm.qs[buf][r][d]) = make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(&sm.ks[buf][r][d]) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
         if (threadIdx.x < SCAN_BLK * 8) {
             const int r = threadIdx.x >> 3, d = (threadIdx.x & 7) * 4;
@@ -344,200 +344,196 @@ __global__ void __launch_bounds__(256, 1) tm_gdn_scan_kernel(const TmGdn p) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // a block's gate inputs are loaded a block ahead by sixteen lanes of warp 1, which turn them into gates and decays
+    // gate inputs of a block: loaded a block ahead by 16 threads, turned into gates when the block starts
     float ga = 0.f, gb = 0.f;
     auto gate_load = [&](int r0) {
-        if (warp == 1 && lane < SCAN_BLK && r0 + lane < p.n_rows) {
-            const float* a = p.ab + (uint64_t)(r0 + lane) * (2 * g.n_v) + h;
+        if (threadIdx.x < SCAN_BLK && r0 + (int)threadIdx.x < p.n_rows) {
+            const float* a = p.ab + (uint64_t)(r0 + threadIdx.x) * (2 * g.n_v) + h;
             ga = __ldcg(a);
             gb = __ldcg(a + g.n_v);
         }
     };
-    auto gate_store = [&](int r0, int par) {
-        if (warp != 1) return;
-        const int n = next_of(r0) - r0;
-        if (lane < SCAN_BLK) {
-            sm.gs[par][lane] = lane < n ? expf(softplus_f(ga + dtb) * alog) : 1.f;
-            sm.bs[par][lane] = lane < n ? sigmoid_f(gb) : 0.f;
-            const int kr = r0 + lane - ckpt;
-            if (p.last_rows && kr >= 0 && lane < n && blockIdx.y == 0) {
-                p.keep_ab[(uint64_t)kr * (2 * g.n_v) + h] = ga;
-                p.keep_ab[(uint64_t)kr * (2 * g.n_v) + g.n_v + h] = gb;
-            }
+    auto gate_store = [&](int r0, int buf) {
+        if (threadIdx.x >= SCAN_BLK) return;
+        const int n = next_of(r0) - r0, i = threadIdx.x;
+        sm.gs[buf][i] = i < n ? expf(softplus_f(ga + dtb) * alog) : 1.f;
+        sm.bs[buf][i] = i < n ? sigmoid_f(gb) : 0.f;
+        const int kr = r0 + i - ckpt;
+        if (p.last_rows && kr >= 0 && i < n && blockIdx.y == 0) {
+            p.keep_ab[(uint64_t)kr * (2 * g.n_v) + h] = ga;
+            p.keep_ab[(uint64_t)kr * (2 * g.n_v) + g.n_v + h] = gb;
         }
-        __syncwarp();
-        const int i = lane & 15;   // G_i and D_15,i
-        float v = 1.f;
-#pragma unroll
-        for (int t = 0; t < SCAN_BLK; ++t)
-            if (lane < 16 ? t <= i : t > i) v *= sm.gs[par][t];
-        (lane < 16 ? sm.G : sm.D)[par][i] = v;
     };
-    // k_j . k_i and k_j . q_i of a block: warp 4 + x = channels 32 x .., lane = two rows j x eight vectors
-    auto gram = [&](int buf) {
-        if (warp < 4) return;
-        float acc[2][8];
+    auto put = [&](float* dst) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + s_off + (r ^ rr) * 128) = make_float4(S[r][0], S[r][1], S[r][2], S[r][3]);
+    };
+    // dot products of the four rows with the block's sixteen rows of `src`, summed over the lanes: tokens 2 lg and 2 lg + 1 of row rr
+    auto dots = [&](const float (*src)[128], float& d0, float& d1) {
+        float v[64];   // [row slot][token slot]; token slot t is token t ^ 2 lg
 #pragma unroll
-            for (int n = 0; n < 8; ++n) acc[i][n] = 0.f;
-#pragma unroll 2
-        for (int kk = 0; kk < 32; kk += 4) {
-            float4 r[2];
+        for (int t = 0; t < SCAN_BLK; ++t) {
+            const float4 x = *reinterpret_cast<const float4*>(&src[t ^ (2 * lg)][4 * lane]);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) r[i] = *reinterpret_cast<const float4*>(&sm.kq[buf][rg + 8 * i][c0 + kk]);
-#pragma unroll
-            for (int n = 0; n < 8; ++n) {
-                const float4 x = *reinterpret_cast<const float4*>(&sm.kq[buf][vg + 4 * n][c0 + kk]);
-#pragma unroll
-                for (int i = 0; i < 2; ++i) acc[i][n] = fmaf(r[i].w, x.w, fmaf(r[i].z, x.z, fmaf(r[i].y, x.y, fmaf(r[i].x, x.x, acc[i][n]))));
-            }
+            for (int r = 0; r < 4; ++r) v[16 * r + t] = fmaf(S[r][3], x.w, fmaf(S[r][2], x.z, fmaf(S[r][1], x.y, S[r][0] * x.x)));
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int n = 32; n >= 2; n >>= 1) {
 #pragma unroll
-            for (int n = 0; n < 8; ++n) sm.gram[warp & 3][(rg + 8 * i) * SCAN_RS + vg + 4 * n] = acc[i][n];
+            for (int i = 0; i < n; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i + n], n / 2);
+        }
+        d0 = v[0]; d1 = v[1];
     };
     // the conv rows before the last block replace the pass's first ones, which the front kernel has read; one slice per CTA
     if (p.last_rows) {
         const int n = 3 * g.conv_dim() / 4, per = (n + gridDim.x * gridDim.y - 1) / (gridDim.x * gridDim.y);
-        const int first = (blockIdx.y * gridDim.x + blockIdx.x) * per;
-        for (int i = first + threadIdx.x; i < min(n, first + per); i += 256)
+        const int c0 = (blockIdx.y * gridDim.x + blockIdx.x) * per;
+        for (int i = c0 + threadIdx.x; i < min(n, c0 + per); i += 256)
             reinterpret_cast<float4*>(p.conv_in)[i] = __ldcg(reinterpret_cast<const float4*>(p.keep_pre) + i);
     }
     fetch(0, 0);
     gate_load(0);
-    fetch(next_of(0), 1);
-    gate_store(0, 0);
-    gate_load(next_of(0));
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
-    gram(0);
-    int buf = 0, par = 0;
-    for (int r0 = 0; r0 < p.n_rows;) {
-        const int r1 = next_of(r0), n = r1 - r0, nbuf = buf == SCAN_BUFS - 1 ? 0 : buf + 1, fbuf = nbuf == SCAN_BUFS - 1 ? 0 : nbuf + 1;
-        // ---- A: u = S0 k, w = S0 q
-        {
-            const int v0 = (warp >> 2) * 16;
-            float acc[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int m = 0; m < 4; ++m) acc[i][m] = 0.f;
-#pragma unroll 4
-            for (int kk = 0; kk < 32; kk += 4) {
-                float4 r[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(&sm.s[rg + 8 * i][c0 + kk]);
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const float4 x = *reinterpret_cast<const float4*>(&sm.kq[buf][v0 + vg + 4 * m][c0 + kk]);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[i][m] = fmaf(r[i].w, x.w, fmaf(r[i].z, x.z, fmaf(r[i].y, x.y, fmaf(r[i].x, x.x, acc[i][m]))));
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int m = 0; m < 4; ++m) sm.red[warp & 3][(rg + 8 * i) * SCAN_RS + v0 + vg + 4 * m] = acc[i][m];
-        }
-        __syncthreads();   // also: gram and gates of this block
-        // ---- B: lane = vector
-        if (r1 < p.n_rows) fetch(next_of(r1), fbuf);   // its last reader was phase D of the block before
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int at = (warp + 8 * m) * SCAN_RS + lane;
-            sm.a[lane][warp + 8 * m] = (sm.red[0][at] + sm.red[1][at]) + (sm.red[2][at] + sm.red[3][at]);
-        }
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int j = warp + 8 * m, i = lane & 15, at = j * SCAN_RS + lane;
-            float d = 1.f;   // D_ij
-#pragma unroll
-            for (int t = 1; t < SCAN_BLK; ++t)
-                if (t > j && t <= i) d *= sm.gs[par][t];
-            const float dot = (sm.gram[0][at] + sm.gram[1][at]) + (sm.gram[2][at] + sm.gram[3][at]);
-            if (lane < 16) sm.L[j][i] = i > j ? sm.bs[par][i] * d * dot : 0.f;
-            else sm.M[j][i] = i >= j ? d * dot : 0.f;
-        }
-        if (r1 < p.n_rows) asm volatile("cp.async.wait_group 1;" ::: "memory");   // the next block's rows
-        __syncthreads();
-        // ---- C
-        if (warp == 0) {   // lane = state row
-            float u[SCAN_BLK];
-#pragma unroll
-            for (int i = 0; i < SCAN_BLK; ++i) u[i] = sm.bs[par][i] * (sm.vs[buf][i][lane] - sm.G[par][i] * sm.a[i][lane]);
-#pragma unroll
-            for (int j = 0; j < SCAN_BLK; ++j) {
-                sm.C[j][lane] = u[j];
-#pragma unroll
-                for (int i4 = (j + 1) / 4; i4 < 4; ++i4) {
-                    const float4 l = *reinterpret_cast<const float4*>(&sm.L[j][4 * i4]);
-                    if (4 * i4 > j) u[4 * i4] = fmaf(-l.x, u[j], u[4 * i4]);
-                    if (4 * i4 + 1 > j) u[4 * i4 + 1] = fmaf(-l.y, u[j], u[4 * i4 + 1]);
-                    if (4 * i4 + 2 > j) u[4 * i4 + 2] = fmaf(-l.z, u[j], u[4 * i4 + 2]);
-                    if (4 * i4 + 3 > j) u[4 * i4 + 3] = fmaf(-l.w, u[j], u[4 * i4 + 3]);
-                }
-            }
-        } else if (r1 < p.n_rows) {
-            if (warp == 1) {
-                gate_store(r1, par ^ 1);
-                gate_load(next_of(r1));
-            }
-            gram(nbuf);
+    int buf = 0;
+    for (int r0 = 0; r0 < p.n_rows; buf ^= 1) {
+        const int r1 = next_of(r0), n = r1 - r0;
+        gate_store(r0, buf);
+        if (r1 < p.n_rows) {
+            fetch(r1, buf ^ 1);
+            gate_load(r1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncthreads();
-        // ---- D: outputs of tokens warp, warp + 8 (lane = state row); state rows 4 warp .. + 3 (lane = four channels)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int i = warp + 8 * half;
-            float o0 = sm.G[par][i] * sm.a[16 + i][lane], o1 = 0.f;
-#pragma unroll
-            for (int j = 0; j < SCAN_BLK; j += 2) {   // M is zero for j > i
-                o0 = fmaf(sm.M[j][i], sm.C[j][lane], o0);
-                o1 = fmaf(sm.M[j + 1][i], sm.C[j + 1][lane], o1);
-            }
-            if (i < n) p.o[((uint64_t)(r0 + i) * g.n_v + h) * 128 + dv_cta + lane] = o0 + o1;
-        }
+        // ---- the block's Gram matrices and decays: a thread computes a 4 x 4 tile of K K^T or Q K^T over sixteen of the 128 channels,
+        // eight lanes share a tile (the eight warps: 2 matrices x 16 tiles)
         {
-            const float Gend = sm.G[par][SCAN_BLK - 1];
-            float4 s4[4];
+            const int tile = threadIdx.x >> 3, i0 = ((tile >> 2) & 3) * 4, j0 = (tile & 3) * 4;
+            const bool is_m = tile >= 16;
+            if (j0 <= i0) {   // uniform over the tile's eight lanes
+                const float(*ri)[128] = is_m ? sm.qs[buf] : sm.ks[buf];
+                float acc[16];
+#pragma unroll
+                for (int x = 0; x < 16; ++x) acc[x] = 0.f;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float4 a[4], b[4];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        a[x] = *reinterpret_cast<const float4*>(&ri[i0 + x][32 * c + 4 * lg]);
+                        b[x] = *reinterpret_cast<const float4*>(&sm.ks[buf][j0 + x][32 * c + 4 * lg]);
+                    }
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+#pragma unroll
+                        for (int y = 0; y < 4; ++y)
+                            acc[4 * x + y] = fmaf(a[x].w, b[y].w, fmaf(a[x].z, b[y].z, fmaf(a[x].y, b[y].y, fmaf(a[x].x, b[y].x, acc[4 * x + y]))));
+                }
+                const uint32_t mask = 0xffu << (lane & 24);
+#pragma unroll
+                for (int n = 8; n >= 2; n >>= 1) {   // lane lg keeps entries 2 lg, 2 lg + 1
+                    const bool up = lg & (n / 2);
+#pragma unroll
+                    for (int x = 0; x < n; ++x) {
+                        const float give = up ? acc[x] : acc[x + n], keep = up ? acc[x + n] : acc[x];
+                        acc[x] = keep + __shfl_xor_sync(mask, give, n / 2);
+                    }
+                }
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int e = 2 * lg + x, i = i0 + (e >> 2), j = j0 + (e & 3);
+                    float dec = 1.f;   // D_ij
+#pragma unroll
+                    for (int t = 1; t < SCAN_BLK; ++t) dec *= (t > j && t <= i) ? sm.gs[buf][t] : 1.f;
+                    if (is_m) sm.M[i][j] = j <= i ? dec * acc[x] : 0.f;
+                    else sm.L[j][i] = j < i ? sm.bs[buf][i] * dec * acc[x] : 0.f;
+                }
+            } else if (is_m) {   // above the diagonal
+                sm.M[i0 + (lg >> 1)][j0 + 2 * (lg & 1)] = 0.f;
+                sm.M[i0 + (lg >> 1)][j0 + 2 * (lg & 1) + 1] = 0.f;
+            }
+            if (threadIdx.x >= 256 - 32) {   // G_i and D_15,i
+                const int i = lane & 15;
+                float v = 1.f;
+#pragma unroll
+                for (int t = 0; t < SCAN_BLK; ++t) v *= (lane < 16 ? t <= i : t > i) ? sm.gs[buf][t] : 1.f;
+                (lane < 16 ? sm.G : sm.D)[i] = v;
+            }
+        }
+        // ---- u = S0 k, w = S0 q
+        float u01[2], w01[2];
+        dots(sm.ks[buf], u01[0], u01[1]);
+        dots(sm.qs[buf], w01[0], w01[1]);
+        __syncthreads();   // L, M, G, D
+        // ---- substitution, by all eight lanes of a row alike: u becomes c
+        float u[SCAN_BLK];
+#pragma unroll
+        for (int i = 0; i < SCAN_BLK; ++i) u[i] = __shfl_sync(0xffffffffu, u01[i & 1], 8 * rr + (i >> 1));
+#pragma unroll
+        for (int i = 0; i < SCAN_BLK; ++i) u[i] = sm.bs[buf][i] * (sm.vs[buf][i][dv_l] - sm.G[i] * u[i]);
+#pragma unroll
+        for (int j = 0; j < SCAN_BLK - 1; ++j) {
+#pragma unroll
+            for (int i4 = (j + 1) / 4; i4 < 4; ++i4) {
+                const float4 l = *reinterpret_cast<const float4*>(&sm.L[j][4 * i4]);
+                if (4 * i4 > j) u[4 * i4] = fmaf(-l.x, u[j], u[4 * i4]);
+                if (4 * i4 + 1 > j) u[4 * i4 + 1] = fmaf(-l.y, u[j], u[4 * i4 + 1]);
+                if (4 * i4 + 2 > j) u[4 * i4 + 2] = fmaf(-l.z, u[j], u[4 * i4 + 2]);
+                if (4 * i4 + 3 > j) u[4 * i4 + 3] = fmaf(-l.w, u[j], u[4 * i4 + 3]);
+            }
+        }
+        // ---- outputs of tokens 2 lg, 2 lg + 1; c for the state
+        float* o_row = p.o + (uint64_t)r0 * g.n_v * 128 + h * 128 + dv;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const int i = 2 * lg + t;
+            float o0 = sm.G[i] * w01[t], o1 = 0.f;
+#pragma unroll
+            for (int j4 = 0; j4 < 4; ++j4) {
+                const float4 m = *reinterpret_cast<const float4*>(&sm.M[i][4 * j4]);
+                o0 = fmaf(m.x, u[4 * j4], o0); o1 = fmaf(m.y, u[4 * j4 + 1], o1);
+                o0 = fmaf(m.z, u[4 * j4 + 2], o0); o1 = fmaf(m.w, u[4 * j4 + 3], o1);
+            }
+            if (i < n) o_row[(uint64_t)i * g.n_v * 128] = o0 + o1;
+        }
+        if (lg == 0) {
+#pragma unroll
+            for (int j4 = 0; j4 < 4; ++j4) {
+                const float4 d = *reinterpret_cast<const float4*>(&sm.D[4 * j4]);
+                *reinterpret_cast<float4*>(&sm.C[dv_l][4 * j4]) = make_float4(u[4 * j4] * d.x, u[4 * j4 + 1] * d.y, u[4 * j4 + 2] * d.z, u[4 * j4 + 3] * d.w);
+            }
+        }
+        __syncwarp();
+        // ---- state
+        const float Gend = sm.G[SCAN_BLK - 1];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) S[r][e] *= Gend;
+#pragma unroll
+        for (int i4 = 0; i4 < 4; ++i4) {
+            float4 k4[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) k4[t] = *reinterpret_cast<const float4*>(&sm.ks[buf][4 * i4 + t][4 * lane]);
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                s4[r] = *reinterpret_cast<const float4*>(&sm.s[4 * warp + r][4 * lane]);
-                s4[r].x *= Gend; s4[r].y *= Gend; s4[r].z *= Gend; s4[r].w *= Gend;
-            }
+                const float4 c4 = *reinterpret_cast<const float4*>(&sm.C[warp * 4 + (r ^ rr)][4 * i4]);
+                const float c[4] = {c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
-            for (int j = 0; j < SCAN_BLK; ++j) {
-                const float4 k = *reinterpret_cast<const float4*>(&sm.kq[buf][j][4 * lane]), c4 = *reinterpret_cast<const float4*>(&sm.C[j][4 * warp]);
-                const float d = sm.D[par][j], c[4] = {d * c4.x, d * c4.y, d * c4.z, d * c4.w};
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    s4[r].x = fmaf(c[r], k.x, s4[r].x); s4[r].y = fmaf(c[r], k.y, s4[r].y);
-                    s4[r].z = fmaf(c[r], k.z, s4[r].z); s4[r].w = fmaf(c[r], k.w, s4[r].w);
+                for (int t = 0; t < 4; ++t) {
+                    S[r][0] = fmaf(c[t], k4[t].x, S[r][0]); S[r][1] = fmaf(c[t], k4[t].y, S[r][1]);
+                    S[r][2] = fmaf(c[t], k4[t].z, S[r][2]); S[r][3] = fmaf(c[t], k4[t].w, S[r][3]);
                 }
             }
-            float* out = r1 == p.n_rows ? p.state_out : p.last_rows && r1 == ckpt ? p.state_in : nullptr;
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                *reinterpret_cast<float4*>(&sm.s[4 * warp + r][4 * lane]) = s4[r];
-                if (out) *reinterpret_cast<float4*>(out + s_off + (4 * warp + r) * 128 + 4 * lane) = s4[r];
-            }
         }
-        __syncthreads();
-        r0 = r1; buf = nbuf; par ^= 1;
+        r0 = r1;
+        if (p.last_rows && r0 == ckpt) put(p.state_in);
+        __syncthreads();   // this block's buffers, L, M, G and D are free
     }
+    put(p.state_out);
 }
 
 dfl_status launch_tm_gdn_scan(cudaStream_t st, const TmGdn& p) {
-    static std::once_flag once[16];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaError_t e = cudaSuccess;
-    auto allow = [&] { e = cudaFuncSetAttribute(tm_gdn_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ScanSmem)); };
-    if (dev >= 0 && dev < 16) std::call_once(once[dev], allow);
-    else allow();
-    DFL_CUDA(e);
     launch_k(tm_gdn_scan_kernel, dim3((unsigned)p.g.n_v, 4), dim3(256), sizeof(ScanSmem), st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
