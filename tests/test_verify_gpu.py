@@ -197,6 +197,27 @@ def test_routed_expert_ffn_matches_oracle():
     gm.close()
 
 
+@pytest.mark.parametrize("experts,used", [(40, 3), (256, 8), (257, 5), (400, 32)])
+def test_routing_of_many_experts_matches_oracle(experts, used):
+    # one warp's registers hold 8 or 32 experts a lane (the line lies at 256); 400 experts with 32 a row leave the down projection some
+    # seventy slices, more than the glue stages at a time.  f32 throughout: the file's tolerances.
+    arch = modelgen.tiny_arch(n_layer=1, expert_count=experts, expert_used_count=used, expert_feed_forward_length=256,
+                              expert_shared_feed_forward_length=256)
+    T = modelgen.target_tensors(arch, seed=23)
+    om, gm = modelgen.OracleModel(arch, T), pkg.Model(arch, T)
+    sess, scr = pkg.Session(gm, 64, False), pkg.Scratch(gm, 16, 1)
+    ost, start = om.new_state(64, False), 0
+    rng = np.random.default_rng(7)
+    for n in (16, 1, 5):
+        tokens = rng.integers(0, arch.vocab_size, size=n)
+        want, _ = oracle_block(om, ost, tokens, start, [0])
+        _, _, got = pkg.packed_verify(gm, sess, scr, [0], tokens, start, want_logits=True)
+        np.testing.assert_allclose(got, want, rtol=RTOL, atol=ATOL)
+        start += n
+    for o in (sess, scr, gm):
+        o.close()
+
+
 @pytest.mark.parametrize("kv_f16", [False, True])
 def test_verify_over_a_multi_chunk_kv_cache_with_rollback(tiny, kv_f16):
     # long-context shape of the step in miniature: the block attends over several 64-position KV chunks (partial
