@@ -199,8 +199,8 @@ struct dfl_c1 {
     int device;   // kept here: a pipeline may be dropped after its matrices
     cudaStream_t st;
     float *x, *part1, *part2, *logits;
-    uint8_t *acts1, *acts2;
-    uint8_t* block;   // backs x .. acts2
+    uint8_t *acts1, *acts2, *dry;   // dry: GlueParams::dry
+    uint8_t* block;   // backs x .. dry
     int splits1, splits2;
     cudaEvent_t e0, e1;
     // pinned host memory that the kernels read and write themselves: the results and the error word (HostOut), then the block's rows
@@ -340,7 +340,7 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
     // the block's buffers from the pool, one after another in one block: pipelines come and go with their requests
     auto up = [](size_t bytes) { return (bytes + 511) / 512 * 512; };
     const size_t sizes[] = {up(MAX_ROWS * k1 * 4), up((size_t)p->splits1 * MAX_ROWS * n1 * 4), up((size_t)p->splits2 * MAX_ROWS * v * 4), up(MAX_ROWS * v * 4),
-                            up(acts_bytes_for(w1->m)), up(acts_bytes_for(head->m))};
+                            up(acts_bytes_for(w1->m)), up(acts_bytes_for(head->m)), up(GLUE_DRY_BYTES)};
     size_t total = 0;
     for (size_t n : sizes) total += n;
     ok = ok && (p->block = (uint8_t*)pool_alloc(total));
@@ -353,6 +353,7 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
         p->logits = (float*)next(3);
         p->acts1 = next(4);
         p->acts2 = next(5);
+        p->dry = next(6);
     }
     ok = ok && cudaEventCreate(&p->e0) == cudaSuccess && cudaEventCreate(&p->e1) == cudaSuccess;
     static_assert(sizeof(dfl_c1::HostOut) <= 256, "the rows follow 256 bytes further");
@@ -366,6 +367,7 @@ dfl_status dfl_c1_create(const dfl_qmatrix* w1, const dfl_qmatrix* head, dfl_c1*
     // the parts of the packed rows that the glue kernel does not write stay zero
     cudaMemsetAsync(p->acts1, 0, acts_bytes_for(w1->m), p->st);
     cudaMemsetAsync(p->acts2, 0, acts_bytes_for(head->m), p->st);
+    cudaMemsetAsync(p->dry, 0, GLUE_DRY_BYTES, p->st);
     cudaStreamSynchronize(p->st);
     *out = p;
     return DFL_OK;
@@ -398,6 +400,7 @@ static dfl_status c1_enqueue(dfl_c1* p, const float* x, int n_rows) {
     GlueParams mid;
     mid.part = p->part1; mid.splits = p->splits1; mid.ld_part = (int)a.n_out; mid.acts = p->acts2; mid.bf3 = act_layout_of(b);
     mid.n_rows = n_rows; mid.err = err;
+    mid.dry = p->dry;
     DFL_CHECK(launch_glue(p->st, mid, a.n_out));
     DFL_CHECK(launch_gemm_fewrow(p->st, b, p->acts2, p->splits2 == 1 ? p->logits : p->part2, p->splits2, GemmEpilogue{}, err, true));
     if (p->splits2 == 1) return launch_argmax_top2(p->st, p->logits, n_rows, b.n_out, b.n_out, p->out->argmax, p->out->gap);

@@ -154,15 +154,20 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
     if (!p.trigger_late) pdl_launch_dependents();
+    // Without a wait of its own a kernel still must not find older lines in its SM's first-level cache: what the wait would do, a fence does.
+    auto wait_inputs = [&] {
+        if (p.wait_last) __threadfence();
+        else pdl_wait();
+    };
     int row_tiles = p.row_tiles, kblocks = p.kblocks, splits = p.splits, cps = p.ctas_per_split;
     if (p.tile_map || p.kb_map) {   // the lists come from the preceding kernel: nothing may be fetched before it is complete
-        if (!p.wait_last) pdl_wait();
-        if (p.tile_map) row_tiles = __ldcg(p.n_tiles);
+        wait_inputs();
+        if (p.tile_map) row_tiles = *p.n_tiles;
         if (p.kb_map) {
-            kblocks = __ldcg(p.n_kb);
-            if (__ldcg(p.n_kb + 1) > 0) {   // the list's author also chose the split geometry for its length (the launch is the worst case)
-                splits = __ldcg(p.n_kb + 1);
-                cps = __ldcg(p.n_kb + 2);
+            kblocks = p.n_kb[0];
+            if (p.n_kb[1] > 0) {   // the list's author also chose the split geometry for its length (the launch is the worst case)
+                splits = p.n_kb[1];
+                cps = p.n_kb[2];
             }
         }
     }
@@ -198,8 +203,8 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
             if (round == 1 && s == 0) trigger();
             if (mapped) {
                 const int slot = c + pt * cps;
-                src = p.w + (uint64_t)(p.tile_map ? __ldcg(p.tile_map + slot) : slot) * tile_stride +
-                      (uint64_t)(p.kb_map ? __ldcg(p.kb_map + kb0 + pk) : kb0 + pk) * F::STAGE;
+                src = p.w + (uint64_t)(p.tile_map ? p.tile_map[slot] : slot) * tile_stride +
+                      (uint64_t)(p.kb_map ? p.kb_map[kb0 + pk] : kb0 + pk) * F::STAGE;
             }
             if (lane == 0) {
                 uint64_t* fb = full_bar(full, e, s);
@@ -331,7 +336,7 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
         if (uses < 2) trigger();
     } else {
         // ------------------------------ draining warps ------------------------------
-        if (!p.wait_last) pdl_wait();
+        wait_inputs();
         trigger();
         const int dtid = threadIdx.x - DRAIN_WARP0 * 32;   // 0..127 = weight row of the tile = tensor-memory lane
         if (dtid == 0 && n_it > 0) {
@@ -340,7 +345,7 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
             // busy priming the weight ring.
             for (int k = 0; k < n_kb; ++k) {
                 mbar_arrive_expect_tx(&acts_bar[k], ACTTS_CHUNK);
-                bulk_g2s(acts_res + k * ACTTS_CHUNK, p.acts + (uint64_t)(p.kb_map ? __ldcg(p.kb_map + kb0 + k) : kb0 + k) * ACTTS_CHUNK, ACTTS_CHUNK, &acts_bar[k]);
+                bulk_g2s(acts_res + k * ACTTS_CHUNK, p.acts + (uint64_t)(p.kb_map ? p.kb_map[kb0 + k] : kb0 + k) * ACTTS_CHUNK, ACTTS_CHUNK, &acts_bar[k]);
             }
         }
         {
@@ -348,7 +353,7 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
             const int tok = dtid >> 3, part = dtid & 7;
             float ss = 0.f;
             if (p.sumsq)
-                for (int q = part; q < p.n_sumsq; q += 8) ss += __ldcg(p.sumsq + q * MAX_ROWS + tok);
+                for (int q = part; q < p.n_sumsq; q += 8) ss += p.sumsq[q * MAX_ROWS + tok];
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
             if (part == 0) tok_scale[tok] = p.sumsq ? p.out_scale * (1.0f / sqrtf(ss / p.norm_k + p.eps)) : p.out_scale;
@@ -404,7 +409,7 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
                 kb_e = 0;
                 const int slot = c + tile * cps;
                 ++tile;
-                const uint32_t orow = (uint32_t)(p.tile_map ? __ldcg(p.tile_map + slot) : slot) * TILE_R + row;
+                const uint32_t orow = (uint32_t)(p.tile_map ? p.tile_map[slot] : slot) * TILE_R + row;
                 if (orow < p.n_out) {
                     float* dst = p.out + (uint64_t)sp * MAX_ROWS * p.ld_out + orow;
 #pragma unroll
