@@ -157,6 +157,25 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src_gmem, uint32_t 
 // allow dependents to start their prologue.  Both are no-ops for plain launches.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Start of a kernel that reads, without a dependency wait, what a grid two or more launches back wrote: launch_dependents orders no memory, so the
+// kernel between says through a mark that it has passed its own wait, which made those writes visible to it.  late_publish: by one thread of
+// that kernel, behind the wait.  late_peek, at the reader's start, and late_acquire, by every thread before its first read: the mark is usually
+// there when the reader looks, and the fence makes an acquire of the look; should it not come, the dependency wait proper takes its place.
+__device__ __forceinline__ void late_publish(uint32_t* mark, uint32_t value) { asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(mark), "r"(value) : "memory"); }
+__device__ __forceinline__ uint32_t late_peek(const uint32_t* mark) {
+    uint32_t seen;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(mark) : "memory");
+    return seen;
+}
+static __device__ __noinline__ void late_wait(const uint32_t* mark, uint32_t value) {
+    for (int i = 0; i < 64; ++i)
+        if ((int32_t)(late_peek(mark) - value) >= 0) return;
+    pdl_wait();
+}
+__device__ __forceinline__ void late_acquire(const uint32_t* mark, uint32_t value, uint32_t seen) {
+    if ((int32_t)(seen - value) < 0) late_wait(mark, value);
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+}
 
 #endif  // __CUDACC__
 

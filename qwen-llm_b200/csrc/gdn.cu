@@ -40,20 +40,22 @@ dfl_status launch_gdn_conv_restore(cudaStream_t st, const GdnGeom& g, const floa
 // ---- alpha and beta projections ----------------------------------------------------------------------
 // A CTA of 128 threads per four outputs and 512 columns, a thread four columns; rows four at a time, so that a CTA's registers fit beside
 // the qkv projection's GEMM CTA and the whole kernel runs in its shadow.  (As CTAs of their own behind the z projection, sixteen that read all rows,
-// the projections held up the mixer for 7 us.)  Its start says that xn is complete when the GEMM before was launched with trigger_late; the
+// the projections held up the mixer for 7 us.)  Behind a GEMM launched with trigger_late it acquires that launch's mark instead of waiting, and the
 // dependency wait at its end makes its own completion say that the GEMM's outputs are there too, which the kernels behind rely on.
 constexpr int AB_OUT = 4;
 static_assert(AB_COLS == 128 * 4, "four columns a thread");
 __global__ void __launch_bounds__(128, 7) ab_proj_kernel(const float* __restrict__ w, const float* xn, int ld_xn, int n_rows, int k, int n_out,
-                                                         float* ab_part, int wait_first) {
+                                                         float* ab_part, LateMark late) {
     __shared__ float red[4][MAX_ROWS * AB_OUT];
     const int o0 = blockIdx.x * AB_OUT, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.y * AB_COLS + threadIdx.x * 4;
+    const uint32_t late_seen = late.word ? late_peek(late.word) : 0u;
     float4 wv[AB_OUT];   // outputs beyond the last read its row and are not stored
 #pragma unroll
     for (int j = 0; j < AB_OUT; ++j)
         wv[j] = c < k ? *reinterpret_cast<const float4*>(w + (uint64_t)min(o0 + j, n_out - 1) * k + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     pdl_launch_dependents();
-    if (wait_first) pdl_wait();
+    if (late.word) late_acquire(late.word, late.value, late_seen);
+    else pdl_wait();
     float4 x[4];
     auto fetch = [&](int t0) {
 #pragma unroll
@@ -87,14 +89,14 @@ __global__ void __launch_bounds__(128, 7) ab_proj_kernel(const float* __restrict
         const float t = (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
         if (tok < n_rows && o < n_out) ab_part[((uint64_t)blockIdx.y * MAX_ROWS + tok) * n_out + o] = t;
     }
-    if (!wait_first) pdl_wait();
+    if (late.word) pdl_wait();
 }
 
 dfl_status launch_ab_proj(cudaStream_t st, const float* w, const float* xn, int ld_xn, int n_rows, uint64_t k, int n_out, float* ab_part,
-                          bool behind_late_gemm) {
+                          LateMark late) {
     if (k % 4) return fail(DFL_ERR_BAD_SHAPE, "ab_proj: k must be a multiple of 4");
     launch_k(ab_proj_kernel, dim3((unsigned)((n_out + AB_OUT - 1) / AB_OUT), (unsigned)ab_slices(k)), dim3(128), 0, st, w, xn, ld_xn, n_rows, (int)k,
-             n_out, ab_part, behind_late_gemm ? 0 : 1);
+             n_out, ab_part, late);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

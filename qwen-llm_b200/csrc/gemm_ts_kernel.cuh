@@ -39,9 +39,15 @@ struct Params {
     const int32_t* n_tiles;
     const int32_t* kb_map;     // optional: column blocks to sum over, and how many (device memory)
     const int32_t* n_kb;
-    int trigger_late;          // let the next kernel start behind the dependency wait instead of at once
-    int wait_last;             // the kernels before were launched so: the inputs are complete, the dependency wait is for the kernels behind
+    uint32_t* late_word;       // LateMark
+    uint32_t late_value;
+    int late_mode;             // LATE_FIRST: lets the next kernel start behind the dependency wait instead of at once, and publishes the mark there;
+                               // LATE_BEHIND: acquires it before the inputs, the dependency wait is for the kernels behind
 };
+
+constexpr int LATE_FIRST = 1, LATE_BEHIND = 2;
+// Every launch fetches its parameters cold: with sixteen bytes more a 9B-class verify block of 340 launches took 0.3 - 0.5 % longer.
+static_assert(sizeof(Params) <= 128, "parameters of the few-row GEMM");
 
 constexpr int FR_GROUP_WARPS = 4;                           // unpacking warps per group; thread = weight row = 32 * (warp % 4) + lane
 constexpr int FR_UNPACK_WARPS = 2 * FR_GROUP_WARPS;         // two groups that take the entries alternately
@@ -132,6 +138,7 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
     __shared__ int abort_flag;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp-uniform by construction
+    const uint32_t late_seen = p.late_mode == LATE_BEHIND ? late_peek(p.late_word) : 0u;
     if (threadIdx.x == 0) {
         for (int s = 0; s < FULL_SETS * STAGES; ++s) mbar_init(&full[s], 1);
         for (int s = 0; s < STAGES; ++s) mbar_init(&empty[s], FR_GROUP_WARPS);
@@ -153,10 +160,9 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = tmem_slot;
-    if (!p.trigger_late) pdl_launch_dependents();
-    // Without a wait of its own a kernel still must not find older lines in its SM's first-level cache: what the wait would do, a fence does.
+    if (p.late_mode != LATE_FIRST) pdl_launch_dependents();
     auto wait_inputs = [&] {
-        if (p.wait_last) __threadfence();
+        if (p.late_mode == LATE_BEHIND) late_acquire(p.late_word, p.late_value, late_seen);
         else pdl_wait();
     };
     int row_tiles = p.row_tiles, kblocks = p.kblocks, splits = p.splits, cps = p.ctas_per_split;
@@ -180,7 +186,7 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
     // The late form: every thread passes the dependency wait first, each role where it has nothing else to do (it does not matter how many of
     // a CTA's threads the hardware counts, and a second call does nothing).
     auto trigger = [&] {
-        if (!p.trigger_late) return;
+        if (p.late_mode != LATE_FIRST) return;
         pdl_wait();
         pdl_launch_dependents();
     };
@@ -221,6 +227,9 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
         }
         if (!ok) abort_flag = 1;
         trigger();
+        // Here the warp has nothing left to do, and the next kernel finds no room before this CTA and others have ended (the other roles of the
+        // first CTA, where the fence of the release held them up, made the launch 0.8 us longer).
+        if (p.late_mode == LATE_FIRST && blockIdx.x == 0 && lane == 0) late_publish(p.late_word, p.late_value);
     } else if (warp >= MMA_WARP0 && warp < MMA_WARP0 + MMA_WARPS) {
         // ------------------------------ MMA issuers ------------------------------
         // Warp (g, c) issues the halves h with h % 2 == c of group g's entries into accumulator c of that group.  The
@@ -343,6 +352,7 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
             // the activations (the previous kernel's output), in the order of their first use, one barrier each: the
             // first MMA waits for one chunk only.  Issued here rather than by the producer, whose first iterations are
             // busy priming the weight ring.
+            if (p.late_mode == LATE_BEHIND) asm volatile("fence.proxy.async.global;" ::: "memory");   // the acquire above counts for bulk copies too
             for (int k = 0; k < n_kb; ++k) {
                 mbar_arrive_expect_tx(&acts_bar[k], ACTTS_CHUNK);
                 bulk_g2s(acts_res + k * ACTTS_CHUNK, p.acts + (uint64_t)(p.kb_map ? p.kb_map[kb0 + k] : kb0 + k) * ACTTS_CHUNK, ACTTS_CHUNK, &acts_bar[k]);
@@ -446,7 +456,7 @@ __global__ void __maxnreg__(REGS) gemm_ts_kernel(const Params p) {
         fence_after_sync();
         tmem_free(tmem, TM_COLS);
     }
-    if (p.wait_last) pdl_wait();   // this kernel's completion says that those before are complete too
+    if (p.late_mode == LATE_BEHIND) pdl_wait();   // this kernel's completion says that those before are complete too
 }
 
 template <int DT, int KC>
@@ -542,9 +552,10 @@ dfl_status launch_gemm_ts(cudaStream_t st, const QMatrix& m, const uint8_t* acts
     p.n_tiles = ep.n_tiles;
     p.kb_map = ep.kb_map;
     p.n_kb = ep.n_kb;
-    p.trigger_late = ep.trigger_late;
-    p.wait_last = ep.behind_late;
-    if (ep.behind_late && ep.trigger_late) return fail(DFL_ERR_BAD_ARG, "gemm: dependency options");
+    p.late_mode = ep.trigger_late ? ts::LATE_FIRST : ep.behind_late ? ts::LATE_BEHIND : 0;
+    p.late_word = ep.late.word;
+    p.late_value = ep.late.value;
+    if ((ep.behind_late && ep.trigger_late) || ((ep.behind_late || ep.trigger_late) && !ep.late.word)) return fail(DFL_ERR_BAD_ARG, "gemm: dependency options");
     int grid = p.ctas_per_split * splits;
     if (ep.kb_map && ep.dynamic_splits && grid < sm_count()) grid = sm_count();   // room for the geometry chosen on the device
     // four resident column blocks leave room for a fourth ring slot of a 35 KB stage (4096 x 32768 Q6_K 32.0 -> 31.0 us)

@@ -223,6 +223,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
 
     DFL_CHECK(launch_embed_block(st, m->embd_dtype, m->embd_ggml, H, tokens, (int)n, sc->x, (int)H));
 
+    auto next_mark = [&] { return LateMark{sc->late_word, ++sc->late_value}; };
     auto norm_glue = [&](const float* part, int splits, int ld_part, const float* norm_w, bool want_xn, float* capture,
                          const int32_t* splits_dev = nullptr) -> dfl_status {
         GlueParams p;
@@ -257,13 +258,15 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
             // qkv: they start as its CTAs leave, and wait for it at their ends
             const MatGroup& G = L.in_qkv_z;
             const bool late = G.mats[0].layout == LAYOUT_TS && G.mats[0].dtype != DFL_BF16;
+            const LateMark mark = late ? next_mark() : LateMark{};
             for (size_t i = 0; i < G.mats.size(); ++i) {
                 GemmEpilogue ep = ep_norm;
                 ep.trigger_late = i == 0 && late;
                 ep.behind_late = i > 0 && late;
+                if (late) ep.late = mark;
                 DFL_CHECK(launch_gemm_fewrow(st, G.mats[i], sc->acts_h, sc->part + G.col_off[i], G.splits, ep, s->err, pdl_enabled(), G.total_cols));
             }
-            DFL_CHECK(launch_ab_proj(st, L.w_ab, sc->xn, (int)H, (int)n, H, 2 * gg.n_v, sc->ab_part, late));
+            DFL_CHECK(launch_ab_proj(st, L.w_ab, sc->xn, (int)H, (int)n, H, 2 * gg.n_v, sc->ab_part, mark));
             const int cur = s->ssm_cur[gi];
             GdnMixParams p;
             p.g = gg;
@@ -301,7 +304,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
                 const int min_tiles = gemm_ts_ctas_per_split(GU.mats[0].row_tiles, GU.splits);
                 const int down_tiles = down_chosen ? L.moe_down.mats[0].row_tiles : 1, down_max = down_chosen ? L.moe_down.splits : 0;
                 int32_t* kb_map = down_chosen ? sc->moe_kb_map : nullptr;
-                DFL_CHECK(launch_ab_proj(st, L.router_w, sc->xn, (int)H, (int)n, H, E + 1, sc->route_logits, false));
+                DFL_CHECK(launch_ab_proj(st, L.router_w, sc->xn, (int)H, (int)n, H, E + 1, sc->route_logits, LateMark{}));
                 RouterLogits x;
                 x.part = sc->route_logits; x.slices = ab_slices(H); x.sumsq = sc->sumsq; x.n_sumsq = kb_h; x.norm_k = (float)H; x.eps = ep_norm.eps;
                 DFL_CHECK(launch_moe_route_lists(st, x, E, (int)a.expert_used_count, (int)n, sc->route_w, sc->route_sg, sc->route_idx, (int)m->ep_e0, En,
@@ -348,6 +351,7 @@ dfl_status verify_core(const dfl_model* m, dfl_session* s, dfl_scratch* sc, cons
                 const bool late = L.moe_down_sh.mats.size() == 1 && L.moe_down_sh.mats[0].layout == LAYOUT_TS && L.moe_down_sh.mats[0].dtype != DFL_BF16 &&
                                   L.moe_down.mats.size() == 1 && L.moe_down.mats[0].layout == LAYOUT_TS && L.moe_down.mats[0].dtype != DFL_BF16;
                 ep_down.trigger_late = ep_down_exps.behind_late = late;
+                if (late) ep_down.late = ep_down_exps.late = next_mark();
                 DFL_CHECK(launch_group(st, L.moe_down_sh, sc->acts_f + (uint64_t)(En * Fe / TILE_K) * act_chunk_bytes(m->act_layout), sc->part,
                                        ep_down, s->err));
             }
@@ -848,6 +852,7 @@ dfl_status dfl_scratch_create(const dfl_model* m, uint32_t block_size, uint32_t 
     alloc(&sc->part, part * 4);
     alloc(&sc->sumsq, (H / GLUE_COLS) * MAX_ROWS * 4);
     alloc(&sc->dry, GLUE_DRY_BYTES);
+    alloc(&sc->late_word, 4);
     alloc(&sc->ab_part, (uint64_t)ab_slices(H) * MAX_ROWS * 2 * gg.n_v * 4);
     const uint64_t chunk = (uint64_t)std::max(act_chunk_bytes(ACT_F16), act_chunk_bytes(ACT_TS));
     alloc(&sc->acts_h, H / TILE_K * chunk);

@@ -188,6 +188,8 @@ struct dfl_scratch {
     uint32_t block_size = 0, k_layers = 0;
     float *x = nullptr, *xn = nullptr, *part = nullptr, *sumsq = nullptr;
     uint8_t* dry = nullptr;       // what the glue kernel runs over before its dependency wait (GlueParams::dry)
+    uint32_t* late_word = nullptr;   // LateMark of the passes over this scratch, one after another
+    uint32_t late_value = 0;
     float* ab_part = nullptr;     // alpha / beta projections of the layer at hand, in slices of columns
     uint8_t *acts_h = nullptr, *acts_f = nullptr, *acts_v = nullptr;
     float *q_rot = nullptr, *gate = nullptr;

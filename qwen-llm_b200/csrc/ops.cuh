@@ -334,12 +334,12 @@ struct GdnMixParams {
     uint64_t prefetch_bytes = 0;
 };
 dfl_status launch_gdn_mix(cudaStream_t st, const GdnMixParams& p);
-// ab_part[slice][16][o] = sum over the slice's AB_COLS columns of xn[tok][c] * w[o][c], o < n_out.  behind_late_gemm: the kernel before is a GEMM
-// launched with ep.trigger_late, so that xn is complete when this one starts; it then runs beside that GEMM.
+// ab_part[slice][16][o] = sum over the slice's AB_COLS columns of xn[tok][c] * w[o][c], o < n_out.  `late` with a word: launched as GemmEpilogue's
+// behind_late, on rows older than the GEMM with trigger_late; without: behind whatever wrote xn.
 constexpr int AB_COLS = 512;
 inline int ab_slices(uint64_t k) { return (int)((k + AB_COLS - 1) / AB_COLS); }
 dfl_status launch_ab_proj(cudaStream_t st, const float* w, const float* xn, int ld_xn, int n_rows, uint64_t k, int n_out, float* ab_part,
-                          bool behind_late_gemm);
+                          LateMark late);
 // Advances the recurrent state over the first n_rows kept rows of a block (the re-scan of a partial accept).
 dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* state_in, float* state_out, const float* k_n, const float* v,
                              const float* ab, const float* dt_bias, const float* a_log, int n_rows);
