@@ -38,9 +38,9 @@ dfl_status launch_gdn_conv_restore(cudaStream_t st, const GdnGeom& g, const floa
 }
 
 // ---- alpha and beta projections ----------------------------------------------------------------------
-// A CTA of 128 threads per four outputs and 512 columns, a thread four columns; rows four at a time, so that a CTA's registers fit beside
-// the qkv projection's GEMM CTA and the whole kernel runs in its shadow.  (As CTAs of their own behind the z projection, sixteen that read all rows,
-// the projections held up the mixer for 7 us.)  Behind a GEMM launched with trigger_late it acquires that launch's mark instead of waiting, and the
+// A CTA of 128 threads per four outputs and 512 columns, a thread four columns, rows four at a time.  Its 72 registers a thread find no room beside a
+// GEMM CTA: the CTAs start where the last projection has ended early, next to each other, and fill its uneven end.  (As sixteen CTAs behind the z
+// projection, each reading all rows, the projections held up the mixer for 7 us.)  Behind a GEMM launched with trigger_late it acquires that launch's mark instead of waiting, and the
 // dependency wait at its end makes its own completion say that the GEMM's outputs are there too, which the kernels behind rely on.
 constexpr int AB_OUT = 4;
 static_assert(AB_COLS == 128 * 4, "four columns a thread");

@@ -10,16 +10,14 @@
 
 namespace dfl {
 
-
 // grid = (k / 64, 2), block 128: thread = (token = 8 y + tid / 16, four consecutive columns).  One float4 per split per
 // thread keeps every global load of the kernel independent (one latency round); the norm weight does not depend on the
-// kernel before and is fetched ahead of the dependency wait.  128 threads, so that two such CTAs fit beside a GEMM CTA (480 threads of 96
-// registers): the following GEMM cannot start on an SM before the glue CTAs that belong there have, and its late CTAs set the
-// end of every link of the chain (verify block 3160 -> 3132 us when 256 threads became 128).
+// kernel before and is fetched ahead of the dependency wait.  128 threads: the following GEMM cannot start on an SM before the glue CTAs that
+// belong there have left, and its late CTAs set the end of every link of the chain (verify block 3160 -> 3132 us when 256 threads became 128).
 // What bounds the kernel is latency, and a good part of it was its own code: between two of its launches GEMMs stream 100 MB and more through
-// L2, so that every line of it came from far away behind the dependency wait.  The first warp therefore runs through it once
-// before, on a buffer that nobody reads (p.dry): a link of the chain 5.6 -> 5.1 us (residual), 5.6 -> 4.7 us (SwiGLU), a 9B-class verify block
-// of 97 links 2937 -> 2894 us under tracing.
+// L2, so that every line of it came from far away behind the dependency wait.  Two things follow.  The slices are fetched four at a time and not eight:
+// the shorter code was worth 1.3 % of a token, 0.9 % of a verify block.  And with DRY the first warp runs through it once before the wait, on a buffer
+// that nobody reads (p.dry); launch_glue says where.
 template <bool DRY>
 __global__ void __launch_bounds__(128, 7) glue_kernel(const GlueParams p) {
     const int quad = threadIdx.x & 15;
@@ -51,7 +49,7 @@ __global__ void __launch_bounds__(128, 7) glue_kernel(const GlueParams p) {
             }
             n_splits = p.splits_dev ? p.splits + *p.splits_dev : p.splits;
         }
-        glue_quad<DRY ? 4 : 8>(q, n_splits, cb, blockIdx.y * 8 + (threadIdx.x >> 4), quad, w);
+        glue_quad(q, n_splits, cb, blockIdx.y * 8 + (threadIdx.x >> 4), quad, w);
     }
 }
 
@@ -107,8 +105,14 @@ dfl_status launch_glue(cudaStream_t st, const GlueParams& p, uint64_t k) {
         DFL_CUDA(cudaGetLastError());
         return DFL_OK;
     }
-    // the first pass only where (nearly) all CTAs wait beside the GEMM before: behind it, it would be time lost
-    launch_k(p.dry && 2 * k / GLUE_COLS <= 3 * (uint64_t)sm_count() ? glue_kernel<true> : glue_kernel<false>, dim3((unsigned)(k / GLUE_COLS), MAX_ROWS / 8), dim3(128), 0, st, p);
+    // The run before the wait is time lost unless the CTA waits anyway.  Beside a tensor-memory GEMM CTA (17 warps of 96 registers: five on one
+    // scheduler leave room for no sixth) none does: CTAs start where that GEMM has ended early, at most one an SM of a residual glue, and a SwiGLU glue's
+    // further ones ran it behind the GEMM (verify block of 16 rows 2791 without any, 2773 with both, 2762 us with the residual one alone).  With few
+    // rows the pass proper is too short to gain (two rows 2561 without, 2588 with; five to eight 2688, 2674).  The bf16 GEMM's six warps
+    // leave room for three CTAs and more (draft 716 without, 710 with the residual one, 705 us with both).
+    const uint64_t n_cta = 2 * k / GLUE_COLS, n_sm = (uint64_t)sm_count();
+    const bool dry = p.dry && p.n_rows > 4 && (p.bf3 == ACT_TSB ? n_cta <= 3 * n_sm : p.mode != GLUE_SWIGLU && n_cta <= n_sm);
+    launch_k(dry ? glue_kernel<true> : glue_kernel<false>, dim3((unsigned)(k / GLUE_COLS), MAX_ROWS / 8), dim3(128), 0, st, p);
     count_launch();
     DFL_CUDA(cudaGetLastError());
     return DFL_OK;

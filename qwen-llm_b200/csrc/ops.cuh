@@ -143,7 +143,6 @@ __device__ __forceinline__ void glue_finish(const GlueParams& p, int cb, int tok
 // The glue of one (token, four consecutive columns) item: columns 64 cb + 4 quad .. + 3 of token `tok`.  The 32 lanes of
 // the calling warp must be two tokens x the sixteen quads of one 64-column block (lane = 16 (tok & 1) + quad): the sum
 // of squares is reduced over a token's 16 lanes and the 32-column sub-block sums over 8 lanes.
-template <int DEPTH = 4>   // residual mode: slices fetched at a time
 __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int cb, int tok, int quad, const float4 w) {   // w: the quad's mul_w
     const int col0 = cb * GLUE_COLS + quad * 4;
     const bool live = tok < p.n_rows;
@@ -180,7 +179,7 @@ __device__ __forceinline__ void glue_quad(const GlueParams& p, int n_splits, int
                 float acc[4] = {0.f, 0.f, 0.f, 0.f};
                 const float* base = p.part + (uint64_t)tok * p.ld_part + col0;
                 const uint64_t stride = (uint64_t)p.part_rows * p.ld_part;
-#pragma unroll DEPTH
+#pragma unroll 4
                 for (int s = 0; s < n_splits; ++s) {
                     const float4 a = __ldcg(reinterpret_cast<const float4*>(base + s * stride));
                     acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;

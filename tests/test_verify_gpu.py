@@ -87,6 +87,19 @@ def test_packed_verify_equals_single_token_steps_bitwise(tiny):
         x.close()
 
 
+@pytest.mark.parametrize("n", [4, 5])
+def test_blocks_on_either_side_of_the_glue_rule_give_the_same_bits(tiny, n):
+    # up to four rows the residual glue has no run ahead of its dependency wait, from five on it has one
+    arch, om, gm = tiny
+    tokens = np.random.default_rng(3).integers(0, arch.vocab_size, size=16)
+    got = []
+    for count in (n, 16):
+        sess, scr = pkg.Session(gm, 64), pkg.Scratch(gm, 16, 1)
+        got.append(pkg.packed_verify(gm, sess, scr, [3], tokens[:count], 0, want_logits=True)[2][:n].copy())
+        sess.close(); scr.close()
+    assert got[0].tobytes() == got[1].tobytes()
+
+
 @pytest.mark.parametrize("n_keep", [1, 8, 15, 16])
 def test_restore_then_marker_equals_sequential(tiny, n_keep):
     # tests.rs:6949-7110: restore(n_keep) then one marker token == n_keep sequential tokens then marker
