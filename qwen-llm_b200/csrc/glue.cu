@@ -187,8 +187,7 @@ dfl_status launch_embed_block(cudaStream_t st, int dtype, const uint8_t* ggml, u
 // ---- small f32 matrices --------------------------------------------------------------
 // A CTA of 512 threads per four output columns, a thread four columns of k at a time over all rows: the rows, which every CTA reads
 // from L2, are read a quarter as often as with one output per CTA (257 outputs over 2048 columns and 16 rows: 33 -> 8.5 MB,
-// 11.2 -> 7 us cold), and their loads are independent.  The first weights are on their way before the dependency wait, and so is the code: where
-// one round of columns is all there is, the kernel runs through it once before, on whatever xn holds, and stores nothing.  Sums over
+// 11.2 -> 7 us cold), and their loads are independent.  The first weights are on their way before the dependency wait.  Sums over
 // lanes, then warps, in a fixed order.
 constexpr int SMALL_OUT = 4;
 __global__ void __launch_bounds__(512) small_matmul_kernel(const float* __restrict__ w, const float* xn, int ld_xn,
@@ -207,59 +206,53 @@ __global__ void __launch_bounds__(512) small_matmul_kernel(const float* __restri
     }
     __shared__ float scale_s[MAX_ROWS];
     __shared__ float red[16][MAX_ROWS * SMALL_OUT];
-    pdl_launch_dependents();
-#pragma unroll 1
-    for (int pass = k <= 512 * 4 ? 0 : 1; pass < 2; ++pass) {
-        if (pass) pdl_wait();
-        c = (uint64_t)threadIdx.x * 4;
-        float acc[MAX_ROWS * SMALL_OUT];   // [row][output]
+    pdl_prologue();
+    float acc[MAX_ROWS * SMALL_OUT];   // [row][output]
 #pragma unroll
-        for (int i = 0; i < MAX_ROWS * SMALL_OUT; ++i) acc[i] = 0.f;
-        while (c < k) {
+    for (int i = 0; i < MAX_ROWS * SMALL_OUT; ++i) acc[i] = 0.f;
+    while (c < k) {
 #pragma unroll
-            for (int r = 0; r < MAX_ROWS; ++r) {
-                if (r < n_rows) {
-                    const float4 xv = __ldcg(reinterpret_cast<const float4*>(xn + (uint64_t)r * ld_xn + c));
+        for (int r = 0; r < MAX_ROWS; ++r) {
+            if (r < n_rows) {
+                const float4 xv = *reinterpret_cast<const float4*>(xn + (uint64_t)r * ld_xn + c);
 #pragma unroll
-                    for (int j = 0; j < SMALL_OUT; ++j)
-                        acc[SMALL_OUT * r + j] = fmaf(wv[j].w, xv.w, fmaf(wv[j].z, xv.z, fmaf(wv[j].y, xv.y, fmaf(wv[j].x, xv.x, acc[SMALL_OUT * r + j]))));
-                }
-            }
-            c += 512 * 4;
-            if (c < k) {
-#pragma unroll
-                for (int j = 0; j < SMALL_OUT; ++j) wv[j] = *reinterpret_cast<const float4*>(wr[j] + c);
+                for (int j = 0; j < SMALL_OUT; ++j)
+                    acc[SMALL_OUT * r + j] = fmaf(wv[j].w, xv.w, fmaf(wv[j].z, xv.z, fmaf(wv[j].y, xv.y, fmaf(wv[j].x, xv.x, acc[SMALL_OUT * r + j]))));
             }
         }
-        // per-token output scale (16 threads per token, fixed tree)
-        if (threadIdx.x < 256) {
-            const int tok = threadIdx.x >> 4, part = threadIdx.x & 15;
-            float ss = 0.f;
-            if (sumsq)
-                for (int i = part; i < n_sumsq; i += 16) ss += __ldcg(sumsq + i * MAX_ROWS + tok);
+        c += 512 * 4;
+        if (c < k) {
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            if (part == 0) scale_s[tok] = sumsq ? out_scale * (1.0f / sqrtf(ss / norm_k + eps)) : out_scale;
+            for (int j = 0; j < SMALL_OUT; ++j) wv[j] = *reinterpret_cast<const float4*>(wr[j] + c);
         }
+    }
+    // per-token output scale (16 threads per token, fixed tree)
+    if (threadIdx.x < 256) {
+        const int tok = threadIdx.x >> 4, part = threadIdx.x & 15;
+        float ss = 0.f;
+        if (sumsq)
+            for (int i = part; i < n_sumsq; i += 16) ss += sumsq[i * MAX_ROWS + tok];
 #pragma unroll
-        for (int n = 32; n >= 2; n >>= 1) {   // lane l ends with values 2 l, 2 l + 1
-            const bool up = lane & (n >> 1);
+        for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (part == 0) scale_s[tok] = sumsq ? out_scale * (1.0f / sqrtf(ss / norm_k + eps)) : out_scale;
+    }
 #pragma unroll
-            for (int i = 0; i < n; ++i) {
-                const float give = up ? acc[i] : acc[i + n], keep = up ? acc[i + n] : acc[i];
-                acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, n >> 1);
-            }
+    for (int n = 32; n >= 2; n >>= 1) {   // lane l ends with values 2 l, 2 l + 1
+        const bool up = lane & (n >> 1);
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float give = up ? acc[i] : acc[i + n], keep = up ? acc[i + n] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, n >> 1);
         }
-        *reinterpret_cast<float2*>(&red[warp][2 * lane]) = make_float2(acc[0], acc[1]);
-        __syncthreads();
-        if (threadIdx.x < MAX_ROWS * SMALL_OUT) {
-            const int r = threadIdx.x / SMALL_OUT, j = threadIdx.x % SMALL_OUT;
-            float s = 0.f;
+    }
+    *reinterpret_cast<float2*>(&red[warp][2 * lane]) = make_float2(acc[0], acc[1]);
+    __syncthreads();
+    if (threadIdx.x < MAX_ROWS * SMALL_OUT) {
+        const int r = threadIdx.x / SMALL_OUT, j = threadIdx.x % SMALL_OUT;
+        float s = 0.f;
 #pragma unroll
-            for (int wi = 0; wi < 16; ++wi) s += red[wi][threadIdx.x];
-            if (pass && r < n_rows && o0 + j < n_out) out[(uint64_t)r * ld_out + o0 + j] = s * scale_s[r];
-        }
-        __syncthreads();   // red and scale_s are free
+        for (int wi = 0; wi < 16; ++wi) s += red[wi][threadIdx.x];
+        if (r < n_rows && o0 + j < n_out) out[(uint64_t)r * ld_out + o0 + j] = s * scale_s[r];
     }
 }
 

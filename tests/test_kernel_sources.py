@@ -89,6 +89,15 @@ def test_kernels_of_the_chain_wait_before_they_read():
     assert len(launched) > 20 and launched <= waits, launched - waits
 
 
+def test_the_side_stream_s_kernels_do_not_run_ahead_of_their_wait():
+    # they start behind an event, a full dependency: there is nothing to hide a second run of the code behind
+    model = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "model.cu")).read())
+    assert set(re.findall(r"(launch_\w+)\(side,", model)) == {"launch_small_matmul", "launch_moe_route"}
+    bodies = {name: body for _, name, body in all_kernels()}
+    for name in ("small_matmul_kernel", "moe_route_kernel"):
+        assert "pdl_prologue();" in bodies[name] and not re.search(r"\bpass\b", bodies[name]), name
+
+
 def _enclosing(text, at):
     """Headers of the blocks around a position, innermost first."""
     depth = 0

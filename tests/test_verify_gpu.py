@@ -231,6 +231,27 @@ def test_routing_of_many_experts_matches_oracle(experts, used):
         o.close()
 
 
+@pytest.mark.parametrize("hidden", [256, 2304])
+def test_experts_of_two_formats_are_all_streamed_and_match_the_oracle(hidden):
+    # gate Q4_K, up Q5_K: no list of chosen tiles, the router's projection runs beside the GEMMs (one round of 2048 columns, and a second of 256)
+    arch = modelgen.tiny_arch(n_layer=1, hidden_size=hidden, expert_count=7, expert_used_count=2, expert_feed_forward_length=256,
+                              expert_shared_feed_forward_length=256)
+    rng = np.random.default_rng(8)
+    T = [(n, orc.Q5_K, s, orc.quantize(orc.Q5_K, (rng.standard_normal((7 * 256, hidden)) * 0.02).astype(np.float32))) if n.endswith("ffn_up_exps.weight") else (n, d, s, r)
+         for n, d, s, r in modelgen.target_tensors(arch, seed=29)]
+    om, gm = modelgen.OracleModel(arch, T), pkg.Model(arch, T)
+    sess, scr = pkg.Session(gm, 64, False), pkg.Scratch(gm, 16, 1)
+    ost, start = om.new_state(64, False), 0
+    for n in (16, 1):
+        tokens = rng.integers(0, arch.vocab_size, size=n)
+        want, _ = oracle_block(om, ost, tokens, start, [0])
+        _, _, got = pkg.packed_verify(gm, sess, scr, [0], tokens, start, want_logits=True)
+        np.testing.assert_allclose(got, want, rtol=RTOL, atol=ATOL)
+        start += n
+    for o in (sess, scr, gm):
+        o.close()
+
+
 @pytest.mark.parametrize("kv_f16", [False, True])
 def test_verify_over_a_multi_chunk_kv_cache_with_rollback(tiny, kv_f16):
     # long-context shape of the step in miniature: the block attends over several 64-position KV chunks (partial
