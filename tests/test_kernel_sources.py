@@ -98,6 +98,12 @@ def test_the_side_stream_s_kernels_do_not_run_ahead_of_their_wait():
         assert "pdl_prologue();" in bodies[name] and not re.search(r"\bpass\b", bodies[name]), name
 
 
+def test_both_routing_kernels_have_both_register_widths():
+    moe = open(os.path.join(CSRC, "moe.cu")).read()
+    for kernel in ("moe_route_kernel", "moe_route_lists_kernel"):
+        assert re.search(r"n_expert <= ROUTE_NARROW \? " + kernel + r"<ROUTE_NARROW / 32> : " + kernel + r"<MOE_MAX_EXPERTS / 32>", moe), kernel
+
+
 def _enclosing(text, at):
     """Headers of the blocks around a position, innermost first."""
     depth = 0

@@ -93,6 +93,16 @@ def test_prompt_pass_with_routed_experts(n, start):
     gm.close()
 
 
+@pytest.mark.parametrize("experts", [256, 257])
+def test_prompt_routing_on_either_side_of_the_register_widths(experts):
+    # a row's probabilities sit in 8 registers a lane up to 256 experts, in 32 beyond
+    arch = modelgen.tiny_arch(n_layer=1, expert_count=experts, expert_used_count=5, expert_feed_forward_length=256, expert_shared_feed_forward_length=256,
+                              intermediate_size=0)
+    gm = pkg.Model(arch, modelgen.target_tensors(arch, seed=3))
+    _check(arch, gm, 40, 0, [0])
+    gm.close()
+
+
 def test_prompt_pass_at_routed_widths():
     arch = syn.arch_35b_a3b()
     arch.n_layer = 4
