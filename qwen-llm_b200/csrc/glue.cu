@@ -54,8 +54,9 @@ __global__ void __launch_bounds__(128, 7) glue_kernel(const GlueParams p) {
 }
 
 // The residual glue behind the routed experts, whose device-chosen split count can be 40 and more: grid (k / 64, 8); the four warps fetch a quarter
-// of the slices each (lane = token 2 y + lane / 16, four columns) and the first adds them in order, as one thread to all slices would: slices
-// that a row has no part in are zeros, so its sum does not depend on what the block's other rows chose.  With a thread to all slices the
+// of the slices each (lane = token 2 y + lane / 16, four columns) and the first adds them in order, as one thread to all slices would.  (Slices
+// that a row has no part in are zeros.  Where one slice ends and the next begins follows the list of all chosen experts, though, so the other rows of a
+// block do move how a row's sum is grouped, and with it the last bits.)  With a thread to all slices the
 // kernel was ten rounds of loads on a third of the chip (32 x 2 CTAs): a link of the chain 12.0 -> 8.9 us, with the join it no longer waits for.
 constexpr int SLICES_STAGED = 64;
 __global__ void __launch_bounds__(128) glue_slices_kernel(const GlueParams p) {

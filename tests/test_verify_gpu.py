@@ -210,11 +210,12 @@ def test_routed_expert_ffn_matches_oracle():
     gm.close()
 
 
-@pytest.mark.parametrize("experts,used", [(40, 3), (256, 8), (257, 5), (400, 32)])
-def test_routing_of_many_experts_matches_oracle(experts, used):
+@pytest.mark.parametrize("experts,used,hidden", [(40, 3, 256), (256, 8, 256), (257, 5, 256), (400, 32, 256), (800, 4, 256), (40, 8, 1280)])
+def test_routing_of_many_experts_matches_oracle(experts, used, hidden):
     # one warp's registers hold 8 or 32 experts a lane (the line lies at 256); 400 experts with 32 a row leave the down projection some
-    # seventy slices, more than the glue stages at a time.  f32 throughout: the file's tolerances.
-    arch = modelgen.tiny_arch(n_layer=1, expert_count=experts, expert_used_count=used, expert_feed_forward_length=256,
+    # seventy slices, more than the glue stages at a time; 800 need more shared memory than a launch has without asking; over 1280 columns the
+    # router has three slices, the last half full, and a slice of the down projection holds several experts.  f32 throughout: the file's tolerances.
+    arch = modelgen.tiny_arch(n_layer=1, hidden_size=hidden, expert_count=experts, expert_used_count=used, expert_feed_forward_length=256,
                               expert_shared_feed_forward_length=256)
     T = modelgen.target_tensors(arch, seed=23)
     om, gm = modelgen.OracleModel(arch, T), pkg.Model(arch, T)
@@ -227,7 +228,16 @@ def test_routing_of_many_experts_matches_oracle(experts, used):
         _, _, got = pkg.packed_verify(gm, sess, scr, [0], tokens, start, want_logits=True)
         np.testing.assert_allclose(got, want, rtol=RTOL, atol=ATOL)
         start += n
-    for o in (sess, scr, gm):
+    # the same first block token by token: the experts that the other rows chose move the borders of the down projection's slices, so the
+    # sums of at most `used` + 1 numbers are grouped otherwise (2^-23 each), and the head takes the changed rows as 22-bit operands (2^-22 either side)
+    one, tokens = pkg.Session(gm, 64, False), np.random.default_rng(7).integers(0, arch.vocab_size, size=16)
+    sess.close()
+    sess = pkg.Session(gm, 64, False)
+    _, _, packed = pkg.packed_verify(gm, sess, scr, [0], tokens, 0, want_logits=True)
+    for i, t in enumerate(tokens):
+        row, _ = pkg.single_token(gm, one, scr, [0], int(t), i)
+        assert np.linalg.norm(row - packed[i]) <= ((used + 1) * 2.0 ** -23 + 2.0 ** -21) * np.linalg.norm(packed[i]), i
+    for o in (sess, one, scr, gm):
         o.close()
 
 
