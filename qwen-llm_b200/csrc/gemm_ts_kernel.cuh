@@ -558,8 +558,12 @@ dfl_status launch_gemm_ts(cudaStream_t st, const QMatrix& m, const uint8_t* acts
     if ((ep.behind_late && ep.trigger_late) || ((ep.behind_late || ep.trigger_late) && !ep.late.word)) return fail(DFL_ERR_BAD_ARG, "gemm: dependency options");
     int grid = p.ctas_per_split * splits;
     if (ep.kb_map && ep.dynamic_splits && grid < sm_count()) grid = sm_count();   // room for the geometry chosen on the device
-    // four resident column blocks leave room for a fourth ring slot of a 35 KB stage (4096 x 32768 Q6_K 32.0 -> 31.0 us)
-    const bool four = !ep.kb_map && (m.kblocks + splits - 1) / splits <= 4;
+    // Four resident column blocks leave room for a fourth ring slot of a 35 KB stage.  It pays where a CTA has more than three stages to fetch
+    // (4096 -> 4096 -> 32000 matrix step, its head in Q6_K, 92.3 -> 89.5 us; 9B-class token 2546 -> 2534).  Where it has not, there is nothing to gain, and
+    // the other form is the one that the launch behind may use too: the shared expert's down projection, one stage a CTA, ahead of the routed
+    // experts' (token of the routed model 2972 us with four slots there, 2849 without; four rows 3647, 3579).
+    const int blocks = (m.kblocks + splits - 1) / splits, rounds = (m.row_tiles + p.ctas_per_split - 1) / p.ctas_per_split;
+    const bool four = !ep.kb_map && blocks <= 4 && rounds * blocks > 3;
     switch (m.dtype) {
         case DFL_Q4_K: return ts::launch_t<DFL_Q4_K, ts::KC_MAX>(st, p, grid, pdl);
         case DFL_Q5_K: return ts::launch_t<DFL_Q5_K, ts::KC_MAX>(st, p, grid, pdl);

@@ -11,7 +11,7 @@
 // so that a pair is one byte permute and one f16x2 multiply-add for each matrix, A1 / 16 = (72 + q / 16) s - 72 s with s the even part of the
 // scale and A2 / 16 likewise with its odd bit: every term is exact (72 s is 9 s / 2 x 16, 9 x 64 < 2048), and the 16 goes into d.  Byte permutes and
 // f16x2 arithmetic both issue at half rate, on different pipes; the form before (permute, subtract, multiply, mask) had
-// half as many again of the first kind (4096 x 32768 32.3 -> 32.0 us; a fourth ring slot beside it 30.5).
+// half as many again of the first kind (4096 x 32768 32.3 -> 32.0 us).
 // The values are ggml's, bit for bit.
 //
 // Stage (128 rows x 256 columns): [row 128][16 x i8 scales] [row 128][f16 d] [block 8][half 2][row 128][16 bytes], byte j

@@ -62,6 +62,21 @@ def test_matmul_matches_oracle(dtype, name, n_in, n_out, n_rows):
     m.close()
 
 
+@pytest.mark.parametrize("dtype", [orc.Q6_K, orc.Q8_0])
+@pytest.mark.parametrize("n_in,n_out", [(256, 38400), (1024, 8192), (1024, 18944), (512, 19072), (2048, 8192)])
+def test_ring_of_four_slots_at_its_edges(dtype, n_in, n_out):
+    # at most four column blocks a CTA: three ring slots while a CTA has up to three stages (the first two on 148 SMs), four beyond; in a split
+    # of two and in one; the bound of the test above
+    raw, wf = make_weight(dtype, n_in, n_out, 13)
+    x = np.random.default_rng(19).standard_normal((16, n_in)).astype(np.float32)
+    m = pkg.QMatrix(dtype, n_in, n_out, raw)
+    got = m.matmul(x)
+    exact = x.astype(np.float64) @ wf.astype(np.float64).T
+    bound = (np.abs(x).astype(np.float64) @ np.abs(wf).astype(np.float64).T) * (n_in * 2.0 ** -24) + 1e-30
+    assert np.all(np.abs(got - exact) <= bound)
+    m.close()
+
+
 @pytest.mark.parametrize("dtype,name", DTYPES)
 def test_rows_do_not_depend_on_row_count(dtype, name):
     # q6_k_f32_tile.rs:261-312: bitwise the same row for any number of rows in the call
