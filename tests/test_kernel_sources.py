@@ -63,7 +63,7 @@ def test_launches_without_a_dependency_wait_acquire_a_mark():
     trigger = gemm[gemm.index("auto trigger"):]
     assert trigger.index("pdl_wait()") < trigger.index("pdl_launch_dependents()")
     publish = gemm.index("late_publish(")
-    assert re.search(r"trigger\(\);\s*if \(p\.late_mode == LATE_FIRST && blockIdx\.x == 0 && lane == 0\) $", gemm[:publish])   # behind the wait in trigger
+    assert re.search(r"trigger\(\);\s*if \(p\.late_mode == LATE_FIRST && blockIdx\.x == gridDim\.x - 1 && lane == 0\) $", gemm[:publish])   # behind the wait in trigger
     copies = gemm.index("bulk_g2s(acts_res")
     assert gemm.rindex('"fence.proxy.async.global;"', 0, copies) > gemm.rindex("wait_inputs();", 0, copies)
     ab = readers["ab_proj_kernel"]
