@@ -234,7 +234,7 @@ void dfl_model_destroy(dfl_model* m);
 /* Bytes of quantised weights one verify step streams (the roofline numerator). */
 uint64_t dfl_model_verify_weight_bytes(const dfl_model* m);
 /* The same matrices counted as they are resident in HBM: equal to the above except that Q6_K tiles of the
- * tensor-memory GEMM hold one six-bit code per byte (274 bytes per 256 weights against ggml's 210). */
+ * tensor-memory GEMM hold one weight per byte (274 bytes per 256 weights against ggml's 210). */
 uint64_t dfl_model_verify_resident_bytes(const dfl_model* m);
 /* Expert parallelism for routed-expert models (one process per GPU of one node).
  * Rank r of ep_world keeps experts [r*E/ep_world, (r+1)*E/ep_world) of every layer

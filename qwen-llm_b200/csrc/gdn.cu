@@ -221,8 +221,8 @@ dfl_status launch_gdn_rescan(cudaStream_t st, const GdnGeom& g, const float* sta
 //     one cluster barrier, rank-ordered sum, then packs its 32 columns (one sub-block) of the output projection's activations.
 // Loops stay loops: the kernel runs once a layer between kernels that fill the instruction caches, and straight code is fetched once per pass.
 // (Three warps running through the code once before the wait, as the glue does, took longer than the 1 - 5 us there are: verify block 2747 -> 2953 us.)
-// A row's result does not depend on how many rows the block has.  Measured (9B-class widths, 16 rows, end of
-// the projections to end of the mixer): 20.9 -> 12.8 us, of which waiting for alpha / beta 6.5, exchanging q and k 1.5 - 2, the recurrence 2 were saved.
+// A row's result does not depend on how many rows the block has.  Measured (9B-class widths, 16 rows, end of the projections to end of the
+// mixer): 20.9 -> 13.4 us, 2.4 of them the alpha / beta kernel, which the mixer waited for before.
 constexpr int MIX_THREADS = 288;
 __global__ void __cluster_dims__(1, 4, 1) __launch_bounds__(MIX_THREADS) gdn_mix_kernel(const GdnMixParams p) {
     __shared__ __align__(16) float raw[(MAX_ROWS + 3) * 288];   // input rows of the convolution behind the three old ones

@@ -6,9 +6,9 @@
 //   * a producer thread streams 128-row x 256-column stages of packed weights with bulk copies
 //     into a shared-memory ring; the packed activations of the CTA's column range are copied
 //     once and stay resident as the B operand;
-//   * sixteen unpacking warps turn the integer quants into exact f16 integers q * sc (the
+//   * eight unpacking warps in two groups turn the integer quants into exact f16 integers q * sc (the
 //     6-bit sub-block scale folded in, still exact: q * sc < 2048) and store them with
-//     tcgen05.st into tensor memory, thread = (row, quarter of the columns), row = TMEM lane.
+//     tcgen05.st into tensor memory, thread = weight row = TMEM lane.
 //     They do nothing else, so their instruction stream never waits for an accumulator;
 //   * four warps, one per scheduler, issue tcgen05.mma (A from tensor memory, B = activations
 //     hi / lo planes from shared memory, M = 128, N = 32, K = 16 per instruction), sixteen per
